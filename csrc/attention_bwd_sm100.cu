@@ -45,6 +45,18 @@ constexpr int KV_MAX_TILES = 512;  // query tiles whose position range fits the 
 constexpr int DQ_KSTAGES = 3;      // dQ kernel: K tile ring (a K tile is held from S(j) to dQ(j))
 constexpr int DQ_VSTAGES = 2;      // dQ kernel: V tile ring
 constexpr float kLog2e = 1.4426950408889634f;
+constexpr int SEG_BLK = 64;        // tokens per entry of the segment-range tables
+
+// Segment-id range of the 128-token tile `t` of batch row `b` from the table of 64-token ranges.
+__device__ __forceinline__ int2 seg_range128(const int2* rng, int b, int t, int S) {
+  const int2* r = rng + (long long)b * ((S + SEG_BLK - 1) / SEG_BLK) + t * (BWD_T / SEG_BLK);
+  int2 a = r[0];
+  if (t * BWD_T + SEG_BLK < S) {
+    const int2 c = r[1];
+    a.x = min(a.x, c.x); a.y = max(a.y, c.y);
+  }
+  return a;
+}
 
 struct AttnBwdParams {
   int B, Sq, Sk, Hq, Hkv;
@@ -55,6 +67,8 @@ struct AttnBwdParams {
   const int* q_pos;
   const int* q_seg;
   const int* kv_seg;
+  const int2* q_rng;    // smallest and largest segment id of every 64 queries / keys, or null
+  const int2* kv_rng;   // (attn_seg_ranges_kernel of the forward)
   const float* lse2;    // [B,Hq,Sq_pad] log-sum-exp in log2 units, +inf in the padding rows
   const float* delta;   // [B,Hq,Sq_pad] rowsum(dO o O), 0 in the padding rows
   int Sq_pad;           // Sq rounded up to 128
@@ -73,8 +87,10 @@ constexpr int OFF_DO = OFF_Q + KV_QSTAGES * TILE_BYTES;
 constexpr int OFF_AUX = OFF_DO + KV_DOSTAGES * TILE_BYTES;   // per Q stage: lse2[128], delta[128], qpos[128], qseg[128]
 constexpr int AUX_STAGE = 4 * BWD_T * 4;
 constexpr int OFF_TILES = OFF_AUX + KV_QSTAGES * AUX_STAGE;  // tile min/max table: 2 * KV_MAX_TILES ints
-constexpr int OFF_BAR = OFF_TILES + 2 * KV_MAX_TILES * 4;
+constexpr int OFF_SEGONE = OFF_TILES + 2 * KV_MAX_TILES * 4;  // per tile: 1 = all of its and this block's ids are one id
+constexpr int OFF_BAR = OFF_SEGONE + KV_MAX_TILES;
 constexpr int TOTAL = OFF_BAR + 256 + 1024;
+static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
 constexpr int T_DK = 0, T_DV = 128, T_S = 256, T_DP = 384;
 }  // namespace dkv
 
@@ -195,7 +211,8 @@ __device__ __forceinline__ uint32_t a_col(int k) { return (uint32_t)((k >> 2) * 
 // ------------------------------------------------------------------------------------------
 // dK / dV
 // ------------------------------------------------------------------------------------------
-template <bool SOFTCAP>
+// SEG: segment ids come with their range tables.
+template <bool SOFTCAP, bool SEG>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                     const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -217,6 +234,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 5);
   int* tile_min = reinterpret_cast<int*>(smem + OFF_TILES);
   int* tile_max = tile_min + KV_MAX_TILES;
+  uint8_t* seg_one = smem + OFF_SEGONE;
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   // linear block id is key-block major so that under a causal mask the blocks with the most
@@ -241,6 +259,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tmem_relinquish();
   }
   // position range of every query tile (decides which tiles this key block can see)
+  const int2 kseg_rng = SEG ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
   for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
     const int r0 = t * BWD_T, r1 = min(p.Sq, r0 + BWD_T);
     int mn = 0x7fffffff, mx = -0x7fffffff;
@@ -252,6 +271,11 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     } else {
       mn = r0 + pos_off; mx = r1 - 1 + pos_off;
     }
+    if (SEG) {
+      const int2 qr = seg_range128(p.q_rng, b, t, p.Sq);
+      seg_one[t] = qr.x == qr.y && kseg_rng.x == kseg_rng.y && qr.x == kseg_rng.x;
+      if (qr.y < kseg_rng.x || qr.x > kseg_rng.y) { mn = 0x7fffffff; mx = -0x7fffffff; }   // no segment in common
+    }
     tile_min[t] = mn; tile_max[t] = mx;
   }
   tc_fence_before();
@@ -260,6 +284,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const uint32_t tmem_base = *tmem_slot;
 
   auto visible = [&](int t) -> bool {
+    if (SEG && tile_min[t] > tile_max[t]) return false;
     if (p.causal && tile_max[t] < kv0) return false;
     if (p.window > 0 && tile_min[t] - (kv0 + BWD_T - 1) >= p.window) return false;
     return true;
@@ -426,7 +451,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         const float* aux = reinterpret_cast<const float*>(smem + OFF_AUX + sq * AUX_STAGE);
         const int* auxi = reinterpret_cast<const int*>(aux);
         const bool need_mask = !key_ok || (kv0 + BWD_T > p.Sk) || (p.causal && tile_min[t] < kv0 + BWD_T - 1) ||
-                               (p.window > 0 && tile_max[t] - kv0 >= p.window) || p.q_seg != nullptr;
+                               (p.window > 0 && tile_max[t] - kv0 >= p.window) ||
+                               (p.q_seg != nullptr && !(SEG && seg_one[t]));
         // ---- phase 1: P^T = exp2(S^T * c - lse), kept packed for phase 2 and written over S^T
         if (!mbar_wait(s_full, step & 1, p.status, kTimeoutAccFull, 27)) { ok = false; break; }
         tc_fence_after();
@@ -546,7 +572,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 // ------------------------------------------------------------------------------------------
 // dQ
 // ------------------------------------------------------------------------------------------
-template <bool SOFTCAP>
+template <bool SOFTCAP, bool SEG>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                    const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -566,6 +592,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   uint64_t* acc_done = s_full + 4;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 5);
   int* tile_minmax = reinterpret_cast<int*>(s_full + 6);  // [2]
+  int* seg_lohi = reinterpret_cast<int*>(s_full + 7);     // [2] first and last key block with a segment of this tile
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qtiles = (p.Sq + BWD_T - 1) / BWD_T;
@@ -585,6 +612,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     mbar_init(acc_done, 1);
     tile_minmax[0] = 0x7fffffff;
     tile_minmax[1] = -0x7fffffff;
+    if (SEG) { seg_lohi[0] = 0x7fffffff; seg_lohi[1] = -1; }
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -610,6 +638,20 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   int blk_hi = p.causal ? min(nblk_total, qpos_max / BWD_T + 1) : nblk_total;
   int blk_lo = (p.window > 0) ? max(0, (qpos_min - p.window + 1) / BWD_T) : 0;
   if (qpos_max < 0) blk_hi = 0;
+  int2 qr = make_int2(0, 0);
+  if (SEG) {   // as in the forward: only the key blocks between the first and last with a common segment
+    qr = seg_range128(p.q_rng, b, qt, p.Sq);
+    for (int i = blk_lo + (int)threadIdx.x; i < blk_hi; i += BWD_THREADS) {
+      const int2 kr = seg_range128(p.kv_rng, b, i, p.Sk);
+      if (kr.x <= qr.y && kr.y >= qr.x) {
+        atomicMin(&seg_lohi[0], i);
+        atomicMax(&seg_lohi[1], i);
+      }
+    }
+    __syncthreads();
+    blk_lo = max(blk_lo, seg_lohi[0]);
+    blk_hi = min(blk_hi, seg_lohi[1] + 1);
+  }
   const int nblk = max(0, blk_hi - blk_lo);
 
   if (warp == 0) {
@@ -715,8 +757,13 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
     for (int j = 0; j < nblk && ok; ++j) {
       const int kv0 = (blk_lo + j) * BWD_T;
+      bool seg_mask = p.q_seg != nullptr;
+      if (SEG) {
+        const int2 kr = seg_range128(p.kv_rng, b, blk_lo + j, p.Sk);
+        seg_mask = !(qr.x == qr.y && kr.x == kr.y && qr.x == kr.x);
+      }
       const bool need_mask = (p.causal && kv0 + BWD_T - 1 > qpos_min) || (kv0 + BWD_T > p.Sk) ||
-                             (p.window > 0 && qpos_max - kv0 >= p.window) || p.q_seg != nullptr;
+                             (p.window > 0 && qpos_max - kv0 >= p.window) || seg_mask;
       const uint32_t tS = tb + T_S + (j & 1) * BWD_T + half * 64;
       // ---- phase 1: P = exp2(S * c - lse), packed bf16 in registers
       if (!mbar_wait(&s_full[j & 1], (j >> 1) & 1, p.status, kTimeoutAccFull, 36)) { ok = false; break; }
@@ -751,7 +798,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
             for (int e = 0; e < 2; ++e) {
               const int kp = kbase + c + e;
               bool keep = (kp <= kmax) & (qpos - kp < win);
-              if (ks) keep = keep & (__ldg(ks + min(kp, p.Sk - 1)) == qseg);
+              if (ks && (!SEG || seg_mask)) keep = keep & (__ldg(ks + min(kp, p.Sk - 1)) == qseg);
               float sv = __uint_as_float(s[c + e]), fv = 1.f;
               if (SOFTCAP) {
                 sv = tanh_approx(sv * p.softcap_in);
@@ -813,7 +860,8 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
                                     int Sk, int Hq, int Hkv, int dqk, int dvd, long long ldq, long long ldk,
                                     long long ldv, long long lddo, long long lddq, long long lddk, long long lddv,
                                     float scale, int causal, int window, const int* q_pos, const int* q_seg,
-                                    const int* kv_seg, float softcap, void* stream_) {
+                                    const int* kv_seg, const int* q_rng, const int* kv_rng, float softcap,
+                                    void* stream_) {
   if (dqk != 128 || dvd != 128 || Hq % Hkv) return -2;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (lddo % 8) || (lddq % 8) || (lddk % 8) || (lddv % 8)) return -2;
   if (lddo != (long long)Hq * dvd) return -2;   // dO and O are contiguous [B*Sq, Hq, 128]
@@ -839,6 +887,9 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
   p.scale_log2 = (softcap > 0.f ? softcap : scale) * kLog2e;
   p.causal = causal; p.window = window;
   p.q_pos = q_pos; p.q_seg = q_seg; p.kv_seg = kv_seg;
+  const bool ranges = q_seg && kv_seg && q_rng && kv_rng;
+  p.q_rng = ranges ? reinterpret_cast<const int2*>(q_rng) : nullptr;
+  p.kv_rng = ranges ? reinterpret_cast<const int2*>(kv_rng) : nullptr;
   p.lse2 = lse2; p.delta = delta; p.Sq_pad = sq_pad;
   p.aux_bulk = (Sq % 4 == 0) && (reinterpret_cast<uintptr_t>(q_pos) % 16 == 0) &&
                (reinterpret_cast<uintptr_t>(q_seg) % 16 == 0);
@@ -848,13 +899,14 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
   p.status = status_block();
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(attn_bwd_dkv_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dkv::TOTAL);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_bwd_dq_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, dqk::TOTAL);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_bwd_dkv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dkv::TOTAL);
-    if (e == cudaSuccess)
-      e = cudaFuncSetAttribute(attn_bwd_dq_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, dqk::TOTAL);
+    cudaError_t e = cudaSuccess;
+    auto allow = [&](const void* kernel, int bytes) {
+      if (e == cudaSuccess) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    allow((const void*)attn_bwd_dkv_kernel<false, false>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<false, false>, dqk::TOTAL);
+    allow((const void*)attn_bwd_dkv_kernel<false, true>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<false, true>, dqk::TOTAL);
+    allow((const void*)attn_bwd_dkv_kernel<true, false>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<true, false>, dqk::TOTAL);
+    allow((const void*)attn_bwd_dkv_kernel<true, true>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<true, true>, dqk::TOTAL);
     if (e != cudaSuccess) return 1000 + (int)e;
     configured = true;
   }
@@ -865,13 +917,15 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
   if (make_tmap_3d(&tv, v, dvd, (uint64_t)B * Sk, Hkv, ldv, dvd, 64, BWD_T)) return -5;
   if (make_tmap_3d(&tdo, dO, dvd, (uint64_t)B * Sq, Hq, lddo, dvd, 64, BWD_T)) return -5;
   dim3 grid_kv(((Sk + BWD_T - 1) / BWD_T) * Hkv * B, 1, 1);
-  if (softcap > 0.f) attn_bwd_dkv_kernel<true><<<grid_kv, BWD_THREADS, dkv::TOTAL, stream>>>(tq, tk, tv, tdo, p);
-  else attn_bwd_dkv_kernel<false><<<grid_kv, BWD_THREADS, dkv::TOTAL, stream>>>(tq, tk, tv, tdo, p);
+  (softcap > 0.f ? (ranges ? attn_bwd_dkv_kernel<true, true> : attn_bwd_dkv_kernel<true, false>)
+                 : (ranges ? attn_bwd_dkv_kernel<false, true> : attn_bwd_dkv_kernel<false, false>))
+      <<<grid_kv, BWD_THREADS, dkv::TOTAL, stream>>>(tq, tk, tv, tdo, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return 1000 + (int)e;
   dim3 grid_q(((Sq + BWD_T - 1) / BWD_T) * Hq * B, 1, 1);
-  if (softcap > 0.f) attn_bwd_dq_kernel<true><<<grid_q, BWD_THREADS, dqk::TOTAL, stream>>>(tq, tk, tv, tdo, p);
-  else attn_bwd_dq_kernel<false><<<grid_q, BWD_THREADS, dqk::TOTAL, stream>>>(tq, tk, tv, tdo, p);
+  (softcap > 0.f ? (ranges ? attn_bwd_dq_kernel<true, true> : attn_bwd_dq_kernel<true, false>)
+                 : (ranges ? attn_bwd_dq_kernel<false, true> : attn_bwd_dq_kernel<false, false>))
+      <<<grid_q, BWD_THREADS, dqk::TOTAL, stream>>>(tq, tk, tv, tdo, p);
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }
@@ -882,5 +936,5 @@ extern "C" int tpb_attn_bwd(const void* dO, const void* q, const void* k, const 
                             long long lddo, long long lddq, long long lddk, long long lddv, float scale, int causal,
                             int window, const int* q_pos, const int* q_seg, const int* kv_seg, void* stream_) {
   return tpb_attn_bwd_softcap(dO, q, k, v, o, lse, scratch, dq, dk, dv, B, Sq, Sk, Hq, Hkv, dqk, dvd, ldq, ldk, ldv, lddo,
-                              lddq, lddk, lddv, scale, causal, window, q_pos, q_seg, kv_seg, 0.f, stream_);
+                              lddq, lddk, lddv, scale, causal, window, q_pos, q_seg, kv_seg, nullptr, nullptr, 0.f, stream_);
 }

@@ -165,7 +165,10 @@ int tpb_attn_fwd(const void* q, const void* k, const void* v, void* o, float* ls
 int tpb_attn_fwd_softcap(const void* q, const void* k, const void* v, void* o, float* lse, int B, int Sq, int Sk,
                          int Hq, int Hkv, int dqk, int dv, long long ldq, long long ldk, long long ldv, long long ldo,
                          float scale, int causal, int window, const int* q_pos, const int* q_seg, const int* kv_seg,
-                         float softcap, void* stream);
+                         const int* q_rng, const int* kv_rng, float softcap, void* stream);
+// Segment-id ranges of every 64 tokens, out [B, ceil(S / 64)] pairs (min, max): with both tables (q_rng of the
+// queries, kv_rng of the keys) the attention kernels skip key blocks that share no segment with a query tile.
+int tpb_attn_seg_ranges(const int* seg, int* out, int B, int S, void* stream);
 // Causal forward with the context-parallel K/V exchange fused in (see attention_fwd_sm100.cu).
 int tpb_attn_fwd_cp(const void* q, const void* k_local, const void* v_local, void* const* k_all, void* const* v_all,
                     unsigned* const* flags, void* o, float* lse, int B, int Sq, int s_local, int Hq, int Hkv,
@@ -183,7 +186,7 @@ int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k, const voi
                  float* scratch, void* dq, void* dk, void* dv, int B, int Sq, int Sk, int Hq, int Hkv,
                  int dqk, int dvd, long long ldq, long long ldk, long long ldv, long long lddo, long long lddq,
                  long long lddk, long long lddv, float scale, int causal, int window, const int* q_pos,
-                 const int* q_seg, const int* kv_seg, float softcap, void* stream);
+                 const int* q_seg, const int* kv_seg, const int* q_rng, const int* kv_rng, float softcap, void* stream);
 
 // ---- symmetric-memory runtime (symm_runtime.cu): segments that every rank maps, and a bounded
 // device-side barrier on their signal pads.

@@ -1,0 +1,70 @@
+"""Attention kernels skip key blocks that share no segment with a query tile (ranges of the ids)."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from torchprime_b200.ops import attention_sm100 as A
+from torchprime_b200.ops import reference as ref
+from torchprime_b200.ops._lib import check, lib, ptr, stream_ptr
+
+
+def _ids(kind, b, s):
+  g = torch.Generator(device="cuda").manual_seed(s + b)
+  if kind == "sorted":
+    cuts = torch.randint(0, s, (b, 5), device="cuda", generator=g)
+    at = torch.arange(s, device="cuda")
+    return (at[None, :, None] >= cuts[:, None, :]).sum(-1).to(torch.int32)
+  if kind == "one":
+    return torch.full((b, s), 3, dtype=torch.int32, device="cuda")
+  if kind == "blocks":       # ids that change at tile edges, decreasing, with the int32 extremes
+    at = torch.arange(s, device="cuda") // 64
+    ids = (-at).to(torch.int32)
+    ids[at == 0] = 2 ** 31 - 1
+    ids[at == at.max()] = -2 ** 31
+    return ids.expand(b, s).contiguous()
+  return torch.randint(-2, 2, (b, s), device="cuda", generator=g).to(torch.int32)   # no order at all
+
+
+@pytest.mark.parametrize("s", [1, 63, 64, 65, 200])
+@pytest.mark.parametrize("kind", ["sorted", "blocks", "mixed"])
+def test_range_tables(cuda_lib, s, kind):
+  ids = _ids(kind, 3, s)
+  n = (s + 63) // 64
+  out = torch.empty(3, n, 2, dtype=torch.int32, device="cuda")
+  check(lib().tpb_attn_seg_ranges(ptr(ids), ptr(out), 3, s, stream_ptr()), "seg_ranges")
+  for i in range(n):
+    part = ids[:, 64 * i:64 * (i + 1)]
+    assert torch.equal(out[:, i, 0], part.amin(-1)) and torch.equal(out[:, i, 1], part.amax(-1))
+
+
+@pytest.mark.parametrize("causal,window", [(True, None), (False, None), (True, 70)])
+@pytest.mark.parametrize("s", [40, 128, 129, 320, 777])
+@pytest.mark.parametrize("kind", ["sorted", "one", "blocks", "mixed"])
+def test_forward_and_backward(cuda_lib, s, kind, causal, window):
+  """Against the fp32 definition; the bound is that of the unsegmented kernels' tests."""
+  torch.manual_seed(s)
+  b, hq, hkv = 2, 4, 2
+  q, k, v = (torch.randn(b, s, h, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True) for h in (hq, hkv, hkv))
+  ids = _ids(kind, b, s)
+  o = A.attention(q, k, v, causal=causal, window=window, q_segment_ids=ids)
+  do = torch.randn_like(o)
+  got = torch.autograd.grad(o, (q, k, v), do)
+  qf, kf, vf = (t.detach().float().requires_grad_(True) for t in (q, k, v))
+  w = ref.attention(qf, kf, vf, causal=causal, window=window, q_segment_ids=ids)
+  want = torch.autograd.grad(w, (qf, kf, vf), do.float())
+  for g, r in zip((o, *got), (w, *want)):
+    assert ((g.float() - r.float()).norm() / r.float().norm()).item() < 2e-2
+
+
+def test_keys_and_queries_with_other_ids(cuda_lib):
+  """Key ids of their own: a query tile whose segment no key has gives zeros and zero gradients."""
+  q, k, v = (torch.randn(1, 300, 2, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
+  q_seg = torch.zeros(1, 300, dtype=torch.int32, device="cuda")
+  kv_seg = torch.zeros(1, 300, dtype=torch.int32, device="cuda")
+  q_seg[:, 128:256] = 9
+  o = A.attention(q, k, v, causal=False, q_segment_ids=q_seg, kv_segment_ids=kv_seg)
+  dq, dk, dv = torch.autograd.grad(o, (q, k, v), torch.randn_like(o))
+  assert bool((o[:, 128:256] == 0).all()) and bool((dq[:, 128:256] == 0).all())
+  assert bool(torch.isfinite(dk).all()) and bool(torch.isfinite(dv).all()) and bool((dv != 0).any())

@@ -22,11 +22,12 @@ P, I, LL, F = c_void_p, c_int, c_longlong, c_float
 _lib.register_signature("tpb_attn_fwd", [P, P, P, P, P, I, I, I, I, I, I, I, LL, LL, LL, LL, F, I, I, P, P, P, P])
 _lib.register_signature("tpb_attn_bwd", [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, LL, LL, LL, LL, LL,
                                          LL, LL, F, I, I, P, P, P, P])
-# the same with a logit soft cap (a float before the stream)
-_lib.register_signature("tpb_attn_fwd_softcap", [P, P, P, P, P, I, I, I, I, I, I, I, LL, LL, LL, LL, F, I, I, P, P, P, F,
-                                                 P])
+# the same with segment-id range tables and a logit soft cap before the stream
+_lib.register_signature("tpb_attn_fwd_softcap", [P, P, P, P, P, I, I, I, I, I, I, I, LL, LL, LL, LL, F, I, I, P, P, P, P,
+                                                 P, F, P])
 _lib.register_signature("tpb_attn_bwd_softcap", [P, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, LL, LL, LL, LL, LL,
-                                                 LL, LL, F, I, I, P, P, P, F, P])
+                                                 LL, LL, F, I, I, P, P, P, P, P, F, P])
+_lib.register_signature("tpb_attn_seg_ranges", [P, P, I, I, P])
 
 
 _lib.register_signature("tpb_attn_fwd_cp", [P, P, P, P, P, P, P, P, I, I, I, I, I, LL, LL, LL, LL, F, P, I, I, I, I,
@@ -85,6 +86,22 @@ def _i32(t):
   return None if t is None else t.reshape(-1).to(torch.int32).contiguous()
 
 
+def _seg_ranges(q_seg, kv_seg, b, sq, sk):
+  """(smallest, largest) segment id of every 64 queries and of every 64 keys: the kernels skip key
+  blocks that share no segment with a query tile.  (None, None) without segments."""
+  if q_seg is None or kv_seg is None:
+    return None, None
+
+  def table(seg, s):
+    out = torch.empty(b, (s + 63) // 64, 2, dtype=torch.int32, device=seg.device)
+    check(lib().tpb_attn_seg_ranges(ptr(seg), ptr(out), b, s, stream_ptr()), "attn_seg_ranges")
+    return out
+
+  kv = table(kv_seg, sk)
+  same = sq == sk and q_seg.data_ptr() == kv_seg.data_ptr()
+  return (kv if same else table(q_seg, sq)), kv
+
+
 def attn_fwd(q, k, v, causal=True, scale=None, window=None, q_pos=None, q_seg=None, kv_seg=None, softcap=None):
   """Returns (o [B,Sq,Hq,128] contiguous, lse [B,Hq,Sq] fp32 in natural-log units).  ``softcap``: the scores
   become ``softcap * tanh(q.k * scale / softcap)`` before the softmax."""
@@ -93,10 +110,11 @@ def attn_fwd(q, k, v, causal=True, scale=None, window=None, q_pos=None, q_seg=No
   scale = scale if scale is not None else 1.0 / math.sqrt(dqk)
   o = torch.empty(b, sq, hq, dv, dtype=q.dtype, device=q.device)
   lse = torch.empty(b, hq, sq, dtype=torch.float32, device=q.device)
+  q_rng, kv_rng = _seg_ranges(q_seg, kv_seg, b, sq, sk)
   rc = lib().tpb_attn_fwd_softcap(ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), b, sq, sk, hq, hkv, dqk, dv, q.stride(1),
                                   k.stride(1), v.stride(1), hq * dv, float(scale), int(bool(causal)),
-                                  int(window or 0), ptr(q_pos), ptr(q_seg), ptr(kv_seg), float(softcap or 0.0),
-                                  stream_ptr())
+                                  int(window or 0), ptr(q_pos), ptr(q_seg), ptr(kv_seg), ptr(q_rng), ptr(kv_rng),
+                                  float(softcap or 0.0), stream_ptr())
   check(rc, f"attn_fwd q{tuple(q.shape)} k{tuple(k.shape)}")
   return o, lse
 
@@ -117,11 +135,12 @@ def attn_bwd(do, q, k, v, o, lse, causal=True, scale=None, window=None, q_pos=No
     assert not softcap, "the capped backward exists for head dim 128 only"
     return _eager_bwd(do, q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv)
   scratch = torch.empty(2 * b * hq * ((sq + 127) // 128 * 128), dtype=torch.float32, device=q.device)
+  q_rng, kv_rng = _seg_ranges(q_seg, kv_seg, b, sq, sk)
   rc = lib().tpb_attn_bwd_softcap(ptr(do), ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), ptr(scratch), ptr(dq),
                                   ptr(dk), ptr(dv), b, sq, sk, hq, hkv, dqk, dvd, q.stride(1), k.stride(1),
                                   v.stride(1), do.stride(1), dq.stride(1), dk.stride(1), dv.stride(1), float(scale),
                                   int(bool(causal)), int(window or 0), ptr(q_pos), ptr(q_seg), ptr(kv_seg),
-                                  float(softcap or 0.0), stream_ptr())
+                                  ptr(q_rng), ptr(kv_rng), float(softcap or 0.0), stream_ptr())
   check(rc, f"attn_bwd q{tuple(q.shape)} k{tuple(k.shape)}")
   return dq, dk, dv
 
