@@ -197,6 +197,9 @@ int tpb_symm_copy(void* dst, const void* src, long long bytes, void* stream);
 int tpb_symm_live_segments(void);
 int tpb_symm_barrier(void* const* payloads, int rank, int world, unsigned epoch, void* stream);
 
+// dst[i] = bf16(src[i] * *scale), scale in device memory; n % 8 == 0
+int tpb_scale_cast_bf16(const float* src, void* dst, long long n, const float* scale, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -74,6 +74,7 @@ def _declare(L):
     "tpb_embedding_fwd": [P, P, P, I, I, LL, LL, P],
     "tpb_embedding_bwd": [P, P, P, I, I, LL, LL, I, P],
     "tpb_cast_f32_to_bf16": [P, P, LL, F, I, P],
+    "tpb_scale_cast_bf16": [P, P, LL, P, P],
   }
   for name, args in sigs.items():
     fn = getattr(L, name, None)

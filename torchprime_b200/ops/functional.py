@@ -650,7 +650,9 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
     sink = _grad_sink([w]) if need_dw else None
     dw_local = None
     if need_dw and sink is None:
-      dw_local = torch.zeros(w.shape, dtype=torch.float32, device=w.device)
+      dw_local = torch.empty(w.shape, dtype=torch.float32, device=w.device)   # the first chunk overwrites it
+      if rows == 0:
+        dw_local.zero_()
     logits = torch.empty(min(chunk_rows, rows), vocab, dtype=torch.bfloat16, device=h.device)
     for r0 in range(0, rows, chunk_rows):
       r1 = min(rows, r0 + chunk_rows)
@@ -663,7 +665,7 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
         if sink is not None:
           _wgrad_into(sink, [w], lg, h2[r0:r1])
         else:
-          k.gemm(lg, h2[r0:r1], a_mn=True, b_mn=True, out=dw_local, epi=k.EPI_F32_ACC)
+          k.gemm(lg, h2[r0:r1], a_mn=True, b_mn=True, out=dw_local, epi=k.EPI_F32 if r0 == 0 else k.EPI_F32_ACC)
     ctx.save_for_backward(dh if need_dh else None, dw_local)
     ctx.h_shape = h.shape
     return (loss_sum * scale).reshape(())
@@ -672,7 +674,12 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
   def backward(ctx, dloss):
     dh, dw_local = ctx.saved_tensors
     gh = (dh * dloss.to(dh.dtype)).view(ctx.h_shape) if dh is not None else None
-    gw = (dw_local * dloss).to(torch.bfloat16) if dw_local is not None else None
+    gw = None
+    if dw_local is not None and torch.is_grad_enabled() and dloss.requires_grad:
+      gw = (dw_local * dloss).to(torch.bfloat16)      # a derivative with respect to dloss is wanted
+    elif dw_local is not None:
+      from . import kernels as k
+      gw = k.scale_cast_bf16(dw_local, dloss.float())
     return gh, gw, None, None, None
 
 

@@ -177,3 +177,11 @@ def cast_f32_to_bf16_(src, dst, scale=1.0, accumulate=False):
   check(lib().tpb_cast_f32_to_bf16(ptr(src), ptr(dst), src.numel(), float(scale), int(accumulate), stream_ptr()),
         "cast_f32_to_bf16")
   return dst
+
+
+def scale_cast_bf16(src, scale):
+  """bf16(src * scale) of a contiguous fp32 tensor and a one-element fp32 tensor, in one pass."""
+  assert src.dtype == scale.dtype == torch.float32 and scale.numel() == 1 and src.is_contiguous()
+  out = torch.empty(src.shape, dtype=torch.bfloat16, device=src.device)
+  check(lib().tpb_scale_cast_bf16(ptr(src), ptr(out), src.numel(), ptr(scale), stream_ptr()), "scale_cast_bf16")
+  return out
