@@ -1,0 +1,37 @@
+"""Operators with nothing recorded."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from torchprime_b200.ops import functional as ops
+
+
+def test_operators_without_a_graph_equal_those_with_one(cuda_lib):
+  """Nothing recorded: the operators skip their autograd functions; results, in-place writes and version
+  counters are the same."""
+  torch.manual_seed(0)
+  x = torch.randn(2, 40, 256, device="cuda", dtype=torch.bfloat16)
+  w = torch.randn(256, 256, device="cuda", dtype=torch.bfloat16) / 16
+  g = torch.randn(512, 256, device="cuda", dtype=torch.bfloat16) / 16
+  n = torch.randn(256, device="cuda", dtype=torch.bfloat16)
+  ids = torch.randint(0, 256, (2, 40), device="cuda")
+  cos, sin = torch.randn(40, 64, device="cuda"), torch.randn(40, 64, device="cuda")
+  def every():
+    qkv = torch.randn(2, 40, 6 * 128, device="cuda", dtype=torch.bfloat16, generator=torch.Generator("cuda").manual_seed(1))
+    r = ops.rope_inplace(qkv * 1, cos, sin, 5, 128, 40)
+    return [ops.linear(x, w), ops.linear(x, w, residual=x), ops.linear_swiglu(x, g[:256], g[256:]), ops.rms_norm(x, n, 1e-5),
+            *ops.rms_norm_residual(x, n, 1e-5), r, ops.embedding(ids, w),
+            ops.attention_qkv(r, 4, 1, 128)]
+  with_graph = every()
+  with torch.no_grad():
+    without = every()
+  for a, b in zip(with_graph, without):
+    assert torch.equal(a, b) and not b.requires_grad
+  t = torch.randn(1, 40, 256, device="cuda", dtype=torch.bfloat16)
+  v = t._version
+  with torch.no_grad():
+    assert ops.rope_inplace(t, cos, sin, 2, 128, 40) is t and t._version == v + 1
+  with torch.inference_mode():
+    ops.rope_inplace(torch.randn(1, 40, 256, device="cuda", dtype=torch.bfloat16), cos, sin, 2, 128, 40)

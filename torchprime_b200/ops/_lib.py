@@ -40,7 +40,7 @@ def lib_path() -> str:
 
 
 def available() -> bool:
-  return os.path.exists(_LIB_PATH)
+  return _lib is not None or os.path.exists(_LIB_PATH)   # (a loaded library needs no look at the file system)
 
 
 def lib():
@@ -106,7 +106,7 @@ def _declare_optional(L):
 
 
 def stream_ptr() -> int:
-  return torch.cuda.current_stream().cuda_stream
+  return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device())
 
 
 def ptr(t: torch.Tensor | None):

@@ -56,6 +56,12 @@ def use_kernels(*tensors) -> bool:
   return True
 
 
+def inference_only() -> bool:
+  """Neither reverse- nor forward-mode derivatives are being recorded, so an operator may run without
+  its autograd function."""
+  return not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
+
+
 # --------------------------------------------------------------------------- helpers
 def _adjacent(ts) -> bool:
   for a, b in zip(ts[:-1], ts[1:]):
@@ -223,8 +229,58 @@ def _gemm_friendly(x, ws) -> bool:
   """Shapes the TMA-fed GEMM accepts: 16-byte aligned rows for every operand."""
   n = sum(w.shape[0] for w in ws)
   k = ws[0].shape[1]
+  if x.is_contiguous():       # (no views to look at; x.reshape(-1, k) has row pitch k)
+    return n % 8 == 0 and k % 8 == 0 and all(w.dim() == 2 and w.is_contiguous() for w in ws) and x.shape[-1] == k
   return (n % 8 == 0 and k % 8 == 0 and all(w.dim() == 2 and w.is_contiguous() for w in ws)
           and x.shape[-1] == k and x.reshape(-1, k).stride(-1) == 1 and x.reshape(-1, k).stride(0) % 8 == 0)
+
+
+def _back_to_back(ws) -> bool:
+  """Contiguous 2-D weights of one width that follow one another in one storage."""
+  w0 = ws[0]
+  if w0.dim() != 2 or not w0.is_contiguous():
+    return False
+  if len(ws) == 1:
+    return True
+  k, at, store = w0.shape[1], w0.data_ptr() + 2 * w0.numel(), w0.untyped_storage().data_ptr()
+  for w in ws[1:]:
+    if (w.dim() != 2 or w.shape[1] != k or not w.is_contiguous() or w.data_ptr() != at
+        or w.untyped_storage().data_ptr() != store):
+      return False
+    at += 2 * w.numel()
+  return True
+
+
+def _linear_now(x, ws, residual, swiglu=False):
+  """The forward of :class:`_LinearFn` (or :class:`_LinearSwigluFn`) where nothing is recorded and no
+  collective is involved, without the views and checks that recording needs.  None: not such a call."""
+  if not (_AG_CTX[0] is None and inference_only() and use_kernels(x, *ws) and x.is_contiguous() and _back_to_back(ws)):
+    return None
+  n, k = sum(w.shape[0] for w in ws), ws[0].shape[1]
+  n_out = n // 2 if swiglu else n
+  rows = x.numel() // k if k else 0
+  if x.shape[-1] != k or k % 8 or n_out % 8 or rows == 0:
+    return None
+  epi, aux = (_lib.EPI_SWIGLU if swiglu else _lib.EPI_BF16), None
+  if residual is not None:
+    if (residual.dtype != x.dtype or residual.device != x.device or not residual.is_contiguous()
+        or residual.numel() != rows * n):
+      return None
+    epi, aux = _lib.EPI_BF16_RES, residual.data_ptr()
+  y = torch.empty(*x.shape[:-1], n_out, dtype=x.dtype, device=x.device)
+  _lib.check(_lib.lib().tpb_gemm_bf16(x.data_ptr(), ws[0].data_ptr(), y.data_ptr(), rows, n, k, k, k, n_out, 0, 0, epi, 1.0,
+                                      aux, n, None, 0, 0, _lib.stream_ptr()), "gemm")
+  return y
+
+
+def _norm_now(x, w, eps):
+  """The forward of :class:`_RMSNormFn` where nothing is recorded."""
+  xc = x.contiguous()
+  d = x.shape[-1]
+  y = torch.empty_like(xc)
+  _lib.check(_lib.lib().tpb_rmsnorm_fwd(xc.data_ptr(), None, w.data_ptr(), y.data_ptr(), None, None, xc.numel() // d, d,
+                                        float(eps), _lib.stream_ptr()), "rmsnorm_fwd")
+  return y
 
 
 def _reducer_ok(reducer, x, n_out, k_in) -> bool:
@@ -241,6 +297,10 @@ def linear(x, weights, bias=None, residual=None, tp_reduce=None, tp_reduce_grad=
   reduce again), ``tp_reduce_grad`` sums the INPUT GRADIENT (column-parallel weight).  Callers ask
   ``reducer.usable(rows, n, k)`` first; a request that cannot be honoured raises."""
   ws = list(weights) if isinstance(weights, (list, tuple)) else [weights]
+  if bias is None and tp_reduce is None and tp_reduce_grad is None:
+    y = _linear_now(x, ws, residual)
+    if y is not None:
+      return y
   if (use_kernels(x, *ws) and bias is None and (len(ws) == 1 or _adjacent(ws)) and _gemm_friendly(x, ws)
       and (residual is None or residual.dtype == x.dtype)):
     n_out, k_in = sum(w.shape[0] for w in ws), ws[0].shape[1]
@@ -312,6 +372,10 @@ class _LinearSwigluFn(torch.autograd.Function):
 
 def linear_swiglu(x, w_gate, w_up, tp_reduce_grad=None):
   """silu(x @ w_gate^T) * (x @ w_up^T) as one GEMM with a fused epilogue."""
+  if tp_reduce_grad is None and w_gate.shape == w_up.shape:
+    y = _linear_now(x, [w_gate, w_up], None, swiglu=True)
+    if y is not None:
+      return y
   if (use_kernels(x, w_gate, w_up) and _adjacent([w_gate, w_up]) and w_gate.shape[0] % 8 == 0
       and _gemm_friendly(x, [w_gate, w_up])):
     if tp_reduce_grad is not None and not _reducer_ok(tp_reduce_grad, x, x.shape[-1], 2 * w_gate.shape[0]):
@@ -377,6 +441,8 @@ class _AddRMSNormFn(torch.autograd.Function):
 
 def rms_norm(x, w, eps):
   if use_kernels(x, w) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192:
+    if inference_only() and w.is_contiguous():
+      return _norm_now(x, w, eps)
     return _RMSNormFn.apply(x, w, eps)
   return ref.rms_norm(x, w, eps)
 
@@ -409,6 +475,8 @@ def rms_norm_residual(x, w, eps):
   """Returns (rmsnorm(x) * w, x).  Use the second value wherever ``x`` is needed again (the
   residual connection): its gradient is then added inside the norm's backward kernel."""
   if use_kernels(x, w) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192:
+    if inference_only() and w.is_contiguous():
+      return _norm_now(x, w, eps), x.view_as(x)
     return _RMSNormPassFn.apply(x, w, eps)
   return ref.rms_norm(x, w, eps), x
 
@@ -447,10 +515,22 @@ class _RopeInplaceFn(torch.autograd.Function):
     return d, None, None, None, None, None, None, None, None, None
 
 
+def _rope_now(x, cos_half, sin_half, heads, dim, seq_len, pos, interleaved, col0=0, head_stride=None):
+  """The forward of :class:`_RopeInplaceFn` where nothing is recorded."""
+  from . import kernels as k
+  k.rope_(x.view(-1, x.shape[-1]), col0, heads, dim, cos_half, sin_half, seq_len, pos=pos, interleaved=interleaved,
+          head_stride=head_stride)
+  if not x.is_inference():
+    torch.autograd.graph.increment_version(x)    # an earlier graph that saved x has to notice
+  return x
+
+
 def rope_slices(x, cos_half, sin_half, heads, dim, seq_len, col0, head_stride, pos=None, interleaved=False):
   """Rotate ``heads`` slices of width ``dim`` that start at column ``col0`` and lie ``head_stride``
   apart in the last dimension of ``x`` [B,S,C] (the rope part of MLA heads).  In place on CUDA."""
   if use_kernels(x):
+    if inference_only():
+      return _rope_now(x, cos_half, sin_half, heads, dim, seq_len, pos, interleaved, col0, head_stride)
     return _RopeInplaceFn.apply(x, cos_half, sin_half, heads, dim, seq_len, pos, interleaved, col0, head_stride)
   b, s, c = x.shape
   cols = (col0 + torch.arange(heads, device=x.device)[:, None] * head_stride
@@ -466,6 +546,8 @@ def rope_inplace(qkv, cos_half, sin_half, heads, dim, seq_len, pos=None, interle
   """Rotate the first ``heads`` heads of a fused ``[B, S, (heads + rest) * dim]`` projection in
   place (q and k heads; v is left alone).  cos/sin: fp32 [max_pos, dim/2]."""
   if use_kernels(qkv):
+    if inference_only():
+      return _rope_now(qkv, cos_half, sin_half, heads, dim, seq_len, pos, interleaved)
     return _RopeInplaceFn.apply(qkv, cos_half, sin_half, heads, dim, seq_len, pos, interleaved)
   b, s, _ = qkv.shape
   head = qkv[..., : heads * dim].reshape(b, s, heads, dim)
@@ -563,6 +645,9 @@ def embedding_peer(ids, table, peer):
 
 def embedding(ids, table):
   if use_kernels(table) and table.shape[1] % 8 == 0:
+    if inference_only():
+      from . import kernels as k
+      return k.embedding_fwd(table, ids.contiguous())
     return _EmbeddingFn.apply(ids, table)
   return F.embedding(ids, table)
 
