@@ -1,0 +1,421 @@
+// GEMMs with few rows (decode steps, short sequences): Y[T,N] = X[T,K] W^T, bound by streaming W once.
+//
+// The tiled kernel of gemm_sm100.cu gives a CTA 128 rows of X and 256 outputs: with 77 rows the
+// output projection of a 4096-wide layer is 16 CTAs, each pulling 2 MB of weights through one SM
+// (about 80 GB/s), while HBM would feed all 148.  Here the roles are swapped and the contraction is split:
+//   * W is the A operand: 128 output features are the 128 lanes of the accumulator, and the tokens
+//     are the N dimension of the MMA (16, 32, 64 or 128), so no MMA or shared-memory bandwidth goes into rows
+//     that do not exist beyond the next of those sizes;
+//   * a cluster of S <= 8 CTAs shares one 128-feature tile, each CTA contracting over 1/S of K.
+//     The fp32 partial tiles meet in distributed shared memory, where every CTA adds the S partials of
+//     1/S of the tokens in rank order (no workspace, no atomics, the same result every run).
+// Two CTAs fit an SM, so one's pipeline fill overlaps the other's epilogue.
+// 77 rows of a 4096-wide layer with 14336-wide MLP, us per call before / now: q|k|v 36 / 18, o 34 / 15, gate|up
+// 56 / 49, down 98 / 29 (4.0 TB/s); one row of a 102,400 x 2048 head 133 / 66 (6.3 TB/s).
+//
+//   warp 0      TMA producer: ring of {W 128x64, X NTx64} stages
+//   warp 1      MMA issuer: tcgen05.mma 128 x NT x 16
+//   warps 2..5  accumulator (TMEM) -> shared memory; then all warps reduce and write
+//
+// W may be stored [N][K] (forward) or [K][N] (input gradients, expert weights).  With the SwiGLU
+// epilogue a tile is 64 gate and the same 64 up features.  Grouped mode: rows are grouped by expert in
+// segments padded to the token-tile width, so a token tile belongs to one expert.
+
+#include "common.cuh"
+#include "tpb.h"
+
+namespace tpb {
+
+int make_tmap_2d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint64_t pitch_elems,
+                 uint32_t box_inner, uint32_t box_outer, int elem_bytes);  // tma.cu
+int make_tmap_3d(CUtensorMap* map, const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_elems,
+                 uint64_t stride2_elems, uint32_t box0, uint32_t box1);
+int sm_count();  // runtime.cu
+
+constexpr int SK_THREADS = 192;
+constexpr int SK_TN = 128;                       // output features per tile
+constexpr int SK_BK = 64;
+constexpr int SK_W_BYTES = SK_TN * SK_BK * 2;    // 16 KB
+constexpr int SK_MAX_SPLIT = 8;                  // portable cluster size
+
+template <int NT>
+struct SkinnySmem {
+  static constexpr int STAGE = SK_W_BYTES + NT * SK_BK * 2;
+  static constexpr int STAGES = NT <= 16 ? 6 : NT <= 32 ? 5 : NT <= 64 ? 4 : 3;
+  static constexpr int RING = STAGES * STAGE;
+  static constexpr int TOTAL = RING + 1024 + 256;
+  static_assert(NT * SK_TN * 4 <= RING, "the fp32 partial tile reuses the ring");
+  static_assert(2 * (TOTAL + 1024) <= 227 * 1024 + 1024, "two CTAs per SM");
+};
+
+struct SkinnyParams {
+  int T, N, K;          // N: output columns (for SwiGLU: of the activation, i.e. half the features of W)
+  void* C;
+  long long ldc;
+  const __nv_bfloat16* aux;
+  long long ldaux;
+  __nv_bfloat16* c2;    // SwiGLU: [gate | up] before the activation, or null
+  long long ldc2;
+  int up_off;           // SwiGLU: feature offset of the "up" half inside the second W map
+  float alpha;
+  int epi;
+  int t_tiles, splits, num_kb, kb_per;
+  const int* tile_expert;   // grouped: expert of every token tile (-1: unused); null: dense
+  int* status;
+};
+
+__device__ __forceinline__ float4 ld_dsmem4(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+
+// Sum of the S partials of 4 consecutive features, in rank order; all loads are in flight together.
+__device__ __forceinline__ float4 sum_partials(uint32_t local_addr, int splits) {
+  float4 v[SK_MAX_SPLIT];
+#pragma unroll
+  for (int s = 0; s < SK_MAX_SPLIT; ++s)
+    if (s < splits) v[s] = ld_dsmem4(map_to_cta(local_addr, s));
+  float4 a = v[0];
+#pragma unroll
+  for (int s = 1; s < SK_MAX_SPLIT; ++s)
+    if (s < splits) { a.x += v[s].x; a.y += v[s].y; a.z += v[s].z; a.w += v[s].w; }
+  return a;
+}
+
+// `n` (1..4) consecutive bf16 results; 8-byte store when all four exist.
+__device__ __forceinline__ void store4(__nv_bfloat16* dst, const float4& v, int n) {
+  if (n >= 4) {
+    *reinterpret_cast<uint2*>(dst) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+  } else {
+    const float f[4] = {v.x, v.y, v.z, v.w};
+    for (int j = 0; j < n; ++j) dst[j] = __float2bfloat16(f[j]);
+  }
+}
+
+template <int NT, bool W_MN>
+__global__ void __launch_bounds__(SK_THREADS, 2)
+gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
+                   const __grid_constant__ CUtensorMap tmX, const SkinnyParams p) {
+  using L = SkinnySmem<NT>;
+  constexpr int NST = L::STAGES;
+  constexpr uint32_t TMEM_COLS = NT < 32 ? 32 : NT;
+  const bool swiglu = p.epi == TPB_EPI_SWIGLU;
+  const int rank = (int)blockIdx.x % p.splits;          // == %cluster_ctarank of the 1-D cluster
+  const int unit = (int)blockIdx.x / p.splits;
+  const int bt = unit % p.t_tiles, nt = unit / p.t_tiles;   // token tiles of one W tile run together (L2)
+  const int t0 = bt * NT;
+  const int n0 = nt * (swiglu ? SK_TN / 2 : SK_TN);
+  int ez = 0;
+  if (p.tile_expert) {
+    ez = p.tile_expert[bt];
+    if (ez < 0) return;      // the whole cluster leaves together
+  }
+
+  extern __shared__ uint8_t sk_smem_raw[];
+  uint8_t* smem = sk_smem_raw + ((1024u - (smem_u32(sk_smem_raw) & 1023u)) & 1023u);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::RING);
+  uint64_t* empty = full + NST;
+  uint64_t* acc_full = empty + NST;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  float* part = reinterpret_cast<float*>(smem);         // [NT][128] after the main loop
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kb0 = rank * p.kb_per, kb1 = min(p.num_kb, kb0 + p.kb_per);
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < NST; ++s) {
+      mbar_init(&full[s], 1);
+      mbar_init(&empty[s], 1);
+    }
+    mbar_init(acc_full, 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, TMEM_COLS);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (warp == 0) {
+    if (lane == 0) {
+      tma_prefetch_desc(&tmW);
+      tma_prefetch_desc(&tmX);
+      int stage = 0;
+      uint32_t phase = 0;
+      const int nb = swiglu ? p.up_off + n0 : n0 + 64;   // second half of the 128 features
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&empty[stage], phase ^ 1, p.status, kTimeoutStageFree, 81)) break;
+        uint8_t* sW = smem + stage * L::STAGE;
+        const int k0 = kb * SK_BK;
+        mbar_expect_tx(&full[stage], L::STAGE);
+        if (!W_MN) {          // boxes {64 k, 64 features}
+          tma_load_3d(sW, &tmW, &full[stage], k0, n0, ez);
+          tma_load_3d(sW + SK_W_BYTES / 2, &tmW2, &full[stage], k0, nb, ez);
+        } else {              // boxes {64 features, 64 k}
+          tma_load_3d(sW, &tmW, &full[stage], n0, k0, ez);
+          tma_load_3d(sW + SK_W_BYTES / 2, &tmW2, &full[stage], nb, k0, ez);
+        }
+        tma_load_2d(sW + SK_W_BYTES, &tmX, &full[stage], k0, t0);
+        if (++stage == NST) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0 && kb1 > kb0) {
+      constexpr uint32_t idesc = make_idesc_bf16(SK_TN, NT, W_MN, false);
+      constexpr uint32_t desc_hi = smem_desc_hi(1024);
+      const uint32_t base = smem_u32(smem);
+      int stage = 0;
+      uint32_t phase = 0;
+      bool ok = true;
+      for (int kb = kb0; kb < kb1; ++kb) {
+        if (!mbar_wait(&full[stage], phase, p.status, kTimeoutTmaFull, 82)) { ok = false; break; }
+        tc_fence_after();
+        const uint32_t sW = base + stage * L::STAGE;
+        const uint32_t a_lo = smem_desc_lo(sW, W_MN ? 8192 : 16);
+        const uint32_t b_lo = smem_desc_lo(sW + SK_W_BYTES, 16);
+#pragma unroll
+        for (int k = 0; k < SK_BK / 16; ++k)
+          mma_ss_w(tmem_base, a_lo + (W_MN ? k * 128 : k * 2), desc_hi, b_lo + k * 2, desc_hi, idesc,
+                   ((kb - kb0) | k) != 0);
+        tc_commit(&empty[stage]);
+        if (++stage == NST) {
+          stage = 0;
+          phase ^= 1;
+        }
+      }
+      if (ok) tc_commit(acc_full);
+    }
+  } else {
+    // accumulator lane = feature, column = token: part[token][feature], conflict-free
+    const int q = warp & 3;
+    const int f = q * 32 + lane;
+    const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+    bool have = kb1 > kb0;
+    if (have) have = mbar_wait(acc_full, 0, p.status, kTimeoutAccFull, 83);
+    tc_fence_after();
+    if (kb1 <= kb0 || have) {   // (after a wait that ran out copies may still be landing in the ring)
+      constexpr int CH = NT < 32 ? 16 : 32;
+#pragma unroll 1
+      for (int c = 0; c < NT; c += CH) {
+        uint32_t v[CH];
+        if (have) {
+          if (CH == 16) tmem_ld16(t_addr + c, v); else tmem_ld32(t_addr + c, v);
+          tmem_wait_ld();
+        } else {
+#pragma unroll
+          for (int j = 0; j < CH; ++j) v[j] = 0;
+        }
+#pragma unroll
+        for (int j = 0; j < CH; ++j) part[(c + j) * SK_TN + f] = __uint_as_float(v[j]);
+      }
+    }
+    tc_fence_before();
+  }
+  __syncwarp();
+  cluster_sync_all();           // every CTA's partial tile is in its shared memory
+
+  {
+    const int per = NT / p.splits;                    // tokens this CTA finishes (splits divides 16)
+    const int gpt = swiglu ? SK_TN / 8 : SK_TN / 4;   // groups of four features per token
+    for (int i = threadIdx.x; i < per * gpt; i += SK_THREADS) {
+      const int t = rank * per + i / gpt, c = (i % gpt) * 4;
+      const int row = t0 + t, col = n0 + c;
+      if (row >= p.T || col >= p.N) continue;
+      const int n = min(4, p.N - col);
+      float4 a = sum_partials(smem_u32(part + t * SK_TN + c), p.splits);
+      a.x *= p.alpha; a.y *= p.alpha; a.z *= p.alpha; a.w *= p.alpha;
+      if (swiglu) {
+        float4 u = sum_partials(smem_u32(part + t * SK_TN + SK_TN / 2 + c), p.splits);
+        u.x *= p.alpha; u.y *= p.alpha; u.z *= p.alpha; u.w *= p.alpha;
+        if (p.c2) {
+          store4(p.c2 + (long long)row * p.ldc2 + col, a, n);
+          store4(p.c2 + (long long)row * p.ldc2 + p.N + col, u, n);
+        }
+        a.x = a.x / (1.0f + __expf(-a.x)) * u.x; a.y = a.y / (1.0f + __expf(-a.y)) * u.y;
+        a.z = a.z / (1.0f + __expf(-a.z)) * u.z; a.w = a.w / (1.0f + __expf(-a.w)) * u.w;
+      }
+      if (p.epi == TPB_EPI_F32) {
+        float* dst = reinterpret_cast<float*>(p.C) + (long long)row * p.ldc + col;
+        if (n >= 4) {
+          *reinterpret_cast<float4*>(dst) = a;
+        } else {
+          const float f[4] = {a.x, a.y, a.z, a.w};
+          for (int j = 0; j < n; ++j) dst[j] = f[j];
+        }
+        continue;
+      }
+      if (p.epi == TPB_EPI_BF16_RES) {
+        const __nv_bfloat16* r = p.aux + (long long)row * p.ldaux + col;
+        if (n >= 4) {
+          const uint2 o = *reinterpret_cast<const uint2*>(r);
+          const float2 r0 = unpack_bf16(o.x), r1 = unpack_bf16(o.y);
+          a.x += r0.x; a.y += r0.y; a.z += r1.x; a.w += r1.y;
+        } else {
+          a.x += __bfloat162float(r[0]);
+          if (n > 1) a.y += __bfloat162float(r[1]);
+          if (n > 2) a.z += __bfloat162float(r[2]);
+        }
+      }
+      store4(reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)row * p.ldc + col, a, n);
+    }
+  }
+  cluster_sync_all();           // nobody's shared memory goes away while a neighbour reads it
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, TMEM_COLS);
+  }
+}
+
+template <int NT, bool W_MN>
+static cudaError_t launch_skinny(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tx,
+                                 const SkinnyParams& p, int grid, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<NT, W_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         SkinnySmem<NT>::TOTAL);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid, 1, 1);
+  cfg.blockDim = dim3(SK_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = SkinnySmem<NT>::TOTAL;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = p.splits;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<NT, W_MN>, tw, tw2, tx, p);
+}
+
+// Token-tile width for `rows` rows: the smallest one that holds them, 128 at most.
+static int skinny_nt(int rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
+
+// K splits: double while the grid still fits the machine at two CTAs per SM and every CTA keeps four
+// k-blocks (256 of K) to amortise its pipeline fill.
+static int skinny_splits(long long tiles, int num_kb) {
+  int s = 1;
+  while (s < SK_MAX_SPLIT && tiles * s * 2 <= 2LL * sm_count() && num_kb / (2 * s) >= 4) s *= 2;
+  return s;
+}
+
+// Whether this kernel is the faster one for a dense product of M rows: always up to 128 rows (one token
+// tile; even a 102,400-wide head takes 98 us instead of 108 with 128 rows and 66 instead of 133 with one),
+// and beyond that while the tiled kernel's 128 x 256 tiles leave half of the SMs idle.  The time per call in
+// us with weights from HBM, tiled kernel / this one, by the number of its tiles (N x K):
+//   4096 x 4096:   384 rows, 48 tiles 34 / 23    512 rows, 64 tiles 35 / 24    768 rows, 96 tiles 35 / 36
+//   4096 x 14336:  512 rows, 64 tiles 98 / 62    768 rows, 96 tiles 98 / 97
+//   2048 x 10944: 1024 rows, 64 tiles 77 / 47    3072 x 2048: 768 rows, 72 tiles 22 / 16, 1024 rows, 96 tiles 23 / 23
+//   14336 x 4096:  128 rows, 56 tiles 39 / 28    192 rows, 112 tiles 39 / 40
+bool skinny_wins(int M, int N, bool swiglu) {
+  if (M <= 128) return true;
+  const long long tiles = (long long)((M + 127) / 128) * (((swiglu ? N / 2 : N) + (swiglu ? 127 : 255)) / (swiglu ? 128 : 256));
+  return tiles <= sm_count() / 2;
+}
+
+// x [T,K] (for grouped mode: all padded rows), w dense [N,K] (w_mn = 0) or [K,N] (w_mn = 1), with
+// `experts` of them `w_stride` elements apart.  N counts both halves for SwiGLU.  nt / splits 0: by
+// the rules above.  Returns -2 when the shape or alignment is not supported.
+int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, int experts,
+                long long ldx, long long ldw, long long w_stride, long long ldc, int w_mn, int epi, float alpha,
+                const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit,
+                int nt, int splits, cudaStream_t stream) {
+  if (T <= 0 || N <= 0 || K <= 0) return 0;
+  const bool swiglu = epi == TPB_EPI_SWIGLU;
+  if (!swiglu && epi != TPB_EPI_BF16 && epi != TPB_EPI_BF16_RES && epi != TPB_EPI_F32) return -2;
+  auto misaligned = [](const void* q) { return (reinterpret_cast<uintptr_t>(q) % 16) != 0; };
+  if ((ldx % 8) || (ldw % 8) || (w_stride % 8) || (ldc % (epi == TPB_EPI_F32 ? 4 : 8)) || misaligned(x) ||
+      misaligned(w) || (w2 && misaligned(w2)) || misaligned(c))
+    return -2;
+  if (swiglu && ((N % 2) || ((N / 2) % 8) || (c2 && ((ldc2 % 4) || (reinterpret_cast<uintptr_t>(c2) % 8))))) return -2;
+  if (epi == TPB_EPI_BF16_RES && (!aux || (ldaux % 4) || (reinterpret_cast<uintptr_t>(aux) % 8))) return -2;
+  if (tile_expert && (nt == 0 || T % nt)) return -2;
+  const bool two_w = swiglu && w2 != nullptr && w2 != w;
+  const int extent = two_w ? N / 2 : N;
+  const int tile_n = swiglu ? SK_TN / 2 : SK_TN;
+  const int n_out = swiglu ? N / 2 : N;
+  if (nt == 0) nt = skinny_nt(T);
+  if (nt != 16 && nt != 32 && nt != 64 && nt != 128) return -2;
+  SkinnyParams p;
+  p.T = T; p.N = n_out; p.K = K;
+  p.C = c; p.ldc = ldc;
+  p.aux = reinterpret_cast<const __nv_bfloat16*>(aux); p.ldaux = ldaux;
+  p.c2 = reinterpret_cast<__nv_bfloat16*>(c2); p.ldc2 = ldc2;
+  p.up_off = two_w ? 0 : N / 2;
+  p.alpha = alpha; p.epi = epi;
+  p.t_tiles = (T + nt - 1) / nt;
+  p.num_kb = (K + SK_BK - 1) / SK_BK;
+  p.tile_expert = tile_expert;
+  p.status = status_block();
+  const long long n_tiles = (n_out + tile_n - 1) / tile_n;
+  const long long tiles = n_tiles * p.t_tiles;
+  // grouped: about one token tile runs per expert that is hit
+  if (splits == 0) splits = skinny_splits(tile_expert ? n_tiles * experts_hit : tiles, p.num_kb);
+  if (splits != 1 && splits != 2 && splits != 4 && splits != 8) return -2;
+  p.splits = splits;
+  p.kb_per = (p.num_kb + splits - 1) / splits;
+  if (tiles * splits > 0x7fffffffLL) return -2;
+  CUtensorMap tw, tw2, tx;
+  const uint64_t stride = experts > 1 ? (uint64_t)w_stride : (uint64_t)ldw * (w_mn ? K : extent);
+  auto make_w = [&](CUtensorMap* m, const void* ptr) {
+    return !w_mn ? make_tmap_3d(m, ptr, K, extent, experts, ldw, stride, 64, 64)
+                 : make_tmap_3d(m, ptr, extent, K, experts, ldw, stride, 64, 64);
+  };
+  if (make_tmap_2d(&tx, x, K, T, ldx, 64, nt, 2)) return -3;
+  if (make_w(&tw, w)) return -4;
+  if (two_w) {
+    if (make_w(&tw2, w2)) return -5;
+  } else {
+    tw2 = tw;
+  }
+  const int grid = (int)(tiles * splits);
+  cudaError_t e;
+#define TPB_SK(NT_) (w_mn ? launch_skinny<NT_, true>(tw, tw2, tx, p, grid, stream) \
+                          : launch_skinny<NT_, false>(tw, tw2, tx, p, grid, stream))
+  switch (nt) {
+    case 16: e = TPB_SK(16); break;
+    case 32: e = TPB_SK(32); break;
+    case 64: e = TPB_SK(64); break;
+    case 128: e = TPB_SK(128); break;
+    default: return -2;
+  }
+#undef TPB_SK
+  return e == cudaSuccess ? 0 : 1000 + (int)e;
+}
+
+}  // namespace tpb
+
+using namespace tpb;
+
+// The kernel with an explicit token-tile width and K split (0: by rule); see tpb_gemm_bf16 for the rest.
+extern "C" int tpb_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, int T, int N, int K,
+                                    long long ldx, long long ldw, long long ldc, int w_mn, int epi, float alpha,
+                                    const void* aux, long long ldaux, void* c2, long long ldc2, int nt, int splits,
+                                    void* stream) {
+  return skinny_gemm(x, w, w2, c, T, N, K, 1, ldx, ldw, 0, ldc, w_mn, epi, alpha, aux, ldaux, c2, ldc2, nullptr, 0, nt,
+                     splits, reinterpret_cast<cudaStream_t>(stream));
+}
+
+// Rows grouped by expert in segments padded to `nt` rows; tile_expert[rows / nt].  Token tiles of expert -1
+// are not written.  experts_hit: how many experts have rows, at most.
+extern "C" int tpb_grouped_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, int rows, int N,
+                                            int K, int E, long long ldx, long long ldw, long long w_stride,
+                                            long long ldc, int w_mn, int epi, const int* tile_expert, int experts_hit,
+                                            int nt, void* stream) {
+  if (!tile_expert || E < 1 || experts_hit < 1) return -2;
+  return skinny_gemm(x, w, w2, c, rows, N, K, E, ldx, ldw, w_stride, ldc, w_mn, epi, 1.0f, nullptr, 0, nullptr, 0,
+                     tile_expert, experts_hit, nt, 0, reinterpret_cast<cudaStream_t>(stream));
+}

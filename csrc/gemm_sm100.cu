@@ -770,6 +770,19 @@ cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const
 
 
 
+// gemm_skinny_sm100.cu
+int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, int experts,
+                long long ldx, long long ldw, long long w_stride, long long ldc, int w_mn, int epi, float alpha,
+                const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit, int nt,
+                int splits, cudaStream_t stream);
+bool skinny_wins(int M, int N, bool swiglu);
+
+// TPB_GEMM_PAIR: 0 = never CTA pairs, 2 = pairs for every dense shape (tests), default = by shape
+static int gemm_pair_mode() {
+  static const int mode = []() { const char* v = getenv("TPB_GEMM_PAIR"); return v ? atoi(v) : 1; }();
+  return mode;
+}
+
 struct GemmCall {
   const void* A; const void* B; const void* B2; void* C;
   int M, N, K, E;
@@ -877,10 +890,8 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   if (rs_rotate)
     p.tile_rot = (int)(tiles * g.rs_rank / g.rs_world);   // every rank starts in a different owner's part of C
   cudaError_t e;
-  // CTA pairs for dense GEMMs with enough 256 x 256 tiles to fill the machine (TPB_GEMM_PAIR=0
-  // keeps the single-CTA kernel)
-  // TPB_GEMM_PAIR: 0 = never, 2 = for every dense shape (tests), default = when the tiles fill the machine
-  static const int pair_mode = []() { const char* v = getenv("TPB_GEMM_PAIR"); return v ? atoi(v) : 1; }();
+  // CTA pairs for dense GEMMs with enough 256 x 256 tiles to fill the machine
+  const int pair_mode = gemm_pair_mode();
   static const int max_pairs = []() {
     // clusters of two that can be resident at once (an SM without a free partner stays idle)
     cudaLaunchConfig_t cfg = {};
@@ -932,6 +943,12 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
                              long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha,
                              const void* aux, long long ldaux, void* c2, long long ldc2, int max_ctas,
                              void* stream_) {
+  // few rows: the kernel that streams B once and splits the contraction
+  if (!a_mn && max_ctas == 0 && gemm_pair_mode() == 1 && skinny_wins(M, N, epi == TPB_EPI_SWIGLU)) {
+    const int r = skinny_gemm(A, B, nullptr, C, M, N, K, 1, lda, ldb, 0, ldc, b_mn, epi, alpha, aux, ldaux, c2, ldc2,
+                              nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_));
+    if (r != -2) return r;     // -2: an epilogue or alignment it does not take
+  }
   GemmCall g{};
   g.A = A; g.B = B; g.B2 = nullptr; g.C = C;
   g.M = M; g.N = N; g.K = K; g.E = 1;

@@ -1,0 +1,118 @@
+"""GEMMs with few rows (csrc/gemm_skinny_sm100.cu)."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from torchprime_b200.ops import kernels as k
+from torchprime_b200.ops._lib import lib, ptr, stream_ptr
+
+BF16_EPS = 2.0 ** -8
+
+
+def _skinny(x, w, *, b_mn=False, epi=k.EPI_BF16, alpha=1.0, aux=None, w2=None, c2=None, nt=0, splits=0, out=None):
+  t, kk = x.shape
+  n = w.shape[1] if b_mn else w.shape[0]
+  n *= 2 if w2 is not None else 1
+  n_out = n // 2 if epi == k.EPI_SWIGLU else n
+  if out is None:
+    out = torch.empty(t, n_out, device="cuda", dtype=torch.float32 if epi == k.EPI_F32 else torch.bfloat16)
+  rc = lib().tpb_gemm_skinny_bf16(ptr(x), ptr(w), ptr(w2), ptr(out), t, n, kk, x.stride(0), w.stride(0), out.stride(0),
+                                  int(b_mn), epi, alpha, ptr(aux), aux.stride(0) if aux is not None else 0, ptr(c2),
+                                  c2.stride(0) if c2 is not None else 0, nt, splits, stream_ptr())
+  assert rc == 0, rc
+  return out
+
+
+@pytest.fixture(autouse=True)
+def _signature():
+  from ctypes import c_float as F, c_int as I, c_longlong as LL, c_void_p as P
+  fn = lib().tpb_gemm_skinny_bf16
+  fn.argtypes, fn.restype = [P, P, P, P, I, I, I, LL, LL, LL, I, I, F, P, LL, P, LL, I, I, P], I
+
+
+def _close(got, want, scale):
+  """One rounding to the result's type plus fp32 sums in another order (``scale``: size of the terms' sum)."""
+  err = (got.float() - want).abs()
+  eps = BF16_EPS if got.dtype == torch.bfloat16 else 0.0
+  assert bool((err <= eps * want.abs() + 2e-6 * scale).all()), (err - eps * want.abs()).max()
+
+
+@pytest.mark.parametrize("t,nt", [(1, 0), (15, 0), (16, 16), (17, 0), (33, 32), (64, 0), (77, 0), (128, 0), (129, 128), (50, 16)])
+@pytest.mark.parametrize("n,kk,splits", [(8, 64, 1), (128, 72, 0), (136, 520, 2), (1000, 2048, 0), (264, 1096, 8), (384, 256, 4)])
+def test_dense_layouts_and_epilogues(cuda_lib, t, nt, n, kk, splits):
+  torch.manual_seed(t * 1000 + n)
+  x = torch.randn(t, kk + 16, device="cuda", dtype=torch.bfloat16)[:, 8:kk + 8]       # rows with a pitch
+  w = torch.randn(n, kk, device="cuda", dtype=torch.bfloat16)
+  res = torch.randn(t, n + 8, device="cuda", dtype=torch.bfloat16)[:, :n]
+  want = x.double() @ w.double().t()
+  scale = float(kk)
+  # results land in the middle of a larger buffer whose border must stay as it is
+  for b_mn in (False, True):
+    ww = w.t().contiguous() if b_mn else w
+    for epi, aux, ref_ in ((k.EPI_BF16, None, want), (k.EPI_F32, None, want), (k.EPI_BF16_RES, res, want + res.double())):
+      big = torch.full((t + 2, n + 16), 7.0, device="cuda", dtype=torch.float32 if epi == k.EPI_F32 else torch.bfloat16)
+      out = big[1:t + 1, 8:n + 8]
+      _skinny(x, ww, b_mn=b_mn, epi=epi, aux=aux, nt=nt, splits=splits, out=out)
+      _close(out, ref_, scale)
+      out.fill_(7.0)
+      assert bool((big == 7.0).all())
+
+
+@pytest.mark.parametrize("t", [1, 16, 40, 128])
+@pytest.mark.parametrize("f,kk,splits", [(8, 64, 1), (72, 136, 2), (192, 1024, 8), (1408, 512, 0)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_dense_swiglu(cuda_lib, t, f, kk, splits, b_mn):
+  torch.manual_seed(f)
+  x = torch.randn(t, kk, device="cuda", dtype=torch.bfloat16)
+  g, u = (torch.randn(f, kk, device="cuda", dtype=torch.bfloat16) / kk ** 0.5 for _ in range(2))
+  gate, up = x.double() @ g.double().t(), x.double() @ u.double().t()
+  want = torch.nn.functional.silu(gate) * up
+  both = torch.cat([g, u])
+  lay = (lambda m: m.t().contiguous()) if b_mn else (lambda m: m)
+  for w, w2 in ((lay(both), None), (lay(g), lay(u))):
+    gu = torch.empty(t, 2 * f, device="cuda", dtype=torch.bfloat16)
+    act = _skinny(x, w, b_mn=b_mn, epi=k.EPI_SWIGLU, w2=w2, c2=gu, splits=splits)
+    _close(gu, torch.cat([gate, up], -1), 8.0)
+    # silu amplifies an error of the gate by at most 1.1
+    err = (act.double() - want).abs()
+    assert bool((err <= BF16_EPS * want.abs() + 1e-5 * (1 + up.abs())).all()), err.max()
+
+
+def test_split_sums_do_not_depend_on_the_run(cuda_lib):
+  x = torch.randn(40, 4096, device="cuda", dtype=torch.bfloat16)
+  w = torch.randn(512, 4096, device="cuda", dtype=torch.bfloat16)
+  a = _skinny(x, w, epi=k.EPI_F32, splits=8)
+  for _ in range(3):
+    assert torch.equal(a, _skinny(x, w, epi=k.EPI_F32, splits=8))
+
+
+def test_linear_f32_logits(cuda_lib):
+  from torchprime_b200.ops import functional as ops
+  x = torch.randn(3, 256, device="cuda", dtype=torch.bfloat16)
+  w = torch.randn(1000, 256, device="cuda", dtype=torch.bfloat16)
+  with torch.no_grad():
+    got = ops.linear_f32(x, w)
+  assert got.dtype == torch.float32
+  _close(got, x.double() @ w.double().t(), 256.0)
+  w.requires_grad_(True)
+  assert ops.linear_f32(x, w).requires_grad
+
+@pytest.mark.parametrize("M,N,K", [(1, 64, 128), (77, 512, 256), (128, 1000, 136), (300, 512, 512), (700, 64, 2048)])
+def test_route_of_a_gemm_call(cuda_lib, M, N, K):
+  """Calls the rule gives to this kernel against the tiled kernel (max_ctas keeps a call there)."""
+  torch.manual_seed(M)
+  x = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+  w = torch.randn(N, K, device="cuda", dtype=torch.bfloat16) / K ** 0.5
+  res = torch.randn(M, N, device="cuda", dtype=torch.bfloat16)
+  for b_mn in (False, True):
+    ww = w.t().contiguous() if b_mn else w
+    for epi, aux in ((k.EPI_BF16, None), (k.EPI_F32, None), (k.EPI_BF16_RES, res), (k.EPI_SWIGLU, None)):
+      if epi == k.EPI_SWIGLU and (N // 2) % 8:
+        continue
+      a = k.gemm(x, ww, b_mn=b_mn, epi=epi, aux=aux, alpha=0.5)
+      b = k.gemm(x, ww, b_mn=b_mn, epi=epi, aux=aux, alpha=0.5, max_ctas=148)
+      # two fp32 sums of K random terms in other orders: each strays by about 2^-24 sqrt(K / 2) of the result
+      bound = 2.0 ** -23 * K ** 0.5
+      assert ((a.float() - b.float()).norm() / b.float().norm()).item() < (bound if epi == k.EPI_F32 else 2.0 ** -9)

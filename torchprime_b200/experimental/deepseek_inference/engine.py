@@ -118,7 +118,7 @@ class DeepseekInferenceEngine:
       h = h + a
       h = layer.mlp(layer.post_attention_layernorm(h), residual=h)
     last = m.norm(h[:, -1:, :].contiguous())
-    return torch.nn.functional.linear(last[:, 0].float(), self.model.lm_head.weight.float())
+    return ops.linear_f32(last[:, 0], self.model.lm_head.weight)
 
   __call__ = forward
 

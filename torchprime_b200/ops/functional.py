@@ -326,6 +326,34 @@ def linear(x, weights, bias=None, residual=None, tp_reduce=None, tp_reduce_grad=
   return y if residual is None else y + residual
 
 
+class _LinearF32Fn(torch.autograd.Function):
+  @staticmethod
+  def forward(ctx, x, w):
+    from . import kernels as k
+    ctx.save_for_backward(x, w)
+    return k.gemm(x, w, epi=k.EPI_F32)
+
+  @staticmethod
+  def backward(ctx, dy):
+    x, w = ctx.saved_tensors
+    dx = (dy @ w.float()).to(x.dtype) if ctx.needs_input_grad[0] else None
+    dw = (dy.t() @ x.float()).to(w.dtype) if ctx.needs_input_grad[1] else None
+    return dx, dw
+
+
+def linear_f32(x, w):
+  """x @ w^T of a [T, K] input in fp32 (fp32 products, sums and result): router and inference logits.
+  bf16 operands go into the GEMM as they are (their products are exact in fp32) instead of through fp32
+  copies."""
+  _settle(w)
+  if x.dim() == 2 and use_kernels(x, w) and x.shape[0] > 0 and _gemm_friendly(x, [w]):
+    if inference_only():
+      from . import kernels as k
+      return k.gemm(x, w, epi=k.EPI_F32)
+    return _LinearF32Fn.apply(x, w)
+  return F.linear(x.float(), w.float())
+
+
 class _LinearSwigluFn(torch.autograd.Function):
   @staticmethod
   def forward(ctx, x, w_gate, w_up, grad_reduce=None):
