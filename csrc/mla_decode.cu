@@ -1,0 +1,404 @@
+// One decode step of latent attention over a compressed cache (one new token per sequence).
+//
+// The cache holds, per token, the normalised latent (C values) and the shared rotary key (R values), both
+// bf16.  The key up-projection is folded into the query and the value up-projection is applied to the
+// weighted sum, so a step has to read C + R numbers per cached token and the up-projection weights once.
+// All arithmetic is fp32 on bf16 inputs (queries folded through the up-projection stay fp32): the work is a few FMAs
+// per byte, far below the FP32 pipe's share, and what bounds the step is latency and launches.
+// Written as torch operators the same step converts the whole cache and the up-projection to fp32 and
+// runs about thirty kernels per layer.  Four sequences of 1500 cached tokens, 16 heads, C = 512, us per layer: prep 4,
+// fold 4, split 22, merge 9; the torch form about 150 and the host's time for it.
+//
+//   mla_prep_kernel     per sequence: rotate the queries' rotary part, normalise the new latent and rotate
+//                       the new rotary key straight into the cache
+//   mla_fold_kernel     qa[b,h,:] = sum_d q[b,h,d] Wk[h,d,:]               (reads Wk once)
+//   mla_split_kernel    per (sequence, 16 heads, range of keys): scores, running softmax, weighted latent sum
+//   mla_merge_kernel    per (sequence, head): merge the ranges, out[j] = sum_c olat[c] Wv[h,j,c]
+
+#include "common.cuh"
+#include "tpb.h"
+
+namespace tpb {
+
+int sm_count();
+
+constexpr int MLA_MAX_C = 512;      // latent width: two columns per thread of 256
+constexpr int MLA_R = 64;           // rotary width
+constexpr int MLA_HG = 16;          // heads per CTA of the split kernel
+constexpr int MLA_KEYS = 32;        // keys per step of the split kernel: one per lane
+constexpr int MLA_THREADS = 256;
+constexpr int MLA_MAX_B = 8;        // sequences per CTA of the fold kernel
+
+__device__ __forceinline__ float mla_rbf(float v) { return __bfloat162float(__float2bfloat16(v)); }
+
+// Rotation of pair i of a rotary slice; interleaved pairs (2i, 2i+1) stay where they are.
+__device__ __forceinline__ void mla_rotate(const __nv_bfloat16* x, __nv_bfloat16* y, int i, int interleaved, float cs,
+                                           float sn) {
+  const int ia = interleaved ? 2 * i : i, ib = interleaved ? 2 * i + 1 : i + MLA_R / 2;
+  const float a = __bfloat162float(x[ia]), b = __bfloat162float(x[ib]);
+  y[ia] = __float2bfloat16(a * cs - b * sn);
+  y[ib] = __float2bfloat16(b * cs + a * sn);
+}
+
+// One CTA per sequence.  q [B, H * (dn + R)] is rotated in place; ckv [B, C + R] goes to row `pos` of
+// the caches [B, S, C] and [B, S, R].
+__global__ void __launch_bounds__(MLA_THREADS)
+mla_prep_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ ckv,
+                const __nv_bfloat16* __restrict__ norm_w, const float* __restrict__ cosT,
+                const float* __restrict__ sinT, __nv_bfloat16* __restrict__ kv_cache,
+                __nv_bfloat16* __restrict__ pe_cache, long long kv_bs, long long pe_bs, int pos, int H, int dn, int C,
+                float eps, int interleaved) {
+  __shared__ float red[8];
+  const int b = blockIdx.x;
+  const float* cs = cosT + (size_t)pos * (MLA_R / 2);
+  const float* sn = sinT + (size_t)pos * (MLA_R / 2);
+  for (int i = threadIdx.x; i < H * (MLA_R / 2); i += MLA_THREADS) {
+    const int h = i / (MLA_R / 2), j = i % (MLA_R / 2);
+    __nv_bfloat16* x = q + ((size_t)b * H + h) * (dn + MLA_R) + dn;
+    mla_rotate(x, x, j, interleaved, cs[j], sn[j]);
+  }
+  const __nv_bfloat16* row = ckv + (size_t)b * (C + MLA_R);
+  if (threadIdx.x < MLA_R / 2)
+    mla_rotate(row + C, pe_cache + b * pe_bs + (size_t)pos * MLA_R, threadIdx.x, interleaved, cs[threadIdx.x],
+               sn[threadIdx.x]);
+  float ss = 0.f;
+  for (int i = threadIdx.x; i < C; i += MLA_THREADS) {
+    const float v = __bfloat162float(row[i]);
+    ss += v * v;
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  ss = 0.f;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) ss += red[w];
+  const float rstd = rsqrtf(ss / (float)C + eps);
+  // the same two roundings as the norm kernel of the other paths
+  for (int i = threadIdx.x; i < C; i += MLA_THREADS)
+    kv_cache[b * kv_bs + (size_t)pos * C + i] =
+        __float2bfloat16(__bfloat162float(norm_w[i]) * mla_rbf(__bfloat162float(row[i]) * rstd));
+}
+
+// Grid (H, C / 64, ceil(B / 8)).  A thread holds 8 columns of every 32nd d: its 16-byte loads of the weight
+// (four for dn = 128) are all in flight at once; the 32 slices meet by shuffles and in shared memory.  (With
+// 4-byte loads, sixteen per thread one after the other, 10 us instead of 5 at B = 4, H = 16.)
+__global__ void __launch_bounds__(MLA_THREADS)
+mla_fold_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ w, float* __restrict__ qa, int B,
+                int H, int dn, int dv, int C) {
+  __shared__ float acc_s[8][MLA_MAX_B][64];
+  extern __shared__ float fold_q[];                  // [MLA_MAX_B][dn]
+  const int h = blockIdx.x, c0 = blockIdx.y * 64, b0 = blockIdx.z * MLA_MAX_B;
+  const int nb = min(MLA_MAX_B, B - b0);
+  const int vec = threadIdx.x & 7, slice = threadIdx.x >> 3;
+  const uint4* wr = reinterpret_cast<const uint4*>(w + (size_t)h * (dn + dv) * C + c0) + vec;
+  uint4 wv[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (slice + 32 * i < dn) wv[i] = wr[(size_t)(slice + 32 * i) * (C / 8)];
+  for (int i = threadIdx.x; i < MLA_MAX_B * dn; i += MLA_THREADS) {
+    const int b = i / dn, d = i % dn;
+    fold_q[i] = b < nb ? __bfloat162float(q[((size_t)(b0 + b) * H + h) * (dn + MLA_R) + d]) : 0.f;
+  }
+  __syncthreads();
+  float a[MLA_MAX_B][8] = {};
+  auto add = [&](const uint4& u, int d) {
+    const float2 p0 = unpack_bf16(u.x), p1 = unpack_bf16(u.y), p2 = unpack_bf16(u.z), p3 = unpack_bf16(u.w);
+#pragma unroll
+    for (int b = 0; b < MLA_MAX_B; ++b) {
+      if (b >= nb) break;
+      const float x = fold_q[b * dn + d];
+      a[b][0] += x * p0.x; a[b][1] += x * p0.y; a[b][2] += x * p1.x; a[b][3] += x * p1.y;
+      a[b][4] += x * p2.x; a[b][5] += x * p2.y; a[b][6] += x * p3.x; a[b][7] += x * p3.y;
+    }
+  };
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    if (slice + 32 * i < dn) add(wv[i], slice + 32 * i);
+  for (int d = slice + 128; d < dn; d += 32) add(wr[(size_t)d * (C / 8)], d);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+  for (int b = 0; b < MLA_MAX_B; ++b) {
+    if (b >= nb) break;
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+      float v = a[b][e];
+      v += __shfl_xor_sync(0xffffffffu, v, 8);
+      v += __shfl_xor_sync(0xffffffffu, v, 16);
+      if (lane < 8) acc_s[warp][b][vec * 8 + e] = v;
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < nb * 64; i += MLA_THREADS) {
+    const int b = i / 64, c = i % 64;
+    float s = 0.f;
+#pragma unroll
+    for (int k = 0; k < 8; ++k) s += acc_s[k][b][c];
+    qa[((size_t)(b0 + b) * H + h) * C + c0 + c] = s;
+  }
+}
+
+struct MlaSplitSmem {
+  // rows of keys are padded by 16 bytes: lanes read 16 bytes of 32 different rows without bank conflicts
+  static __host__ __device__ int key_pitch(int C) { return (C + MLA_R) * 2 + 16; }
+  static __host__ __device__ int bytes(int C) {
+    return MLA_HG * (C + MLA_R) * 4 + MLA_KEYS * key_pitch(C) + MLA_KEYS * MLA_HG * 4 + 2 * MLA_HG * 4;
+  }
+};
+
+// Grid (ranges, head groups, B).  Keys [range * per, min(n_keys, (range + 1) * per)), per a multiple of 32.
+// part_o [B, H, ranges, C], part_ml [B, H, ranges, 2] = (running maximum in log2 units, sum).
+__global__ void __launch_bounds__(MLA_THREADS)
+mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__ q,
+                 const __nv_bfloat16* __restrict__ kv_cache, const __nv_bfloat16* __restrict__ pe_cache,
+                 long long kv_bs, long long pe_bs, float* __restrict__ part_o, float* __restrict__ part_ml, int n_keys,
+                 int per, int H, int dn, int C, float scale_log2) {
+  extern __shared__ uint8_t split_smem[];
+  const int D = C + MLA_R, pitch = MlaSplitSmem::key_pitch(C);
+  float* sq = reinterpret_cast<float*>(split_smem);                 // [16][D]
+  uint8_t* sk = split_smem + MLA_HG * D * 4;                        // [32][pitch]
+  float* sp = reinterpret_cast<float*>(sk + MLA_KEYS * pitch);      // [32 keys][16 heads]
+  float* s_alpha = sp + MLA_KEYS * MLA_HG;                          // [16]
+  const int range = blockIdx.x, h0 = blockIdx.y * MLA_HG, b = blockIdx.z, ranges = gridDim.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  // the folded queries, then the rotary parts, four values per load and nothing waiting for anything
+  // (a scalar loop over both took 20 of the kernel's 31 us)
+#pragma unroll 8
+  for (int i = threadIdx.x; i < MLA_HG * (C / 4); i += MLA_THREADS) {
+    const int h = i / (C / 4), d = (i % (C / 4)) * 4;
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (h0 + h < H) v = *reinterpret_cast<const float4*>(qa + ((size_t)b * H + h0 + h) * C + d);
+    *reinterpret_cast<float4*>(sq + h * D + d) = v;
+  }
+  {
+    const int h = threadIdx.x / (MLA_R / 4), d = (threadIdx.x % (MLA_R / 4)) * 4;   // 16 heads x 16 groups of four
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (h0 + h < H) {
+      const uint2 u = *reinterpret_cast<const uint2*>(q + ((size_t)b * H + h0 + h) * (dn + MLA_R) + dn + d);
+      const float2 lo = unpack_bf16(u.x), hi = unpack_bf16(u.y);
+      v = make_float4(lo.x, lo.y, hi.x, hi.y);
+    }
+    *reinterpret_cast<float4*>(sq + h * D + C + d) = v;
+  }
+  const int k_begin = range * per, k_end = min(n_keys, k_begin + per);
+  const int hw = warp * 2;                       // this warp's two heads in the score phase
+  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  const bool owner = 2 * (int)threadIdx.x < C;   // this thread's two latent columns in the sum phase
+  float acc[MLA_HG][2] = {};
+  const int cv = C / 8, dvec = D / 8;
+  for (int k0 = k_begin; k0 < k_end; k0 += MLA_KEYS) {
+    if (k0 != k_begin) __syncthreads();          // the previous step's keys and weights are used up
+#pragma unroll 9
+    for (int i = threadIdx.x; i < MLA_KEYS * dvec; i += MLA_THREADS) {
+      const int r = i / dvec, c = i % dvec, key = k0 + r;
+      uint4 v = make_uint4(0, 0, 0, 0);
+      if (key < k_end)
+        v = c < cv ? reinterpret_cast<const uint4*>(kv_cache + b * kv_bs + (size_t)key * C)[c]
+                   : reinterpret_cast<const uint4*>(pe_cache + b * pe_bs + (size_t)key * MLA_R)[c - cv];
+      *reinterpret_cast<uint4*>(sk + r * pitch + c * 16) = v;
+    }
+    __syncthreads();
+    float s0 = 0.f, s1 = 0.f;
+    const float* q0 = sq + hw * D;
+    const float* q1 = q0 + D;
+#pragma unroll 4
+    for (int c = 0; c < dvec; ++c) {
+      const uint4 kv = *reinterpret_cast<const uint4*>(sk + lane * pitch + c * 16);
+      const float2 a = unpack_bf16(kv.x), bb = unpack_bf16(kv.y), cc = unpack_bf16(kv.z), d = unpack_bf16(kv.w);
+      const float4 x0 = *reinterpret_cast<const float4*>(q0 + c * 8), x1 = *reinterpret_cast<const float4*>(q0 + c * 8 + 4);
+      const float4 y0 = *reinterpret_cast<const float4*>(q1 + c * 8), y1 = *reinterpret_cast<const float4*>(q1 + c * 8 + 4);
+      s0 += x0.x * a.x + x0.y * a.y + x0.z * bb.x + x0.w * bb.y + x1.x * cc.x + x1.y * cc.y + x1.z * d.x + x1.w * d.y;
+      s1 += y0.x * a.x + y0.y * a.y + y0.z * bb.x + y0.w * bb.y + y1.x * cc.x + y1.y * cc.y + y1.z * d.x + y1.w * d.y;
+    }
+    const bool live = k0 + lane < k_end;
+    s0 = live ? s0 * scale_log2 : -INFINITY;
+    s1 = live ? s1 * scale_log2 : -INFINITY;
+    float n0 = s0, n1 = s1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      n0 = fmaxf(n0, __shfl_xor_sync(0xffffffffu, n0, o));
+      n1 = fmaxf(n1, __shfl_xor_sync(0xffffffffu, n1, o));
+    }
+    n0 = fmaxf(m0, n0);                          // finite: the step has at least one key
+    n1 = fmaxf(m1, n1);
+    const float p0 = exp2f(s0 - n0), p1 = exp2f(s1 - n1);
+    const float al0 = exp2f(m0 - n0), al1 = exp2f(m1 - n1);
+    float t0 = p0, t1 = p1;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      t0 += __shfl_xor_sync(0xffffffffu, t0, o);
+      t1 += __shfl_xor_sync(0xffffffffu, t1, o);
+    }
+    l0 = l0 * al0 + t0; l1 = l1 * al1 + t1;
+    m0 = n0; m1 = n1;
+    sp[lane * MLA_HG + hw] = p0;
+    sp[lane * MLA_HG + hw + 1] = p1;
+    if (lane == 0) { s_alpha[hw] = al0; s_alpha[hw + 1] = al1; }
+    __syncthreads();
+    if (owner) {
+#pragma unroll
+      for (int h = 0; h < MLA_HG; ++h) { acc[h][0] *= s_alpha[h]; acc[h][1] *= s_alpha[h]; }
+      const uint8_t* col = sk + threadIdx.x * 4;
+#pragma unroll 4
+      for (int r = 0; r < MLA_KEYS; ++r) {
+        const float2 v = unpack_bf16(*reinterpret_cast<const uint32_t*>(col + r * pitch));
+        const float4* pr = reinterpret_cast<const float4*>(sp + r * MLA_HG);
+#pragma unroll
+        for (int h4 = 0; h4 < MLA_HG / 4; ++h4) {
+          const float4 w4 = pr[h4];
+          acc[4 * h4][0] += w4.x * v.x; acc[4 * h4][1] += w4.x * v.y;
+          acc[4 * h4 + 1][0] += w4.y * v.x; acc[4 * h4 + 1][1] += w4.y * v.y;
+          acc[4 * h4 + 2][0] += w4.z * v.x; acc[4 * h4 + 2][1] += w4.z * v.y;
+          acc[4 * h4 + 3][0] += w4.w * v.x; acc[4 * h4 + 3][1] += w4.w * v.y;
+        }
+      }
+    }
+  }
+  if (owner) {
+#pragma unroll
+    for (int h = 0; h < MLA_HG; ++h)
+      if (h0 + h < H)
+        *reinterpret_cast<float2*>(part_o + (((size_t)b * H + h0 + h) * ranges + range) * C + 2 * threadIdx.x) =
+            make_float2(acc[h][0], acc[h][1]);
+  }
+  if (lane == 0) {
+    if (h0 + hw < H) {
+      float* ml = part_ml + (((size_t)b * H + h0 + hw) * ranges + range) * 2;
+      ml[0] = m0; ml[1] = l0;
+    }
+    if (h0 + hw + 1 < H) {
+      float* ml = part_ml + (((size_t)b * H + h0 + hw + 1) * ranges + range) * 2;
+      ml[0] = m1; ml[1] = l1;
+    }
+  }
+}
+
+// Grid (H, B, slices of `rows` outputs).  Every range holds at least one key, so its sum is positive and its
+// maximum finite.  Every slice merges the ranges again: their partial sums come from L2 and the up-projection's
+// rows are spread over more SMs (18 us with one slice and one row per warp at a time).
+__global__ void __launch_bounds__(MLA_THREADS)
+mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const __nv_bfloat16* __restrict__ w,
+                 __nv_bfloat16* __restrict__ out, int ranges, int H, int dn, int dv, int C, int rows) {
+  __shared__ __align__(16) float olat[MLA_MAX_C];
+  extern __shared__ float merge_w[];             // [ranges]
+  const int h = blockIdx.x, b = blockIdx.y;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const float* ml = part_ml + ((size_t)b * H + h) * ranges * 2;
+  if (warp == 0) {
+    float m = -INFINITY;
+    for (int r = lane; r < ranges; r += 32) m = fmaxf(m, ml[2 * r]);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+    float l = 0.f;
+    for (int r = lane; r < ranges; r += 32) {
+      const float e = exp2f(ml[2 * r] - m);
+      merge_w[r] = e;
+      l += e * ml[2 * r + 1];
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) l += __shfl_xor_sync(0xffffffffu, l, o);
+    const float inv = 1.f / l;
+    for (int r = lane; r < ranges; r += 32) merge_w[r] *= inv;
+  }
+  __syncthreads();
+  if (2 * (int)threadIdx.x < C) {
+    const float* po = part_o + ((size_t)b * H + h) * ranges * C + 2 * threadIdx.x;
+    float x = 0.f, y = 0.f;
+#pragma unroll 8
+    for (int r = 0; r < ranges; ++r) {
+      const float2 v = *reinterpret_cast<const float2*>(po + (size_t)r * C);
+      x += merge_w[r] * v.x;
+      y += merge_w[r] * v.y;
+    }
+    olat[2 * threadIdx.x] = x;
+    olat[2 * threadIdx.x + 1] = y;
+  }
+  __syncthreads();
+  // a warp takes four rows at a time: their loads are in flight together
+  const uint4* wv = reinterpret_cast<const uint4*>(w + ((size_t)h * (dn + dv) + dn) * C);
+  const int cv = C / 8;
+  const int j0 = blockIdx.z * rows, j1 = min(dv, j0 + rows);
+  for (int j = j0 + 4 * warp; j < j1; j += 4 * (MLA_THREADS / 32)) {
+    float s[4] = {};
+#pragma unroll
+    for (int k = 0; k < MLA_MAX_C / 8 / 32; ++k) {
+      const int c = lane + 32 * k;
+      uint4 v[4];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) v[r] = (c < cv && j + r < j1) ? wv[(size_t)(j + r) * cv + c] : make_uint4(0, 0, 0, 0);
+      if (c < cv) {
+        const float4 x0 = *reinterpret_cast<const float4*>(olat + c * 8), x1 = *reinterpret_cast<const float4*>(olat + c * 8 + 4);
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+          const float2 a = unpack_bf16(v[r].x), bb = unpack_bf16(v[r].y), cc = unpack_bf16(v[r].z), d = unpack_bf16(v[r].w);
+          s[r] += x0.x * a.x + x0.y * a.y + x0.z * bb.x + x0.w * bb.y + x1.x * cc.x + x1.y * cc.y + x1.z * d.x + x1.w * d.y;
+        }
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 4; ++r) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) s[r] += __shfl_xor_sync(0xffffffffu, s[r], o);
+      if (lane == 0 && j + r < j1) out[((size_t)b * H + h) * dv + j + r] = __float2bfloat16(s[r]);
+    }
+  }
+}
+
+}  // namespace tpb
+
+using namespace tpb;
+
+// Ranges of keys the split kernel uses for `n_keys` cached tokens: one step of 32 keys each until the
+// machine holds two CTAs per SM, then longer ranges.
+extern "C" int tpb_mla_decode_ranges(int B, int H, int n_keys) {
+  if (B < 1 || H < 1 || n_keys < 1) return 0;
+  const long long groups = (long long)B * ((H + MLA_HG - 1) / MLA_HG);
+  const int steps = (n_keys + MLA_KEYS - 1) / MLA_KEYS;
+  long long want = 2LL * sm_count() / groups;
+  if (want < 1) want = 1;
+  const int per = (int)((steps + want - 1) / want);
+  return (steps + per - 1) / per;
+}
+
+// q [B, H * (dn + 64)] (rotated in place), ckv [B, C + 64], w = kv_b_proj [H * (dn + dv), C], out [B, H * dv], all
+// contiguous bf16; the new token goes to row `pos` of the caches (rows C and 64 wide, kv_bs / pe_bs
+// elements between sequences) and attends to rows 0 .. pos.  qa: B*H*C floats; part_o: B*H*ranges*C;
+// part_ml: B*H*ranges*2, with ranges = tpb_mla_decode_ranges(B, H, pos + 1).
+extern "C" int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, const float* cosT, const float* sinT,
+                              void* kv_cache, void* pe_cache, long long kv_bs, long long pe_bs, const void* w, void* out,
+                              float* qa, float* part_o, float* part_ml, int B, int H, int dn, int dv, int C, int R,
+                              int pos, float scale, float eps, int interleaved, int ranges, void* stream_) {
+  if (R != MLA_R || C % 64 || C > MLA_MAX_C || C < 64 || dn < 8 || dn % 8 || dn > 512 || dv < 1 || dv > 4096 || H < 1 || pos < 0) return -2;
+  if (kv_bs % 8 || pe_bs % 8 || B > 65535) return -2;
+  for (const void* a : {(const void*)q, ckv, norm_w, (const void*)kv_cache, (const void*)pe_cache, w, (const void*)out})
+    if (reinterpret_cast<uintptr_t>(a) % 16) return -2;
+  if (B <= 0) return 0;
+  const int n_keys = pos + 1;
+  if (ranges != tpb_mla_decode_ranges(B, H, n_keys)) return -2;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  auto* qb = reinterpret_cast<__nv_bfloat16*>(q);
+  auto* kc = reinterpret_cast<__nv_bfloat16*>(kv_cache);
+  auto* pc = reinterpret_cast<__nv_bfloat16*>(pe_cache);
+  const auto* wb = reinterpret_cast<const __nv_bfloat16*>(w);
+  mla_prep_kernel<<<B, MLA_THREADS, 0, stream>>>(qb, reinterpret_cast<const __nv_bfloat16*>(ckv),
+                                                 reinterpret_cast<const __nv_bfloat16*>(norm_w), cosT, sinT, kc, pc,
+                                                 kv_bs, pe_bs, pos, H, dn, C, eps, interleaved);
+  mla_fold_kernel<<<dim3(H, C / 64, (B + MLA_MAX_B - 1) / MLA_MAX_B), MLA_THREADS, MLA_MAX_B * dn * 4, stream>>>(
+      qb, wb, qa, B, H, dn, dv, C);
+  const int steps = (n_keys + MLA_KEYS - 1) / MLA_KEYS;
+  const int per = (steps + ranges - 1) / ranges * MLA_KEYS;
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(mla_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         MlaSplitSmem::bytes(MLA_MAX_C));
+    if (e != cudaSuccess) return 1000 + (int)e;
+    configured = true;
+  }
+  mla_split_kernel<<<dim3(ranges, (H + MLA_HG - 1) / MLA_HG, B), MLA_THREADS, MlaSplitSmem::bytes(C), stream>>>(
+      qa, qb, kc, pc, kv_bs, pe_bs, part_o, part_ml, n_keys, per, H, dn, C, scale * 1.4426950408889634f);
+  const int rows = 32;     // one pass of the eight warps
+  mla_merge_kernel<<<dim3(H, B, (dv + rows - 1) / rows), MLA_THREADS, ranges * 4, stream>>>(
+      part_o, part_ml, wb, reinterpret_cast<__nv_bfloat16*>(out), ranges, H, dn, dv, C, rows);
+  cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 1000 + (int)e;
+}

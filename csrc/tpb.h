@@ -206,6 +206,13 @@ int tpb_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, 
                          long long ldw, long long ldc, int w_mn, int epi, float alpha, const void* aux, long long ldaux,
                          void* c2, long long ldc2, int nt, int splits, void* stream);
 
+// ---- cached latent attention, one token per sequence (mla_decode.cu)
+int tpb_mla_decode_ranges(int B, int H, int n_keys);
+int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, const float* cosT, const float* sinT, void* kv_cache,
+                   void* pe_cache, long long kv_bs, long long pe_bs, const void* w, void* out, float* qa, float* part_o,
+                   float* part_ml, int B, int H, int dn, int dv, int C, int R, int pos, float scale, float eps,
+                   int interleaved, int ranges, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

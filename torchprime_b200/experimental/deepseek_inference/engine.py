@@ -15,15 +15,19 @@ checkpoint trained or converted for the training model serves as is.  Two cache 
   ``kv_lora_rank + dr`` numbers per cached token instead of ``H * (dn + dr + dv)`` (576 against
   40960 for the 671B model) — on a bandwidth-bound decode that ratio is the speed-up.
 
-Prefill at position 0 with the ``naive`` layout goes through the flash-attention kernel; decode
-steps and the ``absorb`` layout use batched matrix products over the cache.
+Prefill at position 0 with the ``naive`` layout goes through the flash-attention kernel and a bf16
+decode step of the ``absorb`` layout through the kernels of ``ops/mla_decode.py``; everything else uses
+batched matrix products over the cache.
 """
 
 from __future__ import annotations
 
+import functools
+
 import torch
 
 from ...ops import functional as ops
+from ...ops import mla_decode
 from ...ops import reference as ref
 
 
@@ -55,7 +59,7 @@ class DeepseekInferenceEngine:
     return sum(t.numel() * t.element_size() for t in bufs)
 
   # -------------------------------------------------------------------------------------
-  def _attention(self, li: int, attn, x, start: int, pos):
+  def _attention(self, li: int, attn, x, start: int, residual, positions):
     b, s, _ = x.shape
     end = start + s
     h, dn, dr, dv, c = attn.num_heads, attn.qk_nope_head_dim, attn.qk_rope_head_dim, attn.v_head_dim, attn.kv_lora_rank
@@ -64,9 +68,17 @@ class DeepseekInferenceEngine:
     else:
       q = ops.linear(attn.q_a_layernorm(ops.linear(x, attn.q_a_proj.weight, bias=attn.q_a_proj.bias)),
                      attn.q_b_proj.weight)
+    ckv = ops.linear(x, attn.kv_a_proj_with_mqa.weight, bias=attn.kv_a_proj_with_mqa.bias)
+    norm = attn.kv_a_layernorm
+    if self.attn_impl == "absorb" and mla_decode.supported(q, ckv, norm.weight, self.kv_cache[li], self.pe_cache[li],
+                                                           attn.kv_b_proj.weight, h, dn, dr, dv, c):
+      o = mla_decode.absorb_step(q, ckv, norm.weight, norm.variance_epsilon, self.cos, self.sin, start,
+                                 self.kv_cache[li], self.pe_cache[li], attn.kv_b_proj.weight, h, dn, dv, attn.scaling,
+                                 attn.rope_interleave)
+      return ops.linear(o, attn.o_proj.weight, bias=attn.o_proj.bias, residual=residual)
+    pos = positions()
     q = ops.rope_slices(q, self.cos, self.sin, h, dr, s, col0=dn, head_stride=dn + dr, pos=pos,
                         interleaved=attn.rope_interleave)
-    ckv = ops.linear(x, attn.kv_a_proj_with_mqa.weight, bias=attn.kv_a_proj_with_mqa.bias)
     ckv = ops.rope_slices(ckv, self.cos, self.sin, 1, dr, s, col0=c, head_stride=dr, pos=pos,
                           interleaved=attn.rope_interleave)
     latent = attn.kv_a_layernorm(ckv[..., :c].contiguous())
@@ -103,7 +115,7 @@ class DeepseekInferenceEngine:
       o_lat = torch.einsum("bsht,btc->bshc", scores.softmax(-1), lc)
       o = torch.einsum("bshc,hdc->bshd", o_lat, w[:, dn:].float()).to(x.dtype)
     o = o.reshape(b, s, h * dv)
-    return ops.linear(o, attn.o_proj.weight, bias=attn.o_proj.bias)
+    return ops.linear(o, attn.o_proj.weight, bias=attn.o_proj.bias, residual=residual)
 
   @torch.no_grad()
   def forward(self, tokens: torch.Tensor, start_pos: int = 0) -> torch.Tensor:
@@ -112,10 +124,13 @@ class DeepseekInferenceEngine:
     assert b <= self.max_batch_size and start_pos + s <= self.max_seq_len, (b, start_pos, s)
     m = self.model.model
     h = m.embed_tokens(tokens.to(self.device))
-    pos = (start_pos + torch.arange(s, device=self.device, dtype=torch.int32)).repeat(b).contiguous()
+
+    @functools.cache
+    def positions():       # of every token, for the layers that need them as a tensor
+      return (start_pos + torch.arange(s, device=self.device, dtype=torch.int32)).repeat(b).contiguous()
+
     for li, layer in enumerate(m.layers):
-      a = self._attention(li, layer.self_attn, layer.input_layernorm(h), start_pos, pos)
-      h = h + a
+      h = self._attention(li, layer.self_attn, layer.input_layernorm(h), start_pos, h, positions)
       h = layer.mlp(layer.post_attention_layernorm(h), residual=h)
     last = m.norm(h[:, -1:, :].contiguous())
     return ops.linear_f32(last[:, 0], self.model.lm_head.weight)
