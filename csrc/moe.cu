@@ -155,6 +155,8 @@ __global__ void router_topk_kernel(const T* __restrict__ logits, const float* __
 }
 
 // out[r, :] = (src_row[r] >= 0) ? scale[r] * x[src_row[r], :] : 0       (rows of 16-byte vectors)
+// PAD false: padding rows are left unwritten (for readers that ignore them).
+template <bool PAD>
 __global__ void moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ src_row,
                                   const float* __restrict__ row_scale, uint4* __restrict__ out, long long rows,
                                   int nvec) {
@@ -164,6 +166,7 @@ __global__ void moe_gather_kernel(const uint4* __restrict__ x, const int* __rest
     const long long r = i / nvec;
     const int c = (int)(i % nvec);
     const int src = src_row[r];
+    if (!PAD && src < 0) continue;
     uint4 v = make_uint4(0, 0, 0, 0);
     if (src >= 0) {
       v = x[(long long)src * nvec + c];
@@ -280,19 +283,21 @@ __global__ void a2a_push_kernel(const A2APushParams p) {
 // expert), a prefix over warps gives each warp its first row in every expert's segment, sweep 2
 // walks the range again and hands out rows in order (match_any groups equal experts inside a
 // warp, the lane order breaks ties), so the result does not depend on scheduling.
-// Outputs: counts[E], k_offsets[E+1] (multiples of 128), dest[n] (row of each pair), src_row[M]
-// (token feeding a row) and src_pair[M] (pair feeding a row), both pre-filled with -1 by the
-// host, tile_expert[M/128] (pre-filled with -1).
+// Outputs: counts[E], k_offsets[E+1] (multiples of `align`), dest[n] (row of each pair), src_row[M]
+// (token feeding a row), src_pair[M] (pair feeding a row; both -1 in padding rows) and
+// tile_expert[M / tile] (-1 past the last segment), tile = min(align, 128) rows.
 // ----------------------------------------------------------------------------
 constexpr int PLAN_THREADS = 1024;
 constexpr int PLAN_MAX_E = 256;
 
 __global__ void __launch_bounds__(PLAN_THREADS, 1)
-moe_plan_kernel(const int* __restrict__ idx, int n, int K, int E, int align, int* __restrict__ counts,
+moe_plan_kernel(const int* __restrict__ idx, int n, int K, int E, int M, int align, int* __restrict__ counts,
                 int* __restrict__ k_offsets, int* __restrict__ dest, int* __restrict__ src_row,
                 long long* __restrict__ src_pair, int* __restrict__ tile_expert) {
   __shared__ int wcount[32][PLAN_MAX_E];     // sweep 1: pairs of (warp, expert); sweep 2: next row
   __shared__ int off_pad[PLAN_MAX_E + 1];
+  __shared__ int total_s[PLAN_MAX_E];
+  const int tile = min(align, 128);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   for (int i = threadIdx.x; i < 32 * PLAN_MAX_E; i += PLAN_THREADS) (&wcount[0][0])[i] = 0;
   __syncthreads();
@@ -311,6 +316,7 @@ moe_plan_kernel(const int* __restrict__ idx, int n, int K, int E, int align, int
     int total = 0;
     for (int w = 0; w < 32; ++w) total += wcount[w][threadIdx.x];
     counts[threadIdx.x] = total;
+    total_s[threadIdx.x] = total;
     off_pad[threadIdx.x + 1] = (total + align - 1) / align * align;
   }
   if (threadIdx.x == 0) off_pad[0] = 0;
@@ -326,9 +332,22 @@ moe_plan_kernel(const int* __restrict__ idx, int n, int K, int E, int align, int
       wcount[w][threadIdx.x] = run;
       run += c;
     }
-    for (int t = off_pad[threadIdx.x] / 128; t < off_pad[threadIdx.x + 1] / 128; ++t) tile_expert[t] = threadIdx.x;
+    for (int t = off_pad[threadIdx.x] / tile; t < off_pad[threadIdx.x + 1] / tile; ++t) tile_expert[t] = threadIdx.x;
   }
+  for (int t = off_pad[E] / tile + threadIdx.x; t < M / tile; t += PLAN_THREADS) tile_expert[t] = -1;
   __syncthreads();
+  // padding rows: the end of every expert's segment (one warp per expert) and everything past the last
+  // one (filled here and not by memsets of the whole arrays: three launches fewer)
+  for (int e = warp; e < E; e += 32) {
+    for (int r = off_pad[e] + total_s[e] + lane; r < off_pad[e + 1]; r += 32) {
+      src_row[r] = -1;
+      src_pair[r] = -1;
+    }
+  }
+  for (int r = off_pad[E] + threadIdx.x; r < M; r += PLAN_THREADS) {
+    src_row[r] = -1;
+    src_pair[r] = -1;
+  }
   for (int base = lo; base < hi; base += 32) {
     const int i = base + lane;
     const int e = i < hi ? idx[i] : -1;
@@ -446,8 +465,18 @@ extern "C" int tpb_moe_gather(const void* x, const int* src_row, const float* ro
                               int dim, void* stream) {
   if (dim % 8) return -2;
   if (rows <= 0) return 0;
-  moe_gather_kernel<<<grid_for_items(rows * (dim / 8), 256), 256, 0, STREAM(stream)>>>(
+  moe_gather_kernel<true><<<grid_for_items(rows * (dim / 8), 256), 256, 0, STREAM(stream)>>>(
       (const uint4*)x, src_row, row_scale, (uint4*)out, rows, dim / 8);
+  return rc_of(cudaGetLastError());
+}
+
+// The same without a scale and without writing the padding rows.
+extern "C" int tpb_moe_gather_real(const void* x, const int* src_row, void* out, long long rows, int dim,
+                                   void* stream) {
+  if (dim % 8) return -2;
+  if (rows <= 0) return 0;
+  moe_gather_kernel<false><<<grid_for_items(rows * (dim / 8), 256), 256, 0, STREAM(stream)>>>(
+      (const uint4*)x, src_row, nullptr, (uint4*)out, rows, dim / 8);
   return rc_of(cudaGetLastError());
 }
 
@@ -490,19 +519,17 @@ extern "C" int tpb_a2a_push_rows(const void* src, int n_rows, int dim, int world
   return rc_of(cudaGetLastError());
 }
 
-// idx [tokens, K] int32 (entries outside [0, E) are dropped: dest = -1).  align: 128 or 256 rows per
-// segment step.  rows = static row count of the padded layout (>= round_up(tokens * K, align) + align * E).  Everything is on the device; no host read.
+// idx [tokens, K] int32 (entries outside [0, E) are dropped: dest = -1).  align: 16, 32, 64, 128 or 256 rows per
+// segment step.  rows = static row count of the padded layout, a multiple of align that holds n pairs and
+// align - 1 padding rows for every expert that can be hit.  Everything is on the device; no host read.
 extern "C" int tpb_moe_plan(const int* idx, int tokens, int K, int E, int rows, int align, int* counts, int* k_offsets,
                             int* dest, int* src_row, long long* src_pair, int* tile_expert, void* stream) {
-  if (E < 1 || E > PLAN_MAX_E || K < 1 || tokens < 0 || (align != 128 && align != 256) || rows % align) return -2;
+  if (E < 1 || E > PLAN_MAX_E || K < 1 || tokens < 0 || rows < 0) return -2;
+  if ((align != 16 && align != 32 && align != 64 && align != 128 && align != 256) || rows % align) return -2;
   const long long n = (long long)tokens * K;
-  if (n > (1LL << 30) || rows < (n + align - 1) / align * align + (long long)align * E) return -2;
-  cudaError_t e = cudaMemsetAsync(src_row, 0xFF, sizeof(int) * rows, STREAM(stream));
-  if (e == cudaSuccess) e = cudaMemsetAsync(src_pair, 0xFF, sizeof(long long) * rows, STREAM(stream));
-  if (e == cudaSuccess) e = cudaMemsetAsync(tile_expert, 0xFF, sizeof(int) * (rows / 128), STREAM(stream));
-  if (e != cudaSuccess) return rc_of(e);
-  moe_plan_kernel<<<1, PLAN_THREADS, 0, STREAM(stream)>>>(idx, (int)n, K, E, align, counts, k_offsets, dest, src_row, src_pair,
-                                                          tile_expert);
+  if (n > (1LL << 30) || rows < n + (long long)(align - 1) * (n < E ? n : E)) return -2;
+  moe_plan_kernel<<<1, PLAN_THREADS, 0, STREAM(stream)>>>(idx, (int)n, K, E, rows, align, counts, k_offsets, dest, src_row,
+                                                          src_pair, tile_expert);
   return rc_of(cudaGetLastError());
 }
 

@@ -213,6 +213,12 @@ int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, const float* co
                    float* part_ml, int B, int H, int dn, int dv, int C, int R, int pos, float scale, float eps,
                    int interleaved, int ranges, void* stream);
 
+// ---- experts with few rows each: segments padded to nt rows, tile_expert[rows / nt]
+int tpb_moe_gather_real(const void* x, const int* src_row, void* out, long long rows, int dim, void* stream);
+int tpb_grouped_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, int rows, int N, int K, int E,
+                                 long long ldx, long long ldw, long long w_stride, long long ldc, int w_mn, int epi,
+                                 const int* tile_expert, int experts_hit, int nt, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,11 +1,11 @@
-"""GEMMs with few rows (csrc/gemm_skinny_sm100.cu)."""
+"""GEMMs with few rows (csrc/gemm_skinny_sm100.cu): dense and grouped by expert."""
 
 import pytest
 import torch
 
 pytestmark = pytest.mark.gpu
 
-from torchprime_b200.ops import kernels as k
+from torchprime_b200.ops import kernels as k, moe
 from torchprime_b200.ops._lib import lib, ptr, stream_ptr
 
 BF16_EPS = 2.0 ** -8
@@ -86,6 +86,58 @@ def test_split_sums_do_not_depend_on_the_run(cuda_lib):
   a = _skinny(x, w, epi=k.EPI_F32, splits=8)
   for _ in range(3):
     assert torch.equal(a, _skinny(x, w, epi=k.EPI_F32, splits=8))
+
+
+@pytest.mark.parametrize("align", [16, 32, 64])
+@pytest.mark.parametrize("t,kk,e", [(1, 6, 64), (4, 6, 64), (37, 2, 8), (128, 8, 256), (5, 1, 3)])
+def test_plan_with_narrow_segments(cuda_lib, align, t, kk, e):
+  torch.manual_seed(t)
+  idx = torch.randint(0, e, (t, kk), device="cuda", dtype=torch.int32)      # repeated experts in a token too
+  plan = moe._build_dispatch_plan_kernel(idx, e, align)
+  assert plan.num_rows % align == 0 and int(plan.k_offsets[-1]) <= plan.num_rows
+  flat = idx.reshape(-1).long()
+  order = torch.argsort(flat, stable=True)
+  counts = torch.bincount(flat, minlength=e)
+  off = torch.cat([counts.new_zeros(1), ((counts + align - 1) // align * align).cumsum(0)])
+  assert torch.equal(plan.k_offsets.long(), off) and torch.equal(plan.counts.long(), counts)
+  rank = torch.arange(flat.numel(), device="cuda") - (counts.cumsum(0) - counts)[flat[order]]
+  dest = torch.empty_like(flat)
+  dest[order] = off[flat[order]] + rank
+  assert torch.equal(plan.dest.reshape(-1).long(), dest)
+  pair = torch.full((plan.num_rows,), -1, device="cuda")
+  pair[dest] = torch.arange(flat.numel(), device="cuda")
+  assert torch.equal(plan.src_pair, pair)
+  assert torch.equal(plan.src_row.long(), torch.where(pair >= 0, pair // kk, pair))
+  tiles = torch.arange(plan.num_rows // align, device="cuda") * align
+  te = torch.bucketize(tiles, off[1:], right=True)
+  assert torch.equal(plan.tile_expert.long(), torch.where(te < e, te, torch.full_like(te, -1)))
+
+
+@pytest.mark.parametrize("fused", [False, True])
+@pytest.mark.parametrize("t,kk,e,d,f", [(1, 6, 64, 256, 192), (4, 6, 64, 2048, 1408), (16, 2, 8, 512, 1024), (100, 2, 16, 256, 320),
+                                        (128, 1, 2, 128, 64)])
+def test_grouped_mlp_without_gradients(cuda_lib, t, kk, e, d, f, fused):
+  """The few-rows path against the tiled grouped GEMMs' oracle, one expert hit by nobody."""
+  torch.manual_seed(t + e)
+  x = torch.randn(t, d, device="cuda", dtype=torch.bfloat16)
+  wg, wu = ((torch.randn(e, d, f, device="cuda") / d ** 0.5).to(torch.bfloat16) for _ in range(2))
+  wd = (torch.randn(e, f, d, device="cuda") / f ** 0.5).to(torch.bfloat16)
+  if fused:
+    wg = torch.cat([wg, wu], dim=2)
+  logits = torch.randn(t, e, device="cuda")
+  logits[:, 0] = -1e9
+  w, idx, _ = moe.router_topk(logits, kk, mode="softmax")
+  with torch.no_grad():
+    y = moe.grouped_mlp(x, w, idx, wg, None if fused else wu, wd, fused_gate_up=fused)
+  want = moe.grouped_mlp_reference(x.double(), w.double(), idx, wg.double(), wu.double(), wd.double(), fused)
+  # act and rows are rounded to bf16 once each, the result once more
+  assert ((y.double() - want).norm() / want.norm()).item() < 3 * BF16_EPS
+
+
+def test_route_of_the_few_rows_path():
+  assert moe.few_rows_align(4, 6, 64) == 16 and moe.few_rows_align(128, 6, 64) == 32
+  assert moe.few_rows_align(128, 2, 8) == 64 and moe.few_rows_align(129, 2, 8) is None
+  assert moe.few_rows_align(128, 8, 8) is None
 
 
 def test_linear_f32_logits(cuda_lib):

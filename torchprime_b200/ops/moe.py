@@ -7,7 +7,7 @@ model/deepseek_v3/model.py:274-338) is organised here around one layout: the ``T
 (token, slot) pairs are sorted by expert and every expert's rows are padded to a multiple of
 128, so a 128-row GEMM tile never straddles two experts and padded rows are zero.  All index
 bookkeeping stays on the device (no host synchronisation): the padded row count is bounded
-by ``T*K + 128*E`` and tiles past the real end are marked unused.
+by ``T*K + 127*min(T*K, E)`` and tiles past the real end are marked unused.
 
 On CUDA/bf16 the heavy parts run as sm_100a kernels (router top-k, row gather, grouped
 tcgen05 GEMMs with fused SwiGLU, combine); elsewhere the same math runs in plain PyTorch.
@@ -30,6 +30,8 @@ _lib.register_signature("tpb_grouped_gemm_bf16", [P, P, P, P, I, I, I, I, LL, LL
 _lib.register_signature("tpb_router_topk", [P, I, P, P, P, P, I, I, I, I, I, I, I, FL, P])
 _lib.register_signature("tpb_moe_plan", [P, I, I, I, I, I, P, P, P, P, P, P, P])
 _lib.register_signature("tpb_moe_gather", [P, P, P, P, LL, I, P])
+_lib.register_signature("tpb_moe_gather_real", [P, P, P, LL, I, P])
+_lib.register_signature("tpb_grouped_gemm_skinny_bf16", [P, P, P, P, I, I, I, I, LL, LL, LL, LL, I, I, P, I, I, P])
 _lib.register_signature("tpb_moe_combine", [P, P, P, P, LL, I, I, P])
 _lib.register_signature("tpb_moe_combine_dw", [P, P, P, P, LL, I, I, P])
 
@@ -103,13 +105,14 @@ class DispatchPlan:
   src_row: torch.Tensor      # [M] int32: token feeding padded row r, -1 for padding
   src_pair: torch.Tensor     # [M] int64: flat (token*K+slot) feeding row r, -1 for padding
   dest: torch.Tensor         # [T,K] int32: padded row of each pair, -1 if dropped
-  tile_expert: torch.Tensor  # [M/128] int32
-  k_offsets: torch.Tensor    # [E+1] int32 (multiples of 128)
+  tile_expert: torch.Tensor  # [M / min(row_align, 128)] int32
+  k_offsets: torch.Tensor    # [E+1] int32 (multiples of row_align)
   counts: torch.Tensor       # [E] rows per expert (after dropping)
   num_rows: int              # M (static upper bound)
   num_experts: int
   top_k: int
-  row_align: int = 128       # expert segments are padded to this many rows (256 lets the CTA-pair GEMM run)
+  row_align: int = 128       # expert segments are padded to this many rows (256 lets the CTA-pair GEMM run;
+                             # below 128 only grouped_mlp_few_rows can read the plan)
 
 
 def build_dispatch_plan(idx: torch.Tensor, num_experts: int, capacity: int | None = None,
@@ -160,7 +163,8 @@ def build_dispatch_plan(idx: torch.Tensor, num_experts: int, capacity: int | Non
   valid = sorted_e < e
   dest_sorted = torch.where(valid, torch.cat([off_pad, off_pad.new_zeros(1)])[sorted_e] + rank,
                             torch.full_like(rank, -1))
-  m = (n + align - 1) // align * align + e * align
+  # at most min(n, e) experts are hit (one segment step at least: without tokens gradients are still written)
+  m = max(align, (n + (align - 1) * min(n, e) + align - 1) // align * align)
   dest = torch.empty(n, dtype=torch.long, device=dev)
   dest[order] = dest_sorted
   src_pair = torch.full((m + 1,), -1, dtype=torch.long, device=dev)
@@ -182,10 +186,12 @@ def _build_dispatch_plan_kernel(idx: torch.Tensor, e: int, align: int = ROW_ALIG
   t, k = idx.shape
   dev = idx.device
   n = t * k
-  m = (n + align - 1) // align * align + e * align
+  # at most min(n, e) experts are hit (one segment step at least: without tokens gradients are still written)
+  m = max(align, (n + (align - 1) * min(n, e) + align - 1) // align * align)
+  tile = min(align, ROW_ALIGN)
   idx32 = idx.to(torch.int32).contiguous()
-  ints = torch.empty(e + (e + 1) + n + m + m // ROW_ALIGN, dtype=torch.int32, device=dev)
-  counts, k_offsets, dest, src_row, tile_expert = torch.split(ints, [e, e + 1, n, m, m // ROW_ALIGN])
+  ints = torch.empty(e + (e + 1) + n + m + m // tile, dtype=torch.int32, device=dev)
+  counts, k_offsets, dest, src_row, tile_expert = torch.split(ints, [e, e + 1, n, m, m // tile])
   src_pair = torch.empty(m, dtype=torch.int64, device=dev)
   check(lib().tpb_moe_plan(ptr(idx32), t, k, e, m, align, ptr(counts), ptr(k_offsets), ptr(dest), ptr(src_row), ptr(src_pair),
                            ptr(tile_expert), stream_ptr()), "moe_plan")
@@ -200,6 +206,37 @@ def gather_rows(x, src_row, row_scale=None):
   _debug.check_index("moe_gather", "src_row", src_row, 0, x.reshape(-1, d).shape[0], also_allowed=-1)
   check(lib().tpb_moe_gather(ptr(x), ptr(src_row), ptr(row_scale), ptr(out), m, d, stream_ptr()), "moe_gather")
   return out
+
+
+def few_rows_align(t: int, k: int, e: int) -> int | None:
+  """Token-tile width of the few-rows path for ``t`` tokens, or None where the tiled grouped GEMMs are
+  the better ones.  It is about twice the average number of rows an expert sees."""
+  per = t * k / e
+  if t > 128 or per > 64:
+    return None
+  want = min(t, 2 * per)
+  return 16 if want <= 16 else 32 if want <= 32 else 64
+
+
+def grouped_mlp_few_rows(x, weights, idx, w_gate, w_up, w_down, fused_gate_up, align):
+  """The routed MLP without gradients when experts see a handful of rows each (decode): segments are
+  padded to ``align`` rows instead of 128 and both GEMMs stream every hit expert's weights once."""
+  t, k = idx.shape
+  e, d = w_gate.shape[0], x.shape[1]
+  f = w_down.shape[1]
+  plan = _build_dispatch_plan_kernel(idx, e, align)
+  m, hit = plan.num_rows, min(e, t * k)
+  xg = torch.empty(m, d, dtype=x.dtype, device=x.device)
+  check(lib().tpb_moe_gather_real(ptr(x), ptr(plan.src_row), ptr(xg), m, d, stream_ptr()), "moe_gather_real")
+  act = torch.empty(m, f, dtype=x.dtype, device=x.device)
+  rows = torch.empty(m, d, dtype=x.dtype, device=x.device)
+  check(lib().tpb_grouped_gemm_skinny_bf16(
+    ptr(xg), ptr(w_gate), None if fused_gate_up else ptr(w_up), ptr(act), m, 2 * f, d, e, d, w_gate.stride(1),
+    w_gate.stride(0), f, 1, _lib.EPI_SWIGLU, ptr(plan.tile_expert), hit, align, stream_ptr()), "grouped_gemm_skinny gate/up")
+  check(lib().tpb_grouped_gemm_skinny_bf16(
+    ptr(act), ptr(w_down), None, ptr(rows), m, d, f, e, f, d, w_down.stride(0), d, 1, _lib.EPI_BF16,
+    ptr(plan.tile_expert), hit, align, stream_ptr()), "grouped_gemm_skinny down")
+  return combine_rows(rows, plan.dest, weights)
 
 
 def combine_rows(rows, dest, w=None):
@@ -348,8 +385,15 @@ def grouped_mlp(x, weights, idx, w_gate, w_up, w_down, *, fused_gate_up=False, c
   (``fused_gate_up``: w_gate is [E,D,2F] = [gate | up] and w_up is ignored)."""
   e = w_gate.shape[0]
   f = w_down.shape[1]
+  from .functional import inference_only
   ok = (_kernels_ok(x, w_gate, w_down) and x.shape[-1] % 64 == 0 and f % 64 == 0 and x.is_cuda)
   if ok:
+    if (capacity is None and e <= 256 and inference_only()
+        and all(w.is_contiguous() and w.data_ptr() % 16 == 0 for w in (w_gate, w_up, w_down) if w is not None)):
+      align = few_rows_align(*idx.shape, e)
+      if align is not None:
+        return grouped_mlp_few_rows(x.contiguous(), weights.float().contiguous(), idx, w_gate, w_up, w_down,
+                                    fused_gate_up, align)
     plan = build_dispatch_plan(idx, e, capacity, rows_per_group)
     wu = w_gate if fused_gate_up else w_up
     return _GroupedMLPFn.apply(x.contiguous(), weights.float().contiguous(), w_gate, wu, w_down, plan, fused_gate_up)
