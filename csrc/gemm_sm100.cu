@@ -31,9 +31,10 @@ constexpr int BM = 128, BN = 256, BK = 64, STAGES = 4;
 constexpr int A_BYTES = BM * BK * 2;                 // 16 KB
 constexpr int B_BYTES = BN * BK * 2;                 // 32 KB
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;       // 48 KB
-constexpr int EPI_SLAB_BYTES = 4 * 4096;              // one 32-row x 128-byte transpose slab per epilogue warp
+constexpr int EPI_SLAB_BYTES = 4 * 2 * 4096;          // two 32-row x 128-byte slabs per epilogue warp
 constexpr int GEMM_SMEM = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + EPI_SLAB_BYTES;
-static_assert(6 * 32768 + 64 <= STAGES * STAGE_BYTES + 256, "copier ring must fit the GEMM shared memory");
+static_assert(GEMM_SMEM <= 227 * 1024, "shared memory of one CTA");
+static_assert(6 * 32768 + 64 <= STAGES * STAGE_BYTES + EPI_SLAB_BYTES, "copier ring must fit the GEMM shared memory");
 constexpr int GEMM_THREADS = 192;
 
 struct GemmParams {
@@ -88,6 +89,7 @@ struct GemmParams {
   // owner's bf16 gradient shard over P2P with vector red.add.
   int rs_world;
   int tile_rot;                 // tiles are visited starting from this one (rotation by rank, see tpb_gemm_rs_bf16)
+  int tma_store;                // results leave through shared memory and the maps tmC / tmC2 (see slab_store)
   int te_stride;                // tile_expert entries per m-tile (2 for CTA-pair tiles of 256 rows)
   void* rs_dst[8];              // gradient shard base of every rank (symmetric memory), bf16
   long long rs_shard_elems;
@@ -297,6 +299,38 @@ __device__ void ag_pusher(const GemmParams& p) {
   }
 }
 
+// Results leave the SM by TMA: a warp writes 32 rows x 128 bytes (64 bf16 or 32 fp32 columns; each lane
+// owns a row of the accumulator) into a 128B-swizzled slab and one lane stores the box, which the copy engine
+// clips at the edges of C.  Stored from registers, every 16-byte vector of a warp goes to another row: 32
+// separate lines per instruction, and tiles with a short contraction (per-expert weight gradients: K of a
+// few hundred) spend longer in such an epilogue than in their MMAs.  An fp32 accumulation becomes a reduction at the
+// L2 and C is not read by the SM.  The three weight gradients of 64 experts (2048 x 1408, 128-256 rows each):
+// 890 -> 460 us; the accumulated 128,256 x 4096 fp32 gradient of two chunks with its first pass overwriting: 4.09 -> 2.60 ms.
+// (Eight epilogue warps instead of four: 1 % better there and 1 % worse for the vocabulary head.)  Two slabs per warp: one is read by the copy while the other is filled.
+template <bool REDUCE>
+__device__ __forceinline__ void slab_store(uint4* slabs, int& buf, const uint32_t* r, const CUtensorMap* map, int x,
+                                           int y, int z, int lane) {
+  uint4* slab = slabs + buf * 256;
+  buf ^= 1;
+  if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+  __syncwarp();
+#pragma unroll
+  for (int v = 0; v < 8; ++v) slab[lane * 8 + (v ^ (lane & 7))] = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+  fence_proxy_async();
+  __syncwarp();
+  if (lane == 0) {
+    if (REDUCE)
+      asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map),
+                   "r"(smem_u32(slab)), "r"(x), "r"(y), "r"(z)
+                   : "memory");
+    else
+      asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map),
+                   "r"(smem_u32(slab)), "r"(x), "r"(y), "r"(z)
+                   : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+  }
+}
+
 // PAIR: the kernel runs as clusters of two CTAs on 256 x 256 output tiles.  Each CTA stages its
 // 128 rows of A and ONE 128-row half of B per k-block (32 KB instead of 48 KB, in a 6-deep ring),
 // the even CTA issues tcgen05.mma.cta_group::2 (M = 256) for both, and each CTA drains its own
@@ -305,20 +339,20 @@ __device__ void ag_pusher(const GemmParams& p) {
 template <bool A_MN, bool B_MN, bool PAIR>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-            const __grid_constant__ CUtensorMap tmB2, const GemmParams p) {
+            const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
+            const __grid_constant__ CUtensorMap tmC2, const GemmParams p) {
   constexpr int NST = PAIR ? 6 : STAGES;                 // ring depth
   constexpr int SBYTES = PAIR ? 32768 : STAGE_BYTES;     // bytes per stage in this CTA
   constexpr int TM = PAIR ? 2 * BM : BM;                 // output rows per tile
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
                                              ~static_cast<uintptr_t>(1023));
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES);   // == 6 * 32768
+  uint4* epi_stage = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES);    // == 6 * 32768; 1024-byte aligned
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + STAGES * STAGE_BYTES + EPI_SLAB_BYTES);
   uint64_t* empty = full + NST;
   uint64_t* acc_full = empty + NST;
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
-  uint4* epi_stage = reinterpret_cast<uint4*>(smem + STAGES * STAGE_BYTES + 256);   // after the barrier block
-
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (!PAIR && (int)blockIdx.x < p.ag_copiers) {
     if (p.ag_push) ag_pusher(p); else ag_copier(p, smem);
@@ -514,6 +548,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   } else {
     // ---------------------------------------------------------------- epilogue
     const int q = warp & 3;  // TMEM lane quarter this warp may access
+    uint4* slabs = epi_stage + q * 512;
+    int buf = 0;
     int local = 0;
     for (int t = cta; t < num_tiles; t += n_ctas) {
       const TileInfo ti = tile_info(p, t, m_tiles, n_tiles, num_kb);
@@ -531,7 +567,73 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const uint32_t t_addr = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
       const bool row_ok = row < p.M;
 
-      if (swiglu) {
+      if (p.tma_store) {
+        const int row0 = tm * TM + rank * BM + q * 32;   // this warp's 32 rows
+        if (row0 < p.M) {
+          if (swiglu) {
+#pragma unroll 1
+            for (int c = 0; c < 2; ++c) {
+              const int col = n0 + c * 64;
+              if (col >= n_logical) break;
+              uint32_t o[32], pg[32], pu[32];
+#pragma unroll
+              for (int h = 0; h < 4; ++h) {
+                uint32_t g[16], u[16];
+                tmem_ld16(t_addr + c * 64 + h * 16, g);
+                tmem_ld16(t_addr + 128 + c * 64 + h * 16, u);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 8; ++j) {
+                  float g0 = __uint_as_float(g[2 * j]) * p.alpha, g1 = __uint_as_float(g[2 * j + 1]) * p.alpha;
+                  float u0 = __uint_as_float(u[2 * j]) * p.alpha, u1 = __uint_as_float(u[2 * j + 1]) * p.alpha;
+                  o[h * 8 + j] = pack_bf16(silu_f(g0) * u0, silu_f(g1) * u1);
+                  pg[h * 8 + j] = pack_bf16(g0, g1);
+                  pu[h * 8 + j] = pack_bf16(u0, u1);
+                }
+              }
+              slab_store<false>(slabs, buf, o, &tmC, col, row0, 0, lane);
+              if (p.c2) {
+                slab_store<false>(slabs, buf, pg, &tmC2, col, row0, 0, lane);
+                slab_store<false>(slabs, buf, pu, &tmC2, col, row0, 1, lane);
+              }
+            }
+          } else {
+            const int ez = p.mode == 2 ? ti.e : 0;
+            if (p.epi == TPB_EPI_BF16) {
+#pragma unroll 1
+              for (int c = 0; c < BN / 64; ++c) {
+                const int col = n0 + c * 64;
+                if (col >= p.N) break;
+                uint32_t o[32];
+#pragma unroll
+                for (int h = 0; h < 2; ++h) {
+                  uint32_t r[32];
+                  tmem_ld32(t_addr + c * 64 + h * 32, r);
+                  tmem_wait_ld();
+#pragma unroll
+                  for (int j = 0; j < 16; ++j)
+                    o[h * 16 + j] = empty_k ? 0u : pack_bf16(__uint_as_float(r[2 * j]) * p.alpha,
+                                                             __uint_as_float(r[2 * j + 1]) * p.alpha);
+                }
+                slab_store<false>(slabs, buf, o, &tmC, col, row0, ez, lane);
+              }
+            } else {
+#pragma unroll 1
+              for (int c = 0; c < BN / 32; ++c) {
+                const int col = n0 + c * 32;
+                if (col >= p.N) break;
+                uint32_t r[32];
+                tmem_ld32(t_addr + c * 32, r);
+                tmem_wait_ld();
+#pragma unroll
+                for (int j = 0; j < 32; ++j) r[j] = empty_k ? 0u : __float_as_uint(__uint_as_float(r[j]) * p.alpha);
+                if (p.epi == TPB_EPI_F32) slab_store<false>(slabs, buf, r, &tmC, col, row0, ez, lane);
+                else slab_store<true>(slabs, buf, r, &tmC, col, row0, ez, lane);
+              }
+            }
+          }
+        }
+      } else if (swiglu) {
         __nv_bfloat16* C = reinterpret_cast<__nv_bfloat16*>(p.C) + c_off + (long long)row * p.ldc;
         __nv_bfloat16* C2 =
             p.c2 ? reinterpret_cast<__nv_bfloat16*>(p.c2) + (long long)row * p.ldc2 : nullptr;
@@ -582,7 +684,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         // small request over NVLink.  The warp therefore transposes 64 columns through a 4 KB
         // shared-memory slab (XOR-swizzled, conflict-free both ways): afterwards eight consecutive
         // lanes hold the eight vectors of one row and reduce 128 contiguous bytes.
-        uint4* slab = epi_stage + q * 256;
+        uint4* slab = slabs;
         const int row_base = tm * TM + rank * BM + q * 32;
         const bool all_reduce = p.epi == TPB_EPI_AR_BF16;
 #pragma unroll 1
@@ -708,6 +810,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         else mbar_arrive(&acc_empty[acc]);
       }
     }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");   // the slabs go away
   }
 
   tc_fence_before();
@@ -726,11 +829,13 @@ int make_tmap_2d(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t out
                  uint32_t box_inner, uint32_t box_outer, int elem_bytes);  // tma.cu
 int make_tmap_3d(CUtensorMap* map, const void* ptr, uint64_t d0, uint64_t d1, uint64_t d2, uint64_t stride1_elems,
                  uint64_t stride2_elems, uint32_t box0, uint32_t box1);
+int make_tmap_out(CUtensorMap* map, const void* ptr, uint64_t cols, uint64_t rows, uint64_t planes, uint64_t ld_elems,
+                  uint64_t plane_elems, int elem_bytes);
 int sm_count();  // runtime.cu
 
 template <bool A_MN, bool B_MN>
-cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb2, const GemmParams& p,
-                        int grid, cudaStream_t stream) {
+cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb2, const CUtensorMap& tc,
+                        const CUtensorMap& tc2, const GemmParams& p, int grid, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_kernel<A_MN, B_MN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -738,14 +843,14 @@ cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  gemm_kernel<A_MN, B_MN, false><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, tb2, p);
+  gemm_kernel<A_MN, B_MN, false><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, tb2, tc, tc2, p);
   return cudaGetLastError();
 }
 
 // Launch as clusters of two CTAs (`grid` is even).
 template <bool A_MN, bool B_MN>
-cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb2, const GemmParams& p,
-                             int grid, cudaStream_t stream) {
+cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb2, const CUtensorMap& tc,
+                             const CUtensorMap& tc2, const GemmParams& p, int grid, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_kernel<A_MN, B_MN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
@@ -765,7 +870,7 @@ cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_kernel<A_MN, B_MN, true>, ta, tb, tb2, p);
+  return cudaLaunchKernelEx(&cfg, gemm_kernel<A_MN, B_MN, true>, ta, tb, tb2, tc, tc2, p);
 }
 
 
@@ -838,7 +943,22 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
     tb2 = tb;
   }
 
+  // Results that are plain stores (or fp32 accumulations) leave through TMA; residual adds, bf16
+  // accumulations and the epilogues that write to other GPUs read or write from registers.
+  CUtensorMap tc = ta, tc2 = ta;
+  bool tma_store = g.epi == TPB_EPI_BF16 || g.epi == TPB_EPI_F32 || g.epi == TPB_EPI_F32_ACC ||
+                   (swiglu && (!g.c2 || (g.ldc2 % 8 == 0 && !misaligned(g.c2))));
+  if (g.mode == 2 && (g.c_stride % (f32out ? 4 : 8))) tma_store = false;
+  if (tma_store) {
+    const uint64_t n_cols = swiglu ? g.N / 2 : g.N, planes = g.mode == 2 ? g.E : 1;
+    const uint64_t plane = g.mode == 2 && g.E > 1 ? (uint64_t)g.c_stride : (uint64_t)g.ldc * g.M;
+    if (make_tmap_out(&tc, g.C, n_cols, g.M, planes, g.ldc, plane, f32out ? 4 : 2)) return -3;
+    // [gate | up]: two planes, so that a box of the gate half is clipped where the up half begins
+    if (swiglu && g.c2 && make_tmap_out(&tc2, g.c2, n_cols, g.M, 2, g.ldc2, n_cols, 2)) return -3;
+  }
+
   GemmParams p;
+  p.tma_store = tma_store ? 1 : 0;
   p.M = g.M; p.N = g.N; p.K = g.K;
   p.C = g.C; p.ldc = g.ldc;
   p.aux = g.aux; p.ldaux = g.ldaux;
@@ -922,16 +1042,16 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
     const int pairs = pair_tiles > max_pairs ? max_pairs : (int)pair_tiles;
     const int m_tiles2 = (g.M + 2 * BM - 1) / (2 * BM);
     p.group_m = m_tiles2 < 8 ? m_tiles2 : 8;
-    if (!g.a_mn && !g.b_mn)      e = launch_gemm_pair<false, false>(ta, tb, tb2, p, 2 * pairs, stream);
-    else if (!g.a_mn && g.b_mn)  e = launch_gemm_pair<false, true>(ta, tb, tb2, p, 2 * pairs, stream);
-    else if (g.a_mn && !g.b_mn)  e = launch_gemm_pair<true, false>(ta, tb, tb2, p, 2 * pairs, stream);
-    else                         e = launch_gemm_pair<true, true>(ta, tb, tb2, p, 2 * pairs, stream);
+    if (!g.a_mn && !g.b_mn)      e = launch_gemm_pair<false, false>(ta, tb, tb2, tc, tc2, p, 2 * pairs, stream);
+    else if (!g.a_mn && g.b_mn)  e = launch_gemm_pair<false, true>(ta, tb, tb2, tc, tc2, p, 2 * pairs, stream);
+    else if (g.a_mn && !g.b_mn)  e = launch_gemm_pair<true, false>(ta, tb, tb2, tc, tc2, p, 2 * pairs, stream);
+    else                         e = launch_gemm_pair<true, true>(ta, tb, tb2, tc, tc2, p, 2 * pairs, stream);
     return e == cudaSuccess ? 0 : 1000 + (int)e;
   }
-  if (!g.a_mn && !g.b_mn)      e = launch_gemm<false, false>(ta, tb, tb2, p, grid, stream);
-  else if (!g.a_mn && g.b_mn)  e = launch_gemm<false, true>(ta, tb, tb2, p, grid, stream);
-  else if (g.a_mn && !g.b_mn)  e = launch_gemm<true, false>(ta, tb, tb2, p, grid, stream);
-  else                         e = launch_gemm<true, true>(ta, tb, tb2, p, grid, stream);
+  if (!g.a_mn && !g.b_mn)      e = launch_gemm<false, false>(ta, tb, tb2, tc, tc2, p, grid, stream);
+  else if (!g.a_mn && g.b_mn)  e = launch_gemm<false, true>(ta, tb, tb2, tc, tc2, p, grid, stream);
+  else if (g.a_mn && !g.b_mn)  e = launch_gemm<true, false>(ta, tb, tb2, tc, tc2, p, grid, stream);
+  else                         e = launch_gemm<true, true>(ta, tb, tb2, tc, tc2, p, grid, stream);
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }
 

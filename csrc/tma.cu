@@ -68,4 +68,20 @@ int make_tmap_3d(CUtensorMap* map, const void* ptr, uint64_t d0, uint64_t d1, ui
   return r == CUDA_SUCCESS ? 0 : (int)r;
 }
 
+// Map of an output matrix (bf16 or fp32) of `planes` planes of [rows, cols], for stores of 32 rows x 128 bytes.
+int make_tmap_out(CUtensorMap* map, const void* ptr, uint64_t cols, uint64_t rows, uint64_t planes, uint64_t ld_elems,
+                  uint64_t plane_elems, int elem_bytes) {
+  EncodeTiledFn fn = encode_tiled_fn();
+  if (!fn) return -1;
+  bind_context_once();
+  cuuint64_t dims[3] = {cols, rows, planes};
+  cuuint64_t strides[2] = {ld_elems * elem_bytes, plane_elems * elem_bytes};
+  cuuint32_t box[3] = {(cuuint32_t)(128 / elem_bytes), 32, 1};
+  cuuint32_t estr[3] = {1, 1, 1};
+  CUtensorMapDataType dt = elem_bytes == 2 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32;
+  CUresult r = fn(map, dt, 3, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                  CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : (int)r;
+}
+
 }  // namespace tpb
