@@ -47,6 +47,7 @@ struct GemmParams {
   long long ldc2;
   int b_split;       // EPI_SWIGLU: column of c2 where the "up" half starts (= F)
   int b2_off;        // EPI_SWIGLU: row/column offset of the "up" half inside the second B map
+  int kb_b2;         // k-blocks from this one on take B from the second map (its k-block kb - kb_b2); INT_MAX: none
   float alpha;
   int epi;
   int group_m;       // rasterisation: m-tiles per group
@@ -431,6 +432,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           uint8_t* sA = smem + stage * SBYTES;
           uint8_t* sB = sA + A_BYTES;
           const int k0 = kb * BK;
+          // contraction over [A1 | A2] with B in two tensors (the input gradient of separate gate and up weights)
+          const bool second_b = kb >= p.kb_b2;
+          const CUtensorMap* mB = second_b ? &tmB2 : &tmB;
+          const int kB = second_b ? k0 - p.kb_b2 * BK : k0;
           if (PAIR) {
             // Both CTAs' bytes are counted on the even CTA's barrier, which alone expects them.
             const uint32_t bar = map_to_cta(smem_u32(&full[stage]), 0);
@@ -443,13 +448,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             }
             // this CTA's half of B: rows/columns [n0 + rank * 128, +128) (for SwiGLU the odd CTA
             // takes the "up" half)
-            const CUtensorMap* mb = (swiglu && rank == 1) ? &tmB2 : &tmB;
+            const CUtensorMap* mb = (swiglu && rank == 1) ? &tmB2 : mB;
             const int nb = (swiglu && rank == 1) ? p.b2_off + n0 : n0 + rank * 128;
             if (!B_MN) {
-              tma_load_3d_pair(sB, mb, bar, k0, nb, ez);
+              tma_load_3d_pair(sB, mb, bar, kB, nb, ez);
             } else {
 #pragma unroll
-              for (int c = 0; c < 2; ++c) tma_load_3d_pair(sB + c * 8192, mb, bar, nb + c * 64, k0, ez);
+              for (int c = 0; c < 2; ++c) tma_load_3d_pair(sB + c * 8192, mb, bar, nb + c * 64, kB, ez);
             }
           } else {
           mbar_expect_tx(&full[stage], STAGE_BYTES);
@@ -463,15 +468,15 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           if (!B_MN) {
             // two boxes {64 k, 128 rows}; for SwiGLU the second one comes from the "up" half
             // (with two B maps the "up" half is the same rows of the second tensor)
-            tma_load_3d(sB, &tmB, &full[stage], k0, n0, ez);
-            tma_load_3d(sB + 16384, &tmB2, &full[stage], k0, swiglu ? p.b2_off + n0 : n0 + 128, ez);
+            tma_load_3d(sB, mB, &full[stage], kB, n0, ez);
+            tma_load_3d(sB + 16384, swiglu ? &tmB2 : mB, &full[stage], kB, swiglu ? p.b2_off + n0 : n0 + 128, ez);
           } else {
 #pragma unroll
             for (int c = 0; c < BN / 64; ++c) {
               if (swiglu && c >= 2)
                 tma_load_3d(sB + c * 8192, &tmB2, &full[stage], p.b2_off + n0 + (c - 2) * 64, k0, ez);
               else
-                tma_load_3d(sB + c * 8192, &tmB, &full[stage], n0 + c * 64, k0, ez);
+                tma_load_3d(sB + c * 8192, mB, &full[stage], n0 + c * 64, kB, ez);
             }
           }
           }
@@ -922,6 +927,9 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   if (g.mode == 2 && !(g.a_mn && g.b_mn)) return -2;
   if (g.mode == 1 && g.a_mn) return -2;
   const bool two_b = swiglu && g.B2 != nullptr && g.B2 != g.B;
+  const bool cat_k = !swiglu && g.B2 != nullptr;    // B = [B | B2] along the contraction, half of K each
+  if (cat_k && (g.K % (2 * BK))) return -2;
+  const int k_one = cat_k ? g.K / 2 : g.K;
   const int b_extent = two_b ? g.N / 2 : g.N;       // rows (K-major) or columns (MN-major) of one B tensor
   const int b_experts = g.mode == 1 ? g.E : 1;
   CUtensorMap ta, tb, tb2;
@@ -929,14 +937,14 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   if (!g.a_mn) r = make_tmap_2d(&ta, g.A, g.K, g.M, g.lda, 64, 128, 2);
   else         r = make_tmap_2d(&ta, g.A, g.M, g.K, g.lda, 64, 64, 2);
   if (r) return r < 0 ? -3 : -4;
-  const uint64_t estride = b_experts > 1 ? (uint64_t)g.b_expert_stride : (uint64_t)g.ldb * (g.b_mn ? g.K : b_extent);
+  const uint64_t estride = b_experts > 1 ? (uint64_t)g.b_expert_stride : (uint64_t)g.ldb * (g.b_mn ? k_one : b_extent);
   auto make_b = [&](CUtensorMap* m, const void* ptr) {
-    return !g.b_mn ? make_tmap_3d(m, ptr, g.K, b_extent, b_experts, g.ldb, estride, 64, 128)
-                   : make_tmap_3d(m, ptr, b_extent, g.K, b_experts, g.ldb, estride, 64, 64);
+    return !g.b_mn ? make_tmap_3d(m, ptr, k_one, b_extent, b_experts, g.ldb, estride, 64, 128)
+                   : make_tmap_3d(m, ptr, b_extent, k_one, b_experts, g.ldb, estride, 64, 64);
   };
   r = make_b(&tb, g.B);
   if (r) return r < 0 ? -3 : -5;
-  if (two_b) {
+  if (two_b || cat_k) {
     r = make_b(&tb2, g.B2);
     if (r) return r < 0 ? -3 : -5;
   } else {
@@ -965,6 +973,7 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   p.c2 = g.c2; p.ldc2 = g.ldc2;
   p.b_split = g.N / 2;
   p.b2_off = two_b ? 0 : g.N / 2;
+  p.kb_b2 = cat_k ? k_one / BK : 0x7fffffff;
   p.alpha = g.alpha;
   p.epi = g.epi;
   p.status = status_block();

@@ -261,7 +261,8 @@ def grouped_gemm_rows(a, b, plan: DispatchPlan, *, b_mn: bool, b2=None, epi=_lib
                       n_total=None):
   """out[rows of e] = a[rows of e] @ B[e]^T.  ``b``: [E, N, K] (``b_mn=False``) or [E, K, N]
   (``b_mn=True``).  With ``epi=EPI_SWIGLU``: ``b`` = gate, ``b2`` = up (or ``b`` holds both
-  halves along N when ``b2`` is None)."""
+  halves along N when ``b2`` is None).  With other epilogues ``b2`` continues ``b`` along K: ``a`` then
+  has 2K columns."""
   m, k = a.shape
   e = b.shape[0]
   n_one = b.shape[2] if b_mn else b.shape[1]
@@ -278,6 +279,16 @@ def grouped_gemm_rows(a, b, plan: DispatchPlan, *, b_mn: bool, b2=None, epi=_lib
                                    stream_ptr())
   check(rc, f"grouped_gemm rows M={m} N={n} K={k} E={e}")
   return out
+
+
+def grouped_dgrad_gate_up(dgu, w_gate, w_up, plan: DispatchPlan):
+  """d_xg = dgu[:, :F] @ Wg[e]^T + dgu[:, F:] @ Wu[e]^T as one contraction over 2F (one fp32 sum, one
+  rounding, no second pass over d_xg)."""
+  f = w_gate.shape[2]
+  if f % 64 == 0 and dgu.is_contiguous():
+    return grouped_gemm_rows(dgu, w_gate, plan, b_mn=False, b2=w_up)
+  d_xg = grouped_gemm_rows(dgu[:, :f], w_gate, plan, b_mn=False)
+  return grouped_gemm_rows(dgu[:, f:], w_up, plan, b_mn=False, epi=_lib.EPI_BF16_ACC, out=d_xg)
 
 
 def grouped_gemm_wgrad(a_rows, b_rows, plan: DispatchPlan, out, accumulate: bool):
@@ -348,8 +359,7 @@ class _GroupedMLPFn(torch.autograd.Function):
       g_up = None
     else:
       dg, du = dgu[:, :f], dgu[:, f:]
-      d_xg = grouped_gemm_rows(dg, w_gate, plan, b_mn=False)
-      grouped_gemm_rows(du, w_up, plan, b_mn=False, epi=_lib.EPI_BF16_ACC, out=d_xg)
+      d_xg = grouped_dgrad_gate_up(dgu, w_gate, w_up, plan)
       g_gate = _deliver_wgrad(w_gate, lambda out, acc: grouped_gemm_wgrad(xg, dg, plan, out, acc))
       g_up = _deliver_wgrad(w_up, lambda out, acc: grouped_gemm_wgrad(xg, du, plan, out, acc))
     dx = combine_rows(d_xg, plan.dest, None) if ctx.needs_input_grad[0] else None

@@ -230,8 +230,7 @@ class _EPGroupedMLPFn(torch.autograd.Function):
         g_up = None
       else:
         dg, du = dgu[:, :f], dgu[:, f:]
-        d_xg = moe_ops.grouped_gemm_rows(dg, w_gate, plan, b_mn=False)
-        moe_ops.grouped_gemm_rows(du, w_up, plan, b_mn=False, epi=_lib.EPI_BF16_ACC, out=d_xg)
+        d_xg = moe_ops.grouped_dgrad_gate_up(dgu, w_gate, w_up, plan)
         g_gate = deliver(w_gate, lambda out, acc: moe_ops.grouped_gemm_wgrad(xg, dg, plan, out, acc))
         g_up = deliver(w_up, lambda out, acc: moe_ops.grouped_gemm_wgrad(xg, du, plan, out, acc))
     else:
