@@ -219,6 +219,12 @@ int tpb_grouped_gemm_skinny_bf16(const void* x, const void* w, const void* w2, v
                                  long long ldx, long long ldw, long long w_stride, long long ldc, int w_mn, int epi,
                                  const int* tile_expert, int experts_hit, int nt, void* stream);
 
+// ---- latent attention: k = [kv[:dn] | rot], v = kv[dn:] per head, and the gradients (mla_pack.cu)
+int tpb_mla_pack(const void* kv, const void* rot, long long rot_ld, void* k, void* v, long long tokens, int H, int dn,
+                 int dr, int dv, void* stream);
+int tpb_mla_unpack(const void* dk, const void* dv_, void* dkv, void* drot, long long tokens, int H, int dn, int dr, int dv,
+                   void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -1,0 +1,35 @@
+"""Key / value layout passes of latent attention."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from torchprime_b200.ops import functional as ops
+
+
+@pytest.mark.parametrize("b,s,heads,dn,dr,dv", [(1, 1, 1, 8, 8, 8), (2, 37, 16, 128, 64, 128), (1, 5, 3, 24, 16, 40),
+                                                (1, 300, 128, 128, 64, 128)])
+def test_mla_pack(cuda_lib, b, s, heads, dn, dr, dv):
+  torch.manual_seed(s)
+  kv = torch.randn(b, s, heads * (dn + dv), device="cuda", dtype=torch.bfloat16, requires_grad=True)
+  rot = torch.randn(b, s, dr, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+  kk, v = ops.mla_pack(kv, rot, heads, dn, dv)
+  kv4 = kv.view(b, s, heads, dn + dv)
+  assert torch.equal(v, kv4[..., dn:]) and kk.is_contiguous() and v.is_contiguous()
+  assert torch.equal(kk, torch.cat([kv4[..., :dn], rot[:, :, None].expand(b, s, heads, dr)], -1))
+  dk, dv_ = torch.randn_like(kk), torch.randn_like(v)
+  dkv, drot = torch.autograd.grad([kk, v], [kv, rot], [dk, dv_])
+  assert torch.equal(dkv.view_as(kv4), torch.cat([dk[..., :dn], dv_], -1))
+  want = dk[..., dn:].double().sum(2)
+  assert bool(((drot.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6 * heads * 4).all())
+
+
+def test_latent_split(cuda_lib):
+  x = torch.randn(2, 9, 48, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+  a, b = ops.latent_split(x, 32)
+  assert torch.equal(torch.cat([a, b], -1), x)
+  (g,) = torch.autograd.grad([a, b], [x], [torch.ones_like(a), 2 * torch.ones_like(b)])
+  assert bool((g[..., :32] == 1).all()) and bool((g[..., 32:] == 2).all())
+  (g,) = torch.autograd.grad(ops.latent_split(x, 32)[1].sum(), x)
+  assert bool((g[..., :32] == 0).all()) and bool((g[..., 32:] == 1).all())

@@ -81,26 +81,26 @@ class DeepseekInferenceEngine:
                         interleaved=attn.rope_interleave)
     ckv = ops.rope_slices(ckv, self.cos, self.sin, 1, dr, s, col0=c, head_stride=dr, pos=pos,
                           interleaved=attn.rope_interleave)
-    latent = attn.kv_a_layernorm(ckv[..., :c].contiguous())
-    k_rot = ckv[..., c:]
+    latent, k_rot = ops.latent_split(ckv, c)
+    latent = norm(latent)
     q4 = q.view(b, s, h, dn + dr)
-    causal = None
-    if s > 1:
+
+    def mask(scores):          # keys after a query's own position
+      if s == 1:
+        return scores
       t = torch.arange(end, device=x.device)
       causal = t[None, :] > (start + torch.arange(s, device=x.device))[:, None]          # [s, end]
+      return scores.masked_fill(causal[None, :, None, :], float("-inf"))
+
     if self.attn_impl == "naive":
-      kv = ops.linear(latent, attn.kv_b_proj.weight).view(b, s, h, dn + dv)
-      k = torch.cat([kv[..., :dn], k_rot[:, :, None, :].expand(b, s, h, dr)], dim=-1)
-      v = kv[..., dn:]
+      k, v = ops.mla_pack(ops.linear(latent, attn.kv_b_proj.weight), k_rot, h, dn, dv)
       self.k_cache[li][:b, start:end] = k
       self.v_cache[li][:b, start:end] = v
       if start == 0 and x.is_cuda and s >= 128:
-        o = ops.attention(q4, k.contiguous(), v.contiguous(), causal=True, scale=attn.scaling)
+        o = ops.attention(q4, k, v, causal=True, scale=attn.scaling)
       else:
         kc, vc = self.k_cache[li][:b, :end], self.v_cache[li][:b, :end]
-        scores = torch.einsum("bshd,bthd->bsht", q4.float(), kc.float()) * attn.scaling
-        if causal is not None:
-          scores = scores.masked_fill(causal[None, :, None, :], float("-inf"))
+        scores = mask(torch.einsum("bshd,bthd->bsht", q4.float(), kc.float()) * attn.scaling)
         o = torch.einsum("bsht,bthd->bshd", scores.softmax(-1), vc.float()).to(x.dtype)
     else:
       w = attn.kv_b_proj.weight.view(h, dn + dv, c)
@@ -108,10 +108,8 @@ class DeepseekInferenceEngine:
       self.pe_cache[li][:b, start:end] = k_rot
       q_abs = torch.einsum("bshd,hdc->bshc", q4[..., :dn].float(), w[:, :dn].float())
       lc, pc = self.kv_cache[li][:b, :end].float(), self.pe_cache[li][:b, :end].float()
-      scores = (torch.einsum("bshc,btc->bsht", q_abs, lc)
-                + torch.einsum("bshr,btr->bsht", q4[..., dn:].float(), pc)) * attn.scaling
-      if causal is not None:
-        scores = scores.masked_fill(causal[None, :, None, :], float("-inf"))
+      scores = mask((torch.einsum("bshc,btc->bsht", q_abs, lc)
+                     + torch.einsum("bshr,btr->bsht", q4[..., dn:].float(), pc)) * attn.scaling)
       o_lat = torch.einsum("bsht,btc->bshc", scores.softmax(-1), lc)
       o = torch.einsum("bshc,hdc->bshd", o_lat, w[:, dn:].float()).to(x.dtype)
     o = o.reshape(b, s, h * dv)

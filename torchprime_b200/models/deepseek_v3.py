@@ -199,12 +199,10 @@ class DeepseekV3Attention(nn.Module):
       ckv = ops.linear(x, self.kv_a_proj_with_mqa.weight, bias=self.kv_a_proj_with_mqa.bias)
       ckv = ops.rope_slices(ckv, rope_cos, rope_sin, 1, dr, s, col0=self.kv_lora_rank, head_stride=dr,
                             pos=position_ids, interleaved=self.rope_interleave)
-      k_lat, k_rot = ckv[..., : self.kv_lora_rank], to_tp(ckv[..., self.kv_lora_rank:])
-      kv = ops.linear(to_tp(self.kv_a_layernorm(k_lat.contiguous())), self.kv_b_proj.weight).view(b, s, h, dn + dv)
-      k_nope, v = kv[..., :dn], kv[..., dn:]
-      k = torch.cat([k_nope, k_rot[:, :, None, :].expand(b, s, h, dr)], dim=-1)
+      k_lat, k_rot = ops.latent_split(ckv, self.kv_lora_rank)
+      kv = ops.linear(to_tp(self.kv_a_layernorm(k_lat)), self.kv_b_proj.weight)
+      k, v = ops.mla_pack(kv, to_tp(k_rot), h, dn, dv)
       q4 = q.view(b, s, h, dn + dr)
-      v = v.contiguous()
       if cp is not None:
         o = cp.attention(q4, k, v, segment_ids=segment_ids, scale=self.scaling)
       elif self.attention_kernel is None and not x.is_cuda:

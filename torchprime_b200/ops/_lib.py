@@ -75,6 +75,8 @@ def _declare(L):
     "tpb_embedding_bwd": [P, P, P, I, I, LL, LL, I, P],
     "tpb_cast_f32_to_bf16": [P, P, LL, F, I, P],
     "tpb_scale_cast_bf16": [P, P, LL, P, P],
+    "tpb_mla_pack": [P, P, LL, P, P, LL, I, I, I, I, P],
+    "tpb_mla_unpack": [P, P, P, P, LL, I, I, I, I, P],
   }
   for name, args in sigs.items():
     fn = getattr(L, name, None)

@@ -739,6 +739,54 @@ def attention_qkv(qkv, hq, hkv, d, causal=True, scale=None, window=None, q_segme
                    q_positions=q_positions)
 
 
+# --------------------------------------------------------------------------- latent attention layout
+class _LatentSplitFn(torch.autograd.Function):
+  """The latent and the rotary key of a compressed projection as two contiguous tensors.  A single node,
+  so that the projection's gradient is one concatenation and not two zero-filled slices and their sum."""
+
+  @staticmethod
+  def forward(ctx, ckv, c):
+    return ckv[..., :c].contiguous(), ckv[..., c:].contiguous()
+
+  @staticmethod
+  def backward(ctx, dlat, drot):
+    return torch.cat([dlat, drot], dim=-1), None
+
+
+def latent_split(ckv, c):
+  """(ckv[..., :c], ckv[..., c:]), both contiguous."""
+  if use_kernels(ckv):
+    return _LatentSplitFn.apply(ckv, c)
+  return ckv[..., :c].contiguous(), ckv[..., c:]
+
+
+class _MlaPackFn(torch.autograd.Function):
+  @staticmethod
+  def forward(ctx, kv, rot, heads, dn, dv):
+    from . import kernels as k
+    ctx.args = (heads, dn, dv)
+    return k.mla_pack(kv, rot, heads, dn, dv)
+
+  @staticmethod
+  def backward(ctx, dk, dv_):
+    from . import kernels as k
+    heads, dn, dv = ctx.args
+    dkv, drot = k.mla_unpack(dk.contiguous(), dv_.contiguous(), heads, dn, dv)
+    return dkv, drot, None, None, None
+
+
+def mla_pack(kv, rot, heads, dn, dv):
+  """Keys [B,S,heads,dn+dr] and values [B,S,heads,dv] from the up-projection ``kv`` [B,S,heads*(dn+dv)] and the
+  rotary key ``rot`` [B,S,dr] that all heads share."""
+  b, s, dr = rot.shape
+  if (use_kernels(kv, rot) and dn % 8 == 0 and dr % 8 == 0 and dv % 8 == 0 and dr <= 512 and kv.is_contiguous()
+      and rot.is_contiguous() and kv.data_ptr() % 16 == 0 and rot.data_ptr() % 16 == 0):
+    return _MlaPackFn.apply(kv, rot, heads, dn, dv)
+  kv = kv.view(b, s, heads, dn + dv)
+  k = torch.cat([kv[..., :dn], rot[:, :, None, :].expand(b, s, heads, dr)], dim=-1)
+  return k, kv[..., dn:].contiguous()
+
+
 # --------------------------------------------------------------------------- lm head + CE
 class _LinearCrossEntropyFn(torch.autograd.Function):
   """Chunked lm_head + softmax cross entropy.  The forward pass also produces the

@@ -185,3 +185,23 @@ def scale_cast_bf16(src, scale):
   out = torch.empty(src.shape, dtype=torch.bfloat16, device=src.device)
   check(lib().tpb_scale_cast_bf16(ptr(src), ptr(out), src.numel(), ptr(scale), stream_ptr()), "scale_cast_bf16")
   return out
+
+
+def mla_pack(kv, rot, heads, dn, dv):
+  b, s, dr = rot.shape
+  assert kv.is_contiguous() and rot.is_contiguous() and kv.shape == (b, s, heads * (dn + dv))
+  k = torch.empty(b, s, heads, dn + dr, dtype=kv.dtype, device=kv.device)
+  v = torch.empty(b, s, heads, dv, dtype=kv.dtype, device=kv.device)
+  check(lib().tpb_mla_pack(ptr(kv), ptr(rot), dr, ptr(k), ptr(v), b * s, heads, dn, dr, dv, stream_ptr()), "mla_pack")
+  return k, v
+
+
+def mla_unpack(dk, dv_, heads, dn, dv):
+  """Gradients of :func:`mla_pack`: (dkv [B,S,heads*(dn+dv)], drot [B,S,dr])."""
+  b, s, _, dqk = dk.shape
+  assert dk.is_contiguous() and dv_.is_contiguous()
+  dkv = torch.empty(b, s, heads * (dn + dv), dtype=dk.dtype, device=dk.device)
+  drot = torch.empty(b, s, dqk - dn, dtype=dk.dtype, device=dk.device)
+  check(lib().tpb_mla_unpack(ptr(dk), ptr(dv_), ptr(dkv), ptr(drot), b * s, heads, dn, dqk - dn, dv, stream_ptr()),
+        "mla_unpack")
+  return dkv, drot
