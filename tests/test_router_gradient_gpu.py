@@ -1,0 +1,43 @@
+"""Router logits in fp32 and the gradient of the routing weights."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+from torchprime_b200.ops import functional as ops
+from torchprime_b200.ops import moe
+
+
+@pytest.mark.parametrize("E,K", [(8, 2), (33, 3), (64, 6), (256, 8), (5, 5), (4, 1)])
+@pytest.mark.parametrize("mode", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("norm", [True, False])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_router_backward(cuda_lib, E, K, mode, norm, dtype):
+  """Weights and scores both carry gradients; fp64 autograd through the same choice is the oracle."""
+  torch.manual_seed(E)
+  lg = torch.randn(77, E, device="cuda").to(dtype).requires_grad_(True)
+  w, idx, sc = moe.router_topk(lg, K, mode=mode, norm_topk=norm, scale=1.7)
+  gw, gs = torch.randn_like(w), torch.randn_like(sc)
+  x = lg.detach().double().requires_grad_(True)
+  s = torch.softmax(x, -1) if mode == "softmax" else torch.sigmoid(x)
+  wr = s.gather(1, idx.long())
+  if norm:
+    wr = wr / wr.sum(-1, keepdim=True)
+  wr = wr * 1.7
+  tol = 2.0 ** -8 if dtype == torch.bfloat16 else 2e-6
+  for outs, refs, grads in (([w, sc], [wr, s], [gw, gs]), ([w], [wr], [gw]), ([sc], [s], [gs])):
+    (got,) = torch.autograd.grad(outs, lg, grads, retain_graph=True)
+    (want,) = torch.autograd.grad(refs, x, [g.double() for g in grads], retain_graph=True)
+    assert got.dtype == dtype
+    assert bool(((got.double() - want).abs() <= tol * want.abs() + 5e-6).all()), (got - want).abs().max()
+
+
+def test_linear_f32_gradients(cuda_lib):
+  x = torch.randn(50, 256, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+  w = torch.randn(64, 256, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+  y = ops.linear_f32(x, w)
+  assert y.dtype == torch.float32
+  dy = torch.randn_like(y)
+  dx, dw = torch.autograd.grad(y, (x, w), dy)
+  assert torch.equal(dx, (dy @ w.float()).to(torch.bfloat16)) and torch.equal(dw, (dy.t() @ x.float()).to(torch.bfloat16))

@@ -78,7 +78,7 @@ class DeepseekV3TopkRouter(nn.Module):
     self.register_buffer("e_score_correction_bias", torch.zeros(self.n_routed_experts, device="cpu"))
 
   def forward(self, x):
-    logits = F.linear(x.reshape(-1, x.shape[-1]).float(), self.weight.float())
+    logits = ops.linear_f32(x.reshape(-1, x.shape[-1]), self.weight)
     bias = self.e_score_correction_bias
     if bias.device != logits.device:
       bias = bias.to(logits.device)

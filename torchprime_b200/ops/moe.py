@@ -28,6 +28,7 @@ P, I, LL, FL = c_void_p, c_int, c_longlong, c_float
 _lib.register_signature("tpb_grouped_gemm_bf16", [P, P, P, P, I, I, I, I, LL, LL, LL, LL, I, I, I, FL, P, LL, I, P, P,
                                                   LL, I, P])
 _lib.register_signature("tpb_router_topk", [P, I, P, P, P, P, I, I, I, I, I, I, I, FL, P])
+_lib.register_signature("tpb_router_bwd", [P, I, P, P, P, P, I, I, I, I, I, FL, P])
 _lib.register_signature("tpb_moe_plan", [P, I, I, I, I, I, P, P, P, P, P, P, P])
 _lib.register_signature("tpb_moe_gather", [P, P, P, P, LL, I, P])
 _lib.register_signature("tpb_moe_gather_real", [P, P, P, LL, I, P])
@@ -44,43 +45,44 @@ def _kernels_ok(*ts) -> bool:
 
 
 # ----------------------------------------------------------------------------- routing
+def _router_forward(lg, bias, k, mode, n_group, topk_group, norm_topk, scale):
+  t, e = lg.shape
+  w = torch.empty(t, k, dtype=torch.float32, device=lg.device)
+  idx = torch.empty(t, k, dtype=torch.int32, device=lg.device)
+  scores = torch.empty(t, e, dtype=torch.float32, device=lg.device)
+  b = bias.float().contiguous() if bias is not None else None
+  check(lib().tpb_router_topk(ptr(lg), int(lg.dtype == torch.bfloat16), ptr(b), ptr(w), ptr(idx), ptr(scores), t, e,
+                              k, mode, n_group, topk_group, int(norm_topk), float(scale), stream_ptr()),
+        "router_topk")
+  return w, idx, scores
+
+
 class _RouterFn(torch.autograd.Function):
-  """Kernel forward; the (tiny) backward re-derives the weights with PyTorch ops on the
-  selected experts so gradients reach the gate."""
+  """Kernels both ways; the backward re-derives the scores from the logits."""
 
   @staticmethod
   def forward(ctx, logits, bias, k, mode, n_group, topk_group, norm_topk, scale):
-    t, e = logits.shape
     lg = logits.contiguous()
-    w = torch.empty(t, k, dtype=torch.float32, device=logits.device)
-    idx = torch.empty(t, k, dtype=torch.int32, device=logits.device)
-    scores = torch.empty(t, e, dtype=torch.float32, device=logits.device)
-    b = bias.float().contiguous() if bias is not None else None
-    check(lib().tpb_router_topk(ptr(lg), int(lg.dtype == torch.bfloat16), ptr(b), ptr(w), ptr(idx), ptr(scores), t, e,
-                                k, mode, n_group, topk_group, int(norm_topk), float(scale), stream_ptr()),
-          "router_topk")
-    ctx.save_for_backward(logits, idx)
+    w, idx, scores = _router_forward(lg, bias, k, mode, n_group, topk_group, norm_topk, scale)
+    ctx.save_for_backward(lg, idx)
+    ctx.set_materialize_grads(False)
     ctx.args = (mode, norm_topk, scale)
     ctx.mark_non_differentiable(idx)
     return w, idx, scores
 
   @staticmethod
   def backward(ctx, dw, _didx, dscores):
-    logits, idx = ctx.saved_tensors
+    lg, idx = ctx.saved_tensors
     mode, norm_topk, scale = ctx.args
-    with torch.enable_grad():
-      lg = logits.detach().float().requires_grad_(True)
-      s = torch.softmax(lg, dim=-1) if mode == 0 else torch.sigmoid(lg)
-      w = s.gather(1, idx.long())
-      if norm_topk:
-        w = w / (w.sum(-1, keepdim=True) + (0.0 if mode == 0 else 1e-20))
-      w = w * scale
-      outs, grads = [w], [dw]
-      if dscores is not None:
-        outs.append(s)
-        grads.append(dscores)
-      (g,) = torch.autograd.grad(outs, lg, grads)
-    return g.to(logits.dtype), None, None, None, None, None, None, None
+    if dw is None and dscores is None:
+      return (None,) * 8
+    t, e = lg.shape
+    dw = dw.float().contiguous() if dw is not None else None
+    dscores = dscores.float().contiguous() if dscores is not None else None
+    g = torch.empty_like(lg)
+    check(lib().tpb_router_bwd(ptr(lg), int(lg.dtype == torch.bfloat16), ptr(idx), ptr(dw), ptr(dscores), ptr(g), t, e,
+                               idx.shape[1], mode, int(norm_topk), float(scale), stream_ptr()), "router_bwd")
+    return g, None, None, None, None, None, None, None
 
 
 def router_topk(logits, k, mode="softmax", bias=None, n_group=1, topk_group=1, norm_topk=True, scale=1.0):
@@ -91,6 +93,9 @@ def router_topk(logits, k, mode="softmax", bias=None, n_group=1, topk_group=1, n
   m = 0 if mode == "softmax" else 1
   e = logits.shape[-1]
   if logits.is_cuda and _kernels_ok() and e <= 256 and logits.dtype in (torch.float32, torch.bfloat16):
+    from .functional import inference_only
+    if inference_only():
+      return _router_forward(logits.contiguous(), bias, k, m, n_group, topk_group, norm_topk, scale)
     return _RouterFn.apply(logits, bias, k, m, n_group, topk_group, norm_topk, scale)
   if m == 0:
     w, idx, s = ref.router_softmax_topk(logits, k, renormalize=norm_topk)
