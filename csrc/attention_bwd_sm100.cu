@@ -843,6 +843,641 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   }
 }
 
+// ------------------------------------------------------------------------------------------
+// Query / key head dim 192 with value dim 128 (latent attention).
+//
+// The same two kernels with the tiles that 512 TMEM columns and 227 KB of shared memory leave room for:
+//   dK/dV: dK takes 192 columns and dV 128, so score tiles are 128 keys x 64 queries; S^T is double
+//          buffered and the score product of step i + 1 runs beside both compute phases of step i.
+//          TMEM: dK [0,192), dV [192,320), S^T [320,448), dP^T [448,512).
+//          (A 128 x 64 MMA is bound by operand fetch at 2/3 of the tensor rate; with 128 x 128 tiles the
+//          accumulators and two score tiles would need 576 columns.)
+//   dQ:    128 x 128 tiles, one S buffer: S(j + 1) is issued as soon as the compute warps hold S(j) in
+//          registers.  TMEM: dQ [0,192), S [192,320), dP [320,448).
+// One row of 2048 tokens, 16 heads, causal: dK/dV 69, dQ 42, delta 8 us.  (torch's scaled_dot_product_attention, used
+// here before: backward 90 us after running its own forward again, 41 us, and three copies.)
+// ------------------------------------------------------------------------------------------
+constexpr int W_D = 192;                       // query / key head dim
+constexpr int W_QT = 64;                       // query rows per step of the dK/dV kernel
+constexpr int W_STAGES = 3;                    // its Q and dO rings
+constexpr int W_MAX_TILES = 2048;              // its query-tile table: 131,072 queries
+constexpr int W_K_BYTES = BWD_T * W_D * 2;     // 48 KB: 128 rows of Q or K
+constexpr int W_Q_BYTES = W_QT * W_D * 2;      // 24 KB
+constexpr int W_DO_BYTES = W_QT * BWD_D * 2;   // 16 KB
+
+namespace wkv {
+constexpr int OFF_K = 0;
+constexpr int OFF_V = OFF_K + W_K_BYTES;
+constexpr int OFF_Q = OFF_V + TILE_BYTES;
+constexpr int OFF_DO = OFF_Q + W_STAGES * W_Q_BYTES;
+constexpr int OFF_AUX = OFF_DO + W_STAGES * W_DO_BYTES;      // per Q stage: lse2[64], delta[64], qpos[64], qseg[64]
+constexpr int AUX_STAGE = 4 * W_QT * 4;
+constexpr int OFF_TILES = OFF_AUX + W_STAGES * AUX_STAGE;
+constexpr int OFF_SEGONE = OFF_TILES + 2 * W_MAX_TILES * 4;
+constexpr int OFF_BAR = OFF_SEGONE + W_MAX_TILES;
+constexpr int TOTAL = OFF_BAR + 256 + 1024;
+static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
+constexpr int T_DK = 0, T_DV = 192, T_S = 320, T_DP = 448;
+}  // namespace wkv
+
+namespace wdq {
+constexpr int OFF_Q = 0;
+constexpr int OFF_DO = OFF_Q + W_K_BYTES;
+constexpr int OFF_K = OFF_DO + TILE_BYTES;
+constexpr int OFF_V = OFF_K + 2 * W_K_BYTES;
+constexpr int OFF_BAR = OFF_V + TILE_BYTES;
+constexpr int TOTAL = OFF_BAR + 256 + 1024;
+static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
+constexpr int T_DQ = 0, T_S = 192, T_DP = 320;
+}  // namespace wdq
+
+// Columns [c0, c0 + 32 * n) of one fp32 TMEM accumulator row times `mul` as bf16.
+__device__ __forceinline__ void store_acc_cols(uint32_t tsrc, int c0, int n, __nv_bfloat16* dst, bool have, bool write,
+                                               float mul) {
+#pragma unroll 1
+  for (int c = c0; c < c0 + 32 * n; c += 32) {
+    uint32_t o[32];
+    if (have) {
+      tmem_ld32(tsrc + c, o);
+      tmem_wait_ld();
+    } else {
+#pragma unroll
+      for (int e = 0; e < 32; ++e) o[e] = 0;
+    }
+    if (write) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        *reinterpret_cast<uint4*>(dst + c + v * 8) = make_uint4(
+            pack_bf16(__uint_as_float(o[8 * v]) * mul, __uint_as_float(o[8 * v + 1]) * mul),
+            pack_bf16(__uint_as_float(o[8 * v + 2]) * mul, __uint_as_float(o[8 * v + 3]) * mul),
+            pack_bf16(__uint_as_float(o[8 * v + 4]) * mul, __uint_as_float(o[8 * v + 5]) * mul),
+            pack_bf16(__uint_as_float(o[8 * v + 6]) * mul, __uint_as_float(o[8 * v + 7]) * mul));
+    }
+  }
+}
+
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
+                       const AttnBwdParams p) {
+  using namespace wkv;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
+  uint64_t* kv_full = bars;
+  uint64_t* q_full = bars + 1;                    // [W_STAGES]
+  uint64_t* q_empty = q_full + W_STAGES;
+  uint64_t* do_full = q_empty + W_STAGES;
+  uint64_t* do_empty = do_full + W_STAGES;
+  uint64_t* s_full = do_empty + W_STAGES;         // [2] S^T of a step is in its buffer
+  uint64_t* p_full = s_full + 2;                  // [2] count 256: P^T written over it
+  uint64_t* dp_full = p_full + 2;
+  uint64_t* ds_full = dp_full + 1;                // count 256: dS^T written
+  uint64_t* acc_done = ds_full + 1;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
+  int* tile_min = reinterpret_cast<int*>(smem + OFF_TILES);
+  int* tile_max = tile_min + W_MAX_TILES;
+  uint8_t* seg_one = smem + OFF_SEGONE;
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int kb = blockIdx.x / (p.Hkv * p.B);      // key-block major: the heaviest blocks first under a causal mask
+  const int hkv = (blockIdx.x / p.B) % p.Hkv, b = blockIdx.x % p.B;
+  const int G = p.Hq / p.Hkv;
+  const int kv0 = kb * BWD_T;
+  const int pos_off = p.Sk - p.Sq;
+  const int n_tiles = (p.Sq + W_QT - 1) / W_QT;   // host guarantees <= W_MAX_TILES
+
+  if (threadIdx.x == 0) {
+    mbar_init(kv_full, 1);
+    for (int i = 0; i < W_STAGES; ++i) {
+      mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1);
+      mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1);
+    }
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 256); }
+    mbar_init(dp_full, 1); mbar_init(ds_full, 256);
+    mbar_init(acc_done, 1);
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  // position range of every query tile; a tile that shares no segment with this key block gets an empty one
+  const int2 kseg_rng = p.kv_rng ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
+  for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
+    const int r0 = t * W_QT, r1 = min(p.Sq, r0 + W_QT);
+    int mn = 0x7fffffff, mx = -0x7fffffff;
+    if (p.q_pos) {
+      for (int r = r0; r < r1; ++r) {
+        const int v = p.q_pos[(long long)b * p.Sq + r];
+        mn = min(mn, v); mx = max(mx, v);
+      }
+    } else {
+      mn = r0 + pos_off; mx = r1 - 1 + pos_off;
+    }
+    if (p.kv_rng) {
+      const int2 qr = p.q_rng[(long long)b * n_tiles + t];   // W_QT == SEG_BLK
+      seg_one[t] = qr.x == qr.y && kseg_rng.x == kseg_rng.y && qr.x == kseg_rng.x;
+      if (qr.y < kseg_rng.x || qr.x > kseg_rng.y) { mn = 0x7fffffff; mx = -0x7fffffff; }
+    }
+    tile_min[t] = mn; tile_max[t] = mx;
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  auto visible = [&](int t) -> bool {
+    if (tile_min[t] > tile_max[t]) return false;
+    if (p.causal && tile_max[t] < kv0) return false;
+    if (p.window > 0 && tile_min[t] - (kv0 + BWD_T - 1) >= p.window) return false;
+    return true;
+  };
+  int n_vis = 0;
+  for (int t = 0; t < n_tiles; ++t) n_vis += visible(t) ? 1 : 0;
+  const int n_steps = n_vis * G;
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ producer
+    if (n_steps > 0) {
+      if (lane == 0) {
+        tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
+        mbar_expect_tx(kv_full, W_K_BYTES + TILE_BYTES);
+        for (int c = 0; c < W_D / 64; ++c)
+          tma_load_3d(smem + OFF_K + c * (BWD_T * 128), &tmK, kv_full, c * 64, b * p.Sk + kv0, hkv);
+        for (int c = 0; c < BWD_D / 64; ++c)
+          tma_load_3d(smem + OFF_V + c * (BWD_T * 128), &tmV, kv_full, c * 64, b * p.Sk + kv0, hkv);
+      }
+      const bool aux_rows = p.q_pos != nullptr || p.q_seg != nullptr;
+      int step = 0;
+      bool ok = true;
+      for (int g = 0; g < G && ok; ++g) {
+        const int hq = hkv * G + g;
+        for (int t = 0; t < n_tiles && ok; ++t) {
+          if (!visible(t)) continue;
+          const int st = step % W_STAGES;
+          const uint32_t ph = ((step / W_STAGES) & 1) ^ 1;
+          const int q0 = t * W_QT;
+          int okw = 1;
+          if (lane == 0) okw = mbar_wait(&q_empty[st], ph, p.status, kTimeoutStageFree, 121) ? 1 : 0;
+          okw = __shfl_sync(0xffffffffu, okw, 0);
+          if (!okw) { ok = false; break; }
+          float* aux = reinterpret_cast<float*>(smem + OFF_AUX + st * AUX_STAGE);
+          int* auxi = reinterpret_cast<int*>(aux);
+          if (aux_rows && !p.aux_bulk) {
+            for (int c = lane; c < W_QT; c += 32) {
+              const int r = min(q0 + c, p.Sq - 1);
+              auxi[2 * W_QT + c] = p.q_pos ? p.q_pos[(long long)b * p.Sq + r] : 0;
+              auxi[3 * W_QT + c] = p.q_seg ? p.q_seg[(long long)b * p.Sq + r] : 0;
+            }
+            __syncwarp();
+          }
+          if (lane == 0) {
+            const uint32_t rows_bytes = (uint32_t)min(W_QT, p.Sq - q0) * 4u;
+            uint32_t tx = W_Q_BYTES + 2 * W_QT * 4;
+            if (aux_rows && p.aux_bulk) tx += (p.q_pos ? rows_bytes : 0u) + (p.q_seg ? rows_bytes : 0u);
+            mbar_expect_tx(&q_full[st], tx);
+            for (int c = 0; c < W_D / 64; ++c)
+              tma_load_3d(smem + OFF_Q + st * W_Q_BYTES + c * (W_QT * 128), &tmQ, &q_full[st], c * 64, b * p.Sq + q0, hq);
+            const long long li = ((long long)b * p.Hq + hq) * p.Sq_pad + q0;
+            bulk_load(aux, p.lse2 + li, W_QT * 4, &q_full[st]);
+            bulk_load(aux + W_QT, p.delta + li, W_QT * 4, &q_full[st]);
+            if (aux_rows && p.aux_bulk) {
+              if (p.q_pos) bulk_load(auxi + 2 * W_QT, p.q_pos + (long long)b * p.Sq + q0, rows_bytes, &q_full[st]);
+              if (p.q_seg) bulk_load(auxi + 3 * W_QT, p.q_seg + (long long)b * p.Sq + q0, rows_bytes, &q_full[st]);
+            }
+            if (mbar_wait(&do_empty[st], ph, p.status, kTimeoutStageFree, 129)) {
+              mbar_expect_tx(&do_full[st], W_DO_BYTES);
+              for (int c = 0; c < BWD_D / 64; ++c)
+                tma_load_3d(smem + OFF_DO + st * W_DO_BYTES + c * (W_QT * 128), &tmdO, &do_full[st], c * 64,
+                            b * p.Sq + q0, hq);
+            } else {
+              okw = 0;
+            }
+          }
+          okw = __shfl_sync(0xffffffffu, okw, 0);
+          if (!okw) { ok = false; break; }
+          ++step;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0 && n_steps > 0) {
+      constexpr uint32_t id_s = make_idesc_bf16(BWD_T, W_QT, false, false);     // S^T, dP^T
+      constexpr uint32_t id_dv = make_idesc_bf16(BWD_T, BWD_D, false, true);    // dV (A in TMEM, B MN-major)
+      constexpr uint32_t id_dk = make_idesc_bf16(BWD_T, W_D, false, true);      // dK
+      const uint32_t dK = kmajor_lo(smem_u32(smem + OFF_K)), dVd = kmajor_lo(smem_u32(smem + OFF_V));
+      const uint32_t aQ0 = smem_u32(smem + OFF_Q), aDO0 = smem_u32(smem + OFF_DO);
+      const uint32_t tDP = tmem_base + T_DP;
+      // k-step k of a K-major tile of `rows` rows in 64-wide blocks, and the TMEM column of a bf16 A operand
+      // whose halves of 32 values lie packed at the start of their own 32 columns
+      auto kstep = [](int rows, int k) { return (uint32_t)(((k >> 2) * (rows * 128) + (k & 3) * 32) >> 4); };
+      auto acol = [](int k) { return (uint32_t)((k >> 1) * 32 + (k & 1) * 8); };
+      auto wait_q = [&](int i) { return mbar_wait(&q_full[i % W_STAGES], (i / W_STAGES) & 1, p.status, kTimeoutTmaFull, 123); };
+      auto wait_do = [&](int i) { return mbar_wait(&do_full[i % W_STAGES], (i / W_STAGES) & 1, p.status, kTimeoutTmaFull, 124); };
+      auto issue_s = [&](int i) -> bool {      // S^T(i) = K Q(i)^T
+        if (!wait_q(i)) return false;
+        tc_fence_after();
+        const uint32_t dQ = kmajor_lo(aQ0 + (i % W_STAGES) * W_Q_BYTES);
+#pragma unroll
+        for (int k = 0; k < W_D / 16; ++k)
+          mma_ss_w(tmem_base + T_S + (i & 1) * W_QT, dK + kstep(BWD_T, k), kDescHi, dQ + kstep(W_QT, k), kDescHi, id_s, k != 0);
+        tc_commit(&s_full[i & 1]);
+        return true;
+      };
+      auto issue_dp = [&](int i) -> bool {     // dP^T(i) = V dO(i)^T
+        if (!wait_do(i)) return false;
+        tc_fence_after();
+        const uint32_t dDO = kmajor_lo(aDO0 + (i % W_STAGES) * W_DO_BYTES);
+#pragma unroll
+        for (int k = 0; k < BWD_D / 16; ++k)
+          mma_ss_w(tDP, dVd + kstep(BWD_T, k), kDescHi, dDO + kstep(W_QT, k), kDescHi, id_s, k != 0);
+        tc_commit(dp_full);
+        return true;
+      };
+      bool ok = mbar_wait(kv_full, 0, p.status, kTimeoutTmaFull, 122);
+      if (ok) ok = issue_s(0) && issue_dp(0);
+      for (int i = 0; i < n_steps && ok; ++i) {
+        const int st = i % W_STAGES;
+        const bool more = i + 1 < n_steps;
+        // its buffer held P^T(i - 1), which dV(i - 1), issued before, has read by then
+        if (more && !issue_s(i + 1)) break;
+        if (!mbar_wait(&p_full[i & 1], (i >> 1) & 1, p.status, kTimeoutSoftmax, 125)) break;
+        tc_fence_after();
+        const uint32_t mDO = smem_desc_lo(aDO0 + st * W_DO_BYTES, W_QT * 128);
+#pragma unroll
+        for (int k = 0; k < W_QT / 16; ++k)    // dV += P^T dO
+          mma_ts_w(tmem_base + T_DV, tmem_base + T_S + (i & 1) * W_QT + acol(k), mDO + mnmajor_k(k), kDescHi, id_dv,
+                   (i | k) != 0);
+        tc_commit(&do_empty[st]);
+        if (!mbar_wait(ds_full, i & 1, p.status, kTimeoutSoftmax, 126)) break;
+        tc_fence_after();
+        const uint32_t mQ = smem_desc_lo(aQ0 + st * W_Q_BYTES, W_QT * 128);
+#pragma unroll
+        for (int k = 0; k < W_QT / 16; ++k)    // dK += dS^T Q
+          mma_ts_w(tmem_base + T_DK, tDP + acol(k), mQ + mnmajor_k(k), kDescHi, id_dk, (i | k) != 0);
+        tc_commit(&q_empty[st]);
+        if (more && !issue_dp(i + 1)) break;
+      }
+      tc_commit(acc_done);
+    }
+  } else {
+    // ------------------------------------------------------------------ compute warps
+    const int qd = warp & 3;
+    const int half = (warp - 2) >> 2;             // which 32 of the 64 query columns
+    const int r_local = qd * 32 + lane;           // key row == TMEM lane
+    const int kp = kv0 + r_local;
+    const bool key_ok = kp < p.Sk;
+    const int kseg = (p.kv_seg && key_ok) ? p.kv_seg[(long long)b * p.Sk + kp] : 0;
+    const uint32_t tb = tmem_base + ((uint32_t)(qd * 32) << 16);
+    const uint32_t tDP = tb + T_DP + half * 32;
+    const int win = p.window > 0 ? p.window : 0x7fffffff;
+    const int cmax = p.causal ? kp : -0x7fffffff;
+    bool ok = true;
+    int step = 0;
+    for (int g = 0; g < G && ok; ++g) {
+      for (int t = 0; t < n_tiles && ok; ++t) {
+        if (!visible(t)) continue;
+        const float* aux = reinterpret_cast<const float*>(smem + OFF_AUX + (step % W_STAGES) * AUX_STAGE);
+        const int* auxi = reinterpret_cast<const int*>(aux);
+        const uint32_t tS = tb + T_S + (step & 1) * W_QT + half * 32;
+        const bool need_mask = !key_ok || (kv0 + BWD_T > p.Sk) || (p.causal && tile_min[t] < kv0 + BWD_T - 1) ||
+                               (p.window > 0 && tile_max[t] - kv0 >= p.window) ||
+                               (p.q_seg != nullptr && !(p.kv_rng && seg_one[t]));
+        // ---- phase 1: P^T = exp2(S^T * c - lse)
+        if (!mbar_wait(&s_full[step & 1], (step >> 1) & 1, p.status, kTimeoutAccFull, 127)) { ok = false; break; }
+        tc_fence_after();
+        uint32_t pk_p[16];
+        {
+          uint32_t s[32];
+          tmem_ld32(tS, s);
+          tmem_wait_ld();
+          const float4* lse4 = reinterpret_cast<const float4*>(aux + half * 32);
+          const int4* qp4 = reinterpret_cast<const int4*>(auxi + 2 * W_QT + half * 32);
+          const int4* qs4 = reinterpret_cast<const int4*>(auxi + 3 * W_QT + half * 32);
+          if (!need_mask) {
+#pragma unroll
+            for (int c4 = 0; c4 < 8; ++c4) {
+              const float4 L = lse4[c4];
+              pk_p[2 * c4] = pack_bf16(exp2f(fmaf(__uint_as_float(s[4 * c4]), p.scale_log2, -L.x)),
+                                       exp2f(fmaf(__uint_as_float(s[4 * c4 + 1]), p.scale_log2, -L.y)));
+              pk_p[2 * c4 + 1] = pack_bf16(exp2f(fmaf(__uint_as_float(s[4 * c4 + 2]), p.scale_log2, -L.z)),
+                                           exp2f(fmaf(__uint_as_float(s[4 * c4 + 3]), p.scale_log2, -L.w)));
+            }
+          } else {
+#pragma unroll
+            for (int c4 = 0; c4 < 8; ++c4) {
+              const float4 L = lse4[c4];
+              const int qn = t * W_QT + pos_off + half * 32 + 4 * c4;   // natural positions
+              const int4 QP = p.q_pos ? qp4[c4] : make_int4(qn, qn + 1, qn + 2, qn + 3);
+              const int4 QS = p.q_seg ? qs4[c4] : make_int4(0, 0, 0, 0);
+              const float l[4] = {L.x, L.y, L.z, L.w};
+              const int qp[4] = {QP.x, QP.y, QP.z, QP.w}, qs[4] = {QS.x, QS.y, QS.z, QS.w};
+              float pv[4];
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                const bool keep = key_ok & (qp[e] >= cmax) & (qp[e] - kp < win) & (qs[e] == kseg);
+                const float pe = exp2f(fmaf(__uint_as_float(s[4 * c4 + e]), p.scale_log2, -l[e]));
+                pv[e] = keep ? pe : 0.f;
+              }
+              pk_p[2 * c4] = pack_bf16(pv[0], pv[1]);
+              pk_p[2 * c4 + 1] = pack_bf16(pv[2], pv[3]);
+            }
+          }
+          tmem_st16(tS, pk_p);
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(&p_full[step & 1]);
+        // ---- phase 2: dS^T = P^T o (dP^T - delta), written over dP^T
+        if (!mbar_wait(dp_full, step & 1, p.status, kTimeoutAccFull, 128)) { ok = false; break; }
+        tc_fence_after();
+        {
+          uint32_t d[32], pk_ds[16];
+          tmem_ld32(tDP, d);
+          tmem_wait_ld();
+          const float4* dlt4 = reinterpret_cast<const float4*>(aux + W_QT + half * 32);
+#pragma unroll
+          for (int c4 = 0; c4 < 8; ++c4) {
+            const float4 Dl = dlt4[c4];
+            pk_ds[2 * c4] = mul_bf16x2(pk_p[2 * c4], pack_bf16(__uint_as_float(d[4 * c4]) - Dl.x,
+                                                               __uint_as_float(d[4 * c4 + 1]) - Dl.y));
+            pk_ds[2 * c4 + 1] = mul_bf16x2(pk_p[2 * c4 + 1], pack_bf16(__uint_as_float(d[4 * c4 + 2]) - Dl.z,
+                                                                       __uint_as_float(d[4 * c4 + 3]) - Dl.w));
+          }
+          tmem_st16(tDP, pk_ds);
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(ds_full);
+        ++step;
+      }
+    }
+    if (ok && n_steps > 0) ok = mbar_wait(acc_done, 0, p.status, kTimeoutAccFull, 130);
+    tc_fence_after();
+    const bool have = ok && n_steps > 0;
+    store_acc_cols(tb + T_DK, half * 96, 3, p.dK + ((long long)b * p.Sk + kp) * p.lddk + (long long)hkv * W_D, have, key_ok,
+                   p.scale);
+    store_acc_cols(tb + T_DV, half * 64, 2, p.dV + ((long long)b * p.Sk + kp) * p.lddv + (long long)hkv * BWD_D, have,
+                   key_ok, 1.f);
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
+__global__ void __launch_bounds__(BWD_THREADS, 1)
+attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
+                      const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
+                      const AttnBwdParams p) {
+  using namespace wdq;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
+  uint64_t* qdo_full = bars;
+  uint64_t* k_full = bars + 1;                    // [2]
+  uint64_t* k_empty = bars + 3;                   // [2]
+  uint64_t* v_full = bars + 5;
+  uint64_t* v_empty = bars + 6;
+  uint64_t* s_full = bars + 7;
+  uint64_t* s_read = bars + 8;                    // count 256: S is in registers
+  uint64_t* dp_full = bars + 9;
+  uint64_t* ds_full = bars + 10;                  // count 256
+  uint64_t* acc_done = bars + 11;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
+  int* tile_minmax = reinterpret_cast<int*>(bars + 13);   // [2]
+  int* seg_lohi = reinterpret_cast<int*>(bars + 14);      // [2]
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int n_qtiles = (p.Sq + BWD_T - 1) / BWD_T;
+  const int qt = n_qtiles - 1 - (int)(blockIdx.x / (p.Hq * p.B));   // heaviest query tiles first
+  const int hq = (blockIdx.x / p.B) % p.Hq, b = blockIdx.x % p.B;
+  const int hkv = hq / (p.Hq / p.Hkv);
+  const int q0 = qt * BWD_T;
+  const int pos_off = p.Sk - p.Sq;
+
+  if (threadIdx.x == 0) {
+    mbar_init(qdo_full, 1);
+    for (int i = 0; i < 2; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
+    mbar_init(v_full, 1); mbar_init(v_empty, 1);
+    mbar_init(s_full, 1); mbar_init(s_read, 256);
+    mbar_init(dp_full, 1); mbar_init(ds_full, 256);
+    mbar_init(acc_done, 1);
+    tile_minmax[0] = 0x7fffffff;
+    tile_minmax[1] = -0x7fffffff;
+    seg_lohi[0] = 0x7fffffff;
+    seg_lohi[1] = -1;
+    fence_barrier_init();
+  }
+  if (warp == 1) {
+    tmem_alloc(tmem_slot, 512);
+    tmem_relinquish();
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+
+  if (threadIdx.x < BWD_T) {
+    const int r = q0 + threadIdx.x;
+    if (r < p.Sq) {
+      const int qp = p.q_pos ? p.q_pos[(long long)b * p.Sq + r] : r + pos_off;
+      atomicMin(&tile_minmax[0], qp);
+      atomicMax(&tile_minmax[1], qp);
+    }
+  }
+  __syncthreads();
+  const int qpos_min = tile_minmax[0], qpos_max = tile_minmax[1];
+  const int nblk_total = (p.Sk + BWD_T - 1) / BWD_T;
+  int blk_hi = p.causal ? min(nblk_total, qpos_max / BWD_T + 1) : nblk_total;
+  int blk_lo = (p.window > 0) ? max(0, (qpos_min - p.window + 1) / BWD_T) : 0;
+  if (qpos_max < 0) blk_hi = 0;
+  int2 qr = make_int2(0, 0);
+  if (p.kv_rng) {
+    qr = seg_range128(p.q_rng, b, qt, p.Sq);
+    for (int i = blk_lo + (int)threadIdx.x; i < blk_hi; i += BWD_THREADS) {
+      const int2 kr = seg_range128(p.kv_rng, b, i, p.Sk);
+      if (kr.x <= qr.y && kr.y >= qr.x) {
+        atomicMin(&seg_lohi[0], i);
+        atomicMax(&seg_lohi[1], i);
+      }
+    }
+    __syncthreads();
+    blk_lo = max(blk_lo, seg_lohi[0]);
+    blk_hi = min(blk_hi, seg_lohi[1] + 1);
+  }
+  const int nblk = max(0, blk_hi - blk_lo);
+
+  if (warp == 0) {
+    // ------------------------------------------------------------------ TMA producer
+    if (lane == 0 && nblk > 0) {
+      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
+      mbar_expect_tx(qdo_full, W_K_BYTES + TILE_BYTES);
+      for (int c = 0; c < W_D / 64; ++c)
+        tma_load_3d(smem + OFF_Q + c * (BWD_T * 128), &tmQ, qdo_full, c * 64, b * p.Sq + q0, hq);
+      for (int c = 0; c < BWD_D / 64; ++c)
+        tma_load_3d(smem + OFF_DO + c * (BWD_T * 128), &tmdO, qdo_full, c * 64, b * p.Sq + q0, hq);
+      for (int j = 0; j < nblk; ++j) {
+        const int st = j & 1;
+        const int row = b * p.Sk + (blk_lo + j) * BWD_T;
+        if (!mbar_wait(&k_empty[st], ((j >> 1) & 1) ^ 1, p.status, kTimeoutStageFree, 131)) break;
+        mbar_expect_tx(&k_full[st], W_K_BYTES);
+        for (int c = 0; c < W_D / 64; ++c)
+          tma_load_3d(smem + OFF_K + st * W_K_BYTES + c * (BWD_T * 128), &tmK, &k_full[st], c * 64, row, hkv);
+        if (!mbar_wait(v_empty, (j & 1) ^ 1, p.status, kTimeoutStageFree, 135)) break;
+        mbar_expect_tx(v_full, TILE_BYTES);
+        for (int c = 0; c < BWD_D / 64; ++c)
+          tma_load_3d(smem + OFF_V + c * (BWD_T * 128), &tmV, v_full, c * 64, row, hkv);
+      }
+    }
+  } else if (warp == 1) {
+    // ------------------------------------------------------------------ MMA issuer
+    if (lane == 0 && nblk > 0) {
+      constexpr uint32_t id_s = make_idesc_bf16(BWD_T, BWD_T, false, false);    // S, dP
+      constexpr uint32_t id_dq = make_idesc_bf16(BWD_T, W_D, false, true);      // dQ (A in TMEM, B MN-major)
+      const uint32_t dQ = kmajor_lo(smem_u32(smem + OFF_Q)), dDO = kmajor_lo(smem_u32(smem + OFF_DO));
+      const uint32_t dV = kmajor_lo(smem_u32(smem + OFF_V));
+      const uint32_t aK0 = smem_u32(smem + OFF_K);
+      const uint32_t tS = tmem_base + T_S, tDP = tmem_base + T_DP;
+      auto kstep = [](int k) { return (uint32_t)(((k >> 2) * (BWD_T * 128) + (k & 3) * 32) >> 4); };
+      auto issue_s = [&](int j) -> bool {      // S(j) = Q K_j^T
+        if (!mbar_wait(&k_full[j & 1], (j >> 1) & 1, p.status, kTimeoutTmaFull, 133)) return false;
+        tc_fence_after();
+        const uint32_t dK = kmajor_lo(aK0 + (j & 1) * W_K_BYTES);
+#pragma unroll
+        for (int k = 0; k < W_D / 16; ++k) mma_ss_w(tS, dQ + kstep(k), kDescHi, dK + kstep(k), kDescHi, id_s, k != 0);
+        tc_commit(s_full);
+        return true;
+      };
+      auto issue_dp = [&](int j) -> bool {     // dP(j) = dO V_j^T
+        if (!mbar_wait(v_full, j & 1, p.status, kTimeoutTmaFull, 137)) return false;
+        tc_fence_after();
+#pragma unroll
+        for (int k = 0; k < BWD_D / 16; ++k) mma_ss_w(tDP, dDO + kstep(k), kDescHi, dV + kstep(k), kDescHi, id_s, k != 0);
+        tc_commit(v_empty);
+        tc_commit(dp_full);
+        return true;
+      };
+      bool ok = mbar_wait(qdo_full, 0, p.status, kTimeoutTmaFull, 132);
+      if (ok) ok = issue_s(0) && issue_dp(0);
+      for (int j = 0; j < nblk && ok; ++j) {
+        const bool more = j + 1 < nblk;
+        if (more) {
+          if (!mbar_wait(s_read, j & 1, p.status, kTimeoutSoftmax, 140)) break;   // S(j) is in registers
+          tc_fence_after();
+          if (!issue_s(j + 1)) break;
+        }
+        if (!mbar_wait(ds_full, j & 1, p.status, kTimeoutSoftmax, 134)) break;
+        tc_fence_after();
+        const uint32_t mK = mnmajor_lo(aK0 + (j & 1) * W_K_BYTES);
+#pragma unroll
+        for (int k = 0; k < BWD_T / 16; ++k)   // dQ += dS K
+          mma_ts_w(tmem_base + T_DQ, tDP + a_col(k), mK + mnmajor_k(k), kDescHi, id_dq, (j | k) != 0);
+        tc_commit(&k_empty[j & 1]);
+        if (more && !issue_dp(j + 1)) break;
+      }
+      tc_commit(acc_done);
+    }
+  } else {
+    // ------------------------------------------------------------------ compute warps
+    const int qd = warp & 3;
+    const int half = (warp - 2) >> 2;             // which 64 of the 128 key columns
+    const int r_local = qd * 32 + lane;           // query row == TMEM lane
+    const int row = q0 + r_local;
+    const bool row_ok = row < p.Sq;
+    const long long grow = (long long)b * p.Sq + row;
+    const int qpos = row_ok ? (p.q_pos ? p.q_pos[grow] : row + pos_off) : -1;
+    const int qseg = (p.q_seg && row_ok) ? p.q_seg[grow] : 0;
+    const long long li = ((long long)b * p.Hq + hq) * p.Sq_pad + row;   // row < Sq_pad: padded to 128
+    const float lse2 = p.lse2[li];
+    const float delta = p.delta[li];
+    const uint32_t tb = tmem_base + ((uint32_t)(qd * 32) << 16);
+    const uint32_t tS = tb + T_S + half * 64, tDP = tb + T_DP + half * 64;
+    const int* ks = p.kv_seg ? p.kv_seg + (long long)b * p.Sk : nullptr;
+    const int win = p.window > 0 ? p.window : 0x7fffffff;
+    const int kmax = p.causal ? min(qpos, p.Sk - 1) : p.Sk - 1;   // keep needs kp <= kmax
+    bool ok = true;
+
+    for (int j = 0; j < nblk && ok; ++j) {
+      const int kv0 = (blk_lo + j) * BWD_T;
+      bool seg_mask = p.q_seg != nullptr;
+      if (p.kv_rng) {
+        const int2 kr = seg_range128(p.kv_rng, b, blk_lo + j, p.Sk);
+        seg_mask = !(qr.x == qr.y && kr.x == kr.y && qr.x == kr.x);
+      }
+      const bool need_mask = (p.causal && kv0 + BWD_T - 1 > qpos_min) || (kv0 + BWD_T > p.Sk) ||
+                             (p.window > 0 && qpos_max - kv0 >= p.window) || seg_mask;
+      // ---- phase 1: P = exp2(S * c - lse), packed bf16 in registers
+      if (!mbar_wait(s_full, j & 1, p.status, kTimeoutAccFull, 136)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t pk_p[32];
+      uint32_t sreg[64];
+      tmem_ld32(tS, sreg);
+      tmem_ld32(tS + 32, sreg + 32);
+      tmem_wait_ld();
+      tc_fence_before();
+      mbar_arrive(s_read);
+#pragma unroll
+      for (int ch = 0; ch < 2; ++ch) {
+        const uint32_t* s = sreg + ch * 32;
+        if (!need_mask) {
+#pragma unroll
+          for (int c = 0; c < 32; c += 2)
+            pk_p[ch * 16 + c / 2] = pack_bf16(exp2f(fmaf(__uint_as_float(s[c]), p.scale_log2, -lse2)),
+                                              exp2f(fmaf(__uint_as_float(s[c + 1]), p.scale_log2, -lse2)));
+        } else {
+          const int kbase = kv0 + half * 64 + ch * 32;
+#pragma unroll
+          for (int c = 0; c < 32; c += 2) {
+            float pv[2];
+#pragma unroll
+            for (int e = 0; e < 2; ++e) {
+              const int kp = kbase + c + e;
+              bool keep = (kp <= kmax) & (qpos - kp < win);
+              if (ks && seg_mask) keep = keep & (__ldg(ks + min(kp, p.Sk - 1)) == qseg);
+              const float pe = exp2f(fmaf(__uint_as_float(s[c + e]), p.scale_log2, -lse2));
+              pv[e] = keep ? pe : 0.f;
+            }
+            pk_p[ch * 16 + c / 2] = pack_bf16(pv[0], pv[1]);
+          }
+        }
+      }
+      // ---- phase 2: dS = P o (dP - delta), written over dP
+      if (!mbar_wait(dp_full, j & 1, p.status, kTimeoutAccFull, 139)) { ok = false; break; }
+      tc_fence_after();
+      {
+        uint32_t dreg[64], pk[32];
+        tmem_ld32(tDP, dreg);
+        tmem_ld32(tDP + 32, dreg + 32);
+        tmem_wait_ld();
+#pragma unroll
+        for (int c = 0; c < 32; ++c)
+          pk[c] = mul_bf16x2(pk_p[c], pack_bf16(__uint_as_float(dreg[2 * c]) - delta,
+                                                __uint_as_float(dreg[2 * c + 1]) - delta));
+        tmem_st32(tDP, pk);
+      }
+      tmem_wait_st();
+      tc_fence_before();
+      mbar_arrive(ds_full);
+    }
+    if (ok && nblk > 0) ok = mbar_wait(acc_done, 0, p.status, kTimeoutAccFull, 138);
+    tc_fence_after();
+    store_acc_cols(tb + T_DQ, half * 96, 3, p.dQ + grow * p.lddq + (long long)hq * W_D, ok && nblk > 0, row_ok, p.scale);
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc(tmem_base, 512);
+  }
+}
+
 }  // namespace tpb
 
 using namespace tpb;
@@ -862,11 +1497,12 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
                                     float scale, int causal, int window, const int* q_pos, const int* q_seg,
                                     const int* kv_seg, const int* q_rng, const int* kv_rng, float softcap,
                                     void* stream_) {
-  if (dqk != 128 || dvd != 128 || Hq % Hkv) return -2;
+  const bool wide = dqk == W_D;
+  if ((dqk != 128 && !wide) || dvd != 128 || Hq % Hkv || (wide && softcap > 0.f)) return -2;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (lddo % 8) || (lddq % 8) || (lddk % 8) || (lddv % 8)) return -2;
   if (lddo != (long long)Hq * dvd) return -2;   // dO and O are contiguous [B*Sq, Hq, 128]
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
-  if ((Sq + BWD_T - 1) / BWD_T > KV_MAX_TILES) return -6;
+  if (wide ? (Sq + W_QT - 1) / W_QT > W_MAX_TILES : (Sq + BWD_T - 1) / BWD_T > KV_MAX_TILES) return -6;
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   const int sq_pad = (Sq + BWD_T - 1) / BWD_T * BWD_T;
   float* lse2 = scratch;
@@ -907,6 +1543,7 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
     allow((const void*)attn_bwd_dkv_kernel<false, true>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<false, true>, dqk::TOTAL);
     allow((const void*)attn_bwd_dkv_kernel<true, false>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<true, false>, dqk::TOTAL);
     allow((const void*)attn_bwd_dkv_kernel<true, true>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<true, true>, dqk::TOTAL);
+    allow((const void*)attn_bwd_dkv192_kernel, wkv::TOTAL); allow((const void*)attn_bwd_dq192_kernel, wdq::TOTAL);
     if (e != cudaSuccess) return 1000 + (int)e;
     configured = true;
   }
@@ -917,6 +1554,17 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
   if (make_tmap_3d(&tv, v, dvd, (uint64_t)B * Sk, Hkv, ldv, dvd, 64, BWD_T)) return -5;
   if (make_tmap_3d(&tdo, dO, dvd, (uint64_t)B * Sq, Hq, lddo, dvd, 64, BWD_T)) return -5;
   dim3 grid_kv(((Sk + BWD_T - 1) / BWD_T) * Hkv * B, 1, 1);
+  if (wide) {
+    CUtensorMap tq64, tdo64;      // the dK/dV kernel takes its queries 64 rows at a time
+    if (make_tmap_3d(&tq64, q, dqk, (uint64_t)B * Sq, Hq, ldq, dqk, 64, W_QT)) return -3;
+    if (make_tmap_3d(&tdo64, dO, dvd, (uint64_t)B * Sq, Hq, lddo, dvd, 64, W_QT)) return -5;
+    attn_bwd_dkv192_kernel<<<grid_kv, BWD_THREADS, wkv::TOTAL, stream>>>(tq64, tk, tv, tdo64, p);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess) return 1000 + (int)e;
+    attn_bwd_dq192_kernel<<<((Sq + BWD_T - 1) / BWD_T) * Hq * B, BWD_THREADS, wdq::TOTAL, stream>>>(tq, tk, tv, tdo, p);
+    e = cudaGetLastError();
+    return e == cudaSuccess ? 0 : 1000 + (int)e;
+  }
   (softcap > 0.f ? (ranges ? attn_bwd_dkv_kernel<true, true> : attn_bwd_dkv_kernel<true, false>)
                  : (ranges ? attn_bwd_dkv_kernel<false, true> : attn_bwd_dkv_kernel<false, false>))
       <<<grid_kv, BWD_THREADS, dkv::TOTAL, stream>>>(tq, tk, tv, tdo, p);

@@ -133,7 +133,8 @@ def attn_bwd(do, q, k, v, o, lse, causal=True, scale=None, window=None, q_pos=No
   o = o.contiguous()
   if dqk != 128:
     assert not softcap, "the capped backward exists for head dim 128 only"
-    return _eager_bwd(do, q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv)
+    if sq > _MAX_WIDE_QUERIES:
+      return _eager_bwd(do, q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv)
   scratch = torch.empty(2 * b * hq * ((sq + 127) // 128 * 128), dtype=torch.float32, device=q.device)
   q_rng, kv_rng = _seg_ranges(q_seg, kv_seg, b, sq, sk)
   rc = lib().tpb_attn_bwd_softcap(ptr(do), ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), ptr(scratch), ptr(dq),
@@ -145,8 +146,11 @@ def attn_bwd(do, q, k, v, o, lse, causal=True, scale=None, window=None, q_pos=No
   return dq, dk, dv
 
 
+_MAX_WIDE_QUERIES = 131072     # rows of the head-dim-192 backward's query-tile table
+
+
 def _eager_bwd(do, q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv):
-  """Gradients for shapes the backward kernel does not cover yet (q/k head dim 192).  Plain causal
+  """Gradients for q/k head dim 192 with more queries than the backward kernel's table holds.  Plain causal
   or full attention goes through torch's scaled_dot_product_attention (a library call: forward is
   recomputed with autograd on); masks it cannot express fall back to the fp32 eager definition,
   one batch element at a time."""
