@@ -17,7 +17,8 @@
 //   warp 1      MMA issuer: tcgen05.mma 128 x NT x 16
 //   warps 2..5  accumulator (TMEM) -> shared memory; then all warps reduce and write
 //
-// W may be stored [N][K] (forward) or [K][N] (input gradients, expert weights).  With the SwiGLU
+// W may be stored [N][K] (forward) or [K][N] (input gradients, expert weights); with the latter X may be
+// [K][T] too (weight gradients with few tiles: C = dY^T X contracts over the tokens).  With the SwiGLU
 // epilogue a tile is 64 gate and the same 64 up features.  Grouped mode: rows are grouped by expert in
 // segments padded to the token-tile width, so a token tile belongs to one expert.
 
@@ -96,7 +97,7 @@ __device__ __forceinline__ void store4(__nv_bfloat16* dst, const float4& v, int 
   }
 }
 
-template <int NT, bool W_MN>
+template <int NT, bool W_MN, bool X_MN>
 __global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
                    const __grid_constant__ CUtensorMap tmX, const SkinnyParams p) {
@@ -162,7 +163,12 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           tma_load_3d(sW, &tmW, &full[stage], n0, k0, ez);
           tma_load_3d(sW + SK_W_BYTES / 2, &tmW2, &full[stage], nb, k0, ez);
         }
-        tma_load_2d(sW + SK_W_BYTES, &tmX, &full[stage], k0, t0);
+        if (!X_MN) {
+          tma_load_2d(sW + SK_W_BYTES, &tmX, &full[stage], k0, t0);
+        } else {              // boxes {64 rows of X, 64 k}
+#pragma unroll
+          for (int c = 0; c < NT / 64; ++c) tma_load_2d(sW + SK_W_BYTES + c * 8192, &tmX, &full[stage], t0 + c * 64, k0);
+        }
         if (++stage == NST) {
           stage = 0;
           phase ^= 1;
@@ -171,7 +177,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
   } else if (warp == 1) {
     if (lane == 0 && kb1 > kb0) {
-      constexpr uint32_t idesc = make_idesc_bf16(SK_TN, NT, W_MN, false);
+      constexpr uint32_t idesc = make_idesc_bf16(SK_TN, NT, W_MN, X_MN);
       constexpr uint32_t desc_hi = smem_desc_hi(1024);
       const uint32_t base = smem_u32(smem);
       int stage = 0;
@@ -182,10 +188,11 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         tc_fence_after();
         const uint32_t sW = base + stage * L::STAGE;
         const uint32_t a_lo = smem_desc_lo(sW, W_MN ? 8192 : 16);
-        const uint32_t b_lo = smem_desc_lo(sW + SK_W_BYTES, 16);
+        const uint32_t b_lo = smem_desc_lo(sW + SK_W_BYTES, X_MN ? 8192 : 16);
 #pragma unroll
         for (int k = 0; k < SK_BK / 16; ++k)
-          mma_ss_w(tmem_base, a_lo + (W_MN ? k * 128 : k * 2), desc_hi, b_lo + k * 2, desc_hi, idesc,
+          mma_ss_w(tmem_base, a_lo + (W_MN ? k * 128 : k * 2), desc_hi, b_lo + (X_MN ? k * 128 : k * 2),
+                   desc_hi, idesc,
                    ((kb - kb0) | k) != 0);
         tc_commit(&empty[stage]);
         if (++stage == NST) {
@@ -276,12 +283,12 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
 }
 
-template <int NT, bool W_MN>
+template <int NT, bool W_MN, bool X_MN = false>
 static cudaError_t launch_skinny(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tx,
                                  const SkinnyParams& p, int grid, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<NT, W_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<NT, W_MN, X_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          SkinnySmem<NT>::TOTAL);
     if (e != cudaSuccess) return e;
     configured = true;
@@ -298,7 +305,7 @@ static cudaError_t launch_skinny(const CUtensorMap& tw, const CUtensorMap& tw2, 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<NT, W_MN>, tw, tw2, tx, p);
+  return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<NT, W_MN, X_MN>, tw, tw2, tx, p);
 }
 
 // Token-tile width for `rows` rows: the smallest one that holds them, 128 at most.
@@ -326,11 +333,17 @@ bool skinny_wins(int M, int N, bool swiglu) {
   return tiles <= sm_count() / 2;
 }
 
-// x [T,K] (for grouped mode: all padded rows), w dense [N,K] (w_mn = 0) or [K,N] (w_mn = 1), with
+// The same for a weight gradient (both operands contracted over their rows): bound by the tensor cores, so
+// only where the tiled kernel leaves half of the SMs idle.
+bool skinny_wins_wgrad(int M, int N) {
+  return (long long)((M + 127) / 128) * ((N + 255) / 256) <= sm_count() / 2;
+}
+
+// x [T,K], or [K,T] with x_mn (for grouped mode: all padded rows), w dense [N,K] (w_mn = 0) or [K,N] (w_mn = 1), with
 // `experts` of them `w_stride` elements apart.  N counts both halves for SwiGLU.  nt / splits 0: by
 // the rules above.  Returns -2 when the shape or alignment is not supported.
 int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, int experts,
-                long long ldx, long long ldw, long long w_stride, long long ldc, int w_mn, int epi, float alpha,
+                long long ldx, long long ldw, long long w_stride, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                 const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit,
                 int nt, int splits, cudaStream_t stream) {
   if (T <= 0 || N <= 0 || K <= 0) return 0;
@@ -348,6 +361,10 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
   const int tile_n = swiglu ? SK_TN / 2 : SK_TN;
   const int n_out = swiglu ? N / 2 : N;
   if (nt == 0) nt = skinny_nt(T);
+  if (x_mn) {
+    if (!w_mn || swiglu || tile_expert) return -2;
+    if (nt < 64) nt = 64;       // X arrives in blocks of 64 rows
+  }
   if (nt != 16 && nt != 32 && nt != 64 && nt != 128) return -2;
   SkinnyParams p;
   p.T = T; p.N = n_out; p.K = K;
@@ -374,7 +391,7 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
     return !w_mn ? make_tmap_3d(m, ptr, K, extent, experts, ldw, stride, 64, 64)
                  : make_tmap_3d(m, ptr, extent, K, experts, ldw, stride, 64, 64);
   };
-  if (make_tmap_2d(&tx, x, K, T, ldx, 64, nt, 2)) return -3;
+  if (!x_mn ? make_tmap_2d(&tx, x, K, T, ldx, 64, nt, 2) : make_tmap_2d(&tx, x, T, K, ldx, 64, 64, 2)) return -3;
   if (make_w(&tw, w)) return -4;
   if (two_w) {
     if (make_w(&tw2, w2)) return -5;
@@ -385,7 +402,10 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
   cudaError_t e;
 #define TPB_SK(NT_) (w_mn ? launch_skinny<NT_, true>(tw, tw2, tx, p, grid, stream) \
                           : launch_skinny<NT_, false>(tw, tw2, tx, p, grid, stream))
-  switch (nt) {
+  if (x_mn)
+    e = nt == 64 ? launch_skinny<64, true, true>(tw, tw2, tx, p, grid, stream)
+                 : launch_skinny<128, true, true>(tw, tw2, tx, p, grid, stream);
+  else switch (nt) {
     case 16: e = TPB_SK(16); break;
     case 32: e = TPB_SK(32); break;
     case 64: e = TPB_SK(64); break;
@@ -402,10 +422,10 @@ using namespace tpb;
 
 // The kernel with an explicit token-tile width and K split (0: by rule); see tpb_gemm_bf16 for the rest.
 extern "C" int tpb_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, int T, int N, int K,
-                                    long long ldx, long long ldw, long long ldc, int w_mn, int epi, float alpha,
+                                    long long ldx, long long ldw, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                                     const void* aux, long long ldaux, void* c2, long long ldc2, int nt, int splits,
                                     void* stream) {
-  return skinny_gemm(x, w, w2, c, T, N, K, 1, ldx, ldw, 0, ldc, w_mn, epi, alpha, aux, ldaux, c2, ldc2, nullptr, 0, nt,
+  return skinny_gemm(x, w, w2, c, T, N, K, 1, ldx, ldw, 0, ldc, x_mn, w_mn, epi, alpha, aux, ldaux, c2, ldc2, nullptr, 0, nt,
                      splits, reinterpret_cast<cudaStream_t>(stream));
 }
 
@@ -416,6 +436,6 @@ extern "C" int tpb_grouped_gemm_skinny_bf16(const void* x, const void* w, const 
                                             long long ldc, int w_mn, int epi, const int* tile_expert, int experts_hit,
                                             int nt, void* stream) {
   if (!tile_expert || E < 1 || experts_hit < 1) return -2;
-  return skinny_gemm(x, w, w2, c, rows, N, K, E, ldx, ldw, w_stride, ldc, w_mn, epi, 1.0f, nullptr, 0, nullptr, 0,
+  return skinny_gemm(x, w, w2, c, rows, N, K, E, ldx, ldw, w_stride, ldc, 0, w_mn, epi, 1.0f, nullptr, 0, nullptr, 0,
                      tile_expert, experts_hit, nt, 0, reinterpret_cast<cudaStream_t>(stream));
 }

@@ -882,10 +882,11 @@ cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const
 
 // gemm_skinny_sm100.cu
 int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, int experts,
-                long long ldx, long long ldw, long long w_stride, long long ldc, int w_mn, int epi, float alpha,
+                long long ldx, long long ldw, long long w_stride, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                 const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit, int nt,
                 int splits, cudaStream_t stream);
 bool skinny_wins(int M, int N, bool swiglu);
+bool skinny_wins_wgrad(int M, int N);
 
 // TPB_GEMM_PAIR: 0 = never CTA pairs, 2 = pairs for every dense shape (tests), default = by shape
 static int gemm_pair_mode() {
@@ -1072,9 +1073,10 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
                              long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha,
                              const void* aux, long long ldaux, void* c2, long long ldc2, int max_ctas,
                              void* stream_) {
-  // few rows: the kernel that streams B once and splits the contraction
-  if (!a_mn && max_ctas == 0 && gemm_pair_mode() == 1 && skinny_wins(M, N, epi == TPB_EPI_SWIGLU)) {
-    const int r = skinny_gemm(A, B, nullptr, C, M, N, K, 1, lda, ldb, 0, ldc, b_mn, epi, alpha, aux, ldaux, c2, ldc2,
+  // few rows or few tiles: the kernel that streams B once and splits the contraction
+  if (max_ctas == 0 && gemm_pair_mode() == 1 &&
+      (a_mn ? b_mn && skinny_wins_wgrad(M, N) : skinny_wins(M, N, epi == TPB_EPI_SWIGLU))) {
+    const int r = skinny_gemm(A, B, nullptr, C, M, N, K, 1, lda, ldb, 0, ldc, a_mn, b_mn, epi, alpha, aux, ldaux, c2, ldc2,
                               nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_));
     if (r != -2) return r;     // -2: an epilogue or alignment it does not take
   }

@@ -11,15 +11,15 @@ from torchprime_b200.ops._lib import lib, ptr, stream_ptr
 BF16_EPS = 2.0 ** -8
 
 
-def _skinny(x, w, *, b_mn=False, epi=k.EPI_BF16, alpha=1.0, aux=None, w2=None, c2=None, nt=0, splits=0, out=None):
-  t, kk = x.shape
+def _skinny(x, w, *, a_mn=False, b_mn=False, epi=k.EPI_BF16, alpha=1.0, aux=None, w2=None, c2=None, nt=0, splits=0, out=None):
+  t, kk = x.shape[::-1] if a_mn else x.shape
   n = w.shape[1] if b_mn else w.shape[0]
   n *= 2 if w2 is not None else 1
   n_out = n // 2 if epi == k.EPI_SWIGLU else n
   if out is None:
     out = torch.empty(t, n_out, device="cuda", dtype=torch.float32 if epi == k.EPI_F32 else torch.bfloat16)
   rc = lib().tpb_gemm_skinny_bf16(ptr(x), ptr(w), ptr(w2), ptr(out), t, n, kk, x.stride(0), w.stride(0), out.stride(0),
-                                  int(b_mn), epi, alpha, ptr(aux), aux.stride(0) if aux is not None else 0, ptr(c2),
+                                  int(a_mn), int(b_mn), epi, alpha, ptr(aux), aux.stride(0) if aux is not None else 0, ptr(c2),
                                   c2.stride(0) if c2 is not None else 0, nt, splits, stream_ptr())
   assert rc == 0, rc
   return out
@@ -29,7 +29,7 @@ def _skinny(x, w, *, b_mn=False, epi=k.EPI_BF16, alpha=1.0, aux=None, w2=None, c
 def _signature():
   from ctypes import c_float as F, c_int as I, c_longlong as LL, c_void_p as P
   fn = lib().tpb_gemm_skinny_bf16
-  fn.argtypes, fn.restype = [P, P, P, P, I, I, I, LL, LL, LL, I, I, F, P, LL, P, LL, I, I, P], I
+  fn.argtypes, fn.restype = [P, P, P, P, I, I, I, LL, LL, LL, I, I, I, F, P, LL, P, LL, I, I, P], I
 
 
 def _close(got, want, scale):
@@ -78,6 +78,19 @@ def test_dense_swiglu(cuda_lib, t, f, kk, splits, b_mn):
     # silu amplifies an error of the gate by at most 1.1
     err = (act.double() - want).abs()
     assert bool((err <= BF16_EPS * want.abs() + 1e-5 * (1 + up.abs())).all()), err.max()
+
+
+@pytest.mark.parametrize("m,n", [(8, 64), (64, 200), (72, 128), (136, 264), (576, 2048)])
+@pytest.mark.parametrize("t,splits", [(1, 1), (63, 0), (64, 1), (200, 2), (1500, 8)])
+def test_weight_gradient(cuda_lib, m, n, t, splits):
+  """C = dY^T X: both operands contracted over their rows."""
+  torch.manual_seed(m + t)
+  dy = torch.randn(t, m, device="cuda", dtype=torch.bfloat16)
+  x = torch.randn(t, n, device="cuda", dtype=torch.bfloat16)
+  want = dy.double().t() @ x.double()
+  for epi in (k.EPI_BF16, k.EPI_F32):
+    for nt in (0, 64, 128):
+      _close(_skinny(dy, x, a_mn=True, b_mn=True, epi=epi, nt=nt, splits=splits), want, float(max(t, 16)))
 
 
 def test_split_sums_do_not_depend_on_the_run(cuda_lib):
