@@ -321,22 +321,27 @@ static int skinny_splits(long long tiles, int num_kb) {
 
 // Whether this kernel is the faster one for a dense product of M rows: always up to 128 rows (one token
 // tile; even a 102,400-wide head takes 98 us instead of 108 with 128 rows and 66 instead of 133 with one),
-// and beyond that while the tiled kernel's 128 x 256 tiles leave half of the SMs idle.  The time per call in
+// and beyond that while the tiled kernel's 128 x 256 tiles leave half of the SMs idle and the contraction is long
+// enough to be split (see the weight gradients below).  The time per call in
 // us with weights from HBM, tiled kernel / this one, by the number of its tiles (N x K):
 //   4096 x 4096:   384 rows, 48 tiles 34 / 23    512 rows, 64 tiles 35 / 24    768 rows, 96 tiles 35 / 36
 //   4096 x 14336:  512 rows, 64 tiles 98 / 62    768 rows, 96 tiles 98 / 97
 //   2048 x 10944: 1024 rows, 64 tiles 77 / 47    3072 x 2048: 768 rows, 72 tiles 22 / 16, 1024 rows, 96 tiles 23 / 23
 //   14336 x 4096:  128 rows, 56 tiles 39 / 28    192 rows, 112 tiles 39 / 40
-bool skinny_wins(int M, int N, bool swiglu) {
+bool skinny_wins(int M, int N, int K, bool swiglu) {
   if (M <= 128) return true;
+  if (K < 1024) return false;
   const long long tiles = (long long)((M + 127) / 128) * (((swiglu ? N / 2 : N) + (swiglu ? 127 : 255)) / (swiglu ? 128 : 256));
   return tiles <= sm_count() / 2;
 }
 
-// The same for a weight gradient (both operands contracted over their rows): bound by the tensor cores, so
-// only where the tiled kernel leaves half of the SMs idle.
-bool skinny_wins_wgrad(int M, int N) {
-  return (long long)((M + 127) / 128) * ((N + 255) / 256) <= sm_count() / 2;
+// The same for a weight gradient (both operands contracted over their rows, K of them): bound by the tensor cores,
+// so only where the tiled kernel leaves half of the SMs idle, and with a contraction that pays for the split.
+// us per call, tiled / this kernel, for 256, 1024, 4096 rows:
+//   576 x 2048, 40 tiles: 7 / 10, 13 / 12, 31 / 22      4096 x 512, 64 tiles: 8 / 11, 13 / 13, 31 / 23
+//   64 x 2048, 8 tiles: 7 / 7, 11 / 7, 31 / 10          2048 x 2048, 128 tiles: 8 / 13, 13 / 18, 34 / 37
+bool skinny_wins_wgrad(int M, int N, int K) {
+  return K >= 1024 && (long long)((M + 127) / 128) * ((N + 255) / 256) <= sm_count() / 2;
 }
 
 // x [T,K], or [K,T] with x_mn (for grouped mode: all padded rows), w dense [N,K] (w_mn = 0) or [K,N] (w_mn = 1), with

@@ -885,8 +885,8 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
                 long long ldx, long long ldw, long long w_stride, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                 const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit, int nt,
                 int splits, cudaStream_t stream);
-bool skinny_wins(int M, int N, bool swiglu);
-bool skinny_wins_wgrad(int M, int N);
+bool skinny_wins(int M, int N, int K, bool swiglu);
+bool skinny_wins_wgrad(int M, int N, int K);
 
 // TPB_GEMM_PAIR: 0 = never CTA pairs, 2 = pairs for every dense shape (tests), default = by shape
 static int gemm_pair_mode() {
@@ -1075,7 +1075,7 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
                              void* stream_) {
   // few rows or few tiles: the kernel that streams B once and splits the contraction
   if (max_ctas == 0 && gemm_pair_mode() == 1 &&
-      (a_mn ? b_mn && skinny_wins_wgrad(M, N) : skinny_wins(M, N, epi == TPB_EPI_SWIGLU))) {
+      (a_mn ? b_mn && skinny_wins_wgrad(M, N, K) : skinny_wins(M, N, K, epi == TPB_EPI_SWIGLU))) {
     const int r = skinny_gemm(A, B, nullptr, C, M, N, K, 1, lda, ldb, 0, ldc, a_mn, b_mn, epi, alpha, aux, ldaux, c2, ldc2,
                               nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_));
     if (r != -2) return r;     // -2: an epilogue or alignment it does not take

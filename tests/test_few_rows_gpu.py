@@ -127,8 +127,8 @@ def test_plan_with_narrow_segments(cuda_lib, align, t, kk, e):
 
 
 @pytest.mark.parametrize("fused", [False, True])
-@pytest.mark.parametrize("t,kk,e,d,f", [(1, 6, 64, 256, 192), (4, 6, 64, 2048, 1408), (16, 2, 8, 512, 1024), (100, 2, 16, 256, 320),
-                                        (128, 1, 2, 128, 64)])
+@pytest.mark.parametrize("t,kk,e,d,f", [(1, 6, 64, 256, 192), (4, 6, 64, 2048, 1408), (16, 2, 8, 512, 1024), (190, 2, 16, 256, 320),
+                                        (48, 1, 2, 128, 64), (260, 6, 64, 128, 64)])
 def test_grouped_mlp_without_gradients(cuda_lib, t, kk, e, d, f, fused):
   """The few-rows path against the tiled grouped GEMMs' oracle, one expert hit by nobody."""
   torch.manual_seed(t + e)
@@ -148,9 +148,9 @@ def test_grouped_mlp_without_gradients(cuda_lib, t, kk, e, d, f, fused):
 
 
 def test_route_of_the_few_rows_path():
-  assert moe.few_rows_align(4, 6, 64) == 16 and moe.few_rows_align(128, 6, 64) == 32
-  assert moe.few_rows_align(128, 2, 8) == 64 and moe.few_rows_align(129, 2, 8) is None
-  assert moe.few_rows_align(128, 8, 8) is None
+  assert moe.few_rows_align(4, 6, 64) == 16 and moe.few_rows_align(128, 6, 64) == 16
+  assert moe.few_rows_align(96, 2, 8) == 32 and moe.few_rows_align(97, 2, 8) is None
+  assert moe.few_rows_align(256, 6, 64) == 32 and moe.few_rows_align(257, 6, 64) is None
 
 
 def test_linear_f32_logits(cuda_lib):

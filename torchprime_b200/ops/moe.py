@@ -214,13 +214,13 @@ def gather_rows(x, src_row, row_scale=None):
 
 
 def few_rows_align(t: int, k: int, e: int) -> int | None:
-  """Token-tile width of the few-rows path for ``t`` tokens, or None where the tiled grouped GEMMs are
-  the better ones.  It is about twice the average number of rows an expert sees."""
+  """Token-tile width of the few-rows path for ``t`` tokens, or None where the tiled grouped GEMMs are as good.
+  Both paths are bound by the weights of the experts that are hit; what counts is the average number of rows per
+  expert (us for the routed MLP, tiled / 16 / 32 / 64 rows per segment step): 64 experts of 2048 x 1408, 6 rows
+  225 / 210 / 224 / 257, 12 rows 228 / 217 / 227 / 258, 24 rows 231 / 268 / 231 / 259; 8 experts of 4096 x 14336,
+  8 rows 469 / 448 / 453 / 475, 16 rows 471 / 485 / 454 / 476, 24 rows 555 / 525 / 459 / 482."""
   per = t * k / e
-  if t > 128 or per > 64:
-    return None
-  want = min(t, 2 * per)
-  return 16 if want <= 16 else 32 if want <= 32 else 64
+  return 16 if per <= 12 else 32 if per <= 24 else None
 
 
 def grouped_mlp_few_rows(x, weights, idx, w_gate, w_up, w_down, fused_gate_up, align):
