@@ -40,7 +40,7 @@ def test_range_tables(cuda_lib, s, kind):
 
 
 @pytest.mark.parametrize("causal,window", [(True, None), (False, None), (True, 70)])
-@pytest.mark.parametrize("s", [40, 128, 129, 320, 777])
+@pytest.mark.parametrize("s", [40, 129, 256, 257, 320, 777])
 @pytest.mark.parametrize("kind", ["sorted", "one", "blocks", "mixed"])
 def test_forward_and_backward(cuda_lib, s, kind, causal, window):
   """Against the fp32 definition; the bound is that of the unsegmented kernels' tests."""
@@ -60,9 +60,9 @@ def test_forward_and_backward(cuda_lib, s, kind, causal, window):
 
 def test_keys_and_queries_with_other_ids(cuda_lib):
   """Key ids of their own: a query tile whose segment no key has gives zeros and zero gradients."""
-  q, k, v = (torch.randn(1, 300, 2, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
-  q_seg = torch.zeros(1, 300, dtype=torch.int32, device="cuda")
-  kv_seg = torch.zeros(1, 300, dtype=torch.int32, device="cuda")
+  q, k, v = (torch.randn(1, 400, 2, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(3))
+  q_seg = torch.zeros(1, 400, dtype=torch.int32, device="cuda")
+  kv_seg = torch.zeros(1, 400, dtype=torch.int32, device="cuda")
   q_seg[:, 128:256] = 9
   o = A.attention(q, k, v, causal=False, q_segment_ids=q_seg, kv_segment_ids=kv_seg)
   dq, dk, dv = torch.autograd.grad(o, (q, k, v), torch.randn_like(o))

@@ -88,8 +88,10 @@ def _i32(t):
 
 def _seg_ranges(q_seg, kv_seg, b, sq, sk):
   """(smallest, largest) segment id of every 64 queries and of every 64 keys: the kernels skip key
-  blocks that share no segment with a query tile.  (None, None) without segments."""
-  if q_seg is None or kv_seg is None:
+  blocks that share no segment with a query tile.  (None, None) without segments, and up to 256 keys, where
+  there is next to nothing to skip and the table's launches cost more than they save (forward and backward of
+  100 tokens, 32 heads: 167 us without, 185 before there was a table; from 300 tokens on 183 with and before)."""
+  if q_seg is None or kv_seg is None or sk <= 256:
     return None, None
 
   def table(seg, s):
@@ -102,7 +104,8 @@ def _seg_ranges(q_seg, kv_seg, b, sq, sk):
   return (kv if same else table(q_seg, sq)), kv
 
 
-def attn_fwd(q, k, v, causal=True, scale=None, window=None, q_pos=None, q_seg=None, kv_seg=None, softcap=None):
+def attn_fwd(q, k, v, causal=True, scale=None, window=None, q_pos=None, q_seg=None, kv_seg=None, softcap=None,
+             ranges=None):
   """Returns (o [B,Sq,Hq,128] contiguous, lse [B,Hq,Sq] fp32 in natural-log units).  ``softcap``: the scores
   become ``softcap * tanh(q.k * scale / softcap)`` before the softmax."""
   b, sq, hq, dqk = q.shape
@@ -110,7 +113,7 @@ def attn_fwd(q, k, v, causal=True, scale=None, window=None, q_pos=None, q_seg=No
   scale = scale if scale is not None else 1.0 / math.sqrt(dqk)
   o = torch.empty(b, sq, hq, dv, dtype=q.dtype, device=q.device)
   lse = torch.empty(b, hq, sq, dtype=torch.float32, device=q.device)
-  q_rng, kv_rng = _seg_ranges(q_seg, kv_seg, b, sq, sk)
+  q_rng, kv_rng = ranges if ranges is not None else _seg_ranges(q_seg, kv_seg, b, sq, sk)
   rc = lib().tpb_attn_fwd_softcap(ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), b, sq, sk, hq, hkv, dqk, dv, q.stride(1),
                                   k.stride(1), v.stride(1), hq * dv, float(scale), int(bool(causal)),
                                   int(window or 0), ptr(q_pos), ptr(q_seg), ptr(kv_seg), ptr(q_rng), ptr(kv_rng),
@@ -120,7 +123,7 @@ def attn_fwd(q, k, v, causal=True, scale=None, window=None, q_pos=None, q_seg=No
 
 
 def attn_bwd(do, q, k, v, o, lse, causal=True, scale=None, window=None, q_pos=None, q_seg=None, kv_seg=None,
-             dq=None, dk=None, dv=None, softcap=None):
+             dq=None, dk=None, dv=None, softcap=None, ranges=None):
   """Gradients of :func:`attn_fwd`.  dq/dk/dv may be preallocated token-major views (for
   example slices of one fused dQKV buffer); they are fully overwritten."""
   b, sq, hq, dqk = q.shape
@@ -136,7 +139,7 @@ def attn_bwd(do, q, k, v, o, lse, causal=True, scale=None, window=None, q_pos=No
     if sq > _MAX_WIDE_QUERIES:
       return _eager_bwd(do, q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv)
   scratch = torch.empty(2 * b * hq * ((sq + 127) // 128 * 128), dtype=torch.float32, device=q.device)
-  q_rng, kv_rng = _seg_ranges(q_seg, kv_seg, b, sq, sk)
+  q_rng, kv_rng = ranges if ranges is not None else _seg_ranges(q_seg, kv_seg, b, sq, sk)
   rc = lib().tpb_attn_bwd_softcap(ptr(do), ptr(q), ptr(k), ptr(v), ptr(o), ptr(lse), ptr(scratch), ptr(dq),
                                   ptr(dk), ptr(dv), b, sq, sk, hq, hkv, dqk, dvd, q.stride(1), k.stride(1),
                                   v.stride(1), do.stride(1), dq.stride(1), dk.stride(1), dv.stride(1), float(scale),
@@ -186,14 +189,15 @@ def _eager_bwd(do, q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk,
 class _AttentionFn(torch.autograd.Function):
   @staticmethod
   def forward(ctx, q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, softcap=None):
-    o, lse = attn_fwd(q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, softcap)
-    ctx.save_for_backward(q, k, v, o, lse, q_pos, q_seg, kv_seg)
+    ranges = _seg_ranges(q_seg, kv_seg, q.shape[0], q.shape[1], k.shape[1])
+    o, lse = attn_fwd(q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, softcap, ranges)
+    ctx.save_for_backward(q, k, v, o, lse, q_pos, q_seg, kv_seg, *ranges)
     ctx.args = (causal, scale, window, softcap)
     return o
 
   @staticmethod
   def backward(ctx, do):
-    q, k, v, o, lse, q_pos, q_seg, kv_seg = ctx.saved_tensors
+    q, k, v, o, lse, q_pos, q_seg, kv_seg, *ranges = ctx.saved_tensors
     causal, scale, window, softcap = ctx.args
     dq = dk = dv = None
     fused = _fused_qkv_layout(q, k, v)
@@ -207,7 +211,7 @@ class _AttentionFn(torch.autograd.Function):
       dq = buf[..., : hq * d].view(b, s, hq, d)
       dk = buf[..., hq * d: (hq + hkv) * d].view(b, s, hkv, d)
       dv = buf[..., (hq + hkv) * d:].view(b, s, hkv, d)
-    dq, dk, dv = attn_bwd(do, q, k, v, o, lse, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv, softcap)
+    dq, dk, dv = attn_bwd(do, q, k, v, o, lse, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv, softcap, ranges)
     return dq, dk, dv, None, None, None, None, None, None, None
 
 
@@ -225,14 +229,15 @@ class _AttentionQKVFn(torch.autograd.Function):
     q = qkv[..., : hq * d].view(b, s, hq, d)
     k = qkv[..., hq * d: (hq + hkv) * d].view(b, s, hkv, d)
     v = qkv[..., (hq + hkv) * d:].view(b, s, hkv, d)
-    o, lse = attn_fwd(q, k, v, causal, scale, window, q_pos, q_seg, kv_seg)
-    ctx.save_for_backward(qkv, o, lse, q_pos, q_seg, kv_seg)
+    ranges = _seg_ranges(q_seg, kv_seg, b, s, s)
+    o, lse = attn_fwd(q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, ranges=ranges)
+    ctx.save_for_backward(qkv, o, lse, q_pos, q_seg, kv_seg, *ranges)
     ctx.args = (hq, hkv, d, causal, scale, window)
     return o
 
   @staticmethod
   def backward(ctx, do):
-    qkv, o, lse, q_pos, q_seg, kv_seg = ctx.saved_tensors
+    qkv, o, lse, q_pos, q_seg, kv_seg, *ranges = ctx.saved_tensors
     hq, hkv, d, causal, scale, window = ctx.args
     b, s, _ = qkv.shape
     q = qkv[..., : hq * d].view(b, s, hq, d)
@@ -242,7 +247,7 @@ class _AttentionQKVFn(torch.autograd.Function):
     dq = buf[..., : hq * d].view(b, s, hq, d)
     dk = buf[..., hq * d: (hq + hkv) * d].view(b, s, hkv, d)
     dv = buf[..., (hq + hkv) * d:].view(b, s, hkv, d)
-    attn_bwd(do, q, k, v, o, lse, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv)
+    attn_bwd(do, q, k, v, o, lse, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv, ranges=ranges)
     return buf, None, None, None, None, None, None, None, None, None
 
 
