@@ -153,6 +153,19 @@ def test_route_of_the_few_rows_path():
   assert moe.few_rows_align(256, 6, 64) == 32 and moe.few_rows_align(257, 6, 64) is None
 
 
+def test_no_tokens(cuda_lib):
+  """Without tokens no expert is hit: an empty result, recorded or not."""
+  assert moe.few_rows_align(0, 6, 64) is None
+  wg, wu = (torch.randn(8, 128, 64, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+  wd = torch.randn(8, 64, 128, device="cuda", dtype=torch.bfloat16)
+  x = torch.empty(0, 128, device="cuda", dtype=torch.bfloat16)
+  w, idx = torch.empty(0, 2, device="cuda"), torch.empty(0, 2, device="cuda", dtype=torch.int32)
+  for recorded in (False, True):
+    with torch.set_grad_enabled(recorded):
+      y = moe.grouped_mlp(x, w, idx, wg, wu, wd)
+    assert y.shape == (0, 128) and y.dtype == x.dtype
+
+
 def test_linear_f32_logits(cuda_lib):
   from torchprime_b200.ops import functional as ops
   x = torch.randn(3, 256, device="cuda", dtype=torch.bfloat16)
