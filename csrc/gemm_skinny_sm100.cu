@@ -21,6 +21,14 @@
 // [K][T] too (weight gradients with few tiles: C = dY^T X contracts over the tokens).  With the SwiGLU
 // epilogue a tile is 64 gate and the same 64 up features.  Grouped mode: rows are grouped by expert in
 // segments padded to the token-tile width, so a token tile belongs to one expert.
+//
+// F32 instantiations are for results that are kept in fp32 (router and inference logits).  The tensor core cuts an
+// accumulator to 24 bits after every MMA, towards zero: over K = 2048 such a sum is 2e-6 off, an fp32 one 1e-7.  Here
+// every MMA (16 products) starts from zero in columns of its own, and warps 2..5 add up the results k-block by k-block
+// as pairs of floats (sum and what the sum's rounding lost).  Distance from 64 bits 3e-8 to 5e-8 for K from 512 to 7168,
+// where the library's fp32 product of fp32 copies is 6e-8 to 1.2e-6 off.  Bound by memory for a vocabulary head and by those
+// additions for a router; us, this / sums left in the accumulator / library: 4 x 102,400 x 2048 71 / 68 / 790,
+// 1500 x 64 x 2048 15 / 7 / 46, 3000 x 256 x 7168 119 / 20 / 353.
 
 #include "common.cuh"
 #include "tpb.h"
@@ -65,6 +73,13 @@ struct SkinnyParams {
   int* status;
 };
 
+// (hi, lo) += c, with lo the sum of hi's rounding errors.
+__device__ __forceinline__ void add_two(float& hi, float& lo, float c) {
+  const float s = __fadd_rn(hi, c), t = __fsub_rn(s, hi);
+  lo = __fadd_rn(lo, __fadd_rn(__fsub_rn(hi, __fsub_rn(s, t)), __fsub_rn(c, t)));
+  hi = s;
+}
+
 __device__ __forceinline__ float4 ld_dsmem4(uint32_t addr) {
   float4 v;
   asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
@@ -87,6 +102,16 @@ __device__ __forceinline__ float4 sum_partials(uint32_t local_addr, int splits) 
   return a;
 }
 
+// The same for partials kept as pairs (`lo_off` bytes apart), added in 64 bits and rounded once.
+__device__ __forceinline__ float4 sum_pairs(uint32_t local_addr, uint32_t lo_off, int splits) {
+  double a[4] = {};
+  for (int s = 0; s < splits; ++s) {
+    const float4 h = ld_dsmem4(map_to_cta(local_addr, s)), l = ld_dsmem4(map_to_cta(local_addr + lo_off, s));
+    a[0] += (double)h.x + l.x; a[1] += (double)h.y + l.y; a[2] += (double)h.z + l.z; a[3] += (double)h.w + l.w;
+  }
+  return make_float4((float)a[0], (float)a[1], (float)a[2], (float)a[3]);
+}
+
 // `n` (1..4) consecutive bf16 results; 8-byte store when all four exist.
 __device__ __forceinline__ void store4(__nv_bfloat16* dst, const float4& v, int n) {
   if (n >= 4) {
@@ -97,13 +122,15 @@ __device__ __forceinline__ void store4(__nv_bfloat16* dst, const float4& v, int 
   }
 }
 
-template <int NT, bool W_MN, bool X_MN>
+template <int NT, bool W_MN, bool X_MN, bool F32>
 __global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
                    const __grid_constant__ CUtensorMap tmX, const SkinnyParams p) {
   using L = SkinnySmem<NT>;
   constexpr int NST = L::STAGES;
-  constexpr uint32_t TMEM_COLS = NT < 32 ? 32 : NT;
+  constexpr int KSTEPS = SK_BK / 16;
+  constexpr uint32_t TMEM_COLS = F32 ? 2 * KSTEPS * NT : NT < 32 ? 32 : NT;   // F32: two buffers of a k-block's results
+  static_assert(!F32 || (TMEM_COLS <= 256 && 2 * NT * SK_TN * 4 <= L::RING), "two CTAs per SM; pairs fit the ring");
   const bool swiglu = p.epi == TPB_EPI_SWIGLU;
   const int rank = (int)blockIdx.x % p.splits;          // == %cluster_ctarank of the 1-D cluster
   const int unit = (int)blockIdx.x / p.splits;
@@ -121,7 +148,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::RING);
   uint64_t* empty = full + NST;
   uint64_t* acc_full = empty + NST;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_full + 1);
+  uint64_t* blk_full = acc_full + 1;      // F32: [2] a k-block's results are in their buffer
+  uint64_t* blk_empty = blk_full + 2;     // F32: [2] and have been read (one arrival per warp)
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(blk_empty + 2);
   float* part = reinterpret_cast<float*>(smem);         // [NT][128] after the main loop
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -133,6 +162,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       mbar_init(&empty[s], 1);
     }
     mbar_init(acc_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&blk_full[i], 1);
+      mbar_init(&blk_empty[i], 4);
+    }
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -185,23 +218,74 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       bool ok = true;
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(&full[stage], phase, p.status, kTimeoutTmaFull, 82)) { ok = false; break; }
+        const int blk = kb - kb0;
+        if (F32 && !mbar_wait(&blk_empty[blk & 1], ((blk >> 1) & 1) ^ 1, p.status, kTimeoutAccFree, 84)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sW = base + stage * L::STAGE;
         const uint32_t a_lo = smem_desc_lo(sW, W_MN ? 8192 : 16);
         const uint32_t b_lo = smem_desc_lo(sW + SK_W_BYTES, X_MN ? 8192 : 16);
 #pragma unroll
-        for (int k = 0; k < SK_BK / 16; ++k)
-          mma_ss_w(tmem_base, a_lo + (W_MN ? k * 128 : k * 2), desc_hi, b_lo + (X_MN ? k * 128 : k * 2),
+        for (int k = 0; k < KSTEPS; ++k)
+          mma_ss_w(F32 ? tmem_base + ((blk & 1) * KSTEPS + k) * NT : tmem_base, a_lo + (W_MN ? k * 128 : k * 2), desc_hi, b_lo + (X_MN ? k * 128 : k * 2),
                    desc_hi, idesc,
-                   ((kb - kb0) | k) != 0);
+                   !F32 && (blk | k) != 0);
         tc_commit(&empty[stage]);
+        if (F32) tc_commit(&blk_full[blk & 1]);
         if (++stage == NST) {
           stage = 0;
           phase ^= 1;
         }
       }
-      if (ok) tc_commit(acc_full);
+      if (ok && !F32) tc_commit(acc_full);
     }
+  } else if (F32) {
+    const int q = warp & 3;
+    const uint32_t t_addr = tmem_base + ((uint32_t)(q * 32) << 16);
+    const int live = min(NT, p.T - t0);          // tokens of this tile
+    float hi[NT], lo[NT];
+#pragma unroll
+    for (int j = 0; j < NT; ++j) hi[j] = lo[j] = 0.f;
+    bool have = true;
+    for (int kb = kb0; kb < kb1; ++kb) {
+      const int blk = kb - kb0;
+      have = __all_sync(0xffffffffu, mbar_wait(&blk_full[blk & 1], (blk >> 1) & 1, p.status, kTimeoutAccFull, 85));
+      if (!have) break;
+      tc_fence_after();
+      constexpr int PER = 64 / NT;               // MMAs whose results are read together
+#pragma unroll
+      for (int k0 = 0; k0 < KSTEPS; k0 += PER) {
+        uint32_t v[64];
+#pragma unroll
+        for (int k = 0; k < PER; ++k) {
+          const uint32_t col = t_addr + ((blk & 1) * KSTEPS + k0 + k) * NT;
+          if (NT == 16) tmem_ld16(col, v + k * NT); else tmem_ld32(col, v + k * NT);
+        }
+        tmem_wait_ld();
+        if (k0 + PER == KSTEPS) {
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&blk_empty[blk & 1]);
+        }
+#pragma unroll
+        for (int j0 = 0; j0 < NT; j0 += 4)
+          if (j0 < live) {
+#pragma unroll
+            for (int j = j0; j < j0 + 4; ++j) {
+              float c = __fadd_rn(__uint_as_float(v[j]), __uint_as_float(v[NT + j]));
+              if (PER == 4) c = __fadd_rn(c, __fadd_rn(__uint_as_float(v[2 * NT + j]), __uint_as_float(v[3 * NT + j])));
+              add_two(hi[j], lo[j], c);
+            }
+          }
+      }
+    }
+    if (have) {                                  // (every MMA has read its operands: the ring is free)
+#pragma unroll
+      for (int j = 0; j < NT; ++j) {
+        part[j * SK_TN + q * 32 + lane] = hi[j];
+        part[(NT + j) * SK_TN + q * 32 + lane] = fabsf(hi[j]) <= 3.402823466e38f ? lo[j] : 0.f;   // inf and NaN stay as they are
+      }
+    }
+    tc_fence_before();
   } else {
     // accumulator lane = feature, column = token: part[token][feature], conflict-free
     const int q = warp & 3;
@@ -239,7 +323,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const int row = t0 + t, col = n0 + c;
       if (row >= p.T || col >= p.N) continue;
       const int n = min(4, p.N - col);
-      float4 a = sum_partials(smem_u32(part + t * SK_TN + c), p.splits);
+      float4 a = F32 ? sum_pairs(smem_u32(part + t * SK_TN + c), NT * SK_TN * 4, p.splits)
+                     : sum_partials(smem_u32(part + t * SK_TN + c), p.splits);
       a.x *= p.alpha; a.y *= p.alpha; a.z *= p.alpha; a.w *= p.alpha;
       if (swiglu) {
         float4 u = sum_partials(smem_u32(part + t * SK_TN + SK_TN / 2 + c), p.splits);
@@ -283,12 +368,12 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   }
 }
 
-template <int NT, bool W_MN, bool X_MN = false>
+template <int NT, bool W_MN, bool X_MN = false, bool F32 = false>
 static cudaError_t launch_skinny(const CUtensorMap& tw, const CUtensorMap& tw2, const CUtensorMap& tx,
                                  const SkinnyParams& p, int grid, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<NT, W_MN, X_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<NT, W_MN, X_MN, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          SkinnySmem<NT>::TOTAL);
     if (e != cudaSuccess) return e;
     configured = true;
@@ -305,7 +390,7 @@ static cudaError_t launch_skinny(const CUtensorMap& tw, const CUtensorMap& tw2, 
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<NT, W_MN, X_MN>, tw, tw2, tx, p);
+  return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<NT, W_MN, X_MN, F32>, tw, tw2, tx, p);
 }
 
 // Token-tile width for `rows` rows: the smallest one that holds them, 128 at most.
@@ -346,11 +431,12 @@ bool skinny_wins_wgrad(int M, int N, int K) {
 
 // x [T,K], or [K,T] with x_mn (for grouped mode: all padded rows), w dense [N,K] (w_mn = 0) or [K,N] (w_mn = 1), with
 // `experts` of them `w_stride` elements apart.  N counts both halves for SwiGLU.  nt / splits 0: by
-// the rules above.  Returns -2 when the shape or alignment is not supported.
+// the rules above.  f32: sums as exact as fp32 ones (the F32 kernels; w [N,K], x [T,K]).  Returns -2 when the shape or
+// alignment is not supported.
 int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, int experts,
                 long long ldx, long long ldw, long long w_stride, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                 const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit,
-                int nt, int splits, cudaStream_t stream) {
+                int nt, int splits, cudaStream_t stream, bool f32) {
   if (T <= 0 || N <= 0 || K <= 0) return 0;
   const bool swiglu = epi == TPB_EPI_SWIGLU;
   if (!swiglu && epi != TPB_EPI_BF16 && epi != TPB_EPI_BF16_RES && epi != TPB_EPI_F32) return -2;
@@ -365,7 +451,8 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
   const int extent = two_w ? N / 2 : N;
   const int tile_n = swiglu ? SK_TN / 2 : SK_TN;
   const int n_out = swiglu ? N / 2 : N;
-  if (nt == 0) nt = skinny_nt(T);
+  if (nt == 0) nt = f32 && T > 16 ? 32 : skinny_nt(T);
+  if (f32 && (epi != TPB_EPI_F32 || x_mn || w_mn || tile_expert || nt > 32)) return -2;
   if (x_mn) {
     if (!w_mn || swiglu || tile_expert) return -2;
     if (nt < 64) nt = 64;       // X arrives in blocks of 64 rows
@@ -407,7 +494,10 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
   cudaError_t e;
 #define TPB_SK(NT_) (w_mn ? launch_skinny<NT_, true>(tw, tw2, tx, p, grid, stream) \
                           : launch_skinny<NT_, false>(tw, tw2, tx, p, grid, stream))
-  if (x_mn)
+  if (f32)
+    e = nt == 16 ? launch_skinny<16, false, false, true>(tw, tw2, tx, p, grid, stream)
+                 : launch_skinny<32, false, false, true>(tw, tw2, tx, p, grid, stream);
+  else if (x_mn)
     e = nt == 64 ? launch_skinny<64, true, true>(tw, tw2, tx, p, grid, stream)
                  : launch_skinny<128, true, true>(tw, tw2, tx, p, grid, stream);
   else switch (nt) {
@@ -425,13 +515,20 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
 
 using namespace tpb;
 
+// y = x w^T of bf16 operands in fp32: x [T,K], w [N,K], y [T,N].
+extern "C" int tpb_linear_f32(const void* x, const void* w, float* y, int T, int N, int K, long long ldx, long long ldw,
+                              long long ldy, void* stream) {
+  return skinny_gemm(x, w, nullptr, y, T, N, K, 1, ldx, ldw, 0, ldy, 0, 0, TPB_EPI_F32, 1.0f, nullptr, 0, nullptr, 0, nullptr,
+                     0, 0, 0, reinterpret_cast<cudaStream_t>(stream), true);
+}
+
 // The kernel with an explicit token-tile width and K split (0: by rule); see tpb_gemm_bf16 for the rest.
 extern "C" int tpb_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, int T, int N, int K,
                                     long long ldx, long long ldw, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                                     const void* aux, long long ldaux, void* c2, long long ldc2, int nt, int splits,
                                     void* stream) {
   return skinny_gemm(x, w, w2, c, T, N, K, 1, ldx, ldw, 0, ldc, x_mn, w_mn, epi, alpha, aux, ldaux, c2, ldc2, nullptr, 0, nt,
-                     splits, reinterpret_cast<cudaStream_t>(stream));
+                     splits, reinterpret_cast<cudaStream_t>(stream), false);
 }
 
 // Rows grouped by expert in segments padded to `nt` rows; tile_expert[rows / nt].  Token tiles of expert -1
@@ -442,5 +539,5 @@ extern "C" int tpb_grouped_gemm_skinny_bf16(const void* x, const void* w, const 
                                             int nt, void* stream) {
   if (!tile_expert || E < 1 || experts_hit < 1) return -2;
   return skinny_gemm(x, w, w2, c, rows, N, K, E, ldx, ldw, w_stride, ldc, 0, w_mn, epi, 1.0f, nullptr, 0, nullptr, 0,
-                     tile_expert, experts_hit, nt, 0, reinterpret_cast<cudaStream_t>(stream));
+                     tile_expert, experts_hit, nt, 0, reinterpret_cast<cudaStream_t>(stream), false);
 }

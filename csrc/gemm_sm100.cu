@@ -884,7 +884,7 @@ cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const
 int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, int experts,
                 long long ldx, long long ldw, long long w_stride, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                 const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit, int nt,
-                int splits, cudaStream_t stream);
+                int splits, cudaStream_t stream, bool f32);
 bool skinny_wins(int M, int N, int K, bool swiglu);
 bool skinny_wins_wgrad(int M, int N, int K);
 
@@ -1077,7 +1077,7 @@ extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, int M, int N
   if (max_ctas == 0 && gemm_pair_mode() == 1 &&
       (a_mn ? b_mn && skinny_wins_wgrad(M, N, K) : skinny_wins(M, N, K, epi == TPB_EPI_SWIGLU))) {
     const int r = skinny_gemm(A, B, nullptr, C, M, N, K, 1, lda, ldb, 0, ldc, a_mn, b_mn, epi, alpha, aux, ldaux, c2, ldc2,
-                              nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_));
+                              nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_), false);
     if (r != -2) return r;     // -2: an epilogue or alignment it does not take
   }
   GemmCall g{};

@@ -205,6 +205,9 @@ int tpb_scale_cast_bf16(const float* src, void* dst, long long n, const float* s
 int tpb_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, long long ldx,
                          long long ldw, long long ldc, int x_mn, int w_mn, int epi, float alpha, const void* aux,
                          long long ldaux, void* c2, long long ldc2, int nt, int splits, void* stream);
+// y = x w^T in fp32 with sums as exact as fp32 ones: x [T,K], w [N,K] bf16, 16-byte aligned rows; ldy % 4 == 0
+int tpb_linear_f32(const void* x, const void* w, float* y, int T, int N, int K, long long ldx, long long ldw, long long ldy,
+                   void* stream);
 
 // ---- cached latent attention, one token per sequence (mla_decode.cu)
 int tpb_mla_decode_ranges(int B, int H, int n_keys);

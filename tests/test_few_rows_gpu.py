@@ -177,6 +177,36 @@ def test_linear_f32_logits(cuda_lib):
   w.requires_grad_(True)
   assert ops.linear_f32(x, w).requires_grad
 
+
+@pytest.mark.parametrize("shift", [0.0, 0.5])
+@pytest.mark.parametrize("t,n,kk", [(1, 64, 2048), (4, 102400, 2048), (1500, 64, 2048), (16, 256, 7168), (17, 1000, 520), (33, 8, 8),
+                                    (2, 136, 72), (300, 256, 7168)])
+def test_linear_f32_is_as_exact_as_fp32(cuda_lib, t, n, kk, shift):
+  """Distance from 64 bits: what an MMA gives for 16 products and the sum are cut to 24 bits once each (2^-24 of
+  their size on average); and not above the fp32 library product's by more than the last rounding."""
+  from torchprime_b200.ops import functional as ops
+  torch.manual_seed(t + n)
+  x = (torch.randn(t, kk, device="cuda") + shift).to(torch.bfloat16)
+  w = ((torch.randn(n, kk, device="cuda") + shift) / 50).to(torch.bfloat16)
+  want = torch.cat([x.double() @ part.double().t() for part in w.split(8192)], 1)
+  far = lambda y: ((y.double() - want).norm() / want.norm()).item()  # noqa: E731
+  with torch.no_grad():
+    got = far(ops.linear_f32(x, w))
+  assert got < 2.0 ** -23
+  assert got < far(torch.nn.functional.linear(x.float(), w.float())) + 2.0 ** -25
+
+
+def test_linear_f32_not_finite(cuda_lib):
+  from torchprime_b200.ops import functional as ops
+  x = torch.randn(20, 512, device="cuda", dtype=torch.bfloat16)
+  w = torch.randn(64, 512, device="cuda", dtype=torch.bfloat16)
+  x[3, 7], x[4, 500], x[18, 0] = float("inf"), float("-inf"), float("nan")
+  with torch.no_grad():
+    got = ops.linear_f32(x, w)
+  want = torch.nn.functional.linear(x.float(), w.float())
+  assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[3:5], want[3:5])
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 64, 128), (77, 512, 256), (128, 1000, 136), (300, 512, 512), (700, 64, 2048)])
 def test_route_of_a_gemm_call(cuda_lib, M, N, K):
   """Calls the rule gives to this kernel against the tiled kernel (max_ctas keeps a call there)."""

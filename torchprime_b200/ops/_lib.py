@@ -75,6 +75,7 @@ def _declare(L):
     "tpb_embedding_bwd": [P, P, P, I, I, LL, LL, I, P],
     "tpb_cast_f32_to_bf16": [P, P, LL, F, I, P],
     "tpb_scale_cast_bf16": [P, P, LL, P, P],
+    "tpb_linear_f32": [P, P, P, I, I, I, LL, LL, LL, P],
     "tpb_mla_pack": [P, P, LL, P, P, LL, I, I, I, I, P],
     "tpb_mla_unpack": [P, P, P, P, LL, I, I, I, I, P],
   }

@@ -64,6 +64,16 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, epi=EPI_BF16, alpha=1.0, aux
   return out
 
 
+def linear_f32(x, w):
+  """x @ w^T of bf16 operands [T,K] and [N,K] in fp32, with sums as exact as fp32 ones."""
+  t, kk, ldx = _row_major_2d(x, "x")
+  n, kw, ldw = _row_major_2d(w, "w")
+  assert x.dtype == w.dtype == torch.bfloat16 and kk == kw
+  out = torch.empty(t, n, dtype=torch.float32, device=x.device)
+  check(lib().tpb_linear_f32(ptr(x), ptr(w), ptr(out), t, n, kk, ldx, ldw, n, stream_ptr()), f"linear_f32 {t}x{n}x{kk}")
+  return out
+
+
 def rmsnorm_fwd(x, w, eps, res=None, want_h=False):
   """Returns (y, rstd, h) with h = x + res (None unless ``res`` given and ``want_h``)."""
   d = x.shape[-1]
