@@ -71,6 +71,7 @@ struct AttnBwdParams {
   const int2* kv_rng;   // (attn_seg_ranges_kernel of the forward)
   const float* lse2;    // [B,Hq,Sq_pad] log-sum-exp in log2 units, +inf in the padding rows
   const float* delta;   // [B,Hq,Sq_pad] rowsum(dO o O), 0 in the padding rows
+  float* delta_out;     // the same, for the kernel that replaces it (attn_bwd_dq192_kernel<true>)
   int Sq_pad;           // Sq rounded up to 128
   int aux_bulk;         // q_pos / q_seg rows can be bulk-copied (16-byte aligned for every tile)
   __nv_bfloat16* dQ; long long lddq;
@@ -854,7 +855,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 //          accumulators and two score tiles would need 576 columns.)
 //   dQ:    128 x 128 tiles, one S buffer: S(j + 1) is issued as soon as the compute warps hold S(j) in
 //          registers.  TMEM: dQ [0,192), S [192,320), dP [320,448).
-// One row of 2048 tokens, 16 heads, causal: dK/dV 69, dQ 42, delta 8 us.  (torch's scaled_dot_product_attention, used
+// P stays in fp32 until dS = P o (dP - delta) is formed, which is rounded once.
+// FINE: masked calls, whose gradients are those of fp32 probabilities.  P and dS enter the products as two bf16 terms
+// (x = hi + lo to 2^-17; the second term lies in the columns the first leaves free), and the dQ kernel, run first, makes a
+// pass of its own over the keys for delta = rowsum(P o dP), which from the bf16 result would carry its rounding.  Error of
+// dq / dk / dv against 64 bits, 1024 tokens in segments: 1.66e-3, the rounding of the gradients themselves (single bf16 terms:
+// 3.5e-3, 3.5e-3, 2.3e-3).
+// One row of 2048 tokens, 16 heads, causal: dK/dV 70, dQ 44, delta 8 us; with all tokens in one segment, so that FINE does it, 1.4
+// times that.  (torch's scaled_dot_product_attention, used
 // here before: backward 90 us after running its own forward again, 41 us, and three copies.)
 // ------------------------------------------------------------------------------------------
 constexpr int W_D = 192;                       // query / key head dim
@@ -885,7 +893,8 @@ constexpr int OFF_Q = 0;
 constexpr int OFF_DO = OFF_Q + W_K_BYTES;
 constexpr int OFF_K = OFF_DO + TILE_BYTES;
 constexpr int OFF_V = OFF_K + 2 * W_K_BYTES;
-constexpr int OFF_BAR = OFF_V + TILE_BYTES;
+constexpr int OFF_RED = OFF_V + TILE_BYTES;    // FINE: [2][128] partial deltas of the two column halves
+constexpr int OFF_BAR = OFF_RED + 2 * BWD_T * 4;
 constexpr int TOTAL = OFF_BAR + 256 + 1024;
 static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
 constexpr int T_DQ = 0, T_S = 192, T_DP = 320;
@@ -916,6 +925,23 @@ __device__ __forceinline__ void store_acc_cols(uint32_t tsrc, int c0, int n, __n
   }
 }
 
+// 32 values of a row as a bf16 A operand in 16 TMEM columns; FINE: what the rounding lost in 16 more, `lo_cols` further on.
+template <bool FINE>
+__device__ __forceinline__ void store_operand(uint32_t dst, int lo_cols, const float* v) {
+  uint32_t hi[16], lo[16];
+#pragma unroll
+  for (int c = 0; c < 16; ++c) {
+    hi[c] = pack_bf16(v[2 * c], v[2 * c + 1]);
+    if (FINE) {
+      const float2 h = unpack_bf16(hi[c]);     // (no second term for what is not finite)
+      lo[c] = pack_bf16(fabsf(h.x) < INFINITY ? v[2 * c] - h.x : 0.f, fabsf(h.y) < INFINITY ? v[2 * c + 1] - h.y : 0.f);
+    }
+  }
+  tmem_st16(dst, hi);
+  if (FINE) tmem_st16(dst + lo_cols, lo);
+}
+
+template <bool FINE>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                        const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -1071,7 +1097,7 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       const uint32_t aQ0 = smem_u32(smem + OFF_Q), aDO0 = smem_u32(smem + OFF_DO);
       const uint32_t tDP = tmem_base + T_DP;
       // k-step k of a K-major tile of `rows` rows in 64-wide blocks, and the TMEM column of a bf16 A operand
-      // whose halves of 32 values lie packed at the start of their own 32 columns
+      // whose halves of 32 values lie packed at the start of their own 32 columns (FINE: second terms behind them)
       auto kstep = [](int rows, int k) { return (uint32_t)(((k >> 2) * (rows * 128) + (k & 3) * 32) >> 4); };
       auto acol = [](int k) { return (uint32_t)((k >> 1) * 32 + (k & 1) * 8); };
       auto wait_q = [&](int i) { return mbar_wait(&q_full[i % W_STAGES], (i / W_STAGES) & 1, p.status, kTimeoutTmaFull, 123); };
@@ -1107,16 +1133,20 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         tc_fence_after();
         const uint32_t mDO = smem_desc_lo(aDO0 + st * W_DO_BYTES, W_QT * 128);
 #pragma unroll
-        for (int k = 0; k < W_QT / 16; ++k)    // dV += P^T dO
-          mma_ts_w(tmem_base + T_DV, tmem_base + T_S + (i & 1) * W_QT + acol(k), mDO + mnmajor_k(k), kDescHi, id_dv,
-                   (i | k) != 0);
+        for (int k = 0; k < W_QT / 16; ++k) {  // dV += P^T dO
+          const uint32_t a = tmem_base + T_S + (i & 1) * W_QT + acol(k);
+          mma_ts_w(tmem_base + T_DV, a, mDO + mnmajor_k(k), kDescHi, id_dv, (i | k) != 0);
+          if (FINE) mma_ts_w(tmem_base + T_DV, a + 16, mDO + mnmajor_k(k), kDescHi, id_dv, 1);
+        }
         tc_commit(&do_empty[st]);
         if (!mbar_wait(ds_full, i & 1, p.status, kTimeoutSoftmax, 126)) break;
         tc_fence_after();
         const uint32_t mQ = smem_desc_lo(aQ0 + st * W_Q_BYTES, W_QT * 128);
 #pragma unroll
-        for (int k = 0; k < W_QT / 16; ++k)    // dK += dS^T Q
+        for (int k = 0; k < W_QT / 16; ++k) {  // dK += dS^T Q
           mma_ts_w(tmem_base + T_DK, tDP + acol(k), mQ + mnmajor_k(k), kDescHi, id_dk, (i | k) != 0);
+          if (FINE) mma_ts_w(tmem_base + T_DK, tDP + acol(k) + 16, mQ + mnmajor_k(k), kDescHi, id_dk, 1);
+        }
         tc_commit(&q_empty[st]);
         if (more && !issue_dp(i + 1)) break;
       }
@@ -1148,7 +1178,7 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         // ---- phase 1: P^T = exp2(S^T * c - lse)
         if (!mbar_wait(&s_full[step & 1], (step >> 1) & 1, p.status, kTimeoutAccFull, 127)) { ok = false; break; }
         tc_fence_after();
-        uint32_t pk_p[16];
+        float pf[32];
         {
           uint32_t s[32];
           tmem_ld32(tS, s);
@@ -1160,10 +1190,10 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
 #pragma unroll
             for (int c4 = 0; c4 < 8; ++c4) {
               const float4 L = lse4[c4];
-              pk_p[2 * c4] = pack_bf16(exp2f(fmaf(__uint_as_float(s[4 * c4]), p.scale_log2, -L.x)),
-                                       exp2f(fmaf(__uint_as_float(s[4 * c4 + 1]), p.scale_log2, -L.y)));
-              pk_p[2 * c4 + 1] = pack_bf16(exp2f(fmaf(__uint_as_float(s[4 * c4 + 2]), p.scale_log2, -L.z)),
-                                           exp2f(fmaf(__uint_as_float(s[4 * c4 + 3]), p.scale_log2, -L.w)));
+              pf[4 * c4] = exp2f(fmaf(__uint_as_float(s[4 * c4]), p.scale_log2, -L.x));
+              pf[4 * c4 + 1] = exp2f(fmaf(__uint_as_float(s[4 * c4 + 1]), p.scale_log2, -L.y));
+              pf[4 * c4 + 2] = exp2f(fmaf(__uint_as_float(s[4 * c4 + 2]), p.scale_log2, -L.z));
+              pf[4 * c4 + 3] = exp2f(fmaf(__uint_as_float(s[4 * c4 + 3]), p.scale_log2, -L.w));
             }
           } else {
 #pragma unroll
@@ -1174,18 +1204,15 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
               const int4 QS = p.q_seg ? qs4[c4] : make_int4(0, 0, 0, 0);
               const float l[4] = {L.x, L.y, L.z, L.w};
               const int qp[4] = {QP.x, QP.y, QP.z, QP.w}, qs[4] = {QS.x, QS.y, QS.z, QS.w};
-              float pv[4];
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 const bool keep = key_ok & (qp[e] >= cmax) & (qp[e] - kp < win) & (qs[e] == kseg);
                 const float pe = exp2f(fmaf(__uint_as_float(s[4 * c4 + e]), p.scale_log2, -l[e]));
-                pv[e] = keep ? pe : 0.f;
+                pf[4 * c4 + e] = keep ? pe : 0.f;
               }
-              pk_p[2 * c4] = pack_bf16(pv[0], pv[1]);
-              pk_p[2 * c4 + 1] = pack_bf16(pv[2], pv[3]);
             }
           }
-          tmem_st16(tS, pk_p);
+          store_operand<FINE>(tS, 16, pf);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -1194,19 +1221,19 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         if (!mbar_wait(dp_full, step & 1, p.status, kTimeoutAccFull, 128)) { ok = false; break; }
         tc_fence_after();
         {
-          uint32_t d[32], pk_ds[16];
+          uint32_t d[32];
           tmem_ld32(tDP, d);
           tmem_wait_ld();
           const float4* dlt4 = reinterpret_cast<const float4*>(aux + W_QT + half * 32);
 #pragma unroll
           for (int c4 = 0; c4 < 8; ++c4) {
             const float4 Dl = dlt4[c4];
-            pk_ds[2 * c4] = mul_bf16x2(pk_p[2 * c4], pack_bf16(__uint_as_float(d[4 * c4]) - Dl.x,
-                                                               __uint_as_float(d[4 * c4 + 1]) - Dl.y));
-            pk_ds[2 * c4 + 1] = mul_bf16x2(pk_p[2 * c4 + 1], pack_bf16(__uint_as_float(d[4 * c4 + 2]) - Dl.z,
-                                                                       __uint_as_float(d[4 * c4 + 3]) - Dl.w));
+            pf[4 * c4] *= __uint_as_float(d[4 * c4]) - Dl.x;
+            pf[4 * c4 + 1] *= __uint_as_float(d[4 * c4 + 1]) - Dl.y;
+            pf[4 * c4 + 2] *= __uint_as_float(d[4 * c4 + 2]) - Dl.z;
+            pf[4 * c4 + 3] *= __uint_as_float(d[4 * c4 + 3]) - Dl.w;
           }
-          tmem_st16(tDP, pk_ds);
+          store_operand<FINE>(tDP, 16, pf);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -1231,6 +1258,8 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   }
 }
 
+// FINE: the key blocks are run through twice, first for delta (S and dP only), then for dQ.
+template <bool FINE>
 __global__ void __launch_bounds__(BWD_THREADS, 1)
 attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__ CUtensorMap tmK,
                       const __grid_constant__ CUtensorMap tmV, const __grid_constant__ CUtensorMap tmdO,
@@ -1252,6 +1281,7 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 12);
   int* tile_minmax = reinterpret_cast<int*>(bars + 13);   // [2]
   int* seg_lohi = reinterpret_cast<int*>(bars + 14);      // [2]
+  float* red = reinterpret_cast<float*>(smem + OFF_RED);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n_qtiles = (p.Sq + BWD_T - 1) / BWD_T;
@@ -1312,6 +1342,7 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     blk_hi = min(blk_hi, seg_lohi[1] + 1);
   }
   const int nblk = max(0, blk_hi - blk_lo);
+  const int n_steps = FINE ? 2 * nblk : nblk;
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
@@ -1322,9 +1353,9 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         tma_load_3d(smem + OFF_Q + c * (BWD_T * 128), &tmQ, qdo_full, c * 64, b * p.Sq + q0, hq);
       for (int c = 0; c < BWD_D / 64; ++c)
         tma_load_3d(smem + OFF_DO + c * (BWD_T * 128), &tmdO, qdo_full, c * 64, b * p.Sq + q0, hq);
-      for (int j = 0; j < nblk; ++j) {
+      for (int j = 0; j < n_steps; ++j) {
         const int st = j & 1;
-        const int row = b * p.Sk + (blk_lo + j) * BWD_T;
+        const int row = b * p.Sk + (blk_lo + (j < nblk ? j : j - nblk)) * BWD_T;
         if (!mbar_wait(&k_empty[st], ((j >> 1) & 1) ^ 1, p.status, kTimeoutStageFree, 131)) break;
         mbar_expect_tx(&k_full[st], W_K_BYTES);
         for (int c = 0; c < W_D / 64; ++c)
@@ -1365,8 +1396,9 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       };
       bool ok = mbar_wait(qdo_full, 0, p.status, kTimeoutTmaFull, 132);
       if (ok) ok = issue_s(0) && issue_dp(0);
-      for (int j = 0; j < nblk && ok; ++j) {
-        const bool more = j + 1 < nblk;
+      for (int j = 0; j < n_steps && ok; ++j) {
+        const bool more = j + 1 < n_steps;
+        const int jq = FINE ? j - nblk : j;      // step of the dQ pass
         if (more) {
           if (!mbar_wait(s_read, j & 1, p.status, kTimeoutSoftmax, 140)) break;   // S(j) is in registers
           tc_fence_after();
@@ -1375,9 +1407,13 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
         if (!mbar_wait(ds_full, j & 1, p.status, kTimeoutSoftmax, 134)) break;
         tc_fence_after();
         const uint32_t mK = mnmajor_lo(aK0 + (j & 1) * W_K_BYTES);
+        if (jq >= 0) {
 #pragma unroll
-        for (int k = 0; k < BWD_T / 16; ++k)   // dQ += dS K
-          mma_ts_w(tmem_base + T_DQ, tDP + a_col(k), mK + mnmajor_k(k), kDescHi, id_dq, (j | k) != 0);
+          for (int k = 0; k < BWD_T / 16; ++k) {   // dQ += dS K
+            mma_ts_w(tmem_base + T_DQ, tDP + a_col(k), mK + mnmajor_k(k), kDescHi, id_dq, (jq | k) != 0);
+            if (FINE) mma_ts_w(tmem_base + T_DQ, tDP + a_col(k) + 32, mK + mnmajor_k(k), kDescHi, id_dq, 1);
+          }
+        }
         tc_commit(&k_empty[j & 1]);
         if (more && !issue_dp(j + 1)) break;
       }
@@ -1395,7 +1431,7 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int qseg = (p.q_seg && row_ok) ? p.q_seg[grow] : 0;
     const long long li = ((long long)b * p.Hq + hq) * p.Sq_pad + row;   // row < Sq_pad: padded to 128
     const float lse2 = p.lse2[li];
-    const float delta = p.delta[li];
+    float delta = FINE ? 0.f : p.delta[li];
     const uint32_t tb = tmem_base + ((uint32_t)(qd * 32) << 16);
     const uint32_t tS = tb + T_S + half * 64, tDP = tb + T_DP + half * 64;
     const int* ks = p.kv_seg ? p.kv_seg + (long long)b * p.Sk : nullptr;
@@ -1403,67 +1439,74 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     const int kmax = p.causal ? min(qpos, p.Sk - 1) : p.Sk - 1;   // keep needs kp <= kmax
     bool ok = true;
 
-    for (int j = 0; j < nblk && ok; ++j) {
-      const int kv0 = (blk_lo + j) * BWD_T;
-      bool seg_mask = p.q_seg != nullptr;
-      if (p.kv_rng) {
-        const int2 kr = seg_range128(p.kv_rng, b, blk_lo + j, p.Sk);
-        seg_mask = !(qr.x == qr.y && kr.x == kr.y && qr.x == kr.x);
-      }
-      const bool need_mask = (p.causal && kv0 + BWD_T - 1 > qpos_min) || (kv0 + BWD_T > p.Sk) ||
-                             (p.window > 0 && qpos_max - kv0 >= p.window) || seg_mask;
-      // ---- phase 1: P = exp2(S * c - lse), packed bf16 in registers
-      if (!mbar_wait(s_full, j & 1, p.status, kTimeoutAccFull, 136)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t pk_p[32];
-      uint32_t sreg[64];
-      tmem_ld32(tS, sreg);
-      tmem_ld32(tS + 32, sreg + 32);
-      tmem_wait_ld();
-      tc_fence_before();
-      mbar_arrive(s_read);
+    for (int pass = FINE ? 0 : 1; pass < 2; ++pass) {
+      float own = 0.f;              // this thread's part of delta
+      for (int jb = 0; jb < nblk && ok; ++jb) {
+        const int j = FINE && pass ? nblk + jb : jb;
+        const int kv0 = (blk_lo + jb) * BWD_T;
+        bool seg_mask = p.q_seg != nullptr;
+        if (p.kv_rng) {
+          const int2 kr = seg_range128(p.kv_rng, b, blk_lo + jb, p.Sk);
+          seg_mask = !(qr.x == qr.y && kr.x == kr.y && qr.x == kr.x);
+        }
+        const bool need_mask = (p.causal && kv0 + BWD_T - 1 > qpos_min) || (kv0 + BWD_T > p.Sk) ||
+                               (p.window > 0 && qpos_max - kv0 >= p.window) || seg_mask;
+        // ---- phase 1: P = exp2(S * c - lse), in registers
+        if (!mbar_wait(s_full, j & 1, p.status, kTimeoutAccFull, 136)) { ok = false; break; }
+        tc_fence_after();
+        float pf[64];
+        uint32_t sreg[64];
+        tmem_ld32(tS, sreg);
+        tmem_ld32(tS + 32, sreg + 32);
+        tmem_wait_ld();
+        tc_fence_before();
+        mbar_arrive(s_read);
 #pragma unroll
-      for (int ch = 0; ch < 2; ++ch) {
-        const uint32_t* s = sreg + ch * 32;
-        if (!need_mask) {
+        for (int ch = 0; ch < 2; ++ch) {
+          const uint32_t* s = sreg + ch * 32;
+          if (!need_mask) {
 #pragma unroll
-          for (int c = 0; c < 32; c += 2)
-            pk_p[ch * 16 + c / 2] = pack_bf16(exp2f(fmaf(__uint_as_float(s[c]), p.scale_log2, -lse2)),
-                                              exp2f(fmaf(__uint_as_float(s[c + 1]), p.scale_log2, -lse2)));
-        } else {
-          const int kbase = kv0 + half * 64 + ch * 32;
+            for (int c = 0; c < 32; ++c) pf[ch * 32 + c] = exp2f(fmaf(__uint_as_float(s[c]), p.scale_log2, -lse2));
+          } else {
+            const int kbase = kv0 + half * 64 + ch * 32;
 #pragma unroll
-          for (int c = 0; c < 32; c += 2) {
-            float pv[2];
-#pragma unroll
-            for (int e = 0; e < 2; ++e) {
-              const int kp = kbase + c + e;
+            for (int c = 0; c < 32; ++c) {
+              const int kp = kbase + c;
               bool keep = (kp <= kmax) & (qpos - kp < win);
               if (ks && seg_mask) keep = keep & (__ldg(ks + min(kp, p.Sk - 1)) == qseg);
-              const float pe = exp2f(fmaf(__uint_as_float(s[c + e]), p.scale_log2, -lse2));
-              pv[e] = keep ? pe : 0.f;
+              const float pe = exp2f(fmaf(__uint_as_float(s[c]), p.scale_log2, -lse2));
+              pf[ch * 32 + c] = keep ? pe : 0.f;
             }
-            pk_p[ch * 16 + c / 2] = pack_bf16(pv[0], pv[1]);
           }
         }
-      }
-      // ---- phase 2: dS = P o (dP - delta), written over dP
-      if (!mbar_wait(dp_full, j & 1, p.status, kTimeoutAccFull, 139)) { ok = false; break; }
-      tc_fence_after();
-      {
-        uint32_t dreg[64], pk[32];
-        tmem_ld32(tDP, dreg);
-        tmem_ld32(tDP + 32, dreg + 32);
-        tmem_wait_ld();
+        // ---- phase 2: dS = P o (dP - delta), written over dP; or this block's share of delta
+        if (!mbar_wait(dp_full, j & 1, p.status, kTimeoutAccFull, 139)) { ok = false; break; }
+        tc_fence_after();
+        {
+          uint32_t dreg[64];
+          tmem_ld32(tDP, dreg);
+          tmem_ld32(tDP + 32, dreg + 32);
+          tmem_wait_ld();
+          if (pass == 0) {
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
-          pk[c] = mul_bf16x2(pk_p[c], pack_bf16(__uint_as_float(dreg[2 * c]) - delta,
-                                                __uint_as_float(dreg[2 * c + 1]) - delta));
-        tmem_st32(tDP, pk);
+            for (int c = 0; c < 64; ++c) own = fmaf(pf[c], __uint_as_float(dreg[c]), own);
+          } else {
+#pragma unroll
+            for (int c = 0; c < 64; ++c) pf[c] *= __uint_as_float(dreg[c]) - delta;
+            store_operand<FINE>(tDP, 32, pf);
+            store_operand<FINE>(tDP + 16, 32, pf + 32);
+          }
+        }
+        tmem_wait_st();
+        tc_fence_before();
+        mbar_arrive(ds_full);
       }
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(ds_full);
+      if (pass == 0) {              // (reached by every compute thread, whatever became of its waits)
+        red[half * BWD_T + r_local] = own;
+        named_bar_sync(1, 256);
+        delta = row_ok ? red[r_local] + red[BWD_T + r_local] : 0.f;
+        if (half == 0) p.delta_out[li] = delta;
+      }
     }
     if (ok && nblk > 0) ok = mbar_wait(acc_done, 0, p.status, kTimeoutAccFull, 138);
     tc_fence_after();
@@ -1526,7 +1569,7 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
   const bool ranges = q_seg && kv_seg && q_rng && kv_rng;
   p.q_rng = ranges ? reinterpret_cast<const int2*>(q_rng) : nullptr;
   p.kv_rng = ranges ? reinterpret_cast<const int2*>(kv_rng) : nullptr;
-  p.lse2 = lse2; p.delta = delta; p.Sq_pad = sq_pad;
+  p.lse2 = lse2; p.delta = delta; p.delta_out = delta; p.Sq_pad = sq_pad;
   p.aux_bulk = (Sq % 4 == 0) && (reinterpret_cast<uintptr_t>(q_pos) % 16 == 0) &&
                (reinterpret_cast<uintptr_t>(q_seg) % 16 == 0);
   p.dQ = reinterpret_cast<__nv_bfloat16*>(dq); p.lddq = lddq;
@@ -1543,7 +1586,8 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
     allow((const void*)attn_bwd_dkv_kernel<false, true>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<false, true>, dqk::TOTAL);
     allow((const void*)attn_bwd_dkv_kernel<true, false>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<true, false>, dqk::TOTAL);
     allow((const void*)attn_bwd_dkv_kernel<true, true>, dkv::TOTAL); allow((const void*)attn_bwd_dq_kernel<true, true>, dqk::TOTAL);
-    allow((const void*)attn_bwd_dkv192_kernel, wkv::TOTAL); allow((const void*)attn_bwd_dq192_kernel, wdq::TOTAL);
+    allow((const void*)attn_bwd_dkv192_kernel<false>, wkv::TOTAL); allow((const void*)attn_bwd_dq192_kernel<false>, wdq::TOTAL);
+    allow((const void*)attn_bwd_dkv192_kernel<true>, wkv::TOTAL); allow((const void*)attn_bwd_dq192_kernel<true>, wdq::TOTAL);
     if (e != cudaSuccess) return 1000 + (int)e;
     configured = true;
   }
@@ -1558,10 +1602,13 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
     CUtensorMap tq64, tdo64;      // the dK/dV kernel takes its queries 64 rows at a time
     if (make_tmap_3d(&tq64, q, dqk, (uint64_t)B * Sq, Hq, ldq, dqk, 64, W_QT)) return -3;
     if (make_tmap_3d(&tdo64, dO, dvd, (uint64_t)B * Sq, Hq, lddo, dvd, 64, W_QT)) return -5;
-    attn_bwd_dkv192_kernel<<<grid_kv, BWD_THREADS, wkv::TOTAL, stream>>>(tq64, tk, tv, tdo64, p);
+    const bool fine = q_pos || q_seg || kv_seg || window > 0 || (causal && Sq != Sk);
+    const int grid_wq = ((Sq + BWD_T - 1) / BWD_T) * Hq * B;
+    // (FINE: dK/dV takes the deltas that the dQ kernel leaves)
+    (fine ? attn_bwd_dq192_kernel<true> : attn_bwd_dq192_kernel<false>)<<<grid_wq, BWD_THREADS, wdq::TOTAL, stream>>>(tq, tk, tv, tdo, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return 1000 + (int)e;
-    attn_bwd_dq192_kernel<<<((Sq + BWD_T - 1) / BWD_T) * Hq * B, BWD_THREADS, wdq::TOTAL, stream>>>(tq, tk, tv, tdo, p);
+    (fine ? attn_bwd_dkv192_kernel<true> : attn_bwd_dkv192_kernel<false>)<<<grid_kv, BWD_THREADS, wkv::TOTAL, stream>>>(tq64, tk, tv, tdo64, p);
     e = cudaGetLastError();
     return e == cudaSuccess ? 0 : 1000 + (int)e;
   }

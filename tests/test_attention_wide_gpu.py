@@ -56,6 +56,38 @@ def test_positions(cuda_lib):
   _check(1, 128, 384, 2, 2, causal=True, q_positions=pos.long())
 
 
+ROUNDED = 1.66e-3     # relative error (2-norm) of values rounded to bf16 once
+
+
+@pytest.mark.parametrize("sq,sk,kind", [(77, 77, "plain"), (1024, 1024, "plain"), (300, 300, "full"), (77, 77, "segments"),
+                                        (300, 300, "segments"), (1024, 1024, "segments"), (300, 300, "window"),
+                                        (257, 400, "plain"), (128, 384, "positions")])
+def test_roundings(cuda_lib, sq, sk, kind):
+  """Against 64 bits.  Plain calls round P and dS to bf16 once each, the forward's result in delta and the gradient itself;
+  masked ones and those with more keys than queries keep fp32 probabilities, so that only the gradient is rounded."""
+  g = torch.Generator(device="cuda").manual_seed(sq)
+  q, k, v, do = (torch.randn(2, s, 4, d, device="cuda", generator=g).to(torch.bfloat16)
+                 for s, d in ((sq, 192), (sk, 192), (sk, 128), (sq, 128)))
+  kw = {"causal": kind != "full"}
+  if kind == "segments":
+    cuts = torch.randint(0, sq, (2, 4), device="cuda", generator=g)
+    kw["q_segment_ids"] = (torch.arange(sq, device="cuda")[None, :, None] >= cuts[:, None, :]).sum(-1).to(torch.int32)
+  if kind == "window":
+    kw["window"] = 100
+  if kind == "positions":
+    kw["q_positions"] = torch.cat([torch.arange(64, 128), torch.arange(256, 320)]).to("cuda")[None].expand(2, -1).contiguous()
+  lead = [t.requires_grad_(True) for t in (q, k, v)]
+  got = torch.autograd.grad(A.attention(*lead, **kw), lead, do)
+  exact = [t.detach().double().requires_grad_(True) for t in lead]
+  keep = ref.build_mask(sq, sk, "cuda", **kw)
+  p = (torch.einsum("bqhd,bkhd->bhqk", exact[0], exact[1]) * 192 ** -0.5).masked_fill(~keep, float("-inf")).softmax(-1)
+  want = torch.autograd.grad(torch.einsum("bhqk,bkhd->bqhd", p, exact[2]), exact, do.double())
+  fine = kind in ("segments", "window", "positions") or sq != sk
+  for name, a, w in zip("dq dk dv".split(), got, want):
+    err = ((a.double() - w).norm() / w.norm()).item()
+    assert err < (1.03 * ROUNDED if fine else 3 ** 0.5 * ROUNDED), (name, err)
+
+
 def test_reproducible(cuda_lib):
   torch.manual_seed(0)
   q, k = (torch.randn(1, 700, 4, 192, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(2))
