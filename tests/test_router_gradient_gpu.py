@@ -41,3 +41,27 @@ def test_linear_f32_gradients(cuda_lib):
   dy = torch.randn_like(y)
   dx, dw = torch.autograd.grad(y, (x, w), dy)
   assert torch.equal(dx, (dy @ w.float()).to(torch.bfloat16)) and torch.equal(dw, (dy.t() @ x.float()).to(torch.bfloat16))
+
+
+@pytest.mark.parametrize("E,K", [(8, 2), (64, 6), (256, 8)])
+@pytest.mark.parametrize("mode", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("norm", [True, False])
+def test_router_backward_rounds_like_fp32(cuda_lib, E, K, mode, norm):
+  """Wide logits, where a fast exponential is tens of ulp off.  Scores, W, the selected experts' terms and the products
+  are fp32: each is off by a few roundings of the terms that are added (16 ulp of the larger side)."""
+  torch.manual_seed(E)
+  lg = (torch.randn(200, E, device="cuda") * 12).requires_grad_(True)
+  w, idx, sc = moe.router_topk(lg, K, mode=mode, norm_topk=norm)
+  gw, gs = torch.randn_like(w), torch.randn_like(sc)
+  x = lg.detach().double().requires_grad_(True)
+  s = torch.softmax(x, -1) if mode == "softmax" else torch.sigmoid(x)
+  sel = s.gather(1, idx.long())
+  total = sel.sum(-1, keepdim=True) if norm else torch.ones_like(sel[:, :1])
+  (got,) = torch.autograd.grad([w, sc], lg, [gw, gs])
+  (want,) = torch.autograd.grad([sel / total, s], x, [gw.double(), gs.double()])
+  # |ds| of every expert, with the terms of the normalisation taken at their size and not at their difference
+  c = (gw.double().abs() * sel).sum(-1, keepdim=True) / total if norm else 0.0
+  ds = gs.double().abs().scatter_add(1, idx.long(), (gw.double().abs() + c) / total)
+  size = s * (ds + (s * ds).sum(-1, keepdim=True)) if mode == "softmax" else s * ds
+  err = ((got.double() - want).abs() / (size.detach() + 1e-30))
+  assert err.max().item() < 16 * 2.0 ** -23, err.max().item() * 2.0 ** 23
