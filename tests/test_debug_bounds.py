@@ -55,6 +55,19 @@ def test_exchange_descriptors(monkeypatch):
   _debug.check_exchange_descriptors("a2a", good[:-1], 3, 10, 2, 16)    # off: nothing is looked at
 
 
+def test_few_rows_experts_refuse_a_bad_plan(monkeypatch):
+  """The routed MLP without gradients looks at its gather indices like the one with them."""
+  monkeypatch.setenv("TPB_DEBUG_BOUNDS", "1")
+  plan = moe.DispatchPlan(src_row=torch.tensor([0, 1, 2, 4] + [-1] * 12, dtype=torch.int32), src_pair=torch.arange(16),
+                          dest=torch.zeros(4, 1, dtype=torch.int32), tile_expert=torch.zeros(1, dtype=torch.int32),
+                          k_offsets=torch.tensor([0, 16], dtype=torch.int32), counts=torch.tensor([4]), num_rows=16,
+                          num_experts=1, top_k=1, row_align=16)
+  monkeypatch.setattr(moe, "_build_dispatch_plan_kernel", lambda *_: plan)
+  x, w = torch.zeros(4, 64, dtype=torch.bfloat16), torch.zeros(1, 64, 64, dtype=torch.bfloat16)
+  with pytest.raises(IndexError, match="moe_gather: 1 of 16 entries of `src_row`"):
+    moe.grouped_mlp_few_rows(x, torch.ones(4, 1), torch.zeros(4, 1, dtype=torch.int32), w, w, w, False, 16)
+
+
 @pytest.mark.gpu
 def test_valid_indices_pass_and_bad_ones_leave_the_context_usable(cuda_lib, monkeypatch):
   monkeypatch.setenv("TPB_DEBUG_BOUNDS", "1")

@@ -205,11 +205,16 @@ def _build_dispatch_plan_kernel(idx: torch.Tensor, e: int, align: int = ROW_ALIG
 
 
 # ----------------------------------------------------------------------------- raw kernels
-def gather_rows(x, src_row, row_scale=None):
+def gather_rows(x, src_row, row_scale=None, pad=True):
+  """``pad=False``: rows of index -1 are left unwritten (for readers that ignore them; no ``row_scale`` then)."""
   m, d = src_row.numel(), x.shape[-1]
   out = torch.empty(m, d, dtype=x.dtype, device=x.device)
   _debug.check_index("moe_gather", "src_row", src_row, 0, x.reshape(-1, d).shape[0], also_allowed=-1)
-  check(lib().tpb_moe_gather(ptr(x), ptr(src_row), ptr(row_scale), ptr(out), m, d, stream_ptr()), "moe_gather")
+  if pad:
+    check(lib().tpb_moe_gather(ptr(x), ptr(src_row), ptr(row_scale), ptr(out), m, d, stream_ptr()), "moe_gather")
+  else:
+    assert row_scale is None
+    check(lib().tpb_moe_gather_real(ptr(x), ptr(src_row), ptr(out), m, d, stream_ptr()), "moe_gather_real")
   return out
 
 
@@ -234,8 +239,7 @@ def grouped_mlp_few_rows(x, weights, idx, w_gate, w_up, w_down, fused_gate_up, a
   f = w_down.shape[1]
   plan = _build_dispatch_plan_kernel(idx, e, align)
   m, hit = plan.num_rows, min(e, t * k)
-  xg = torch.empty(m, d, dtype=x.dtype, device=x.device)
-  check(lib().tpb_moe_gather_real(ptr(x), ptr(plan.src_row), ptr(xg), m, d, stream_ptr()), "moe_gather_real")
+  xg = gather_rows(x, plan.src_row, pad=False)
   act = torch.empty(m, f, dtype=x.dtype, device=x.device)
   rows = torch.empty(m, d, dtype=x.dtype, device=x.device)
   check(lib().tpb_grouped_gemm_skinny_bf16(
