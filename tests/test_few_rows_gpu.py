@@ -153,6 +153,22 @@ def test_route_of_the_few_rows_path():
   assert moe.few_rows_align(256, 6, 64) == 32 and moe.few_rows_align(257, 6, 64) is None
 
 
+def test_recomputed_forward_gives_the_recorded_bits(cuda_lib):
+  """A forward that will be repeated with gradients runs the same kernels as the repetition."""
+  from torchprime_b200.ops import functional as ops
+  torch.manual_seed(0)
+  t, kk, e, d, f = 40, 2, 8, 1024, 512
+  assert moe.few_rows_align(t, kk, e) is not None
+  x = torch.randn(t, d, device="cuda", dtype=torch.bfloat16)
+  wg, wu = ((torch.randn(e, d, f, device="cuda") / 32).to(torch.bfloat16) for _ in range(2))
+  wd = (torch.randn(e, f, d, device="cuda") / 32).to(torch.bfloat16).requires_grad_(True)
+  w, idx, _ = moe.router_topk(torch.randn(t, e, device="cuda"), kk)
+  recorded = moe.grouped_mlp(x, w, idx, wg, wu, wd)
+  assert recorded.requires_grad
+  with torch.no_grad(), ops.recomputed_forward():
+    assert torch.equal(moe.grouped_mlp(x, w, idx, wg, wu, wd), recorded)
+
+
 def test_no_tokens(cuda_lib):
   """Without tokens no expert is hit: an empty result, recorded or not."""
   assert moe.few_rows_align(0, 6, 64) is None

@@ -266,3 +266,24 @@ def test_device_timeout_is_raised_at_the_step_it_is_seen(tmp_path, monkeypatch):
   with pytest.raises(_lib.KernelError, match="at training step 2"):
     tr.train_loop()
   assert calls["n"] >= 3
+
+
+def test_recomputing_unit_marks_its_first_forward():
+  """A unit whose forward is repeated in the backward pass tells its operators so, in the first run only."""
+  from types import SimpleNamespace
+
+  from torchprime_b200.ops import functional as ops
+  from torchprime_b200.parallel import fsdp
+  seen = []
+
+  def forward(x):
+    seen.append((torch.is_grad_enabled(), ops.in_recomputed_forward()))
+    return 2 * x
+
+  nothing = lambda *_, **__: None  # noqa: E731
+  engine = SimpleNamespace(is_cuda=False, pre_forward=nothing, post_forward=nothing, pre_backward=nothing, post_backward=nothing)
+  unit = SimpleNamespace(offload=False, orig_forward=forward, slots=[])
+  x = torch.ones(3, requires_grad=True)
+  fsdp._RematFn.apply(engine, unit, {}, torch.zeros(1, requires_grad=True), x).sum().backward()
+  assert seen == [(False, True), (True, False)] and not ops.in_recomputed_forward()
+  assert torch.equal(x.grad, torch.full((3,), 2.0))

@@ -12,6 +12,7 @@ normally.
 from __future__ import annotations
 
 import math
+import threading
 from contextlib import contextmanager
 
 import torch
@@ -60,6 +61,25 @@ def inference_only() -> bool:
   """Neither reverse- nor forward-mode derivatives are being recorded, so an operator may run without
   its autograd function."""
   return not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
+
+
+_RECOMPUTED = threading.local()
+
+
+@contextmanager
+def recomputed_forward():
+  """Around a forward that runs without gradients now and once more with them in the backward pass: this thread's
+  operators keep to the kernels of the recorded form, so that both runs give the same bits."""
+  old = in_recomputed_forward()
+  _RECOMPUTED.on = True
+  try:
+    yield
+  finally:
+    _RECOMPUTED.on = old
+
+
+def in_recomputed_forward() -> bool:
+  return getattr(_RECOMPUTED, "on", False)
 
 
 # --------------------------------------------------------------------------- helpers

@@ -404,13 +404,16 @@ def grouped_mlp_reference(x, weights, idx, w_gate, w_up, w_down, fused_gate_up=F
 
 def grouped_mlp(x, weights, idx, w_gate, w_up, w_down, *, fused_gate_up=False, capacity=None, rows_per_group=None):
   """Routed SwiGLU experts.  x [T,D]; weights/idx [T,K]; w_gate/w_up [E,D,F]; w_down [E,F,D]
-  (``fused_gate_up``: w_gate is [E,D,2F] = [gate | up] and w_up is ignored)."""
+  (``fused_gate_up``: w_gate is [E,D,2F] = [gate | up] and w_up is ignored).
+
+  Calls without gradients and with a handful of rows per expert take :func:`grouped_mlp_few_rows`, whose sums are split
+  differently; a forward that a backward pass will repeat says so with ``functional.recomputed_forward`` and does not."""
   e = w_gate.shape[0]
   f = w_down.shape[1]
-  from .functional import inference_only
+  from .functional import in_recomputed_forward, inference_only
   ok = (_kernels_ok(x, w_gate, w_down) and x.shape[-1] % 64 == 0 and f % 64 == 0 and x.is_cuda)
   if ok:
-    if (capacity is None and e <= 256 and inference_only()
+    if (capacity is None and e <= 256 and inference_only() and not in_recomputed_forward()
         and all(w.is_contiguous() and w.data_ptr() % 16 == 0 for w in (w_gate, w_up, w_down) if w is not None)):
       align = few_rows_align(*idx.shape, e)
       if align is not None:

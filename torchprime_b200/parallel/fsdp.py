@@ -1050,7 +1050,8 @@ class _RematFn(torch.autograd.Function):
     else:
       ctx.save_for_backward(*tensors)
     engine.pre_forward(u)
-    with torch.no_grad():
+    from ..ops import functional as ops
+    with torch.no_grad(), ops.recomputed_forward():
       out = u.orig_forward(*args, **kwargs)
     engine.post_forward(u, backward_follows=True)
     ctx.out_is_tuple = isinstance(out, tuple)
