@@ -30,3 +30,15 @@ def test_head_gradient_over_chunks(cuda_lib, rows, chunk):
   (2.5 * F.cross_entropy((hd @ wd.t())[0], t[0])).backward()
   for got, want in ((h.grad, hd.grad), (w.grad, wd.grad)):
     assert ((got.double() - want).norm() / want.norm()).item() < 1e-2      # bf16 logits and bf16 d(logits)
+
+
+def test_batched_gradients(cuda_lib):
+  """Several gradients in one backward pass give what one pass each gives."""
+  h = torch.randn(1, 70, 64, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+  w = (torch.randn(512, 64, device="cuda") / 8).to(torch.bfloat16).requires_grad_(True)
+  loss = ops.linear_cross_entropy(h, w, torch.randint(0, 512, (1, 70), device="cuda"))
+  scales = torch.tensor([1.0, -0.5, 3.0], device="cuda", dtype=loss.dtype)
+  got = torch.autograd.grad(loss, (h, w), scales, is_grads_batched=True, retain_graph=True)
+  for i in range(3):
+    for a, b in zip(got, torch.autograd.grad(loss, (h, w), scales[i], retain_graph=True)):
+      assert torch.equal(a[i], b)

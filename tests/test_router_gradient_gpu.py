@@ -65,3 +65,18 @@ def test_router_backward_rounds_like_fp32(cuda_lib, E, K, mode, norm):
   size = s * (ds + (s * ds).sum(-1, keepdim=True)) if mode == "softmax" else s * ds
   err = ((got.double() - want).abs() / (size.detach() + 1e-30))
   assert err.max().item() < 16 * 2.0 ** -23, err.max().item() * 2.0 ** 23
+
+
+@pytest.mark.parametrize("mode", ["softmax", "sigmoid"])
+@pytest.mark.parametrize("norm", [True, False])
+def test_router_batched_gradients(cuda_lib, mode, norm):
+  """Several gradients in one backward pass give what one pass each gives (fp32 both ways: a few roundings apart)."""
+  torch.manual_seed(1)
+  lg = torch.randn(30, 16, device="cuda", requires_grad=True)
+  w, _, sc = moe.router_topk(lg, 4, mode=mode, norm_topk=norm, scale=1.5)
+  gw, gs = torch.randn(3, *w.shape, device="cuda"), torch.randn(3, *sc.shape, device="cuda")
+  for outs, grads in (([w, sc], [gw, gs]), ([w], [gw]), ([sc], [gs])):
+    (got,) = torch.autograd.grad(outs, lg, grads, is_grads_batched=True, retain_graph=True)
+    for i in range(3):
+      (one,) = torch.autograd.grad(outs, lg, [g[i] for g in grads], retain_graph=True)
+      assert torch.allclose(got[i], one, rtol=1e-5, atol=1e-6)

@@ -63,6 +63,13 @@ def inference_only() -> bool:
   return not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
 
 
+def batched(*tensors) -> bool:
+  """Whether a backward pass runs for several gradients at once (``is_grads_batched``, ``vmap`` over ``grad``): kernels
+  cannot be given such tensors, torch operators can."""
+  c = torch._C._functorch
+  return any(t is not None and (c.is_legacy_batchedtensor(t) or c.is_batchedtensor(t)) for t in tensors)
+
+
 _RECOMPUTED = threading.local()
 
 
@@ -858,8 +865,8 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
     dh, dw_local = ctx.saved_tensors
     gh = (dh * dloss.to(dh.dtype)).view(ctx.h_shape) if dh is not None else None
     gw = None
-    if dw_local is not None and torch.is_grad_enabled() and dloss.requires_grad:
-      gw = (dw_local * dloss).to(torch.bfloat16)      # a derivative with respect to dloss is wanted
+    if dw_local is not None and (batched(dloss) or (torch.is_grad_enabled() and dloss.requires_grad)):
+      gw = (dw_local * dloss).to(torch.bfloat16)      # several gradients, or one with respect to dloss, are wanted
     elif dw_local is not None:
       from . import kernels as k
       gw = k.scale_cast_bf16(dw_local, dloss.float())

@@ -57,6 +57,20 @@ def _router_forward(lg, bias, k, mode, n_group, topk_group, norm_topk, scale):
   return w, idx, scores
 
 
+def _router_backward(lg, idx, dw, dscores, mode, norm_topk, scale):
+  """The gradient of the logits in torch operators (for batched gradients)."""
+  s = torch.softmax(lg.float(), dim=-1) if mode == 0 else torch.sigmoid(lg.float())
+  ds = dscores if dscores is not None else torch.zeros_like(s)
+  if dw is not None:
+    sel, dsel = s.gather(1, idx.long()), dw * scale
+    if norm_topk:
+      total = sel.sum(-1, keepdim=True) + (0.0 if mode == 0 else 1e-20)
+      dsel = (dsel - (dsel * sel).sum(-1, keepdim=True) / total) / total
+    ds = ds + torch.zeros_like(s).scatter(1, idx.long(), dsel)
+  g = s * (ds - (s * ds).sum(-1, keepdim=True)) if mode == 0 else ds * s * (1 - s)
+  return g.to(lg.dtype)
+
+
 class _RouterFn(torch.autograd.Function):
   """Kernels both ways; the backward re-derives the scores from the logits."""
 
@@ -76,6 +90,9 @@ class _RouterFn(torch.autograd.Function):
     mode, norm_topk, scale = ctx.args
     if dw is None and dscores is None:
       return (None,) * 8
+    from .functional import batched
+    if batched(dw, dscores):
+      return _router_backward(lg, idx, dw, dscores, mode, norm_topk, scale), None, None, None, None, None, None, None
     t, e = lg.shape
     dw = dw.float().contiguous() if dw is not None else None
     dscores = dscores.float().contiguous() if dscores is not None else None
