@@ -35,3 +35,13 @@ def test_operators_without_a_graph_equal_those_with_one(cuda_lib):
     assert ops.rope_inplace(t, cos, sin, 2, 128, 40) is t and t._version == v + 1
   with torch.inference_mode():
     ops.rope_inplace(torch.randn(1, 40, 256, device="cuda", dtype=torch.bfloat16), cos, sin, 2, 128, 40)
+
+
+def test_fused_projection_with_a_row_pitch(cuda_lib):
+  """A projection that is a slice of wider rows gives the same result with and without a graph."""
+  from torchprime_b200.ops import attention_sm100 as A
+  qkv = torch.randn(2, 70, 6 * 128 + 64, device="cuda", dtype=torch.bfloat16)[..., :6 * 128]
+  with_graph = A.attention_qkv(qkv, 4, 1, 128)
+  with torch.no_grad():
+    assert torch.equal(A.attention_qkv(qkv, 4, 1, 128), with_graph)
+    assert torch.equal(A.attention_qkv(qkv.contiguous(), 4, 1, 128), with_graph)

@@ -259,7 +259,7 @@ def _nothing_recorded() -> bool:
 def attention_qkv(qkv, hq, hkv, d, causal=True, scale=None, window=None, q_segment_ids=None, q_positions=None):
   """Self-attention on a fused [B, S, (Hq + 2 Hkv) * D] projection (head dim 128, contiguous)."""
   seg = _i32(q_segment_ids)
-  if _nothing_recorded() and qkv.dim() == 3 and hkv > 0 and hq % hkv == 0 and qkv.shape[-1] == (hq + 2 * hkv) * d:
+  if _nothing_recorded() and qkv.dim() == 3 and qkv.is_contiguous() and hkv > 0 and hq % hkv == 0 and qkv.shape[-1] == (hq + 2 * hkv) * d:
     b, s, width = qkv.shape
     o = torch.empty(b, s, hq, d, dtype=qkv.dtype, device=qkv.device)
     lse = torch.empty(b, hq, s, dtype=torch.float32, device=qkv.device)
