@@ -70,3 +70,12 @@ def test_other_layouts_keep_the_matrix_product_form(cuda_lib):
     assert not mla_decode.supported(q, torch.randn(2, 1, 600, device="cuda", dtype=torch.bfloat16)[..., :576], *args)
     with ops.backend("torch"):
       assert not mla_decode.supported(q, ckv, *args)
+
+
+def test_values_wider_than_the_kernel_takes(cuda_lib):
+  """Value heads of more than 4096 columns run as matrix products."""
+  eng = _engine(num_attention_heads=1, num_key_value_heads=1, v_head_dim=4104)
+  x = torch.randn(2, 1, 256, device="cuda", dtype=torch.bfloat16)
+  with torch.no_grad():
+    y = eng._attention(0, eng.model.model.layers[0].self_attn, x, 0, x, lambda: torch.zeros(2, dtype=torch.int32, device="cuda"))
+  assert y.shape == x.shape and bool(torch.isfinite(y).all())

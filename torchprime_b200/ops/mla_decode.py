@@ -23,12 +23,13 @@ def _rows(t, width) -> bool:
 
 
 def supported(q, ckv, norm_w, kv_cache, pe_cache, w, heads, dn, dr, dv, c) -> bool:
-  """One token per sequence, bf16 throughout, rotary width 64 and a latent of at most 512 values."""
+  """One token per sequence, bf16 throughout, rotary width 64, a latent of at most 512 values, value width up to 4096
+  and as many sequences as a grid dimension holds."""
   from .functional import inference_only, use_kernels
   ts = (q, ckv, norm_w, kv_cache, pe_cache, w)
   if not all(t.is_cuda and t.dtype == torch.bfloat16 for t in ts) or not use_kernels(*ts):
     return False
-  return (q.shape[1] == 1 and dr == 64 and c % 64 == 0 and 64 <= c <= 512 and dn % 8 == 0 and 8 <= dn <= 512
+  return (q.shape[1] == 1 and q.shape[0] <= 65535 and dv <= 4096 and dr == 64 and c % 64 == 0 and 64 <= c <= 512 and dn % 8 == 0 and 8 <= dn <= 512
           and _rows(q, heads * (dn + dr)) and _rows(ckv, c + dr) and _rows(norm_w, c) and _rows(w, c)
           and w.numel() == heads * (dn + dv) * c and _rows(kv_cache, c) and _rows(pe_cache, dr)
           and inference_only())
