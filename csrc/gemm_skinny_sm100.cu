@@ -404,20 +404,21 @@ static int skinny_splits(long long tiles, int num_kb) {
   return s;
 }
 
-// Whether this kernel is the faster one for a dense product of M rows: always up to 128 rows (one token
-// tile; even a 102,400-wide head takes 98 us instead of 108 with 128 rows and 66 instead of 133 with one),
-// and beyond that while the tiled kernel's 128 x 256 tiles leave half of the SMs idle and the contraction is long
-// enough to be split (see the weight gradients below).  The time per call in
-// us with weights from HBM, tiled kernel / this one, by the number of its tiles (N x K):
-//   4096 x 4096:   384 rows, 48 tiles 34 / 23    512 rows, 64 tiles 35 / 24    768 rows, 96 tiles 35 / 36
-//   4096 x 14336:  512 rows, 64 tiles 98 / 62    768 rows, 96 tiles 98 / 97
-//   2048 x 10944: 1024 rows, 64 tiles 77 / 47    3072 x 2048: 768 rows, 72 tiles 22 / 16, 1024 rows, 96 tiles 23 / 23
-//   14336 x 4096:  128 rows, 56 tiles 39 / 28    192 rows, 112 tiles 39 / 40
+// Whether this kernel is the faster one for a dense product of M rows.  Up to 128 rows (one token tile) the tiled kernel
+// has few CTAs, each with the whole contraction; what this one adds is an epilogue whose length goes with the rows, so a
+// short contraction does not pay for many of them (us, weights from HBM, tiled kernel / this one, 4096 outputs):
+//   K = 256:  32 rows 6.5 / 5.8, 64 rows 6.6 / 7.1     K = 512: 64 rows 8.5 / 7.4, 96 rows 8.7 / 9.1
+//   K = 1024: 128 rows 12.2 / 9.2                      K = 4096: 32 / 15    (28672 outputs, K = 1024: 20.3 / 21.0)
+// Beyond that while the tiled kernel's 128 x 256 tiles leave half of the SMs idle (three quarters for a contraction that is
+// hardly worth splitting); by the number of its tiles (N x K):
+//   1024 x 1024: 32 tiles 10.8 / 10.5, 48 tiles 10.6 / 12.0      576 x 1536: 36 tiles 12.8 / 10.7, 72 tiles 13.0 / 13.8
+//   4096 x 2048: 32 tiles 18.7 / 13.0, 64 tiles 18.6 / 16.3      3072 x 2048: 36 tiles 18.4 / 19.2, 72 tiles 18.5 / 16.3
+//   4096 x 4096: 64 tiles 32 / 24, 96 tiles 32 / 36              2048 x 10944: 64 tiles 74 / 47, 96 tiles 75 / 77
 bool skinny_wins(int M, int N, int K, bool swiglu) {
-  if (M <= 128) return true;
+  if (M <= 128) return M <= 32 || 8 * M <= K;
   if (K < 1024) return false;
   const long long tiles = (long long)((M + 127) / 128) * (((swiglu ? N / 2 : N) + (swiglu ? 127 : 255)) / (swiglu ? 128 : 256));
-  return tiles <= sm_count() / 2;
+  return tiles <= sm_count() / (K < 2048 ? 4 : 2);
 }
 
 // The same for a weight gradient (both operands contracted over their rows, K of them): bound by the tensor cores,

@@ -223,7 +223,9 @@ def test_linear_f32_not_finite(cuda_lib):
   assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got[3:5], want[3:5])
 
 
-@pytest.mark.parametrize("M,N,K", [(1, 64, 128), (77, 512, 256), (128, 1000, 136), (300, 512, 512), (700, 64, 2048)])
+@pytest.mark.parametrize("M,N,K", [(1, 64, 128), (77, 512, 256), (128, 1000, 136), (300, 512, 512), (700, 64, 2048),
+                                   (32, 512, 64), (33, 512, 264), (64, 264, 512), (65, 264, 512), (128, 264, 1024), (129, 256, 1024),
+                                   (1100, 1024, 1024), (1300, 1024, 1024), (900, 2048, 2048), (1200, 2048, 2048)])
 def test_route_of_a_gemm_call(cuda_lib, M, N, K):
   """Calls the rule gives to this kernel against the tiled kernel (max_ctas keeps a call there)."""
   torch.manual_seed(M)
