@@ -532,13 +532,13 @@ extern "C" int tpb_gemm_skinny_bf16(const void* x, const void* w, const void* w2
                      splits, reinterpret_cast<cudaStream_t>(stream), false);
 }
 
-// Rows grouped by expert in segments padded to `nt` rows; tile_expert[rows / nt].  Token tiles of expert -1
+// Rows grouped by expert in segments padded to `nt` rows (16 or 32); tile_expert[rows / nt].  Token tiles of expert -1
 // are not written.  experts_hit: how many experts have rows, at most.
 extern "C" int tpb_grouped_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, int rows, int N,
                                             int K, int E, long long ldx, long long ldw, long long w_stride,
                                             long long ldc, int w_mn, int epi, const int* tile_expert, int experts_hit,
                                             int nt, void* stream) {
-  if (!tile_expert || E < 1 || experts_hit < 1) return -2;
+  if (!tile_expert || E < 1 || experts_hit < 1 || (nt != 16 && nt != 32)) return -2;
   return skinny_gemm(x, w, w2, c, rows, N, K, E, ldx, ldw, w_stride, ldc, 0, w_mn, epi, 1.0f, nullptr, 0, nullptr, 0,
                      tile_expert, experts_hit, nt, 0, reinterpret_cast<cudaStream_t>(stream), false);
 }

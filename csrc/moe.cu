@@ -617,13 +617,13 @@ extern "C" int tpb_a2a_push_rows(const void* src, int n_rows, int dim, int world
   return rc_of(cudaGetLastError());
 }
 
-// idx [tokens, K] int32 (entries outside [0, E) are dropped: dest = -1).  align: 16, 32, 64, 128 or 256 rows per
+// idx [tokens, K] int32 (entries outside [0, E) are dropped: dest = -1).  align: 16, 32, 128 or 256 rows per
 // segment step.  rows = static row count of the padded layout, a multiple of align that holds n pairs and
 // align - 1 padding rows for every expert that can be hit.  Everything is on the device; no host read.
 extern "C" int tpb_moe_plan(const int* idx, int tokens, int K, int E, int rows, int align, int* counts, int* k_offsets,
                             int* dest, int* src_row, long long* src_pair, int* tile_expert, void* stream) {
   if (E < 1 || E > PLAN_MAX_E || K < 1 || tokens < 0 || rows < 0) return -2;
-  if ((align != 16 && align != 32 && align != 64 && align != 128 && align != 256) || rows % align) return -2;
+  if ((align != 16 && align != 32 && align != 128 && align != 256) || rows % align) return -2;
   const long long n = (long long)tokens * K;
   if (n > (1LL << 30) || rows < n + (long long)(align - 1) * (n < E ? n : E)) return -2;
   moe_plan_kernel<<<1, PLAN_THREADS, 0, STREAM(stream)>>>(idx, (int)n, K, E, rows, align, counts, k_offsets, dest, src_row,

@@ -238,10 +238,10 @@ def gather_rows(x, src_row, row_scale=None, pad=True):
 def few_rows_align(t: int, k: int, e: int) -> int | None:
   """Token-tile width of the few-rows path for ``t`` tokens, or None where the tiled grouped GEMMs are as good.
   Both paths are bound by the weights of the experts that are hit; what counts is the average number of rows per
-  expert (us for the routed MLP, tiled / 16 / 32 / 64 rows per segment step): 64 experts of 2048 x 1408, 6 rows
-  225 / 210 / 224 / 257, 12 rows 228 / 217 / 227 / 258, 24 rows 231 / 268 / 231 / 259; 8 experts of 4096 x 14336,
-  8 rows 469 / 448 / 453 / 475, 16 rows 471 / 485 / 454 / 476, 24 rows 555 / 525 / 459 / 482.  Without tokens no
-  expert is hit and there is nothing for that path to launch."""
+  expert (us for the routed MLP, tiled / 16 / 32 rows per segment step): 64 experts of 2048 x 1408, 6 rows 225 / 210 / 224,
+  12 rows 228 / 217 / 226, 24 rows 231 / 268 / 231, 36 rows 234 / 337 / 286; 8 experts of 4096 x 14336, 8 rows 469 / 448 / 453,
+  16 rows 471 / 485 / 454, 24 rows 555 / 525 / 459.  Without tokens no expert is hit and there is nothing for that path to
+  launch."""
   per = t * k / e
   if per == 0:
     return None
