@@ -958,8 +958,10 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   bool tma_store = g.epi == TPB_EPI_BF16 || g.epi == TPB_EPI_F32 || g.epi == TPB_EPI_F32_ACC ||
                    (swiglu && (!g.c2 || (g.ldc2 % 8 == 0 && !misaligned(g.c2))));
   if (g.mode == 2 && (g.c_stride % (f32out ? 4 : 8))) tma_store = false;
+  const uint64_t n_cols = swiglu ? g.N / 2 : g.N;
+  if (n_cols % (f32out ? 4 : 8)) tma_store = false;   // a box is clipped in steps of 16 bytes: it would write past the last column
   if (tma_store) {
-    const uint64_t n_cols = swiglu ? g.N / 2 : g.N, planes = g.mode == 2 ? g.E : 1;
+    const uint64_t planes = g.mode == 2 ? g.E : 1;
     const uint64_t plane = g.mode == 2 && g.E > 1 ? (uint64_t)g.c_stride : (uint64_t)g.ldc * g.M;
     if (make_tmap_out(&tc, g.C, n_cols, g.M, planes, g.ldc, plane, f32out ? 4 : 2)) return -3;
     // [gate | up]: two planes, so that a box of the gate half is clipped where the up half begins

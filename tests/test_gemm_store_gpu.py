@@ -61,3 +61,21 @@ def test_per_expert_weight_gradients(cuda_lib, da, db, dtype, accumulate):
     want = a[off[x]:off[x + 1]].double().t() @ b[off[x]:off[x + 1]].double() + (before[x] if accumulate else 0.0)
     err = (out[x].double() - want).abs()
     assert bool((err <= (2.0 ** -8 if dtype == torch.bfloat16 else 0.0) * want.abs() + 1e-4).all()), (x, err.max())
+
+
+@pytest.mark.parametrize("M", [20, 100, 300])
+@pytest.mark.parametrize("N", [100, 101, 259])
+@pytest.mark.parametrize("epi", [k.EPI_BF16, k.EPI_F32, k.EPI_F32_ACC])
+def test_columns_that_end_inside_a_vector(cuda_lib, M, N, epi):
+  """Rows of C with a 16-byte pitch but any number of columns: the rest of the row stays as it is."""
+  torch.manual_seed(M + N)
+  a = torch.randn(M, 136, device="cuda", dtype=torch.bfloat16)
+  b = torch.randn(N, 136, device="cuda", dtype=torch.bfloat16)
+  dt = torch.bfloat16 if epi == k.EPI_BF16 else torch.float32
+  big = torch.full((M, (N + 15) // 8 * 8), 5.0, device="cuda", dtype=dt)
+  out = big[:, :N]
+  k.gemm(a, b, out=out, epi=epi)
+  want = a.double() @ b.double().t() + (5.0 if epi == k.EPI_F32_ACC else 0.0)
+  err = (out.double() - want).abs()
+  assert bool((err <= (2.0 ** -8 if dt == torch.bfloat16 else 0.0) * want.abs() + 2e-6 * 136).all()), err.max()
+  assert bool((big[:, N:] == 5.0).all())
