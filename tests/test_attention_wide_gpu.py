@@ -8,6 +8,8 @@ pytestmark = pytest.mark.gpu
 from torchprime_b200.ops import attention_sm100 as A
 from torchprime_b200.ops import reference as ref
 
+ROUNDED = 1.66e-3     # relative error (2-norm) of values rounded to bf16 once
+
 
 def _check(b, sq, sk, hq, hkv, bound=2e-2, **kw):
   """The bound is that of the head-dim-128 tests (bf16 P and dS)."""
@@ -56,7 +58,66 @@ def test_positions(cuda_lib):
   _check(1, 128, 384, 2, 2, causal=True, q_positions=pos.long())
 
 
-ROUNDED = 1.66e-3     # relative error (2-norm) of values rounded to bf16 once
+def _ids(kind, b, s):
+  g = torch.Generator(device="cuda").manual_seed(s + b)
+  at = torch.arange(s, device="cuda")
+  if kind == "sorted":
+    cuts = torch.randint(0, s, (b, 5), device="cuda", generator=g)
+    return (at[None, :, None] >= cuts[:, None, :]).sum(-1).to(torch.int32)
+  if kind == "one":
+    return torch.full((b, s), 3, dtype=torch.int32, device="cuda")
+  if kind == "blocks":       # ids that change at tile edges, decreasing, with the int32 extremes
+    ids = (-(at // 64)).to(torch.int32)
+    ids[at < 64] = 2 ** 31 - 1
+    ids[at // 64 == (s - 1) // 64] = -2 ** 31
+    return ids.expand(b, s).contiguous()
+  return torch.randint(-2, 2, (b, s), device="cuda", generator=g).to(torch.int32)   # no order at all
+
+
+@pytest.mark.parametrize("causal,window", [(True, None), (False, None), (True, 70)])
+@pytest.mark.parametrize("s", [257, 320, 777])
+@pytest.mark.parametrize("kind", ["sorted", "one", "blocks", "mixed"])
+def test_range_tables(cuda_lib, s, kind, causal, window):
+  """Lengths with range tables: forward and gradients against the fp32 definition."""
+  torch.manual_seed(s)
+  q, k, v = (torch.randn(2, s, h, d, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+             for h, d in ((4, 192), (2, 192), (2, 128)))
+  kw = {"causal": causal, "window": window, "q_segment_ids": _ids(kind, 2, s)}
+  assert A._seg_ranges(kw["q_segment_ids"], kw["q_segment_ids"], 2, s, s)[0] is not None
+  o = A.attention(q, k, v, **kw)
+  do = torch.randn_like(o)
+  got = torch.autograd.grad(o, (q, k, v), do)
+  qf, kf, vf = (t.detach().float().requires_grad_(True) for t in (q, k, v))
+  w = ref.attention(qf, kf, vf, **kw)
+  want = torch.autograd.grad(w, (qf, kf, vf), do.float())
+  # P is rounded once in the forward, o once; the gradients keep fp32 probabilities and are rounded once
+  for a, r, bound in zip((o, *got), (w, *want), (2 ** 0.5, 1.1, 1.1, 1.1)):
+    assert ((a.float() - r.float()).norm() / r.float().norm()).item() < bound * ROUNDED * 1.05
+
+
+def test_keys_and_queries_with_other_ids(cuda_lib):
+  """A query tile whose segment no key has, and a key block whose segment no query has, give zeros."""
+  torch.manual_seed(0)
+  q, k = (torch.randn(1, 400, 2, 192, device="cuda", dtype=torch.bfloat16, requires_grad=True) for _ in range(2))
+  v = torch.randn(1, 400, 2, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+  q_seg, kv_seg = (torch.zeros(1, 400, dtype=torch.int32, device="cuda") for _ in range(2))
+  q_seg[:, 128:256] = 9
+  kv_seg[:, 256:384] = 5
+  o = A.attention(q, k, v, causal=False, q_segment_ids=q_seg, kv_segment_ids=kv_seg)
+  dq, dk, dv = torch.autograd.grad(o, (q, k, v), torch.randn_like(o))
+  for zero in (o[:, 128:256], dq[:, 128:256], dk[:, 256:384], dv[:, 256:384]):
+    assert bool((zero == 0).all())
+  for t in (o, dq, dk, dv):
+    assert bool(torch.isfinite(t).all()) and bool((t[:, :128] != 0).any())
+
+
+@pytest.mark.parametrize("kw", [{"causal": True}, {"causal": False}, {"causal": True, "window": 40}])
+def test_more_queries_than_the_table_holds(cuda_lib, monkeypatch, kw):
+  """The route of calls beyond the query-tile table, at a size that can be run."""
+  monkeypatch.setattr(A, "_MAX_WIDE_QUERIES", 64)
+  _check(2, 100, 100, 2, 2, **kw)
+  ids = (torch.arange(100, device="cuda") // 30).to(torch.int32).expand(2, 100).contiguous()
+  _check(2, 100, 100, 2, 2, q_segment_ids=ids, **kw)
 
 
 @pytest.mark.parametrize("sq,sk,kind", [(77, 77, "plain"), (1024, 1024, "plain"), (300, 300, "full"), (77, 77, "segments"),

@@ -147,6 +147,24 @@ def test_grouped_mlp_without_gradients(cuda_lib, t, kk, e, d, f, fused):
   assert ((y.double() - want).norm() / want.norm()).item() < 3 * BF16_EPS
 
 
+@pytest.mark.parametrize("t,kk,e", [(40, 2, 8), (90, 1, 4), (33, 6, 64)])
+def test_grouped_mlp_with_uneven_routing(cuda_lib, t, kk, e):
+  """All tokens go to the same experts, which then span several segment steps; the other experts get nothing."""
+  torch.manual_seed(t)
+  d, f = 256, 128
+  x = torch.randn(t, d, device="cuda", dtype=torch.bfloat16)
+  wg, wu = ((torch.randn(e, d, f, device="cuda") / 16).to(torch.bfloat16) for _ in range(2))
+  wd = (torch.randn(e, f, d, device="cuda") / 11).to(torch.bfloat16)
+  idx = torch.arange(kk, device="cuda", dtype=torch.int32).flip(0)[None].expand(t, -1).contiguous()
+  w = torch.rand(t, kk, device="cuda")
+  align = moe.few_rows_align(t, kk, e)
+  assert align is not None and t > align
+  with torch.no_grad():
+    y = moe.grouped_mlp(x, w, idx, wg, wu, wd)
+  want = moe.grouped_mlp_reference(x.double(), w.double(), idx, wg.double(), wu.double(), wd.double())
+  assert ((y.double() - want).norm() / want.norm()).item() < 3 * BF16_EPS
+
+
 def test_route_of_the_few_rows_path():
   assert moe.few_rows_align(4, 6, 64) == 16 and moe.few_rows_align(128, 6, 64) == 16
   assert moe.few_rows_align(96, 2, 8) == 32 and moe.few_rows_align(97, 2, 8) is None
