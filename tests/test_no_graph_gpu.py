@@ -45,3 +45,25 @@ def test_fused_projection_with_a_row_pitch(cuda_lib):
   with torch.no_grad():
     assert torch.equal(A.attention_qkv(qkv, 4, 1, 128), with_graph)
     assert torch.equal(A.attention_qkv(qkv.contiguous(), 4, 1, 128), with_graph)
+
+
+@pytest.mark.parametrize("op", ["linear", "swiglu", "norm", "embedding", "attention", "segments", "router"])
+def test_traces_follow_their_input(cuda_lib, op):
+  """An operator traced with nothing recorded computes from the input of each call."""
+  from torchprime_b200.ops import moe
+  torch.manual_seed(0)
+  w = torch.randn(128, 64, device="cuda", dtype=torch.bfloat16) / 8
+  ids = torch.arange(300, device="cuda")[None] // 70
+  fn, shape = {
+    "linear": (lambda x: ops.linear(x, w), (30, 64)),
+    "swiglu": (lambda x: ops.linear_swiglu(x, w[:64], w[64:]), (30, 64)),
+    "norm": (lambda x: ops.rms_norm(x, w[0], 1e-5), (30, 64)),
+    "embedding": (lambda x: ops.embedding((x[:, 0].float().abs() * 10).long().clamp(0, 127), w), (30, 64)),
+    "attention": (lambda x: ops.attention_qkv(x, 4, 1, 128), (1, 40, 6 * 128)),
+    "segments": (lambda x: ops.attention_qkv(x, 4, 1, 128, q_segment_ids=ids), (1, 300, 6 * 128)),
+    "router": (lambda x: moe.router_topk(x.float(), 6)[0], (30, 64)),
+  }[op]
+  first, second = (torch.randn(*shape, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+  with torch.no_grad():
+    traced = torch.jit.trace(fn, (first,), check_trace=False)
+    assert torch.equal(traced(second), fn(second)) and torch.equal(traced(first), fn(first))

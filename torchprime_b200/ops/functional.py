@@ -58,9 +58,10 @@ def use_kernels(*tensors) -> bool:
 
 
 def inference_only() -> bool:
-  """Neither reverse- nor forward-mode derivatives are being recorded, so an operator may run without
-  its autograd function."""
-  return not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
+  """Neither reverse- nor forward-mode derivatives nor a trace are being recorded, so an operator may run without
+  its autograd function (which a trace holds and calls again; it would not see a kernel launched by hand)."""
+  return (not torch.is_grad_enabled() and torch.autograd.forward_ad._current_level < 0
+          and not torch._C._is_tracing())
 
 
 def batched(*tensors) -> bool:
