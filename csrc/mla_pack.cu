@@ -2,7 +2,8 @@
 //
 // The up-projection yields [token][head][dn key values | dv values]; every head's key is completed by the
 // token's one rotary key.  Forward: k[t,h] = [kv[t,h,:dn] | rot[t]], v[t,h] = kv[t,h,dn:].  Backward: dkv from
-// dk and dv, drot[t] = sum_h dk[t,h,dn:] (fp32 sum in head order).  One pass each, 16-byte vectors, bound by
+// dk and dv, drot[t] = sum_h dk[t,h,dn:] (fp32, in a fixed order: heads modulo 256 / (dr / 8)
+// first, then those groups).  One pass each, 16-byte vectors, bound by
 // memory; as torch operators the same is a concatenation and a copy forward and seven launches backward
 // (zero-filled slice gradients and their sum), each over the whole tensors: about 110 us together at 2048 tokens and
 // 16 heads of 128 + 64 / 128, against 11 + 10 us.

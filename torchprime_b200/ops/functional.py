@@ -784,7 +784,7 @@ class _LatentSplitFn(torch.autograd.Function):
 
 
 def latent_split(ckv, c):
-  """(ckv[..., :c], ckv[..., c:]), both contiguous."""
+  """(ckv[..., :c], ckv[..., c:]); contiguous where kernels run."""
   if use_kernels(ckv):
     return _LatentSplitFn.apply(ckv, c)
   return ckv[..., :c].contiguous(), ckv[..., c:]
