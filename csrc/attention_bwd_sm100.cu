@@ -638,7 +638,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int nblk_total = (p.Sk + BWD_T - 1) / BWD_T;
   int blk_hi = p.causal ? min(nblk_total, qpos_max / BWD_T + 1) : nblk_total;
   int blk_lo = (p.window > 0) ? max(0, (qpos_min - p.window + 1) / BWD_T) : 0;
-  if (qpos_max < 0) blk_hi = 0;
+  if (p.causal && qpos_max < 0) blk_hi = 0;
   int2 qr = make_int2(0, 0);
   if (SEG) {   // as in the forward: only the key blocks between the first and last with a common segment
     qr = seg_range128(p.q_rng, b, qt, p.Sq);
@@ -1326,7 +1326,7 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int nblk_total = (p.Sk + BWD_T - 1) / BWD_T;
   int blk_hi = p.causal ? min(nblk_total, qpos_max / BWD_T + 1) : nblk_total;
   int blk_lo = (p.window > 0) ? max(0, (qpos_min - p.window + 1) / BWD_T) : 0;
-  if (qpos_max < 0) blk_hi = 0;
+  if (p.causal && qpos_max < 0) blk_hi = 0;
   int2 qr = make_int2(0, 0);
   if (p.kv_rng) {
     qr = seg_range128(p.q_rng, b, qt, p.Sq);

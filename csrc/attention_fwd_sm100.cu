@@ -321,7 +321,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int nblk_total = (p.Sk + FWD_BN - 1) / FWD_BN;
   int blk_hi = p.causal ? min(nblk_total, qpos_max / FWD_BN + 1) : nblk_total;
   int blk_lo = (p.window > 0) ? max(0, (qpos_min - p.window + 1) / FWD_BN) : 0;
-  if (qpos_max < 0) blk_hi = 0;
+  if (p.causal && qpos_max < 0) blk_hi = 0;
   int2 qr = make_int2(0, 0);   // segment ids of this tile's rows
   if (SEG) {
     // drop the leading and trailing key blocks that hold none of this tile's segments (packed
@@ -700,7 +700,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const int mn = tile_minmax[2 * x], mx = tile_minmax[2 * x + 1];
     hi[x] = p.causal ? min(nblk_total, mx / F2_T + 1) : nblk_total;
     lo[x] = (p.window > 0) ? max(0, (mn - p.window + 1) / F2_T) : 0;
-    if (mx < 0) hi[x] = 0;
+    if (mx < 0 && (p.causal || mx == -0x7fffffff)) hi[x] = 0;   // nothing to see, or no rows
     if (hi[x] <= lo[x]) { lo[x] = 0; hi[x] = 0; }
   }
   const int any = (hi[0] > lo[0]) || (hi[1] > lo[1]);

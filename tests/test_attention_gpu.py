@@ -148,3 +148,22 @@ def test_attention_logit_soft_cap(cuda_lib, b, s, hq, hkv, causal, window, cap):
   assert ops.attention_impl_in_use().startswith("sm100")
   oa.backward(do)
   assert _rel(qa.grad, qf.grad) < 3e-2
+
+
+@pytest.mark.parametrize("dqk", [128, 192])
+@pytest.mark.parametrize("sq,sk", [(300, 64), (513, 100), (200, 30)])
+@pytest.mark.parametrize("window", [None, 350])
+def test_more_queries_than_keys_without_a_causal_mask(cuda_lib, dqk, sq, sk, window):
+  """Queries whose natural position lies before the first key see every key unless the mask is causal."""
+  from torchprime_b200.ops import attention_sm100 as A
+  torch.manual_seed(sq)
+  q, k, v = (torch.randn(1, s, h, d, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+             for s, h, d in ((sq, 4, dqk), (sk, 2, dqk), (sk, 2, 128)))
+  o = A.attention(q, k, v, causal=False, window=window)
+  do = torch.randn_like(o)
+  got = torch.autograd.grad(o, (q, k, v), do)
+  qf, kf, vf = (t.detach().float().requires_grad_(True) for t in (q, k, v))
+  w = ref.attention(qf, kf, vf, causal=False, window=window)
+  want = torch.autograd.grad(w, (qf, kf, vf), do.float())
+  for a, r in zip((o, *got), (w, *want)):
+    assert ((a.float() - r.float()).norm() / r.float().norm()).item() < 2e-2
