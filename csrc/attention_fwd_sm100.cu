@@ -835,7 +835,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t tS = tmem_base + x * F2_T + lane_addr, tO = tmem_base + 256 + x * F2_T + lane_addr;
     const int* ks = p.kv_seg ? p.kv_seg + (long long)b * p.Sk : nullptr;
-    const int win = p.window > 0 ? p.window : 0x7fffffff;
+    const int win = p.window > 0 ? p.window : 0x40000000;         // (qpos - win must not wrap for positions before the first key)
     const int kmax = p.causal ? min(qpos, p.Sk - 1) : p.Sk - 1;   // keep needs kp <= kmax
     float* xch = reinterpret_cast<float*>(smem + OFF_X) + x * (4 * F2_T);   // [parity][half][row]
     // The two warps that share the rows of a TMEM lane quarter (one per key half) synchronise on a named
