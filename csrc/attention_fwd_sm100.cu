@@ -973,6 +973,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     slot[h * F2_T + r_local] = l;
     named_bar_sync(pair_bar, 64);
     l += slot[(h ^ 1) * F2_T + r_local];
+    if (m_used == -INFINITY) l = 0.f;   // a row without keys (exp2_fma_pair ends at 2^-127, not at 0)
     const float inv_l = (l > 0.f) ? 1.f / l : 0.f;
     if (row_ok && p.lse && h == 0) {
       const float lse = (l > 0.f) ? (m_used + log2f(l)) * 0.6931471805599453f : INFINITY;

@@ -153,7 +153,7 @@ def test_attention_logit_soft_cap(cuda_lib, b, s, hq, hkv, causal, window, cap):
 @pytest.mark.parametrize("dqk", [128, 192])
 @pytest.mark.parametrize("sq,sk", [(300, 64), (513, 100), (200, 30)])
 @pytest.mark.parametrize("window", [None, 350])
-def test_more_queries_than_keys_without_a_causal_mask(cuda_lib, dqk, sq, sk, window):
+def test_forward_and_backward_with_more_queries_than_keys_and_no_causal_mask(cuda_lib, dqk, sq, sk, window):
   """Queries whose natural position lies before the first key see every key unless the mask is causal."""
   from torchprime_b200.ops import attention_sm100 as A
   torch.manual_seed(sq)
@@ -167,3 +167,20 @@ def test_more_queries_than_keys_without_a_causal_mask(cuda_lib, dqk, sq, sk, win
   want = torch.autograd.grad(w, (qf, kf, vf), do.float())
   for a, r in zip((o, *got), (w, *want)):
     assert ((a.float() - r.float()).norm() / r.float().norm()).item() < 2e-2
+
+
+@pytest.mark.parametrize("dqk", [128, 192])
+def test_forward_of_rows_without_keys(cuda_lib, dqk):
+  """Rows that see no key (positions before the first one, an id that no key has) give zeros, next to rows that do."""
+  from torchprime_b200.ops import attention_sm100 as A
+  torch.manual_seed(0)
+  q, k = (torch.randn(1, 200, 2, dqk, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+  v = torch.randn(1, 200, 2, 128, device="cuda", dtype=torch.bfloat16)
+  pos = torch.arange(200, device="cuda")[None] - 37
+  got = A.attention(q, k, v, causal=True, q_positions=pos)
+  want = ref.attention(q.float(), k.float(), v.float(), causal=True, q_positions=pos)
+  assert bool((got[:, :37] == 0).all()) and _rel(got[:, 37:], want[:, 37:]) < 2e-2
+  ids = (torch.arange(200, device="cuda") % 3)[None].int()
+  got = A.attention(q, k, v, causal=False, q_segment_ids=ids, kv_segment_ids=torch.zeros_like(ids))
+  want = ref.attention(q.float(), k.float(), v.float(), causal=False, q_segment_ids=ids, kv_segment_ids=torch.zeros_like(ids))
+  assert bool((got[:, ids[0] != 0] == 0).all()) and _rel(got[:, ids[0] == 0], want[:, ids[0] == 0]) < 2e-2
