@@ -426,6 +426,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const int qseg = (p.q_seg && row_ok) ? p.q_seg[grow] : 0;
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t tS = tmem_base + lane_addr, tO = tmem_base + 128 + lane_addr;
+    const int* ks = p.kv_seg ? p.kv_seg + (long long)b * p.Sk : nullptr;
+    const int win = p.window > 0 ? p.window : 0x40000000;         // (qpos - win must not wrap for positions before the first key)
+    const int kmax = p.causal ? min(qpos, p.Sk - 1) : p.Sk - 1;   // last key this row may see
 
     float m_used = -INFINITY;   // maximum the exponentials are currently taken against (log2 units)
     float l = 0.f;
@@ -433,12 +436,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     for (int j = 0; j < nblk && ok; ++j) {
       const int s = j & 1;
       const uint32_t ph = (j >> 1) & 1;
-      if (!mbar_wait(&s_full[s], ph, p.status, kTimeoutAccFull, 17)) { ok = false; break; }
-      tc_fence_after();
-      uint32_t r[64];
-      tmem_ld32(tS + s * FWD_BN, r);
-      tmem_ld32(tS + s * FWD_BN + 32, r + 32);
-      tmem_wait_ld();
       const int kv0 = (blk_lo + j) * FWD_BN;
       bool seg_mask = p.q_seg != nullptr;
       if (SEG) {   // rows and keys of one and the same segment need no comparison
@@ -447,6 +444,21 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       }
       const bool need_mask = (p.causal && kv0 + FWD_BN - 1 > qpos_min) || (kv0 + FWD_BN > p.Sk) ||
                              (p.window > 0 && qpos_max - kv0 >= p.window) || seg_mask;
+      uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;   // keys kv0 + [0, 32) and kv0 + [32, 64) this row may see
+      if (need_mask) {
+        const int hi = row_ok ? kmax - kv0 : -1, lo = qpos - win - kv0;   // lo < key - kv0 <= hi
+        keep0 = bits_upto(hi) & ~bits_upto(lo);
+        keep1 = bits_upto(hi - 32) & ~bits_upto(lo - 32);
+        if (ks && (!SEG || seg_mask))
+          same_segment_bits(__ldg(ks + min(kv0 + lane, p.Sk - 1)), __ldg(ks + min(kv0 + 32 + lane, p.Sk - 1)), qseg, keep0,
+                            keep1);
+      }
+      if (!mbar_wait(&s_full[s], ph, p.status, kTimeoutAccFull, 17)) { ok = false; break; }
+      tc_fence_after();
+      uint32_t r[64];
+      tmem_ld32(tS + s * FWD_BN, r);
+      tmem_ld32(tS + s * FWD_BN + 32, r + 32);
+      tmem_wait_ld();
       if (p.softcap_in != 0.f) {
 #pragma unroll
         for (int c = 0; c < 64; ++c) r[c] = __float_as_uint(tanh_approx(__uint_as_float(r[c]) * p.softcap_in));
@@ -455,15 +467,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
       // the raw scores); the maximum runs as four chains of three-input max instructions
       float m_blk;
       if (need_mask) {
-        const int* ks = (p.kv_seg && (!SEG || seg_mask)) ? p.kv_seg + (long long)b * p.Sk : nullptr;
 #pragma unroll
-        for (int c = 0; c < 64; ++c) {
-          const int kp = kv0 + c;
-          bool keep = kp < p.Sk && row_ok;
-          if (p.causal) keep = keep && kp <= qpos;
-          if (p.window > 0) keep = keep && (qpos - kp < p.window);
-          if (ks) keep = keep && (kp < p.Sk) && (__ldg(ks + min(kp, p.Sk - 1)) == qseg);
-          r[c] = keep ? r[c] : 0xff800000u;
+        for (int c = 0; c < 32; ++c) {
+          r[c] = (keep0 & (1u << c)) ? r[c] : 0xff800000u;
+          r[c + 32] = (keep1 & (1u << c)) ? r[c + 32] : 0xff800000u;
         }
       }
       {

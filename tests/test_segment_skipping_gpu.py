@@ -68,3 +68,27 @@ def test_keys_and_queries_with_other_ids(cuda_lib):
   dq, dk, dv = torch.autograd.grad(o, (q, k, v), torch.randn_like(o))
   assert bool((o[:, 128:256] == 0).all()) and bool((dq[:, 128:256] == 0).all())
   assert bool(torch.isfinite(dk).all()) and bool(torch.isfinite(dv).all()) and bool((dv != 0).any())
+
+
+@pytest.mark.parametrize("s,window", [(63, 2), (65, 64), (130, 65), (200, 127), (300, None)])
+@pytest.mark.parametrize("positions", ["natural", "reversed halves"])
+def test_masks_as_bits(cuda_lib, s, window, positions):
+  """Masks of 64-score words: window edges inside and at the words' ends, explicit positions, many segments in a warp."""
+  torch.manual_seed(s)
+  q, k, v = (torch.randn(2, s, h, 128, device="cuda", dtype=torch.bfloat16, requires_grad=True) for h in (4, 2, 2))
+  ids = torch.randint(0, 40, (2, s), device="cuda").sort(dim=-1)[0].to(torch.int32)
+  ids[1] = torch.randint(0, 3, (s,), device="cuda")
+  pos, q_ids = None, ids
+  if positions != "natural":
+    pos = torch.cat([torch.arange(s // 2, s), torch.arange(0, s // 2)]).to("cuda", torch.int32).expand(2, s).contiguous()
+    q_ids = ids.gather(1, pos.long())     # (a query sees at least the key at its own position)
+  o = A.attention(q, k, v, causal=True, window=window, q_segment_ids=q_ids, kv_segment_ids=ids, q_positions=pos)
+  do = torch.randn_like(o)
+  got = torch.autograd.grad(o, (q, k, v), do)
+  qf, kf, vf = (t.detach().float().requires_grad_(True) for t in (q, k, v))
+  w = ref.attention(qf, kf, vf, causal=True, window=window, q_segment_ids=q_ids, kv_segment_ids=ids,
+                    q_positions=None if pos is None else pos.long())
+  want = torch.autograd.grad(w, (qf, kf, vf), do.float())
+  for g, r in zip((o, *got), (w, *want)):
+    assert torch.isfinite(g).all()
+    assert ((g.float() - r.float()).norm() / r.float().norm()).item() < 2e-2
