@@ -507,13 +507,20 @@ __global__ void swiglu_bwd_kernel(const uint4* __restrict__ dact, const uint4* _
 
 // ----------------------------------------------------------------------------
 // Cross entropy: one CTA per row, online (max, sum) pass then gradient pass.
+// Two resident CTAs per SM, so that the rows being worked on (296 x 256 KB at a 128k vocabulary) stay in L2 between the
+// passes, and four vectors in flight per thread.  Bound by reading the rows from HBM once and writing them once, with two
+// exponentials per element close behind (16 per clock and SM).  (Four CTAs per SM, one vector at a time and a 64-bit
+// compare per element: 414 us for 3001 rows of 128,256 logits; this way 323.)
 // ----------------------------------------------------------------------------
 constexpr int CE_THREADS = 512;
-__global__ void __launch_bounds__(CE_THREADS)
+constexpr int CE_UNROLL = 4;
+__global__ void __launch_bounds__(CE_THREADS, 2)
 ce_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long* __restrict__ targets,
           float* __restrict__ loss_sum, const float* __restrict__ grad_scale, int rows, int vocab) {
   __shared__ float red[32];
   const int nvec = vocab / 8;  // host guarantees vocab % 8 == 0
+  const float log2e = 1.4426950408889634f;
+  const f32x2 log2e2 = f2_pack(log2e, log2e);
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     uint4* lr = reinterpret_cast<uint4*>(logits + (size_t)row * ld);
     const long long tgt = targets[row];
@@ -522,18 +529,40 @@ ce_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long* __r
       continue;
     }
     float m = -INFINITY, s = 0.f;
-    for (int i = threadIdx.x; i < nvec; i += CE_THREADS) {
-      float f[8];
-      unpack8(lr[i], f);
-      float lm = f[0];
+    for (int i0 = threadIdx.x; i0 < nvec; i0 += CE_THREADS * CE_UNROLL) {
+      uint4 v[CE_UNROLL];
 #pragma unroll
-      for (int e = 1; e < 8; ++e) lm = fmaxf(lm, f[e]);
+      for (int u = 0; u < CE_UNROLL; ++u) {
+        const int i = i0 + u * CE_THREADS;
+        v[u] = i < nvec ? lr[i] : make_uint4(0xff80ff80u, 0xff80ff80u, 0xff80ff80u, 0xff80ff80u);   // -inf
+      }
+      float f[CE_UNROLL][8], mx[CE_UNROLL];
+#pragma unroll
+      for (int u = 0; u < CE_UNROLL; ++u) {
+        unpack8(v[u], f[u]);
+        mx[u] = fmaxf(fmax3(fmaxf(f[u][0], f[u][1]), f[u][2], f[u][3]), fmax3(fmaxf(f[u][4], f[u][5]), f[u][6], f[u][7]));
+      }
+      float lm = mx[0];
+#pragma unroll
+      for (int u = 1; u < CE_UNROLL; ++u) lm = fmaxf(lm, mx[u]);
       if (lm > m) {
         s *= __expf(m - lm);
         m = lm;
       }
+      const float m_fin = m == -INFINITY ? 0.f : m;      // (nothing but -inf so far: their exponentials are 0)
+      const f32x2 nm = f2_pack(-m_fin, -m_fin);
+      f32x2 acc = 0ull;
 #pragma unroll
-      for (int e = 0; e < 8; ++e) s += __expf(f[e] - m);
+      for (int u = 0; u < CE_UNROLL; ++u)
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          float a, b;
+          f2_unpack(f2_mul(f2_add(f2_pack(f[u][e], f[u][e + 1]), nm), log2e2), a, b);
+          acc = f2_add(acc, f2_pack(ex2_approx(a), ex2_approx(b)));
+        }
+      float a, b;
+      f2_unpack(acc, a, b);
+      s += a + b;
     }
     const float gm = block_max(m, red);
     s *= (m == -INFINITY) ? 0.f : __expf(m - gm);
@@ -546,16 +575,33 @@ ce_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long* __r
     }
     __syncthreads();  // the target logit is read before it is overwritten below
     const float inv = 1.f / gs;
-    for (int i = threadIdx.x; i < nvec; i += CE_THREADS) {
-      float f[8];
-      unpack8(lr[i], f);
+    const f32x2 ngm = f2_pack(-gm, -gm), inv2 = f2_pack(inv, inv), scale2 = f2_pack(scale, scale);
+    const int tgt_vec = (int)(tgt / 8), tgt_e = (int)(tgt % 8);
+    for (int i0 = threadIdx.x; i0 < nvec; i0 += CE_THREADS * CE_UNROLL) {
+      uint4 v[CE_UNROLL];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        float p = __expf(f[e] - gm) * inv;
-        if ((long long)i * 8 + e == tgt) p -= 1.f;
-        f[e] = p * scale;
+      for (int u = 0; u < CE_UNROLL; ++u)
+        if (i0 + u * CE_THREADS < nvec) v[u] = lr[i0 + u * CE_THREADS];
+#pragma unroll
+      for (int u = 0; u < CE_UNROLL; ++u) {
+        const int i = i0 + u * CE_THREADS;
+        if (i >= nvec) break;
+        float f[8], p[8];
+        unpack8(v[u], f);
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) {
+          float a, b;
+          f2_unpack(f2_mul(f2_add(f2_pack(f[e], f[e + 1]), ngm), log2e2), a, b);
+          f2_unpack(f2_mul(f2_pack(ex2_approx(a), ex2_approx(b)), inv2), p[e], p[e + 1]);
+        }
+        if (i == tgt_vec) {
+#pragma unroll
+          for (int e = 0; e < 8; ++e) p[e] -= e == tgt_e ? 1.f : 0.f;
+        }
+#pragma unroll
+        for (int e = 0; e < 8; e += 2) f2_unpack(f2_mul(f2_pack(p[e], p[e + 1]), scale2), p[e], p[e + 1]);
+        lr[i] = pack8(p);
       }
-      lr[i] = pack8(f);
     }
   }
 }
@@ -867,7 +913,7 @@ extern "C" int tpb_ce_fwd_bwd(void* logits, long long ld, const long long* targe
                               const float* grad_scale, int rows, int vocab, void* stream) {
   if (vocab % 8 || ld % 8) return -2;
   if (rows <= 0) return 0;
-  int grid = rows < sm_count() * 4 ? rows : sm_count() * 4;
+  const int grid = rows < sm_count() * 2 ? rows : sm_count() * 2;
   ce_kernel<<<grid, CE_THREADS, 0, STREAM(stream)>>>((__nv_bfloat16*)logits, ld, targets, loss_sum, grad_scale, rows,
                                                      vocab);
   return rc(cudaGetLastError());

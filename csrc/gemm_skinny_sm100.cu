@@ -67,6 +67,7 @@ struct SkinnyParams {
   long long ldc2;
   int up_off;           // SwiGLU: feature offset of the "up" half inside the second W map
   float alpha;
+  const float* alpha_dev;   // one more factor, in device memory, or null
   int epi;
   int t_tiles, splits, num_kb, kb_per;
   const int* tile_expert;   // grouped: expert of every token tile (-1: unused); null: dense
@@ -316,6 +317,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   cluster_sync_all();           // every CTA's partial tile is in its shared memory
 
   {
+    const float alpha = p.alpha_dev ? p.alpha * __ldg(p.alpha_dev) : p.alpha;
     const int per = NT / p.splits;                    // tokens this CTA finishes (splits divides 16)
     const int gpt = swiglu ? SK_TN / 8 : SK_TN / 4;   // groups of four features per token
     for (int i = threadIdx.x; i < per * gpt; i += SK_THREADS) {
@@ -325,10 +327,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const int n = min(4, p.N - col);
       float4 a = F32 ? sum_pairs(smem_u32(part + t * SK_TN + c), NT * SK_TN * 4, p.splits)
                      : sum_partials(smem_u32(part + t * SK_TN + c), p.splits);
-      a.x *= p.alpha; a.y *= p.alpha; a.z *= p.alpha; a.w *= p.alpha;
+      a.x *= alpha; a.y *= alpha; a.z *= alpha; a.w *= alpha;
       if (swiglu) {
         float4 u = sum_partials(smem_u32(part + t * SK_TN + SK_TN / 2 + c), p.splits);
-        u.x *= p.alpha; u.y *= p.alpha; u.z *= p.alpha; u.w *= p.alpha;
+        u.x *= alpha; u.y *= alpha; u.z *= alpha; u.w *= alpha;
         if (p.c2) {
           store4(p.c2 + (long long)row * p.ldc2 + col, a, n);
           store4(p.c2 + (long long)row * p.ldc2 + p.N + col, u, n);
@@ -437,7 +439,7 @@ bool skinny_wins_wgrad(int M, int N, int K) {
 int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, int experts,
                 long long ldx, long long ldw, long long w_stride, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                 const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit,
-                int nt, int splits, cudaStream_t stream, bool f32) {
+                int nt, int splits, cudaStream_t stream, bool f32, const float* alpha_dev) {
   if (T <= 0 || N <= 0 || K <= 0) return 0;
   const bool swiglu = epi == TPB_EPI_SWIGLU;
   if (!swiglu && epi != TPB_EPI_BF16 && epi != TPB_EPI_BF16_RES && epi != TPB_EPI_F32) return -2;
@@ -465,7 +467,7 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
   p.aux = reinterpret_cast<const __nv_bfloat16*>(aux); p.ldaux = ldaux;
   p.c2 = reinterpret_cast<__nv_bfloat16*>(c2); p.ldc2 = ldc2;
   p.up_off = two_w ? 0 : N / 2;
-  p.alpha = alpha; p.epi = epi;
+  p.alpha = alpha; p.alpha_dev = alpha_dev; p.epi = epi;
   p.t_tiles = (T + nt - 1) / nt;
   p.num_kb = (K + SK_BK - 1) / SK_BK;
   p.tile_expert = tile_expert;
@@ -520,7 +522,7 @@ using namespace tpb;
 extern "C" int tpb_linear_f32(const void* x, const void* w, float* y, int T, int N, int K, long long ldx, long long ldw,
                               long long ldy, void* stream) {
   return skinny_gemm(x, w, nullptr, y, T, N, K, 1, ldx, ldw, 0, ldy, 0, 0, TPB_EPI_F32, 1.0f, nullptr, 0, nullptr, 0, nullptr,
-                     0, 0, 0, reinterpret_cast<cudaStream_t>(stream), true);
+                     0, 0, 0, reinterpret_cast<cudaStream_t>(stream), true, nullptr);
 }
 
 // The kernel with an explicit token-tile width and K split (0: by rule); see tpb_gemm_bf16 for the rest.
@@ -529,7 +531,7 @@ extern "C" int tpb_gemm_skinny_bf16(const void* x, const void* w, const void* w2
                                     const void* aux, long long ldaux, void* c2, long long ldc2, int nt, int splits,
                                     void* stream) {
   return skinny_gemm(x, w, w2, c, T, N, K, 1, ldx, ldw, 0, ldc, x_mn, w_mn, epi, alpha, aux, ldaux, c2, ldc2, nullptr, 0, nt,
-                     splits, reinterpret_cast<cudaStream_t>(stream), false);
+                     splits, reinterpret_cast<cudaStream_t>(stream), false, nullptr);
 }
 
 // Rows grouped by expert in segments padded to `nt` rows (16 or 32); tile_expert[rows / nt].  Token tiles of expert -1
@@ -540,5 +542,5 @@ extern "C" int tpb_grouped_gemm_skinny_bf16(const void* x, const void* w, const 
                                             int nt, void* stream) {
   if (!tile_expert || E < 1 || experts_hit < 1 || (nt != 16 && nt != 32)) return -2;
   return skinny_gemm(x, w, w2, c, rows, N, K, E, ldx, ldw, w_stride, ldc, 0, w_mn, epi, 1.0f, nullptr, 0, nullptr, 0,
-                     tile_expert, experts_hit, nt, 0, reinterpret_cast<cudaStream_t>(stream), false);
+                     tile_expert, experts_hit, nt, 0, reinterpret_cast<cudaStream_t>(stream), false, nullptr);
 }

@@ -49,6 +49,7 @@ struct GemmParams {
   int b2_off;        // EPI_SWIGLU: row/column offset of the "up" half inside the second B map
   int kb_b2;         // k-blocks from this one on take B from the second map (its k-block kb - kb_b2); INT_MAX: none
   float alpha;
+  const float* alpha_dev;   // one more factor, in device memory (the gradient of a loss), or null
   int epi;
   int group_m;       // rasterisation: m-tiles per group
   int* status;
@@ -553,6 +554,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   } else {
     // ---------------------------------------------------------------- epilogue
     const int q = warp & 3;  // TMEM lane quarter this warp may access
+    const float alpha = p.alpha_dev ? p.alpha * __ldg(p.alpha_dev) : p.alpha;
     uint4* slabs = epi_stage + q * 512;
     int buf = 0;
     int local = 0;
@@ -589,8 +591,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 tmem_wait_ld();
 #pragma unroll
                 for (int j = 0; j < 8; ++j) {
-                  float g0 = __uint_as_float(g[2 * j]) * p.alpha, g1 = __uint_as_float(g[2 * j + 1]) * p.alpha;
-                  float u0 = __uint_as_float(u[2 * j]) * p.alpha, u1 = __uint_as_float(u[2 * j + 1]) * p.alpha;
+                  float g0 = __uint_as_float(g[2 * j]) * alpha, g1 = __uint_as_float(g[2 * j + 1]) * alpha;
+                  float u0 = __uint_as_float(u[2 * j]) * alpha, u1 = __uint_as_float(u[2 * j + 1]) * alpha;
                   o[h * 8 + j] = pack_bf16(silu_f(g0) * u0, silu_f(g1) * u1);
                   pg[h * 8 + j] = pack_bf16(g0, g1);
                   pu[h * 8 + j] = pack_bf16(u0, u1);
@@ -617,8 +619,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                   tmem_wait_ld();
 #pragma unroll
                   for (int j = 0; j < 16; ++j)
-                    o[h * 16 + j] = empty_k ? 0u : pack_bf16(__uint_as_float(r[2 * j]) * p.alpha,
-                                                             __uint_as_float(r[2 * j + 1]) * p.alpha);
+                    o[h * 16 + j] = empty_k ? 0u : pack_bf16(__uint_as_float(r[2 * j]) * alpha,
+                                                             __uint_as_float(r[2 * j + 1]) * alpha);
                 }
                 slab_store<false>(slabs, buf, o, &tmC, col, row0, ez, lane);
               }
@@ -631,7 +633,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                 tmem_ld32(t_addr + c * 32, r);
                 tmem_wait_ld();
 #pragma unroll
-                for (int j = 0; j < 32; ++j) r[j] = empty_k ? 0u : __float_as_uint(__uint_as_float(r[j]) * p.alpha);
+                for (int j = 0; j < 32; ++j) r[j] = empty_k ? 0u : __float_as_uint(__uint_as_float(r[j]) * alpha);
                 if (p.epi == TPB_EPI_F32) slab_store<false>(slabs, buf, r, &tmC, col, row0, ez, lane);
                 else slab_store<true>(slabs, buf, r, &tmC, col, row0, ez, lane);
               }
@@ -653,8 +655,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             uint32_t o[16], pg[16], pu[16];
 #pragma unroll
             for (int j = 0; j < 16; ++j) {
-              float g0 = __uint_as_float(g[2 * j]) * p.alpha, g1 = __uint_as_float(g[2 * j + 1]) * p.alpha;
-              float u0 = __uint_as_float(u[2 * j]) * p.alpha, u1 = __uint_as_float(u[2 * j + 1]) * p.alpha;
+              float g0 = __uint_as_float(g[2 * j]) * alpha, g1 = __uint_as_float(g[2 * j + 1]) * alpha;
+              float u0 = __uint_as_float(u[2 * j]) * alpha, u1 = __uint_as_float(u[2 * j + 1]) * alpha;
               o[j] = pack_bf16(silu_f(g0) * u0, silu_f(g1) * u1);
               pg[j] = pack_bf16(g0, g1);
               pu[j] = pack_bf16(u0, u1);
@@ -707,7 +709,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             for (int v = 0; v < 4; ++v) {
               float f[8];
 #pragma unroll
-              for (int j = 0; j < 8; ++j) f[j] = empty_k ? 0.f : __uint_as_float(r[8 * v + j]) * p.alpha;
+              for (int j = 0; j < 8; ++j) f[j] = empty_k ? 0.f : __uint_as_float(r[8 * v + j]) * alpha;
               if (R && col + 8 * v + 8 <= p.N) {
                 const uint4 old = *reinterpret_cast<const uint4*>(R + 8 * v);
                 const float2 a = unpack_bf16(old.x), b = unpack_bf16(old.y), cc = unpack_bf16(old.z), d = unpack_bf16(old.w);
@@ -763,8 +765,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             if (full_chunk) {
 #pragma unroll
               for (int v = 0; v < 8; ++v) {
-                float4 o = make_float4(__uint_as_float(r[4 * v]) * p.alpha, __uint_as_float(r[4 * v + 1]) * p.alpha,
-                                       __uint_as_float(r[4 * v + 2]) * p.alpha, __uint_as_float(r[4 * v + 3]) * p.alpha);
+                float4 o = make_float4(__uint_as_float(r[4 * v]) * alpha, __uint_as_float(r[4 * v + 1]) * alpha,
+                                       __uint_as_float(r[4 * v + 2]) * alpha, __uint_as_float(r[4 * v + 3]) * alpha);
                 if (accm) {
                   float4 old = *reinterpret_cast<float4*>(C + 4 * v);
                   o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
@@ -773,7 +775,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               }
             } else {
               for (int j = 0; j < 32 && col + j < p.N; ++j) {
-                float o = __uint_as_float(r[j]) * p.alpha;
+                float o = __uint_as_float(r[j]) * alpha;
                 C[j] = accm ? C[j] + o : o;
               }
             }
@@ -788,7 +790,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               for (int v = 0; v < 4; ++v) {
                 float f[8];
 #pragma unroll
-                for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[8 * v + j]) * p.alpha;
+                for (int j = 0; j < 8; ++j) f[j] = __uint_as_float(r[8 * v + j]) * alpha;
                 if (R) {
                   uint4 old = *reinterpret_cast<const uint4*>(R + 8 * v);
                   float2 a = unpack_bf16(old.x), b = unpack_bf16(old.y), cc = unpack_bf16(old.z), d = unpack_bf16(old.w);
@@ -800,7 +802,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
               }
             } else {
               for (int j = 0; j < 32 && col + j < p.N; ++j) {
-                float o = __uint_as_float(r[j]) * p.alpha;
+                float o = __uint_as_float(r[j]) * alpha;
                 if (R) o += __bfloat162float(R[j]);
                 C[j] = __float2bfloat16(o);
               }
@@ -884,7 +886,7 @@ cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const
 int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, int experts,
                 long long ldx, long long ldw, long long w_stride, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                 const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit, int nt,
-                int splits, cudaStream_t stream, bool f32);
+                int splits, cudaStream_t stream, bool f32, const float* alpha_dev = nullptr);
 bool skinny_wins(int M, int N, int K, bool swiglu);
 bool skinny_wins_wgrad(int M, int N, int K);
 
@@ -899,7 +901,7 @@ struct GemmCall {
   int M, N, K, E;
   long long lda, ldb, b_expert_stride, ldc;
   int a_mn, b_mn, epi;
-  float alpha;
+  float alpha; const float* alpha_dev;
   const void* aux; long long ldaux;
   void* c2; long long ldc2;
   int max_ctas;
@@ -977,7 +979,7 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   p.b_split = g.N / 2;
   p.b2_off = two_b ? 0 : g.N / 2;
   p.kb_b2 = cat_k ? k_one / BK : 0x7fffffff;
-  p.alpha = g.alpha;
+  p.alpha = g.alpha; p.alpha_dev = g.alpha_dev;
   p.epi = g.epi;
   p.status = status_block();
   p.mode = g.mode; p.num_experts = g.E; p.tile_expert = g.tile_expert; p.k_offsets = g.k_offsets;
@@ -1071,25 +1073,34 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
 
 using namespace tpb;
 
-extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
-                             long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha,
-                             const void* aux, long long ldaux, void* c2, long long ldc2, int max_ctas,
-                             void* stream_) {
+// tpb_gemm_bf16 with one more factor read from device memory (or null) when the result is written: alpha * *scale.
+extern "C" int tpb_gemm_scaled_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                                    long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha,
+                                    const float* scale, const void* aux, long long ldaux, void* c2, long long ldc2,
+                                    int max_ctas, void* stream_) {
   // few rows or few tiles: the kernel that streams B once and splits the contraction
   if (max_ctas == 0 && gemm_pair_mode() == 1 &&
       (a_mn ? b_mn && skinny_wins_wgrad(M, N, K) : skinny_wins(M, N, K, epi == TPB_EPI_SWIGLU))) {
     const int r = skinny_gemm(A, B, nullptr, C, M, N, K, 1, lda, ldb, 0, ldc, a_mn, b_mn, epi, alpha, aux, ldaux, c2, ldc2,
-                              nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_), false);
+                              nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_), false, scale);
     if (r != -2) return r;     // -2: an epilogue or alignment it does not take
   }
   GemmCall g{};
   g.A = A; g.B = B; g.B2 = nullptr; g.C = C;
   g.M = M; g.N = N; g.K = K; g.E = 1;
   g.lda = lda; g.ldb = ldb; g.b_expert_stride = 0; g.ldc = ldc;
-  g.a_mn = a_mn; g.b_mn = b_mn; g.epi = epi; g.alpha = alpha;
+  g.a_mn = a_mn; g.b_mn = b_mn; g.epi = epi; g.alpha = alpha; g.alpha_dev = scale;
   g.aux = aux; g.ldaux = ldaux; g.c2 = c2; g.ldc2 = ldc2; g.max_ctas = max_ctas;
   g.mode = 0;
   return run_gemm(g, reinterpret_cast<cudaStream_t>(stream_));
+}
+
+extern "C" int tpb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                             long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha,
+                             const void* aux, long long ldaux, void* c2, long long ldc2, int max_ctas,
+                             void* stream_) {
+  return tpb_gemm_scaled_bf16(A, B, C, M, N, K, lda, ldb, ldc, a_mn, b_mn, epi, alpha, nullptr, aux, ldaux, c2, ldc2,
+                              max_ctas, stream_);
 }
 
 extern "C" int tpb_grouped_gemm_bf16(const void* A, const void* B, const void* B2, void* C, int M, int N, int K,

@@ -35,6 +35,11 @@ int tpb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lo
                   long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha,
                   const void* aux, long long ldaux, void* c2, long long ldc2, int max_ctas,
                   void* stream);
+// The same with one more factor, *scale in device memory (null: 1), when the result is written.
+int tpb_gemm_scaled_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
+                         long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha, const float* scale,
+                         const void* aux, long long ldaux, void* c2, long long ldc2, int max_ctas,
+                         void* stream);
 
 // y = rmsnorm(x [+ res]) * w.  h_out (optional) receives x + res.  rstd: [rows] fp32.
 int tpb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd,

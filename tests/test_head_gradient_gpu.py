@@ -42,3 +42,47 @@ def test_batched_gradients(cuda_lib):
   for i in range(3):
     for a, b in zip(got, torch.autograd.grad(loss, (h, w), scales[i], retain_graph=True)):
       assert torch.equal(a[i], b)
+
+
+@pytest.mark.parametrize("m,n,kk", [(40, 128, 512), (304, 264, 200), (2560, 2816, 128)])   # few rows, tiles, CTA pairs
+@pytest.mark.parametrize("mn", [False, True])
+def test_gemm_scaled_on_the_device(cuda_lib, m, n, kk, mn):
+  """The factor in device memory multiplies the fp32 sums: the same bits as scaling an fp32 result and rounding."""
+  torch.manual_seed(m)
+  a, b = (torch.randn(*((kk, r) if mn else (r, kk)), device="cuda", dtype=torch.bfloat16) for r in (m, n))
+  s = torch.tensor(-0.37, device="cuda")
+  want = (k.gemm(a, b, a_mn=mn, b_mn=mn, epi=k.EPI_F32) * s).to(torch.bfloat16)
+  assert torch.equal(k.gemm(a, b, a_mn=mn, b_mn=mn, scale=s), want)
+
+
+@pytest.mark.parametrize("wanted", ["both", "weight", "hidden"])
+def test_head_in_one_piece(cuda_lib, wanted):
+  """All rows in one chunk: the weight gradient is made in the backward pass, as often as it is asked for."""
+  h = torch.randn(1, 130, 64, device="cuda", dtype=torch.bfloat16, requires_grad=wanted != "weight")
+  w = (torch.randn(520, 64, device="cuda") / 8).to(torch.bfloat16).requires_grad_(wanted != "hidden")
+  t = torch.randint(0, 520, (1, 130), device="cuda")
+  t[0, 3:50] = -100
+  inputs = [x for x in (h, w) if x.requires_grad]
+  loss = ops.linear_cross_entropy(h, w, t)
+  first = torch.autograd.grad(loss, inputs, retain_graph=True)
+  again = torch.autograd.grad(loss * 2, inputs)
+  ref_in = [x.detach().double().requires_grad_(x.requires_grad) for x in (h, w)]
+  want = torch.autograd.grad(F.cross_entropy((ref_in[0] @ ref_in[1].t())[0], t[0]), [x for x in ref_in if x.requires_grad])
+  for a, b, r in zip(first, again, want):
+    assert torch.equal(2 * a, b)
+    assert ((a.double() - r).norm() / r.norm()).item() < 1e-2      # bf16 logits and bf16 d(logits)
+
+
+@pytest.mark.parametrize("vocab", [8, 16376, 16384, 16392, 49160])
+def test_cross_entropy_at_the_edges_of_its_loops(cuda_lib, vocab):
+  logits = (3 * torch.randn(5, vocab, device="cuda")).to(torch.bfloat16)
+  logits[1, :vocab // 2] = float("-inf")
+  t = torch.tensor([0, vocab - 1, -100, vocab // 2, vocab - 8], device="cuda")
+  x = logits.double().requires_grad_(True)
+  want = F.cross_entropy(x, t, ignore_index=-100, reduction="sum")
+  want.backward()
+  loss = torch.zeros(1, device="cuda")
+  k.ce_fwd_bwd_(logits, t, loss, torch.tensor([0.5], device="cuda"))
+  assert abs(loss.item() / want.item() - 1) < 1e-5
+  # bf16 results: 2^-9 of each value
+  assert ((logits.double() - 0.5 * x.grad).abs() <= 2.0 ** -8 * (0.5 * x.grad).abs() + 1e-9).all()

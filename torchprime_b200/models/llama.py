@@ -209,7 +209,8 @@ class CausalLMHead(nn.Module):
       h = self.norm(hidden)
       n_valid = self._valid_count(targets) if targets is not None else None
       if targets is not None and not want_logits:
-        return None, ops.linear_cross_entropy(h, self.lm_head.weight, targets, n_valid=n_valid)
+        w = self.lm_head.weight
+        return None, ops.linear_cross_entropy(h, w, targets, chunk_rows=ops.head_chunk_rows(w), n_valid=n_valid)
       logits = ops.linear(h, self.lm_head.weight).float()
       loss = None
       if targets is not None:

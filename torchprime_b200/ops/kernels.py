@@ -28,12 +28,13 @@ def _row_major_2d(t: torch.Tensor, name: str):
   return t.shape[0], t.shape[1], t.stride(0) if t.shape[0] > 1 else max(t.stride(0), t.shape[1])
 
 
-def gemm(a, b, *, a_mn=False, b_mn=False, out=None, epi=EPI_BF16, alpha=1.0, aux=None, c2=None, max_ctas=0):
+def gemm(a, b, *, a_mn=False, b_mn=False, out=None, epi=EPI_BF16, alpha=1.0, aux=None, c2=None, max_ctas=0, scale=None):
   """C = alpha * A @ B^T with logical A [M,K], B [N,K].
 
   ``a_mn``/``b_mn`` say that the tensor passed is the transposed storage ([K,M]
   resp. [K,N]).  ``epi`` selects the fused epilogue (see csrc/tpb.h).  For
-  ``EPI_SWIGLU`` B holds [gate; up] rows and the result has N/2 columns.
+  ``EPI_SWIGLU`` B holds [gate; up] rows and the result has N/2 columns.  ``scale``: a
+  one-element fp32 tensor that multiplies the result before it is rounded.
   """
   assert a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16
   r0, r1, lda = _row_major_2d(a, "a")
@@ -58,8 +59,9 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, epi=EPI_BF16, alpha=1.0, aux
   if c2 is not None:
     assert epi == EPI_SWIGLU and c2.shape == (M, N) and c2.stride(1) == 1 and c2.dtype == torch.bfloat16
     ldc2 = c2.stride(0)
-  rc = lib().tpb_gemm_bf16(ptr(a), ptr(b), ptr(out), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), epi, float(alpha),
-                           ptr(aux), ldaux, ptr(c2), ldc2, int(max_ctas), stream_ptr())
+  assert scale is None or (scale.dtype == torch.float32 and scale.numel() == 1 and scale.device == a.device)
+  rc = lib().tpb_gemm_scaled_bf16(ptr(a), ptr(b), ptr(out), M, N, K, lda, ldb, ldc, int(a_mn), int(b_mn), epi,
+                                  float(alpha), ptr(scale), ptr(aux), ldaux, ptr(c2), ldc2, int(max_ctas), stream_ptr())
   check(rc, f"gemm M={M} N={N} K={K} a_mn={a_mn} b_mn={b_mn} epi={epi}")
   return out
 
