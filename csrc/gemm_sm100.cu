@@ -63,6 +63,7 @@ struct GemmParams {
   int num_experts;
   const int* tile_expert;
   const int* k_offsets;
+  const int* k_counts;      // mode 2: rows of expert e that are not padding (at the front of its range), or null: all
   long long c_stride;
   // All-gather fusion: the flat buffer that contains B is sharded over ag_world GPUs.  The
   // first ag_copiers CTAs pull every shard (peer memory, plain bulk copies) into the local
@@ -129,7 +130,7 @@ __device__ __forceinline__ TileInfo tile_info(const GemmParams& p, int t, int m_
     ti.e = t / per;
     tile_coords(t - ti.e * per, m_tiles, n_tiles, p.group_m, ti.tm, ti.tn);
     ti.kb0 = p.k_offsets[ti.e] / BK;
-    ti.kb1 = p.k_offsets[ti.e + 1] / BK;
+    ti.kb1 = p.k_counts ? (p.k_offsets[ti.e] + p.k_counts[ti.e] + BK - 1) / BK : p.k_offsets[ti.e + 1] / BK;
   } else {
     tile_coords(t, m_tiles, n_tiles, p.group_m, ti.tm, ti.tn);
     if (p.mode == 1) {
@@ -905,7 +906,7 @@ struct GemmCall {
   const void* aux; long long ldaux;
   void* c2; long long ldc2;
   int max_ctas;
-  int mode; const int* tile_expert; const int* k_offsets; long long c_stride;
+  int mode; const int* tile_expert; const int* k_offsets; const int* k_counts; long long c_stride;
   int row_align;                // grouped rows mode: expert segments are padded to this many rows (128 or 256)
   // fusion with collectives (0 / null when unused)
   int ag_world, ag_copiers, ag_local; const void* const* ag_src; void* ag_dst; long long ag_shard_elems, ag_b_offset;
@@ -983,6 +984,7 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   p.epi = g.epi;
   p.status = status_block();
   p.mode = g.mode; p.num_experts = g.E; p.tile_expert = g.tile_expert; p.k_offsets = g.k_offsets;
+  p.k_counts = g.k_counts;
   p.c_stride = g.c_stride;
   p.ag_world = g.ag_world; p.ag_copiers = g.ag_world > 0 ? g.ag_copiers : 0;
   p.ag_dst = g.ag_dst; p.ag_shard_elems = g.ag_shard_elems; p.ag_chunk_elems = 16384; p.ag_b_offset = g.ag_b_offset;
@@ -1122,6 +1124,22 @@ extern "C" int tpb_grouped_gemm_bf16(const void* A, const void* B, const void* B
   return run_gemm(g, reinterpret_cast<cudaStream_t>(stream_));
 }
 
+
+// Per-expert weight gradients (mode 2 of tpb_grouped_gemm_bf16) that contract over the rows in front of every segment's
+// padding only: expert e's rows are k_offsets[e] + [0, k_counts[e]), to the next multiple of 64, and those up to there are
+// zero.  k_counts null: the whole segments.
+extern "C" int tpb_grouped_wgrad_bf16(const void* A, const void* B, void* C, int M, int N, int rows, int E, long long lda,
+                                      long long ldb, long long ldc, int epi, const int* k_offsets, const int* k_counts,
+                                      long long c_stride, void* stream_) {
+  if (!k_offsets) return -2;
+  GemmCall g{};
+  g.A = A; g.B = B; g.C = C;
+  g.M = M; g.N = N; g.K = rows; g.E = E;
+  g.lda = lda; g.ldb = ldb; g.ldc = ldc;
+  g.a_mn = 1; g.b_mn = 1; g.epi = epi; g.alpha = 1.f;
+  g.mode = 2; g.k_offsets = k_offsets; g.k_counts = k_counts; g.c_stride = c_stride;
+  return run_gemm(g, reinterpret_cast<cudaStream_t>(stream_));
+}
 
 // C = A * B^T where the flat bf16 buffer holding B is sharded over `world` GPUs: shard_ptrs[r] is
 // rank r's shard (peer-mapped symmetric memory), `gathered` the local buffer that receives all

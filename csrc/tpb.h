@@ -101,6 +101,10 @@ int tpb_grouped_gemm_bf16(const void* A, const void* B, const void* B2, void* C,
                           long long lda, long long ldb, long long b_expert_stride, long long ldc, int a_mn, int b_mn,
                           int epi, float alpha, void* c2, long long ldc2, int mode, const int* tile_expert,
                           const int* k_offsets, long long c_stride, int row_align, void* stream);
+// Mode 2 without the padding: expert e contracts over k_counts[e] rows from k_offsets[e] on (null: its whole segment).
+int tpb_grouped_wgrad_bf16(const void* A, const void* B, void* C, int M, int N, int rows, int E, long long lda,
+                           long long ldb, long long ldc, int epi, const int* k_offsets, const int* k_counts,
+                           long long c_stride, void* stream);
 
 // GEMM fused with the all-gather of the (flat, sharded) buffer that holds B, and GEMM fused with the
 // reduce-scatter of C into the owners' shards; see the comments at the definitions in gemm_sm100.cu.

@@ -79,3 +79,23 @@ def test_columns_that_end_inside_a_vector(cuda_lib, M, N, epi):
   err = (out.double() - want).abs()
   assert bool((err <= (2.0 ** -8 if dt == torch.bfloat16 else 0.0) * want.abs() + 2e-6 * 136).all()), err.max()
   assert bool((big[:, N:] == 5.0).all())
+
+
+@pytest.mark.parametrize("counts", [[1, 63, 64, 65], [128, 0, 129, 300]])
+@pytest.mark.parametrize("align", [128, 256])
+def test_weight_gradients_stop_at_the_padding(cuda_lib, counts, align):
+  """An expert's contraction ends at the multiple of 64 behind its rows: what the rest of its segment holds is not read."""
+  torch.manual_seed(align)
+  idx = torch.cat([torch.full((c,), i) for i, c in enumerate(counts)])[:, None].to("cuda", torch.int32)
+  plan = moe.build_dispatch_plan(idx, len(counts), row_align=align)
+  a, b = (torch.randn(plan.num_rows, d, device="cuda", dtype=torch.bfloat16) for d in (72, 136))
+  off = plan.k_offsets.tolist()
+  out = torch.empty(len(counts), 72, 136, device="cuda", dtype=torch.float32)
+  for x, c in enumerate(counts):
+    for t in (a, b):
+      t[off[x] + c:off[x + 1]] = 0.0
+      t[off[x] + (c + 63) // 64 * 64:off[x + 1]] = float("nan")
+  moe.grouped_gemm_wgrad(a, b, plan, out, False)
+  for x, c in enumerate(counts):
+    want = a[off[x]:off[x] + c].double().t() @ b[off[x]:off[x] + c].double()
+    assert bool(((out[x].double() - want).abs() <= 2e-6 * max(c, 1) + 1e-6).all())

@@ -27,6 +27,7 @@ from ._lib import check, lib, ptr, stream_ptr
 P, I, LL, FL = c_void_p, c_int, c_longlong, c_float
 _lib.register_signature("tpb_grouped_gemm_bf16", [P, P, P, P, I, I, I, I, LL, LL, LL, LL, I, I, I, FL, P, LL, I, P, P,
                                                   LL, I, P])
+_lib.register_signature("tpb_grouped_wgrad_bf16", [P, P, P, I, I, I, I, LL, LL, LL, I, P, P, LL, P])
 _lib.register_signature("tpb_router_topk", [P, I, P, P, P, P, I, I, I, I, I, I, I, FL, P])
 _lib.register_signature("tpb_router_bwd", [P, I, P, P, P, P, I, I, I, I, I, FL, P])
 _lib.register_signature("tpb_moe_plan", [P, I, I, I, I, I, P, P, P, P, P, P, P])
@@ -328,9 +329,11 @@ def grouped_gemm_wgrad(a_rows, b_rows, plan: DispatchPlan, out, accumulate: bool
     epi = _lib.EPI_F32_ACC if accumulate else _lib.EPI_F32
   else:
     epi = _lib.EPI_BF16_ACC if accumulate else _lib.EPI_BF16
-  rc = lib().tpb_grouped_gemm_bf16(ptr(a_rows), ptr(b_rows), None, ptr(out), da, db, a_rows.shape[0], e,
-                                   a_rows.stride(0), b_rows.stride(0), 0, out.stride(1), 1, 1, epi, 1.0, None, 0, 2,
-                                   None, ptr(plan.k_offsets), out.stride(0), 0, stream_ptr())
+  # (the kernel's plan has its rows in front of each segment's padding, which then need not be read)
+  counts = plan.counts if isinstance(plan, DispatchPlan) and plan.counts.dtype == torch.int32 else None
+  rc = lib().tpb_grouped_wgrad_bf16(ptr(a_rows), ptr(b_rows), ptr(out), da, db, a_rows.shape[0], e, a_rows.stride(0),
+                                    b_rows.stride(0), out.stride(1), epi, ptr(plan.k_offsets), ptr(counts), out.stride(0),
+                                    stream_ptr())
   check(rc, f"grouped_gemm wgrad E={e} {da}x{db}")
   return out
 
