@@ -989,6 +989,15 @@ extern "C" int tpb_scale_cast_bf16(const float* src, void* dst, long long n, con
   return rc(cudaGetLastError());
 }
 
+// tpb_rmsnorm_bwd with the weight gradient's sums cleared first and, with dw_bf16, delivered in bf16 (dim % 4 == 0).
+extern "C" int tpb_rmsnorm_bwd_dw(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
+                                  float* dw_f32, void* dw_bf16, int rows, int dim, void* stream) {
+  cudaError_t e = cudaMemsetAsync(dw_f32, 0, sizeof(float) * dim, STREAM(stream));
+  if (e != cudaSuccess) return rc(e);
+  const int r = tpb_rmsnorm_bwd(dy, x, w, rstd, dres, dx, dw_f32, rows, dim, stream);
+  return r || !dw_bf16 ? r : tpb_cast_f32_to_bf16(dw_f32, dw_bf16, dim, 1.f, 0, stream);
+}
+
 // ----------------------------------------------------------------------------
 // Allocation-free variant of the RMSNorm backward (see tpb_noalloc.h).
 // ----------------------------------------------------------------------------

@@ -47,6 +47,9 @@ int tpb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void
 // dx = d/dx of the above (+ dres if given).  dw_f32 [dim] is accumulated with atomics.
 int tpb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres,
                     void* dx, float* dw_f32, int rows, int dim, void* stream);
+// The same with dw_f32 cleared first and, if dw_bf16 is given, its sums delivered there.
+int tpb_rmsnorm_bwd_dw(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
+                       float* dw_f32, void* dw_bf16, int rows, int dim, void* stream);
 
 // In-place rotate-half RoPE on `heads` heads of width `dim` starting at column
 // `col0` of a [tokens, ld] bf16 matrix.  cos/sin: fp32 [max_pos, dim/2].

@@ -16,6 +16,7 @@ import torch
 
 _LIB_PATH = os.path.join(os.path.dirname(os.path.dirname(os.path.abspath(__file__))), "lib", "libtpb200.so")
 _lib = None
+_native = None      # the operators of csrc/torch_ops.cpp, loaded with the library
 
 EPI_BF16, EPI_F32, EPI_F32_ACC, EPI_BF16_ACC, EPI_BF16_RES, EPI_SWIGLU = range(6)
 EPI_RS_BF16, EPI_AR_BF16 = 6, 7     # reduce-scatter / all-reduce epilogues of the fused collective GEMMs
@@ -50,9 +51,31 @@ def lib():
       raise KernelError(
         f"{_LIB_PATH} is missing: run `python -m torchprime_b200.build` (nvcc, sm_100a) first"
       )
-    _lib = ctypes.CDLL(_LIB_PATH)
-    _declare(_lib)
+    L = ctypes.CDLL(_LIB_PATH)
+    _declare(L)
+    _load_native()
+    _lib = L
   return _lib
+
+
+def _load_native():
+  global _native
+  path = os.path.join(os.path.dirname(_LIB_PATH), "_tpb_torch.so")
+  if not os.path.exists(path):
+    raise KernelError(f"{path} is missing: run `python -m torchprime_b200.build` first")
+  import importlib.util
+
+  from . import functional
+  spec = importlib.util.spec_from_file_location("_tpb_torch", path)
+  mod = importlib.util.module_from_spec(spec)
+  spec.loader.exec_module(mod)
+  mod.configure(check, functional._late_wgrads, functional._norm_wgrad)
+  _native = mod
+
+
+def native():
+  """The native operators once the library is loaded, else None (the first call of an operator loads it)."""
+  return _native if _lib is not None else None
 
 
 def _declare(L):
@@ -122,7 +145,7 @@ _LAUNCHES = [0]
 
 def launch_count() -> int:
   """Number of kernel launches issued through this binding so far."""
-  return _LAUNCHES[0]
+  return _LAUNCHES[0] + (_native.launch_count() if _native is not None else 0)
 
 
 def check(rc: int, what: str):

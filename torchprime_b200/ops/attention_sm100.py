@@ -259,17 +259,6 @@ def _nothing_recorded() -> bool:
 def attention_qkv(qkv, hq, hkv, d, causal=True, scale=None, window=None, q_segment_ids=None, q_positions=None):
   """Self-attention on a fused [B, S, (Hq + 2 Hkv) * D] projection (head dim 128, contiguous)."""
   seg = _i32(q_segment_ids)
-  if _nothing_recorded() and qkv.dim() == 3 and qkv.is_contiguous() and hkv > 0 and hq % hkv == 0 and qkv.shape[-1] == (hq + 2 * hkv) * d:
-    b, s, width = qkv.shape
-    o = torch.empty(b, s, hq, d, dtype=qkv.dtype, device=qkv.device)
-    lse = torch.empty(b, hq, s, dtype=torch.float32, device=qkv.device)
-    q_rng, kv_rng = _seg_ranges(seg, seg, b, s, s)
-    pos, at = _i32(q_positions), qkv.data_ptr()
-    check(lib().tpb_attn_fwd_softcap(at, at + 2 * hq * d, at + 2 * (hq + hkv) * d, ptr(o), ptr(lse), b, s, s, hq, hkv, d, d,
-                                     width, width, width, hq * d, float(scale if scale is not None else d ** -0.5),
-                                     int(bool(causal)), int(window or 0), ptr(pos), ptr(seg), ptr(seg), ptr(q_rng),
-                                     ptr(kv_rng), 0.0, stream_ptr()), f"attn_fwd qkv{tuple(qkv.shape)}")
-    return o
   return _AttentionQKVFn.apply(qkv, hq, hkv, d, causal, scale, window, _i32(q_positions), seg, seg)
 
 

@@ -18,7 +18,7 @@ from contextlib import contextmanager
 import torch
 import torch.nn.functional as F
 
-from . import _lib, reference as ref
+from . import _debug, _lib, reference as ref
 
 _STATE = {"backend": "auto", "attention": "auto"}
 
@@ -168,6 +168,14 @@ def get_gather_context():
   return _AG_CTX[0]
 
 
+def _native():
+  """The native operators (csrc/torch_ops.cpp), which answer None for calls they are not meant for; or None: kernels are
+  switched off or not loaded yet, or a gather is in flight."""
+  if _AG_CTX[0] is None and _STATE["backend"] != "torch":
+    return _lib.native()
+  return None
+
+
 def _inflight(w):
   """(context, element offset) when ``w`` belongs to a gather that is still in flight."""
   ctx = _AG_CTX[0]
@@ -253,6 +261,17 @@ class _LinearFn(torch.autograd.Function):
     return (dx, dres, None, None, *wgrads)
 
 
+def _late_wgrads(ws, dy2, x2):
+  """Weight gradients of a native linear whose weights were given a main_grad after its forward pass: collected there,
+  or returned."""
+  from . import kernels as k
+  sink = _grad_sink(ws)
+  if sink is not None:
+    _wgrad_into(sink, ws, dy2, x2)
+    return [None] * len(ws)
+  return list(k.gemm(dy2, x2, a_mn=True, b_mn=True).split([w.shape[0] for w in ws]))
+
+
 def _gemm_friendly(x, ws) -> bool:
   """Shapes the TMA-fed GEMM accepts: 16-byte aligned rows for every operand."""
   n = sum(w.shape[0] for w in ws)
@@ -261,54 +280,6 @@ def _gemm_friendly(x, ws) -> bool:
     return n % 8 == 0 and k % 8 == 0 and all(w.dim() == 2 and w.is_contiguous() for w in ws) and x.shape[-1] == k
   return (n % 8 == 0 and k % 8 == 0 and all(w.dim() == 2 and w.is_contiguous() for w in ws)
           and x.shape[-1] == k and x.reshape(-1, k).stride(-1) == 1 and x.reshape(-1, k).stride(0) % 8 == 0)
-
-
-def _back_to_back(ws) -> bool:
-  """Contiguous 2-D weights of one width that follow one another in one storage."""
-  w0 = ws[0]
-  if w0.dim() != 2 or not w0.is_contiguous():
-    return False
-  if len(ws) == 1:
-    return True
-  k, at, store = w0.shape[1], w0.data_ptr() + 2 * w0.numel(), w0.untyped_storage().data_ptr()
-  for w in ws[1:]:
-    if (w.dim() != 2 or w.shape[1] != k or not w.is_contiguous() or w.data_ptr() != at
-        or w.untyped_storage().data_ptr() != store):
-      return False
-    at += 2 * w.numel()
-  return True
-
-
-def _linear_now(x, ws, residual, swiglu=False):
-  """The forward of :class:`_LinearFn` (or :class:`_LinearSwigluFn`) where nothing is recorded and no
-  collective is involved, without the views and checks that recording needs.  None: not such a call."""
-  if not (_AG_CTX[0] is None and inference_only() and use_kernels(x, *ws) and x.is_contiguous() and _back_to_back(ws)):
-    return None
-  n, k = sum(w.shape[0] for w in ws), ws[0].shape[1]
-  n_out = n // 2 if swiglu else n
-  rows = x.numel() // k if k else 0
-  if x.shape[-1] != k or k % 8 or n_out % 8 or rows == 0:
-    return None
-  epi, aux = (_lib.EPI_SWIGLU if swiglu else _lib.EPI_BF16), None
-  if residual is not None:
-    if (residual.dtype != x.dtype or residual.device != x.device or not residual.is_contiguous()
-        or residual.numel() != rows * n):
-      return None
-    epi, aux = _lib.EPI_BF16_RES, residual.data_ptr()
-  y = torch.empty(*x.shape[:-1], n_out, dtype=x.dtype, device=x.device)
-  _lib.check(_lib.lib().tpb_gemm_bf16(x.data_ptr(), ws[0].data_ptr(), y.data_ptr(), rows, n, k, k, k, n_out, 0, 0, epi, 1.0,
-                                      aux, n, None, 0, 0, _lib.stream_ptr()), "gemm")
-  return y
-
-
-def _norm_now(x, w, eps):
-  """The forward of :class:`_RMSNormFn` where nothing is recorded."""
-  xc = x.contiguous()
-  d = x.shape[-1]
-  y = torch.empty_like(xc)
-  _lib.check(_lib.lib().tpb_rmsnorm_fwd(xc.data_ptr(), None, w.data_ptr(), y.data_ptr(), None, None, xc.numel() // d, d,
-                                        float(eps), _lib.stream_ptr()), "rmsnorm_fwd")
-  return y
 
 
 def _reducer_ok(reducer, x, n_out, k_in) -> bool:
@@ -325,8 +296,8 @@ def linear(x, weights, bias=None, residual=None, tp_reduce=None, tp_reduce_grad=
   reduce again), ``tp_reduce_grad`` sums the INPUT GRADIENT (column-parallel weight).  Callers ask
   ``reducer.usable(rows, n, k)`` first; a request that cannot be honoured raises."""
   ws = list(weights) if isinstance(weights, (list, tuple)) else [weights]
-  if bias is None and tp_reduce is None and tp_reduce_grad is None:
-    y = _linear_now(x, ws, residual)
+  if bias is None and tp_reduce is None and tp_reduce_grad is None and (nat := _native()) is not None:
+    y = nat.linear(x, ws, residual)
     if y is not None:
       return y
   if (use_kernels(x, *ws) and bias is None and (len(ws) == 1 or _adjacent(ws)) and _gemm_friendly(x, ws)
@@ -374,12 +345,13 @@ def linear_f32(x, w):
   bf16 operands go into the kernel as they are instead of through fp32 copies: their products are exact, and the sum is
   kept as exact as an fp32 one (an ordinary GEMM's, cut to 24 bits along the whole contraction, is not: K = 2048 of
   a 102,400-wide head 2e-6 instead of 1e-7 from the 64-bit result)."""
+  if (nat := _native()) is not None:
+    y = nat.linear_f32(x, w)
+    if y is not None:
+      return y
   _settle(w)
   if (x.dim() == 2 and use_kernels(x, w) and x.shape[0] > 0 and _gemm_friendly(x, [w])
       and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
-    if inference_only():
-      from . import kernels as k
-      return k.linear_f32(x, w)
     return _LinearF32Fn.apply(x, w)
   return F.linear(x.float(), w.float())
 
@@ -430,8 +402,8 @@ class _LinearSwigluFn(torch.autograd.Function):
 
 def linear_swiglu(x, w_gate, w_up, tp_reduce_grad=None):
   """silu(x @ w_gate^T) * (x @ w_up^T) as one GEMM with a fused epilogue."""
-  if tp_reduce_grad is None and w_gate.shape == w_up.shape:
-    y = _linear_now(x, [w_gate, w_up], None, swiglu=True)
+  if tp_reduce_grad is None and (nat := _native()) is not None:
+    y = nat.linear_swiglu(x, w_gate, w_up)
     if y is not None:
       return y
   if (use_kernels(x, w_gate, w_up) and _adjacent([w_gate, w_up]) and w_gate.shape[0] % 8 == 0
@@ -498,9 +470,11 @@ class _AddRMSNormFn(torch.autograd.Function):
 
 
 def rms_norm(x, w, eps):
+  if (nat := _native()) is not None:
+    y = nat.rms_norm(x, w, eps)
+    if y is not None:
+      return y
   if use_kernels(x, w) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192:
-    if inference_only() and w.is_contiguous():
-      return _norm_now(x, w, eps)
     return _RMSNormFn.apply(x, w, eps)
   return ref.rms_norm(x, w, eps)
 
@@ -532,9 +506,11 @@ class _RMSNormPassFn(torch.autograd.Function):
 def rms_norm_residual(x, w, eps):
   """Returns (rmsnorm(x) * w, x).  Use the second value wherever ``x`` is needed again (the
   residual connection): its gradient is then added inside the norm's backward kernel."""
+  if (nat := _native()) is not None:
+    both = nat.rms_norm_residual(x, w, eps)
+    if both is not None:
+      return both
   if use_kernels(x, w) and x.shape[-1] % 8 == 0 and x.shape[-1] <= 8192:
-    if inference_only() and w.is_contiguous():
-      return _norm_now(x, w, eps), x.view_as(x)
     return _RMSNormPassFn.apply(x, w, eps)
   return ref.rms_norm(x, w, eps), x
 
@@ -573,22 +549,14 @@ class _RopeInplaceFn(torch.autograd.Function):
     return d, None, None, None, None, None, None, None, None, None
 
 
-def _rope_now(x, cos_half, sin_half, heads, dim, seq_len, pos, interleaved, col0=0, head_stride=None):
-  """The forward of :class:`_RopeInplaceFn` where nothing is recorded."""
-  from . import kernels as k
-  k.rope_(x.view(-1, x.shape[-1]), col0, heads, dim, cos_half, sin_half, seq_len, pos=pos, interleaved=interleaved,
-          head_stride=head_stride)
-  if not x.is_inference():
-    torch.autograd.graph.increment_version(x)    # an earlier graph that saved x has to notice
-  return x
-
-
 def rope_slices(x, cos_half, sin_half, heads, dim, seq_len, col0, head_stride, pos=None, interleaved=False):
   """Rotate ``heads`` slices of width ``dim`` that start at column ``col0`` and lie ``head_stride``
   apart in the last dimension of ``x`` [B,S,C] (the rope part of MLA heads).  In place on CUDA."""
+  if (nat := _native()) is not None and (pos is None or not _debug.bounds_enabled()):
+    y = nat.rope(x, cos_half, sin_half, heads, dim, seq_len, pos, interleaved, col0, head_stride)
+    if y is not None:
+      return y
   if use_kernels(x):
-    if inference_only():
-      return _rope_now(x, cos_half, sin_half, heads, dim, seq_len, pos, interleaved, col0, head_stride)
     return _RopeInplaceFn.apply(x, cos_half, sin_half, heads, dim, seq_len, pos, interleaved, col0, head_stride)
   b, s, c = x.shape
   cols = (col0 + torch.arange(heads, device=x.device)[:, None] * head_stride
@@ -603,9 +571,11 @@ def rope_slices(x, cos_half, sin_half, heads, dim, seq_len, col0, head_stride, p
 def rope_inplace(qkv, cos_half, sin_half, heads, dim, seq_len, pos=None, interleaved=False):
   """Rotate the first ``heads`` heads of a fused ``[B, S, (heads + rest) * dim]`` projection in
   place (q and k heads; v is left alone).  cos/sin: fp32 [max_pos, dim/2]."""
+  if (nat := _native()) is not None and (pos is None or not _debug.bounds_enabled()):
+    y = nat.rope(qkv, cos_half, sin_half, heads, dim, seq_len, pos, interleaved, 0, None)
+    if y is not None:
+      return y
   if use_kernels(qkv):
-    if inference_only():
-      return _rope_now(qkv, cos_half, sin_half, heads, dim, seq_len, pos, interleaved)
     return _RopeInplaceFn.apply(qkv, cos_half, sin_half, heads, dim, seq_len, pos, interleaved)
   b, s, _ = qkv.shape
   head = qkv[..., : heads * dim].reshape(b, s, heads, dim)
@@ -702,10 +672,11 @@ def embedding_peer(ids, table, peer):
 
 
 def embedding(ids, table):
+  if (nat := _native()) is not None:
+    y = nat.embedding(ids, table)
+    if y is not None:
+      return y
   if use_kernels(table) and table.shape[1] % 8 == 0:
-    if inference_only():
-      from . import kernels as k
-      return k.embedding_fwd(table, ids.contiguous())
     return _EmbeddingFn.apply(ids, table)
   return F.embedding(ids, table)
 
@@ -729,6 +700,13 @@ def attention(q, k, v, causal=True, scale=None, window=None, q_segment_ids=None,
               softcap=None, q_positions=None, kv_positions=None):
   """softmax(q k^T * scale + mask) v on ``[B, S, H, D]`` tensors, GQA-native."""
   impl = _STATE["attention"]
+  if impl in ("auto", "sm100") and kv_positions is None and (nat := _native()) is not None:
+    from . import attention_sm100
+    o = nat.attention(q, k, v, causal, scale, window, q_segment_ids, kv_segment_ids, softcap, q_positions,
+                      attention_sm100._MAX_WIDE_QUERIES)
+    if o is not None:
+      _ATTN_USED["last"] = "sm100 tcgen05 kernel"
+      return o
   plain = (window is None and q_segment_ids is None and softcap is None and q_positions is None
            and kv_positions is None)
   if impl in ("auto", "sm100") and q.is_cuda and q.dtype == torch.bfloat16 and _STATE["backend"] != "torch":
@@ -755,6 +733,11 @@ def attention_qkv(qkv, hq, hkv, d, causal=True, scale=None, window=None, q_segme
   """Self-attention on a fused projection output ``qkv`` [B, S, (Hq + 2 Hkv) * d]: same result as
   slicing q, k, v out of it and calling :func:`attention`, but on the kernel path the tensor is a
   single autograd input, so its gradient is produced in one piece."""
+  if _STATE["attention"] in ("auto", "sm100") and (nat := _native()) is not None:
+    o = nat.attention_qkv(qkv, hq, hkv, d, causal, scale, window, q_segment_ids, q_positions)
+    if o is not None:
+      _ATTN_USED["last"] = "sm100 tcgen05 kernel"
+      return o
   b, s, _ = qkv.shape
   if (_STATE["attention"] in ("auto", "sm100") and _STATE["backend"] != "torch" and qkv.is_cuda
       and qkv.dtype == torch.bfloat16 and d == 128 and qkv.is_contiguous()):
@@ -785,6 +768,10 @@ class _LatentSplitFn(torch.autograd.Function):
 
 def latent_split(ckv, c):
   """(ckv[..., :c], ckv[..., c:]); contiguous where kernels run."""
+  if (nat := _native()) is not None:
+    both = nat.latent_split(ckv, c)
+    if both is not None:
+      return both
   if use_kernels(ckv):
     return _LatentSplitFn.apply(ckv, c)
   return ckv[..., :c].contiguous(), ckv[..., c:]
@@ -808,6 +795,10 @@ class _MlaPackFn(torch.autograd.Function):
 def mla_pack(kv, rot, heads, dn, dv):
   """Keys [B,S,heads,dn+dr] and values [B,S,heads,dv] from the up-projection ``kv`` [B,S,heads*(dn+dv)] and the
   rotary key ``rot`` [B,S,dr] that all heads share."""
+  if (nat := _native()) is not None:
+    both = nat.mla_pack(kv, rot, heads, dn, dv)
+    if both is not None:
+      return both
   b, s, dr = rot.shape
   if (use_kernels(kv, rot) and dn % 8 == 0 and dr % 8 == 0 and dv % 8 == 0 and dr <= 512 and kv.is_contiguous()
       and rot.is_contiguous() and kv.data_ptr() % 16 == 0 and rot.data_ptr() % 16 == 0):

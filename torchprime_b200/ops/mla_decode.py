@@ -55,3 +55,15 @@ def absorb_step(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads
                             stream_ptr())
   check(rc, f"mla_decode B={b} H={heads} pos={pos}")
   return out
+
+
+def decode_attention(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads, dn, dr, dv, c, scale, interleaved):
+  """:func:`absorb_step`, or None where it does not support the call."""
+  from .functional import _native
+  if (nat := _native()) is not None and dr == 64:
+    o = nat.absorb_step(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads, dn, dv, scale, interleaved)
+    if o is not None:
+      return o
+  if not supported(q, ckv, norm_w, kv_cache, pe_cache, w, heads, dn, dr, dv, c):
+    return None
+  return absorb_step(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads, dn, dv, scale, interleaved)

@@ -108,12 +108,14 @@ def router_topk(logits, k, mode="softmax", bias=None, n_group=1, topk_group=1, n
 
   ``mode="softmax"``: Mixtral (softmax, top-k, renormalise).  ``mode="sigmoid"``: DeepSeek-V3
   (sigmoid, optional selection bias, group-limited top-k, normalise, scale)."""
+  from .functional import _native
   m = 0 if mode == "softmax" else 1
+  if (nat := _native()) is not None:
+    r = nat.router_topk(logits, bias, k, m, n_group, topk_group, norm_topk, scale)
+    if r is not None:
+      return r
   e = logits.shape[-1]
   if logits.is_cuda and _kernels_ok() and e <= 256 and logits.dtype in (torch.float32, torch.bfloat16):
-    from .functional import inference_only
-    if inference_only():
-      return _router_forward(logits.contiguous(), bias, k, m, n_group, topk_group, norm_topk, scale)
     return _RouterFn.apply(logits, bias, k, m, n_group, topk_group, norm_topk, scale)
   if m == 0:
     w, idx, s = ref.router_softmax_topk(logits, k, renormalize=norm_topk)
@@ -430,13 +432,17 @@ def grouped_mlp(x, weights, idx, w_gate, w_up, w_down, *, fused_gate_up=False, c
   differently; a forward that a backward pass will repeat says so with ``functional.recomputed_forward`` and does not."""
   e = w_gate.shape[0]
   f = w_down.shape[1]
-  from .functional import in_recomputed_forward, inference_only
+  from .functional import _native, in_recomputed_forward, inference_only
   ok = (_kernels_ok(x, w_gate, w_down) and x.shape[-1] % 64 == 0 and f % 64 == 0 and x.is_cuda)
   if ok:
     if (capacity is None and e <= 256 and inference_only() and not in_recomputed_forward()
         and all(w.is_contiguous() and w.data_ptr() % 16 == 0 for w in (w_gate, w_up, w_down) if w is not None)):
       align = few_rows_align(*idx.shape, e)
       if align is not None:
+        if (nat := _native()) is not None and not _debug.bounds_enabled():
+          y = nat.grouped_mlp_few_rows(x, weights, idx, w_gate, w_up, w_down, fused_gate_up, align)
+          if y is not None:
+            return y
         return grouped_mlp_few_rows(x.contiguous(), weights.float().contiguous(), idx, w_gate, w_up, w_down,
                                     fused_gate_up, align)
     plan = build_dispatch_plan(idx, e, capacity, rows_per_group)
