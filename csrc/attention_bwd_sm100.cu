@@ -117,6 +117,7 @@ __global__ void __launch_bounds__(DELTA_THREADS)
 attn_bwd_delta_kernel(const __nv_bfloat16* __restrict__ dO, const __nv_bfloat16* __restrict__ O,
                       const float* __restrict__ lse, float* __restrict__ lse2, float* __restrict__ delta, int Sq,
                       int Sq_pad, int Hq) {
+  if (!chain_begin()) return;
   constexpr int ROWS = DELTA_T * DELTA_H / (DELTA_THREADS / 16);   // rows per group of sixteen lanes
   __shared__ float sums[DELTA_H][DELTA_T];
   const int q_tiles = Sq_pad / DELTA_T, h_tiles = (Hq + DELTA_H - 1) / DELTA_H;
@@ -254,6 +255,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  chain_wait();
   // position range of every query tile (decides which tiles this key block can see)
   const int2 kseg_rng = SEG ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
   for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
@@ -278,6 +280,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_launch();
 
   auto visible = [&](int t) -> bool {
     if (SEG && tile_min[t] > tile_max[t]) return false;
@@ -640,6 +643,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // No wait for the kernel before: that is dK/dV, which lets this one start only after it has waited for the deltas, and
+  // nothing of it is read here.  Its last CTAs and the first ones here share the chip; the wait comes at the end, so that
+  // this kernel does not end before it.
+  chain_launch();
 
   if (threadIdx.x < BWD_T) {
     const int r = q0 + threadIdx.x;
@@ -857,6 +864,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                   p.scale);
   }
 
+  chain_wait();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -1009,6 +1017,7 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
+  if (FINE) chain_wait();   // the deltas of the dQ kernel; otherwise as in attn_bwd_dq_kernel: the wait comes at the end
   // position range of every query tile; a tile that shares no segment with this key block gets an empty one
   const int2 kseg_rng = p.kv_rng ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
   for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
@@ -1033,6 +1042,7 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_launch();
 
   auto visible = [&](int t) -> bool {
     if (tile_min[t] > tile_max[t]) return false;
@@ -1271,6 +1281,7 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                    key_ok, 1.f);
   }
 
+  if (!FINE) chain_wait();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -1333,6 +1344,8 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_wait();
+  chain_launch();   // (after the wait: the dK/dV kernel relies on the deltas being there)
 
   if (threadIdx.x < BWD_T) {
     const int r = q0 + threadIdx.x;
@@ -1574,8 +1587,8 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
   {
     const long long blocks = (long long)B * ((Hq + DELTA_H - 1) / DELTA_H) * (sq_pad / DELTA_T);
     if (blocks > 0x7fffffff) return -2;
-    attn_bwd_delta_kernel<<<(int)blocks, DELTA_THREADS, 0, stream>>>(
-        reinterpret_cast<const __nv_bfloat16*>(dO), reinterpret_cast<const __nv_bfloat16*>(o), lse, lse2, delta, Sq, sq_pad, Hq);
+    chain(attn_bwd_delta_kernel, (int)blocks, DELTA_THREADS, 0, stream,
+          reinterpret_cast<const __nv_bfloat16*>(dO), reinterpret_cast<const __nv_bfloat16*>(o), lse, lse2, delta, Sq, sq_pad, Hq);
   }
   AttnBwdParams p;
   p.B = B; p.Sq = Sq; p.Sk = Sk; p.Hq = Hq; p.Hkv = Hkv;
@@ -1623,22 +1636,24 @@ extern "C" int tpb_attn_bwd_softcap(const void* dO, const void* q, const void* k
     const bool fine = q_pos || q_seg || kv_seg || window > 0 || (causal && Sq != Sk);
     const int grid_wq = ((Sq + BWD_T - 1) / BWD_T) * Hq * B;
     // (FINE: dK/dV takes the deltas that the dQ kernel leaves)
-    (fine ? attn_bwd_dq192_kernel<true> : attn_bwd_dq192_kernel<false>)<<<grid_wq, BWD_THREADS, wdq::TOTAL, stream>>>(tq, tk, tv, tdo, p);
+    chain(fine ? attn_bwd_dq192_kernel<true> : attn_bwd_dq192_kernel<false>, grid_wq, BWD_THREADS, wdq::TOTAL, stream,
+          tq, tk, tv, tdo, p);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return 1000 + (int)e;
-    (fine ? attn_bwd_dkv192_kernel<true> : attn_bwd_dkv192_kernel<false>)<<<grid_kv, BWD_THREADS, wkv::TOTAL, stream>>>(tq64, tk, tv, tdo64, p);
+    chain(fine ? attn_bwd_dkv192_kernel<true> : attn_bwd_dkv192_kernel<false>, grid_kv, BWD_THREADS, wkv::TOTAL, stream,
+          tq64, tk, tv, tdo64, p);
     e = cudaGetLastError();
     return e == cudaSuccess ? 0 : 1000 + (int)e;
   }
-  (softcap > 0.f ? (ranges ? attn_bwd_dkv_kernel<true, true> : attn_bwd_dkv_kernel<true, false>)
-                 : (ranges ? attn_bwd_dkv_kernel<false, true> : attn_bwd_dkv_kernel<false, false>))
-      <<<grid_kv, BWD_THREADS, dkv::TOTAL, stream>>>(tq, tk, tv, tdo, p);
+  chain(softcap > 0.f ? (ranges ? attn_bwd_dkv_kernel<true, true> : attn_bwd_dkv_kernel<true, false>)
+                      : (ranges ? attn_bwd_dkv_kernel<false, true> : attn_bwd_dkv_kernel<false, false>),
+        grid_kv, BWD_THREADS, dkv::TOTAL, stream, tq, tk, tv, tdo, p);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return 1000 + (int)e;
   dim3 grid_q(((Sq + BWD_T - 1) / BWD_T) * Hq * B, 1, 1);
-  (softcap > 0.f ? (ranges ? attn_bwd_dq_kernel<true, true> : attn_bwd_dq_kernel<true, false>)
-                 : (ranges ? attn_bwd_dq_kernel<false, true> : attn_bwd_dq_kernel<false, false>))
-      <<<grid_q, BWD_THREADS, dqk::TOTAL, stream>>>(tq, tk, tv, tdo, p);
+  chain(softcap > 0.f ? (ranges ? attn_bwd_dq_kernel<true, true> : attn_bwd_dq_kernel<true, false>)
+                      : (ranges ? attn_bwd_dq_kernel<false, true> : attn_bwd_dq_kernel<false, false>),
+        grid_q, BWD_THREADS, dqk::TOTAL, stream, tq, tk, tv, tdo, p);
   e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }

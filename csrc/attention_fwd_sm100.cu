@@ -221,6 +221,7 @@ __device__ __forceinline__ bool cp_wait_keys(const AttnFwdParams& p, int b, int 
 // Two rows of 1999 tokens in seven segments each, 32/8 heads, forward and backward: 1003 -> 415 us (forward 624 -> 188).
 __global__ void attn_seg_ranges_kernel(const int* __restrict__ seg, int2* __restrict__ out, int S, int nblk,
                                        int total) {
+  if (!chain_begin()) return;
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (w >= total) return;
   const int b = w / nblk, s0 = (w % nblk) * SEG_BLK;
@@ -306,6 +307,8 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_launch();
+  chain_wait();
 
   // Range of positions covered by this tile's query rows.
   if (threadIdx.x < FWD_BM) {
@@ -1029,7 +1032,7 @@ cudaError_t launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     configured = true;
   }
   dim3 grid((p.Sq + FWD_BM - 1) / FWD_BM, p.Hq, p.B);
-  attn_fwd_kernel<DQK, SEG><<<grid, FWD_THREADS, FwdSmem<DQK>::TOTAL, stream>>>(tq, tk, tv, p);
+  chain(attn_fwd_kernel<DQK, SEG>, grid, FWD_THREADS, FwdSmem<DQK>::TOTAL, stream, tq, tk, tv, p);
   return cudaGetLastError();
 }
 
@@ -1123,8 +1126,8 @@ extern "C" int tpb_attn_seg_ranges(const int* seg, int* out, int B, int S, void*
   const int nblk = (S + SEG_BLK - 1) / SEG_BLK;
   const long long total = (long long)B * nblk;
   if (total > (1LL << 26)) return -2;
-  attn_seg_ranges_kernel<<<(int)((total + 7) / 8), 256, 0, reinterpret_cast<cudaStream_t>(stream_)>>>(
-      seg, reinterpret_cast<int2*>(out), S, nblk, (int)total);
+  chain(attn_seg_ranges_kernel, (int)((total + 7) / 8), 256, 0, reinterpret_cast<cudaStream_t>(stream_),
+        seg, reinterpret_cast<int2*>(out), S, nblk, (int)total);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }

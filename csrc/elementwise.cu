@@ -64,6 +64,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, const uint4* __restrict__ w,
                    uint4* __restrict__ y, uint4* __restrict__ h_out, float* __restrict__ rstd_out, int rows,
                    int nvec, float eps) {
+  if (!chain_begin()) return;
   __shared__ float red[32];
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const uint4* xr = x + (size_t)row * nvec;
@@ -107,6 +108,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x, const uint4* __restrict__ w,
                    const float* __restrict__ rstd, const uint4* __restrict__ dres, uint4* __restrict__ dx,
                    float* __restrict__ dw, int rows, int nvec) {
+  if (!chain_begin()) return;
   __shared__ float red[32];
   float dw_acc[VPT][8];
   float wv[VPT][8];
@@ -189,6 +191,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_bulk_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, const uint4* __restrict__ w,
                         uint4* __restrict__ y, uint4* __restrict__ h_out, float* __restrict__ rstd_out, int rows,
                         int nvec, float eps, int stages, int* status) {
+  if (!chain_begin()) return;
   extern __shared__ uint8_t nf_smem_raw[];
   uint8_t* smem = nf_smem_raw + ((128u - (smem_u32(nf_smem_raw) & 127u)) & 127u);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);   // [NB_MAX_STAGES]
@@ -288,6 +291,7 @@ __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_bwd_bulk_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x, const uint4* __restrict__ w,
                         const float* __restrict__ rstd, const uint4* __restrict__ dres, uint4* __restrict__ dx,
                         float* __restrict__ dw, int rows, int nvec, int stages, int* status) {
+  if (!chain_begin()) return;
   extern __shared__ uint8_t nb_smem_raw[];
   uint8_t* smem = nb_smem_raw + ((128u - (smem_u32(nb_smem_raw) & 127u)) & 127u);
   uint64_t* full = reinterpret_cast<uint64_t*>(smem);   // [NB_MAX_STAGES]
@@ -410,6 +414,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, int col
                             const float* __restrict__ cosT, const float* __restrict__ sinT,
                             const int* __restrict__ pos, long long tokens, int seq_len, float sign,
                             int interleaved) {
+  if (!chain_begin()) return;
   const int half = dim / 2;
   const int vec_per_head = half / 8;
   const long long total = tokens * heads * vec_per_head;
@@ -469,6 +474,7 @@ __global__ void rope_kernel(__nv_bfloat16* __restrict__ x, long long ld, int col
 // SwiGLU
 // ----------------------------------------------------------------------------
 __global__ void swiglu_fwd_kernel(const uint4* __restrict__ gu, uint4* __restrict__ act, long long rows, int fvec) {
+  if (!chain_begin()) return;
   const long long total = rows * fvec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -484,6 +490,7 @@ __global__ void swiglu_fwd_kernel(const uint4* __restrict__ gu, uint4* __restric
 }
 __global__ void swiglu_bwd_kernel(const uint4* __restrict__ dact, const uint4* __restrict__ gu,
                                   uint4* __restrict__ dgu, long long rows, int fvec) {
+  if (!chain_begin()) return;
   const long long total = rows * fvec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -517,6 +524,7 @@ constexpr int CE_UNROLL = 4;
 __global__ void __launch_bounds__(CE_THREADS, 2)
 ce_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long* __restrict__ targets,
           float* __restrict__ loss_sum, const float* __restrict__ grad_scale, int rows, int vocab) {
+  if (!chain_begin()) return;
   __shared__ float red[32];
   const int nvec = vocab / 8;  // host guarantees vocab % 8 == 0
   const float log2e = 1.4426950408889634f;
@@ -612,6 +620,7 @@ ce_kernel(__nv_bfloat16* __restrict__ logits, long long ld, const long long* __r
 __global__ void embedding_fwd_kernel(const uint4* __restrict__ table, const long long* __restrict__ ids,
                                      uint4* __restrict__ out, long long tokens, int nvec, long long vocab,
                                      long long row0) {
+  if (!chain_begin()) return;
   const long long total = tokens * nvec;
   for (long long idx = blockIdx.x * (long long)blockDim.x + threadIdx.x; idx < total;
        idx += (long long)gridDim.x * blockDim.x) {
@@ -724,6 +733,7 @@ __global__ void clip_coef_kernel(const float* sumsq, float max_norm, float* coef
 
 __global__ void cast_kernel(const float4* __restrict__ src, uint2* __restrict__ dst, long long n4, float scale,
                             int accumulate) {
+  if (!chain_begin()) return;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n4;
        i += (long long)gridDim.x * blockDim.x) {
     float4 s = src[i];
@@ -742,6 +752,7 @@ __global__ void cast_kernel(const float4* __restrict__ src, uint2* __restrict__ 
 // 128,256 x 4096 values: 0.51 ms (6.1 TB/s) where a multiplication and a cast took 1.86 ms.
 __global__ void scale_cast_kernel(const float4* __restrict__ src, uint4* __restrict__ dst, long long n8,
                                   const float* __restrict__ scale) {
+  if (!chain_begin()) return;
   const float sc = *scale;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < n8;
        i += (long long)gridDim.x * blockDim.x) {
@@ -766,7 +777,7 @@ static void launch_rmsnorm_bwd(const void* dy, const void* x, const void* w, con
   const int vpt = (nvec + NORM_THREADS - 1) / NORM_THREADS;
   const int per_sm = vpt <= 2 ? 4 : 2;
   const int grid = rows < sm_count() * per_sm ? rows : sm_count() * per_sm;
-#define TPB_LAUNCH_NORM_BWD(V) rmsnorm_bwd_kernel<V><<<grid, NORM_THREADS, 0, stream>>>( \
+#define TPB_LAUNCH_NORM_BWD(V) chain(rmsnorm_bwd_kernel<V>, grid, NORM_THREADS, 0, stream, \
       (const uint4*)dy, (const uint4*)x, (const uint4*)w, rstd, (const uint4*)dres, (uint4*)dx, dw_f32, rows, nvec)
   if (vpt <= 1) TPB_LAUNCH_NORM_BWD(1); else if (vpt == 2) TPB_LAUNCH_NORM_BWD(2); else TPB_LAUNCH_NORM_BWD(4);
 #undef TPB_LAUNCH_NORM_BWD
@@ -807,7 +818,7 @@ static bool launch_rmsnorm_fwd_bulk(const void* x, const void* res, const void* 
         return false;                                                                                                 \
       configured[slot] = true;                                                                                        \
     }                                                                                                                 \
-    rmsnorm_fwd_bulk_kernel<V><<<grid, NORM_THREADS, smem, stream>>>((const uint4*)x, (const uint4*)res,             \
+    chain(rmsnorm_fwd_bulk_kernel<V>, grid, NORM_THREADS, smem, stream, (const uint4*)x, (const uint4*)res,             \
                                                                      (const uint4*)w, (uint4*)y, (uint4*)h_out, rstd, \
                                                                      rows, nvec, eps, stages, status_block());        \
   } while (0)
@@ -825,7 +836,7 @@ extern "C" int tpb_rmsnorm_fwd(const void* x, const void* res, const void* w, vo
   const int vpt = (nvec + NORM_THREADS - 1) / NORM_THREADS;
   const int per_sm = vpt <= 2 ? 8 : 4;
   const int grid = rows < sm_count() * per_sm ? rows : sm_count() * per_sm;
-#define TPB_LAUNCH_NORM_FWD(V) rmsnorm_fwd_kernel<V><<<grid, NORM_THREADS, 0, STREAM(stream)>>>( \
+#define TPB_LAUNCH_NORM_FWD(V) chain(rmsnorm_fwd_kernel<V>, grid, NORM_THREADS, 0, STREAM(stream), \
       (const uint4*)x, (const uint4*)res, (const uint4*)w, (uint4*)y, (uint4*)h_out, rstd, rows, nvec, eps)
   if (vpt <= 1) TPB_LAUNCH_NORM_FWD(1); else if (vpt == 2) TPB_LAUNCH_NORM_FWD(2); else TPB_LAUNCH_NORM_FWD(4);
 #undef TPB_LAUNCH_NORM_FWD
@@ -859,7 +870,7 @@ static bool launch_rmsnorm_bwd_bulk(const void* dy, const void* x, const void* w
         return false;                                                                                                  \
       configured[slot] = true;                                                                                         \
     }                                                                                                                  \
-    rmsnorm_bwd_bulk_kernel<V><<<grid, NORM_THREADS, smem, stream>>>((const uint4*)dy, (const uint4*)x, (const uint4*)w, \
+    chain(rmsnorm_bwd_bulk_kernel<V>, grid, NORM_THREADS, smem, stream, (const uint4*)dy, (const uint4*)x, (const uint4*)w, \
                                                                      rstd, (const uint4*)dres, (uint4*)dx, dw_f32,  \
                                                                      rows, nvec, stages, status_block());              \
   } while (0)
@@ -883,7 +894,7 @@ extern "C" int tpb_rope_strided(void* x, long long ld, int col0, int heads, int 
   if (dim % 16 || ld % 8 || col0 % 8 || head_stride % 8 || head_stride < dim) return -2;
   if (tokens <= 0 || heads <= 0) return 0;
   long long total = (long long)tokens * heads * (dim / 16);
-  rope_kernel<<<grid_for(total, 256), 256, 0, STREAM(stream)>>>((__nv_bfloat16*)x, ld, col0, heads, dim, head_stride,
+  chain(rope_kernel, grid_for(total, 256), 256, 0, STREAM(stream), (__nv_bfloat16*)x, ld, col0, heads, dim, head_stride,
                                                                 cos, sin, pos, tokens, seq_len,
                                                                 inverse ? -1.f : 1.f, interleaved);
   return rc(cudaGetLastError());
@@ -897,15 +908,15 @@ extern "C" int tpb_rope(void* x, long long ld, int col0, int heads, int dim, con
 extern "C" int tpb_swiglu_fwd(const void* gu, void* act, int rows, int f, void* stream) {
   if (f % 8) return -2;
   if (rows <= 0) return 0;
-  swiglu_fwd_kernel<<<grid_for((long long)rows * (f / 8), 256), 256, 0, STREAM(stream)>>>((const uint4*)gu,
+  chain(swiglu_fwd_kernel, grid_for((long long)rows * (f / 8), 256), 256, 0, STREAM(stream), (const uint4*)gu,
                                                                                          (uint4*)act, rows, f / 8);
   return rc(cudaGetLastError());
 }
 extern "C" int tpb_swiglu_bwd(const void* dact, const void* gu, void* dgu, int rows, int f, void* stream) {
   if (f % 8) return -2;
   if (rows <= 0) return 0;
-  swiglu_bwd_kernel<<<grid_for((long long)rows * (f / 8), 256), 256, 0, STREAM(stream)>>>(
-      (const uint4*)dact, (const uint4*)gu, (uint4*)dgu, rows, f / 8);
+  chain(swiglu_bwd_kernel, grid_for((long long)rows * (f / 8), 256), 256, 0, STREAM(stream),
+        (const uint4*)dact, (const uint4*)gu, (uint4*)dgu, rows, f / 8);
   return rc(cudaGetLastError());
 }
 
@@ -914,7 +925,7 @@ extern "C" int tpb_ce_fwd_bwd(void* logits, long long ld, const long long* targe
   if (vocab % 8 || ld % 8) return -2;
   if (rows <= 0) return 0;
   const int grid = rows < sm_count() * 2 ? rows : sm_count() * 2;
-  ce_kernel<<<grid, CE_THREADS, 0, STREAM(stream)>>>((__nv_bfloat16*)logits, ld, targets, loss_sum, grad_scale, rows,
+  chain(ce_kernel, grid, CE_THREADS, 0, STREAM(stream), (__nv_bfloat16*)logits, ld, targets, loss_sum, grad_scale, rows,
                                                      vocab);
   return rc(cudaGetLastError());
 }
@@ -954,8 +965,8 @@ extern "C" int tpb_embedding_fwd(const void* table, const long long* ids, void* 
                                  long long vocab, long long row0, void* stream) {
   if (dim % 8) return -2;
   if (tokens <= 0) return 0;
-  embedding_fwd_kernel<<<grid_for((long long)tokens * (dim / 8), 256), 256, 0, STREAM(stream)>>>(
-      (const uint4*)table, ids, (uint4*)out, tokens, dim / 8, vocab, row0);
+  chain(embedding_fwd_kernel, grid_for((long long)tokens * (dim / 8), 256), 256, 0, STREAM(stream),
+        (const uint4*)table, ids, (uint4*)out, tokens, dim / 8, vocab, row0);
   return rc(cudaGetLastError());
 }
 extern "C" int tpb_embedding_bwd(const void* dout, const long long* ids, void* dtable, int tokens, int dim,
@@ -976,7 +987,7 @@ extern "C" int tpb_cast_f32_to_bf16(const float* src, void* dst, long long n, fl
                                     void* stream) {
   if (n % 4) return -2;
   if (n <= 0) return 0;
-  cast_kernel<<<grid_for(n / 4, 256), 256, 0, STREAM(stream)>>>((const float4*)src, (uint2*)dst, n / 4, scale,
+  chain(cast_kernel, grid_for(n / 4, 256), 256, 0, STREAM(stream), (const float4*)src, (uint2*)dst, n / 4, scale,
                                                                 accumulate);
   return rc(cudaGetLastError());
 }
@@ -985,7 +996,7 @@ extern "C" int tpb_cast_f32_to_bf16(const float* src, void* dst, long long n, fl
 extern "C" int tpb_scale_cast_bf16(const float* src, void* dst, long long n, const float* scale, void* stream) {
   if ((n % 8) || (reinterpret_cast<uintptr_t>(src) % 16) || (reinterpret_cast<uintptr_t>(dst) % 16)) return -2;
   if (n <= 0) return 0;
-  scale_cast_kernel<<<grid_for(n / 8, 256, 16), 256, 0, STREAM(stream)>>>((const float4*)src, (uint4*)dst, n / 8, scale);
+  chain(scale_cast_kernel, grid_for(n / 8, 256, 16), 256, 0, STREAM(stream), (const float4*)src, (uint4*)dst, n / 8, scale);
   return rc(cudaGetLastError());
 }
 

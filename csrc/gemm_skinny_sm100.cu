@@ -46,6 +46,7 @@ constexpr int SK_TN = 128;                       // output features per tile
 constexpr int SK_BK = 64;
 constexpr int SK_W_BYTES = SK_TN * SK_BK * 2;    // 16 KB
 constexpr int SK_MAX_SPLIT = 8;                  // portable cluster size
+constexpr int SK_PREFETCH = 8;                   // k-blocks asked for ahead of the kernel before: 128 KB a CTA, 38 MB in all
 
 template <int NT>
 struct SkinnySmem {
@@ -140,6 +141,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const int n0 = nt * (swiglu ? SK_TN / 2 : SK_TN);
   int ez = 0;
   if (p.tile_expert) {
+    chain_wait();
     ez = p.tile_expert[bt];
     if (ez < 0) return;      // the whole cluster leaves together
   }
@@ -168,6 +170,15 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       mbar_init(&blk_empty[i], 4);
     }
     fence_barrier_init();
+    if (!p.tile_expert) {
+      // The weights do not come from the kernel before: their first tiles move to L2 while it still runs.
+      const int nb = swiglu ? p.up_off + n0 : n0 + 64;
+      for (int kb = kb0; kb < min(kb1, kb0 + SK_PREFETCH); ++kb) {
+        const int k0 = kb * SK_BK;
+        tma_prefetch_3d(&tmW, W_MN ? n0 : k0, W_MN ? k0 : n0, 0);
+        tma_prefetch_3d(&tmW2, W_MN ? nb : k0, W_MN ? k0 : nb, 0);
+      }
+    }
   }
   if (warp == 1) {
     tmem_alloc(tmem_slot, TMEM_COLS);
@@ -177,6 +188,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_launch();
+  chain_wait();
 
   if (warp == 0) {
     if (lane == 0) {
@@ -317,7 +330,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   cluster_sync_all();           // every CTA's partial tile is in its shared memory
 
   {
-    const float alpha = p.alpha_dev ? p.alpha * __ldg(p.alpha_dev) : p.alpha;
+    const float alpha = p.alpha_dev ? p.alpha * *p.alpha_dev : p.alpha;
     const int per = NT / p.splits;                    // tokens this CTA finishes (splits divides 16)
     const int gpt = swiglu ? SK_TN / 8 : SK_TN / 4;   // groups of four features per token
     for (int i = threadIdx.x; i < per * gpt; i += SK_THREADS) {
@@ -380,19 +393,8 @@ static cudaError_t launch_skinny(const CUtensorMap& tw, const CUtensorMap& tw2, 
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid, 1, 1);
-  cfg.blockDim = dim3(SK_THREADS, 1, 1);
-  cfg.dynamicSmemBytes = SkinnySmem<NT>::TOTAL;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = p.splits;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_skinny_kernel<NT, W_MN, X_MN, F32>, tw, tw2, tx, p);
+  return chain_clusters(gemm_skinny_kernel<NT, W_MN, X_MN, F32>, p.splits, grid, SK_THREADS, SkinnySmem<NT>::TOTAL, stream, tw, tw2,
+                        tx, p);
 }
 
 // Token-tile width for `rows` rows: the smallest one that holds them, 128 at most.

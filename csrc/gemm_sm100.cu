@@ -398,6 +398,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (PAIR) cluster_sync_all();   // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_launch();
+  chain_wait();
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
@@ -555,7 +557,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   } else {
     // ---------------------------------------------------------------- epilogue
     const int q = warp & 3;  // TMEM lane quarter this warp may access
-    const float alpha = p.alpha_dev ? p.alpha * __ldg(p.alpha_dev) : p.alpha;
+    const float alpha = p.alpha_dev ? p.alpha * *p.alpha_dev : p.alpha;
     uint4* slabs = epi_stage + q * 512;
     int buf = 0;
     int local = 0;
@@ -841,6 +843,9 @@ int make_tmap_out(CUtensorMap* map, const void* ptr, uint64_t cols, uint64_t row
                   uint64_t plane_elems, int elem_bytes);
 int sm_count();  // runtime.cu
 
+// Kernels that exchange data with other GPUs are launched the ordinary way.
+static bool chainable(const GemmParams& p) { return p.ag_world == 0 && p.rs_world == 0 && p.epi != TPB_EPI_AR_BF16; }
+
 template <bool A_MN, bool B_MN>
 cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tb2, const CUtensorMap& tc,
                         const CUtensorMap& tc2, const GemmParams& p, int grid, cudaStream_t stream) {
@@ -851,6 +856,7 @@ cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
     if (e != cudaSuccess) return e;
     configured = true;
   }
+  if (chainable(p)) return chain(gemm_kernel<A_MN, B_MN, false>, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb2, tc, tc2, p);
   gemm_kernel<A_MN, B_MN, false><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, tb2, tc, tc2, p);
   return cudaGetLastError();
 }
@@ -866,6 +872,8 @@ cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const
     if (e != cudaSuccess) return e;
     configured = true;
   }
+  if (chainable(p))
+    return chain_clusters(gemm_kernel<A_MN, B_MN, true>, 2, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb2, tc, tc2, p);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3(GEMM_THREADS, 1, 1);

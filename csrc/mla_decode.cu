@@ -48,6 +48,7 @@ mla_prep_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__
                 const float* __restrict__ sinT, __nv_bfloat16* __restrict__ kv_cache,
                 __nv_bfloat16* __restrict__ pe_cache, long long kv_bs, long long pe_bs, int pos, int H, int dn, int C,
                 float eps, int interleaved) {
+  if (!chain_begin()) return;
   __shared__ float red[8];
   const int b = blockIdx.x;
   const float* cs = cosT + (size_t)pos * (MLA_R / 2);
@@ -86,6 +87,7 @@ mla_prep_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__
 __global__ void __launch_bounds__(MLA_THREADS)
 mla_fold_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ w, float* __restrict__ qa, int B,
                 int H, int dn, int dv, int C) {
+  if (!chain_begin()) return;
   __shared__ float acc_s[8][MLA_MAX_B][64];
   extern __shared__ float fold_q[];                  // [MLA_MAX_B][dn]
   const int h = blockIdx.x, c0 = blockIdx.y * 64, b0 = blockIdx.z * MLA_MAX_B;
@@ -153,6 +155,7 @@ mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__
                  const __nv_bfloat16* __restrict__ kv_cache, const __nv_bfloat16* __restrict__ pe_cache,
                  long long kv_bs, long long pe_bs, float* __restrict__ part_o, float* __restrict__ part_ml, int n_keys,
                  int per, int H, int dn, int C, float scale_log2) {
+  if (!chain_begin()) return;
   extern __shared__ uint8_t split_smem[];
   const int D = C + MLA_R, pitch = MlaSplitSmem::key_pitch(C);
   float* sq = reinterpret_cast<float*>(split_smem);                 // [16][D]
@@ -279,6 +282,7 @@ mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__
 __global__ void __launch_bounds__(MLA_THREADS)
 mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const __nv_bfloat16* __restrict__ w,
                  __nv_bfloat16* __restrict__ out, int ranges, int H, int dn, int dv, int C, int rows) {
+  if (!chain_begin()) return;
   __shared__ __align__(16) float olat[MLA_MAX_C];
   extern __shared__ float merge_w[];             // [ranges]
   const int h = blockIdx.x, b = blockIdx.y;
@@ -380,11 +384,11 @@ extern "C" int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, cons
   auto* kc = reinterpret_cast<__nv_bfloat16*>(kv_cache);
   auto* pc = reinterpret_cast<__nv_bfloat16*>(pe_cache);
   const auto* wb = reinterpret_cast<const __nv_bfloat16*>(w);
-  mla_prep_kernel<<<B, MLA_THREADS, 0, stream>>>(qb, reinterpret_cast<const __nv_bfloat16*>(ckv),
+  chain(mla_prep_kernel, B, MLA_THREADS, 0, stream, qb, reinterpret_cast<const __nv_bfloat16*>(ckv),
                                                  reinterpret_cast<const __nv_bfloat16*>(norm_w), cosT, sinT, kc, pc,
                                                  kv_bs, pe_bs, pos, H, dn, C, eps, interleaved);
-  mla_fold_kernel<<<dim3(H, C / 64, (B + MLA_MAX_B - 1) / MLA_MAX_B), MLA_THREADS, MLA_MAX_B * dn * 4, stream>>>(
-      qb, wb, qa, B, H, dn, dv, C);
+  chain(mla_fold_kernel, dim3(H, C / 64, (B + MLA_MAX_B - 1) / MLA_MAX_B), MLA_THREADS, MLA_MAX_B * dn * 4, stream,
+        qb, wb, qa, B, H, dn, dv, C);
   const int steps = (n_keys + MLA_KEYS - 1) / MLA_KEYS;
   const int per = (steps + ranges - 1) / ranges * MLA_KEYS;
   static bool configured = false;
@@ -394,11 +398,11 @@ extern "C" int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, cons
     if (e != cudaSuccess) return 1000 + (int)e;
     configured = true;
   }
-  mla_split_kernel<<<dim3(ranges, (H + MLA_HG - 1) / MLA_HG, B), MLA_THREADS, MlaSplitSmem::bytes(C), stream>>>(
-      qa, qb, kc, pc, kv_bs, pe_bs, part_o, part_ml, n_keys, per, H, dn, C, scale * 1.4426950408889634f);
+  chain(mla_split_kernel, dim3(ranges, (H + MLA_HG - 1) / MLA_HG, B), MLA_THREADS, MlaSplitSmem::bytes(C), stream,
+        qa, qb, kc, pc, kv_bs, pe_bs, part_o, part_ml, n_keys, per, H, dn, C, scale * 1.4426950408889634f);
   const int rows = 32;     // one pass of the eight warps
-  mla_merge_kernel<<<dim3(H, B, (dv + rows - 1) / rows), MLA_THREADS, ranges * 4, stream>>>(
-      part_o, part_ml, wb, reinterpret_cast<__nv_bfloat16*>(out), ranges, H, dn, dv, C, rows);
+  chain(mla_merge_kernel, dim3(H, B, (dv + rows - 1) / rows), MLA_THREADS, ranges * 4, stream,
+        part_o, part_ml, wb, reinterpret_cast<__nv_bfloat16*>(out), ranges, H, dn, dv, C, rows);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }

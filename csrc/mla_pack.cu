@@ -18,6 +18,7 @@ int sm_count();
 __global__ void mla_pack_kernel(const uint4* __restrict__ kv, const uint4* __restrict__ rot, long long rot_ld,
                                 uint4* __restrict__ k, uint4* __restrict__ v, long long heads_total, int H, int dn8,
                                 int dr8, int dv8) {
+  if (!chain_begin()) return;
   const int per = dn8 + dr8 + dv8;
   const long long total = heads_total * per;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
@@ -37,6 +38,7 @@ constexpr int UNPACK_THREADS = 256;
 __global__ void __launch_bounds__(UNPACK_THREADS)
 mla_unpack_kernel(const uint4* __restrict__ dk, const uint4* __restrict__ dv, uint4* __restrict__ dkv,
                   uint4* __restrict__ drot, long long tokens, int H, int dn8, int dr8, int dv8) {
+  if (!chain_begin()) return;
   extern __shared__ float unpack_s[];            // [G][dr]
   const int G = UNPACK_THREADS / dr8, dr = dr8 * 8;
   for (long long t = blockIdx.x; t < tokens; t += gridDim.x) {
@@ -89,8 +91,8 @@ extern "C" int tpb_mla_pack(const void* kv, const void* rot, long long rot_ld, v
   if (tokens <= 0) return 0;
   const long long items = tokens * H * ((dn + dr + dv) / 8);
   long long blocks = (items + 255) / 256, cap = (long long)sm_count() * 16;
-  mla_pack_kernel<<<(int)(blocks < cap ? blocks : cap), 256, 0, reinterpret_cast<cudaStream_t>(stream)>>>(
-      (const uint4*)kv, (const uint4*)rot, rot_ld / 8, (uint4*)k, (uint4*)v, tokens * H, H, dn / 8, dr / 8, dv / 8);
+  chain(mla_pack_kernel, (int)(blocks < cap ? blocks : cap), 256, 0, reinterpret_cast<cudaStream_t>(stream),
+        (const uint4*)kv, (const uint4*)rot, rot_ld / 8, (uint4*)k, (uint4*)v, tokens * H, H, dn / 8, dr / 8, dv / 8);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }
@@ -104,8 +106,8 @@ extern "C" int tpb_mla_unpack(const void* dk, const void* dv_, void* dkv, void* 
   if (tokens <= 0) return 0;
   const long long cap = (long long)sm_count() * 8;
   const int smem = UNPACK_THREADS / (dr / 8) * dr * 4;
-  mla_unpack_kernel<<<(int)(tokens < cap ? tokens : cap), UNPACK_THREADS, smem, reinterpret_cast<cudaStream_t>(stream)>>>(
-      (const uint4*)dk, (const uint4*)dv_, (uint4*)dkv, (uint4*)drot, tokens, H, dn / 8, dr / 8, dv / 8);
+  chain(mla_unpack_kernel, (int)(tokens < cap ? tokens : cap), UNPACK_THREADS, smem, reinterpret_cast<cudaStream_t>(stream),
+        (const uint4*)dk, (const uint4*)dv_, (uint4*)dkv, (uint4*)drot, tokens, H, dn / 8, dr / 8, dv / 8);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }

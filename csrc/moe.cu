@@ -41,6 +41,7 @@ __global__ void router_topk_kernel(const T* __restrict__ logits, const float* __
                                    float* __restrict__ w_out, int* __restrict__ idx_out,
                                    float* __restrict__ scores_out, int tokens, int E, int K, int mode, int n_group,
                                    int topk_group, int norm_topk, float scale) {
+  if (!chain_begin()) return;
   const int lane = threadIdx.x & 31;
   const int per_lane = (E + 31) / 32;
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tokens; t += (gridDim.x * blockDim.x) >> 5) {
@@ -165,6 +166,7 @@ __global__ void router_bwd_kernel(const T* __restrict__ logits, const int* __res
                                   const float* __restrict__ dw, const float* __restrict__ dscores,
                                   T* __restrict__ dlogits, int tokens, int E, int K, int mode, int norm_topk,
                                   float scale) {
+  if (!chain_begin()) return;
   const int lane = threadIdx.x & 31;
   for (int t = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; t < tokens; t += (gridDim.x * blockDim.x) >> 5) {
     float s[ROUTER_MAX_PER_LANE], ds[ROUTER_MAX_PER_LANE];
@@ -242,6 +244,7 @@ template <bool PAD>
 __global__ void moe_gather_kernel(const uint4* __restrict__ x, const int* __restrict__ src_row,
                                   const float* __restrict__ row_scale, uint4* __restrict__ out, long long rows,
                                   int nvec) {
+  if (!chain_begin()) return;
   const long long total = rows * nvec;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -267,6 +270,7 @@ __global__ void moe_gather_kernel(const uint4* __restrict__ x, const int* __rest
 __global__ void moe_combine_kernel(const uint4* __restrict__ rows, const int* __restrict__ dest,
                                    const float* __restrict__ w, uint4* __restrict__ out, long long tokens, int K,
                                    int nvec) {
+  if (!chain_begin()) return;
   const long long total = tokens * nvec;
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < total;
        i += (long long)gridDim.x * blockDim.x) {
@@ -291,6 +295,7 @@ __global__ void moe_combine_kernel(const uint4* __restrict__ rows, const int* __
 __global__ void moe_combine_dw_kernel(const uint4* __restrict__ rows, const int* __restrict__ dest,
                                       const uint4* __restrict__ dout, float* __restrict__ dw, long long pairs, int K,
                                       int nvec) {
+  if (!chain_begin()) return;
   const int lane = threadIdx.x & 31;
   for (long long pr = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5; pr < pairs;
        pr += ((long long)gridDim.x * blockDim.x) >> 5) {
@@ -376,6 +381,7 @@ __global__ void __launch_bounds__(PLAN_THREADS, 1)
 moe_plan_kernel(const int* __restrict__ idx, int n, int K, int E, int M, int align, int* __restrict__ counts,
                 int* __restrict__ k_offsets, int* __restrict__ dest, int* __restrict__ src_row,
                 long long* __restrict__ src_pair, int* __restrict__ tile_expert) {
+  if (!chain_begin()) return;
   __shared__ int wcount[32][PLAN_MAX_E];     // sweep 1: pairs of (warp, expert); sweep 2: next row
   __shared__ int off_pad[PLAN_MAX_E + 1];
   __shared__ int total_s[PLAN_MAX_E];
@@ -533,11 +539,11 @@ extern "C" int tpb_router_topk(const void* logits, int logits_is_bf16, const flo
   if (tokens <= 0) return 0;
   const int grid = grid_for_items((long long)tokens * 32, 256);
   if (logits_is_bf16)
-    router_topk_kernel<__nv_bfloat16><<<grid, 256, 0, STREAM(stream)>>>(
-        (const __nv_bfloat16*)logits, bias, w_out, idx_out, scores_out, tokens, E, K, mode, n_group, topk_group,
+    chain(router_topk_kernel<__nv_bfloat16>, grid, 256, 0, STREAM(stream),
+          (const __nv_bfloat16*)logits, bias, w_out, idx_out, scores_out, tokens, E, K, mode, n_group, topk_group,
         norm_topk, scale);
   else
-    router_topk_kernel<float><<<grid, 256, 0, STREAM(stream)>>>((const float*)logits, bias, w_out, idx_out, scores_out,
+    chain(router_topk_kernel<float>, grid, 256, 0, STREAM(stream), (const float*)logits, bias, w_out, idx_out, scores_out,
                                                                 tokens, E, K, mode, n_group, topk_group, norm_topk,
                                                                 scale);
   return rc_of(cudaGetLastError());
@@ -551,10 +557,10 @@ extern "C" int tpb_router_bwd(const void* logits, int logits_is_bf16, const int*
   if (tokens <= 0) return 0;
   const int grid = grid_for_items((long long)tokens * 32, 256);
   if (logits_is_bf16)
-    router_bwd_kernel<__nv_bfloat16><<<grid, 256, 0, STREAM(stream)>>>(
-        (const __nv_bfloat16*)logits, idx, dw, dscores, (__nv_bfloat16*)dlogits, tokens, E, K, mode, norm_topk, scale);
+    chain(router_bwd_kernel<__nv_bfloat16>, grid, 256, 0, STREAM(stream),
+          (const __nv_bfloat16*)logits, idx, dw, dscores, (__nv_bfloat16*)dlogits, tokens, E, K, mode, norm_topk, scale);
   else
-    router_bwd_kernel<float><<<grid, 256, 0, STREAM(stream)>>>((const float*)logits, idx, dw, dscores, (float*)dlogits,
+    chain(router_bwd_kernel<float>, grid, 256, 0, STREAM(stream), (const float*)logits, idx, dw, dscores, (float*)dlogits,
                                                                tokens, E, K, mode, norm_topk, scale);
   return rc_of(cudaGetLastError());
 }
@@ -563,8 +569,8 @@ extern "C" int tpb_moe_gather(const void* x, const int* src_row, const float* ro
                               int dim, void* stream) {
   if (dim % 8) return -2;
   if (rows <= 0) return 0;
-  moe_gather_kernel<true><<<grid_for_items(rows * (dim / 8), 256), 256, 0, STREAM(stream)>>>(
-      (const uint4*)x, src_row, row_scale, (uint4*)out, rows, dim / 8);
+  chain(moe_gather_kernel<true>, grid_for_items(rows * (dim / 8), 256), 256, 0, STREAM(stream),
+        (const uint4*)x, src_row, row_scale, (uint4*)out, rows, dim / 8);
   return rc_of(cudaGetLastError());
 }
 
@@ -573,8 +579,8 @@ extern "C" int tpb_moe_gather_real(const void* x, const int* src_row, void* out,
                                    void* stream) {
   if (dim % 8) return -2;
   if (rows <= 0) return 0;
-  moe_gather_kernel<false><<<grid_for_items(rows * (dim / 8), 256), 256, 0, STREAM(stream)>>>(
-      (const uint4*)x, src_row, nullptr, (uint4*)out, rows, dim / 8);
+  chain(moe_gather_kernel<false>, grid_for_items(rows * (dim / 8), 256), 256, 0, STREAM(stream),
+        (const uint4*)x, src_row, nullptr, (uint4*)out, rows, dim / 8);
   return rc_of(cudaGetLastError());
 }
 
@@ -582,8 +588,8 @@ extern "C" int tpb_moe_combine(const void* rows, const int* dest, const float* w
                                int dim, void* stream) {
   if (dim % 8) return -2;
   if (tokens <= 0) return 0;
-  moe_combine_kernel<<<grid_for_items(tokens * (dim / 8), 256), 256, 0, STREAM(stream)>>>(
-      (const uint4*)rows, dest, w, (uint4*)out, tokens, K, dim / 8);
+  chain(moe_combine_kernel, grid_for_items(tokens * (dim / 8), 256), 256, 0, STREAM(stream),
+        (const uint4*)rows, dest, w, (uint4*)out, tokens, K, dim / 8);
   return rc_of(cudaGetLastError());
 }
 
@@ -591,8 +597,8 @@ extern "C" int tpb_moe_combine_dw(const void* rows, const int* dest, const void*
                                   int K, int dim, void* stream) {
   if (dim % 8) return -2;
   if (tokens <= 0) return 0;
-  moe_combine_dw_kernel<<<grid_for_items(tokens * K * 32, 256), 256, 0, STREAM(stream)>>>(
-      (const uint4*)rows, dest, (const uint4*)dout, dw, tokens * K, K, dim / 8);
+  chain(moe_combine_dw_kernel, grid_for_items(tokens * K * 32, 256), 256, 0, STREAM(stream),
+        (const uint4*)rows, dest, (const uint4*)dout, dw, tokens * K, K, dim / 8);
   return rc_of(cudaGetLastError());
 }
 
@@ -626,7 +632,8 @@ extern "C" int tpb_moe_plan(const int* idx, int tokens, int K, int E, int rows, 
   if ((align != 16 && align != 32 && align != 128 && align != 256) || rows % align) return -2;
   const long long n = (long long)tokens * K;
   if (n > (1LL << 30) || rows < n + (long long)(align - 1) * (n < E ? n : E)) return -2;
-  moe_plan_kernel<<<1, PLAN_THREADS, 0, STREAM(stream)>>>(idx, (int)n, K, E, rows, align, counts, k_offsets, dest, src_row,
+  chain(moe_plan_kernel, 1, PLAN_THREADS, 0, STREAM(stream),
+        idx, (int)n, K, E, rows, align, counts, k_offsets, dest, src_row,
                                                           src_pair, tile_expert);
   return rc_of(cudaGetLastError());
 }

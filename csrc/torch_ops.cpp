@@ -768,6 +768,7 @@ py::object router_topk(py::handle lg_, py::handle bias_, int64_t k, int64_t mode
                        bool norm_topk, double scale) {
   Tensor lg, bias, w, idx, scores;
   if (at::GradMode::is_enabled() || !unobserved() || !unpack(lg_, lg) || !unpack(bias_, bias)) return py::none();
+  if (bias.defined() && plain_rows(bias)) bias = bias.to(at::kFloat);
   if (!(plain_rows(lg, at::kFloat) || plain_rows(lg)) || lg.dim() != 2 || lg.size(1) > 256 || k < 1 || k > lg.size(1) ||
       !small(lg.size(0)) || (bias.defined() && (!plain_rows(bias, at::kFloat) || bias.numel() != lg.size(1))))
     return py::none();
