@@ -312,6 +312,26 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// Bounded wait on a barrier of this CTA that other CTAs of the cluster arrive on after writing to its shared memory.
+__device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int* st, int code, int where) {
+  const uint32_t at = smem_u32(bar);
+  long long t0 = 0;
+  for (int i = 0;; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred P;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 P, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, P;\n\t}"
+        : "=r"(ok)
+        : "r"(at), "r"(parity)
+        : "memory");
+    if (ok) return true;
+    if ((i & 63) == 63) {
+      if (t0 == 0) t0 = clock64();
+      else if (clock64() - t0 > kSpinBudgetCycles) { report(st, code, where); return false; }
+    }
+  }
+}
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_result, uint32_t ncols) {
   asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_result)),
                "r"(ncols)
@@ -335,9 +355,9 @@ __device__ __forceinline__ void mma_ss_pair_w(uint32_t d_tmem, uint32_t a_lo, ui
       : "memory");
 }
 // Arrive on the barrier at this shared-memory offset in both CTAs of the pair once every MMA
-// issued so far has completed.
-__device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {
-  const uint16_t mask = 3;
+// issued so far has completed.  `lead`: cluster rank of the pair's even CTA.
+__device__ __forceinline__ void tc_commit_pair(uint64_t* bar, int lead = 0) {
+  const uint16_t mask = (uint16_t)(3 << lead);
   asm volatile(
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(
           smem_u32(bar)),

@@ -141,6 +141,13 @@ __device__ __forceinline__ TileInfo tile_info(const GemmParams& p, int t, int m_
   return ti;
 }
 
+// This pair's part of the tile's contraction.
+__device__ __forceinline__ void take_part(TileInfo& ti, int part, int parts) {
+  const int per = (ti.kb1 - ti.kb0 + parts - 1) / parts;
+  ti.kb0 = min(ti.kb1, ti.kb0 + part * per);
+  ti.kb1 = min(ti.kb1, ti.kb0 + per);
+}
+
 __device__ __forceinline__ float silu_f(float x) { return x / (1.0f + __expf(-x)); }
 
 __device__ __forceinline__ long long ag_chunks_per_shard(const GemmParams& p) {
@@ -339,7 +346,14 @@ __device__ __forceinline__ void slab_store(uint4* slabs, int& buf, const uint32_
 // the even CTA issues tcgen05.mma.cta_group::2 (M = 256) for both, and each CTA drains its own
 // 128 accumulator rows.  Shared-memory traffic per FLOP drops by a third, which is what bounds
 // the single-CTA kernel (TMA writes plus operand reads exceed 128 B/clk).  Dense mode only.
-template <bool A_MN, bool B_MN, bool PAIR>
+//
+// KSPLIT (pairs, dense): two pairs (a cluster of four CTAs) share a tile, each contracting over half of K, and each finishes
+// half of the tile's columns.  With the main loop over, the ring is free: an epilogue warp lays its 32 rows of the other
+// half's fp32 sums out there, sends them to the warp that holds the same rows in the other pair with one bulk copy between
+// the SMs, and adds what it gets to its own (no workspace, no atomics, the same result every run).  The next tile's loads
+// wait for that.  (Stored into the other SM's shared memory 16 bytes a lane, the exchange took a third longer.)
+// For products whose tiles leave pairs idle; the rule and its measurements stand at ksplit_wins().
+template <bool A_MN, bool B_MN, bool PAIR, bool KSPLIT>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
             const __grid_constant__ CUtensorMap tmB2, const __grid_constant__ CUtensorMap tmC,
@@ -356,15 +370,21 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   uint64_t* acc_full = empty + NST;
   uint64_t* acc_empty = acc_full + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_empty + 2);
+  uint64_t* rx_full = acc_empty + 3;      // KSPLIT: [4 epilogue warps] the other pair's sums have arrived
+  uint64_t* peer_ready = rx_full + 4;     // KSPLIT: [4] the other pair's main loop is over: its ring can be written
+  uint64_t* ring_free = rx_full + 8;      // KSPLIT: the exchange is over on both sides (four warps here, four there)
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (!PAIR && (int)blockIdx.x < p.ag_copiers) {
     if (p.ag_push) ag_pusher(p); else ag_copier(p, smem);
     return;
   }
-  const int rank = PAIR ? (int)cluster_ctarank() : 0;    // 0: issues the MMAs of the pair
-  // tiles are dealt to CTAs (or to CTA pairs)
-  const int cta = PAIR ? (int)blockIdx.x / 2 : (int)blockIdx.x - p.ag_copiers;
-  const int n_ctas = PAIR ? (int)gridDim.x / 2 : (int)gridDim.x - p.ag_copiers;
+  const int crank = PAIR ? (int)cluster_ctarank() : 0;
+  const int rank = crank & 1, lead = crank & ~1;         // rank 0: issues the MMAs of the pair
+  const int part = KSPLIT ? crank >> 1 : 0;
+  constexpr int parts = KSPLIT ? 2 : 1;
+  // tiles are dealt to CTAs (or to CTA pairs, or to clusters of pairs)
+  const int cta = PAIR ? (int)blockIdx.x / (2 * parts) : (int)blockIdx.x - p.ag_copiers;
+  const int n_ctas = PAIR ? (int)gridDim.x / (2 * parts) : (int)gridDim.x - p.ag_copiers;
   const bool swiglu = p.epi == TPB_EPI_SWIGLU;
   const int tile_n_out = swiglu ? BN / 2 : BN;  // output columns covered by one tile
   const int n_logical = swiglu ? p.N / 2 : p.N;
@@ -382,6 +402,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       mbar_init(&acc_full[a], 1);
       mbar_init(&acc_empty[a], PAIR ? 8 : 4);   // one arrival per epilogue warp (of both CTAs)
     }
+    if (KSPLIT)
+      for (int w = 0; w < 9; ++w) mbar_init(&rx_full[w], w < 8 ? 1 : 8);
     fence_barrier_init();
   }
   if (warp == 1) {
@@ -407,12 +429,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       tma_prefetch_desc(&tmB2);
-      int stage = 0;
+      int stage = 0, tiles_done = 0;
       uint32_t phase = 0;
       bool ok = true;
       for (int t = cta; t < num_tiles && ok; t += n_ctas) {
-        const TileInfo ti = tile_info(p, t, m_tiles, n_tiles, num_kb);
+        TileInfo ti = tile_info(p, t, m_tiles, n_tiles, num_kb);
         if (ti.skip) continue;
+        if (KSPLIT) take_part(ti, part, parts);
         const int m0 = ti.tm * TM + rank * BM, n0 = ti.tn * tile_n_out;
         const int ez = p.mode == 1 ? ti.e : 0;
         if (p.ag_world > 0) {
@@ -428,6 +451,10 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             if (!ag_wait_range(p, lo2, hi2)) { ok = false; break; }
           }
         }
+        if (KSPLIT && t != cta) {
+          if (!mbar_wait_cluster(ring_free, tiles_done & 1, p.status, kTimeoutStageFree, 9)) { ok = false; break; }
+          ++tiles_done;
+        }
         for (int kb = ti.kb0; kb < ti.kb1; ++kb) {
           if (!mbar_wait(&empty[stage], phase ^ 1, p.status, kTimeoutStageFree, 1)) {
             ok = false;
@@ -442,7 +469,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           const int kB = second_b ? k0 - p.kb_b2 * BK : k0;
           if (PAIR) {
             // Both CTAs' bytes are counted on the even CTA's barrier, which alone expects them.
-            const uint32_t bar = map_to_cta(smem_u32(&full[stage]), 0);
+            const uint32_t bar = map_to_cta(smem_u32(&full[stage]), lead);
             if (rank == 0) mbar_expect_tx(&full[stage], 2 * SBYTES);
             if (!A_MN) {
               tma_load_2d_pair(sA, &tmA, bar, k0, m0);
@@ -502,8 +529,9 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       bool ok = true;
       int local = 0;
       for (int t = cta; t < num_tiles && ok; t += n_ctas) {
-        const TileInfo ti = tile_info(p, t, m_tiles, n_tiles, num_kb);
+        TileInfo ti = tile_info(p, t, m_tiles, n_tiles, num_kb);
         if (ti.skip) continue;
+        if (KSPLIT) take_part(ti, part, parts);
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1;
         ++local;
@@ -545,13 +573,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
                        ((kb - ti.kb0) | k) != 0);
           }
           if (!ok) break;
-          if (PAIR) tc_commit_pair(&empty[stage]); else tc_commit(&empty[stage]);
+          if (PAIR) tc_commit_pair(&empty[stage], lead); else tc_commit(&empty[stage]);
           if (++stage == NST) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) { if (PAIR) tc_commit_pair(&acc_full[acc]); else tc_commit(&acc_full[acc]); }
+        if (ok) { if (PAIR) tc_commit_pair(&acc_full[acc], lead); else tc_commit(&acc_full[acc]); }
       }
     }
   } else {
@@ -577,7 +605,80 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       const uint32_t t_addr = tmem_base + acc * BN + ((uint32_t)(q * 32) << 16);
       const bool row_ok = row < p.M;
 
-      if (p.tma_store) {
+      if (KSPLIT) {
+        // in the ring: this warp's 32 rows x 128 columns of fp32, as [16-byte vector][lane], to send and as received
+        uint4* tx = reinterpret_cast<uint4*>(smem) + q * 1024;
+        uint4* rx = reinterpret_cast<uint4*>(smem + 65536) + q * 1024;
+        const uint32_t other = crank ^ 2;
+        const int row0 = tm * TM + rank * BM + q * 32;   // the same rows in the other pair
+        const uint32_t par = (local - 1) & 1;
+        if (lane == 0) {
+          mbar_expect_tx(&rx_full[q], 16384);
+          mbar_arrive_cluster(map_to_cta(smem_u32(&peer_ready[q]), other));
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t r[32];
+          tmem_ld32(t_addr + (part ^ 1) * 128 + c * 32, r);
+          tmem_wait_ld();
+#pragma unroll
+          for (int v = 0; v < 8; ++v) tx[(c * 8 + v) * 32 + lane] = make_uint4(r[4 * v], r[4 * v + 1], r[4 * v + 2], r[4 * v + 3]);
+        }
+        fence_proxy_async();
+        __syncwarp();
+        bool ok = true;
+        if (lane == 0) {
+          ok = mbar_wait_cluster(&peer_ready[q], par, p.status, kTimeoutAccFull, 7);
+          if (ok)
+            asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                             map_to_cta(smem_u32(rx), other)),
+                         "r"(smem_u32(tx)), "r"(16384), "r"(map_to_cta(smem_u32(&rx_full[q]), other))
+                         : "memory");
+        }
+        ok = __all_sync(0xffffffffu, mbar_wait_cluster(&rx_full[q], par, p.status, kTimeoutAccFull, 8)) &&
+             __shfl_sync(0xffffffffu, (int)ok, 0);
+        if (lane == 0) mbar_arrive_cluster(map_to_cta(smem_u32(ring_free), other));   // what it sent has left its ring
+        if (ok && row0 < p.M) {
+#pragma unroll 1
+          for (int c = 0; c < 128; c += 64) {
+            const int col = n0 + part * 128 + c;
+            if (col >= p.N) break;
+            uint32_t o[32];
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+              uint32_t r[32];
+              float f[32];
+              tmem_ld32(t_addr + part * 128 + c + h * 32, r);
+              tmem_wait_ld();
+#pragma unroll
+              for (int v = 0; v < 8; ++v) {
+                const uint4 x = rx[(c / 4 + h * 8 + v) * 32 + lane];
+                f[4 * v] = (__uint_as_float(r[4 * v]) + __uint_as_float(x.x)) * alpha;
+                f[4 * v + 1] = (__uint_as_float(r[4 * v + 1]) + __uint_as_float(x.y)) * alpha;
+                f[4 * v + 2] = (__uint_as_float(r[4 * v + 2]) + __uint_as_float(x.z)) * alpha;
+                f[4 * v + 3] = (__uint_as_float(r[4 * v + 3]) + __uint_as_float(x.w)) * alpha;
+              }
+              if (p.epi == TPB_EPI_BF16_RES && row_ok) {
+                const __nv_bfloat16* R = reinterpret_cast<const __nv_bfloat16*>(p.aux) + (long long)row * p.ldaux + col + h * 32;
+#pragma unroll
+                for (int v = 0; v < 4; ++v) {
+                  if (col + h * 32 + 8 * v >= p.N) break;      // (N is a multiple of 8)
+                  const uint4 old = *reinterpret_cast<const uint4*>(R + 8 * v);
+                  const float2 a = unpack_bf16(old.x), b = unpack_bf16(old.y), cc = unpack_bf16(old.z), d = unpack_bf16(old.w);
+                  f[8 * v] += a.x; f[8 * v + 1] += a.y; f[8 * v + 2] += b.x; f[8 * v + 3] += b.y;
+                  f[8 * v + 4] += cc.x; f[8 * v + 5] += cc.y; f[8 * v + 6] += d.x; f[8 * v + 7] += d.y;
+                }
+              }
+#pragma unroll
+              for (int j = 0; j < 16; ++j) o[16 * h + j] = pack_bf16(f[2 * j], f[2 * j + 1]);
+            }
+            slab_store<false>(slabs, buf, o, &tmC, col, row0, 0, lane);
+          }
+        }
+        fence_proxy_async();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ring_free);
+      } else if (p.tma_store) {
         const int row0 = tm * TM + rank * BM + q * 32;   // this warp's 32 rows
         if (row0 < p.M) {
           if (swiglu) {
@@ -816,7 +917,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
       tc_fence_before();
       __syncwarp();
       if (lane == 0) {
-        if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[acc]), 0));
+        if (PAIR) mbar_arrive_cluster(map_to_cta(smem_u32(&acc_empty[acc]), lead));
         else mbar_arrive(&acc_empty[acc]);
       }
     }
@@ -851,13 +952,13 @@ cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
                         const CUtensorMap& tc2, const GemmParams& p, int grid, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<A_MN, B_MN, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<A_MN, B_MN, false, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          GEMM_SMEM);
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (chainable(p)) return chain(gemm_kernel<A_MN, B_MN, false>, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb2, tc, tc2, p);
-  gemm_kernel<A_MN, B_MN, false><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, tb2, tc, tc2, p);
+  if (chainable(p)) return chain(gemm_kernel<A_MN, B_MN, false, false>, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb2, tc, tc2, p);
+  gemm_kernel<A_MN, B_MN, false, false><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, tb2, tc, tc2, p);
   return cudaGetLastError();
 }
 
@@ -867,13 +968,13 @@ cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const
                              const CUtensorMap& tc2, const GemmParams& p, int grid, cudaStream_t stream) {
   static bool configured = false;
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<A_MN, B_MN, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<A_MN, B_MN, true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          GEMM_SMEM);
     if (e != cudaSuccess) return e;
     configured = true;
   }
   if (chainable(p))
-    return chain_clusters(gemm_kernel<A_MN, B_MN, true>, 2, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb2, tc, tc2, p);
+    return chain_clusters(gemm_kernel<A_MN, B_MN, true, false>, 2, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb2, tc, tc2, p);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
   cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
@@ -886,10 +987,62 @@ cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  return cudaLaunchKernelEx(&cfg, gemm_kernel<A_MN, B_MN, true>, ta, tb, tb2, tc, tc2, p);
+  return cudaLaunchKernelEx(&cfg, gemm_kernel<A_MN, B_MN, true, false>, ta, tb, tb2, tc, tc2, p);
 }
 
 
+
+// Launch as clusters of two pairs that share a tile.
+template <bool B_MN>
+cudaError_t launch_gemm_ksplit(const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap& tc, const GemmParams& p,
+                               int clusters, cudaStream_t stream) {
+  static bool configured = false;
+  if (!configured) {
+    cudaError_t e = cudaFuncSetAttribute(gemm_kernel<false, B_MN, true, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         GEMM_SMEM);
+    if (e != cudaSuccess) return e;
+    configured = true;
+  }
+  return chain_clusters(gemm_kernel<false, B_MN, true, true>, 4, 4 * clusters, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb, tc,
+                        tc, p);
+}
+
+// Clusters of `ctas` CTAs of the GEMM kernel that can be resident at once (an SM without free partners stays idle).
+static int resident_clusters(int ctas) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(sm_count() / ctas * ctas, 1, 1);
+  cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = GEMM_SMEM;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = ctas; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  int n = 0;
+  const auto kernel = gemm_kernel<false, false, true, true>;
+  cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess || n < 1) n = 0;
+  (void)cudaGetLastError();
+  return n < sm_count() / ctas ? n : sm_count() / ctas;
+}
+
+// Whether two pairs to a tile are the faster way for bf16 results of M rows (dense, A K-major).  T 256 x 256 tiles run on
+// 74 pairs or on C = 36 clusters; the exchange of partial sums costs 5 to 10 us a tile, during which its cluster does nothing
+// else, so the contraction has to be long, and fewer half-length waves than twice the whole ones have to come out (us, the
+// kernel used otherwise / this one):
+//   T = 24: 6144 x 4096 24.6 / 22.5    T = 32: 4096 x 4096 24 / 22, x 6144 31 / 27.5, x 14336 60 / 50, x 28672 113 / 94
+//   T = 48: 4096 x 4096 36 / 41, x 14336 108 / 95, x 28672 201 / 171, 2048 x 10944 84 / 80    T = 64: x 14336 102 / 94
+//   T = 96: 4096 x 6144 78 / 79, x 14336 166 / 143, x 28672 324 / 268      T = 128: x 14336 172 / 192, x 28672 340 / 360
+// Up to 16 tiles the few-rows kernel, which splits further, is ahead (T = 16, 4096 x 14336: 37 / 46).
+static bool ksplit_wins(int M, int N, int K) {
+  if (M <= 128 || K < 4096) return false;
+  const long long t = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
+  if (t < 24) return false;
+  static const int clusters = resident_clusters(4), pairs = resident_clusters(2);
+  if (clusters < 1 || pairs < 1) return false;
+  if (t <= clusters) return true;
+  const long long half = (t + clusters - 1) / clusters, whole = (t + pairs - 1) / pairs;
+  return K >= 8192 && (whole == 1 || (half < 2 * whole && (whole == 2 || K >= 20480)));
+}
 
 // gemm_skinny_sm100.cu
 int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, int experts,
@@ -923,6 +1076,7 @@ struct GemmCall {
   int rs_world; void* const* rs_dst; long long rs_shard_elems, rs_c_offset;
   int rs_rank;
   int rs_store;
+  int ksplit;                   // 1: two CTA pairs share a tile's contraction
   long long ag_chunk_elems;     // external gather (ag_copiers == 0): elements per flag
 };
 
@@ -971,6 +1125,11 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   if (g.mode == 2 && (g.c_stride % (f32out ? 4 : 8))) tma_store = false;
   const uint64_t n_cols = swiglu ? g.N / 2 : g.N;
   if (n_cols % (f32out ? 4 : 8)) tma_store = false;   // a box is clipped in steps of 16 bytes: it would write past the last column
+  // A split contraction: results (the residual sum among them) leave through TMA, both halves have k-blocks.
+  const bool res = g.epi == TPB_EPI_BF16_RES;
+  if (g.ksplit && res && n_cols % 8 == 0) tma_store = true;
+  const bool ksplit_ok = g.mode == 0 && g.ag_world == 0 && g.rs_world == 0 && !g.a_mn && !cat_k && tma_store && g.K > BK &&
+                         (g.epi == TPB_EPI_BF16 || (res && g.aux && !misaligned(g.aux) && g.ldaux % 8 == 0));
   if (tma_store) {
     const uint64_t planes = g.mode == 2 ? g.E : 1;
     const uint64_t plane = g.mode == 2 && g.E > 1 ? (uint64_t)g.c_stride : (uint64_t)g.ldc * g.M;
@@ -1036,22 +1195,7 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   cudaError_t e;
   // CTA pairs for dense GEMMs with enough 256 x 256 tiles to fill the machine
   const int pair_mode = gemm_pair_mode();
-  static const int max_pairs = []() {
-    // clusters of two that can be resident at once (an SM without a free partner stays idle)
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(2 * 74, 1, 1);
-    cfg.blockDim = dim3(GEMM_THREADS, 1, 1);
-    cfg.dynamicSmemBytes = GEMM_SMEM;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
-    cfg.attrs = attr; cfg.numAttrs = 1;
-    int n = 0;
-    cudaFuncSetAttribute(gemm_kernel<false, false, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, GEMM_SMEM);
-    if (cudaOccupancyMaxActiveClusters(&n, gemm_kernel<false, false, true>, &cfg) != cudaSuccess || n < 1) n = 0;
-    (void)cudaGetLastError();
-    return n < sm_count() / 2 ? n : sm_count() / 2;
-  }();
+  static const int max_pairs = resident_clusters(2);
   const long long pair_tiles = (long long)((g.M + 2 * BM - 1) / (2 * BM)) * n_tiles * (g.mode == 2 ? g.E : 1);
   // grouped modes: rows mode needs expert segments padded to whole 256-row tiles; the per-expert
   // K-range mode (weight gradients) has no such condition
@@ -1059,6 +1203,15 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   // (the in-kernel copier CTAs of the fused all-gather and the red.add reduce-scatter were tuned on the
   // single-CTA kernel and stay there; waiting on an external gather and the store-mode scatter run on pairs)
   const bool pair_coll_ok = (g.ag_world == 0 || p.ag_copiers == 0) && (g.epi != TPB_EPI_RS_BF16 || g.rs_store);
+  if (g.ksplit) {
+    static const int resident = resident_clusters(4);
+    if (!ksplit_ok || resident < 1) return -2;
+    const int n = pair_tiles > resident ? resident : (int)pair_tiles;
+    const int m_tiles2 = (g.M + 2 * BM - 1) / (2 * BM);
+    p.group_m = m_tiles2 < 8 ? m_tiles2 : 8;
+    e = g.b_mn ? launch_gemm_ksplit<true>(ta, tb, tc, p, n, stream) : launch_gemm_ksplit<false>(ta, tb, tc, p, n, stream);
+    return e == cudaSuccess ? 0 : 1000 + (int)e;
+  }
   if (pair_mode != 0 && max_pairs > 0 && pair_shape_ok && pair_coll_ok &&
       g.max_ctas == 0 && (pair_mode == 2 || pair_tiles >= max_pairs)) {
     p.te_stride = 2;
@@ -1088,8 +1241,9 @@ extern "C" int tpb_gemm_scaled_bf16(const void* A, const void* B, void* C, int M
                                     long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha,
                                     const float* scale, const void* aux, long long ldaux, void* c2, long long ldc2,
                                     int max_ctas, void* stream_) {
+  const bool split = max_ctas == 0 && gemm_pair_mode() == 1 && !a_mn && ksplit_wins(M, N, K);
   // few rows or few tiles: the kernel that streams B once and splits the contraction
-  if (max_ctas == 0 && gemm_pair_mode() == 1 &&
+  if (max_ctas == 0 && gemm_pair_mode() == 1 && !split &&
       (a_mn ? b_mn && skinny_wins_wgrad(M, N, K) : skinny_wins(M, N, K, epi == TPB_EPI_SWIGLU))) {
     const int r = skinny_gemm(A, B, nullptr, C, M, N, K, 1, lda, ldb, 0, ldc, a_mn, b_mn, epi, alpha, aux, ldaux, c2, ldc2,
                               nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_), false, scale);
@@ -1102,6 +1256,12 @@ extern "C" int tpb_gemm_scaled_bf16(const void* A, const void* B, void* C, int M
   g.a_mn = a_mn; g.b_mn = b_mn; g.epi = epi; g.alpha = alpha; g.alpha_dev = scale;
   g.aux = aux; g.ldaux = ldaux; g.c2 = c2; g.ldc2 = ldc2; g.max_ctas = max_ctas;
   g.mode = 0;
+  if (split) {
+    g.ksplit = 1;
+    const int r = run_gemm(g, reinterpret_cast<cudaStream_t>(stream_));
+    if (r != -2) return r;     // -2: an epilogue or alignment it does not take
+    g.ksplit = 0;
+  }
   return run_gemm(g, reinterpret_cast<cudaStream_t>(stream_));
 }
 
@@ -1132,6 +1292,20 @@ extern "C" int tpb_grouped_gemm_bf16(const void* A, const void* B, const void* B
   return run_gemm(g, reinterpret_cast<cudaStream_t>(stream_));
 }
 
+
+// tpb_gemm_bf16 with two CTA pairs to a tile, each contracting over half of K; -2 for what that does not take.
+extern "C" int tpb_gemm_ksplit_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                                    long long ldc, int a_mn, int b_mn, int epi, float alpha, const void* aux,
+                                    long long ldaux, void* c2, long long ldc2, void* stream_) {
+  GemmCall g{};
+  g.A = A; g.B = B; g.C = C;
+  g.M = M; g.N = N; g.K = K; g.E = 1;
+  g.lda = lda; g.ldb = ldb; g.ldc = ldc;
+  g.a_mn = a_mn; g.b_mn = b_mn; g.epi = epi; g.alpha = alpha;
+  g.aux = aux; g.ldaux = ldaux; g.c2 = c2; g.ldc2 = ldc2;
+  g.ksplit = 1;
+  return run_gemm(g, reinterpret_cast<cudaStream_t>(stream_));
+}
 
 // Per-expert weight gradients (mode 2 of tpb_grouped_gemm_bf16) that contract over the rows in front of every segment's
 // padding only: expert e's rows are k_offsets[e] + [0, k_counts[e]), to the next multiple of 64, and those up to there are

@@ -41,6 +41,11 @@ int tpb_gemm_scaled_bf16(const void* A, const void* B, void* C, int M, int N, in
                          const void* aux, long long ldaux, void* c2, long long ldc2, int max_ctas,
                          void* stream);
 
+// The same with two CTA pairs to a tile, each contracting over half of K; -2 for what that does not take.
+int tpb_gemm_ksplit_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda, long long ldb,
+                         long long ldc, int a_mn, int b_mn, int epi, float alpha, const void* aux, long long ldaux, void* c2,
+                         long long ldc2, void* stream);
+
 // y = rmsnorm(x [+ res]) * w.  h_out (optional) receives x + res.  rstd: [rows] fp32.
 int tpb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void* h_out, float* rstd,
                     int rows, int dim, float eps, void* stream);

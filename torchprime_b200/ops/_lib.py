@@ -85,6 +85,7 @@ def _declare(L):
     "tpb_sm_count": [],
     "tpb_gemm_bf16": [P, P, P, I, I, I, LL, LL, LL, I, I, I, F, P, LL, P, LL, I, P],
     "tpb_gemm_scaled_bf16": [P, P, P, I, I, I, LL, LL, LL, I, I, I, F, P, P, LL, P, LL, I, P],
+    "tpb_gemm_ksplit_bf16": [P, P, P, I, I, I, LL, LL, LL, I, I, I, F, P, LL, P, LL, P],
     "tpb_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "tpb_rmsnorm_bwd": [P, P, P, P, P, P, P, I, I, P],
     "tpb_rope": [P, LL, I, I, I, P, P, P, I, I, I, I, P],
