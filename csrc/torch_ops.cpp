@@ -710,23 +710,37 @@ py::object embedding(py::handle ids_, py::handle table_) {
   return py::cast(y);
 }
 
-// One decode step over the compressed cache; see mla_decode.absorb_step (which checks the same things one by one).
+// What mla_decode.supported asks for; the tensors as given to it.
+bool absorb_args(py::handle q_, py::handle ckv_, py::handle nw_, py::handle kvc_, py::handle pec_, py::handle w_, int64_t heads,
+                 int64_t dn, int64_t dv, Tensor& q, Tensor& ckv, Tensor& nw, Tensor& kvc, Tensor& pec, Tensor& w) {
+  if (at::GradMode::is_enabled() || !unobserved() || !unpack(q_, q) || !unpack(ckv_, ckv) || !unpack(nw_, nw) ||
+      !unpack(kvc_, kvc) || !unpack(pec_, pec) || !unpack(w_, w))
+    return false;
+  for (const Tensor* t : {&q, &ckv, &nw, &kvc, &pec, &w})
+    if (!plain_rows(*t) || !aligned(*t)) return false;
+  if (q.dim() != 3 || ckv.dim() != 3 || kvc.dim() != 3 || pec.dim() != 3) return false;
+  const int64_t b = q.size(0), c = kvc.size(2), dr = pec.size(2);
+  return q.size(1) == 1 && b <= 65535 && dv <= 4096 && dr == 64 && c % 64 == 0 && c >= 64 && c <= 512 && dn % 8 == 0 && dn >= 8 &&
+         dn <= 512 && q.size(2) == heads * (dn + dr) && ckv.size(0) == b && ckv.size(1) == 1 && ckv.size(2) == c + dr &&
+         nw.numel() == c && w.size(-1) == c && w.numel() == heads * (dn + dv) * c && kvc.size(0) >= b && pec.size(0) >= b;
+}
+
+bool absorb_supported(py::handle q_, py::handle ckv_, py::handle nw_, py::handle kvc_, py::handle pec_, py::handle w_,
+                      int64_t heads, int64_t dn, int64_t dr, int64_t dv, int64_t c) {
+  Tensor q, ckv, nw, kvc, pec, w;
+  return absorb_args(q_, ckv_, nw_, kvc_, pec_, w_, heads, dn, dv, q, ckv, nw, kvc, pec, w) && pec.size(2) == dr && kvc.size(2) == c;
+}
+
+// One decode step over the compressed cache; see mla_decode.absorb_step.
 py::object absorb_step(py::handle q_, py::handle ckv_, py::handle nw_, double eps, py::handle cos_, py::handle sin_, int64_t pos,
                        py::handle kvc_, py::handle pec_, py::handle w_, int64_t heads, int64_t dn, int64_t dv, double scale,
                        bool interleaved) {
   Tensor q, ckv, nw, cos, sin, kvc, pec, w, out;
-  if (at::GradMode::is_enabled() || !unobserved() || !unpack(q_, q) || !unpack(ckv_, ckv) || !unpack(nw_, nw) ||
-      !unpack(cos_, cos) || !unpack(sin_, sin) || !unpack(kvc_, kvc) || !unpack(pec_, pec) || !unpack(w_, w))
+  if (!absorb_args(q_, ckv_, nw_, kvc_, pec_, w_, heads, dn, dv, q, ckv, nw, kvc, pec, w) || !unpack(cos_, cos) || !unpack(sin_, sin))
     return py::none();
-  for (const Tensor* t : {&q, &ckv, &nw, &kvc, &pec, &w})
-    if (!plain_rows(*t) || !aligned(*t)) return py::none();
-  if (q.dim() != 3 || ckv.dim() != 3 || kvc.dim() != 3 || pec.dim() != 3) return py::none();
   const int64_t b = q.size(0), c = kvc.size(2), dr = pec.size(2);
-  if (q.size(1) != 1 || b > 65535 || dv > 4096 || dr != 64 || c % 64 || c < 64 || c > 512 || dn % 8 || dn < 8 || dn > 512 ||
-      q.size(2) != heads * (dn + dr) || ckv.size(0) != b || ckv.size(1) != 1 || ckv.size(2) != c + dr || nw.numel() != c ||
-      w.size(-1) != c || w.numel() != heads * (dn + dv) * c || kvc.size(0) < b || pec.size(0) < b || pos < 0 || kvc.size(1) <= pos ||
-      pec.size(1) <= pos || !plain_rows(cos, at::kFloat) || !plain_rows(sin, at::kFloat) || cos.dim() != 2 || sin.dim() != 2 ||
-      cos.size(0) <= pos || sin.size(0) <= pos || cos.size(1) != 32 || sin.size(1) != 32)
+  if (pos < 0 || kvc.size(1) <= pos || pec.size(1) <= pos || !plain_rows(cos, at::kFloat) || !plain_rows(sin, at::kFloat) ||
+      cos.dim() != 2 || sin.dim() != 2 || cos.size(0) <= pos || sin.size(0) <= pos || cos.size(1) != 32 || sin.size(1) != 32)
     return py::none();
   {
     py::gil_scoped_release nogil;
@@ -845,6 +859,7 @@ PYBIND11_MODULE(_tpb_torch, m) {
   m.def("latent_split", &latent_split);
   m.def("mla_pack", &mla_pack);
   m.def("embedding", &embedding);
+  m.def("absorb_supported", &absorb_supported);
   m.def("absorb_step", &absorb_step);
   m.def("linear_f32", &linear_f32);
   m.def("router_topk", &router_topk);

@@ -70,12 +70,12 @@ class DeepseekInferenceEngine:
                      attn.q_b_proj.weight)
     ckv = ops.linear(x, attn.kv_a_proj_with_mqa.weight, bias=attn.kv_a_proj_with_mqa.bias)
     norm = attn.kv_a_layernorm
-    if self.attn_impl == "absorb" and s == 1:
-      o = mla_decode.decode_attention(q, ckv, norm.weight, norm.variance_epsilon, self.cos, self.sin, start, self.kv_cache[li],
-                                      self.pe_cache[li], attn.kv_b_proj.weight, h, dn, dr, dv, c, attn.scaling,
-                                      attn.rope_interleave)
-      if o is not None:
-        return ops.linear(o, attn.o_proj.weight, bias=attn.o_proj.bias, residual=residual)
+    if self.attn_impl == "absorb" and mla_decode.supported(q, ckv, norm.weight, self.kv_cache[li], self.pe_cache[li],
+                                                           attn.kv_b_proj.weight, h, dn, dr, dv, c):
+      o = mla_decode.absorb_step(q, ckv, norm.weight, norm.variance_epsilon, self.cos, self.sin, start,
+                                 self.kv_cache[li], self.pe_cache[li], attn.kv_b_proj.weight, h, dn, dv, attn.scaling,
+                                 attn.rope_interleave)
+      return ops.linear(o, attn.o_proj.weight, bias=attn.o_proj.bias, residual=residual)
     pos = positions()
     q = ops.rope_slices(q, self.cos, self.sin, h, dr, s, col0=dn, head_stride=dn + dr, pos=pos,
                         interleaved=attn.rope_interleave)

@@ -25,7 +25,9 @@ def _rows(t, width) -> bool:
 def supported(q, ckv, norm_w, kv_cache, pe_cache, w, heads, dn, dr, dv, c) -> bool:
   """One token per sequence, bf16 throughout, rotary width 64, a latent of at most 512 values, value width up to 4096
   and as many sequences as a grid dimension holds."""
-  from .functional import inference_only, use_kernels
+  from .functional import _native, inference_only, use_kernels
+  if (nat := _native()) is not None and nat.absorb_supported(q, ckv, norm_w, kv_cache, pe_cache, w, heads, dn, dr, dv, c):
+    return True
   ts = (q, ckv, norm_w, kv_cache, pe_cache, w)
   if not all(t.is_cuda and t.dtype == torch.bfloat16 for t in ts) or not use_kernels(*ts):
     return False
@@ -40,6 +42,11 @@ def absorb_step(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads
   normalised latent and rotated key go to position ``pos`` of the caches [>=B, S, C] / [>=B, S, 64] and it
   attends to positions 0 .. pos.  ``w``: the key / value up-projection [heads * (dn + dv), C].
   Returns [B, 1, heads * dv]."""
+  from .functional import _native
+  if (nat := _native()) is not None:
+    o = nat.absorb_step(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads, dn, dv, scale, interleaved)
+    if o is not None:
+      return o
   b, c = q.shape[0], kv_cache.shape[-1]
   assert cos.dtype == sin.dtype == torch.float32 and cos.is_contiguous() and sin.is_contiguous()
   assert cos.shape[0] > pos and cos.shape[1] == 32 and kv_cache.shape[1] > pos and kv_cache.shape[0] >= b
@@ -55,15 +62,3 @@ def absorb_step(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads
                             stream_ptr())
   check(rc, f"mla_decode B={b} H={heads} pos={pos}")
   return out
-
-
-def decode_attention(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads, dn, dr, dv, c, scale, interleaved):
-  """:func:`absorb_step`, or None where it does not support the call."""
-  from .functional import _native
-  if (nat := _native()) is not None and dr == 64:
-    o = nat.absorb_step(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads, dn, dv, scale, interleaved)
-    if o is not None:
-      return o
-  if not supported(q, ckv, norm_w, kv_cache, pe_cache, w, heads, dn, dr, dv, c):
-    return None
-  return absorb_step(q, ckv, norm_w, eps, cos, sin, pos, kv_cache, pe_cache, w, heads, dn, dv, scale, interleaved)
