@@ -3,11 +3,12 @@
 // The cache holds, per token, the normalised latent (C values) and the shared rotary key (R values), both
 // bf16.  The key up-projection is folded into the query and the value up-projection is applied to the
 // weighted sum, so a step has to read C + R numbers per cached token and the up-projection weights once.
-// All arithmetic is fp32 on bf16 inputs (queries folded through the up-projection stay fp32): the work is a few FMAs
-// per byte, far below the FP32 pipe's share, and what bounds the step is latency and launches.
+// All arithmetic is that of fp32 on bf16 inputs (queries folded through the up-projection and the weights of the sum stay
+// fp32, as three bf16 terms where the tensor cores take them): what bounds the step is latency and launches.
 // Written as torch operators the same step converts the whole cache and the up-projection to fp32 and
-// runs about thirty kernels per layer.  Four sequences of 1500 cached tokens, 16 heads, C = 512, us per layer: prep 4,
-// fold 4, split 22, merge 9; the torch form about 150 and the host's time for it.
+// runs about thirty kernels per layer, 150 us and the host's time for them.  A decode step of four sequences of 1500 cached
+// tokens through three layers (16 heads, C = 512, the whole model's step): 372 us with fp32 multiply-adds in the split kernel
+// and every CTA of the merge kernel merging all latent columns, 315 this way.
 //
 //   mla_prep_kernel     per sequence: rotate the queries' rotary part, normalise the new latent and rotate
 //                       the new rotary key straight into the cache
@@ -87,7 +88,8 @@ mla_prep_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__
 __global__ void __launch_bounds__(MLA_THREADS)
 mla_fold_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ w, float* __restrict__ qa, int B,
                 int H, int dn, int dv, int C) {
-  if (!chain_begin()) return;
+  chain_wait();
+  chain_launch();    // (after the wait: the split kernel reads what the kernel before this one wrote)
   __shared__ float acc_s[8][MLA_MAX_B][64];
   extern __shared__ float fold_q[];                  // [MLA_MAX_B][dn]
   const int h = blockIdx.x, c0 = blockIdx.y * 64, b0 = blockIdx.z * MLA_MAX_B;
@@ -141,81 +143,138 @@ mla_fold_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __rest
 }
 
 struct MlaSplitSmem {
-  // rows of keys are padded by 16 bytes: lanes read 16 bytes of 32 different rows without bank conflicts
-  static __host__ __device__ int key_pitch(int C) { return (C + MLA_R) * 2 + 16; }
+  // rows of queries and keys are padded by 16 bytes: 8 rows of 16 bytes at one column touch every bank once
+  static __host__ __device__ int pitch(int C) { return (C + MLA_R) * 2 + 16; }
+  static constexpr int SROW = MLA_KEYS + 8;       // floats per head in the score and weight arrays
   static __host__ __device__ int bytes(int C) {
-    return MLA_HG * (C + MLA_R) * 4 + MLA_KEYS * key_pitch(C) + MLA_KEYS * MLA_HG * 4 + 2 * MLA_HG * 4;
+    return (3 * MLA_HG + MLA_KEYS) * pitch(C) + 3 * MLA_HG * SROW * 4 + MLA_HG * 4;
   }
 };
 
+// x as three bf16 terms, x = hi + mid + lo to 2^-24; two values to a register.
+__device__ __forceinline__ void split3(float a, float b, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = pack_bf16(a, b);
+  const float2 h = unpack_bf16(hi);
+  const float ra = a - h.x, rb = b - h.y;
+  mid = pack_bf16(ra, rb);
+  const float2 m = unpack_bf16(mid);
+  lo = pack_bf16(ra - m.x, rb - m.y);
+}
+__device__ __forceinline__ void ldsm4(uint32_t addr, uint32_t* r) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t addr, uint32_t* r) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+// d += A (16 x 16) B (16 x 8), bf16 operands
+__device__ __forceinline__ void mma16816(float* d, const uint32_t* a, uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
 // Grid (ranges, head groups, B).  Keys [range * per, min(n_keys, (range + 1) * per)), per a multiple of 32.
 // part_o [B, H, ranges, C], part_ml [B, H, ranges, 2] = (running maximum in log2 units, sum).
-__global__ void __launch_bounds__(MLA_THREADS)
+//
+// Sixteen heads are one row block of mma.sync m16n8k16 (a tcgen05 tile would be seven eighths empty): scores from the
+// queries as three bf16 terms, the weighted sum from the weights as three, so that nothing of the fp32 values is lost, and
+// every 16-deep product starts from zero and is added to its sum in fp32 (the tensor core's own sums are cut, not rounded).
+// Bound by latency: the keys are asked for before the kernel in front has ended (it writes the folded queries only).
+__global__ void __launch_bounds__(MLA_THREADS, 2)
 mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__ q,
                  const __nv_bfloat16* __restrict__ kv_cache, const __nv_bfloat16* __restrict__ pe_cache,
                  long long kv_bs, long long pe_bs, float* __restrict__ part_o, float* __restrict__ part_ml, int n_keys,
                  int per, int H, int dn, int C, float scale_log2) {
-  if (!chain_begin()) return;
-  extern __shared__ uint8_t split_smem[];
-  const int D = C + MLA_R, pitch = MlaSplitSmem::key_pitch(C);
-  float* sq = reinterpret_cast<float*>(split_smem);                 // [16][D]
-  uint8_t* sk = split_smem + MLA_HG * D * 4;                        // [32][pitch]
-  float* sp = reinterpret_cast<float*>(sk + MLA_KEYS * pitch);      // [32 keys][16 heads]
-  float* s_alpha = sp + MLA_KEYS * MLA_HG;                          // [16]
+  extern __shared__ __align__(16) uint8_t split_smem[];
+  constexpr int SROW = MlaSplitSmem::SROW;
+  const int D = C + MLA_R, pitch = MlaSplitSmem::pitch(C), plane = MLA_HG * pitch;
+  uint8_t* sq = split_smem;                                         // [3 terms][16 heads][pitch]
+  uint8_t* sk = sq + 3 * plane;                                     // [32 keys][pitch]
+  float* ss = reinterpret_cast<float*>(sk + MLA_KEYS * pitch);      // [2 halves of D][16][SROW] scores
+  float* sp = ss + 2 * MLA_HG * SROW;                               // [16][SROW] weights
+  float* s_alpha = sp + MLA_HG * SROW;                              // [16]
   const int range = blockIdx.x, h0 = blockIdx.y * MLA_HG, b = blockIdx.z, ranges = gridDim.x;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // the folded queries, then the rotary parts, four values per load and nothing waiting for anything
-  // (a scalar loop over both took 20 of the kernel's 31 us)
+  const int k_begin = range * per, k_end = min(n_keys, k_begin + per);
+  const int cv = C / 8, dvec = D / 8;
+  const uint32_t sk_at = smem_u32(sk), sq_at = smem_u32(sq);
+  auto fetch_keys = [&](int k0) {                // asynchronous; keys past the range are zeros
+    for (int i = threadIdx.x; i < MLA_KEYS * dvec; i += MLA_THREADS) {
+      const int r = i / dvec, c = i - r * dvec, key = min(k0 + r, k_end - 1);
+      const void* src = c < cv ? (const void*)(kv_cache + b * kv_bs + (size_t)key * C + c * 8)
+                               : (const void*)(pe_cache + b * pe_bs + (size_t)key * MLA_R + (c - cv) * 8);
+      asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(sk_at + r * pitch + c * 16), "l"(src),
+                   "r"(k0 + r < k_end ? 16 : 0)
+                   : "memory");
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  chain_launch();
+  // The fold kernel lets this one start only after its own wait, so the caches and the rotated queries are there.
+  fetch_keys(k_begin);
+  for (int i = threadIdx.x; i < MLA_HG * (MLA_R / 4); i += MLA_THREADS) {     // the rotary parts: bf16 as they are
+    const int h = i / (MLA_R / 4), d = (i % (MLA_R / 4)) * 4;
+    uint2 u = make_uint2(0, 0);
+    if (h0 + h < H) u = *reinterpret_cast<const uint2*>(q + ((size_t)b * H + h0 + h) * (dn + MLA_R) + dn + d);
+    *reinterpret_cast<uint2*>(sq + h * pitch + (C + d) * 2) = u;
+  }
+  chain_wait();
 #pragma unroll 8
   for (int i = threadIdx.x; i < MLA_HG * (C / 4); i += MLA_THREADS) {
     const int h = i / (C / 4), d = (i % (C / 4)) * 4;
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     if (h0 + h < H) v = *reinterpret_cast<const float4*>(qa + ((size_t)b * H + h0 + h) * C + d);
-    *reinterpret_cast<float4*>(sq + h * D + d) = v;
+    uint2 hi, mid, lo;
+    split3(v.x, v.y, hi.x, mid.x, lo.x);
+    split3(v.z, v.w, hi.y, mid.y, lo.y);
+    uint8_t* at = sq + h * pitch + d * 2;
+    *reinterpret_cast<uint2*>(at) = hi;
+    *reinterpret_cast<uint2*>(at + plane) = mid;
+    *reinterpret_cast<uint2*>(at + 2 * plane) = lo;
   }
-  {
-    const int h = threadIdx.x / (MLA_R / 4), d = (threadIdx.x % (MLA_R / 4)) * 4;   // 16 heads x 16 groups of four
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (h0 + h < H) {
-      const uint2 u = *reinterpret_cast<const uint2*>(q + ((size_t)b * H + h0 + h) * (dn + MLA_R) + dn + d);
-      const float2 lo = unpack_bf16(u.x), hi = unpack_bf16(u.y);
-      v = make_float4(lo.x, lo.y, hi.x, hi.y);
-    }
-    *reinterpret_cast<float4*>(sq + h * D + C + d) = v;
-  }
-  const int k_begin = range * per, k_end = min(n_keys, k_begin + per);
-  const int hw = warp * 2;                       // this warp's two heads in the score phase
+  const int hw = warp * 2;                       // this warp's two heads in the softmax
   float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
-  const bool owner = 2 * (int)threadIdx.x < C;   // this thread's two latent columns in the sum phase
-  float acc[MLA_HG][2] = {};
-  const int cv = C / 8, dvec = D / 8;
+  const int g = lane >> 2, t = lane & 3;         // mma fragment row and column pair
+  const int nt = warp & 3, half = warp >> 2;     // score phase: eight keys, half of the contraction
+  const int ksteps = D / 32;                     // 16-deep steps per half (D is a multiple of 64: an even number)
+  const bool owner = warp * 64 < C;              // sum phase: latent columns [64 warp, 64 warp + 64)
+  float acc[8][4] = {};
   for (int k0 = k_begin; k0 < k_end; k0 += MLA_KEYS) {
-    if (k0 != k_begin) __syncthreads();          // the previous step's keys and weights are used up
-#pragma unroll 9
-    for (int i = threadIdx.x; i < MLA_KEYS * dvec; i += MLA_THREADS) {
-      const int r = i / dvec, c = i % dvec, key = k0 + r;
-      uint4 v = make_uint4(0, 0, 0, 0);
-      if (key < k_end)
-        v = c < cv ? reinterpret_cast<const uint4*>(kv_cache + b * kv_bs + (size_t)key * C)[c]
-                   : reinterpret_cast<const uint4*>(pe_cache + b * pe_bs + (size_t)key * MLA_R)[c - cv];
-      *reinterpret_cast<uint4*>(sk + r * pitch + c * 16) = v;
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
+    __syncthreads();
+    {
+      float s[4] = {};
+      const uint32_t a_at = sq_at + ((lane & 7) + ((lane >> 3) & 1) * 8) * pitch + (lane >> 4) * 16;
+      const uint32_t b_at = sk_at + (nt * 8 + (lane & 7)) * pitch + (lane >> 3) * 16;
+#pragma unroll 2
+      for (int k = half * ksteps; k < (half + 1) * ksteps; k += 2) {
+        uint32_t bb[4];
+        ldsm4(b_at + k * 32, bb);                // two steps' keys
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float d[4] = {};
+          const bool rot = (k + e) * 16 >= C;    // the rotary part has one term
+#pragma unroll
+          for (int term = 2; term >= 0; --term) {
+            if (rot && term > 0) continue;
+            uint32_t a[4];
+            ldsm4(a_at + term * plane + (k + e) * 32, a);
+            mma16816(d, a, bb[2 * e], bb[2 * e + 1]);
+          }
+#pragma unroll
+          for (int x = 0; x < 4; ++x) s[x] += d[x];
+        }
+      }
+      float* dst = ss + (half * MLA_HG + g) * SROW + nt * 8 + 2 * t;
+      *reinterpret_cast<float2*>(dst) = make_float2(s[0], s[1]);
+      *reinterpret_cast<float2*>(dst + 8 * SROW) = make_float2(s[2], s[3]);
     }
     __syncthreads();
-    float s0 = 0.f, s1 = 0.f;
-    const float* q0 = sq + hw * D;
-    const float* q1 = q0 + D;
-#pragma unroll 4
-    for (int c = 0; c < dvec; ++c) {
-      const uint4 kv = *reinterpret_cast<const uint4*>(sk + lane * pitch + c * 16);
-      const float2 a = unpack_bf16(kv.x), bb = unpack_bf16(kv.y), cc = unpack_bf16(kv.z), d = unpack_bf16(kv.w);
-      const float4 x0 = *reinterpret_cast<const float4*>(q0 + c * 8), x1 = *reinterpret_cast<const float4*>(q0 + c * 8 + 4);
-      const float4 y0 = *reinterpret_cast<const float4*>(q1 + c * 8), y1 = *reinterpret_cast<const float4*>(q1 + c * 8 + 4);
-      s0 += x0.x * a.x + x0.y * a.y + x0.z * bb.x + x0.w * bb.y + x1.x * cc.x + x1.y * cc.y + x1.z * d.x + x1.w * d.y;
-      s1 += y0.x * a.x + y0.y * a.y + y0.z * bb.x + y0.w * bb.y + y1.x * cc.x + y1.y * cc.y + y1.z * d.x + y1.w * d.y;
-    }
     const bool live = k0 + lane < k_end;
-    s0 = live ? s0 * scale_log2 : -INFINITY;
-    s1 = live ? s1 * scale_log2 : -INFINITY;
+    const float s0 = live ? (ss[hw * SROW + lane] + ss[(MLA_HG + hw) * SROW + lane]) * scale_log2 : -INFINITY;
+    const float s1 = live ? (ss[(hw + 1) * SROW + lane] + ss[(MLA_HG + hw + 1) * SROW + lane]) * scale_log2 : -INFINITY;
     float n0 = s0, n1 = s1;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -234,35 +293,57 @@ mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__
     }
     l0 = l0 * al0 + t0; l1 = l1 * al1 + t1;
     m0 = n0; m1 = n1;
-    sp[lane * MLA_HG + hw] = p0;
-    sp[lane * MLA_HG + hw + 1] = p1;
+    sp[hw * SROW + lane] = p0;
+    sp[(hw + 1) * SROW + lane] = p1;
     if (lane == 0) { s_alpha[hw] = al0; s_alpha[hw + 1] = al1; }
     __syncthreads();
     if (owner) {
+      uint32_t a[2][3][4];                       // [16 keys][term]
 #pragma unroll
-      for (int h = 0; h < MLA_HG; ++h) { acc[h][0] *= s_alpha[h]; acc[h][1] *= s_alpha[h]; }
-      const uint8_t* col = sk + threadIdx.x * 4;
-#pragma unroll 4
-      for (int r = 0; r < MLA_KEYS; ++r) {
-        const float2 v = unpack_bf16(*reinterpret_cast<const uint32_t*>(col + r * pitch));
-        const float4* pr = reinterpret_cast<const float4*>(sp + r * MLA_HG);
+      for (int ks = 0; ks < 2; ++ks)
 #pragma unroll
-        for (int h4 = 0; h4 < MLA_HG / 4; ++h4) {
-          const float4 w4 = pr[h4];
-          acc[4 * h4][0] += w4.x * v.x; acc[4 * h4][1] += w4.x * v.y;
-          acc[4 * h4 + 1][0] += w4.y * v.x; acc[4 * h4 + 1][1] += w4.y * v.y;
-          acc[4 * h4 + 2][0] += w4.z * v.x; acc[4 * h4 + 2][1] += w4.z * v.y;
-          acc[4 * h4 + 3][0] += w4.w * v.x; acc[4 * h4 + 3][1] += w4.w * v.y;
+        for (int x = 0; x < 4; ++x) {
+          const float2 w = *reinterpret_cast<const float2*>(sp + (g + (x & 1) * 8) * SROW + ks * 16 + (x >> 1) * 8 + 2 * t);
+          split3(w.x, w.y, a[ks][0][x], a[ks][1][x], a[ks][2][x]);
+        }
+      const float alg = s_alpha[g], alh = s_alpha[g + 8];
+      const uint32_t v_at = sk_at + ((lane & 7) + ((lane >> 3) & 1) * 8) * pitch + (warp * 64 + (lane >> 4) * 8) * 2;
+#pragma unroll
+      for (int n = 0; n < 8; n += 2) {
+        uint32_t v0[4], v1[4];                   // keys 0-15 and 16-31 of two column groups
+        ldsm4_t(v_at + n * 16, v0);
+        ldsm4_t(v_at + 16 * pitch + n * 16, v1);
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+          float d[4] = {}, d2[4] = {};
+#pragma unroll
+          for (int term = 2; term >= 0; --term) {
+            mma16816(d, a[0][term], v0[2 * e], v0[2 * e + 1]);
+            mma16816(d2, a[1][term], v1[2 * e], v1[2 * e + 1]);
+          }
+          acc[n + e][0] = acc[n + e][0] * alg + (d[0] + d2[0]);
+          acc[n + e][1] = acc[n + e][1] * alg + (d[1] + d2[1]);
+          acc[n + e][2] = acc[n + e][2] * alh + (d[2] + d2[2]);
+          acc[n + e][3] = acc[n + e][3] * alh + (d[3] + d2[3]);
         }
       }
+    }
+    if (k0 + MLA_KEYS < k_end) {
+      __syncthreads();                           // this step's keys and weights are used up
+      fetch_keys(k0 + MLA_KEYS);
     }
   }
   if (owner) {
 #pragma unroll
-    for (int h = 0; h < MLA_HG; ++h)
-      if (h0 + h < H)
-        *reinterpret_cast<float2*>(part_o + (((size_t)b * H + h0 + h) * ranges + range) * C + 2 * threadIdx.x) =
-            make_float2(acc[h][0], acc[h][1]);
+    for (int hh = 0; hh < 2; ++hh) {
+      const int h = h0 + g + 8 * hh;
+      if (h < H) {
+        float* dst = part_o + (((size_t)b * H + h) * ranges + range) * C + warp * 64 + 2 * t;
+#pragma unroll
+        for (int n = 0; n < 8; ++n)
+          *reinterpret_cast<float2*>(dst + n * 8) = make_float2(acc[n][2 * hh], acc[n][2 * hh + 1]);
+      }
+    }
   }
   if (lane == 0) {
     if (h0 + hw < H) {
@@ -276,14 +357,15 @@ mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__
   }
 }
 
-// Grid (H, B, slices of `rows` outputs).  Every range holds at least one key, so its sum is positive and its
-// maximum finite.  Every slice merges the ranges again: their partial sums come from L2 and the up-projection's
-// rows are spread over more SMs (18 us with one slice and one row per warp at a time).
+// Grid (H, B, slices of `rows` outputs), in clusters of `share` slices.  Every range holds at least one key, so its sum is
+// positive and its maximum finite.  The CTAs of a cluster merge C / share latent columns each and read the others' from
+// their shared memory (each merging all of them, the ranges' partial sums were read four times over.)
 __global__ void __launch_bounds__(MLA_THREADS)
 mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const __nv_bfloat16* __restrict__ w,
-                 __nv_bfloat16* __restrict__ out, int ranges, int H, int dn, int dv, int C, int rows) {
+                 __nv_bfloat16* __restrict__ out, int ranges, int H, int dn, int dv, int C, int rows, int share) {
   if (!chain_begin()) return;
   __shared__ __align__(16) float olat[MLA_MAX_C];
+  __shared__ float2 sums[MLA_THREADS];
   extern __shared__ float merge_w[];             // [ranges]
   const int h = blockIdx.x, b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -305,19 +387,41 @@ mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ par
     for (int r = lane; r < ranges; r += 32) merge_w[r] *= inv;
   }
   __syncthreads();
-  if (2 * (int)threadIdx.x < C) {
-    const float* po = part_o + ((size_t)b * H + h) * ranges * C + 2 * threadIdx.x;
+  const int rank = share > 1 ? (int)cluster_ctarank() : 0;
+  const int cols = C / share, pairs = cols / 2;      // this CTA's columns, two to a thread
+  const int groups = MLA_THREADS / pairs;            // threads with the same columns take every groups-th range
+  const int pr = threadIdx.x % pairs, grp = threadIdx.x / pairs;
+  {
     float x = 0.f, y = 0.f;
+    if (grp < groups) {
+      const float* po = part_o + ((size_t)b * H + h) * ranges * C + rank * cols + 2 * pr;
 #pragma unroll 8
-    for (int r = 0; r < ranges; ++r) {
-      const float2 v = *reinterpret_cast<const float2*>(po + (size_t)r * C);
-      x += merge_w[r] * v.x;
-      y += merge_w[r] * v.y;
+      for (int r = grp; r < ranges; r += groups) {
+        const float2 v = *reinterpret_cast<const float2*>(po + (size_t)r * C);
+        x += merge_w[r] * v.x;
+        y += merge_w[r] * v.y;
+      }
     }
-    olat[2 * threadIdx.x] = x;
-    olat[2 * threadIdx.x + 1] = y;
+    sums[threadIdx.x] = make_float2(x, y);
+    __syncthreads();
+    if ((int)threadIdx.x < pairs) {
+      for (int k = 1; k < groups; ++k) { x += sums[k * pairs + pr].x; y += sums[k * pairs + pr].y; }
+      olat[rank * cols + 2 * pr] = x;
+      olat[rank * cols + 2 * pr + 1] = y;
+    }
   }
-  __syncthreads();
+  if (share > 1) {
+    cluster_sync_all();
+    for (int c = threadIdx.x; c < C; c += MLA_THREADS)
+      if (c / cols != rank) {
+        float v;
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(map_to_cta(smem_u32(olat + c), c / cols)) : "memory");
+        olat[c] = v;
+      }
+    cluster_sync_all();                              // (nobody leaves or reads on while a neighbour still reads here)
+  } else {
+    __syncthreads();
+  }
   // a warp takes four rows at a time: their loads are in flight together
   const uint4* wv = reinterpret_cast<const uint4*>(w + ((size_t)h * (dn + dv) + dn) * C);
   const int cv = C / 8;
@@ -401,8 +505,23 @@ extern "C" int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, cons
   chain(mla_split_kernel, dim3(ranges, (H + MLA_HG - 1) / MLA_HG, B), MLA_THREADS, MlaSplitSmem::bytes(C), stream,
         qa, qb, kc, pc, kv_bs, pe_bs, part_o, part_ml, n_keys, per, H, dn, C, scale * 1.4426950408889634f);
   const int rows = 32;     // one pass of the eight warps
-  chain(mla_merge_kernel, dim3(H, B, (dv + rows - 1) / rows), MLA_THREADS, ranges * 4, stream,
-        part_o, part_ml, wb, reinterpret_cast<__nv_bfloat16*>(out), ranges, H, dn, dv, C, rows);
+  const int slices = (dv + rows - 1) / rows, share = slices % 4 == 0 ? 4 : slices % 2 == 0 ? 2 : 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(H, B, slices);
+  cfg.blockDim = dim3(MLA_THREADS, 1, 1);
+  cfg.dynamicSmemBytes = ranges * 4;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = 1;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = share;
+  cfg.attrs = attr;
+  cfg.numAttrs = 2;
+  cudaLaunchKernelEx(&cfg, mla_merge_kernel, (const float*)part_o, (const float*)part_ml, wb, reinterpret_cast<__nv_bfloat16*>(out),
+                     ranges, H, dn, dv, C, rows, share);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }

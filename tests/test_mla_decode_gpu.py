@@ -79,3 +79,25 @@ def test_values_wider_than_the_kernel_takes(cuda_lib):
   with torch.no_grad():
     y = eng._attention(0, eng.model.model.layers[0].self_attn, x, 0, x, lambda: torch.zeros(2, dtype=torch.int32, device="cuda"))
   assert y.shape == x.shape and bool(torch.isfinite(y).all())
+
+
+@pytest.mark.parametrize("heads,c,start", [(16, 512, 40), (17, 64, 100), (3, 192, 700), (32, 448, 64)])
+def test_widths_and_precision_of_the_split(cuda_lib, heads, c, start):
+  """Other latent widths and head counts, against 64 bits: what the bf16 result's rounding leaves, for scores of +-20."""
+  torch.manual_seed(c)
+  b, dn, dv, n = 2, 128, 128, start + 1
+  q = torch.randn(b, 1, heads * (dn + 64), device="cuda", dtype=torch.bfloat16) * 3
+  ckv = torch.randn(b, 1, c + 64, device="cuda", dtype=torch.bfloat16)
+  nw = torch.ones(c, device="cuda", dtype=torch.bfloat16)
+  cos, sin = torch.ones(4096, 32, device="cuda"), torch.zeros(4096, 32, device="cuda")
+  kv = torch.randn(b, 1024, c, device="cuda", dtype=torch.bfloat16)
+  pe = torch.randn(b, 1024, 64, device="cuda", dtype=torch.bfloat16)
+  w = (torch.randn(heads * (dn + dv), c, device="cuda") / c ** 0.5).to(torch.bfloat16)
+  with torch.no_grad():
+    got = mla_decode.absorb_step(q.clone(), ckv, nw, 1e-6, cos, sin, start, kv, pe, w, heads, dn, dv, 0.1, True)
+  wd = w.double().view(heads, dn + dv, c)
+  qd = q.double().view(b, heads, dn + 64)
+  s = (torch.einsum("bhd,hdc,btc->bht", qd[..., :dn], wd[:, :dn], kv[:, :n].double())
+       + torch.einsum("bhr,btr->bht", qd[..., dn:], pe[:, :n].double())) * 0.1
+  o = torch.einsum("bht,btc,hjc->bhj", s.softmax(-1), kv[:, :n].double(), wd[:, dn:]).reshape(b, 1, -1)
+  assert bool(((got.double() - o).abs() <= 2.0 ** -8 * o.abs() + 2e-5 * o.abs().max()).all()), (got.double() - o).abs().max()
