@@ -147,9 +147,9 @@ struct Weights {
 
 void gemm(const Tensor& a, const Tensor& b, const Tensor& c, int64_t m, int64_t n, int64_t k, bool a_mn, bool b_mn, int epi,
           const Tensor& aux = Tensor(), const Tensor& c2 = Tensor()) {
-  const int64_t n_out = epi == TPB_EPI_SWIGLU ? n / 2 : n;
+  const int64_t n_out = epi == TPB_EPI_SWIGLU ? n / 2 : epi == TPB_EPI_SWIGLU_BWD ? 2 * n : n;
   check(tpb_gemm_bf16(cptr(a), cptr(b), mptr(c), (int)m, (int)n, (int)k, a_mn ? m : k, b_mn ? n : k, n_out, a_mn, b_mn, epi,
-                      1.f, cptr(aux), aux.defined() ? n : 0, mptr(c2), c2.defined() ? n : 0, 0, stream()),
+                      1.f, cptr(aux), aux.defined() ? aux.size(-1) : 0, mptr(c2), c2.defined() ? n : 0, 0, stream()),
         "gemm");
 }
 
@@ -288,6 +288,80 @@ py::object linear_swiglu(py::handle x_, py::handle gate_, py::handle up_) {
       y = empty_as(x, with_last(x, f));
       gemm(x, w.t[0], y, rows, 2 * f, w.k, false, false, TPB_EPI_SWIGLU);
     }
+  }
+  return py::cast(y);
+}
+
+// ------------------------------------------------------------------------------------------- the whole MLP
+// y = (silu(x Wg^T) * (x Wu^T)) Wd^T (+ residual).  One node, so that the gradient of the activation needs no tensor: it
+// becomes that of gate and up inside the down projection's input gradient, where that product is not a split one.
+struct SwigluMlpFn : Function<SwigluMlpFn> {
+  static Tensor forward(AutogradContext* ctx, const Tensor& x, const OptTensor& residual, const Tensor& wg, const Tensor& wu,
+                        const Tensor& wd) {
+    const int64_t k = wg.size(1), f = wg.size(0), n = wd.size(0), rows = x.numel() / k;
+    Tensor gu = empty_as(x, {rows, 2 * f}), act = empty_as(x, {rows, f}), y = empty_as(x, with_last(x, n));
+    gemm(x, wg, act, rows, 2 * f, k, false, false, TPB_EPI_SWIGLU, Tensor(), gu);
+    gemm(act, wd, y, rows, n, f, false, false, residual ? TPB_EPI_BF16_RES : TPB_EPI_BF16, residual ? *residual : Tensor());
+    ctx->save_for_backward({x, gu, act, wg, wu, wd});
+    ctx->saved_data["res"] = residual.has_value();
+    return y;
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list grads) {
+    const variable_list s = ctx->get_saved_variables();
+    const Tensor &x = s[0], &gu = s[1], &act = s[2], *w = &s[3], &wd = s[5];
+    const bool res = ctx->saved_data["res"].toBool();
+    const Tensor dy = grads[0].contiguous();
+    TORCH_CHECK(plain(dy), "swiglu_mlp: gradient of an unexpected kind");
+    const int64_t k = w[0].size(1), f = w[0].size(0), n = wd.size(0), rows = gu.size(0);
+    const int at = res ? 2 : 1;    // edge of the gate weight
+    variable_list out(5);
+    if (res) out[1] = grads[0];
+    const bool up = ctx->needs_input_grad(at) || ctx->needs_input_grad(at + 1), in = ctx->needs_input_grad(0);
+    if (in || up) {
+      Tensor dgu = empty_as(gu, gu.sizes());
+      if (tpb_gemm_swiglu_bwd_pays((int)rows, (int)f, (int)n)) {
+        gemm(dy, wd, dgu, rows, f, n, false, true, TPB_EPI_SWIGLU_BWD, gu);
+      } else {
+        Tensor dact = empty_as(act, act.sizes());
+        gemm(dy, wd, dact, rows, f, n, false, true, TPB_EPI_BF16);
+        check(tpb_swiglu_bwd(cptr(dact), cptr(gu), mptr(dgu), (int)rows, (int)f, stream()), "swiglu_bwd");
+      }
+      if (in) {
+        out[0] = empty_as(x, x.sizes());
+        gemm(dgu, w[0], out[0], rows, k, 2 * f, false, true, TPB_EPI_BF16);
+      }
+      if (up) {
+        const variable_list dw = weight_grads(w, 2, dgu, x, rows, 2 * f, k);
+        out[2] = dw[0];
+        out[3] = dw[1];
+      }
+    }
+    if (ctx->needs_input_grad(at + 2)) out[4] = weight_grads(&wd, 1, dy, act, rows, n, f)[0];
+    return out;
+  }
+};
+
+py::object swiglu_mlp(py::handle x_, py::handle gate_, py::handle up_, py::handle down_, py::handle res_) {
+  Tensor x, residual;
+  Weights w, d;
+  if (!unobserved() || !unpack(x_, x) || !unpack(res_, residual) || !plain_rows(x) || !w.add(gate_.ptr()) || !w.add(up_.ptr()) ||
+      !d.add(down_.ptr()))
+    return py::none();
+  const int64_t f = w.t[0].size(0), n = d.rows, rows = x.numel() / x.size(-1);
+  if (w.t[1].size(0) != f || d.k != f || f % 8 || w.k % 8 || n % 8 || x.size(-1) != w.k || !small(rows) || !small(2 * f) || !small(n) ||
+      x.get_device() != w.t[0].get_device() || x.get_device() != d.t[0].get_device())
+    return py::none();
+  if (residual.defined() && (!plain_rows(residual) || residual.numel() != rows * n || residual.size(-1) != n ||
+                             residual.get_device() != x.get_device()))
+    return py::none();
+  // (without gradients to record there is nothing to join)
+  if (!(at::GradMode::is_enabled() && (recording(x) || w.grads || d.grads || (residual.defined() && recording(residual)))) ||
+      w.collected || d.collected || (residual.defined() && residual.dim() != x.dim()))
+    return py::none();
+  Tensor y;
+  {
+    py::gil_scoped_release nogil;
+    y = SwigluMlpFn::apply(x, residual.defined() ? OptTensor(residual) : OptTensor(), w.t[0], w.t[1], d.t[0]);
   }
   return py::cast(y);
 }
@@ -851,6 +925,7 @@ PYBIND11_MODULE(_tpb_torch, m) {
   m.def("launch_count", []() { return g_launches.load(); });
   m.def("linear", &linear);
   m.def("linear_swiglu", &linear_swiglu);
+  m.def("swiglu_mlp", &swiglu_mlp);
   m.def("rms_norm", &rms_norm);
   m.def("rms_norm_residual", &rms_norm_residual);
   m.def("rope", &rope);

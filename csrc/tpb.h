@@ -19,6 +19,7 @@ enum {
   TPB_EPI_RS_BF16 = 6,   // reduce-scatter: red.add alpha * acc into the owner's bf16 shard over P2P
   TPB_EPI_AR_BF16 = 7,   // all-reduce: C is the NVSwitch multicast address of a zeroed symmetric buffer;
                          // multimem.red adds alpha * acc (+ aux, if given) into every rank's copy
+  TPB_EPI_SWIGLU_BWD = 8,  // acc = gradient of silu(g) * u, aux[M, 2N] = [g | u]: C[M, 2N](bf16) = [dg | du]
 };
 
 // Status block: {code, site, block, thread}; code 0 = no kernel ever timed out.
@@ -35,6 +36,8 @@ int tpb_gemm_bf16(const void* A, const void* B, void* C, int M, int N, int K, lo
                   long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha,
                   const void* aux, long long ldaux, void* c2, long long ldc2, int max_ctas,
                   void* stream);
+// Whether TPB_EPI_SWIGLU_BWD is worth more than a split contraction at these sizes.
+int tpb_gemm_swiglu_bwd_pays(int M, int N, int K);
 // The same with one more factor, *scale in device memory (null: 1), when the result is written.
 int tpb_gemm_scaled_bf16(const void* A, const void* B, void* C, int M, int N, int K, long long lda,
                          long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha, const float* scale,
@@ -104,6 +107,7 @@ int tpb_cast_f32_to_bf16(const float* src, void* dst, long long n, float scale, 
 //          B (and B2 for the "up" half of a SwiGLU epilogue) hold E matrices b_expert_stride apart.
 //  mode 2: per-expert wgrad C[e] = A[:, rows of e] * B[:, rows of e]^T with both operands stored
 //          row-major over the grouped rows (a_mn = b_mn = 1); k_offsets[E+1] are 64-aligned.
+//  TPB_EPI_SWIGLU_BWD takes [g | u] through c2.
 // row_align: rows to which expert segments are padded in mode 1 (128, or 256: CTA-pair tiles may be used).
 int tpb_grouped_gemm_bf16(const void* A, const void* B, const void* B2, void* C, int M, int N, int K, int E,
                           long long lda, long long ldb, long long b_expert_stride, long long ldc, int a_mn, int b_mn,

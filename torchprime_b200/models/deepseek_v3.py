@@ -53,8 +53,7 @@ class DeepseekV3MLP(nn.Module):
   def forward(self, x, residual=None, partial=False):
     """``partial`` (tensor parallel only): return this rank's partial sum, the caller reduces."""
     if self.tp_group is None:
-      act = ops.linear_swiglu(x, self.gate_proj.weight, self.up_proj.weight)
-      return ops.linear(act, self.down_proj.weight, residual=residual)
+      return ops.swiglu_mlp(x, self.gate_proj.weight, self.up_proj.weight, self.down_proj.weight, residual)
     act = ops.linear_swiglu(copy_to_tp(x, self.tp_group), self.gate_proj.weight, self.up_proj.weight)
     y = ops.linear(act, self.down_proj.weight)
     if partial:

@@ -66,8 +66,7 @@ class LlamaMLP(nn.Module):
         act = ops.linear_swiglu(x, self.gate_proj.weight, self.up_proj.weight)
         y = reduce_from_tp(ops.linear(act, self.down_proj.weight), self.tp_group)
         return y if residual is None else y + residual
-      act = ops.linear_swiglu(x, self.gate_proj.weight, self.up_proj.weight)
-      return ops.linear(act, self.down_proj.weight, residual=residual)
+      return ops.swiglu_mlp(x, self.gate_proj.weight, self.up_proj.weight, self.down_proj.weight, residual)
 
 
 def _fused_reducer(module, x, n_out: int, k_in: int, n_col: int):

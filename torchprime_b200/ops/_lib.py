@@ -19,6 +19,7 @@ _lib = None
 _native = None      # the operators of csrc/torch_ops.cpp, loaded with the library
 
 EPI_BF16, EPI_F32, EPI_F32_ACC, EPI_BF16_ACC, EPI_BF16_RES, EPI_SWIGLU = range(6)
+EPI_SWIGLU_BWD = 8
 EPI_RS_BF16, EPI_AR_BF16 = 6, 7     # reduce-scatter / all-reduce epilogues of the fused collective GEMMs
 
 _STATUS_NAMES = {

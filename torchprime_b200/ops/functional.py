@@ -417,6 +417,15 @@ def linear_swiglu(x, w_gate, w_up, tp_reduce_grad=None):
   return F.silu(F.linear(x, w_gate)) * F.linear(x, w_up)
 
 
+def swiglu_mlp(x, w_gate, w_up, w_down, residual=None):
+  """linear(linear_swiglu(x, w_gate, w_up), w_down, residual=residual), as one autograd node where it can be."""
+  if (nat := _native()) is not None:
+    y = nat.swiglu_mlp(x, w_gate, w_up, w_down, residual)
+    if y is not None:
+      return y
+  return linear(linear_swiglu(x, w_gate, w_up), w_down, residual=residual)
+
+
 # --------------------------------------------------------------------------- norm
 def _norm_wgrad(w, dw_f32):
   """Deliver an fp32 norm-weight gradient: into main_grad if present, else return it."""

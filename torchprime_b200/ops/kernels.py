@@ -9,13 +9,13 @@ from __future__ import annotations
 import torch
 
 from . import _debug, _lib
-from ._lib import (EPI_BF16, EPI_BF16_ACC, EPI_BF16_RES, EPI_F32, EPI_F32_ACC, EPI_SWIGLU, check, lib, ptr,
+from ._lib import (EPI_BF16, EPI_BF16_ACC, EPI_BF16_RES, EPI_F32, EPI_F32_ACC, EPI_SWIGLU, EPI_SWIGLU_BWD, check, lib, ptr,
                    stream_ptr)
 
 __all__ = [
   "gemm", "rmsnorm_fwd", "rmsnorm_bwd", "rope_", "swiglu_fwd", "swiglu_bwd", "ce_fwd_bwd_", "adamw_",
   "sumsq_", "clip_coef_", "embedding_fwd", "embedding_bwd_", "cast_f32_to_bf16_",
-  "EPI_BF16", "EPI_F32", "EPI_F32_ACC", "EPI_BF16_ACC", "EPI_BF16_RES", "EPI_SWIGLU",
+  "EPI_BF16", "EPI_F32", "EPI_F32_ACC", "EPI_BF16_ACC", "EPI_BF16_RES", "EPI_SWIGLU", "EPI_SWIGLU_BWD",
 ]
 
 
@@ -42,7 +42,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, epi=EPI_BF16, alpha=1.0, aux
   r0, r1, ldb = _row_major_2d(b, "b")
   N, Kb = (r1, r0) if b_mn else (r0, r1)
   assert K == Kb, f"contraction mismatch {K} vs {Kb}"
-  n_out = N // 2 if epi == EPI_SWIGLU else N
+  n_out = N // 2 if epi == EPI_SWIGLU else 2 * N if epi == EPI_SWIGLU_BWD else N
   if out is None:
     assert epi not in (EPI_F32_ACC, EPI_BF16_ACC), "accumulating epilogues need `out`"
     dt = torch.float32 if epi == EPI_F32 else torch.bfloat16
@@ -52,7 +52,7 @@ def gemm(a, b, *, a_mn=False, b_mn=False, out=None, epi=EPI_BF16, alpha=1.0, aux
   assert out.dtype == want, f"epilogue {epi} writes {want}, out is {out.dtype}"
   ldc = out.stride(0) if M > 1 else max(out.stride(0), n_out)
   ldaux = 0
-  if epi == EPI_BF16_RES:
+  if epi in (EPI_BF16_RES, EPI_SWIGLU_BWD):      # (the latter: aux = [gate | up], the result its gradient)
     assert aux is not None and aux.shape == out.shape and aux.stride(1) == 1 and aux.dtype == torch.bfloat16
     ldaux = aux.stride(0) if M > 1 else max(aux.stride(0), n_out)
   ldc2 = 0

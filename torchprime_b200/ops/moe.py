@@ -293,16 +293,17 @@ def grouped_gemm_rows(a, b, plan: DispatchPlan, *, b_mn: bool, b2=None, epi=_lib
                       n_total=None):
   """out[rows of e] = a[rows of e] @ B[e]^T.  ``b``: [E, N, K] (``b_mn=False``) or [E, K, N]
   (``b_mn=True``).  With ``epi=EPI_SWIGLU``: ``b`` = gate, ``b2`` = up (or ``b`` holds both
-  halves along N when ``b2`` is None).  With other epilogues ``b2`` continues ``b`` along K: ``a`` then
-  has 2K columns."""
+  halves along N when ``b2`` is None).  With ``epi=EPI_SWIGLU_BWD``: ``c2`` = [gate | up] before the activation,
+  and the result is their gradient.  With other epilogues ``b2`` continues ``b`` along K: ``a`` then has 2K columns."""
   m, k = a.shape
   e = b.shape[0]
   n_one = b.shape[2] if b_mn else b.shape[1]
   swiglu = epi == _lib.EPI_SWIGLU
   n = n_total if n_total is not None else (2 * n_one if (swiglu and b2 is not None) else n_one)
-  n_out = n // 2 if swiglu else n
+  n_out = n // 2 if swiglu else 2 * n if epi == _lib.EPI_SWIGLU_BWD else n
   if out is None:
     out = torch.empty(m, n_out, dtype=torch.bfloat16, device=a.device)
+  assert epi != _lib.EPI_SWIGLU_BWD or (c2 is not None and c2.shape == (m, n_out) and c2.stride(1) == 1)
   assert a.stride(1) == 1 and b.is_contiguous() and (b2 is None or b2.is_contiguous())
   ldb = b.stride(1)
   rc = lib().tpb_grouped_gemm_bf16(ptr(a), ptr(b), ptr(b2), ptr(out), m, n, k, e, a.stride(0), ldb, b.stride(0),
@@ -374,7 +375,6 @@ class _GroupedMLPFn(torch.autograd.Function):
 
   @staticmethod
   def backward(ctx, dy):
-    from . import kernels as kk
     x, weights, w_gate, w_up, w_down, xg, gu, act, rows = ctx.saved_tensors
     plan, fused = ctx.plan, ctx.fused
     dy = dy.contiguous()
@@ -384,9 +384,8 @@ class _GroupedMLPFn(torch.autograd.Function):
     row_scale = flat_w[plan.src_pair].contiguous()          # -1 (padding) picks the appended zero
     d_rows = gather_rows(dy, plan.src_row, row_scale)
     # down projection: rows = act @ Wd[e]  (Wd [E, F, D])
-    dact = grouped_gemm_rows(d_rows, w_down, plan, b_mn=False)
+    dgu = grouped_gemm_rows(d_rows, w_down, plan, b_mn=False, epi=_lib.EPI_SWIGLU_BWD, c2=gu)
     g_down = _deliver_wgrad(w_down, lambda out, acc: grouped_gemm_wgrad(act, d_rows, plan, out, acc))
-    dgu = kk.swiglu_bwd(dact, gu)
     if fused:
       d_xg = grouped_gemm_rows(dgu, w_gate, plan, b_mn=False)
       g_gate = _deliver_wgrad(w_gate, lambda out, acc: grouped_gemm_wgrad(xg, dgu, plan, out, acc))
