@@ -725,6 +725,60 @@ py::object latent_split(py::handle x_, int64_t c) {
   return py::make_tuple(y[0], y[1]);
 }
 
+// The same with the rotary key rotated on the way (functional.latent_split_rope).
+variable_list latent_rope_now(const Tensor& x, const Tensor& cos, const Tensor& sin, const Tensor& pos, int64_t c, int64_t seq,
+                              bool interleaved) {
+  const int64_t dr = x.size(-1) - c;
+  Tensor lat = empty_as(x, with_last(x, c)), rot = empty_as(x, with_last(x, dr));
+  check(tpb_latent_split(cptr(x), mptr(lat), mptr(rot), static_cast<const float*>(cptr(cos)), static_cast<const float*>(cptr(sin)),
+                         iptr(pos), x.numel() / x.size(-1), (int)seq, (int)c, (int)dr, interleaved, stream()),
+        "latent_split");
+  return {lat, rot};
+}
+
+struct LatentRopeFn : Function<LatentRopeFn> {
+  static variable_list forward(AutogradContext* ctx, const Tensor& x, const Tensor& cos, const Tensor& sin, const OptTensor& pos,
+                               int64_t c, int64_t seq, bool interleaved) {
+    ctx->save_for_backward({cos, sin, get(pos)});
+    ctx->saved_data["a"] = std::vector<int64_t>{seq, interleaved};
+    return latent_rope_now(x, cos, sin, get(pos), c, seq, interleaved);
+  }
+  static variable_list backward(AutogradContext* ctx, variable_list g) {
+    const variable_list s = ctx->get_saved_variables();
+    const auto a = ctx->saved_data["a"].toIntVector();
+    const Tensor dlat = g[0].contiguous(), drot = g[1].contiguous();
+    TORCH_CHECK(plain(dlat) && plain(drot), "latent_split: gradient of an unexpected kind");
+    const int64_t c = dlat.size(-1), dr = drot.size(-1);
+    Tensor dx = empty_as(dlat, with_last(dlat, c + dr));
+    check(tpb_latent_join(cptr(dlat), cptr(drot), mptr(dx), static_cast<const float*>(cptr(s[0])),
+                          static_cast<const float*>(cptr(s[1])), iptr(s[2]), dlat.numel() / c, (int)a[0], (int)c, (int)dr, a[1] != 0,
+                          stream()),
+          "latent_join");
+    variable_list out(7);
+    out[0] = dx;
+    return out;
+  }
+};
+
+py::object latent_split_rope(py::handle x_, int64_t c, py::handle cos_, py::handle sin_, int64_t seq, py::handle pos_,
+                             bool interleaved) {
+  Tensor x, cos, sin, pos;
+  if (!unobserved() || !unpack(x_, x) || !unpack(cos_, cos) || !unpack(sin_, sin) || !unpack(pos_, pos) || !plain_rows(x) ||
+      !plain_rows(cos, at::kFloat) || !plain_rows(sin, at::kFloat) || recording(cos) || recording(sin) || !aligned(x))
+    return py::none();
+  const int64_t dr = x.size(-1) - c, tokens = x.numel() / x.size(-1);
+  if (c < 8 || c % 8 || dr < 16 || dr % 16 || cos.size(-1) != dr / 2 || sin.size(-1) != dr / 2 || seq < 1 || !small(tokens) ||
+      (pos.defined() && (!plain_rows(pos, at::kInt) || pos.numel() != tokens)))
+    return py::none();
+  variable_list y;
+  {
+    py::gil_scoped_release nogil;
+    if (at::GradMode::is_enabled() && recording(x)) y = LatentRopeFn::apply(x, cos, sin, some(pos), c, seq, interleaved);
+    else y = latent_rope_now(x, cos, sin, pos, c, seq, interleaved);
+  }
+  return py::make_tuple(y[0], y[1]);
+}
+
 variable_list mla_pack_now(const Tensor& kv, const Tensor& rot, int64_t heads, int64_t dn, int64_t dv) {
   const int64_t b = rot.size(0), s = rot.size(1), dr = rot.size(2);
   Tensor k = empty_as(kv, {b, s, heads, dn + dr}), v = empty_as(kv, {b, s, heads, dv});
@@ -932,6 +986,7 @@ PYBIND11_MODULE(_tpb_torch, m) {
   m.def("attention_qkv", &attention_qkv);
   m.def("attention", &attention);
   m.def("latent_split", &latent_split);
+  m.def("latent_split_rope", &latent_split_rope);
   m.def("mla_pack", &mla_pack);
   m.def("embedding", &embedding);
   m.def("absorb_supported", &absorb_supported);

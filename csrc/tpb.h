@@ -249,6 +249,12 @@ int tpb_mla_pack(const void* kv, const void* rot, long long rot_ld, void* k, voi
 int tpb_mla_unpack(const void* dk, const void* dv_, void* dkv, void* drot, long long tokens, int H, int dn, int dr, int dv,
                    void* stream);
 
+// [latent | rotary key] rows into two dense matrices, the key rotated; and the gradient of that (mla_pack.cu)
+int tpb_latent_split(const void* ckv, void* lat, void* rot, const float* cosT, const float* sinT, const int* pos,
+                     long long tokens, int seq_len, int c, int dr, int interleaved, void* stream);
+int tpb_latent_join(const void* dlat, const void* drot, void* dckv, const float* cosT, const float* sinT, const int* pos,
+                    long long tokens, int seq_len, int c, int dr, int interleaved, void* stream);
+
 // gradient of tpb_router_topk's weights (dw [tokens, K]) and scores (dscores [tokens, E]), either may be null
 int tpb_router_bwd(const void* logits, int logits_is_bf16, const int* idx, const float* dw, const float* dscores,
                    void* dlogits, int tokens, int E, int K, int mode, int norm_topk, float scale, void* stream);

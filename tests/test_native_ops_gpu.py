@@ -93,6 +93,15 @@ def _latent():
   return (lat, rot), [x]
 
 
+def _latent_rope(pos, interleaved):
+  def call():
+    x = _r(2, 30, 96 + 64, grad=True)
+    cos, sin = _tables(40, 32)
+    p = (torch.arange(60, device="cuda") * 7 % 40).to(torch.int32) if pos else None
+    return ops.latent_split_rope(x * 1, 96, cos, sin, 30, pos=p, interleaved=interleaved), [x]
+  return call
+
+
 def _pack():
   kv, rot = _r(2, 21, 3 * (64 + 128), grad=True), _r(2, 21, 64, grad=True)
   return ops.mla_pack(kv, rot, 3, 64, 128), [kv, rot]
@@ -130,6 +139,8 @@ CALLS = {
   "attention segments": _attn(192, 300, 300, seg=True),
   "attention cap": _attn(128, 140, 140, softcap=20.0),
   "latent": _latent,
+  "latent, rotated": _latent_rope(False, True),
+  "latent, rotated halves": _latent_rope(True, False),
   "pack": _pack,
 }
 

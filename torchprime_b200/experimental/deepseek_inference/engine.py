@@ -79,9 +79,7 @@ class DeepseekInferenceEngine:
     pos = positions()
     q = ops.rope_slices(q, self.cos, self.sin, h, dr, s, col0=dn, head_stride=dn + dr, pos=pos,
                         interleaved=attn.rope_interleave)
-    ckv = ops.rope_slices(ckv, self.cos, self.sin, 1, dr, s, col0=c, head_stride=dr, pos=pos,
-                          interleaved=attn.rope_interleave)
-    latent, k_rot = ops.latent_split(ckv, c)
+    latent, k_rot = ops.latent_split_rope(ckv, c, self.cos, self.sin, s, pos=pos, interleaved=attn.rope_interleave)
     latent = norm(latent)
     q4 = q.view(b, s, h, dn + dr)
 

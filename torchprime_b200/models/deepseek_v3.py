@@ -196,9 +196,8 @@ class DeepseekV3Attention(nn.Module):
       q = ops.rope_slices(q, rope_cos, rope_sin, h, dr, s, col0=dn, head_stride=dn + dr, pos=position_ids,
                           interleaved=self.rope_interleave)
       ckv = ops.linear(x, self.kv_a_proj_with_mqa.weight, bias=self.kv_a_proj_with_mqa.bias)
-      ckv = ops.rope_slices(ckv, rope_cos, rope_sin, 1, dr, s, col0=self.kv_lora_rank, head_stride=dr,
-                            pos=position_ids, interleaved=self.rope_interleave)
-      k_lat, k_rot = ops.latent_split(ckv, self.kv_lora_rank)
+      k_lat, k_rot = ops.latent_split_rope(ckv, self.kv_lora_rank, rope_cos, rope_sin, s, pos=position_ids,
+                                           interleaved=self.rope_interleave)
       kv = ops.linear(to_tp(self.kv_a_layernorm(k_lat)), self.kv_b_proj.weight)
       k, v = ops.mla_pack(kv, to_tp(k_rot), h, dn, dv)
       q4 = q.view(b, s, h, dn + dr)

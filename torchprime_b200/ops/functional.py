@@ -786,6 +786,17 @@ def latent_split(ckv, c):
   return ckv[..., :c].contiguous(), ckv[..., c:]
 
 
+def latent_split_rope(ckv, c, cos_half, sin_half, seq_len, pos=None, interleaved=False):
+  """The latent ckv[..., :c] and the rotary key ckv[..., c:], the key rotated.  ``ckv`` may be overwritten."""
+  if (nat := _native()) is not None and (pos is None or not _debug.bounds_enabled()):
+    both = nat.latent_split_rope(ckv, c, cos_half, sin_half, seq_len, pos, interleaved)
+    if both is not None:
+      return both
+  dr = ckv.shape[-1] - c
+  return latent_split(rope_slices(ckv, cos_half, sin_half, 1, dr, seq_len, col0=c, head_stride=dr, pos=pos,
+                                  interleaved=interleaved), c)
+
+
 class _MlaPackFn(torch.autograd.Function):
   @staticmethod
   def forward(ctx, kv, rot, heads, dn, dv):
