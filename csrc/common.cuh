@@ -61,9 +61,11 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 // (once all of that one's CTAs have called chain_launch or ended), and everything it does before chain_wait overlaps.
 // chain_wait returns when the kernel before has ended and its writes are visible; every CTA of a chained kernel calls it
 // before it touches global memory, reads or writes.  A kernel that allocates tensor memory calls chain_launch after the
-// allocation: the next kernel's CTAs would otherwise take the columns that this one still waits for.  Both do nothing in a
-// kernel launched the ordinary way.  (A kernel boundary otherwise costs 2 to 3 us of drained SMs, as much as the kernels of
-// a decode step run: 36 launches of a decode step over a short cache 384 -> 307 us, decoder layer of 3 tokens 119 -> 103.)
+// allocation: the next kernel's CTAs would otherwise take the columns that this one still waits for.  chain_launch lets the
+// next kernel in however this one was launched (that the next one is chained is what counts), so a kernel that waits for
+// anything but the stream in front of it (a shard's flag, another GPU) must not call it: the next kernel's CTAs would fill
+// the SMs and keep out whatever is to end that wait.  chain_wait does nothing in a kernel launched the ordinary way.
+// (A kernel boundary otherwise costs 2 to 3 us of drained SMs, as much as the kernels of a decode step run: 36 launches of a decode step over a short cache 384 -> 307 us, decoder layer of 3 tokens 119 -> 103.)
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void chain_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

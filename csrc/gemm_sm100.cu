@@ -52,6 +52,7 @@ struct GemmParams {
   const float* alpha_dev;   // one more factor, in device memory (the gradient of a loss), or null
   int epi;
   int group_m;       // rasterisation: m-tiles per group
+  int chained;       // launched chained, and the next kernel may be; 0 where another GPU or a copy ends a wait of this one
   int* status;
   // Grouped (mixture-of-experts) modes.  0: dense.
   // 1: rows of A/C are grouped by expert in 128-row aligned segments; tile_expert[m_tile] is the
@@ -420,7 +421,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   if (PAIR) cluster_sync_all();   // the peer's barriers exist before anything signals them
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  chain_launch();
+  if (p.chained) chain_launch();
   chain_wait();
 
   if (warp == 0) {
@@ -988,7 +989,9 @@ int make_tmap_out(CUtensorMap* map, const void* ptr, uint64_t cols, uint64_t row
                   uint64_t plane_elems, int elem_bytes);
 int sm_count();  // runtime.cu
 
-// Kernels that exchange data with other GPUs are launched the ordinary way.
+// Kernels that exchange data with other GPUs are launched the ordinary way and let no kernel in behind them: CTAs of the
+// next one, waiting, would fill the SMs, and the kernel that publishes a shard's flag could not start until the wait for
+// that flag ran out.
 static bool chainable(const GemmParams& p) { return p.ag_world == 0 && p.rs_world == 0 && p.epi != TPB_EPI_AR_BF16; }
 
 template <bool A_MN, bool B_MN>
@@ -1001,7 +1004,7 @@ cudaError_t launch_gemm(const CUtensorMap& ta, const CUtensorMap& tb, const CUte
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (chainable(p)) return chain(gemm_kernel<A_MN, B_MN, false, false>, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb2, tc, tc2, p);
+  if (p.chained) return chain(gemm_kernel<A_MN, B_MN, false, false>, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb2, tc, tc2, p);
   gemm_kernel<A_MN, B_MN, false, false><<<grid, GEMM_THREADS, GEMM_SMEM, stream>>>(ta, tb, tb2, tc, tc2, p);
   return cudaGetLastError();
 }
@@ -1017,7 +1020,7 @@ cudaError_t launch_gemm_pair(const CUtensorMap& ta, const CUtensorMap& tb, const
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  if (chainable(p))
+  if (p.chained)
     return chain_clusters(gemm_kernel<A_MN, B_MN, true, false>, 2, grid, GEMM_THREADS, GEMM_SMEM, stream, ta, tb, tb2, tc, tc2, p);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(grid, 1, 1);
@@ -1207,6 +1210,7 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   p.ag_dst = g.ag_dst; p.ag_shard_elems = g.ag_shard_elems; p.ag_chunk_elems = 16384; p.ag_b_offset = g.ag_b_offset;
   p.ag_flags = g.ag_flags; p.ag_epoch = g.ag_epoch; p.ag_local = g.ag_world > 0 ? g.ag_local : -1;
   p.rs_world = g.rs_world; p.rs_shard_elems = g.rs_shard_elems; p.rs_c_offset = g.rs_c_offset;
+  p.chained = chainable(p);
   p.tile_rot = 0;
   p.te_stride = 1;
   p.rs_store = g.rs_store;
