@@ -643,10 +643,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // No wait for the kernel before: that is dK/dV, which lets this one start only after it has waited for the deltas, and
-  // nothing of it is read here.  Its last CTAs and the first ones here share the chip; the wait comes at the end, so that
-  // this kernel does not end before it.
   chain_launch();
+  chain_wait();
 
   if (threadIdx.x < BWD_T) {
     const int r = q0 + threadIdx.x;
@@ -864,7 +862,6 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
                   p.scale);
   }
 
-  chain_wait();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -1017,7 +1014,7 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  if (FINE) chain_wait();   // the deltas of the dQ kernel; otherwise as in attn_bwd_dq_kernel: the wait comes at the end
+  chain_wait();
   // position range of every query tile; a tile that shares no segment with this key block gets an empty one
   const int2 kseg_rng = p.kv_rng ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
   for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
@@ -1281,7 +1278,6 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
                    key_ok, 1.f);
   }
 
-  if (!FINE) chain_wait();
   tc_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -1344,8 +1340,8 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  chain_launch();
   chain_wait();
-  chain_launch();   // (after the wait: the dK/dV kernel relies on the deltas being there)
 
   if (threadIdx.x < BWD_T) {
     const int r = q0 + threadIdx.x;

@@ -59,8 +59,10 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 // ----------------------------------------------------------------------------
 // Chained launches: a kernel launched with chain() may be given SMs while the kernel before it in the stream still runs
 // (once all of that one's CTAs have called chain_launch or ended), and everything it does before chain_wait overlaps.
-// chain_wait returns when the kernel before has ended and its writes are visible; every CTA of a chained kernel calls it
-// before it touches global memory, reads or writes.  A kernel that allocates tensor memory calls chain_launch after the
+// chain_wait returns when the kernel before has ended and its writes are visible; every thread of a chained kernel calls it
+// before it touches global memory, reads or writes (only prefetches to L2, which read nothing it sees, may come earlier).
+// That the kernel before had waited for the one before it before it called chain_launch is no substitute: chain_launch
+// orders no memory.  A kernel that allocates tensor memory calls chain_launch after the
 // allocation: the next kernel's CTAs would otherwise take the columns that this one still waits for.  chain_launch lets the
 // next kernel in however this one was launched (that the next one is chained is what counts), so a kernel that waits for
 // anything but the stream in front of it (a shard's flag, another GPU) must not call it: the next kernel's CTAs would fill

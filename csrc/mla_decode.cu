@@ -88,8 +88,7 @@ mla_prep_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__
 __global__ void __launch_bounds__(MLA_THREADS)
 mla_fold_kernel(const __nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__ w, float* __restrict__ qa, int B,
                 int H, int dn, int dv, int C) {
-  chain_wait();
-  chain_launch();    // (after the wait: the split kernel reads what the kernel before this one wrote)
+  if (!chain_begin()) return;
   __shared__ float acc_s[8][MLA_MAX_B][64];
   extern __shared__ float fold_q[];                  // [MLA_MAX_B][dn]
   const int h = blockIdx.x, c0 = blockIdx.y * 64, b0 = blockIdx.z * MLA_MAX_B;
@@ -181,7 +180,7 @@ __device__ __forceinline__ void mma16816(float* d, const uint32_t* a, uint32_t b
 // Sixteen heads are one row block of mma.sync m16n8k16 (a tcgen05 tile would be seven eighths empty): scores from the
 // queries as three bf16 terms, the weighted sum from the weights as three, so that nothing of the fp32 values is lost, and
 // every 16-deep product starts from zero and is added to its sum in fp32 (the tensor core's own sums are cut, not rounded).
-// Bound by latency: the keys are asked for before the kernel in front has ended (it writes the folded queries only).
+// Bound by latency: the first keys are brought to L2 before the kernel in front has ended.
 __global__ void __launch_bounds__(MLA_THREADS, 2)
 mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__ q,
                  const __nv_bfloat16* __restrict__ kv_cache, const __nv_bfloat16* __restrict__ pe_cache,
@@ -200,6 +199,14 @@ mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__
   const int k_begin = range * per, k_end = min(n_keys, k_begin + per);
   const int cv = C / 8, dvec = D / 8;
   const uint32_t sk_at = smem_u32(sk), sq_at = smem_u32(sq);
+  chain_launch();
+  // The first keys move to L2 while the fold kernel runs (a line each; they are read after the wait).
+  for (int i = threadIdx.x; i < MLA_KEYS * (C / 64 + 1); i += MLA_THREADS) {
+    const int r = i / (C / 64 + 1), c = i - r * (C / 64 + 1), key = min(k_begin + r, k_end - 1);
+    const __nv_bfloat16* at = c < C / 64 ? kv_cache + b * kv_bs + (size_t)key * C + c * 64 : pe_cache + b * pe_bs + (size_t)key * MLA_R;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
+  }
+  chain_wait();
   auto fetch_keys = [&](int k0) {                // asynchronous; keys past the range are zeros
     for (int i = threadIdx.x; i < MLA_KEYS * dvec; i += MLA_THREADS) {
       const int r = i / dvec, c = i - r * dvec, key = min(k0 + r, k_end - 1);
@@ -211,8 +218,6 @@ mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  chain_launch();
-  // The fold kernel lets this one start only after its own wait, so the caches and the rotated queries are there.
   fetch_keys(k_begin);
   for (int i = threadIdx.x; i < MLA_HG * (MLA_R / 4); i += MLA_THREADS) {     // the rotary parts: bf16 as they are
     const int h = i / (MLA_R / 4), d = (i % (MLA_R / 4)) * 4;
@@ -220,7 +225,6 @@ mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__
     if (h0 + h < H) u = *reinterpret_cast<const uint2*>(q + ((size_t)b * H + h0 + h) * (dn + MLA_R) + dn + d);
     *reinterpret_cast<uint2*>(sq + h * pitch + (C + d) * 2) = u;
   }
-  chain_wait();
 #pragma unroll 8
   for (int i = threadIdx.x; i < MLA_HG * (C / 4); i += MLA_THREADS) {
     const int h = i / (C / 4), d = (i % (C / 4)) * 4;
