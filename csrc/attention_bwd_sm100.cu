@@ -255,7 +255,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  chain_wait();
+  if (!chain_wait()) return;
   // position range of every query tile (decides which tiles this key block can see)
   const int2 kseg_rng = SEG ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
   for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
@@ -644,7 +644,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   chain_launch();
-  chain_wait();
+  if (!chain_wait()) return;
 
   if (threadIdx.x < BWD_T) {
     const int r = q0 + threadIdx.x;
@@ -1014,7 +1014,7 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tmem_alloc(tmem_slot, 512);
     tmem_relinquish();
   }
-  chain_wait();
+  if (!chain_wait()) return;
   // position range of every query tile; a tile that shares no segment with this key block gets an empty one
   const int2 kseg_rng = p.kv_rng ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
   for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
@@ -1341,7 +1341,7 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   chain_launch();
-  chain_wait();
+  if (!chain_wait()) return;
 
   if (threadIdx.x < BWD_T) {
     const int r = q0 + threadIdx.x;

@@ -308,7 +308,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   if (p.cp_world <= 1) chain_launch();   // (with an exchange, this kernel waits for other GPUs)
-  chain_wait();
+  if (!chain_wait()) return;
 
   // Range of positions covered by this tile's query rows.
   if (threadIdx.x < FWD_BM) {

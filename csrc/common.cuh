@@ -70,10 +70,15 @@ __device__ __forceinline__ void setmaxnreg_dec() {
 // (A kernel boundary otherwise costs 2 to 3 us of drained SMs, as much as the kernels of a decode step run: 36 launches of a decode step over a short cache 384 -> 307 us, decoder layer of 3 tokens 119 -> 103.)
 // ----------------------------------------------------------------------------
 __device__ __forceinline__ void chain_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-// Both at once, always true: what follows `if (!chain_begin()) return;` depends on the wait, so that no load of read-only
-// data is moved in front of it.
-__device__ __forceinline__ bool chain_begin() {
+// Always true: what follows `if (!chain_wait()) return;` depends on the wait, so that no load of read-only data (__ldg,
+// const __restrict__) is moved in front of it.
+[[nodiscard]] __device__ __forceinline__ bool chain_wait() {
+  uint32_t go;
+  asm volatile("griddepcontrol.wait;\n\tmov.u32 %0, 1;" : "=r"(go)::"memory");
+  return go != 0;
+}
+// Both at once.
+[[nodiscard]] __device__ __forceinline__ bool chain_begin() {
   uint32_t go;
   asm volatile("griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;\n\tmov.u32 %0, 1;" : "=r"(go)::"memory");
   return go != 0;

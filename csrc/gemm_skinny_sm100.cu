@@ -141,7 +141,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const int n0 = nt * (swiglu ? SK_TN / 2 : SK_TN);
   int ez = 0;
   if (p.tile_expert) {
-    chain_wait();
+    if (!chain_wait()) return;
     ez = p.tile_expert[bt];
     if (ez < 0) return;      // the whole cluster leaves together
   }
@@ -189,7 +189,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   chain_launch();
-  chain_wait();
+  if (!chain_wait()) return;
 
   if (warp == 0) {
     if (lane == 0) {

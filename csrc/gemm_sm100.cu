@@ -422,7 +422,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   if (p.chained) chain_launch();
-  chain_wait();
+  if (!chain_wait()) return;
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer

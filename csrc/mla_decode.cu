@@ -206,7 +206,7 @@ mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__
     const __nv_bfloat16* at = c < C / 64 ? kv_cache + b * kv_bs + (size_t)key * C + c * 64 : pe_cache + b * pe_bs + (size_t)key * MLA_R;
     asm volatile("prefetch.global.L2 [%0];" ::"l"(at));
   }
-  chain_wait();
+  if (!chain_wait()) return;
   auto fetch_keys = [&](int k0) {                // asynchronous; keys past the range are zeros
     for (int i = threadIdx.x; i < MLA_KEYS * dvec; i += MLA_THREADS) {
       const int r = i / dvec, c = i - r * dvec, key = min(k0 + r, k_end - 1);

@@ -41,7 +41,7 @@ def test_chained_kernels_wait_before_they_read(name):
     chained |= set(re.findall(r"\w+_kernel\b", call))
   chained |= {k for k, body in kernels.items() if "chain_" in body}
   for k in sorted(chained):
-    waits = list(re.finditer(r"chain_(?:wait|begin)\(\)", kernels[k]))
+    waits = list(re.finditer(r"if \(!chain_(?:wait|begin)\(\)\) return;", kernels[k]))
     assert waits, f"{k} does not wait"
     found = ACCESS.search(kernels[k][:waits[0].start()])
     assert found is None, f"{k} uses global memory ({found.group()}) before its wait"
