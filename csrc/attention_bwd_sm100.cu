@@ -438,8 +438,8 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     const int kseg = (p.kv_seg && key_ok) ? p.kv_seg[(long long)b * p.Sk + kp] : 0;
     const uint32_t tb = tmem_base + ((uint32_t)(qd * 32) << 16);
     const uint32_t tS = tb + T_S + half * 64, tDP = tb + T_DP + half * 64;
-    const int win = p.window > 0 ? p.window : 0x40000000;   // keep needs qp < kp + win
-    const int cmax = p.causal ? kp : -0x40000000;           // and qp >= cmax
+    const int win = p.window > 0 ? p.window : 0x7fffffff;   // keep needs qp - kp < win
+    const int cmax = p.causal ? kp : -0x7fffffff;           // and qp >= cmax
     bool ok = true;
 
     int step = 0;
@@ -472,7 +472,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             }
           } else {
             const int at = t * BWD_T + pos_off + half * 64;   // position of the first one
-            const int hi = kp + win - 1 - at, lo = cmax - 1 - at;
+            const int hi = kp - at + min(win, 0x40000000) - 1, lo = p.causal ? kp - at - 1 : -1;   // (kp - at < 2^30)
             keep0 = bits_upto(hi) & ~bits_upto(lo);
             keep1 = bits_upto(hi - 32) & ~bits_upto(lo - 32);
           }
@@ -658,7 +658,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int qpos_min = tile_minmax[0], qpos_max = tile_minmax[1];
   const int nblk_total = (p.Sk + BWD_T - 1) / BWD_T;
   int blk_hi = p.causal ? min(nblk_total, qpos_max / BWD_T + 1) : nblk_total;
-  int blk_lo = (p.window > 0) ? max(0, (qpos_min - p.window + 1) / BWD_T) : 0;
+  int blk_lo = (p.window > 0 && qpos_min >= p.window) ? (qpos_min - p.window + 1) / BWD_T : 0;
   if (p.causal && qpos_max < 0) blk_hi = 0;
   int2 qr = make_int2(0, 0);
   if (SEG) {   // as in the forward: only the key blocks between the first and last with a common segment
@@ -773,8 +773,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const uint32_t tb = tmem_base + ((uint32_t)(qd * 32) << 16);
     const uint32_t tDP = tb + T_DP + half * 64;
     const int* ks = p.kv_seg ? p.kv_seg + (long long)b * p.Sk : nullptr;
-    const int win = p.window > 0 ? p.window : 0x40000000;
-    const int kmax = p.causal ? min(qpos, p.Sk - 1) : p.Sk - 1;   // keep needs kp <= kmax
+    const int kmin = p.window > 0 && qpos >= p.window ? qpos - p.window : -1;   // keep needs kmin < kp <= kmax
+    const int kmax = p.causal ? min(max(qpos, -1), p.Sk - 1) : p.Sk - 1;
     bool ok = true;
 
     for (int j = 0; j < nblk && ok; ++j) {
@@ -789,7 +789,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       const uint32_t tS = tb + T_S + (j & 1) * BWD_T + half * 64;
       uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;   // this half's 64 keys that the row may see
       if (need_mask) {
-        const int k0 = kv0 + half * 64, hi = kmax - k0, lo = qpos - win - k0;
+        const int k0 = kv0 + half * 64, hi = kmax - k0, lo = kmin - k0;
         keep0 = bits_upto(hi) & ~bits_upto(lo);
         keep1 = bits_upto(hi - 32) & ~bits_upto(lo - 32);
         if (ks && (!SEG || seg_mask))
@@ -1355,7 +1355,7 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   const int qpos_min = tile_minmax[0], qpos_max = tile_minmax[1];
   const int nblk_total = (p.Sk + BWD_T - 1) / BWD_T;
   int blk_hi = p.causal ? min(nblk_total, qpos_max / BWD_T + 1) : nblk_total;
-  int blk_lo = (p.window > 0) ? max(0, (qpos_min - p.window + 1) / BWD_T) : 0;
+  int blk_lo = (p.window > 0 && qpos_min >= p.window) ? (qpos_min - p.window + 1) / BWD_T : 0;
   if (p.causal && qpos_max < 0) blk_hi = 0;
   int2 qr = make_int2(0, 0);
   if (p.kv_rng) {

@@ -323,7 +323,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   const int qpos_min = tile_minmax[0], qpos_max = tile_minmax[1];
   const int nblk_total = (p.Sk + FWD_BN - 1) / FWD_BN;
   int blk_hi = p.causal ? min(nblk_total, qpos_max / FWD_BN + 1) : nblk_total;
-  int blk_lo = (p.window > 0) ? max(0, (qpos_min - p.window + 1) / FWD_BN) : 0;
+  int blk_lo = (p.window > 0 && qpos_min >= p.window) ? (qpos_min - p.window + 1) / FWD_BN : 0;
   if (p.causal && qpos_max < 0) blk_hi = 0;
   int2 qr = make_int2(0, 0);   // segment ids of this tile's rows
   if (SEG) {
@@ -430,8 +430,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t tS = tmem_base + lane_addr, tO = tmem_base + 128 + lane_addr;
     const int* ks = p.kv_seg ? p.kv_seg + (long long)b * p.Sk : nullptr;
-    const int win = p.window > 0 ? p.window : 0x40000000;         // (qpos - win must not wrap for positions before the first key)
-    const int kmax = p.causal ? min(qpos, p.Sk - 1) : p.Sk - 1;   // last key this row may see
+    // keys this row may see: kmin < key <= kmax (no sum here wraps, whatever the window and the position)
+    const int kmin = p.window > 0 && qpos >= p.window ? qpos - p.window : -1;
+    const int kmax = p.causal ? min(max(qpos, -1), p.Sk - 1) : p.Sk - 1;
 
     float m_used = -INFINITY;   // maximum the exponentials are currently taken against (log2 units)
     float l = 0.f;
@@ -449,7 +450,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
                              (p.window > 0 && qpos_max - kv0 >= p.window) || seg_mask;
       uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;   // keys kv0 + [0, 32) and kv0 + [32, 64) this row may see
       if (need_mask) {
-        const int hi = row_ok ? kmax - kv0 : -1, lo = qpos - win - kv0;   // lo < key - kv0 <= hi
+        const int hi = row_ok ? kmax - kv0 : -1, lo = kmin - kv0;
         keep0 = bits_upto(hi) & ~bits_upto(lo);
         keep1 = bits_upto(hi - 32) & ~bits_upto(lo - 32);
         if (ks && (!SEG || seg_mask))
@@ -709,7 +710,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   for (int x = 0; x < 2; ++x) {
     const int mn = tile_minmax[2 * x], mx = tile_minmax[2 * x + 1];
     hi[x] = p.causal ? min(nblk_total, mx / F2_T + 1) : nblk_total;
-    lo[x] = (p.window > 0) ? max(0, (mn - p.window + 1) / F2_T) : 0;
+    lo[x] = (p.window > 0 && mn >= p.window) ? (mn - p.window + 1) / F2_T : 0;
     if (mx < 0 && (p.causal || mx == -0x7fffffff)) hi[x] = 0;   // nothing to see, or no rows
     if (hi[x] <= lo[x]) { lo[x] = 0; hi[x] = 0; }
   }
@@ -845,8 +846,8 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     const uint32_t lane_addr = (uint32_t)(q * 32) << 16;
     const uint32_t tS = tmem_base + x * F2_T + lane_addr, tO = tmem_base + 256 + x * F2_T + lane_addr;
     const int* ks = p.kv_seg ? p.kv_seg + (long long)b * p.Sk : nullptr;
-    const int win = p.window > 0 ? p.window : 0x40000000;         // (qpos - win must not wrap for positions before the first key)
-    const int kmax = p.causal ? min(qpos, p.Sk - 1) : p.Sk - 1;   // keep needs kp <= kmax
+    const int kmin = p.window > 0 && qpos >= p.window ? qpos - p.window : -1;   // keep needs kmin < kp <= kmax
+    const int kmax = p.causal ? min(max(qpos, -1), p.Sk - 1) : p.Sk - 1;
     float* xch = reinterpret_cast<float*>(smem + OFF_X) + x * (4 * F2_T);   // [parity][half][row]
     // The two warps that share the rows of a TMEM lane quarter (one per key half) synchronise on a named
     // barrier of their own: 64 threads, so no warp waits for the slowest of the tile's eight.
@@ -880,7 +881,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
       if (need_mask) {
         // key c of this half is kept iff lo_c < c <= hi_c (causal / window / sequence end / row padding)
         const int hi_c = row_ok ? kmax - kv0 : -1;
-        const int lo_c = qpos - win - kv0;
+        const int lo_c = kmin - kv0;
 #pragma unroll
         for (int c = 0; c < 64; ++c) r[c] = (c <= hi_c && c > lo_c) ? r[c] : 0xff800000u;   // -inf
         if (ks) {

@@ -92,3 +92,30 @@ def test_masks_as_bits(cuda_lib, s, window, positions):
   for g, r in zip((o, *got), (w, *want)):
     assert torch.isfinite(g).all()
     assert ((g.float() - r.float()).norm() / r.float().norm()).item() < 2e-2
+
+
+def _both(q, k, v, **kw):
+  leaves = [t.clone().requires_grad_(True) for t in (q, k, v)]
+  o = A.attention(*leaves, **kw)
+  o.backward(torch.linspace(-1, 1, o.numel(), device="cuda").view(o.shape).to(o.dtype))
+  return [o.detach()] + [t.grad for t in leaves]
+
+
+@pytest.mark.parametrize("sq,sk", [(70, 70), (300, 300), (200, 70)])
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("window", [2 ** 31 - 1, 2 ** 31 - 66, 2 ** 30 + 1])
+def test_a_window_wider_than_any_sequence_is_none(cuda_lib, sq, sk, causal, window):
+  """No sum of a position and the window wraps (more queries than keys: positions before the first key)."""
+  g = torch.Generator(device="cuda").manual_seed(sq + sk)
+  q, k, v = (torch.randn(2, s, 2, 128, device="cuda", generator=g).to(torch.bfloat16) for s in (sq, sk, sk))
+  for got, want in zip(_both(q, k, v, causal=causal, window=window), _both(q, k, v, causal=causal)):
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("first", [2 ** 30 - 3, 2 ** 30 + 100])
+def test_positions_far_past_the_last_key_see_all_of_them(cuda_lib, first):
+  g = torch.Generator(device="cuda").manual_seed(first % 1000)
+  q, k, v = (torch.randn(2, 150, 2, 128, device="cuda", generator=g).to(torch.bfloat16) for _ in range(3))
+  pos = (first + torch.arange(300, device="cuda", dtype=torch.int32) % 150).view(2, 150)
+  for got, want in zip(_both(q, k, v, causal=True, q_positions=pos), _both(q, k, v, causal=False)):
+    assert torch.equal(got, want)
