@@ -86,3 +86,27 @@ def test_cross_entropy_at_the_edges_of_its_loops(cuda_lib, vocab):
   assert abs(loss.item() / want.item() - 1) < 1e-5
   # bf16 results: 2^-9 of each value
   assert ((logits.double() - 0.5 * x.grad).abs() <= 2.0 ** -8 * (0.5 * x.grad).abs() + 1e-9).all()
+
+
+@pytest.mark.parametrize("rows", [2048, 4096, 4097])
+def test_memory_that_a_head_takes(cuda_lib, rows):
+  """Up to 2 * hidden rows d(logits) are held instead of an fp32 weight gradient, above that 2048 rows beside it."""
+  from torchprime_b200.models.llama import CausalLMHead
+  hidden, vocab = 2048, 32768
+  w = (torch.randn(vocab, hidden, device="cuda") / 32).to(torch.bfloat16).requires_grad_(True)
+  h = torch.randn(1, rows, hidden, device="cuda", dtype=torch.bfloat16, requires_grad=True)
+  t = torch.randint(0, vocab, (1, rows), device="cuda")
+  head = CausalLMHead.__new__(CausalLMHead)
+  torch.nn.Module.__init__(head)
+  head.norm, head.lm_head, head.loss_group = torch.nn.Identity(), torch.nn.Linear(1, 1, bias=False), None
+  head.lm_head.weight = torch.nn.Parameter(w.detach())
+  torch.cuda.synchronize()
+  torch.cuda.reset_peak_memory_stats()
+  before = torch.cuda.memory_allocated()
+  loss = head(h, t, want_logits=False)[1]
+  torch.cuda.synchronize()
+  taken = torch.cuda.max_memory_allocated() - before
+  held = 2 * rows * vocab if rows <= 2 * hidden else 4 * hidden * vocab + 2 * 2048 * vocab
+  assert taken <= held + 2 * rows * hidden + (4 << 20)      # and the gradient of the hidden states, a few small tensors
+  loss.backward()
+  assert head.lm_head.weight.grad.dtype == torch.bfloat16 and bool(torch.isfinite(h.grad).all())

@@ -209,7 +209,8 @@ class CausalLMHead(nn.Module):
       n_valid = self._valid_count(targets) if targets is not None else None
       if targets is not None and not want_logits:
         w = self.lm_head.weight
-        return None, ops.linear_cross_entropy(h, w, targets, chunk_rows=ops.head_chunk_rows(w), n_valid=n_valid)
+        chunk = ops.head_chunk_rows(w, targets.numel())
+        return None, ops.linear_cross_entropy(h, w, targets, chunk_rows=chunk, n_valid=n_valid)
       logits = ops.linear(h, self.lm_head.weight).float()
       loss = None
       if targets is not None:

@@ -896,12 +896,13 @@ class _LinearCrossEntropyFn(torch.autograd.Function):
     return gh, gw, None, None, None
 
 
-def head_chunk_rows(w) -> int:
-  """Rows of d(logits) that a head holds at a time: while the weight gradient is returned, as many as take the memory
-  of the fp32 gradient that summing over chunks needs (3001 rows of a 128,256 x 4096 head, forward and
-  backward: 9.1 -> 7.9 ms); 2048 where gradients collect in a flat buffer or none are wanted."""
-  if torch.is_grad_enabled() and w.requires_grad and getattr(w, "main_grad", None) is None:
-    return max(2048, 2 * w.shape[1])
+def head_chunk_rows(w, rows: int) -> int:
+  """Rows of d(logits) that a head of ``rows`` rows holds at a time: all of them where the weight gradient is returned and
+  they take no more memory than the fp32 gradient that summing over chunks needs instead (3001 rows of a 128,256 x 4096
+  head, forward and backward: 9.1 -> 7.9 ms); else 2048, beside that gradient or the flat buffer it collects in."""
+  if (rows <= 2 * w.shape[1] and torch.is_grad_enabled() and w.requires_grad
+      and getattr(w, "main_grad", None) is None):
+    return max(2048, rows)
   return 2048
 
 
