@@ -1295,14 +1295,7 @@ extern "C" int tpb_gemm_scaled_bf16(const void* A, const void* B, void* C, int M
                                     long long ldb, long long ldc, int a_mn, int b_mn, int epi, float alpha,
                                     const float* scale, const void* aux, long long ldaux, void* c2, long long ldc2,
                                     int max_ctas, void* stream_) {
-  const bool split = max_ctas == 0 && gemm_pair_mode() == 1 && !a_mn && ksplit_wins(M, N, K);
-  // few rows or few tiles: the kernel that streams B once and splits the contraction
-  if (max_ctas == 0 && gemm_pair_mode() == 1 && !split &&
-      (a_mn ? b_mn && skinny_wins_wgrad(M, N, K) : skinny_wins(M, N, K, epi == TPB_EPI_SWIGLU))) {
-    const int r = skinny_gemm(A, B, nullptr, C, M, N, K, 1, lda, ldb, 0, ldc, a_mn, b_mn, epi, alpha, aux, ldaux, c2, ldc2,
-                              nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_), false, scale);
-    if (r != -2) return r;     // -2: an epilogue or alignment it does not take
-  }
+  const bool by_rule = max_ctas == 0 && gemm_pair_mode() == 1;
   GemmCall g{};
   g.A = A; g.B = B; g.B2 = nullptr; g.C = C;
   g.M = M; g.N = N; g.K = K; g.E = 1;
@@ -1310,11 +1303,17 @@ extern "C" int tpb_gemm_scaled_bf16(const void* A, const void* B, void* C, int M
   g.a_mn = a_mn; g.b_mn = b_mn; g.epi = epi; g.alpha = alpha; g.alpha_dev = scale;
   g.aux = aux; g.ldaux = ldaux; g.c2 = c2; g.ldc2 = ldc2; g.max_ctas = max_ctas;
   g.mode = 0;
-  if (split) {
+  if (by_rule && !a_mn && (epi == TPB_EPI_BF16 || epi == TPB_EPI_BF16_RES) && ksplit_wins(M, N, K)) {
     g.ksplit = 1;
     const int r = run_gemm(g, reinterpret_cast<cudaStream_t>(stream_));
-    if (r != -2) return r;     // -2: an epilogue or alignment it does not take
+    if (r != -2) return r;     // -2: an alignment it does not take
     g.ksplit = 0;
+  }
+  // few rows or few tiles: the kernel that streams B once and splits the contraction
+  if (by_rule && (a_mn ? b_mn && skinny_wins_wgrad(M, N, K) : skinny_wins(M, N, K, epi == TPB_EPI_SWIGLU))) {
+    const int r = skinny_gemm(A, B, nullptr, C, M, N, K, 1, lda, ldb, 0, ldc, a_mn, b_mn, epi, alpha, aux, ldaux, c2, ldc2,
+                              nullptr, 0, 0, 0, reinterpret_cast<cudaStream_t>(stream_), false, scale);
+    if (r != -2) return r;     // -2: an epilogue or alignment it does not take
   }
   return run_gemm(g, reinterpret_cast<cudaStream_t>(stream_));
 }

@@ -260,3 +260,16 @@ def test_route_of_a_gemm_call(cuda_lib, M, N, K):
       # two fp32 sums of K random terms in other orders: each strays by about 2^-24 sqrt(K / 2) of the result
       bound = 2.0 ** -23 * K ** 0.5
       assert ((a.float() - b.float()).norm() / b.float().norm()).item() < (bound if epi == k.EPI_F32 else 2.0 ** -9)
+
+
+@pytest.mark.parametrize("m,n,kk", [(512, 4096, 4096), (1024, 2048, 4096)])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_fp32_results_that_a_split_tile_does_not_take_stay_here(cuda_lib, m, n, kk, b_mn):
+  """Products that the rule of the split tiles names too, with an epilogue they do not have: this kernel's bits, which
+  adds in another order than the tiled one."""
+  g = torch.Generator("cuda").manual_seed(m)
+  a = torch.randn(m, kk, device="cuda", generator=g).to(torch.bfloat16)
+  b = torch.randn(*((kk, n) if b_mn else (n, kk)), device="cuda", generator=g).to(torch.bfloat16)
+  want = _skinny(a, b, b_mn=b_mn, epi=k.EPI_F32)
+  assert torch.equal(k.gemm(a, b, b_mn=b_mn, epi=k.EPI_F32), want)
+  assert not torch.equal(k.gemm(a, b, b_mn=b_mn, epi=k.EPI_F32, max_ctas=148), want)      # (the tiled kernel)
