@@ -1072,14 +1072,25 @@ static int resident_clusters(int ctas) {
   return n < sm_count() / ctas ? n : sm_count() / ctas;
 }
 
+// gemm_skinny_sm100.cu
+bool skinny_wins(int M, int N, int K, bool swiglu);
+bool skinny_wins_wgrad(int M, int N, int K);
+
 // Whether two pairs to a tile are the faster way for bf16 results of M rows (dense, A K-major).  T 256 x 256 tiles run on
-// 74 pairs or on C = 36 clusters; the exchange of partial sums costs 5 to 10 us a tile, during which its cluster does nothing
-// else, so the contraction has to be long, and fewer half-length waves than twice the whole ones have to come out (us, the
-// kernel used otherwise / this one):
-//   T = 24: 6144 x 4096 24.6 / 22.5    T = 32: 4096 x 4096 24 / 22, x 6144 31 / 27.5, x 14336 60 / 50, x 28672 113 / 94
-//   T = 48: 4096 x 4096 36 / 41, x 14336 108 / 95, x 28672 201 / 171, 2048 x 10944 84 / 80    T = 64: x 14336 102 / 94
-//   T = 96: 4096 x 6144 78 / 79, x 14336 166 / 143, x 28672 324 / 268      T = 128: x 14336 172 / 192, x 28672 340 / 360
-// Up to 16 tiles the few-rows kernel, which splits further, is ahead (T = 16, 4096 x 14336: 37 / 46).
+// 74 pairs or on C clusters, as many as the chip's partition lets be resident (33 of the 37 that 148 SMs would hold, here);
+// the exchange of partial sums costs 5 to 10 us a tile, during which its cluster does nothing else, so the contraction has
+// to be long and the half-length waves fewer than twice the whole ones.  us, the kernel used otherwise / this one, for
+// K = 4096, 8192, 14336 (weights from HBM):
+//   T = 24, 32, 33, one wave:            29 / 27, 37 / 32, 68 / 55      27 / 25, 37 / 31, 68 / 55      24 / 22, 38 / 32, 69 / 55
+//   T = 34, 36, the few-rows kernel's:   24 / 37, 43 / 61, 73 / 102     23 / 35, 40 / 60, 67 / 98
+//   T = 40, 48, 64, two waves:           31 / 35, 60 / 57, 105 / 93     32 / 35, 60 / 57, 108 / 95     31 / 36, 61 / 59, 111 / 101
+//   T = 68, 72, three against one:       31 / 51, 69 / 100, 118 / 164   32 / 52, 65 / 91, 112 / 149
+//   T = 80, 96, three against two:       49 / 53, 95 / 88, 167 / 142    48 / 52, 94 / 88, 170 / 153
+//   T = 105, four against two:           50 / 68, 108 / 127, 182 / 201
+//   T = 160, five against three:         - , 154 / 160, 274 / 261 (K = 20480: 392 / 356)
+// With whole waves of 128-row tiles to fill (48 tiles of 300 rows: 72 of 128 rows), the few-rows kernel is ahead of two
+// waves as well (39 / 57); up to 16 tiles it is ahead of one (T = 16: 24 / 31).  Two waves against one that 128-row tiles
+// fill to five sixths and more need K = 10240 (T = 63: 75 / 77, 84 / 82; T = 66: 64 / 65, 83 / 82 for K = 8192, 10240).
 static bool ksplit_wins(int M, int N, int K) {
   if (M <= 128 || K < 4096) return false;
   const long long t = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
@@ -1088,7 +1099,10 @@ static bool ksplit_wins(int M, int N, int K) {
   if (clusters < 1 || pairs < 1) return false;
   if (t <= clusters) return true;
   const long long half = (t + clusters - 1) / clusters, whole = (t + pairs - 1) / pairs;
-  return K >= 8192 && (whole == 1 || (half < 2 * whole && (whole == 2 || K >= 20480)));
+  if (K < 8192 || skinny_wins(M, N, K, false)) return false;
+  if (whole > 1) return half < 2 * whole && (whole == 2 || K >= 20480);
+  const long long t128 = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
+  return half == 2 && (K >= 10240 || 6 * t128 <= 5 * sm_count());
 }
 
 // gemm_skinny_sm100.cu
@@ -1096,8 +1110,6 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
                 long long ldx, long long ldw, long long w_stride, long long ldc, int x_mn, int w_mn, int epi, float alpha,
                 const void* aux, long long ldaux, void* c2, long long ldc2, const int* tile_expert, int experts_hit, int nt,
                 int splits, cudaStream_t stream, bool f32, const float* alpha_dev = nullptr);
-bool skinny_wins(int M, int N, int K, bool swiglu);
-bool skinny_wins_wgrad(int M, int N, int K);
 
 // TPB_GEMM_PAIR: 0 = never CTA pairs, 2 = pairs for every dense shape (tests), default = by shape
 static int gemm_pair_mode() {

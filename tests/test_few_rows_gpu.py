@@ -273,3 +273,14 @@ def test_fp32_results_that_a_split_tile_does_not_take_stay_here(cuda_lib, m, n, 
   want = _skinny(a, b, b_mn=b_mn, epi=k.EPI_F32)
   assert torch.equal(k.gemm(a, b, b_mn=b_mn, epi=k.EPI_F32), want)
   assert not torch.equal(k.gemm(a, b, b_mn=b_mn, epi=k.EPI_F32, max_ctas=148), want)      # (the tiled kernel)
+
+
+@pytest.mark.parametrize("m,n,few_rows", [(9472, 256, True), (9472, 512, False)])      # 37 and 74 tiles of 256 x 256
+def test_split_tiles_that_take_a_wave_more_are_not_taken(cuda_lib, m, n, few_rows):
+  """One tile more than clusters of four fit the chip once, and twice: the kernels that do not split tiles by pairs."""
+  kk = 8192
+  g = torch.Generator("cuda").manual_seed(m)
+  a = torch.randn(m, kk, device="cuda", generator=g).to(torch.bfloat16)
+  b = torch.randn(n, kk, device="cuda", generator=g).to(torch.bfloat16)
+  want = _skinny(a, b) if few_rows else k.gemm(a, b, max_ctas=148)
+  assert torch.equal(k.gemm(a, b), want)
