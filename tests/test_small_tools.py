@@ -144,3 +144,19 @@ def test_setup_sharding_and_mesh_names_the_batch_and_sequence_axes():
   cfg = compose("default", moe + ["ici_mesh.fsdp=2", "ici_mesh.expert=2", "expert_axis_mode=folded",
                                   "model/sharding=mixtral-fsdp-ep"])
   assert setup_sharding_and_mesh(mm, cfg, mesh=get_mesh(cfg, rank=0, world_size=2)).batch_axes == ("data", "fsdp")
+
+
+def test_native_operators_belong_to_one_torch(monkeypatch):
+  """A library built for another torch is neither loaded nor taken for up to date: its name says which one it fits."""
+  import torch
+  from torchprime_b200 import build
+  from torchprime_b200.ops import _lib
+  here = build.ops_path()
+  monkeypatch.setattr(torch, "__version__", "99.0.1+cu999")
+  other = build.ops_path()
+  assert other != here and "99.0.1_cu999" in other
+  with pytest.raises(_lib.KernelError, match="99.0.1_cu999.*missing"):
+    _lib._load_native()
+  monkeypatch.undo()
+  monkeypatch.setattr(torch._C, "_GLIBCXX_USE_CXX11_ABI", not torch._C._GLIBCXX_USE_CXX11_ABI)
+  assert build.ops_path() != here

@@ -1,5 +1,5 @@
-"""Builds ``libtpb200.so`` (all sm_100a kernels) in-tree with nvcc, and ``_tpb_torch.so`` (the operators
-that issue them as native torch functions, ``csrc/torch_ops.cpp``) with the host compiler.
+"""Builds ``libtpb200.so`` (all sm_100a kernels) in-tree with nvcc, and ``_tpb_torch-*.so`` (the operators
+that issue them as native torch functions, ``csrc/torch_ops.cpp``) with the host compiler, for the torch that is installed.
 
 ``python -m torchprime_b200.build`` compiles every ``csrc/*.cu`` with
 ``-gencode arch=compute_100a,code=sm_100a`` and links them into
@@ -13,9 +13,11 @@ from __future__ import annotations
 import concurrent.futures
 import glob
 import os
+import re
 import shutil
 import subprocess
 import sys
+import sysconfig
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CSRC = os.path.join(ROOT, "csrc")
@@ -23,7 +25,6 @@ BUILD = os.path.join(ROOT, "build")
 LIB_DIR = os.path.join(ROOT, "torchprime_b200", "lib")
 LIB_PATH = os.path.join(LIB_DIR, "libtpb200.so")
 OPS_SRC = os.path.join(CSRC, "torch_ops.cpp")
-OPS_PATH = os.path.join(LIB_DIR, "_tpb_torch.so")
 
 NVCC_FLAGS = [
   "-gencode", "arch=compute_100a,code=sm_100a",
@@ -61,17 +62,23 @@ def _compile(src: str, verbose: bool) -> str:
   return obj
 
 
-def _build_torch_ops() -> None:
-  """Compile and link the native operators against torch and ``libtpb200.so`` (found next to it at load time)."""
-  import sysconfig
+def ops_path() -> str:
+  """The native operators' library.  It fits one torch and one Python (their C++ types are part of its interface), so its
+  name says which: under another one it is missing, and is built anew, instead of being loaded."""
+  import torch
+  tag = re.sub(r"[^0-9A-Za-z.]", "_", torch.__version__)
+  return os.path.join(LIB_DIR, f"_tpb_torch-{tag}-abi{int(torch._C._GLIBCXX_USE_CXX11_ABI)}{sysconfig.get_config_var('EXT_SUFFIX')}")
 
+
+def _build_torch_ops(path: str) -> None:
+  """Compile and link the native operators against torch and ``libtpb200.so`` (found next to it at load time)."""
   import torch
   root = os.path.dirname(torch.__file__)
   cuda = os.path.dirname(os.path.dirname(os.path.realpath(_nvcc())))
   inc = [CSRC, os.path.join(root, "include"), os.path.join(root, "include", "torch", "csrc", "api", "include"),
          os.path.join(cuda, "include"), sysconfig.get_paths()["include"]]
   cmd = [os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared",
-         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc), OPS_SRC, "-o", OPS_PATH,
+         f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}", *(f"-I{d}" for d in inc), OPS_SRC, "-o", path,
          f"-L{LIB_DIR}", "-ltpb200", f"-L{os.path.join(root, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch",
          "-ltorch_python", "-Wl,-rpath,$ORIGIN"]
   res = subprocess.run(cmd, capture_output=True, text=True)
@@ -95,8 +102,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
     if res.returncode != 0:
       raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
   stamp = max(os.path.getmtime(OPS_SRC), os.path.getmtime(os.path.join(CSRC, "tpb.h")))
-  if force or not os.path.exists(OPS_PATH) or os.path.getmtime(OPS_PATH) < stamp:
-    _build_torch_ops()
+  ops = ops_path()
+  if force or not os.path.exists(ops) or os.path.getmtime(ops) < stamp:
+    _build_torch_ops(ops)
   return LIB_PATH
 
 

@@ -61,12 +61,13 @@ def lib():
 
 def _load_native():
   global _native
-  path = os.path.join(os.path.dirname(_LIB_PATH), "_tpb_torch.so")
-  if not os.path.exists(path):
-    raise KernelError(f"{path} is missing: run `python -m torchprime_b200.build` first")
   import importlib.util
 
+  from ..build import ops_path
   from . import functional
+  path = ops_path()
+  if not os.path.exists(path):
+    raise KernelError(f"{path} is missing: run `python -m torchprime_b200.build` first (once for every torch that is used)")
   spec = importlib.util.spec_from_file_location("_tpb_torch", path)
   mod = importlib.util.module_from_spec(spec)
   spec.loader.exec_module(mod)
