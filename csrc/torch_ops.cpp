@@ -34,7 +34,7 @@ namespace {
 
 std::atomic<long long> g_launches{0};
 PyObject* g_check = nullptr;         // _lib.check: raises KernelError for a non-zero code
-PyObject* g_late_wgrads = nullptr;   // functional._late_wgrads: weights that got a main_grad after their forward
+PyObject* g_late_wgrads = nullptr;   // functional._deliver_wgrads: weights that got a main_grad after their forward
 PyObject* g_late_norm = nullptr;     // functional._norm_wgrad
 PyObject* g_main_grad = nullptr;     // "main_grad"
 

@@ -86,3 +86,60 @@ def test_mlp_as_one_node(cuda_lib, rows, grads, monkeypatch):
   monkeypatch.setattr(_lib, "_native", None)
   for a, b in zip(call(ops.swiglu_mlp), want):
     assert torch.equal(a, b)
+
+
+class _Published:
+  """A gather whose shards have all landed."""
+  world, epoch = 1, 1
+
+  def __init__(self, flat):
+    self.flat, self.base, self.shard_elems, self.chunk_elems = flat, flat.data_ptr(), flat.numel(), 4096
+    self.flags = torch.ones((flat.numel() + 4095) // 4096, device="cuda", dtype=torch.int32)
+
+  def offset_of(self, w):
+    return (w.data_ptr() - self.base) // 2
+
+  def wait_all(self):
+    pass
+
+
+# few rows, a few-rows product and a tiled one behind it; `grads` as above without the residual's
+@pytest.mark.parametrize("rows", [40, 129, 400])
+@pytest.mark.parametrize("grads", [(1, 1, 1, 1), (0, 1, 1, 1), (1, 0, 0, 1)])
+@pytest.mark.parametrize("sink", [torch.float32, BF])
+@pytest.mark.parametrize("gather", [False, True])
+def test_mlp_whose_weights_collect_their_gradients(cuda_lib, rows, grads, sink, gather, monkeypatch):
+  """The same node where gradients go to a main_grad, first overwritten and then added to, also while the weights are
+  being gathered: the result of the two operators, gradients but for one rounding less."""
+  g = torch.Generator("cuda").manual_seed(rows)
+  r = lambda *s: torch.randn(*s, device="cuda", generator=g)    # noqa: E731
+  flat = (torch.cat([r(2 * 72 * 64), r(64 * 72)]) / 8).to(BF)
+  x, res, dy = r(1, rows, 64).to(BF), r(1, rows, 64).to(BF), r(1, rows, 64).to(BF)
+
+  def call(fn):
+    mains = torch.full((flat.numel(),), 3.0, device="cuda", dtype=sink)
+    xs, rs = x.clone().requires_grad_(bool(grads[0])), res.clone().requires_grad_(True)
+    ws, at = [], 0
+    for (a, b), on in zip(((72, 64), (72, 64), (64, 72)), grads[1:]):
+      w = flat[at:at + a * b].view(a, b).detach().requires_grad_(bool(on))
+      w.main_grad, w.grad_overwrite = mains[at:at + a * b].view(a, b), True
+      ws.append(w)
+      at += a * b
+    out = []
+    for _ in range(2):
+      ops.set_gather_context(_Published(flat) if gather else None)
+      try:
+        y = fn(xs, *ws, rs)
+      finally:
+        ops.set_gather_context(None)
+      y.backward(dy)
+      out += [y.detach(), mains.clone()]
+    assert all(w.grad is None for w in ws)
+    return out + [t.grad for t in (xs, rs) if t.requires_grad], type(y.grad_fn).__name__
+
+  got, node = call(ops.swiglu_mlp)
+  want, _ = call(lambda x, a, b, c, res: ops.linear(ops.linear_swiglu(x, a, b), c, residual=res))
+  assert node == "_SwigluMlpFnBackward"
+  assert torch.equal(got[0], want[0]) and torch.equal(got[2], want[2])
+  for a, b in zip(got, want):
+    assert ((a.double() - b.double()).norm() / b.double().norm()).item() < 5e-3     # bf16 gradient of the activation

@@ -71,7 +71,7 @@ def _load_native():
   spec = importlib.util.spec_from_file_location("_tpb_torch", path)
   mod = importlib.util.module_from_spec(spec)
   spec.loader.exec_module(mod)
-  mod.configure(check, functional._late_wgrads, functional._norm_wgrad)
+  mod.configure(check, functional._deliver_wgrads, functional._norm_wgrad)
   _native = mod
 
 
@@ -87,6 +87,7 @@ def _declare(L):
     "tpb_sm_count": [],
     "tpb_gemm_bf16": [P, P, P, I, I, I, LL, LL, LL, I, I, I, F, P, LL, P, LL, I, P],
     "tpb_gemm_scaled_bf16": [P, P, P, I, I, I, LL, LL, LL, I, I, I, F, P, P, LL, P, LL, I, P],
+    "tpb_gemm_swiglu_bwd_pays": [I, I, I],
     "tpb_gemm_ksplit_bf16": [P, P, P, I, I, I, LL, LL, LL, I, I, I, F, P, LL, P, LL, P],
     "tpb_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "tpb_rmsnorm_bwd": [P, P, P, P, P, P, P, I, I, P],

@@ -261,9 +261,9 @@ class _LinearFn(torch.autograd.Function):
     return (dx, dres, None, None, *wgrads)
 
 
-def _late_wgrads(ws, dy2, x2):
-  """Weight gradients of a native linear whose weights were given a main_grad after its forward pass: collected there,
-  or returned."""
+def _deliver_wgrads(ws, dy2, x2):
+  """Gradients of adjacent weights: collected in their main_grad, or returned.  (Native nodes come here for weights that
+  were given a main_grad after the forward pass.)"""
   from . import kernels as k
   sink = _grad_sink(ws)
   if sink is not None:
@@ -417,12 +417,82 @@ def linear_swiglu(x, w_gate, w_up, tp_reduce_grad=None):
   return F.silu(F.linear(x, w_gate)) * F.linear(x, w_up)
 
 
+class _SwigluMlpFn(torch.autograd.Function):
+  """linear(linear_swiglu(x, w_gate, w_up), w_down, residual) for weights that collect their gradients in a ``main_grad``,
+  also while their gather is in flight.  One node, so that the gradient of the activation becomes that of gate and up
+  inside the down projection's input gradient."""
+
+  @staticmethod
+  def forward(ctx, x, residual, w_gate, w_up, w_down):
+    from . import kernels as k
+    w = _fused_view([w_gate, w_up])
+    x2 = x.reshape(-1, x.shape[-1])
+    rows, f, n = x2.shape[0], w_gate.shape[0], w_down.shape[0]
+    gu = torch.empty(rows, 2 * f, dtype=x.dtype, device=x.device)
+    act = torch.empty(rows, f, dtype=x.dtype, device=x.device)
+    y = torch.empty(*x.shape[:-1], n, dtype=x.dtype, device=x.device)
+    ag, off = _inflight(w_gate)
+    if ag is not None:
+      from ..parallel.fsdp_comm import gemm_ag_wait
+      gemm_ag_wait(ag, x2, off, 2 * f, w.shape[1], act, k.EPI_SWIGLU, c2=gu)
+    else:
+      k.gemm(x2, w, out=act, epi=k.EPI_SWIGLU, c2=gu)
+    res2 = residual.reshape(-1, n) if residual is not None else None
+    epi = k.EPI_BF16 if residual is None else k.EPI_BF16_RES
+    ag, off = _inflight(w_down)
+    if ag is not None:
+      from ..parallel.fsdp_comm import gemm_ag_wait
+      gemm_ag_wait(ag, act, off, n, f, y.view(-1, n), epi, aux=res2)
+    else:
+      k.gemm(act, w_down, out=y.view(-1, n), epi=epi, aux=res2)
+    ctx.save_for_backward(x2, gu, act, w_gate, w_up, w_down)
+    ctx.has_res = residual is not None
+    ctx.x_shape = x.shape
+    return y
+
+  @staticmethod
+  def backward(ctx, dy):
+    from . import kernels as k
+    x2, gu, act, w_gate, w_up, w_down = ctx.saved_tensors
+    w = _fused_view([w_gate, w_up])
+    dy2 = dy.reshape(-1, dy.shape[-1]).contiguous()
+    need_x, _, need_gate, need_up, need_down = ctx.needs_input_grad
+    dx, grads = None, [None, None, None]
+    dgu = None
+    if need_x or need_gate or need_up:
+      if _lib.lib().tpb_gemm_swiglu_bwd_pays(dy2.shape[0], act.shape[1], dy2.shape[1]):
+        dgu = k.gemm(dy2, w_down, b_mn=True, epi=k.EPI_SWIGLU_BWD, aux=gu)
+      else:
+        dgu = k.swiglu_bwd(k.gemm(dy2, w_down, b_mn=True), gu)
+    if need_down:
+      grads[2:] = _deliver_wgrads([w_down], dy2, act)
+    if need_x:
+      dx = k.gemm(dgu, w, b_mn=True).view(ctx.x_shape)
+    if need_gate or need_up:
+      grads[:2] = _deliver_wgrads([w_gate, w_up], dgu, x2)
+    return (dx, dy if ctx.has_res else None, *grads)
+
+
+def _collected_mlp(x, w_gate, w_up, w_down, residual) -> bool:
+  """Whether :class:`_SwigluMlpFn` is the way: a call that is recorded, weights with a ``main_grad``, and what the two
+  operators ask for to run on kernels."""
+  ws = (w_gate, w_up, w_down)
+  return (torch.is_grad_enabled() and all(getattr(w, "main_grad", None) is not None for w in ws)
+          and any(t is not None and t.requires_grad for t in (x, residual, *ws))
+          and use_kernels(x, *ws) and _adjacent([w_gate, w_up]) and w_gate.shape == w_up.shape
+          and w_gate.shape[0] % 8 == 0 and _gemm_friendly(x, [w_gate, w_up])
+          and w_down.dim() == 2 and w_down.is_contiguous() and w_down.shape[0] % 8 == 0 and w_down.shape[1] == w_gate.shape[0]
+          and (residual is None or (residual.dtype == x.dtype and residual.shape == (*x.shape[:-1], w_down.shape[0]))))
+
+
 def swiglu_mlp(x, w_gate, w_up, w_down, residual=None):
   """linear(linear_swiglu(x, w_gate, w_up), w_down, residual=residual), as one autograd node where it can be."""
   if (nat := _native()) is not None:
     y = nat.swiglu_mlp(x, w_gate, w_up, w_down, residual)
     if y is not None:
       return y
+  if _collected_mlp(x, w_gate, w_up, w_down, residual):
+    return _SwigluMlpFn.apply(x, residual, w_gate, w_up, w_down)
   return linear(linear_swiglu(x, w_gate, w_up), w_down, residual=residual)
 
 
