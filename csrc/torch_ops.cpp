@@ -111,6 +111,25 @@ bool unpack(py::handle h, Tensor& t) {
   return true;
 }
 
+// Options that are a Python number or None; false: something else that counts as one (the Python definition converts it).
+bool whole(py::handle h, int64_t none, int64_t& out) {
+  out = none;
+  if (h.is_none()) return true;
+  int over = 0;
+  if (!PyLong_Check(h.ptr())) return false;
+  out = PyLong_AsLongLongAndOverflow(h.ptr(), &over);
+  return over == 0;
+}
+bool real(py::handle h, double none, double& out) {
+  out = none;
+  if (h.is_none()) return true;
+  if (!PyFloat_Check(h.ptr()) && !PyLong_Check(h.ptr())) return false;
+  out = PyFloat_AsDouble(h.ptr());
+  if (out != -1.0 || !PyErr_Occurred()) return true;
+  PyErr_Clear();      // an integer beyond a double's range
+  return false;
+}
+
 // One to three 2-D weights of one width that follow one another in one storage.
 struct Weights {
   Tensor t[3];
@@ -487,7 +506,10 @@ py::object rope(py::handle x_, py::handle cos_, py::handle sin_, int64_t heads, 
   if (!unobserved() || !unpack(x_, x) || !unpack(cos_, cos) || !unpack(sin_, sin) || !unpack(pos_, pos) || !plain_rows(x) ||
       !plain_rows(cos, at::kFloat) || !plain_rows(sin, at::kFloat) || recording(cos) || recording(sin))
     return py::none();
-  const int64_t c = x.size(-1), tokens = x.numel() / c, hs = head_stride_.is_none() || !head_stride_.cast<int64_t>() ? dim : head_stride_.cast<int64_t>();
+  const int64_t c = x.size(-1), tokens = x.numel() / c;
+  int64_t hs;
+  if (!whole(head_stride_, 0, hs)) return py::none();
+  if (hs == 0) hs = dim;
   if (cos.size(-1) != dim / 2 || sin.size(-1) != dim / 2 || !small(tokens) || !small(c)) return py::none();
   if (pos.defined() && (!plain_rows(pos, at::kInt) || pos.numel() != tokens)) return py::none();
   const bool rec = at::GradMode::is_enabled() && recording(x);
@@ -597,8 +619,9 @@ py::object attention_qkv(py::handle x_, int64_t hq, int64_t hkv, int64_t d, bool
       x.size(2) != (hq + 2 * hkv) * d || !small(x.size(0) * x.size(1)))
     return py::none();
   if (!per_token(seg_, x.size(0) * x.size(1), seg) || !per_token(pos_, x.size(0) * x.size(1), pos)) return py::none();
-  const double scale = scale_.is_none() ? 1.0 / std::sqrt((double)d) : scale_.cast<double>();
-  const int64_t window = window_.is_none() ? 0 : window_.cast<int64_t>();
+  double scale;
+  int64_t window;
+  if (!real(scale_, 1.0 / std::sqrt((double)d), scale) || !whole(window_, 0, window)) return py::none();
   {
     py::gil_scoped_release nogil;
     if (at::GradMode::is_enabled() && recording(x)) {
@@ -672,7 +695,10 @@ py::object attention(py::handle q_, py::handle k_, py::handle v_, bool causal, p
   if (!unobserved() || !unpack(q_, q) || !unpack(k_, k) || !unpack(v_, v) || !token_major(q) || !token_major(k) || !token_major(v))
     return py::none();
   const int64_t b = q.size(0), sq = q.size(1), sk = k.size(1), dqk = q.size(3);
-  const double softcap = softcap_.is_none() ? 0.0 : softcap_.cast<double>();
+  double softcap, scale;
+  int64_t window;
+  if (!real(softcap_, 0.0, softcap) || !real(scale_, 1.0 / std::sqrt((double)dqk), scale) || !whole(window_, 0, window))
+    return py::none();
   if (k.size(0) != b || v.size(0) != b || v.size(1) != sk || k.size(3) != dqk || v.size(3) != 128 || (dqk != 128 && dqk != 192) ||
       k.size(2) != v.size(2) || q.size(2) % k.size(2) || softcap < 0 || (softcap > 0 && dqk != 128) || one_storage(q, k, v) ||
       (dqk != 128 && sq > max_wide_queries) || !small(b * sq) || !small(b * sk))
@@ -684,8 +710,6 @@ py::object attention(py::handle q_, py::handle k_, py::handle v_, bool causal, p
   } else if (!per_token(kvseg_, b * sk, kv_seg)) {
     return py::none();
   }
-  const double scale = scale_.is_none() ? 1.0 / std::sqrt((double)dqk) : scale_.cast<double>();
-  const int64_t window = window_.is_none() ? 0 : window_.cast<int64_t>();
   {
     py::gil_scoped_release nogil;
     if (at::GradMode::is_enabled() && (recording(q) || recording(k) || recording(v))) {

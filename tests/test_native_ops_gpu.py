@@ -1,6 +1,7 @@
 """The native operators (csrc/torch_ops.cpp) give what the Python definitions give, call by call, and leave to those
 whatever they are not meant for."""
 
+import numpy as np
 import pytest
 import torch
 
@@ -289,3 +290,17 @@ def test_experts_without_gradients(cuda_lib, in_python, tokens, fused):
   in_python()
   for a, b in zip(got, call()):
     assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("window,scale,softcap", [(70.0, None, None), (np.int64(70), np.float32(0.25), None),
+                                                  (None, torch.tensor(0.25), 30), (70, 1, 30.0)])
+def test_options_given_as_other_numbers(cuda_lib, window, scale, softcap):
+  """What int() and float() take is taken, as by the Python definitions."""
+  _lib.lib()
+  plain = dict(window=None if window is None else int(window), scale=None if scale is None else float(scale))
+  cap = None if softcap is None else float(softcap)
+  q, k, v = _r(1, 100, 4, 128), _r(1, 100, 2, 128, seed=1), _r(1, 100, 2, 128, seed=2)
+  assert torch.equal(ops.attention(q, k, v, window=window, scale=scale, softcap=softcap),
+                     ops.attention(q, k, v, softcap=cap, **plain))
+  x = _r(1, 100, 8 * 128)
+  assert torch.equal(ops.attention_qkv(x, 4, 2, 128, window=window, scale=scale), ops.attention_qkv(x, 4, 2, 128, **plain))
