@@ -304,3 +304,47 @@ def test_options_given_as_other_numbers(cuda_lib, window, scale, softcap):
                      ops.attention(q, k, v, softcap=cap, **plain))
   x = _r(1, 100, 8 * 128)
   assert torch.equal(ops.attention_qkv(x, 4, 2, 128, window=window, scale=scale), ops.attention_qkv(x, 4, 2, 128, **plain))
+
+
+def _steps(seed, n=6):
+  """A few operators, forward and backward, in the current stream; what they give in the end."""
+  x = _r(2, 130, 256, grad=True, seed=seed)
+  ws = _adjacent((192, 256), (192, 256), grads=(True, True))
+  wd, wn, wq = _r(256, 192, grad=True, seed=1), _r(256, grad=True, seed=2), _r(6 * 128, 256, grad=True, seed=3)
+  cos, sin = _tables(130, 64)
+  leaves = [x, *ws, wd, wn, wq]
+  for t in leaves:
+    t.grad = None
+  for _ in range(n):
+    h, res = ops.rms_norm_residual(x, wn, 1e-5)
+    qkv = ops.rope_inplace(ops.linear(h, wq / 16), cos, sin, 5, 128, 130)
+    a = ops.attention_qkv(qkv, 4, 1, 128)
+    y = ops.swiglu_mlp(h, *ws, wd, res) + a.view(2, 130, 512)[..., :256]
+    y.backward(torch.linspace(-1, 1, y.numel(), device="cuda").view(y.shape).to(BF))
+  return [y.detach()] + [t.grad for t in leaves if t is not wn]      # (the norm's weight gradient is summed by atomics)
+
+
+def test_streams_and_threads(cuda_lib):
+  """Several threads, each in a stream of its own, give what one gives alone in the default stream."""
+  import threading
+  want = [_steps(s) for s in range(3)]
+  torch.cuda.synchronize()
+  got, errors = {}, []
+  def work(s):
+    try:
+      stream = torch.cuda.Stream()
+      with torch.cuda.stream(stream):
+        for _ in range(3):
+          got[s] = _steps(s)
+      stream.synchronize()
+    except BaseException as e:      # noqa: BLE001
+      errors.append(e)
+  threads = [threading.Thread(target=work, args=(s,)) for s in range(3)]
+  for t in threads:
+    t.start()
+  for t in threads:
+    t.join()
+  assert not errors, errors
+  for s in range(3):
+    for a, b in zip(got[s], want[s]):
+      assert torch.equal(a, b)
