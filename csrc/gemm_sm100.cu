@@ -714,8 +714,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
             if (p.epi == TPB_EPI_SWIGLU_BWD) {
               // The gradient of the activation never leaves the SM: dg and du are made from it here, with the gate and up
               // values of a lane's row read while the accumulator is (64 columns of each: one line, in eight loads).
-              // As a pass of its own this read and wrote the gradient once more: a decoder layer of 4096 tokens (14336 wide),
-              // forward and backward, 5150 us with it and 4950 without.
+              // As a pass of its own this read and wrote the gradient once more: 4096 x 14336 x 4096, product and pass 438 us,
+              // this way 414; a decoder layer of 4096 tokens (14336 wide), forward and backward, 5269 and 5152.
 #pragma unroll 1
               for (int c = 0; c < BN / 64; ++c) {
                 const int col = n0 + c * 64;
