@@ -348,3 +348,20 @@ def test_streams_and_threads(cuda_lib):
   for s in range(3):
     for a, b in zip(got[s], want[s]):
       assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("b,s", [(3, 1), (2, 2)])
+@pytest.mark.parametrize("native", [True, False])
+def test_one_token_per_row(cuda_lib, in_python, b, s, native):
+  """A fused projection of one token per row: every batch finds its own heads."""
+  _lib.lib()
+  if not native:
+    in_python()
+  x = _r(b, s, 6 * 128, grad=True)
+  y = ops.attention_qkv(x, 4, 1, 128, causal=False)
+  y.sum().backward()
+  for i in range(b):
+    one = x.detach()[i:i + 1].clone().requires_grad_(True)
+    z = ops.attention_qkv(one, 4, 1, 128, causal=False)
+    z.sum().backward()
+    assert torch.equal(y[i:i + 1], z) and torch.equal(x.grad[i:i + 1], one.grad)

@@ -215,6 +215,18 @@ class _AttentionFn(torch.autograd.Function):
     return dq, dk, dv, None, None, None, None, None, None, None
 
 
+def _qkv_views(t, hq, hkv, d):
+  """The query, key and value heads of a [B, S, (hq + 2 hkv) * d] tensor (rows may have a pitch).  For one token per row the
+  pitch is that of the batches: a view's stride would be the slice's, and batches would be read from the wrong place."""
+  b, s, _ = t.shape
+  pitch = t.stride(1) if s > 1 else t.stride(0)
+  at, out = t.storage_offset(), []
+  for n in (hq, hkv, hkv):
+    out.append(t.as_strided((b, s, n, d), (t.stride(0), pitch, d, 1), at))
+    at += n * d
+  return out
+
+
 class _AttentionQKVFn(torch.autograd.Function):
   """Attention on one fused projection output ``qkv`` [B, S, (Hq + 2 Hkv) * D] (queries, keys, values
   back to back in every row).  A single autograd input means a single gradient: the backward
@@ -226,9 +238,7 @@ class _AttentionQKVFn(torch.autograd.Function):
   @staticmethod
   def forward(ctx, qkv, hq, hkv, d, causal, scale, window, q_pos, q_seg, kv_seg):
     b, s, _ = qkv.shape
-    q = qkv[..., : hq * d].view(b, s, hq, d)
-    k = qkv[..., hq * d: (hq + hkv) * d].view(b, s, hkv, d)
-    v = qkv[..., (hq + hkv) * d:].view(b, s, hkv, d)
+    q, k, v = _qkv_views(qkv, hq, hkv, d)
     ranges = _seg_ranges(q_seg, kv_seg, b, s, s)
     o, lse = attn_fwd(q, k, v, causal, scale, window, q_pos, q_seg, kv_seg, ranges=ranges)
     ctx.save_for_backward(qkv, o, lse, q_pos, q_seg, kv_seg, *ranges)
@@ -240,13 +250,9 @@ class _AttentionQKVFn(torch.autograd.Function):
     qkv, o, lse, q_pos, q_seg, kv_seg, *ranges = ctx.saved_tensors
     hq, hkv, d, causal, scale, window = ctx.args
     b, s, _ = qkv.shape
-    q = qkv[..., : hq * d].view(b, s, hq, d)
-    k = qkv[..., hq * d: (hq + hkv) * d].view(b, s, hkv, d)
-    v = qkv[..., (hq + hkv) * d:].view(b, s, hkv, d)
+    q, k, v = _qkv_views(qkv, hq, hkv, d)
     buf = torch.empty_like(qkv)
-    dq = buf[..., : hq * d].view(b, s, hq, d)
-    dk = buf[..., hq * d: (hq + hkv) * d].view(b, s, hkv, d)
-    dv = buf[..., (hq + hkv) * d:].view(b, s, hkv, d)
+    dq, dk, dv = _qkv_views(buf, hq, hkv, d)
     attn_bwd(do, q, k, v, o, lse, causal, scale, window, q_pos, q_seg, kv_seg, dq, dk, dv, ranges=ranges)
     return buf, None, None, None, None, None, None, None, None, None
 
