@@ -233,7 +233,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   int* tile_max = tile_min + KV_MAX_TILES;
   uint8_t* seg_one = smem + OFF_SEGONE;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   // linear block id is key-block major so that under a causal mask the blocks with the most
   // visible query tiles (lowest key index) are scheduled first on every head
   const int kb = blockIdx.x / (p.Hkv * p.B);
@@ -361,7 +361,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_steps > 0) {
+    if (n_steps > 0) {
       constexpr uint32_t id_s = make_idesc_bf16(BWD_T, BWD_T, false, false);    // S^T, dP^T
       constexpr uint32_t id_acc = make_idesc_bf16(BWD_T, BWD_D, false, true);   // dV, dK (A in TMEM, B MN-major)
       const uint32_t dK = kmajor_lo(smem_u32(smem + OFF_K)), dVd = kmajor_lo(smem_u32(smem + OFF_V));
@@ -370,33 +370,31 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       // The MMA queue is shallow, so whatever this thread does between two MMAs is tensor idle
       // time: every wait is therefore placed before the LAST MMA of the preceding group, where
       // its latency hides behind the seven MMAs still in flight.
-      auto wait_q = [&](int i) { return mbar_wait(&q_full[i % KV_QSTAGES], (i / KV_QSTAGES) & 1, p.status, kTimeoutTmaFull, 23); };
-      auto wait_do = [&](int i) { return mbar_wait(&do_full[i % KV_DOSTAGES], (i / KV_DOSTAGES) & 1, p.status, kTimeoutTmaFull, 24); };
-      auto wait_p = [&](int i) { return mbar_wait(p_full, i & 1, p.status, kTimeoutSoftmax, 25); };
-      auto wait_ds = [&](int i) { return mbar_wait(ds_full, i & 1, p.status, kTimeoutSoftmax, 26); };
-      auto group = [&](auto&& mma, auto&& hook) -> bool {
+      auto wait_q = [&](int i) { return mbar_wait_warp(&q_full[i % KV_QSTAGES], (i / KV_QSTAGES) & 1, p.status, kTimeoutTmaFull, 23); };
+      auto wait_do = [&](int i) { return mbar_wait_warp(&do_full[i % KV_DOSTAGES], (i / KV_DOSTAGES) & 1, p.status, kTimeoutTmaFull, 24); };
+      auto wait_p = [&](int i) { return mbar_wait_warp(p_full, i & 1, p.status, kTimeoutSoftmax, 25); };
+      auto wait_ds = [&](int i) { return mbar_wait_warp(ds_full, i & 1, p.status, kTimeoutSoftmax, 26); };
+      auto group = [&](auto&& mma, auto&& hook, auto&& done) -> bool {
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < 7; ++k) mma(k);
+          for (int k = 0; k < 7; ++k) mma(k);
+        });
         if (!hook()) return false;
         tc_fence_after();
-        mma(7);
+        one_lane([&] { mma(7); done(); });
         return true;
       };
-      bool ok = mbar_wait(kv_full, 0, p.status, kTimeoutTmaFull, 22) && wait_q(0);
+      bool ok = mbar_wait_warp(kv_full, 0, p.status, kTimeoutTmaFull, 22) && wait_q(0);
       tc_fence_after();
       auto issue_s = [&](int i, auto&& hook) -> bool {      // S^T(i) = K Q(i)^T
         const uint32_t dQ = kmajor_lo(aQ0 + (i % KV_QSTAGES) * TILE_BYTES);
-        if (!group([&](int k) { mma_ss_w(tS, dK + kmajor_k(k), kDescHi, dQ + kmajor_k(k), kDescHi, id_s, k != 0); }, hook))
-          return false;
-        tc_commit(s_full);
-        return true;
+        return group([&](int k) { mma_ss_w(tS, dK + kmajor_k(k), kDescHi, dQ + kmajor_k(k), kDescHi, id_s, k != 0); }, hook,
+                     [&] { tc_commit(s_full); });
       };
       auto issue_dp = [&](int i, auto&& hook) -> bool {     // dP^T(i) = V dO(i)^T
         const uint32_t dDO = kmajor_lo(aDO0 + (i % KV_DOSTAGES) * TILE_BYTES);
-        if (!group([&](int k) { mma_ss_w(tDP, dVd + kmajor_k(k), kDescHi, dDO + kmajor_k(k), kDescHi, id_s, k != 0); }, hook))
-          return false;
-        tc_commit(dp_full);
-        return true;
+        return group([&](int k) { mma_ss_w(tDP, dVd + kmajor_k(k), kDescHi, dDO + kmajor_k(k), kDescHi, id_s, k != 0); }, hook,
+                     [&] { tc_commit(dp_full); });
       };
       auto none = [] { return true; };
       if (ok) ok = issue_s(0, [&] { return wait_do(0); });
@@ -411,20 +409,18 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         tc_fence_after();
         // dV += P^T dO
         ok = group([&](int k) { mma_ts_w(tmem_base + T_DV, tS + a_col(k), mDO + mnmajor_k(k), kDescHi, id_acc, (i | k) != 0); },
-                   [&] { return more ? wait_q(i + 1) : true; });
+                   [&] { return more ? wait_q(i + 1) : true; }, [&] { tc_commit(&do_empty[i % KV_DOSTAGES]); });
         if (!ok) break;
-        tc_commit(&do_empty[i % KV_DOSTAGES]);
         if (more && !issue_s(i + 1, none)) break;
         if (!wait_ds(i)) break;
         tc_fence_after();
         // dK += dS^T Q
         ok = group([&](int k) { mma_ts_w(tmem_base + T_DK, tDP + a_col(k), mQ + mnmajor_k(k), kDescHi, id_acc, (i | k) != 0); },
-                   [&] { return more ? wait_do(i + 1) : true; });
+                   [&] { return more ? wait_do(i + 1) : true; }, [&] { tc_commit(&q_empty[i % KV_QSTAGES]); });
         if (!ok) break;
-        tc_commit(&q_empty[i % KV_QSTAGES]);
         if (more && !issue_dp(i + 1, none)) break;
       }
-      tc_commit(acc_done);
+      one_lane([&] { tc_commit(acc_done); });
     }
   } else {
     // ------------------------------------------------------------------ compute warps
@@ -614,7 +610,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   int* tile_minmax = reinterpret_cast<int*>(s_full + 6);  // [2]
   int* seg_lohi = reinterpret_cast<int*>(s_full + 7);     // [2] first and last key block with a segment of this tile
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_qtiles = (p.Sq + BWD_T - 1) / BWD_T;
   // heaviest (latest) query tiles first under a causal mask
   const int qt = n_qtiles - 1 - (int)(blockIdx.x / (p.Hq * p.B));
@@ -678,7 +674,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0 && elect_one()) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
       mbar_expect_tx(qdo_full, 2 * TILE_BYTES);
 #pragma unroll
@@ -703,41 +699,38 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0) {
       constexpr uint32_t id_s = make_idesc_bf16(BWD_T, BWD_T, false, false);    // S, dP
       constexpr uint32_t id_dq = make_idesc_bf16(BWD_T, BWD_D, false, true);    // dQ (A in TMEM, B MN-major)
       const uint32_t dQ = kmajor_lo(smem_u32(smem + OFF_Q)), dDO = kmajor_lo(smem_u32(smem + OFF_DO));
       const uint32_t aK0 = smem_u32(smem + OFF_K), aV0 = smem_u32(smem + OFF_V);
       const uint32_t tDP = tmem_base + T_DP;
       // Waits sit before the last MMA of the preceding group (see the dK/dV kernel).
-      auto wait_k = [&](int j) { return mbar_wait(&k_full[j % DQ_KSTAGES], (j / DQ_KSTAGES) & 1, p.status, kTimeoutTmaFull, 33); };
-      auto wait_v = [&](int j) { return mbar_wait(&v_full[j % DQ_VSTAGES], (j / DQ_VSTAGES) & 1, p.status, kTimeoutTmaFull, 37); };
-      auto wait_ds = [&](int j) { return mbar_wait(ds_full, j & 1, p.status, kTimeoutSoftmax, 34); };
-      auto group = [&](auto&& mma, auto&& hook) -> bool {
+      auto wait_k = [&](int j) { return mbar_wait_warp(&k_full[j % DQ_KSTAGES], (j / DQ_KSTAGES) & 1, p.status, kTimeoutTmaFull, 33); };
+      auto wait_v = [&](int j) { return mbar_wait_warp(&v_full[j % DQ_VSTAGES], (j / DQ_VSTAGES) & 1, p.status, kTimeoutTmaFull, 37); };
+      auto wait_ds = [&](int j) { return mbar_wait_warp(ds_full, j & 1, p.status, kTimeoutSoftmax, 34); };
+      auto group = [&](auto&& mma, auto&& hook, auto&& done) -> bool {
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < 7; ++k) mma(k);
+          for (int k = 0; k < 7; ++k) mma(k);
+        });
         if (!hook()) return false;
         tc_fence_after();
-        mma(7);
+        one_lane([&] { mma(7); done(); });
         return true;
       };
-      bool ok = mbar_wait(qdo_full, 0, p.status, kTimeoutTmaFull, 32) && wait_k(0);
+      bool ok = mbar_wait_warp(qdo_full, 0, p.status, kTimeoutTmaFull, 32) && wait_k(0);
       tc_fence_after();
       auto issue_s = [&](int j, auto&& hook) -> bool {      // S(j) = Q K_j^T
         const uint32_t dK = kmajor_lo(aK0 + (j % DQ_KSTAGES) * TILE_BYTES);
         const uint32_t tS = tmem_base + T_S + (j & 1) * BWD_T;
-        if (!group([&](int k) { mma_ss_w(tS, dQ + kmajor_k(k), kDescHi, dK + kmajor_k(k), kDescHi, id_s, k != 0); }, hook))
-          return false;
-        tc_commit(&s_full[j & 1]);
-        return true;
+        return group([&](int k) { mma_ss_w(tS, dQ + kmajor_k(k), kDescHi, dK + kmajor_k(k), kDescHi, id_s, k != 0); }, hook,
+                     [&] { tc_commit(&s_full[j & 1]); });
       };
       auto issue_dp = [&](int j, auto&& hook) -> bool {     // dP(j) = dO V_j^T
         const uint32_t dV = kmajor_lo(aV0 + (j % DQ_VSTAGES) * TILE_BYTES);
-        if (!group([&](int k) { mma_ss_w(tDP, dDO + kmajor_k(k), kDescHi, dV + kmajor_k(k), kDescHi, id_s, k != 0); }, hook))
-          return false;
-        tc_commit(&v_empty[j % DQ_VSTAGES]);
-        tc_commit(dp_full);
-        return true;
+        return group([&](int k) { mma_ss_w(tDP, dDO + kmajor_k(k), kDescHi, dV + kmajor_k(k), kDescHi, id_s, k != 0); }, hook,
+                     [&] { tc_commit(&v_empty[j % DQ_VSTAGES]); tc_commit(dp_full); });
       };
       auto none = [] { return true; };
       if (ok) ok = issue_s(0, [&] { return wait_v(0); });
@@ -750,12 +743,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const uint32_t mK = mnmajor_lo(aK0 + (j % DQ_KSTAGES) * TILE_BYTES);
         // dQ += dS K   (K tile [128 keys][128 d]: N = d contiguous)
         ok = group([&](int k) { mma_ts_w(tmem_base + T_DQ, tDP + a_col(k), mK + mnmajor_k(k), kDescHi, id_dq, (j | k) != 0); },
-                   [&] { return more ? wait_v(j + 1) : true; });
+                   [&] { return more ? wait_v(j + 1) : true; }, [&] { tc_commit(&k_empty[j % DQ_KSTAGES]); });
         if (!ok) break;
-        tc_commit(&k_empty[j % DQ_KSTAGES]);
         if (more && !issue_dp(j + 1, [&] { return j + 2 < nblk ? wait_k(j + 2) : true; })) break;
       }
-      tc_commit(acc_done);
+      one_lane([&] { tc_commit(acc_done); });
     }
   } else {
     // ------------------------------------------------------------------ compute warps
@@ -991,7 +983,7 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   int* tile_max = tile_min + W_MAX_TILES;
   uint8_t* seg_one = smem + OFF_SEGONE;
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int kb = blockIdx.x / (p.Hkv * p.B);      // key-block major: the heaviest blocks first under a causal mask
   const int hkv = (blockIdx.x / p.B) % p.Hkv, b = blockIdx.x % p.B;
   const int G = p.Hq / p.Hkv;
@@ -1117,7 +1109,7 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && n_steps > 0) {
+    if (n_steps > 0) {
       constexpr uint32_t id_s = make_idesc_bf16(BWD_T, W_QT, false, false);     // S^T, dP^T
       constexpr uint32_t id_dv = make_idesc_bf16(BWD_T, BWD_D, false, true);    // dV (A in TMEM, B MN-major)
       constexpr uint32_t id_dk = make_idesc_bf16(BWD_T, W_D, false, true);      // dK
@@ -1128,57 +1120,65 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       // whose halves of 32 values lie packed at the start of their own 32 columns (FINE: second terms behind them)
       auto kstep = [](int rows, int k) { return (uint32_t)(((k >> 2) * (rows * 128) + (k & 3) * 32) >> 4); };
       auto acol = [](int k) { return (uint32_t)((k >> 1) * 32 + (k & 1) * 8); };
-      auto wait_q = [&](int i) { return mbar_wait(&q_full[i % W_STAGES], (i / W_STAGES) & 1, p.status, kTimeoutTmaFull, 123); };
-      auto wait_do = [&](int i) { return mbar_wait(&do_full[i % W_STAGES], (i / W_STAGES) & 1, p.status, kTimeoutTmaFull, 124); };
+      auto wait_q = [&](int i) { return mbar_wait_warp(&q_full[i % W_STAGES], (i / W_STAGES) & 1, p.status, kTimeoutTmaFull, 123); };
+      auto wait_do = [&](int i) { return mbar_wait_warp(&do_full[i % W_STAGES], (i / W_STAGES) & 1, p.status, kTimeoutTmaFull, 124); };
       auto issue_s = [&](int i) -> bool {      // S^T(i) = K Q(i)^T
         if (!wait_q(i)) return false;
         tc_fence_after();
         const uint32_t dQ = kmajor_lo(aQ0 + (i % W_STAGES) * W_Q_BYTES);
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < W_D / 16; ++k)
-          mma_ss_w(tmem_base + T_S + (i & 1) * W_QT, dK + kstep(BWD_T, k), kDescHi, dQ + kstep(W_QT, k), kDescHi, id_s, k != 0);
-        tc_commit(&s_full[i & 1]);
+          for (int k = 0; k < W_D / 16; ++k)
+            mma_ss_w(tmem_base + T_S + (i & 1) * W_QT, dK + kstep(BWD_T, k), kDescHi, dQ + kstep(W_QT, k), kDescHi, id_s, k != 0);
+          tc_commit(&s_full[i & 1]);
+        });
         return true;
       };
       auto issue_dp = [&](int i) -> bool {     // dP^T(i) = V dO(i)^T
         if (!wait_do(i)) return false;
         tc_fence_after();
         const uint32_t dDO = kmajor_lo(aDO0 + (i % W_STAGES) * W_DO_BYTES);
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < BWD_D / 16; ++k)
-          mma_ss_w(tDP, dVd + kstep(BWD_T, k), kDescHi, dDO + kstep(W_QT, k), kDescHi, id_s, k != 0);
-        tc_commit(dp_full);
+          for (int k = 0; k < BWD_D / 16; ++k)
+            mma_ss_w(tDP, dVd + kstep(BWD_T, k), kDescHi, dDO + kstep(W_QT, k), kDescHi, id_s, k != 0);
+          tc_commit(dp_full);
+        });
         return true;
       };
-      bool ok = mbar_wait(kv_full, 0, p.status, kTimeoutTmaFull, 122);
+      bool ok = mbar_wait_warp(kv_full, 0, p.status, kTimeoutTmaFull, 122);
       if (ok) ok = issue_s(0) && issue_dp(0);
       for (int i = 0; i < n_steps && ok; ++i) {
         const int st = i % W_STAGES;
         const bool more = i + 1 < n_steps;
         // its buffer held P^T(i - 1), which dV(i - 1), issued before, has read by then
         if (more && !issue_s(i + 1)) break;
-        if (!mbar_wait(&p_full[i & 1], (i >> 1) & 1, p.status, kTimeoutSoftmax, 125)) break;
+        if (!mbar_wait_warp(&p_full[i & 1], (i >> 1) & 1, p.status, kTimeoutSoftmax, 125)) break;
         tc_fence_after();
         const uint32_t mDO = smem_desc_lo(aDO0 + st * W_DO_BYTES, W_QT * 128);
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < W_QT / 16; ++k) {  // dV += P^T dO
-          const uint32_t a = tmem_base + T_S + (i & 1) * W_QT + acol(k);
-          mma_ts_w(tmem_base + T_DV, a, mDO + mnmajor_k(k), kDescHi, id_dv, (i | k) != 0);
-          if (FINE) mma_ts_w(tmem_base + T_DV, a + 16, mDO + mnmajor_k(k), kDescHi, id_dv, 1);
-        }
-        tc_commit(&do_empty[st]);
-        if (!mbar_wait(ds_full, i & 1, p.status, kTimeoutSoftmax, 126)) break;
+          for (int k = 0; k < W_QT / 16; ++k) {  // dV += P^T dO
+            const uint32_t a = tmem_base + T_S + (i & 1) * W_QT + acol(k);
+            mma_ts_w(tmem_base + T_DV, a, mDO + mnmajor_k(k), kDescHi, id_dv, (i | k) != 0);
+            if (FINE) mma_ts_w(tmem_base + T_DV, a + 16, mDO + mnmajor_k(k), kDescHi, id_dv, 1);
+          }
+          tc_commit(&do_empty[st]);
+        });
+        if (!mbar_wait_warp(ds_full, i & 1, p.status, kTimeoutSoftmax, 126)) break;
         tc_fence_after();
         const uint32_t mQ = smem_desc_lo(aQ0 + st * W_Q_BYTES, W_QT * 128);
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < W_QT / 16; ++k) {  // dK += dS^T Q
-          mma_ts_w(tmem_base + T_DK, tDP + acol(k), mQ + mnmajor_k(k), kDescHi, id_dk, (i | k) != 0);
-          if (FINE) mma_ts_w(tmem_base + T_DK, tDP + acol(k) + 16, mQ + mnmajor_k(k), kDescHi, id_dk, 1);
-        }
-        tc_commit(&q_empty[st]);
+          for (int k = 0; k < W_QT / 16; ++k) {  // dK += dS^T Q
+            mma_ts_w(tmem_base + T_DK, tDP + acol(k), mQ + mnmajor_k(k), kDescHi, id_dk, (i | k) != 0);
+            if (FINE) mma_ts_w(tmem_base + T_DK, tDP + acol(k) + 16, mQ + mnmajor_k(k), kDescHi, id_dk, 1);
+          }
+          tc_commit(&q_empty[st]);
+        });
         if (more && !issue_dp(i + 1)) break;
       }
-      tc_commit(acc_done);
+      one_lane([&] { tc_commit(acc_done); });
     }
   } else {
     // ------------------------------------------------------------------ compute warps
@@ -1311,7 +1311,7 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   int* seg_lohi = reinterpret_cast<int*>(bars + 14);      // [2]
   float* red = reinterpret_cast<float*>(smem + OFF_RED);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_qtiles = (p.Sq + BWD_T - 1) / BWD_T;
   const int qt = n_qtiles - 1 - (int)(blockIdx.x / (p.Hq * p.B));   // heaviest query tiles first
   const int hq = (blockIdx.x / p.B) % p.Hq, b = blockIdx.x % p.B;
@@ -1376,7 +1376,7 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0 && elect_one()) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
       mbar_expect_tx(qdo_full, W_K_BYTES + TILE_BYTES);
       for (int c = 0; c < W_D / 64; ++c)
@@ -1398,7 +1398,7 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0) {
       constexpr uint32_t id_s = make_idesc_bf16(BWD_T, BWD_T, false, false);    // S, dP
       constexpr uint32_t id_dq = make_idesc_bf16(BWD_T, W_D, false, true);      // dQ (A in TMEM, B MN-major)
       const uint32_t dQ = kmajor_lo(smem_u32(smem + OFF_Q)), dDO = kmajor_lo(smem_u32(smem + OFF_DO));
@@ -1407,47 +1407,53 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
       const uint32_t tS = tmem_base + T_S, tDP = tmem_base + T_DP;
       auto kstep = [](int k) { return (uint32_t)(((k >> 2) * (BWD_T * 128) + (k & 3) * 32) >> 4); };
       auto issue_s = [&](int j) -> bool {      // S(j) = Q K_j^T
-        if (!mbar_wait(&k_full[j & 1], (j >> 1) & 1, p.status, kTimeoutTmaFull, 133)) return false;
+        if (!mbar_wait_warp(&k_full[j & 1], (j >> 1) & 1, p.status, kTimeoutTmaFull, 133)) return false;
         tc_fence_after();
         const uint32_t dK = kmajor_lo(aK0 + (j & 1) * W_K_BYTES);
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < W_D / 16; ++k) mma_ss_w(tS, dQ + kstep(k), kDescHi, dK + kstep(k), kDescHi, id_s, k != 0);
-        tc_commit(s_full);
+          for (int k = 0; k < W_D / 16; ++k) mma_ss_w(tS, dQ + kstep(k), kDescHi, dK + kstep(k), kDescHi, id_s, k != 0);
+          tc_commit(s_full);
+        });
         return true;
       };
       auto issue_dp = [&](int j) -> bool {     // dP(j) = dO V_j^T
-        if (!mbar_wait(v_full, j & 1, p.status, kTimeoutTmaFull, 137)) return false;
+        if (!mbar_wait_warp(v_full, j & 1, p.status, kTimeoutTmaFull, 137)) return false;
         tc_fence_after();
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < BWD_D / 16; ++k) mma_ss_w(tDP, dDO + kstep(k), kDescHi, dV + kstep(k), kDescHi, id_s, k != 0);
-        tc_commit(v_empty);
-        tc_commit(dp_full);
+          for (int k = 0; k < BWD_D / 16; ++k) mma_ss_w(tDP, dDO + kstep(k), kDescHi, dV + kstep(k), kDescHi, id_s, k != 0);
+          tc_commit(v_empty);
+          tc_commit(dp_full);
+        });
         return true;
       };
-      bool ok = mbar_wait(qdo_full, 0, p.status, kTimeoutTmaFull, 132);
+      bool ok = mbar_wait_warp(qdo_full, 0, p.status, kTimeoutTmaFull, 132);
       if (ok) ok = issue_s(0) && issue_dp(0);
       for (int j = 0; j < n_steps && ok; ++j) {
         const bool more = j + 1 < n_steps;
         const int jq = FINE ? j - nblk : j;      // step of the dQ pass
         if (more) {
-          if (!mbar_wait(s_read, j & 1, p.status, kTimeoutSoftmax, 140)) break;   // S(j) is in registers
+          if (!mbar_wait_warp(s_read, j & 1, p.status, kTimeoutSoftmax, 140)) break;   // S(j) is in registers
           tc_fence_after();
           if (!issue_s(j + 1)) break;
         }
-        if (!mbar_wait(ds_full, j & 1, p.status, kTimeoutSoftmax, 134)) break;
+        if (!mbar_wait_warp(ds_full, j & 1, p.status, kTimeoutSoftmax, 134)) break;
         tc_fence_after();
         const uint32_t mK = mnmajor_lo(aK0 + (j & 1) * W_K_BYTES);
-        if (jq >= 0) {
+        one_lane([&] {
+          if (jq >= 0) {
 #pragma unroll
-          for (int k = 0; k < BWD_T / 16; ++k) {   // dQ += dS K
-            mma_ts_w(tmem_base + T_DQ, tDP + a_col(k), mK + mnmajor_k(k), kDescHi, id_dq, (jq | k) != 0);
-            if (FINE) mma_ts_w(tmem_base + T_DQ, tDP + a_col(k) + 32, mK + mnmajor_k(k), kDescHi, id_dq, 1);
+            for (int k = 0; k < BWD_T / 16; ++k) {   // dQ += dS K
+              mma_ts_w(tmem_base + T_DQ, tDP + a_col(k), mK + mnmajor_k(k), kDescHi, id_dq, (jq | k) != 0);
+              if (FINE) mma_ts_w(tmem_base + T_DQ, tDP + a_col(k) + 32, mK + mnmajor_k(k), kDescHi, id_dq, 1);
+            }
           }
-        }
-        tc_commit(&k_empty[j & 1]);
+          tc_commit(&k_empty[j & 1]);
+        });
         if (more && !issue_dp(j + 1)) break;
       }
-      tc_commit(acc_done);
+      one_lane([&] { tc_commit(acc_done); });
     }
   } else {
     // ------------------------------------------------------------------ compute warps

@@ -268,7 +268,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   int* tile_minmax = reinterpret_cast<int*>(bars + 15);  // [2]
   int* seg_lohi = reinterpret_cast<int*>(bars + 16);     // [2] first and last key block with a segment of this tile
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_qtiles = (p.Sq + FWD_BM - 1) / FWD_BM;
   int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
   if (p.cp_world > 1) {
@@ -351,7 +351,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0 && elect_one()) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
       mbar_expect_tx(q_full, L::Q_BYTES);
 #pragma unroll
@@ -376,25 +376,27 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0) {
       constexpr uint32_t idesc_qk = make_idesc_bf16(FWD_BM, FWD_BN, false, false);
       constexpr uint32_t idesc_pv = make_idesc_bf16(FWD_BM, FWD_DV, false, true);
       const uint32_t tS = tmem_base, tO = tmem_base + 128;
-      bool ok = mbar_wait(q_full, 0, p.status, kTimeoutTmaFull, 13);
+      bool ok = mbar_wait_warp(q_full, 0, p.status, kTimeoutTmaFull, 13);
       tc_fence_after();
       auto issue_qk = [&](int j) -> bool {
         const int s = j & 1;
-        if (!mbar_wait(&k_full[s], (j >> 1) & 1, p.status, kTimeoutTmaFull, 14)) return false;
+        if (!mbar_wait_warp(&k_full[s], (j >> 1) & 1, p.status, kTimeoutTmaFull, 14)) return false;
         tc_fence_after();
         const uint32_t aQ = smem_u32(sQ), aK = smem_u32(sK + s * L::K_BYTES);
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < DQK / 16; ++k) {
-          const uint64_t qd = make_smem_desc(aQ + (k >> 2) * (FWD_BM * 128) + (k & 3) * 32, 16, 1024);
-          const uint64_t kd = make_smem_desc(aK + (k >> 2) * (FWD_BN * 128) + (k & 3) * 32, 16, 1024);
-          mma_ss(tS + s * FWD_BN, qd, kd, idesc_qk, k != 0);
-        }
-        tc_commit(&k_empty[s]);
-        tc_commit(&s_full[s]);
+          for (int k = 0; k < DQK / 16; ++k) {
+            const uint64_t qd = make_smem_desc(aQ + (k >> 2) * (FWD_BM * 128) + (k & 3) * 32, 16, 1024);
+            const uint64_t kd = make_smem_desc(aK + (k >> 2) * (FWD_BN * 128) + (k & 3) * 32, 16, 1024);
+            mma_ss(tS + s * FWD_BN, qd, kd, idesc_qk, k != 0);
+          }
+          tc_commit(&k_empty[s]);
+          tc_commit(&s_full[s]);
+        });
         return true;
       };
       if (ok) ok = issue_qk(0);
@@ -404,18 +406,20 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
         if (j + 1 < nblk) {
           if (!issue_qk(j + 1)) break;
         }
-        if (!mbar_wait(&p_full[s], ph, p.status, kTimeoutSoftmax, 15)) break;
-        if (!mbar_wait(&v_full[s], ph, p.status, kTimeoutTmaFull, 16)) break;
+        if (!mbar_wait_warp(&p_full[s], ph, p.status, kTimeoutSoftmax, 15)) break;
+        if (!mbar_wait_warp(&v_full[s], ph, p.status, kTimeoutTmaFull, 16)) break;
         tc_fence_after();
         const uint32_t aV = smem_u32(sV + s * L::V_BYTES);
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < FWD_BN / 16; ++k) {
-          // V tile is [64 keys][128 d] in two 64-wide d blocks: MN-major B (N = d contiguous)
-          const uint64_t vd = make_smem_desc(aV + k * 2048, FWD_BN * 128, 1024);
-          mma_ts(tO, tS + s * FWD_BN + k * 8, vd, idesc_pv, (j | k) != 0);
-        }
-        tc_commit(&v_empty[s]);
-        tc_commit(o_done);
+          for (int k = 0; k < FWD_BN / 16; ++k) {
+            // V tile is [64 keys][128 d] in two 64-wide d blocks: MN-major B (N = d contiguous)
+            const uint64_t vd = make_smem_desc(aV + k * 2048, FWD_BN * 128, 1024);
+            mma_ts(tO, tS + s * FWD_BN + k * 8, vd, idesc_pv, (j | k) != 0);
+          }
+          tc_commit(&v_empty[s]);
+          tc_commit(o_done);
+        });
       }
     }
   } else {
@@ -665,7 +669,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   int* tile_minmax = reinterpret_cast<int*>(bars + 16);  // [2 tiles][2]
   int* pair_fail = reinterpret_cast<int*>(bars + 18);    // [2 tiles][4 quarters][2 halves]: that softmax warp gave up waiting
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_ctiles = (p.Sq + 2 * F2_T - 1) / (2 * F2_T);
   const int ct = n_ctiles - 1 - (int)(blockIdx.x / (p.Hq * p.B));   // heaviest (latest) rows first
   const int hq = (blockIdx.x / p.B) % p.Hq, b = blockIdx.x % p.B;
@@ -726,7 +730,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   setmaxnreg_dec<F2_REGS_IO>();
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0 && elect_one()) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
       mbar_expect_tx(q_full, 2 * F2_TILE_BYTES);
 #pragma unroll
@@ -757,20 +761,21 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
     // themselves the two fall into step, both tiles in their softmax at the same time; made to take
     // turns through a pair of mbarriers they were slower than this single thread, 0.655 against
     // 0.594 ms at S = 8192.)
-    if (lane == 0 && nblk > 0) {
+    if (nblk > 0) {
       constexpr uint32_t id_qk = make_idesc_bf16(F2_T, F2_T, false, false);
       constexpr uint32_t id_pv = make_idesc_bf16(F2_T, FWD_DV, false, true);
       constexpr uint32_t hi_w = smem_desc_hi(1024);
       const uint32_t qlo[2] = {smem_desc_lo(smem_u32(smem + OFF_Q), 16),
                                smem_desc_lo(smem_u32(smem + OFF_Q + F2_TILE_BYTES), 16)};
       const uint32_t k0 = smem_u32(smem + OFF_K), v0 = smem_u32(smem + OFF_V);
-      bool ok = mbar_wait(q_full, 0, p.status, kTimeoutTmaFull, 43);
+      bool ok = mbar_wait_warp(q_full, 0, p.status, kTimeoutTmaFull, 43);
       tc_fence_after();
       int steps[2] = {0, 0};   // steps issued per tile (barrier phases)
       PROF_K_DECL
       auto issue_s = [&](int x, int j) {   // S_x = Q_x K_j^T
         PROF_K_START
         const uint32_t klo = smem_desc_lo(k0 + (j & 1) * F2_TILE_BYTES, 16);
+        one_lane([&] {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           const uint32_t kk = (uint32_t)(((k >> 2) * (F2_T * 128) + (k & 3) * 32) >> 4);
@@ -778,10 +783,12 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           PROF_K_MARK(8 + k)
         }
         tc_commit(&s_full[x]);
+        });
       };
       auto issue_pv = [&](int x, int j, bool first) {   // O_x += P_x V_j
         PROF_K_START
         const uint32_t vlo = smem_desc_lo(v0 + (j & 1) * F2_TILE_BYTES, F2_T * 128);
+        one_lane([&] {
 #pragma unroll
         for (int k = 0; k < 8; ++k) {
           mma_ts_w(tmem_base + 256 + x * F2_T, tmem_base + x * F2_T + k * 8, vlo + (uint32_t)((k * 2048) >> 4), hi_w,
@@ -789,26 +796,27 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           PROF_K_MARK(k)
         }
         tc_commit(&o_done[x]);
+        });
       };
-      if (ok) ok = mbar_wait(&k_full[0], 0, p.status, kTimeoutTmaFull, 44);
+      if (ok) ok = mbar_wait_warp(&k_full[0], 0, p.status, kTimeoutTmaFull, 44);
       tc_fence_after();
       if (ok) {
         if (active(0, 0)) issue_s(0, 0);
         if (active(1, 0)) issue_s(1, 0);
-        tc_commit(&k_empty[0]);
+        one_lane([&] { tc_commit(&k_empty[0]); });
       }
       PROF_I_DECL(7)
       for (int j = 0; j < nblk && ok; ++j) {
         const int jn = j + 1;
         // the tiles this step needs were requested a step ago: these waits are off the softmax handshake
-        if (!mbar_wait(&v_full[j & 1], (j >> 1) & 1, p.status, kTimeoutTmaFull, 46)) { ok = false; break; }
-        if (jn < nblk && !mbar_wait(&k_full[jn & 1], (jn >> 1) & 1, p.status, kTimeoutTmaFull, 47)) { ok = false; break; }
+        if (!mbar_wait_warp(&v_full[j & 1], (j >> 1) & 1, p.status, kTimeoutTmaFull, 46)) { ok = false; break; }
+        if (jn < nblk && !mbar_wait_warp(&k_full[jn & 1], (jn >> 1) & 1, p.status, kTimeoutTmaFull, 47)) { ok = false; break; }
         PROF_I_MARK(5)
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
           if (active(x, j)) {
             PROF_I_MARK(0)
-            if (!mbar_wait(&p_full[x], steps[x] & 1, p.status, kTimeoutSoftmax, 45)) { ok = false; break; }
+            if (!mbar_wait_warp(&p_full[x], steps[x] & 1, p.status, kTimeoutSoftmax, 45)) { ok = false; break; }
             PROF_I_MARK(1)
             PROF_I_COUNT(2)
             tc_fence_after();
@@ -822,8 +830,10 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
           }
         }
         if (!ok) break;
-        tc_commit(&v_empty[j & 1]);
-        if (jn < nblk) tc_commit(&k_empty[jn & 1]);
+        one_lane([&] {
+          tc_commit(&v_empty[j & 1]);
+          if (jn < nblk) tc_commit(&k_empty[jn & 1]);
+        });
         PROF_I_MARK(3)
       }
       PROF_I_FLUSH(8, 7, TPB_ATTN_PROF_LEVEL != 3)

@@ -122,6 +122,22 @@ __device__ __forceinline__ bool elect_one() {
   return pred != 0;
 }
 
+// The warp's index in its block, the same value in every lane as far as the compiler can see: branches on it, and
+// what only depends on it, need no per-lane registers.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
+// Runs `f` in one lane of the whole warp, the same one every time.  Tensor-core instructions take their descriptors from the
+// registers that a warp's lanes share.  A warp that stays together around them (loops and waits in every lane, mbar_wait_warp,
+// and only the instructions themselves in one) has them there; in a branch on the lane's number the compiler fetches each
+// operand from a lane's registers before each MMA, and the tensor core waits.  us, branch around the whole role / this way:
+// attention backward of 8192 tokens, 32/8 heads, 1625 / 1520, of 4096 454 / 417; forward of 8192 543 / 526;
+// 4096 x 14336 x 4096 product 330 / 315.
+template <typename F>
+__device__ __forceinline__ void one_lane(F&& f) {
+  if (elect_one()) f();
+  __syncwarp();
+}
+
 // ----------------------------------------------------------------------------
 // mbarrier
 // ----------------------------------------------------------------------------
@@ -158,6 +174,22 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* s
       if (mbar_test(bar, parity)) return true;
     if (clock64() - t0 > kSpinBudgetCycles) {
       report(st, code, where);
+      return false;
+    }
+  }
+}
+
+// The same for a whole warp, which stays together: every lane gets the same answer.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int* st, int code, int where) {
+  if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+  const long long t0 = clock64();
+  while (true) {
+#pragma unroll 1
+    for (int i = 0; i < 64; ++i)
+      if (__all_sync(0xffffffffu, mbar_test(bar, parity))) return true;
+    if (__any_sync(0xffffffffu, clock64() - t0 > kSpinBudgetCycles)) {
+      if (elect_one()) report(st, code, where);
+      __syncwarp();
       return false;
     }
   }

@@ -156,7 +156,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(blk_empty + 2);
   float* part = reinterpret_cast<float*>(smem);         // [NT][128] after the main loop
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   const int kb0 = rank * p.kb_per, kb1 = min(p.num_kb, kb0 + p.kb_per);
 
   if (threadIdx.x == 0) {
@@ -192,7 +192,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   if (!chain_wait()) return;
 
   if (warp == 0) {
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmW);
       tma_prefetch_desc(&tmX);
       int stage = 0;
@@ -223,7 +223,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && kb1 > kb0) {
+    if (kb1 > kb0) {
       constexpr uint32_t idesc = make_idesc_bf16(SK_TN, NT, W_MN, X_MN);
       constexpr uint32_t desc_hi = smem_desc_hi(1024);
       const uint32_t base = smem_u32(smem);
@@ -231,26 +231,27 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       uint32_t phase = 0;
       bool ok = true;
       for (int kb = kb0; kb < kb1; ++kb) {
-        if (!mbar_wait(&full[stage], phase, p.status, kTimeoutTmaFull, 82)) { ok = false; break; }
+        if (!mbar_wait_warp(&full[stage], phase, p.status, kTimeoutTmaFull, 82)) { ok = false; break; }
         const int blk = kb - kb0;
-        if (F32 && !mbar_wait(&blk_empty[blk & 1], ((blk >> 1) & 1) ^ 1, p.status, kTimeoutAccFree, 84)) { ok = false; break; }
+        if (F32 && !mbar_wait_warp(&blk_empty[blk & 1], ((blk >> 1) & 1) ^ 1, p.status, kTimeoutAccFree, 84)) { ok = false; break; }
         tc_fence_after();
         const uint32_t sW = base + stage * L::STAGE;
         const uint32_t a_lo = smem_desc_lo(sW, W_MN ? 8192 : 16);
         const uint32_t b_lo = smem_desc_lo(sW + SK_W_BYTES, X_MN ? 8192 : 16);
+        one_lane([&] {
 #pragma unroll
-        for (int k = 0; k < KSTEPS; ++k)
-          mma_ss_w(F32 ? tmem_base + ((blk & 1) * KSTEPS + k) * NT : tmem_base, a_lo + (W_MN ? k * 128 : k * 2), desc_hi, b_lo + (X_MN ? k * 128 : k * 2),
-                   desc_hi, idesc,
-                   !F32 && (blk | k) != 0);
-        tc_commit(&empty[stage]);
-        if (F32) tc_commit(&blk_full[blk & 1]);
+          for (int k = 0; k < KSTEPS; ++k)
+            mma_ss_w(F32 ? tmem_base + ((blk & 1) * KSTEPS + k) * NT : tmem_base, a_lo + (W_MN ? k * 128 : k * 2), desc_hi,
+                     b_lo + (X_MN ? k * 128 : k * 2), desc_hi, idesc, !F32 && (blk | k) != 0);
+          tc_commit(&empty[stage]);
+          if (F32) tc_commit(&blk_full[blk & 1]);
+        });
         if (++stage == NST) {
           stage = 0;
           phase ^= 1;
         }
       }
-      if (ok && !F32) tc_commit(acc_full);
+      if (ok && !F32) one_lane([&] { tc_commit(acc_full); });
     }
   } else if (F32) {
     const int q = warp & 3;

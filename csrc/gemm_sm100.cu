@@ -3,7 +3,7 @@
 // Structure (one persistent CTA per SM, 192 threads):
 //   warp 0      TMA producer: fills a 4-stage ring of {A 128x64, B 256x64} bf16
 //               tiles in 128B-swizzled shared memory (non-multicast loads only).
-//   warp 1      MMA issuer: one thread issues tcgen05.mma 128x256x16 into one of
+//   warp 1      MMA issuer: issues tcgen05.mma 128x256x16 (one lane of the whole warp) into one of
 //               two 256-column TMEM accumulators and commits to mbarriers.
 //   warps 2..5  epilogue: tcgen05.ld the finished accumulator (each warp owns a
 //               32-lane quarter) and apply the fused epilogue while the next tile's
@@ -374,7 +374,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
   uint64_t* rx_full = acc_empty + 3;      // KSPLIT: [4 epilogue warps] the other pair's sums have arrived
   uint64_t* peer_ready = rx_full + 4;     // KSPLIT: [4] the other pair's main loop is over: its ring can be written
   uint64_t* ring_free = rx_full + 8;      // KSPLIT: the exchange is over on both sides (four warps here, four there)
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = warp_index(), lane = threadIdx.x & 31;
   if (!PAIR && (int)blockIdx.x < p.ag_copiers) {
     if (p.ag_push) ag_pusher(p); else ag_copier(p, smem);
     return;
@@ -426,7 +426,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (elect_one()) {
       tma_prefetch_desc(&tmA);
       tma_prefetch_desc(&tmB);
       tma_prefetch_desc(&tmB2);
@@ -521,7 +521,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       constexpr uint32_t idesc = make_idesc_bf16(TM, BN, A_MN, B_MN);
       constexpr uint32_t desc_hi = smem_desc_hi(1024);
       const uint32_t smem_base = smem_u32(smem);
@@ -536,7 +536,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1;
         ++local;
-        if (!mbar_wait(&acc_empty[acc], acc_phase ^ 1, p.status, kTimeoutAccFree, 2)) break;
+        if (!mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, p.status, kTimeoutAccFree, 2)) break;
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         // The MMA queue is shallow: whatever this thread does between two MMAs is tensor idle
@@ -544,7 +544,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         // current one, where its latency hides behind the MMAs still in flight.
         bool prewaited = false;
         for (int kb = ti.kb0; kb < ti.kb1; ++kb) {
-          if (!prewaited && !mbar_wait(&full[stage], phase, p.status, kTimeoutTmaFull, 3)) {
+          if (!prewaited && !mbar_wait_warp(&full[stage], phase, p.status, kTimeoutTmaFull, 3)) {
             ok = false;
             break;
           }
@@ -555,32 +555,38 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           const uint32_t sA = smem_base + stage * SBYTES;
           const uint32_t a_lo = smem_desc_lo(sA, A_MN ? 8192 : 16);
           const uint32_t b_lo = smem_desc_lo(sA + A_BYTES, B_MN ? 8192 : 16);
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            if (k == BK / 16 - 1 && kb + 1 < ti.kb1) {
-              const int ns = (stage + 1 == NST) ? 0 : stage + 1;
-              const uint32_t np = (stage + 1 == NST) ? (phase ^ 1) : phase;
-              if (!mbar_wait(&full[ns], np, p.status, kTimeoutTmaFull, 3)) {
-                ok = false;
-                break;
-              }
-              prewaited = true;
-            }
+          auto mma = [&](int k) {
+            const uint32_t acc_on = ((kb - ti.kb0) | k) != 0;
             if (PAIR)
               mma_ss_pair_w(d_tmem, a_lo + (A_MN ? k * 128 : k * 2), desc_hi, b_lo + (B_MN ? k * 128 : k * 2), desc_hi,
-                            idesc, ((kb - ti.kb0) | k) != 0);
+                            idesc, acc_on);
             else
               mma_ss_w(d_tmem, a_lo + (A_MN ? k * 128 : k * 2), desc_hi, b_lo + (B_MN ? k * 128 : k * 2), desc_hi, idesc,
-                       ((kb - ti.kb0) | k) != 0);
+                       acc_on);
+          };
+          one_lane([&] {
+#pragma unroll
+            for (int k = 0; k < BK / 16 - 1; ++k) mma(k);
+          });
+          if (kb + 1 < ti.kb1) {
+            const int ns = (stage + 1 == NST) ? 0 : stage + 1;
+            const uint32_t np = (stage + 1 == NST) ? (phase ^ 1) : phase;
+            if (!mbar_wait_warp(&full[ns], np, p.status, kTimeoutTmaFull, 3)) {
+              ok = false;
+              break;
+            }
+            prewaited = true;
           }
-          if (!ok) break;
-          if (PAIR) tc_commit_pair(&empty[stage], lead); else tc_commit(&empty[stage]);
+          one_lane([&] {
+            mma(BK / 16 - 1);
+            if (PAIR) tc_commit_pair(&empty[stage], lead); else tc_commit(&empty[stage]);
+          });
           if (++stage == NST) {
             stage = 0;
             phase ^= 1;
           }
         }
-        if (ok) { if (PAIR) tc_commit_pair(&acc_full[acc], lead); else tc_commit(&acc_full[acc]); }
+        if (ok) one_lane([&] { if (PAIR) tc_commit_pair(&acc_full[acc], lead); else tc_commit(&acc_full[acc]); });
       }
     }
   } else {
