@@ -24,7 +24,13 @@
 // Both kernels: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 compute.  Warps w and w+4
 // share a TMEM lane quarter and split the 128 score columns of a step; each writes its bf16
 // result over the first half of its OWN 64 input columns, so the two never touch each other's
-// columns and the A operand of the following MMA is addressed per 16-column k-step.
+// columns and the A operand of the following MMA is addressed per 16-column k-step.  That result is handed over in two
+// halves, so that its product starts while the second one is being made.
+//
+// Bound by the products themselves and the cap on power: 2560 clocks of the dK/dV kernel's 128 x 128 step for 2048 of
+// MMAs and 1730 for 1536 in the dQ kernel, at 1.4 GHz.  What the dK/dV kernel waits for is its first phase (1240 clocks
+// between S^T and P^T).  One row of 8192 tokens, 32/8 heads, delta kernel included: 1410 us (1520 before the halves, the exchange of
+// Q's and dO's places and the list of visible tiles); of 4096 388 (417); two rows of 1999 tokens in segments 187 (220).
 
 #include "common.cuh"
 #include "tpb.h"
@@ -39,9 +45,8 @@ constexpr int BWD_D = 128;
 constexpr int BWD_T = 128;         // score tile edge (rows and columns) in both kernels
 constexpr int BWD_THREADS = 320;   // TMA warp, MMA warp, 8 compute warps
 constexpr int TILE_BYTES = BWD_T * BWD_D * 2;   // one 128 x 128 bf16 operand tile: 32 KB
-constexpr int KV_QSTAGES = 2;      // dK/dV kernel: Q tile ring
-constexpr int KV_DOSTAGES = 2;     // dK/dV kernel: dO tile ring
-constexpr int KV_MAX_TILES = 512;  // query tiles whose position range fits the shared-memory table
+constexpr int KV_AUX = 4;          // dK/dV kernel: steps whose lse2 and delta rows are in shared memory
+constexpr int KV_MAX_TILES = 512;  // query tiles whose list fits in shared memory
 constexpr int DQ_KSTAGES = 3;      // dQ kernel: K tile ring (a K tile is held from S(j) to dQ(j))
 constexpr int DQ_VSTAGES = 2;      // dQ kernel: V tile ring
 constexpr float kLog2e = 1.4426950408889634f;
@@ -83,13 +88,18 @@ struct AttnBwdParams {
 namespace dkv {
 constexpr int OFF_K = 0;
 constexpr int OFF_V = OFF_K + TILE_BYTES;
-constexpr int OFF_Q = OFF_V + TILE_BYTES;
-constexpr int OFF_DO = OFF_Q + KV_QSTAGES * TILE_BYTES;
-constexpr int OFF_AUX = OFF_DO + KV_DOSTAGES * TILE_BYTES;   // per Q stage: lse2[128], delta[128], qpos[128], qseg[128]
+constexpr int OFF_QDO = OFF_V + TILE_BYTES;                  // four tiles, see q_slot()
+constexpr int OFF_AUX = OFF_QDO + 4 * TILE_BYTES;            // per step: lse2[128], delta[128], qpos[128], qseg[128]
 constexpr int AUX_STAGE = 4 * BWD_T * 4;
-constexpr int OFF_TILES = OFF_AUX + KV_QSTAGES * AUX_STAGE;  // tile min/max table: 2 * KV_MAX_TILES ints
-constexpr int OFF_SEGONE = OFF_TILES + 2 * KV_MAX_TILES * 4;  // per tile: 1 = all of its and this block's ids are one id
-constexpr int OFF_BAR = OFF_SEGONE + KV_MAX_TILES;
+constexpr int OFF_LIST = OFF_AUX + KV_AUX * AUX_STAGE;       // ushort: the visible tiles in order, kMasked set where scores need a mask
+constexpr int OFF_FLAGS = OFF_LIST + 2 * KV_MAX_TILES;       // uchar per tile: 0 not visible, 1 visible, 2 with a mask
+constexpr int OFF_BAR = OFF_FLAGS + KV_MAX_TILES;
+constexpr uint32_t kMasked = 0x8000;
+// Of a step's two tiles dO is done with first (after dV) and Q last (after dK), and the next step but one needs Q first.  So that
+// step's Q goes where this one's dO was and its dO where this one's Q was: both are asked for two products earlier than they
+// are needed at least.  (A ring of two each asked for Q one product before: 400 of a step's 2970 clocks were spent on its arrival.)
+__device__ __forceinline__ uint32_t q_slot(int i) { return OFF_QDO + (2 * (i & 1) + ((i >> 1) & 1)) * TILE_BYTES; }
+__device__ __forceinline__ uint32_t do_slot(int i) { return OFF_QDO + (2 * (i & 1) + (((i >> 1) & 1) ^ 1)) * TILE_BYTES; }
 constexpr int TOTAL = OFF_BAR + 256 + 1024;
 static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
 constexpr int T_DK = 0, T_DV = 128, T_S = 256, T_DP = 384;
@@ -193,6 +203,26 @@ __device__ __forceinline__ uint32_t mul_bf16x2(uint32_t a, uint32_t b) {
   return *reinterpret_cast<const uint32_t*>(&r);
 }
 
+__device__ __forceinline__ uint32_t pack_pair(f32x2 v) {
+  float a, b;
+  f2_unpack(v, a, b);
+  return pack_bf16(a, b);
+}
+// 2^-u as packed bf16, pair `c` of a row: every fourth pair on the FMA pipe.  A step's 128 x 128 exponentials take the MUFU 1024
+// clocks, half of what the step's MMAs take the tensor core, and stand in the chain between them.  (8192 tokens, 32/8 heads, us:
+// all on the MUFU 1451, every eighth 1421, every fourth 1410, three of eight 1420: the cap on power counts instructions too.)
+__device__ __forceinline__ uint32_t exp2_pair(int c, f32x2 u) {
+  float a, b;
+  if ((c & 3) == 3) {
+    exp2_neg_pair(u, a, b);
+  } else {
+    f2_unpack(u, a, b);
+    a = ex2_approx(-a);
+    b = ex2_approx(-b);
+  }
+  return pack_bf16(a, b);
+}
+
 // Operand tiles are [128 rows][128 d] in two 64-wide d blocks.  Descriptor low words (the high
 // word kDescHi is common): K-major use, k-step k covers 16 d; MN-major use (N = d contiguous,
 // K = rows), k-step k covers 16 rows.  The k-dependent part is a compile-time constant.
@@ -218,20 +248,20 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
-  uint64_t* kv_full = bars;
-  uint64_t* q_full = bars + 1;                    // [KV_QSTAGES]
-  uint64_t* q_empty = q_full + KV_QSTAGES;
-  uint64_t* do_full = q_empty + KV_QSTAGES;       // [KV_DOSTAGES]
-  uint64_t* do_empty = do_full + KV_DOSTAGES;
-  uint64_t* s_full = do_empty + KV_DOSTAGES;      // S^T of a step is in TMEM
-  uint64_t* p_full = s_full + 1;                  // count 256: P^T written
-  uint64_t* dp_full = s_full + 2;
-  uint64_t* ds_full = s_full + 3;                 // count 256: dS^T written
-  uint64_t* acc_done = s_full + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 5);
-  int* tile_min = reinterpret_cast<int*>(smem + OFF_TILES);
-  int* tile_max = tile_min + KV_MAX_TILES;
-  uint8_t* seg_one = smem + OFF_SEGONE;
+  uint64_t* k_full = bars;
+  uint64_t* q_full = bars + 1;                    // [2] by step parity
+  uint64_t* q_empty = q_full + 2;
+  uint64_t* do_full = q_empty + 2;
+  uint64_t* do_empty = do_full + 2;
+  uint64_t* s_full = do_empty + 2;                // S^T of a step is in TMEM
+  uint64_t* p_full = s_full + 1;                  // [2] one arrival per compute warp: each half of its share of P^T written
+  uint64_t* dp_full = s_full + 3;
+  uint64_t* ds_full = s_full + 4;                 // dS^T written
+  uint64_t* acc_done = s_full + 5;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 6);
+  int* n_list = reinterpret_cast<int*>(s_full + 7);
+  uint16_t* list = reinterpret_cast<uint16_t*>(smem + OFF_LIST);
+  uint8_t* flags = smem + OFF_FLAGS;
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   // linear block id is key-block major so that under a causal mask the blocks with the most
@@ -244,10 +274,13 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   const int n_tiles = (p.Sq + BWD_T - 1) / BWD_T;   // host guarantees <= KV_MAX_TILES
 
   if (threadIdx.x == 0) {
-    mbar_init(kv_full, 1);
-    for (int i = 0; i < KV_QSTAGES; ++i) { mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1); }
-    for (int i = 0; i < KV_DOSTAGES; ++i) { mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1); }
-    mbar_init(s_full, 1); mbar_init(p_full, 256); mbar_init(dp_full, 1); mbar_init(ds_full, 256);
+    mbar_init(k_full, 1);
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1);
+      mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1);
+    }
+    mbar_init(s_full, 1); mbar_init(dp_full, 1); mbar_init(ds_full, 8);
+    for (int i = 0; i < 2; ++i) mbar_init(&p_full[i], 8);
     mbar_init(acc_done, 1);
     fence_barrier_init();
   }
@@ -256,7 +289,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tmem_relinquish();
   }
   if (!chain_wait()) return;
-  // position range of every query tile (decides which tiles this key block can see)
+  // which query tiles this key block can see, from the positions (and segments) of each one's rows
   const int2 kseg_rng = SEG ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
   for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
     const int r0 = t * BWD_T, r1 = min(p.Sq, r0 + BWD_T);
@@ -269,27 +302,33 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     } else {
       mn = r0 + pos_off; mx = r1 - 1 + pos_off;
     }
+    bool vis = !(p.causal && mx < kv0) && !(p.window > 0 && mn - (kv0 + BWD_T - 1) >= p.window), one_seg = false;
     if (SEG) {
       const int2 qr = seg_range128(p.q_rng, b, t, p.Sq);
-      seg_one[t] = qr.x == qr.y && kseg_rng.x == kseg_rng.y && qr.x == kseg_rng.x;
-      if (qr.y < kseg_rng.x || qr.x > kseg_rng.y) { mn = 0x7fffffff; mx = -0x7fffffff; }   // no segment in common
+      one_seg = qr.x == qr.y && kseg_rng.x == kseg_rng.y && qr.x == kseg_rng.x;
+      if (qr.y < kseg_rng.x || qr.x > kseg_rng.y) vis = false;   // no segment in common
     }
-    tile_min[t] = mn; tile_max[t] = mx;
+    const bool mask = (kv0 + BWD_T > p.Sk) || (p.causal && mn < kv0 + BWD_T - 1) || (p.window > 0 && mx - kv0 >= p.window) ||
+                      (p.q_seg != nullptr && !one_seg);
+    flags[t] = vis ? (mask ? 2 : 1) : 0;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int n = 0;
+    for (int t0 = 0; t0 < n_tiles; t0 += 32) {
+      const int f = t0 + lane < n_tiles ? flags[t0 + lane] : 0;
+      const uint32_t seen = __ballot_sync(0xffffffffu, f != 0);
+      if (f) list[n + __popc(seen & ((1u << lane) - 1))] = (uint16_t)((t0 + lane) | (f == 2 ? kMasked : 0u));
+      n += __popc(seen);
+    }
+    if (lane == 0) *n_list = n;
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   chain_launch();
-
-  auto visible = [&](int t) -> bool {
-    if (SEG && tile_min[t] > tile_max[t]) return false;
-    if (p.causal && tile_max[t] < kv0) return false;
-    if (p.window > 0 && tile_min[t] - (kv0 + BWD_T - 1) >= p.window) return false;
-    return true;
-  };
-  int n_vis = 0;
-  for (int t = 0; t < n_tiles; ++t) n_vis += visible(t) ? 1 : 0;
+  const int n_vis = *n_list;
   const int n_steps = n_vis * G;
 
   if (warp == 0) {
@@ -297,27 +336,22 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     if (n_steps > 0) {
       if (lane == 0) {
         tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
-        mbar_expect_tx(kv_full, 2 * TILE_BYTES);
-        for (int c = 0; c < BWD_D / 64; ++c) {
-          tma_load_3d(smem + OFF_K + c * (BWD_T * 128), &tmK, kv_full, c * 64, b * p.Sk + kv0, hkv);
-          tma_load_3d(smem + OFF_V + c * (BWD_T * 128), &tmV, kv_full, c * 64, b * p.Sk + kv0, hkv);
-        }
+        mbar_expect_tx(k_full, TILE_BYTES);
+        for (int c = 0; c < BWD_D / 64; ++c)
+          tma_load_3d(smem + OFF_K + c * (BWD_T * 128), &tmK, k_full, c * 64, b * p.Sk + kv0, hkv);
       }
       const bool aux_rows = p.q_pos != nullptr || p.q_seg != nullptr;
       int step = 0;
       bool ok = true;
       for (int g = 0; g < G && ok; ++g) {
         const int hq = hkv * G + g;
-        for (int t = 0; t < n_tiles && ok; ++t) {
-          if (!visible(t)) continue;
-          const int sq = step % KV_QSTAGES, sd = step % KV_DOSTAGES;
-          const int q0 = t * BWD_T;
-          int okw = 1;
-          if (lane == 0)
-            okw = mbar_wait(&q_empty[sq], ((step / KV_QSTAGES) & 1) ^ 1, p.status, kTimeoutStageFree, 21) ? 1 : 0;
-          okw = __shfl_sync(0xffffffffu, okw, 0);
-          if (!okw) { ok = false; break; }
-          float* aux = reinterpret_cast<float*>(smem + OFF_AUX + sq * AUX_STAGE);
+        for (int v = 0; v < n_vis; ++v) {
+          const int st = step & 1;
+          const uint32_t ph = ((step >> 1) & 1) ^ 1;
+          const int q0 = (int)(list[v] & (kMasked - 1)) * BWD_T;
+          // Q takes the place of the dO of two steps ago
+          if (!mbar_wait_warp(&do_empty[st], ph, p.status, kTimeoutStageFree, 21)) { ok = false; break; }
+          float* aux = reinterpret_cast<float*>(smem + OFF_AUX + (step % KV_AUX) * AUX_STAGE);
           int* auxi = reinterpret_cast<int*>(aux);
           if (aux_rows && !p.aux_bulk) {
             // rows that cannot be bulk-copied (unaligned sequence length): plain loads, made
@@ -333,28 +367,29 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
             const uint32_t rows_bytes = (uint32_t)min(BWD_T, p.Sq - q0) * 4u;
             uint32_t tx = TILE_BYTES + 2 * BWD_T * 4;
             if (aux_rows && p.aux_bulk) tx += (p.q_pos ? rows_bytes : 0u) + (p.q_seg ? rows_bytes : 0u);
-            mbar_expect_tx(&q_full[sq], tx);
+            mbar_expect_tx(&q_full[st], tx);
             for (int c = 0; c < BWD_D / 64; ++c)
-              tma_load_3d(smem + OFF_Q + sq * TILE_BYTES + c * (BWD_T * 128), &tmQ, &q_full[sq], c * 64,
-                          b * p.Sq + q0, hq);
+              tma_load_3d(smem + q_slot(step) + c * (BWD_T * 128), &tmQ, &q_full[st], c * 64, b * p.Sq + q0, hq);
             const long long li = ((long long)b * p.Hq + hq) * p.Sq_pad + q0;
-            bulk_load(aux, p.lse2 + li, BWD_T * 4, &q_full[sq]);
-            bulk_load(aux + BWD_T, p.delta + li, BWD_T * 4, &q_full[sq]);
+            bulk_load(aux, p.lse2 + li, BWD_T * 4, &q_full[st]);
+            bulk_load(aux + BWD_T, p.delta + li, BWD_T * 4, &q_full[st]);
             if (aux_rows && p.aux_bulk) {
-              if (p.q_pos) bulk_load(auxi + 2 * BWD_T, p.q_pos + (long long)b * p.Sq + q0, rows_bytes, &q_full[sq]);
-              if (p.q_seg) bulk_load(auxi + 3 * BWD_T, p.q_seg + (long long)b * p.Sq + q0, rows_bytes, &q_full[sq]);
-            }
-            if (mbar_wait(&do_empty[sd], ((step / KV_DOSTAGES) & 1) ^ 1, p.status, kTimeoutStageFree, 29)) {
-              mbar_expect_tx(&do_full[sd], TILE_BYTES);
-              for (int c = 0; c < BWD_D / 64; ++c)
-                tma_load_3d(smem + OFF_DO + sd * TILE_BYTES + c * (BWD_T * 128), &tmdO, &do_full[sd], c * 64,
-                            b * p.Sq + q0, hq);
-            } else {
-              okw = 0;
+              if (p.q_pos) bulk_load(auxi + 2 * BWD_T, p.q_pos + (long long)b * p.Sq + q0, rows_bytes, &q_full[st]);
+              if (p.q_seg) bulk_load(auxi + 3 * BWD_T, p.q_seg + (long long)b * p.Sq + q0, rows_bytes, &q_full[st]);
             }
           }
-          okw = __shfl_sync(0xffffffffu, okw, 0);
-          if (!okw) { ok = false; break; }
+          __syncwarp();
+          // and dO that of its Q
+          if (!mbar_wait_warp(&q_empty[st], ph, p.status, kTimeoutStageFree, 29)) { ok = false; break; }
+          if (lane == 0) {
+            mbar_expect_tx(&do_full[st], step == 0 ? 2 * TILE_BYTES : TILE_BYTES);   // V comes with the first dO
+            if (step == 0)
+              for (int c = 0; c < BWD_D / 64; ++c)
+                tma_load_3d(smem + OFF_V + c * (BWD_T * 128), &tmV, &do_full[0], c * 64, b * p.Sk + kv0, hkv);
+            for (int c = 0; c < BWD_D / 64; ++c)
+              tma_load_3d(smem + do_slot(step) + c * (BWD_T * 128), &tmdO, &do_full[st], c * 64, b * p.Sq + q0, hq);
+          }
+          __syncwarp();
           ++step;
         }
       }
@@ -365,14 +400,14 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       constexpr uint32_t id_s = make_idesc_bf16(BWD_T, BWD_T, false, false);    // S^T, dP^T
       constexpr uint32_t id_acc = make_idesc_bf16(BWD_T, BWD_D, false, true);   // dV, dK (A in TMEM, B MN-major)
       const uint32_t dK = kmajor_lo(smem_u32(smem + OFF_K)), dVd = kmajor_lo(smem_u32(smem + OFF_V));
-      const uint32_t aQ0 = smem_u32(smem + OFF_Q), aDO0 = smem_u32(smem + OFF_DO);
+      const uint32_t base = smem_u32(smem);
       const uint32_t tS = tmem_base + T_S, tDP = tmem_base + T_DP;
       // The MMA queue is shallow, so whatever this thread does between two MMAs is tensor idle
       // time: every wait is therefore placed before the LAST MMA of the preceding group, where
       // its latency hides behind the seven MMAs still in flight.
-      auto wait_q = [&](int i) { return mbar_wait_warp(&q_full[i % KV_QSTAGES], (i / KV_QSTAGES) & 1, p.status, kTimeoutTmaFull, 23); };
-      auto wait_do = [&](int i) { return mbar_wait_warp(&do_full[i % KV_DOSTAGES], (i / KV_DOSTAGES) & 1, p.status, kTimeoutTmaFull, 24); };
-      auto wait_p = [&](int i) { return mbar_wait_warp(p_full, i & 1, p.status, kTimeoutSoftmax, 25); };
+      auto wait_q = [&](int i) { return mbar_wait_warp(&q_full[i & 1], (i >> 1) & 1, p.status, kTimeoutTmaFull, 23); };
+      auto wait_do = [&](int i) { return mbar_wait_warp(&do_full[i & 1], (i >> 1) & 1, p.status, kTimeoutTmaFull, 24); };
+      auto wait_p = [&](int i, int part) { return mbar_wait_warp(&p_full[part], i & 1, p.status, kTimeoutSoftmax, 25); };
       auto wait_ds = [&](int i) { return mbar_wait_warp(ds_full, i & 1, p.status, kTimeoutSoftmax, 26); };
       auto group = [&](auto&& mma, auto&& hook, auto&& done) -> bool {
         one_lane([&] {
@@ -384,15 +419,15 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         one_lane([&] { mma(7); done(); });
         return true;
       };
-      bool ok = mbar_wait_warp(kv_full, 0, p.status, kTimeoutTmaFull, 22) && wait_q(0);
+      bool ok = mbar_wait_warp(k_full, 0, p.status, kTimeoutTmaFull, 22) && wait_q(0);
       tc_fence_after();
       auto issue_s = [&](int i, auto&& hook) -> bool {      // S^T(i) = K Q(i)^T
-        const uint32_t dQ = kmajor_lo(aQ0 + (i % KV_QSTAGES) * TILE_BYTES);
+        const uint32_t dQ = kmajor_lo(base + q_slot(i));
         return group([&](int k) { mma_ss_w(tS, dK + kmajor_k(k), kDescHi, dQ + kmajor_k(k), kDescHi, id_s, k != 0); }, hook,
                      [&] { tc_commit(s_full); });
       };
       auto issue_dp = [&](int i, auto&& hook) -> bool {     // dP^T(i) = V dO(i)^T
-        const uint32_t dDO = kmajor_lo(aDO0 + (i % KV_DOSTAGES) * TILE_BYTES);
+        const uint32_t dDO = kmajor_lo(base + do_slot(i));
         return group([&](int k) { mma_ss_w(tDP, dVd + kmajor_k(k), kDescHi, dDO + kmajor_k(k), kDescHi, id_s, k != 0); }, hook,
                      [&] { tc_commit(dp_full); });
       };
@@ -400,23 +435,27 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
       if (ok) ok = issue_s(0, [&] { return wait_do(0); });
       if (ok) ok = issue_dp(0, none);
       for (int i = 0; i < n_steps && ok; ++i) {
-        const uint32_t mQ = mnmajor_lo(aQ0 + (i % KV_QSTAGES) * TILE_BYTES);
-        const uint32_t mDO = mnmajor_lo(aDO0 + (i % KV_DOSTAGES) * TILE_BYTES);
+        const uint32_t mQ = mnmajor_lo(base + q_slot(i));
+        const uint32_t mDO = mnmajor_lo(base + do_slot(i));
         const bool more = i + 1 < n_steps;
         // Waits on the compute warps stay where the data is needed: hooking them into the previous
         // group would hold back that group's commit, which the compute warps are waiting for.
-        if (!wait_p(i)) break;
+        // dV += P^T dO, first the k-steps whose P^T is there when the exponentials are half done
+        auto dv = [&](int k) { mma_ts_w(tmem_base + T_DV, tS + a_col(k), mDO + mnmajor_k(k), kDescHi, id_acc, (i | k) != 0); };
+        if (!wait_p(i, 0)) break;
         tc_fence_after();
-        // dV += P^T dO
-        ok = group([&](int k) { mma_ts_w(tmem_base + T_DV, tS + a_col(k), mDO + mnmajor_k(k), kDescHi, id_acc, (i | k) != 0); },
-                   [&] { return more ? wait_q(i + 1) : true; }, [&] { tc_commit(&do_empty[i % KV_DOSTAGES]); });
+        one_lane([&] { dv(0); dv(1); dv(4); dv(5); });
+        if (!wait_p(i, 1)) break;
+        tc_fence_after();
+        ok = group([&](int k) { if (k == 2 || k == 3 || k >= 6) dv(k); },
+                   [&] { return more ? wait_q(i + 1) : true; }, [&] { tc_commit(&do_empty[i & 1]); });
         if (!ok) break;
         if (more && !issue_s(i + 1, none)) break;
         if (!wait_ds(i)) break;
         tc_fence_after();
         // dK += dS^T Q
         ok = group([&](int k) { mma_ts_w(tmem_base + T_DK, tDP + a_col(k), mQ + mnmajor_k(k), kDescHi, id_acc, (i | k) != 0); },
-                   [&] { return more ? wait_do(i + 1) : true; }, [&] { tc_commit(&q_empty[i % KV_QSTAGES]); });
+                   [&] { return more ? wait_do(i + 1) : true; }, [&] { tc_commit(&q_empty[i & 1]); });
         if (!ok) break;
         if (more && !issue_dp(i + 1, none)) break;
       }
@@ -440,14 +479,12 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
     int step = 0;
     for (int g = 0; g < G && ok; ++g) {
-      for (int t = 0; t < n_tiles && ok; ++t) {
-        if (!visible(t)) continue;
-        const int sq = step % KV_QSTAGES;
-        const float* aux = reinterpret_cast<const float*>(smem + OFF_AUX + sq * AUX_STAGE);
+      for (int v = 0; v < n_vis && ok; ++v) {
+        const uint32_t entry = list[v];
+        const int t = (int)(entry & (kMasked - 1));
+        const bool need_mask = (entry & kMasked) != 0;
+        const float* aux = reinterpret_cast<const float*>(smem + OFF_AUX + (step % KV_AUX) * AUX_STAGE);
         const int* auxi = reinterpret_cast<const int*>(aux);
-        const bool need_mask = !key_ok || (kv0 + BWD_T > p.Sk) || (p.causal && tile_min[t] < kv0 + BWD_T - 1) ||
-                               (p.window > 0 && tile_max[t] - kv0 >= p.window) ||
-                               (p.q_seg != nullptr && !(SEG && seg_one[t]));
         // ---- phase 1: P^T = exp2(S^T * c - lse), kept packed for phase 2 and written over S^T
         if (!mbar_wait(s_full, step & 1, p.status, kTimeoutAccFull, 27)) { ok = false; break; }
         tc_fence_after();
@@ -488,7 +525,16 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         for (int ch = 0; ch < 2; ++ch) {
           const uint32_t* s = sreg + ch * 32;
           const float4* lse4 = reinterpret_cast<const float4*>(aux + half * 64 + ch * 32);
-          if (!need_mask) {
+          if (!need_mask && !SOFTCAP) {
+            const f32x2 nc2 = f2_pack(-p.scale_log2, -p.scale_log2);
+#pragma unroll
+            for (int c4 = 0; c4 < 8; ++c4) {
+              const float4 L = lse4[c4];
+              pk_p[ch * 16 + 2 * c4] = exp2_pair(2 * c4, f2_fma(f2_pack_bits(s[4 * c4], s[4 * c4 + 1]), nc2, f2_pack(L.x, L.y)));
+              pk_p[ch * 16 + 2 * c4 + 1] =
+                  exp2_pair(2 * c4 + 1, f2_fma(f2_pack_bits(s[4 * c4 + 2], s[4 * c4 + 3]), nc2, f2_pack(L.z, L.w)));
+            }
+          } else if (!need_mask) {
 #pragma unroll
             for (int c4 = 0; c4 < 8; ++c4) {
               const float4 L = lse4[c4];
@@ -532,15 +578,16 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               pk_p[ch * 16 + 2 * c4 + 1] = pack_bf16(pv[2], pv[3]);
             }
           }
+          tmem_st16(tS + ch * 16, pk_p + ch * 16);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&p_full[ch]);
         }
-        tmem_st32(tS, pk_p);
         if (SOFTCAP) {   // dV takes P^T as it is; dS^T takes P^T times the derivative of the cap
 #pragma unroll
           for (int c = 0; c < 32; ++c) pk_p[c] = mul_bf16x2(pk_p[c], pk_f[c]);
         }
-        tmem_wait_st();
-        tc_fence_before();
-        mbar_arrive(p_full);
         // ---- phase 2: dS^T = P^T o (dP^T - delta), written over dP^T
         if (!mbar_wait(dp_full, step & 1, p.status, kTimeoutAccFull, 28)) { ok = false; break; }
         tc_fence_after();
@@ -553,17 +600,17 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 #pragma unroll
           for (int c4 = 0; c4 < 16; ++c4) {
             const float4 Dl = dlt4[c4];
-            pk_ds[2 * c4] = mul_bf16x2(pk_p[2 * c4], pack_bf16(__uint_as_float(dreg[4 * c4]) - Dl.x,
-                                                               __uint_as_float(dreg[4 * c4 + 1]) - Dl.y));
-            pk_ds[2 * c4 + 1] = mul_bf16x2(pk_p[2 * c4 + 1], pack_bf16(__uint_as_float(dreg[4 * c4 + 2]) - Dl.z,
-                                                                       __uint_as_float(dreg[4 * c4 + 3]) - Dl.w));
+            pk_ds[2 * c4] = mul_bf16x2(pk_p[2 * c4], pack_pair(f2_sub(f2_pack_bits(dreg[4 * c4], dreg[4 * c4 + 1]), f2_pack(Dl.x, Dl.y))));
+            pk_ds[2 * c4 + 1] =
+                mul_bf16x2(pk_p[2 * c4 + 1], pack_pair(f2_sub(f2_pack_bits(dreg[4 * c4 + 2], dreg[4 * c4 + 3]), f2_pack(Dl.z, Dl.w))));
           }
           // all 64 inputs of this warp are in registers, so its first 32 columns can be overwritten
           tmem_st32(tDP, pk_ds);
         }
         tmem_wait_st();
         tc_fence_before();
-        mbar_arrive(ds_full);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ds_full);
         ++step;
       }
     }
@@ -597,18 +644,18 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = smem_raw + ((1024u - (smem_u32(smem_raw) & 1023u)) & 1023u);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + OFF_BAR);
-  uint64_t* qdo_full = bars;
+  uint64_t* q_full = bars;
   uint64_t* k_full = bars + 1;                    // [DQ_KSTAGES]
   uint64_t* k_empty = k_full + DQ_KSTAGES;
   uint64_t* v_full = k_empty + DQ_KSTAGES;        // [DQ_VSTAGES]
   uint64_t* v_empty = v_full + DQ_VSTAGES;
   uint64_t* s_full = v_empty + DQ_VSTAGES;        // [2]
   uint64_t* dp_full = s_full + 2;
-  uint64_t* ds_full = s_full + 3;                 // count 256
-  uint64_t* acc_done = s_full + 4;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 5);
-  int* tile_minmax = reinterpret_cast<int*>(s_full + 6);  // [2]
-  int* seg_lohi = reinterpret_cast<int*>(s_full + 7);     // [2] first and last key block with a segment of this tile
+  uint64_t* ds_full = s_full + 3;                 // [2] one arrival per compute warp: each half of its share of dS written
+  uint64_t* acc_done = s_full + 5;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(s_full + 6);
+  int* tile_minmax = reinterpret_cast<int*>(s_full + 7);  // [2]
+  int* seg_lohi = reinterpret_cast<int*>(s_full + 8);     // [2] first and last key block with a segment of this tile
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_qtiles = (p.Sq + BWD_T - 1) / BWD_T;
@@ -620,11 +667,11 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   const int pos_off = p.Sk - p.Sq;
 
   if (threadIdx.x == 0) {
-    mbar_init(qdo_full, 1);
+    mbar_init(q_full, 1);
     for (int i = 0; i < DQ_KSTAGES; ++i) { mbar_init(&k_full[i], 1); mbar_init(&k_empty[i], 1); }
     for (int i = 0; i < DQ_VSTAGES; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
     mbar_init(&s_full[0], 1); mbar_init(&s_full[1], 1);
-    mbar_init(dp_full, 1); mbar_init(ds_full, 256);
+    mbar_init(dp_full, 1); mbar_init(&ds_full[0], 8); mbar_init(&ds_full[1], 8);
     mbar_init(acc_done, 1);
     tile_minmax[0] = 0x7fffffff;
     tile_minmax[1] = -0x7fffffff;
@@ -676,12 +723,10 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     // ------------------------------------------------------------------ TMA producer
     if (nblk > 0 && elect_one()) {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
-      mbar_expect_tx(qdo_full, 2 * TILE_BYTES);
+      mbar_expect_tx(q_full, TILE_BYTES);
 #pragma unroll
-      for (int c = 0; c < BWD_D / 64; ++c) {
-        tma_load_3d(smem + OFF_Q + c * (BWD_T * 128), &tmQ, qdo_full, c * 64, b * p.Sq + q0, hq);
-        tma_load_3d(smem + OFF_DO + c * (BWD_T * 128), &tmdO, qdo_full, c * 64, b * p.Sq + q0, hq);
-      }
+      for (int c = 0; c < BWD_D / 64; ++c)
+        tma_load_3d(smem + OFF_Q + c * (BWD_T * 128), &tmQ, q_full, c * 64, b * p.Sq + q0, hq);
       for (int j = 0; j < nblk; ++j) {
         const int sk = j % DQ_KSTAGES, sv = j % DQ_VSTAGES;
         const int row = b * p.Sk + (blk_lo + j) * BWD_T;
@@ -691,7 +736,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         for (int c = 0; c < BWD_D / 64; ++c)
           tma_load_3d(smem + OFF_K + sk * TILE_BYTES + c * (BWD_T * 128), &tmK, &k_full[sk], c * 64, row, hkv);
         if (!mbar_wait(&v_empty[sv], ((j / DQ_VSTAGES) & 1) ^ 1, p.status, kTimeoutStageFree, 35)) break;
-        mbar_expect_tx(&v_full[sv], TILE_BYTES);
+        mbar_expect_tx(&v_full[sv], j == 0 ? 2 * TILE_BYTES : TILE_BYTES);   // dO comes with the first V
+        if (j == 0) {
+#pragma unroll
+          for (int c = 0; c < BWD_D / 64; ++c)
+            tma_load_3d(smem + OFF_DO + c * (BWD_T * 128), &tmdO, &v_full[0], c * 64, b * p.Sq + q0, hq);
+        }
 #pragma unroll
         for (int c = 0; c < BWD_D / 64; ++c)
           tma_load_3d(smem + OFF_V + sv * TILE_BYTES + c * (BWD_T * 128), &tmV, &v_full[sv], c * 64, row, hkv);
@@ -708,7 +758,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       // Waits sit before the last MMA of the preceding group (see the dK/dV kernel).
       auto wait_k = [&](int j) { return mbar_wait_warp(&k_full[j % DQ_KSTAGES], (j / DQ_KSTAGES) & 1, p.status, kTimeoutTmaFull, 33); };
       auto wait_v = [&](int j) { return mbar_wait_warp(&v_full[j % DQ_VSTAGES], (j / DQ_VSTAGES) & 1, p.status, kTimeoutTmaFull, 37); };
-      auto wait_ds = [&](int j) { return mbar_wait_warp(ds_full, j & 1, p.status, kTimeoutSoftmax, 34); };
+      auto wait_ds = [&](int j, int part) { return mbar_wait_warp(&ds_full[part], j & 1, p.status, kTimeoutSoftmax, 34); };
       auto group = [&](auto&& mma, auto&& hook, auto&& done) -> bool {
         one_lane([&] {
 #pragma unroll
@@ -719,7 +769,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         one_lane([&] { mma(7); done(); });
         return true;
       };
-      bool ok = mbar_wait_warp(qdo_full, 0, p.status, kTimeoutTmaFull, 32) && wait_k(0);
+      bool ok = mbar_wait_warp(q_full, 0, p.status, kTimeoutTmaFull, 32) && wait_k(0);
       tc_fence_after();
       auto issue_s = [&](int j, auto&& hook) -> bool {      // S(j) = Q K_j^T
         const uint32_t dK = kmajor_lo(aK0 + (j % DQ_KSTAGES) * TILE_BYTES);
@@ -738,11 +788,15 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       for (int j = 0; j < nblk && ok; ++j) {
         const bool more = j + 1 < nblk;
         if (more && !issue_s(j + 1, none)) break;
-        if (!wait_ds(j)) break;   // not hooked into S(j+1): that would hold back its commit
-        tc_fence_after();
         const uint32_t mK = mnmajor_lo(aK0 + (j % DQ_KSTAGES) * TILE_BYTES);
-        // dQ += dS K   (K tile [128 keys][128 d]: N = d contiguous)
-        ok = group([&](int k) { mma_ts_w(tmem_base + T_DQ, tDP + a_col(k), mK + mnmajor_k(k), kDescHi, id_dq, (j | k) != 0); },
+        // dQ += dS K   (K tile [128 keys][128 d]: N = d contiguous), in the order in which dS gets there
+        auto dq = [&](int k) { mma_ts_w(tmem_base + T_DQ, tDP + a_col(k), mK + mnmajor_k(k), kDescHi, id_dq, (j | k) != 0); };
+        if (!wait_ds(j, 0)) break;   // not hooked into S(j+1): that would hold back its commit
+        tc_fence_after();
+        one_lane([&] { dq(0); dq(1); dq(4); dq(5); });
+        if (!wait_ds(j, 1)) break;
+        tc_fence_after();
+        ok = group([&](int k) { if (k == 2 || k == 3 || k >= 6) dq(k); },
                    [&] { return more ? wait_v(j + 1) : true; }, [&] { tc_commit(&k_empty[j % DQ_KSTAGES]); });
         if (!ok) break;
         if (more && !issue_dp(j + 1, [&] { return j + 2 < nblk ? wait_k(j + 2) : true; })) break;
@@ -798,7 +852,12 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) {
         const uint32_t* s = sreg + ch * 32;
-        if (!need_mask) {
+        if (!need_mask && !SOFTCAP) {
+          const f32x2 nc2 = f2_pack(-p.scale_log2, -p.scale_log2), l2 = f2_pack(lse2, lse2);
+#pragma unroll
+          for (int c = 0; c < 16; ++c)
+            pk_p[ch * 16 + c] = exp2_pair(c, f2_fma(f2_pack_bits(s[2 * c], s[2 * c + 1]), nc2, l2));
+        } else if (!need_mask) {
 #pragma unroll
           for (int c = 0; c < 32; c += 2) {
             float s0 = __uint_as_float(s[c]), s1 = __uint_as_float(s[c + 1]), f0 = 1.f, f1 = 1.f;
@@ -834,19 +893,23 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       if (!mbar_wait(dp_full, j & 1, p.status, kTimeoutAccFull, 39)) { ok = false; break; }
       tc_fence_after();
       {
-        uint32_t dreg[64], pk[32];
+        uint32_t dreg[64], pk[16];
         tmem_ld32(tDP, dreg);
         tmem_ld32(tDP + 32, dreg + 32);
         tmem_wait_ld();
+        const f32x2 d2 = f2_pack(delta, delta);
 #pragma unroll
-        for (int c = 0; c < 32; ++c)
-          pk[c] = mul_bf16x2(pk_p[c], pack_bf16(__uint_as_float(dreg[2 * c]) - delta,
-                                                __uint_as_float(dreg[2 * c + 1]) - delta));
-        tmem_st32(tDP, pk);
+        for (int ch = 0; ch < 2; ++ch) {
+#pragma unroll
+          for (int c = 0; c < 16; ++c)
+            pk[c] = mul_bf16x2(pk_p[ch * 16 + c], pack_pair(f2_sub(f2_pack_bits(dreg[32 * ch + 2 * c], dreg[32 * ch + 2 * c + 1]), d2)));
+          tmem_st16(tDP + ch * 16, pk);
+          tmem_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&ds_full[ch]);
+        }
       }
-      tmem_wait_st();
-      tc_fence_before();
-      mbar_arrive(ds_full);
     }
     if (ok && nblk > 0) ok = mbar_wait(acc_done, 0, p.status, kTimeoutAccFull, 38);
     tc_fence_after();

@@ -101,6 +101,34 @@ def test_attention_backward(cuda_lib, b, s, hq, hkv, d, causal, window):
   assert _rel(dq, qf.grad) < 3e-2, ("dq", _rel(dq, qf.grad))
 
 
+@pytest.mark.parametrize("s,window,segments", [(4096, None, 0), (4097, 300, 0), (4230, None, 9), (4230, 130, 9)])
+def test_backward_lists_its_query_tiles(cuda_lib, s, window, segments):
+  """Key blocks that see all, few and scattered query tiles, more than one warp counts at a time; bound of the cases above."""
+  from torchprime_b200.ops import attention_sm100 as A
+  q, k, v = _qkv(1, s, 2, 1, 128, fused=False, seed=s)
+  do = torch.randn(1, s, 2, 128, device="cuda", dtype=torch.bfloat16)
+  ids = ((torch.arange(s, device="cuda") * segments // s) % 4).to(torch.int32)[None].contiguous() if segments else None
+  o, lse = A.attn_fwd(q, k, v, causal=True, window=window, q_seg=ids, kv_seg=ids)
+  got = A.attn_bwd(do, q, k, v, o, lse, causal=True, window=window, q_seg=ids, kv_seg=ids)
+  leaves = [t.float().requires_grad_(True) for t in (q, k, v)]
+  ref.attention(*leaves, causal=True, window=window, q_segment_ids=ids).backward(do.float())
+  for g, w in zip(got, leaves):
+    assert _rel(g, w.grad) < 2e-2, _rel(g, w.grad)
+
+
+def test_backward_keeps_nan(cuda_lib):
+  """A NaN in one query row reaches the gradients of every key that the row sees, also through the tiles without a mask."""
+  from torchprime_b200.ops import attention_sm100 as A
+  q, k, v = _qkv(1, 640, 2, 1, 128, fused=False, seed=3)
+  q[0, 600, 0, 7] = float("nan")
+  do = torch.randn(1, 640, 2, 128, device="cuda", dtype=torch.bfloat16)
+  o, lse = A.attn_fwd(q, k, v, causal=True)
+  dq, dk, dv = A.attn_bwd(do, q, k, v, o, lse, causal=True)
+  assert not torch.isfinite(dv[0, :601]).any() and not torch.isfinite(dk[0, :601]).any()
+  assert not torch.isfinite(dq[0, 600, 0]).any()
+  assert torch.isfinite(dv[0, 601:]).all() and torch.isfinite(dq[0, :600]).all() and torch.isfinite(dq[0, :, 1]).all()
+
+
 def test_attention_autograd_fused_qkv(cuda_lib):
   from torchprime_b200.ops import functional as ops
   b, s, hq, hkv, d = 1, 256, 4, 2, 128
