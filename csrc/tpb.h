@@ -55,7 +55,9 @@ int tpb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void
 // dx = d/dx of the above (+ dres if given).  dw_f32 [dim] is accumulated with atomics.
 int tpb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres,
                     void* dx, float* dw_f32, int rows, int dim, void* stream);
-// The same with dw_f32 cleared first and, if dw_bf16 is given, its sums delivered there.
+// The same with the sums written: dw_f32 is [1 + tpb_rmsnorm_bwd_parts(rows, dim)][dim], the first row receives them (the
+// others are scratch) and, if given, dw_bf16.
+int tpb_rmsnorm_bwd_parts(int rows, int dim);
 int tpb_rmsnorm_bwd_dw(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
                        float* dw_f32, void* dw_bf16, int rows, int dim, void* stream);
 

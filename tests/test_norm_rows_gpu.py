@@ -1,0 +1,50 @@
+"""RMSNorm over many rows (rows streamed through shared memory, forward and backward) against 64 bits."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _rel(got, want):
+  return ((got.double() - want).norm() / want.norm()).item()
+
+
+@pytest.mark.parametrize("residual", [False, True])
+@pytest.mark.parametrize("rows,dim", [(2048, 8), (2049, 264), (2047, 1024), (1024, 1032), (3000, 2048), (2300, 2056), (1023, 4096),
+                                      (5000, 4096), (2048, 4104), (1777, 5120), (2100, 5128), (2500, 8192)])
+def test_forward_and_backward(cuda_lib, rows, dim, residual):
+  """Widths around the row's share of a lane or thread, rows around the numbers of warps and the rule's edges.  y and dx are
+  rounded to bf16 twice at most (2^-9 each), dw and rstd are fp32."""
+  from torchprime_b200.ops import kernels as k
+  torch.manual_seed(rows + dim)
+  x, dy, dres = (torch.randn(rows, dim, device="cuda").bfloat16() for _ in range(3))
+  w = (1 + 0.1 * torch.randn(dim, device="cuda")).bfloat16()
+  y, rstd, _ = k.rmsnorm_fwd(x, w, 1e-5)
+  dx, dw = k.rmsnorm_bwd(dy, x, w, rstd, dres=dres if residual else None)
+  again = k.rmsnorm_bwd(dy, x, w, rstd, dres=dres if residual else None)
+  xd, wd = x.double().requires_grad_(True), w.double().requires_grad_(True)
+  r = torch.rsqrt(xd.square().mean(-1, keepdim=True) + 1e-5)
+  want = xd * r * wd
+  want.backward(dy.double())
+  assert _rel(rstd, r[:, 0]) < 1e-6
+  assert _rel(y, want) < 2 ** -8
+  assert _rel(dx, xd.grad + dres.double() if residual else xd.grad) < 2 ** -8
+  assert _rel(dw, wd.grad) < 1e-5
+  if rows >= 1024:
+    assert all(torch.equal(a, b) for a, b in zip((dx, dw), again))
+
+
+def test_bad_values_stay_in_their_row(cuda_lib):
+  from torchprime_b200.ops import kernels as k
+  x = torch.randn(2100, 2048, device="cuda").bfloat16()
+  x[7, 3], x[2099, 0] = float("nan"), float("inf")
+  w = torch.ones(2048, device="cuda").bfloat16()
+  y, rstd, _ = k.rmsnorm_fwd(x, w, 1e-5)
+  dx, dw = k.rmsnorm_bwd(torch.randn_like(x), x, w, rstd)
+  good = torch.ones(2100, dtype=torch.bool, device="cuda")
+  good[7] = good[2099] = False
+  for t in (y, dx):
+    assert torch.isfinite(t[good]).all()
+    assert torch.isnan(t[7]).all() and not torch.isfinite(t[2099]).all()
+  assert torch.isnan(dw).all()

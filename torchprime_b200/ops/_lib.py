@@ -91,6 +91,8 @@ def _declare(L):
     "tpb_gemm_ksplit_bf16": [P, P, P, I, I, I, LL, LL, LL, I, I, I, F, P, LL, P, LL, P],
     "tpb_rmsnorm_fwd": [P, P, P, P, P, P, I, I, F, P],
     "tpb_rmsnorm_bwd": [P, P, P, P, P, P, P, I, I, P],
+    "tpb_rmsnorm_bwd_parts": [I, I],
+    "tpb_rmsnorm_bwd_dw": [P, P, P, P, P, P, P, P, I, I, P],
     "tpb_rope": [P, LL, I, I, I, P, P, P, I, I, I, I, P],
     "tpb_rope_strided": [P, LL, I, I, I, I, P, P, P, I, I, I, I, P],
     "tpb_swiglu_fwd": [P, P, I, I, P],

@@ -95,14 +95,18 @@ def rmsnorm_fwd(x, w, eps, res=None, want_h=False):
 
 
 def rmsnorm_bwd(dy, x, w, rstd, dres=None, dw_f32=None):
-  """dx (+ dres) and dw accumulated (atomics) into fp32 ``dw_f32`` [dim]."""
+  """dx (+ dres) and dw in fp32 [dim]; with ``dw_f32`` it is added (atomics) to what is there."""
   d = x.shape[-1]
   dy2, x2 = dy.reshape(-1, d), x.reshape(-1, d)
   assert dy2.is_contiguous() and x2.is_contiguous()
   dx = torch.empty_like(x2)
-  if dw_f32 is None:
-    dw_f32 = torch.zeros(d, dtype=torch.float32, device=x.device)
   dr2 = dres.reshape(-1, d) if dres is not None else None
+  if dw_f32 is None:
+    rows = x2.shape[0]
+    sums = torch.empty(1 + lib().tpb_rmsnorm_bwd_parts(rows, d), d, dtype=torch.float32, device=x.device)
+    check(lib().tpb_rmsnorm_bwd_dw(ptr(dy2), ptr(x2), ptr(w), ptr(rstd), ptr(dr2), ptr(dx), ptr(sums), None, rows, d,
+                                   stream_ptr()), "rmsnorm_bwd")
+    return dx.view(x.shape), sums[0]
   check(lib().tpb_rmsnorm_bwd(ptr(dy2), ptr(x2), ptr(w), ptr(rstd), ptr(dr2), ptr(dx), ptr(dw_f32), x2.shape[0], d,
                               stream_ptr()), "rmsnorm_bwd")
   return dx.view(x.shape), dw_f32
