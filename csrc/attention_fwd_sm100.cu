@@ -270,18 +270,17 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int n_qtiles = (p.Sq + FWD_BM - 1) / FWD_BM;
-  int bx = blockIdx.x, by = blockIdx.y, bz = blockIdx.z;
-  if (p.cp_world > 1) {
-    // one-dimensional grid: the copier CTAs come first so that they are scheduled first
-    if ((int)blockIdx.x < p.cp_copiers) {
-      cp_pusher(p);
-      return;
-    }
-    const int id = (int)blockIdx.x - p.cp_copiers;
-    bx = id % n_qtiles; by = (id / n_qtiles) % p.Hq; bz = id / (n_qtiles * p.Hq);
+  // the copier CTAs of an exchange come first so that they are scheduled first
+  if (p.cp_world > 1 && (int)blockIdx.x < p.cp_copiers) {
+    cp_pusher(p);
+    return;
   }
-  const int qt = n_qtiles - 1 - bx;   // heaviest (latest) tiles first under a causal mask
-  const int hq = by, b = bz;
+  // The heaviest (latest) tiles of all heads come first under a causal mask, so that what runs last is short.  (Head by head
+  // the last head's longest tile began when the others ended, us: 8192 tokens, 32/8 heads 528, this way 480; 4096 160 and 135; two
+  // rows of 1999 tokens in segments 78 and 64; 2048 tokens, 16 heads of 192, all of whose CTAs run at once, 55 and 43.)
+  const int id = (int)blockIdx.x - (p.cp_world > 1 ? p.cp_copiers : 0);
+  const int qt = n_qtiles - 1 - id / (p.Hq * p.B);
+  const int hq = (id / p.B) % p.Hq, b = id % p.B;
   const int hkv = hq / (p.Hq / p.Hkv);
   const int q0 = qt * FWD_BM;
   const int pos_off = p.Sk - p.Sq;
@@ -1042,8 +1041,9 @@ cudaError_t launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUten
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  dim3 grid((p.Sq + FWD_BM - 1) / FWD_BM, p.Hq, p.B);
-  chain(attn_fwd_kernel<DQK, SEG>, grid, FWD_THREADS, FwdSmem<DQK>::TOTAL, stream, tq, tk, tv, p);
+  const long long n = (long long)((p.Sq + FWD_BM - 1) / FWD_BM) * p.Hq * p.B;
+  if (n > 0x7fffffffLL) return cudaErrorInvalidConfiguration;
+  chain(attn_fwd_kernel<DQK, SEG>, (int)n, FWD_THREADS, FwdSmem<DQK>::TOTAL, stream, tq, tk, tv, p);
   return cudaGetLastError();
 }
 
