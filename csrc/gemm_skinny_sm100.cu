@@ -4,7 +4,7 @@
 // output projection of a 4096-wide layer is 16 CTAs, each pulling 2 MB of weights through one SM
 // (about 80 GB/s), while HBM would feed all 148.  Here the roles are swapped and the contraction is split:
 //   * W is the A operand: 128 output features are the 128 lanes of the accumulator, and the tokens
-//     are the N dimension of the MMA (16, 32, 64 or 128), so no MMA or shared-memory bandwidth goes into rows
+//     are the N dimension of the MMA (a multiple of 16 up to 128), so no MMA or shared-memory bandwidth goes into rows
 //     that do not exist beyond the next of those sizes;
 //   * a cluster of S <= 8 CTAs shares one 128-feature tile, each CTA contracting over 1/S of K.
 //     The fp32 partial tiles meet in distributed shared memory, where every CTA adds the S partials of
@@ -48,15 +48,15 @@ constexpr int SK_W_BYTES = SK_TN * SK_BK * 2;    // 16 KB
 constexpr int SK_MAX_SPLIT = 8;                  // portable cluster size
 constexpr int SK_PREFETCH = 8;                   // k-blocks asked for ahead of the kernel before: 128 KB a CTA, 38 MB in all
 
-template <int NT>
-struct SkinnySmem {
-  static constexpr int STAGE = SK_W_BYTES + NT * SK_BK * 2;
-  static constexpr int STAGES = NT <= 16 ? 6 : NT <= 32 ? 5 : NT <= 64 ? 4 : 3;
-  static constexpr int RING = STAGES * STAGE;
-  static constexpr int TOTAL = RING + 1024 + 256;
-  static_assert(NT * SK_TN * 4 <= RING, "the fp32 partial tile reuses the ring");
-  static_assert(2 * (TOTAL + 1024) <= 227 * 1024 + 1024, "two CTAs per SM");
-};
+// A tile holds `nt` rows of X, a multiple of 16 up to the instantiation's NT: no MMA, no shared memory and no exchange for
+// more.  The smaller tile leaves room for more stages.  (A decoder layer of 77 tokens, 4096 wide with a 14336-wide MLP,
+// as tiles of 80 rows instead of 128: 122 -> 116 us.)
+constexpr int SK_MAX_STAGES = 6;
+constexpr int SK_RING = 108 * 1024;              // two CTAs per SM
+constexpr int SK_SMEM = SK_RING + 1024 + 256;
+static_assert(2 * (SK_SMEM + 1024) <= 227 * 1024 + 1024, "two CTAs per SM");
+static int skinny_stage(int nt) { return SK_W_BYTES + nt * SK_BK * 2; }
+static int skinny_stages(int nt) { return SK_RING / skinny_stage(nt) < SK_MAX_STAGES ? SK_RING / skinny_stage(nt) : SK_MAX_STAGES; }
 
 struct SkinnyParams {
   int T, N, K;          // N: output columns (for SwiGLU: of the activation, i.e. half the features of W)
@@ -71,6 +71,7 @@ struct SkinnyParams {
   const float* alpha_dev;   // one more factor, in device memory, or null
   int epi;
   int t_tiles, splits, num_kb, kb_per;
+  int nt, stages, stage_bytes;
   const int* tile_expert;   // grouped: expert of every token tile (-1: unused); null: dense
   int* status;
 };
@@ -128,17 +129,18 @@ template <int NT, bool W_MN, bool X_MN, bool F32>
 __global__ void __launch_bounds__(SK_THREADS, 2)
 gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmW2,
                    const __grid_constant__ CUtensorMap tmX, const SkinnyParams p) {
-  using L = SkinnySmem<NT>;
-  constexpr int NST = L::STAGES;
   constexpr int KSTEPS = SK_BK / 16;
   constexpr uint32_t TMEM_COLS = F32 ? 2 * KSTEPS * NT : NT < 32 ? 32 : NT;   // F32: two buffers of a k-block's results
-  static_assert(!F32 || (TMEM_COLS <= 256 && 2 * NT * SK_TN * 4 <= L::RING), "two CTAs per SM; pairs fit the ring");
+  static_assert(!F32 || TMEM_COLS <= 256, "two CTAs per SM");
+  static_assert((F32 ? 2 : 1) * NT * SK_TN * 4 <= 4 * (SK_W_BYTES + 16 * SK_BK * 2), "the fp32 partial tiles reuse the ring");
+  const int nt = F32 || X_MN ? NT : p.nt;               // rows of X in a tile
+  const int stages = p.stages, stage_bytes = p.stage_bytes;
   const bool swiglu = p.epi == TPB_EPI_SWIGLU;
   const int rank = (int)blockIdx.x % p.splits;          // == %cluster_ctarank of the 1-D cluster
   const int unit = (int)blockIdx.x / p.splits;
-  const int bt = unit % p.t_tiles, nt = unit / p.t_tiles;   // token tiles of one W tile run together (L2)
-  const int t0 = bt * NT;
-  const int n0 = nt * (swiglu ? SK_TN / 2 : SK_TN);
+  const int bt = unit % p.t_tiles;                      // token tiles of one W tile run together (L2)
+  const int t0 = bt * nt;
+  const int n0 = unit / p.t_tiles * (swiglu ? SK_TN / 2 : SK_TN);
   int ez = 0;
   if (p.tile_expert) {
     if (!chain_wait()) return;
@@ -148,9 +150,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   extern __shared__ uint8_t sk_smem_raw[];
   uint8_t* smem = sk_smem_raw + ((1024u - (smem_u32(sk_smem_raw) & 1023u)) & 1023u);
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + L::RING);
-  uint64_t* empty = full + NST;
-  uint64_t* acc_full = empty + NST;
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem + SK_RING);
+  uint64_t* empty = full + SK_MAX_STAGES;
+  uint64_t* acc_full = empty + SK_MAX_STAGES;
   uint64_t* blk_full = acc_full + 1;      // F32: [2] a k-block's results are in their buffer
   uint64_t* blk_empty = blk_full + 2;     // F32: [2] and have been read (one arrival per warp)
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(blk_empty + 2);
@@ -160,7 +162,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const int kb0 = rank * p.kb_per, kb1 = min(p.num_kb, kb0 + p.kb_per);
 
   if (threadIdx.x == 0) {
-    for (int s = 0; s < NST; ++s) {
+    for (int s = 0; s < stages; ++s) {
       mbar_init(&full[s], 1);
       mbar_init(&empty[s], 1);
     }
@@ -200,9 +202,9 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const int nb = swiglu ? p.up_off + n0 : n0 + 64;   // second half of the 128 features
       for (int kb = kb0; kb < kb1; ++kb) {
         if (!mbar_wait(&empty[stage], phase ^ 1, p.status, kTimeoutStageFree, 81)) break;
-        uint8_t* sW = smem + stage * L::STAGE;
+        uint8_t* sW = smem + stage * stage_bytes;
         const int k0 = kb * SK_BK;
-        mbar_expect_tx(&full[stage], L::STAGE);
+        mbar_expect_tx(&full[stage], stage_bytes);
         if (!W_MN) {          // boxes {64 k, 64 features}
           tma_load_3d(sW, &tmW, &full[stage], k0, n0, ez);
           tma_load_3d(sW + SK_W_BYTES / 2, &tmW2, &full[stage], k0, nb, ez);
@@ -216,7 +218,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 #pragma unroll
           for (int c = 0; c < NT / 64; ++c) tma_load_2d(sW + SK_W_BYTES + c * 8192, &tmX, &full[stage], t0 + c * 64, k0);
         }
-        if (++stage == NST) {
+        if (++stage == stages) {
           stage = 0;
           phase ^= 1;
         }
@@ -224,7 +226,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     }
   } else if (warp == 1) {
     if (kb1 > kb0) {
-      constexpr uint32_t idesc = make_idesc_bf16(SK_TN, NT, W_MN, X_MN);
+      const uint32_t idesc = make_idesc_bf16(SK_TN, nt, W_MN, X_MN);
       constexpr uint32_t desc_hi = smem_desc_hi(1024);
       const uint32_t base = smem_u32(smem);
       int stage = 0;
@@ -235,7 +237,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         const int blk = kb - kb0;
         if (F32 && !mbar_wait_warp(&blk_empty[blk & 1], ((blk >> 1) & 1) ^ 1, p.status, kTimeoutAccFree, 84)) { ok = false; break; }
         tc_fence_after();
-        const uint32_t sW = base + stage * L::STAGE;
+        const uint32_t sW = base + stage * stage_bytes;
         const uint32_t a_lo = smem_desc_lo(sW, W_MN ? 8192 : 16);
         const uint32_t b_lo = smem_desc_lo(sW + SK_W_BYTES, X_MN ? 8192 : 16);
         one_lane([&] {
@@ -246,7 +248,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           tc_commit(&empty[stage]);
           if (F32) tc_commit(&blk_full[blk & 1]);
         });
-        if (++stage == NST) {
+        if (++stage == stages) {
           stage = 0;
           phase ^= 1;
         }
@@ -312,7 +314,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     if (kb1 <= kb0 || have) {   // (after a wait that ran out copies may still be landing in the ring)
       constexpr int CH = NT < 32 ? 16 : 32;
 #pragma unroll 1
-      for (int c = 0; c < NT; c += CH) {
+      for (int c = 0; c < nt; c += CH) {      // (of a last half chunk the rest is written and not read)
         uint32_t v[CH];
         if (have) {
           if (CH == 16) tmem_ld16(t_addr + c, v); else tmem_ld32(t_addr + c, v);
@@ -332,7 +334,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   {
     const float alpha = p.alpha_dev ? p.alpha * *p.alpha_dev : p.alpha;
-    const int per = NT / p.splits;                    // tokens this CTA finishes (splits divides 16)
+    const int per = nt / p.splits;                    // tokens this CTA finishes (splits divides 16)
     const int gpt = swiglu ? SK_TN / 8 : SK_TN / 4;   // groups of four features per token
     for (int i = threadIdx.x; i < per * gpt; i += SK_THREADS) {
       const int t = rank * per + i / gpt, c = (i % gpt) * 4;
@@ -390,16 +392,19 @@ static cudaError_t launch_skinny(const CUtensorMap& tw, const CUtensorMap& tw2, 
   static bool configured = false;
   if (!configured) {
     cudaError_t e = cudaFuncSetAttribute(gemm_skinny_kernel<NT, W_MN, X_MN, F32>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         SkinnySmem<NT>::TOTAL);
+                                         SK_SMEM);
     if (e != cudaSuccess) return e;
     configured = true;
   }
-  return chain_clusters(gemm_skinny_kernel<NT, W_MN, X_MN, F32>, p.splits, grid, SK_THREADS, SkinnySmem<NT>::TOTAL, stream, tw, tw2,
+  return chain_clusters(gemm_skinny_kernel<NT, W_MN, X_MN, F32>, p.splits, grid, SK_THREADS, SK_SMEM, stream, tw, tw2,
                         tx, p);
 }
 
-// Token-tile width for `rows` rows: the smallest one that holds them, 128 at most.
-static int skinny_nt(int rows) { return rows <= 16 ? 16 : rows <= 32 ? 32 : rows <= 64 ? 64 : 128; }
+// Rows of a token tile: equal tiles of 128 rows at most, to the next multiple of 16.
+static int skinny_nt(int rows) {
+  const int tiles = (rows + 127) / 128;
+  return ((rows + tiles - 1) / tiles + 15) / 16 * 16;
+}
 
 // K splits: double while the grid still fits the machine at two CTAs per SM and every CTA keeps four
 // k-blocks (256 of K) to amortise its pipeline fill.
@@ -457,14 +462,15 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
   const int extent = two_w ? N / 2 : N;
   const int tile_n = swiglu ? SK_TN / 2 : SK_TN;
   const int n_out = swiglu ? N / 2 : N;
-  if (nt == 0) nt = f32 && T > 16 ? 32 : skinny_nt(T);
+  if (nt == 0) nt = f32 ? (T > 16 ? 32 : 16) : x_mn ? (T > 64 ? 128 : 64) : skinny_nt(T);
   if (f32 && (epi != TPB_EPI_F32 || x_mn || w_mn || tile_expert || nt > 32)) return -2;
   if (x_mn) {
     if (!w_mn || swiglu || tile_expert) return -2;
     if (nt < 64) nt = 64;       // X arrives in blocks of 64 rows
   }
-  if (nt != 16 && nt != 32 && nt != 64 && nt != 128) return -2;
+  if (nt < 16 || nt > 128 || nt % 16 || (x_mn && nt % 64)) return -2;
   SkinnyParams p;
+  p.nt = nt; p.stages = skinny_stages(nt); p.stage_bytes = skinny_stage(nt);
   p.T = T; p.N = n_out; p.K = K;
   p.C = c; p.ldc = ldc;
   p.aux = reinterpret_cast<const __nv_bfloat16*>(aux); p.ldaux = ldaux;
@@ -506,13 +512,8 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
   else if (x_mn)
     e = nt == 64 ? launch_skinny<64, true, true>(tw, tw2, tx, p, grid, stream)
                  : launch_skinny<128, true, true>(tw, tw2, tx, p, grid, stream);
-  else switch (nt) {
-    case 16: e = TPB_SK(16); break;
-    case 32: e = TPB_SK(32); break;
-    case 64: e = TPB_SK(64); break;
-    case 128: e = TPB_SK(128); break;
-    default: return -2;
-  }
+  else
+    e = nt <= 16 ? TPB_SK(16) : nt <= 32 ? TPB_SK(32) : nt <= 64 ? TPB_SK(64) : TPB_SK(128);
 #undef TPB_SK
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }

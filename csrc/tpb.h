@@ -223,7 +223,7 @@ int tpb_symm_barrier(void* const* payloads, int rank, int world, unsigned epoch,
 // dst[i] = bf16(src[i] * *scale), scale in device memory; n % 8 == 0
 int tpb_scale_cast_bf16(const float* src, void* dst, long long n, const float* scale, void* stream);
 
-// ---- GEMM with few rows (gemm_skinny_sm100.cu): Y[T,N] = alpha * X[T,K] W^T (x_mn: X stored [K,T]); nt (16 / 32 / 64 / 128 rows per tile) and
+// ---- GEMM with few rows (gemm_skinny_sm100.cu): Y[T,N] = alpha * X[T,K] W^T (x_mn: X stored [K,T]); nt (rows per tile, a multiple of 16 up to 128) and
 // splits (1 / 2 / 4 / 8 ways along K): 0 = by rule.  tpb_gemm_bf16 calls it where it is the faster kernel.
 int tpb_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, int T, int N, int K, long long ldx,
                          long long ldw, long long ldc, int x_mn, int w_mn, int epi, float alpha, const void* aux,

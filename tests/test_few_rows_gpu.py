@@ -60,6 +60,20 @@ def test_dense_layouts_and_epilogues(cuda_lib, t, nt, n, kk, splits):
       assert bool((big == 7.0).all())
 
 
+@pytest.mark.parametrize("t", [33, 48, 49, 79, 80, 81, 97, 112, 113, 130, 200, 300])
+@pytest.mark.parametrize("b_mn", [False, True])
+def test_tiles_of_any_multiple_of_sixteen_rows(cuda_lib, t, b_mn):
+  """Tiles narrower than the instantiation they run in, with every split of the contraction and a last tile that is not full."""
+  torch.manual_seed(t)
+  x, w = (torch.randn(r, 1160, device="cuda", dtype=torch.bfloat16) for r in (t, 200))
+  want = x.double() @ w.double().t()
+  ww = w.t().contiguous() if b_mn else w
+  for splits in (0, 1, 2, 4, 8):
+    _close(_skinny(x, ww, b_mn=b_mn, splits=splits), want, 1160.0)
+  for nt in (48, 80, 96, 112):
+    assert torch.equal(_skinny(x, ww, b_mn=b_mn, nt=nt, splits=4), _skinny(x, ww, b_mn=b_mn, nt=128, splits=4))
+
+
 @pytest.mark.parametrize("t", [1, 16, 40, 128])
 @pytest.mark.parametrize("f,kk,splits", [(8, 64, 1), (72, 136, 2), (192, 1024, 8), (1408, 512, 0)])
 @pytest.mark.parametrize("b_mn", [False, True])
