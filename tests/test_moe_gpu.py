@@ -124,6 +124,28 @@ def test_grouped_mlp_on_cta_pair_tiles(cuda_lib):
   _lib.raise_on_device_timeout()
 
 
+@pytest.mark.parametrize("T,align", [(255, 128), (256, 256), (480, 256), (482, 128), (702, 128), (704, 256)])
+def test_segment_rows_by_rule(cuda_lib, T, align):
+  """Both sides of every edge of the rule (4 experts, 2 per token), one expert with many rows and one without any, whatever
+  the average: results are those of the other segment width to the order of fp32 sums."""
+  torch.manual_seed(T)
+  E, D, Fd = 4, 128, 192
+  x, dy = (torch.randn(T, D, device="cuda", dtype=torch.bfloat16) for _ in range(2))
+  ws = [(torch.randn(E, a, b, device="cuda") / a ** 0.5).to(torch.bfloat16) for a, b in ((D, Fd), (D, Fd), (Fd, D))]
+  logits = torch.randn(T, E, device="cuda")
+  logits[:, 0] += 2
+  logits[:, 3] = -1e9
+  w, idx, _ = moe.router_topk(logits, 2, mode="softmax")
+  assert moe.build_dispatch_plan(idx, E).row_align == align
+  got = []
+  for plan in (moe.build_dispatch_plan(idx, E), moe.build_dispatch_plan(idx, E, row_align=384 - align)):
+    leaves = [t.detach().requires_grad_(True) for t in (x, w, *ws)]
+    y = moe._GroupedMLPFn.apply(*leaves, plan, False)
+    got.append((y, *torch.autograd.grad(y, leaves, dy)))
+  for a, b in zip(*got):
+    assert torch.isfinite(a.float()).all() and _rel(a, b) < 2 ** -9
+
+
 @pytest.mark.parametrize("E,K,D,Fd,fused", [(4, 2, 128, 256, False), (8, 2, 256, 192, False), (4, 1, 128, 128, True)])
 def test_grouped_mlp_forward_backward(cuda_lib, E, K, D, Fd, fused):
   torch.manual_seed(4)

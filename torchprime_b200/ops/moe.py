@@ -140,6 +140,16 @@ class DispatchPlan:
                              # below 128 only grouped_mlp_few_rows can read the plan)
 
 
+def pair_tiles_pay(per: float) -> bool:
+  """Whether segments of 256 rows, which let the grouped GEMMs use 256 x 256 CTA-pair tiles, are worth their padding for
+  ``per`` rows per expert on average.  They are where the second half of the last segment is used by most experts, and from
+  two segments on.  Routed MLP, both passes but two weight gradients, 128 / 256 rows (us):
+  64 experts of 2048 x 1408: 112 rows 829 / 883, 144 970 / 915, 224 1080 / 1014, 256 1243 / 1267, 320 1389 / 1478, 448 1547 / 1408
+  16 experts of 5120 x 8192: 112 rows 2687 / 2815, 128 3144 / 2787, 224 3489 / 3244, 288 4498 / 4694, 384 5142 / 4708
+  8 experts of 4096 x 14336: 112 rows 1919 / 1876, 160 2319 / 2032, 288 2978 / 3298, 448 3904 / 3465, 768 6080 / 5610"""
+  return 128 <= per <= 240 or per >= 352
+
+
 def build_dispatch_plan(idx: torch.Tensor, num_experts: int, capacity: int | None = None,
                         rows_per_group: int | None = None, use_kernel: bool | None = None,
                         row_align: int | None = None) -> DispatchPlan:
@@ -152,9 +162,7 @@ def build_dispatch_plan(idx: torch.Tensor, num_experts: int, capacity: int | Non
   e = num_experts
   dev = idx.device
   if row_align is None:
-    # 256-row segments let the grouped GEMMs use 256x256 CTA-pair tiles; worth the extra padding
-    # when an expert sees about a thousand rows or more
-    row_align = 256 if (capacity is None and (t * k) // e >= 1024) else ROW_ALIGN
+    row_align = 256 if capacity is None and pair_tiles_pay(t * k / e) else ROW_ALIGN
   assert row_align in (128, 256)
   if use_kernel is None:
     use_kernel = capacity is None and idx.is_cuda and _kernels_ok() and e <= 256
