@@ -74,6 +74,11 @@ struct SkinnyParams {
   int nt, stages, stage_bytes;
   const int* tile_expert;   // grouped: expert of every token tile (-1: unused); null: dense
   int* status;
+  // Two products of one X: feature tiles from n1_tiles on are those of the second W (the second map), with results of their
+  // own.  INT_MAX: one product.
+  int n1_tiles, N2;
+  void* C2;
+  long long ldC2;
 };
 
 // (hi, lo) += c, with lo the sum of hi's rounding errors.
@@ -140,7 +145,11 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
   const int unit = (int)blockIdx.x / p.splits;
   const int bt = unit % p.t_tiles;                      // token tiles of one W tile run together (L2)
   const int t0 = bt * nt;
-  const int n0 = unit / p.t_tiles * (swiglu ? SK_TN / 2 : SK_TN);
+  const bool second = unit / p.t_tiles >= p.n1_tiles;
+  const int n0 = (unit / p.t_tiles - (second ? p.n1_tiles : 0)) * (swiglu ? SK_TN / 2 : SK_TN);
+  const CUtensorMap* mw = second ? &tmW2 : &tmW;        // the tile's first 64 features
+  const CUtensorMap* mw_hi = swiglu ? &tmW2 : mw;       // and the others
+  const int N = second ? p.N2 : p.N;
   int ez = 0;
   if (p.tile_expert) {
     if (!chain_wait()) return;
@@ -177,8 +186,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const int nb = swiglu ? p.up_off + n0 : n0 + 64;
       for (int kb = kb0; kb < min(kb1, kb0 + SK_PREFETCH); ++kb) {
         const int k0 = kb * SK_BK;
-        tma_prefetch_3d(&tmW, W_MN ? n0 : k0, W_MN ? k0 : n0, 0);
-        tma_prefetch_3d(&tmW2, W_MN ? nb : k0, W_MN ? k0 : nb, 0);
+        tma_prefetch_3d(mw, W_MN ? n0 : k0, W_MN ? k0 : n0, 0);
+        tma_prefetch_3d(mw_hi, W_MN ? nb : k0, W_MN ? k0 : nb, 0);
       }
     }
   }
@@ -195,7 +204,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
 
   if (warp == 0) {
     if (elect_one()) {
-      tma_prefetch_desc(&tmW);
+      tma_prefetch_desc(mw);
       tma_prefetch_desc(&tmX);
       int stage = 0;
       uint32_t phase = 0;
@@ -206,11 +215,11 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         const int k0 = kb * SK_BK;
         mbar_expect_tx(&full[stage], stage_bytes);
         if (!W_MN) {          // boxes {64 k, 64 features}
-          tma_load_3d(sW, &tmW, &full[stage], k0, n0, ez);
-          tma_load_3d(sW + SK_W_BYTES / 2, &tmW2, &full[stage], k0, nb, ez);
+          tma_load_3d(sW, mw, &full[stage], k0, n0, ez);
+          tma_load_3d(sW + SK_W_BYTES / 2, mw_hi, &full[stage], k0, nb, ez);
         } else {              // boxes {64 features, 64 k}
-          tma_load_3d(sW, &tmW, &full[stage], n0, k0, ez);
-          tma_load_3d(sW + SK_W_BYTES / 2, &tmW2, &full[stage], nb, k0, ez);
+          tma_load_3d(sW, mw, &full[stage], n0, k0, ez);
+          tma_load_3d(sW + SK_W_BYTES / 2, mw_hi, &full[stage], nb, k0, ez);
         }
         if (!X_MN) {
           tma_load_2d(sW + SK_W_BYTES, &tmX, &full[stage], k0, t0);
@@ -339,8 +348,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
     for (int i = threadIdx.x; i < per * gpt; i += SK_THREADS) {
       const int t = rank * per + i / gpt, c = (i % gpt) * 4;
       const int row = t0 + t, col = n0 + c;
-      if (row >= p.T || col >= p.N) continue;
-      const int n = min(4, p.N - col);
+      if (row >= p.T || col >= N) continue;
+      const int n = min(4, N - col);
       float4 a = F32 ? sum_pairs(smem_u32(part + t * SK_TN + c), NT * SK_TN * 4, p.splits)
                      : sum_partials(smem_u32(part + t * SK_TN + c), p.splits);
       a.x *= alpha; a.y *= alpha; a.z *= alpha; a.w *= alpha;
@@ -376,7 +385,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
           if (n > 2) a.z += __bfloat162float(r[2]);
         }
       }
-      store4(reinterpret_cast<__nv_bfloat16*>(p.C) + (long long)row * p.ldc + col, a, n);
+      store4(reinterpret_cast<__nv_bfloat16*>(second ? p.C2 : p.C) + (long long)row * (second ? p.ldC2 : p.ldc) + col, a, n);
     }
   }
   cluster_sync_all();           // nobody's shared memory goes away while a neighbour reads it
@@ -469,7 +478,8 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
     if (nt < 64) nt = 64;       // X arrives in blocks of 64 rows
   }
   if (nt < 16 || nt > 128 || nt % 16 || (x_mn && nt % 64)) return -2;
-  SkinnyParams p;
+  SkinnyParams p = {};
+  p.n1_tiles = 0x7fffffff;
   p.nt = nt; p.stages = skinny_stages(nt); p.stage_bytes = skinny_stage(nt);
   p.T = T; p.N = n_out; p.K = K;
   p.C = c; p.ldc = ldc;
@@ -521,6 +531,40 @@ int skinny_gemm(const void* x, const void* w, const void* w2, void* c, int T, in
 }  // namespace tpb
 
 using namespace tpb;
+
+// y1 = x w1^T and y2 = x w2^T, x [T,K], all rows back to back, in one launch (a decode step's query and latent projections: six of
+// its microseconds are a second launch).  -2 where one of the two is not this kernel's by the rules above.
+extern "C" int tpb_linear_pair_bf16(const void* x, const void* w1, const void* w2, void* y1, void* y2, int T, int N1, int N2, int K,
+                                    void* stream) {
+  if (T <= 0 || N1 <= 0 || N2 <= 0 || K <= 0) return -2;
+  if (K % 8 || N1 % 8 || N2 % 8 || !skinny_wins(T, N1, K, false) || !skinny_wins(T, N2, K, false)) return -2;
+  for (const void* q : {x, w1, w2, (const void*)y1, (const void*)y2})
+    if (reinterpret_cast<uintptr_t>(q) % 16) return -2;
+  SkinnyParams p = {};
+  p.T = T; p.N = N1; p.K = K; p.C = y1; p.ldc = N1;
+  p.n1_tiles = (N1 + SK_TN - 1) / SK_TN; p.N2 = N2; p.C2 = y2; p.ldC2 = N2;
+  p.alpha = 1.f; p.epi = TPB_EPI_BF16;
+  const int nt = skinny_nt(T);
+  p.nt = nt; p.stages = skinny_stages(nt); p.stage_bytes = skinny_stage(nt);
+  p.t_tiles = (T + nt - 1) / nt;
+  p.num_kb = (K + SK_BK - 1) / SK_BK;
+  p.status = status_block();
+  const long long tiles = ((long long)p.n1_tiles + (N2 + SK_TN - 1) / SK_TN) * p.t_tiles;
+  p.splits = skinny_splits(tiles, p.num_kb);
+  p.kb_per = (p.num_kb + p.splits - 1) / p.splits;
+  if (tiles * p.splits > 0x7fffffffLL) return -2;
+  CUtensorMap t1, t2, tx;
+  if (make_tmap_2d(&tx, x, K, T, K, 64, nt, 2)) return -3;
+  if (make_tmap_3d(&t1, w1, K, N1, 1, K, (uint64_t)K * N1, 64, 64)) return -4;
+  if (make_tmap_3d(&t2, w2, K, N2, 1, K, (uint64_t)K * N2, 64, 64)) return -5;
+  const int grid = (int)(tiles * p.splits);
+  cudaStream_t st = reinterpret_cast<cudaStream_t>(stream);
+  const cudaError_t e = nt <= 16   ? launch_skinny<16, false>(t1, t2, tx, p, grid, st)
+                        : nt <= 32 ? launch_skinny<32, false>(t1, t2, tx, p, grid, st)
+                        : nt <= 64 ? launch_skinny<64, false>(t1, t2, tx, p, grid, st)
+                                   : launch_skinny<128, false>(t1, t2, tx, p, grid, st);
+  return e == cudaSuccess ? 0 : 1000 + (int)e;
+}
 
 // y = x w^T of bf16 operands in fp32: x [T,K], w [N,K], y [T,N].
 extern "C" int tpb_linear_f32(const void* x, const void* w, float* y, int T, int N, int K, long long ldx, long long ldw,

@@ -257,6 +257,30 @@ py::object linear(py::handle x_, py::handle ws_, py::handle res_) {
   return py::cast(y);
 }
 
+// Two projections of the same few rows in one launch, without a graph; see functional.linear_pair.
+py::object linear_pair(py::handle x_, py::handle w1_, py::handle w2_) {
+  Tensor x;
+  Weights w1, w2;
+  if (at::GradMode::is_enabled() || !unobserved() || !unpack(x_, x) || !plain_rows(x) || !w1.add(w1_.ptr()) || !w2.add(w2_.ptr()))
+    return py::none();
+  const int64_t k = w1.k, rows = x.numel() / x.size(-1);
+  if (x.size(-1) != k || w2.k != k || !small(rows) || !small(w1.rows) || !small(w2.rows) || x.get_device() != w1.t[0].get_device() ||
+      x.get_device() != w2.t[0].get_device())
+    return py::none();
+  Tensor y1, y2;
+  int rc;
+  {
+    py::gil_scoped_release nogil;
+    y1 = empty_as(x, with_last(x, w1.rows));
+    y2 = empty_as(x, with_last(x, w2.rows));
+    rc = tpb_linear_pair_bf16(cptr(x), cptr(w1.t[0]), cptr(w2.t[0]), mptr(y1), mptr(y2), (int)rows, (int)w1.rows, (int)w2.rows, (int)k,
+                              stream());
+    if (rc != -2) check(rc, "linear_pair");
+  }
+  if (rc == -2) return py::none();
+  return py::make_tuple(y1, y2);
+}
+
 // ------------------------------------------------------------------------------------------- gate / up with SwiGLU
 struct LinearSwigluFn : Function<LinearSwigluFn> {
   static Tensor forward(AutogradContext* ctx, const Tensor& x, const Tensor& wg, const Tensor& wu) {
@@ -1003,6 +1027,7 @@ PYBIND11_MODULE(_tpb_torch, m) {
   });
   m.def("launch_count", []() { return g_launches.load(); });
   m.def("linear", &linear);
+  m.def("linear_pair", &linear_pair);
   m.def("linear_swiglu", &linear_swiglu);
   m.def("swiglu_mlp", &swiglu_mlp);
   m.def("rms_norm", &rms_norm);

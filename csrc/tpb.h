@@ -239,6 +239,10 @@ int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, const float* co
                    float* part_ml, int B, int H, int dn, int dv, int C, int R, int pos, float scale, float eps,
                    int interleaved, int ranges, void* stream);
 
+// y1 = x w1^T and y2 = x w2^T in one launch; -2 where one of them is not the few-rows kernel's.
+int tpb_linear_pair_bf16(const void* x, const void* w1, const void* w2, void* y1, void* y2, int T, int N1, int N2, int K,
+                         void* stream);
+
 // ---- experts with few rows each: segments padded to nt rows, tile_expert[rows / nt]
 int tpb_moe_gather_real(const void* x, const int* src_row, void* out, long long rows, int dim, void* stream);
 int tpb_grouped_gemm_skinny_bf16(const void* x, const void* w, const void* w2, void* c, int rows, int N, int K, int E,

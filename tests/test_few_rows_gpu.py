@@ -298,3 +298,41 @@ def test_split_tiles_that_take_a_wave_more_are_not_taken(cuda_lib, m, n, few_row
   b = torch.randn(n, kk, device="cuda", generator=g).to(torch.bfloat16)
   want = _skinny(a, b) if few_rows else k.gemm(a, b, max_ctas=148)
   assert torch.equal(k.gemm(a, b), want)
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (4, 1), (16, 1), (2, 17), (3, 32), (128, 1)])
+@pytest.mark.parametrize("n1,n2,kk", [(3072, 576, 2048), (136, 128, 1024), (8, 264, 1096)])
+def test_two_products_of_one_input(cuda_lib, shape, n1, n2, kk):
+  """One launch for both against 64 bits; the projections' own launches give the same to the order of fp32 sums."""
+  from torchprime_b200.ops import functional as ops
+  torch.manual_seed(n1 + shape[0])
+  x = torch.randn(*shape, kk, device="cuda", dtype=torch.bfloat16)
+  w1, w2 = (torch.randn(n, kk, device="cuda", dtype=torch.bfloat16) for n in (n1, n2))
+  with torch.no_grad():
+    nat = ops._native().linear_pair(x, w1, w2)
+    both = ops.linear_pair(x, w1, w2)
+  rows = shape[0] * shape[1]
+  assert (nat is not None) == (rows <= 32 or 8 * rows <= kk)
+  for y, w in zip(both, (w1, w2)):
+    assert y.shape == (*shape, w.shape[0])
+    _close(y, x.double() @ w.double().t(), float(kk))
+    if nat is None:
+      assert torch.equal(y, ops.linear(x, w))
+
+
+def test_two_products_refuse_what_one_launch_cannot_do(cuda_lib):
+  """Other types, layouts and alignments, and calls with a graph, go through the ordinary projections."""
+  from torchprime_b200.ops import functional as ops
+  nat = ops._native()
+  x = torch.randn(4, 1024, device="cuda", dtype=torch.bfloat16)
+  w1, w2 = (torch.randn(n, 1024, device="cuda", dtype=torch.bfloat16) for n in (256, 128))
+  buf = torch.randn(4 * 1024 + 8, device="cuda", dtype=torch.bfloat16)
+  with torch.no_grad():
+    assert nat.linear_pair(x, w1, w2) is not None
+    for a, b, c in ((x.float(), w1, w2), (x, w1.t(), w2), (x, w1, w2[:, :512]), (x[:0], w1, w2), (buf[1:4097].view(4, 1024), w1, w2),
+                    (x, w1[:255], w2), (torch.randn(200, 1024, device="cuda").bfloat16(), w1, torch.randn(40000, 1024, device="cuda").bfloat16())):
+      assert nat.linear_pair(a, b, c) is None
+  assert nat.linear_pair(x, w1, w2) is None
+  w1.requires_grad_(True)
+  y1, y2 = ops.linear_pair(x, w1, w2)
+  assert y1.requires_grad and not y2.requires_grad

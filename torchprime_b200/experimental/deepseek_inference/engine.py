@@ -63,12 +63,12 @@ class DeepseekInferenceEngine:
     b, s, _ = x.shape
     end = start + s
     h, dn, dr, dv, c = attn.num_heads, attn.qk_nope_head_dim, attn.qk_rope_head_dim, attn.v_head_dim, attn.kv_lora_rank
-    if not attn.q_lora_rank:
-      q = ops.linear(x, attn.q_proj.weight)
+    if not attn.q_lora_rank and attn.kv_a_proj_with_mqa.bias is None:
+      q, ckv = ops.linear_pair(x, attn.q_proj.weight, attn.kv_a_proj_with_mqa.weight)
     else:
-      q = ops.linear(attn.q_a_layernorm(ops.linear(x, attn.q_a_proj.weight, bias=attn.q_a_proj.bias)),
-                     attn.q_b_proj.weight)
-    ckv = ops.linear(x, attn.kv_a_proj_with_mqa.weight, bias=attn.kv_a_proj_with_mqa.bias)
+      q = ops.linear(x, attn.q_proj.weight) if not attn.q_lora_rank else ops.linear(
+        attn.q_a_layernorm(ops.linear(x, attn.q_a_proj.weight, bias=attn.q_a_proj.bias)), attn.q_b_proj.weight)
+      ckv = ops.linear(x, attn.kv_a_proj_with_mqa.weight, bias=attn.kv_a_proj_with_mqa.bias)
     norm = attn.kv_a_layernorm
     if self.attn_impl == "absorb" and mla_decode.supported(q, ckv, norm.weight, self.kv_cache[li], self.pe_cache[li],
                                                            attn.kv_b_proj.weight, h, dn, dr, dv, c):

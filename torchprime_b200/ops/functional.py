@@ -325,6 +325,15 @@ def linear(x, weights, bias=None, residual=None, tp_reduce=None, tp_reduce_grad=
   return y if residual is None else y + residual
 
 
+def linear_pair(x, w1, w2):
+  """(x @ w1^T, x @ w2^T).  Without a graph and for few rows (a decode step) both come from one launch."""
+  if (nat := _native()) is not None:
+    both = nat.linear_pair(x, w1, w2)
+    if both is not None:
+      return both
+  return linear(x, w1), linear(x, w2)
+
+
 class _LinearF32Fn(torch.autograd.Function):
   @staticmethod
   def forward(ctx, x, w):
