@@ -94,7 +94,6 @@ constexpr int AUX_STAGE = 4 * BWD_T * 4;
 constexpr int OFF_LIST = OFF_AUX + KV_AUX * AUX_STAGE;       // ushort: the visible tiles in order, kMasked set where scores need a mask
 constexpr int OFF_FLAGS = OFF_LIST + 2 * KV_MAX_TILES;       // uchar per tile: 0 not visible, 1 visible, 2 with a mask
 constexpr int OFF_BAR = OFF_FLAGS + KV_MAX_TILES;
-constexpr uint32_t kMasked = 0x8000;
 // Of a step's two tiles dO is done with first (after dV) and Q last (after dK), and the next step but one needs Q first.  So that
 // step's Q goes where this one's dO was and its dO where this one's Q was: both are asked for two products earlier than they
 // are needed at least.  (A ring of two each asked for Q one product before: 400 of a step's 2970 clocks were spent on its arrival.)
@@ -235,6 +234,47 @@ __device__ __forceinline__ constexpr uint32_t mnmajor_k(int k) { return (uint32_
 // k >> 2 packed its 64 results into the first 32 columns of its own 64-column range.
 __device__ __forceinline__ uint32_t a_col(int k) { return (uint32_t)((k >> 2) * 64 + (k & 3) * 8); }
 
+// The query tiles of QT rows that key block kb of batch row b can see, in order, kMasked set where scores need a mask; from
+// the positions (and segments) of each one's rows.  All threads of the block call; the caller synchronises behind it.
+constexpr uint32_t kMasked = 0x8000;
+template <int QT>
+__device__ __forceinline__ void list_visible_tiles(const AttnBwdParams& p, bool seg, int b, int kb, int n_tiles, uint8_t* flags,
+                                                   uint16_t* list, int* n_list) {
+  const int kv0 = kb * BWD_T, pos_off = p.Sk - p.Sq, lane = threadIdx.x & 31;
+  const int2 kseg_rng = seg ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
+  for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
+    const int r0 = t * QT, r1 = min(p.Sq, r0 + QT);
+    int mn = 0x7fffffff, mx = -0x7fffffff;
+    if (p.q_pos) {
+      for (int r = r0; r < r1; ++r) {
+        const int v = p.q_pos[(long long)b * p.Sq + r];
+        mn = min(mn, v); mx = max(mx, v);
+      }
+    } else {
+      mn = r0 + pos_off; mx = r1 - 1 + pos_off;
+    }
+    bool vis = !(p.causal && mx < kv0) && !(p.window > 0 && mn - (kv0 + BWD_T - 1) >= p.window), one_seg = false;
+    if (seg) {
+      const int2 qr = QT == SEG_BLK ? p.q_rng[(long long)b * n_tiles + t] : seg_range128(p.q_rng, b, t, p.Sq);
+      one_seg = qr.x == qr.y && kseg_rng.x == kseg_rng.y && qr.x == kseg_rng.x;
+      if (qr.y < kseg_rng.x || qr.x > kseg_rng.y) vis = false;   // no segment in common
+    }
+    const bool mask = (kv0 + BWD_T > p.Sk) || (p.causal && mn < kv0 + BWD_T - 1) || (p.window > 0 && mx - kv0 >= p.window) ||
+                      (p.q_seg != nullptr && !one_seg);
+    flags[t] = vis ? (mask ? 2 : 1) : 0;
+  }
+  __syncthreads();
+  if (threadIdx.x >= 32) return;
+  int n = 0;
+  for (int t0 = 0; t0 < n_tiles; t0 += 32) {
+    const int f = t0 + lane < n_tiles ? flags[t0 + lane] : 0;
+    const uint32_t seen = __ballot_sync(0xffffffffu, f != 0);
+    if (f) list[n + __popc(seen & ((1u << lane) - 1))] = (uint16_t)((t0 + lane) | (f == 2 ? kMasked : 0u));
+    n += __popc(seen);
+  }
+  if (lane == 0) *n_list = n;
+}
+
 // ------------------------------------------------------------------------------------------
 // dK / dV
 // ------------------------------------------------------------------------------------------
@@ -289,40 +329,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tmem_relinquish();
   }
   if (!chain_wait()) return;
-  // which query tiles this key block can see, from the positions (and segments) of each one's rows
-  const int2 kseg_rng = SEG ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
-  for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
-    const int r0 = t * BWD_T, r1 = min(p.Sq, r0 + BWD_T);
-    int mn = 0x7fffffff, mx = -0x7fffffff;
-    if (p.q_pos) {
-      for (int r = r0; r < r1; ++r) {
-        const int v = p.q_pos[(long long)b * p.Sq + r];
-        mn = min(mn, v); mx = max(mx, v);
-      }
-    } else {
-      mn = r0 + pos_off; mx = r1 - 1 + pos_off;
-    }
-    bool vis = !(p.causal && mx < kv0) && !(p.window > 0 && mn - (kv0 + BWD_T - 1) >= p.window), one_seg = false;
-    if (SEG) {
-      const int2 qr = seg_range128(p.q_rng, b, t, p.Sq);
-      one_seg = qr.x == qr.y && kseg_rng.x == kseg_rng.y && qr.x == kseg_rng.x;
-      if (qr.y < kseg_rng.x || qr.x > kseg_rng.y) vis = false;   // no segment in common
-    }
-    const bool mask = (kv0 + BWD_T > p.Sk) || (p.causal && mn < kv0 + BWD_T - 1) || (p.window > 0 && mx - kv0 >= p.window) ||
-                      (p.q_seg != nullptr && !one_seg);
-    flags[t] = vis ? (mask ? 2 : 1) : 0;
-  }
-  __syncthreads();
-  if (warp == 0) {
-    int n = 0;
-    for (int t0 = 0; t0 < n_tiles; t0 += 32) {
-      const int f = t0 + lane < n_tiles ? flags[t0 + lane] : 0;
-      const uint32_t seen = __ballot_sync(0xffffffffu, f != 0);
-      if (f) list[n + __popc(seen & ((1u << lane) - 1))] = (uint16_t)((t0 + lane) | (f == 2 ? kMasked : 0u));
-      n += __popc(seen);
-    }
-    if (lane == 0) *n_list = n;
-  }
+  list_visible_tiles<BWD_T>(p, SEG, b, kb, n_tiles, flags, list, n_list);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -942,7 +949,8 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 // pass of its own over the keys for delta = rowsum(P o dP), which from the bf16 result would carry its rounding.  Error of
 // dq / dk / dv against 64 bits, 1024 tokens in segments: 1.66e-3, the rounding of the gradients themselves (single bf16 terms:
 // 3.5e-3, 3.5e-3, 2.3e-3).
-// One row of 2048 tokens, 16 heads, causal: dK/dV 70, dQ 44, delta 8 us; with all tokens in one segment, so that FINE does it, 1.4
+// One row of 2048 tokens, 16 heads, causal: dK/dV, dQ and delta 124 us, 108 with issuers whose warps stay together and the list
+// of visible tiles; with all tokens in one segment, so that FINE does it, 1.4
 // times that.  (torch's scaled_dot_product_attention, used
 // here before: backward 90 us after running its own forward again, 41 us, and three copies.)
 // ------------------------------------------------------------------------------------------
@@ -961,9 +969,9 @@ constexpr int OFF_Q = OFF_V + TILE_BYTES;
 constexpr int OFF_DO = OFF_Q + W_STAGES * W_Q_BYTES;
 constexpr int OFF_AUX = OFF_DO + W_STAGES * W_DO_BYTES;      // per Q stage: lse2[64], delta[64], qpos[64], qseg[64]
 constexpr int AUX_STAGE = 4 * W_QT * 4;
-constexpr int OFF_TILES = OFF_AUX + W_STAGES * AUX_STAGE;
-constexpr int OFF_SEGONE = OFF_TILES + 2 * W_MAX_TILES * 4;
-constexpr int OFF_BAR = OFF_SEGONE + W_MAX_TILES;
+constexpr int OFF_LIST = OFF_AUX + W_STAGES * AUX_STAGE;     // as in the kernel above
+constexpr int OFF_FLAGS = OFF_LIST + 2 * W_MAX_TILES;
+constexpr int OFF_BAR = OFF_FLAGS + W_MAX_TILES;
 constexpr int TOTAL = OFF_BAR + 256 + 1024;
 static_assert(TOTAL <= 227 * 1024, "shared memory of one CTA");
 constexpr int T_DK = 0, T_DV = 192, T_S = 320, T_DP = 448;
@@ -1037,14 +1045,14 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
   uint64_t* do_full = q_empty + W_STAGES;
   uint64_t* do_empty = do_full + W_STAGES;
   uint64_t* s_full = do_empty + W_STAGES;         // [2] S^T of a step is in its buffer
-  uint64_t* p_full = s_full + 2;                  // [2] count 256: P^T written over it
+  uint64_t* p_full = s_full + 2;                  // [2] one arrival per compute warp: P^T written over it
   uint64_t* dp_full = p_full + 2;
-  uint64_t* ds_full = dp_full + 1;                // count 256: dS^T written
+  uint64_t* ds_full = dp_full + 1;                // the same: dS^T written
   uint64_t* acc_done = ds_full + 1;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(acc_done + 1);
-  int* tile_min = reinterpret_cast<int*>(smem + OFF_TILES);
-  int* tile_max = tile_min + W_MAX_TILES;
-  uint8_t* seg_one = smem + OFF_SEGONE;
+  int* n_list = reinterpret_cast<int*>(acc_done + 2);
+  uint16_t* list = reinterpret_cast<uint16_t*>(smem + OFF_LIST);
+  uint8_t* flags = smem + OFF_FLAGS;
 
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int kb = blockIdx.x / (p.Hkv * p.B);      // key-block major: the heaviest blocks first under a causal mask
@@ -1060,8 +1068,8 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       mbar_init(&q_full[i], 1); mbar_init(&q_empty[i], 1);
       mbar_init(&do_full[i], 1); mbar_init(&do_empty[i], 1);
     }
-    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 256); }
-    mbar_init(dp_full, 1); mbar_init(ds_full, 256);
+    for (int i = 0; i < 2; ++i) { mbar_init(&s_full[i], 1); mbar_init(&p_full[i], 8); }
+    mbar_init(dp_full, 1); mbar_init(ds_full, 8);
     mbar_init(acc_done, 1);
     fence_barrier_init();
   }
@@ -1070,40 +1078,13 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     tmem_relinquish();
   }
   if (!chain_wait()) return;
-  // position range of every query tile; a tile that shares no segment with this key block gets an empty one
-  const int2 kseg_rng = p.kv_rng ? seg_range128(p.kv_rng, b, kb, p.Sk) : make_int2(0, 0);
-  for (int t = threadIdx.x; t < n_tiles; t += BWD_THREADS) {
-    const int r0 = t * W_QT, r1 = min(p.Sq, r0 + W_QT);
-    int mn = 0x7fffffff, mx = -0x7fffffff;
-    if (p.q_pos) {
-      for (int r = r0; r < r1; ++r) {
-        const int v = p.q_pos[(long long)b * p.Sq + r];
-        mn = min(mn, v); mx = max(mx, v);
-      }
-    } else {
-      mn = r0 + pos_off; mx = r1 - 1 + pos_off;
-    }
-    if (p.kv_rng) {
-      const int2 qr = p.q_rng[(long long)b * n_tiles + t];   // W_QT == SEG_BLK
-      seg_one[t] = qr.x == qr.y && kseg_rng.x == kseg_rng.y && qr.x == kseg_rng.x;
-      if (qr.y < kseg_rng.x || qr.x > kseg_rng.y) { mn = 0x7fffffff; mx = -0x7fffffff; }
-    }
-    tile_min[t] = mn; tile_max[t] = mx;
-  }
+  list_visible_tiles<W_QT>(p, p.kv_rng != nullptr, b, kb, n_tiles, flags, list, n_list);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   chain_launch();
-
-  auto visible = [&](int t) -> bool {
-    if (tile_min[t] > tile_max[t]) return false;
-    if (p.causal && tile_max[t] < kv0) return false;
-    if (p.window > 0 && tile_min[t] - (kv0 + BWD_T - 1) >= p.window) return false;
-    return true;
-  };
-  int n_vis = 0;
-  for (int t = 0; t < n_tiles; ++t) n_vis += visible(t) ? 1 : 0;
+  const int n_vis = *n_list;
   const int n_steps = n_vis * G;
 
   if (warp == 0) {
@@ -1122,11 +1103,10 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
       bool ok = true;
       for (int g = 0; g < G && ok; ++g) {
         const int hq = hkv * G + g;
-        for (int t = 0; t < n_tiles && ok; ++t) {
-          if (!visible(t)) continue;
+        for (int v = 0; v < n_vis; ++v) {
           const int st = step % W_STAGES;
           const uint32_t ph = ((step / W_STAGES) & 1) ^ 1;
-          const int q0 = t * W_QT;
+          const int q0 = (int)(list[v] & (kMasked - 1)) * W_QT;
           int okw = 1;
           if (lane == 0) okw = mbar_wait(&q_empty[st], ph, p.status, kTimeoutStageFree, 121) ? 1 : 0;
           okw = __shfl_sync(0xffffffffu, okw, 0);
@@ -1258,14 +1238,13 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
     bool ok = true;
     int step = 0;
     for (int g = 0; g < G && ok; ++g) {
-      for (int t = 0; t < n_tiles && ok; ++t) {
-        if (!visible(t)) continue;
+      for (int v = 0; v < n_vis && ok; ++v) {
+        const uint32_t entry = list[v];
+        const int t = (int)(entry & (kMasked - 1));
         const float* aux = reinterpret_cast<const float*>(smem + OFF_AUX + (step % W_STAGES) * AUX_STAGE);
         const int* auxi = reinterpret_cast<const int*>(aux);
         const uint32_t tS = tb + T_S + (step & 1) * W_QT + half * 32;
-        const bool need_mask = !key_ok || (kv0 + BWD_T > p.Sk) || (p.causal && tile_min[t] < kv0 + BWD_T - 1) ||
-                               (p.window > 0 && tile_max[t] - kv0 >= p.window) ||
-                               (p.q_seg != nullptr && !(p.kv_rng && seg_one[t]));
+        const bool need_mask = (entry & kMasked) != 0;
         // ---- phase 1: P^T = exp2(S^T * c - lse)
         if (!mbar_wait(&s_full[step & 1], (step >> 1) & 1, p.status, kTimeoutAccFull, 127)) { ok = false; break; }
         tc_fence_after();
@@ -1307,7 +1286,8 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         tmem_wait_st();
         tc_fence_before();
-        mbar_arrive(&p_full[step & 1]);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&p_full[step & 1]);
         // ---- phase 2: dS^T = P^T o (dP^T - delta), written over dP^T
         if (!mbar_wait(dp_full, step & 1, p.status, kTimeoutAccFull, 128)) { ok = false; break; }
         tc_fence_after();
@@ -1328,7 +1308,8 @@ attn_bwd_dkv192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_con
         }
         tmem_wait_st();
         tc_fence_before();
-        mbar_arrive(ds_full);
+        __syncwarp();
+        if (lane == 0) mbar_arrive(ds_full);
         ++step;
       }
     }
