@@ -525,9 +525,149 @@ __global__ void a2a_wait_kernel(const unsigned* flags, int world, unsigned epoch
   }
 }
 
+// ----------------------------------------------------------------------------
+// Gradients of fp32 logits y = x w^T (x [T,K], w [N,K] bf16, dy [T,N] fp32), N of a router's size: products and sums in fp32
+// on the FMA pipe, one rounding to bf16.  As library products each operand was first copied to fp32 and each result from it: 72 us
+// for 1500 tokens, 64 experts, K = 2048, of which these take 33.  Bound by FMA issue: 0.2 G of them each.
+// ----------------------------------------------------------------------------
+// dx = dy w.  A CTA makes 64 rows x 128 columns, a warp eight rows, a thread 8 x 4; dy is read as broadcasts.
+constexpr int RG_THREADS = 256, RG_ROWS = 64, RG_COLS = 128, RG_STEP = 64;
+__global__ void __launch_bounds__(RG_THREADS)
+logit_dx_kernel(const float* __restrict__ dy, const __nv_bfloat16* __restrict__ w, __nv_bfloat16* __restrict__ dx, int T, int N,
+                int K, long long ldw) {
+  if (!chain_begin()) return;
+  __shared__ __align__(16) float sdy[RG_ROWS][RG_STEP + 4];
+  __shared__ __align__(16) __nv_bfloat16 sw[RG_STEP][RG_COLS];
+  const int t0 = blockIdx.y * RG_ROWS, c0 = blockIdx.x * RG_COLS;
+  const int lane = threadIdx.x & 31, r0 = (threadIdx.x >> 5) * 8;
+  float acc[8][4] = {};
+  for (int n0 = 0; n0 < N; n0 += RG_STEP) {
+    if (n0) __syncthreads();
+    for (int i = threadIdx.x; i < RG_ROWS * RG_STEP; i += RG_THREADS) {
+      const int r = i / RG_STEP, n = i % RG_STEP;
+      sdy[r][n] = t0 + r < T && n0 + n < N ? dy[(size_t)(t0 + r) * N + n0 + n] : 0.f;
+    }
+    for (int i = threadIdx.x; i < RG_STEP * RG_COLS / 8; i += RG_THREADS) {
+      const int n = i / (RG_COLS / 8), c = i % (RG_COLS / 8) * 8;
+      uint4 v = make_uint4(0, 0, 0, 0);       // (K is a multiple of 8)
+      if (n0 + n < N && c0 + c < K) v = *reinterpret_cast<const uint4*>(w + (size_t)(n0 + n) * ldw + c0 + c);
+      *reinterpret_cast<uint4*>(&sw[n][c]) = v;
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int n = 0; n < RG_STEP; n += 4) {
+      float4 d[8];
+#pragma unroll
+      for (int r = 0; r < 8; ++r) d[r] = *reinterpret_cast<const float4*>(&sdy[r0 + r][n]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const uint2 u = *reinterpret_cast<const uint2*>(&sw[n + e][lane * 4]);
+        const float2 a = unpack_bf16(u.x), b = unpack_bf16(u.y);
+#pragma unroll
+        for (int r = 0; r < 8; ++r) {
+          const float x = e == 0 ? d[r].x : e == 1 ? d[r].y : e == 2 ? d[r].z : d[r].w;
+          acc[r][0] = fmaf(x, a.x, acc[r][0]);
+          acc[r][1] = fmaf(x, a.y, acc[r][1]);
+          acc[r][2] = fmaf(x, b.x, acc[r][2]);
+          acc[r][3] = fmaf(x, b.y, acc[r][3]);
+        }
+      }
+    }
+  }
+  const int c = c0 + lane * 4;
+  if (c >= K) return;
+#pragma unroll
+  for (int r = 0; r < 8; ++r)
+    if (t0 + r0 + r < T)
+      *reinterpret_cast<uint2*>(dx + (size_t)(t0 + r0 + r) * K + c) =
+          make_uint2(pack_bf16(acc[r][0], acc[r][1]), pack_bf16(acc[r][2], acc[r][3]));
+}
+
+// dw = dy^T x.  64 x 64 results to a cluster of eight CTAs, each adding up an eighth of the tokens (a thread 4 x 4); the eight sums of a
+// result meet in distributed shared memory and are added in rank order.
+constexpr int RG_SPLIT = 8, RG_TOK = 32, RG_TILE = 64;
+__global__ void __launch_bounds__(RG_THREADS)
+logit_dw_kernel(const float* __restrict__ dy, const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ dw, int T, int N,
+                int K, long long ldx) {
+  if (!chain_begin()) return;
+  __shared__ __align__(16) float sdy[RG_TOK][RG_TILE];
+  __shared__ __align__(16) float sx[RG_TOK][RG_TILE];
+  __shared__ __align__(16) float part[RG_TILE][RG_TILE];
+  const int rank = (int)cluster_ctarank();
+  const int c0 = (int)(blockIdx.x / RG_SPLIT) * RG_TILE, n0 = blockIdx.y * RG_TILE;
+  const int per = (T + RG_SPLIT - 1) / RG_SPLIT, t_begin = rank * per, t_end = min(T, t_begin + per);
+  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  float acc[4][4] = {};
+  float dreg[RG_TOK * RG_TILE / RG_THREADS];
+  uint4 xreg = make_uint4(0, 0, 0, 0);
+  const int xt = threadIdx.x / (RG_TILE / 8), xc = threadIdx.x % (RG_TILE / 8) * 8;
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int i = 0; i < RG_TOK * RG_TILE / RG_THREADS; ++i) {
+      const int at = i * RG_THREADS + (int)threadIdx.x, t = t0 + at / RG_TILE, n = n0 + at % RG_TILE;
+      dreg[i] = t < t_end && n < N ? dy[(size_t)t * N + n] : 0.f;
+    }
+    xreg = make_uint4(0, 0, 0, 0);
+    if (t0 + xt < t_end && c0 + xc < K) xreg = *reinterpret_cast<const uint4*>(x + (size_t)(t0 + xt) * ldx + c0 + xc);
+  };
+  fetch(t_begin);
+  for (int t0 = t_begin; t0 < t_end; t0 += RG_TOK) {
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < RG_TOK * RG_TILE / RG_THREADS; ++i) (&sdy[0][0])[i * RG_THREADS + threadIdx.x] = dreg[i];
+    const float2 a = unpack_bf16(xreg.x), b = unpack_bf16(xreg.y), c = unpack_bf16(xreg.z), d = unpack_bf16(xreg.w);
+    *reinterpret_cast<float4*>(&sx[xt][xc]) = make_float4(a.x, a.y, b.x, b.y);
+    *reinterpret_cast<float4*>(&sx[xt][xc + 4]) = make_float4(c.x, c.y, d.x, d.y);
+    __syncthreads();
+    fetch(t0 + RG_TOK);
+#pragma unroll 8
+    for (int t = 0; t < RG_TOK; ++t) {
+      const float4 g = *reinterpret_cast<const float4*>(&sdy[t][ty * 4]), v = *reinterpret_cast<const float4*>(&sx[t][tx * 4]);
+      const float gg[4] = {g.x, g.y, g.z, g.w}, vv[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = fmaf(gg[i], vv[j], acc[i][j]);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+    *reinterpret_cast<float4*>(&part[ty * 4 + i][tx * 4]) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+  cluster_sync_all();
+  // this CTA's eight of the 64 rows, two columns to a thread
+  const int n = rank * (RG_TILE / RG_SPLIT) + (int)threadIdx.x / (RG_TILE / 2), c = (int)threadIdx.x % (RG_TILE / 2) * 2;
+  float s0 = 0.f, s1 = 0.f;
+#pragma unroll
+  for (int r = 0; r < RG_SPLIT; ++r) {
+    float a, b;
+    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(map_to_cta(smem_u32(&part[n][c]), r)) : "memory");
+    s0 += a; s1 += b;
+  }
+  if (n0 + n < N && c0 + c < K) *reinterpret_cast<uint32_t*>(dw + (size_t)(n0 + n) * K + c0 + c) = pack_bf16(s0, s1);
+  cluster_sync_all();           // nobody's shared memory goes away while a neighbour reads it
+}
+
 }  // namespace tpb
 
 using namespace tpb;
+
+// Gradients of y = x w^T with fp32 y (tpb_linear_f32): dx [T,K], dw [N,K] bf16, contiguous (either may be null); dy contiguous.
+extern "C" int tpb_linear_f32_bwd(const float* dy, const void* x, const void* w, void* dx, void* dw, int T, int N, int K,
+                                  long long ldx, long long ldw, void* stream) {
+  if (T <= 0 || N <= 0 || K <= 0) return -2;
+  if (K % 8 || ldx % 8 || ldw % 8 || (T + RG_ROWS - 1) / RG_ROWS > 65535 || (N + RG_TILE - 1) / RG_TILE > 65535) return -2;
+  for (const void* p : {x, w, (const void*)dx, (const void*)dw})
+    if (reinterpret_cast<uintptr_t>(p) % 16) return -2;
+  cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
+  if (dx)
+    chain(logit_dx_kernel, dim3((K + RG_COLS - 1) / RG_COLS, (T + RG_ROWS - 1) / RG_ROWS), RG_THREADS, 0, s, dy,
+          (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, T, N, K, ldw);
+  if (dw)
+    chain_clusters(logit_dw_kernel, RG_SPLIT, dim3(RG_SPLIT * ((K + RG_TILE - 1) / RG_TILE), (N + RG_TILE - 1) / RG_TILE), RG_THREADS, 0,
+                   s, dy, (const __nv_bfloat16*)x, (__nv_bfloat16*)dw, T, N, K, ldx);
+  const cudaError_t e = cudaGetLastError();
+  return e == cudaSuccess ? 0 : 1000 + (int)e;
+}
 #define STREAM(s) reinterpret_cast<cudaStream_t>(s)
 static inline int rc_of(cudaError_t e) { return e == cudaSuccess ? 0 : 1000 + (int)e; }
 

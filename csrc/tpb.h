@@ -239,6 +239,10 @@ int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, const float* co
                    float* part_ml, int B, int H, int dn, int dv, int C, int R, int pos, float scale, float eps,
                    int interleaved, int ranges, void* stream);
 
+// Gradients of tpb_linear_f32: dx = dy w, dw = dy^T x in fp32, rounded to bf16 once (either may be null).
+int tpb_linear_f32_bwd(const float* dy, const void* x, const void* w, void* dx, void* dw, int T, int N, int K, long long ldx,
+                       long long ldw, void* stream);
+
 // y1 = x w1^T and y2 = x w2^T in one launch; -2 where one of them is not the few-rows kernel's.
 int tpb_linear_pair_bf16(const void* x, const void* w1, const void* w2, void* y1, void* y2, int T, int N1, int N2, int K,
                          void* stream);

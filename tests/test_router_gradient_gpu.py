@@ -43,6 +43,32 @@ def test_linear_f32_gradients(cuda_lib):
   assert torch.equal(dx, (dy @ w.float()).to(torch.bfloat16)) and torch.equal(dw, (dy.t() @ x.float()).to(torch.bfloat16))
 
 
+@pytest.mark.parametrize("T,N,K", [(256, 64, 2048), (257, 8, 64), (1500, 64, 136), (300, 65, 1032), (1031, 256, 512), (4000, 120, 200)])
+def test_linear_f32_gradient_kernels(cuda_lib, T, N, K):
+  """Edges of rows, experts and columns; a view of wider rows; sums are fp32 ones (T or N terms) rounded to bf16 once."""
+  torch.manual_seed(T)
+  x = torch.randn(T, K + 8, device="cuda").bfloat16()[:, :K].requires_grad_(True)
+  w = torch.randn(N, K, device="cuda").bfloat16().requires_grad_(True)
+  dy = torch.randn(T, N, device="cuda")
+  dx, dw = torch.autograd.grad(ops.linear_f32(x, w), (x, w), dy)
+  for got, a, b in ((dx, dy.double(), w.detach().double()), (dw, dy.double().t(), x.detach().double())):
+    want, size = a @ b, a.abs() @ b.abs()
+    assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6 * size).all())
+  (only,) = torch.autograd.grad(ops.linear_f32(x, w.detach()), x, dy)
+  assert torch.equal(only, dx)
+
+
+def test_linear_f32_gradient_of_a_gradient(cuda_lib):
+  x = torch.randn(300, 64, device="cuda").bfloat16().requires_grad_(True)
+  w = torch.randn(16, 64, device="cuda").bfloat16().requires_grad_(True)
+  dy = torch.randn(300, 16, device="cuda", requires_grad=True)
+  (dx,) = torch.autograd.grad(ops.linear_f32(x, w), x, dy, create_graph=True)
+  ddy, dw = torch.autograd.grad(dx.float().square().sum(), (dy, w))
+  assert ddy.shape == dy.shape and dw.abs().sum() > 0
+  many = torch.autograd.grad(ops.linear_f32(x, w), x, torch.stack([dy, 2 * dy]).detach(), is_grads_batched=True)[0]
+  assert torch.equal(many[0], (dy @ w.float()).to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("E,K", [(8, 2), (64, 6), (256, 8)])
 @pytest.mark.parametrize("mode", ["softmax", "sigmoid"])
 @pytest.mark.parametrize("norm", [True, False])

@@ -76,6 +76,18 @@ def linear_f32(x, w):
   return out
 
 
+def linear_f32_bwd(dy, x, w, want_dx=True, want_dw=True):
+  """Gradients (dx, dw) of :func:`linear_f32`; None for one that is not wanted."""
+  t, kk, ldx = _row_major_2d(x, "x")
+  n, _, ldw = _row_major_2d(w, "w")
+  assert dy.is_contiguous() and dy.dtype == torch.float32 and dy.shape == (t, n)
+  dx = torch.empty(t, kk, dtype=x.dtype, device=x.device) if want_dx else None
+  dw = torch.empty(n, kk, dtype=w.dtype, device=w.device) if want_dw else None
+  check(lib().tpb_linear_f32_bwd(ptr(dy), ptr(x), ptr(w), ptr(dx), ptr(dw), t, n, kk, ldx, ldw, stream_ptr()),
+        f"linear_f32_bwd {t}x{n}x{kk}")
+  return dx, dw
+
+
 def rmsnorm_fwd(x, w, eps, res=None, want_h=False):
   """Returns (y, rstd, h) with h = x + res (None unless ``res`` given and ``want_h``)."""
   d = x.shape[-1]
