@@ -344,6 +344,11 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// The same where nothing written in front of it has to be seen behind it: the CTAs of a cluster have all got here, so none of
+// them reads another's shared memory any more.  (The release above waits until a thread's results have reached memory.)
+__device__ __forceinline__ void cluster_leave() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 // Address of this CTA's shared-memory location `saddr` as seen in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t saddr, uint32_t rank) {
   uint32_t r;

@@ -983,7 +983,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
 
   tc_fence_before();
   __syncthreads();
-  if (PAIR) cluster_sync_all();   // neither CTA's shared memory or TMEM goes away under the other
+  if (PAIR) cluster_leave();   // neither CTA's shared memory or TMEM goes away under the other
   if (warp == 1) {
     tc_fence_after();
     if (PAIR) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512);

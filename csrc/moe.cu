@@ -644,7 +644,7 @@ logit_dw_kernel(const float* __restrict__ dy, const __nv_bfloat16* __restrict__ 
     s0 += a; s1 += b;
   }
   if (n0 + n < N && c0 + c < K) *reinterpret_cast<uint32_t*>(dw + (size_t)(n0 + n) * K + c0 + c) = pack_bf16(s0, s1);
-  cluster_sync_all();           // nobody's shared memory goes away while a neighbour reads it
+  cluster_leave();           // nobody's shared memory goes away while a neighbour reads it
 }
 
 }  // namespace tpb
