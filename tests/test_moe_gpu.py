@@ -98,6 +98,43 @@ def test_dispatch_plan_kernel_equals_the_sort_based_plan(cuda_lib, T, K, E):
   assert torch.equal(a.dest, again.dest)
 
 
+@pytest.mark.parametrize("T,K,E", [(256, 6, 64), (257, 6, 33), (1537, 1, 256), (770, 2, 7), (2600, 7, 1)])
+def test_dispatch_plan_in_one_and_in_eight_blocks(cuda_lib, T, K, E):
+  """Both sides of the number of pairs from which a cluster shares the sort, with entries that are no expert."""
+  torch.manual_seed(T)
+  idx = torch.randint(0, E, (T, K), device="cuda", dtype=torch.int32)
+  idx[::5, 0] = -1
+  a = moe._build_dispatch_plan_kernel(idx, E)
+  flat = idx.reshape(-1).long()
+  order = torch.argsort(torch.where(flat < 0, E, flat), stable=True)[: int((flat >= 0).sum())]
+  counts = torch.bincount(flat[flat >= 0], minlength=E)
+  ends = ((counts + 127) // 128 * 128).cumsum(0)
+  start = ends - (counts + 127) // 128 * 128
+  rank = torch.arange(len(order), device="cuda") - (counts.cumsum(0) - counts)[flat[order]]
+  dest = torch.full_like(flat, -1)
+  dest[order] = start[flat[order]] + rank
+  assert torch.equal(a.counts.long(), counts) and torch.equal(a.k_offsets.long(), torch.cat([ends.new_zeros(1), ends]))
+  assert torch.equal(a.dest.reshape(-1).long(), dest)
+  pair = torch.full((a.num_rows,), -1, dtype=torch.long, device="cuda")
+  pair[dest[order]] = order
+  assert torch.equal(a.src_pair, pair) and torch.equal(a.src_row.long(), torch.where(pair < 0, pair, pair // K))
+
+
+@pytest.mark.parametrize("T,K,D", [(1, 1, 8), (4, 6, 2048), (296, 10, 2048), (297, 9, 2048), (700, 2, 4096)])
+def test_combine_few_and_many_tokens(cuda_lib, T, K, D):
+  """Both sides of the number of threads from which a thread's rows follow one another, more pairs than are taken together."""
+  torch.manual_seed(T)
+  rows = torch.randn(T * K + 3, D, device="cuda").bfloat16()
+  dest = torch.randperm(T * K + 3, device="cuda")[: T * K].reshape(T, K).to(torch.int32)
+  dest[:, K // 2] = torch.where(torch.arange(T, device="cuda") % 3 == 1, -1, dest[:, K // 2])
+  w = torch.randn(T, K, device="cuda")
+  for wt in (w, None):
+    got = moe.combine_rows(rows, dest, wt)
+    terms = rows.double()[dest.clamp(min=0).long()] * (dest >= 0)[..., None] * (1 if wt is None else wt.double()[..., None])
+    want, size = terms.sum(1), terms.abs().sum(1)
+    assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6 * size).all())
+
+
 def test_grouped_mlp_on_cta_pair_tiles(cuda_lib):
   """Enough rows per expert for 256-row segments: the forward, input-gradient and weight-gradient
   grouped GEMMs run on 256x256 CTA-pair tiles; one expert gets no rows at all."""
