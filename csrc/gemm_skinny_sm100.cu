@@ -445,8 +445,12 @@ bool skinny_wins(int M, int N, int K, bool swiglu) {
 // us per call, tiled / this kernel, for 256, 1024, 4096 rows:
 //   576 x 2048, 40 tiles: 7 / 10, 13 / 12, 31 / 22      4096 x 512, 64 tiles: 8 / 11, 13 / 13, 31 / 23
 //   64 x 2048, 8 tiles: 7 / 7, 11 / 7, 31 / 10          2048 x 2048, 128 tiles: 8 / 13, 13 / 18, 34 / 37
+// Against the CTA pairs that take 256 x 256 tiles otherwise, 1500, 2048, 3000 rows, pairs / this kernel (with the launch):
+//   4096 x 512: 12.7 / 14.2, 15.4 / 16.0, 19.6 / 19.2      576 x 2048: 12.1 / 13.0, 14.7 / 14.6, 19.0 / 17.7
+//   2048 x 1024: 12.6 / 13.4, 15.2 / 15.1, 19.6 / 18.5
 bool skinny_wins_wgrad(int M, int N, int K) {
-  return K >= 1024 && (long long)((M + 127) / 128) * ((N + 255) / 256) <= sm_count() / 2;
+  const long long tiles = (long long)((M + 127) / 128) * ((N + 255) / 256);
+  return K >= (tiles <= 16 ? 1024 : 2048) && tiles <= sm_count() / 2;
 }
 
 // x [T,K], or [K,T] with x_mn (for grouped mode: all padded rows), w dense [N,K] (w_mn = 0) or [K,N] (w_mn = 1), with

@@ -1095,14 +1095,12 @@ bool skinny_wins_wgrad(int M, int N, int K);
 // K = 4096, 8192, 14336 (weights from HBM):
 //   T = 24, 32, 33, one wave:            29 / 27, 37 / 32, 68 / 55      27 / 25, 37 / 31, 68 / 55      24 / 22, 38 / 32, 69 / 55
 //   T = 34, 36, the few-rows kernel's:   24 / 37, 43 / 61, 73 / 102     23 / 35, 40 / 60, 67 / 98
-//   T = 40, 48, 64, two waves:           31 / 35, 60 / 57, 105 / 93     32 / 35, 60 / 57, 108 / 95     31 / 36, 61 / 59, 111 / 101
+//   T = 40, 48, 64, two waves against one of pairs (K = 10944):   48: 57 / 65, 64: 61 / 70
 //   T = 68, 72, three against one:       31 / 51, 69 / 100, 118 / 164   32 / 52, 65 / 91, 112 / 149
 //   T = 80, 96, three against two:       49 / 53, 95 / 88, 167 / 142    48 / 52, 94 / 88, 170 / 153
 //   T = 105, four against two:           50 / 68, 108 / 127, 182 / 201
 //   T = 160, five against three:         - , 154 / 160, 274 / 261 (K = 20480: 392 / 356)
-// With whole waves of 128-row tiles to fill (48 tiles of 300 rows: 72 of 128 rows), the few-rows kernel is ahead of two
-// waves as well (39 / 57); up to 16 tiles it is ahead of one (T = 16: 24 / 31).  Two waves against one that 128-row tiles
-// fill to five sixths and more need K = 10240 (T = 63: 75 / 77, 84 / 82; T = 66: 64 / 65, 83 / 82 for K = 8192, 10240).
+// Up to 16 tiles the few-rows kernel is ahead of one wave (T = 16: 24 / 31).
 static bool ksplit_wins(int M, int N, int K) {
   if (M <= 128 || K < 4096) return false;
   const long long t = (long long)((M + 2 * BM - 1) / (2 * BM)) * ((N + BN - 1) / BN);
@@ -1112,9 +1110,7 @@ static bool ksplit_wins(int M, int N, int K) {
   if (t <= clusters) return true;
   const long long half = (t + clusters - 1) / clusters, whole = (t + pairs - 1) / pairs;
   if (K < 8192 || skinny_wins(M, N, K, false)) return false;
-  if (whole > 1) return half < 2 * whole && (whole == 2 || K >= 20480);
-  const long long t128 = (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN);
-  return half == 2 && (K >= 10240 || 6 * t128 <= 5 * sm_count());
+  return whole > 1 && half < 2 * whole && (whole == 2 || K >= 20480);
 }
 
 // gemm_skinny_sm100.cu
@@ -1271,7 +1267,11 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   if (rs_rotate)
     p.tile_rot = (int)(tiles * g.rs_rank / g.rs_world);   // every rank starts in a different owner's part of C
   cudaError_t e;
-  // CTA pairs for dense GEMMs with enough 256 x 256 tiles to fill the machine
+  // CTA pairs: whatever the number of their tiles.  What an SM does is the same (128 x 256 results), but a pair's SM brings in and
+  // reads half of B: 512 clocks a k-block, where the single kernel is bound by shared memory at 768.  us, single / pair, 64 tiles
+  // or fewer of 256 x 256: K = 4096, 300 to 1024 rows 30 / 25; K = 2048, 900 x 3072 17.7 / 16.1, 2048 x 2048 17.7 / 16.1; K = 10944,
+  // 2048 x 2048 73.7 / 61.3; K = 512, 4096 columns 10.5 / 10.3 (profiles/pair_tiles_gemm_sweep.md).  Up to 128 rows half of a pair has
+  // none.  With a gather or a scatter inside, where the tiles fill the machine.
   const int pair_mode = gemm_pair_mode();
   static const int max_pairs = resident_clusters(2);
   const long long pair_tiles = (long long)((g.M + 2 * BM - 1) / (2 * BM)) * n_tiles * (g.mode == 2 ? g.E : 1);
@@ -1291,7 +1291,8 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
     return e == cudaSuccess ? 0 : 1000 + (int)e;
   }
   if (pair_mode != 0 && max_pairs > 0 && pair_shape_ok && pair_coll_ok &&
-      g.max_ctas == 0 && (pair_mode == 2 || pair_tiles >= max_pairs)) {
+      g.max_ctas == 0 && (pair_mode == 2 || pair_tiles >= max_pairs || (g.M > BM && g.ag_world == 0 && g.rs_world == 0 &&
+                                                                        g.epi != TPB_EPI_AR_BF16))) {
     p.te_stride = 2;
     if (rs_rotate) p.tile_rot = (int)(pair_tiles * g.rs_rank / g.rs_world);
     const int pairs = pair_tiles > max_pairs ? max_pairs : (int)pair_tiles;

@@ -99,3 +99,23 @@ def test_weight_gradients_stop_at_the_padding(cuda_lib, counts, align):
   for x, c in enumerate(counts):
     want = a[off[x]:off[x] + c].double().t() @ b[off[x]:off[x] + c].double()
     assert bool(((out[x].double() - want).abs() <= 2e-6 * max(c, 1) + 1e-6).all())
+
+
+@pytest.mark.parametrize("m,n,kk", [(129, 8, 72), (255, 264, 520), (257, 1000, 64), (300, 136, 1000), (640, 512, 200)])
+@pytest.mark.parametrize("a_mn,b_mn", [(False, False), (False, True), (True, True)])
+def test_few_tiles_on_pairs_are_those_of_single_ctas(cuda_lib, m, n, kk, a_mn, b_mn):
+  """Products of a few 256 x 256 tiles run on CTA pairs; the kernel for one CTA (a limit on CTAs asks for it) sums in the
+  same order."""
+  torch.manual_seed(m + n)
+  m8 = (m + 7) // 8 * 8 if a_mn else m
+  a = torch.randn(*((kk, m8) if a_mn else (m8, kk)), device="cuda").bfloat16()
+  b = torch.randn(*((kk, n) if b_mn else (n, kk)), device="cuda").bfloat16()
+  res = torch.randn(m8, n, device="cuda").bfloat16()
+  for epi, aux in ((k.EPI_BF16, None), (k.EPI_F32, None), (k.EPI_BF16_RES, res)):
+    got = k.gemm(a, b, a_mn=a_mn, b_mn=b_mn, epi=epi, aux=aux)
+    assert torch.equal(got, k.gemm(a, b, a_mn=a_mn, b_mn=b_mn, epi=epi, aux=aux, max_ctas=148))
+    want = (a.double().t() if a_mn else a.double()) @ (b.double() if b_mn else b.double().t())
+    want = want + res.double() if aux is not None else want
+    assert ((got.double() - want).norm() / want.norm()).item() < 2 ** -8
+  if not a_mn and n % 16 == 0:
+    assert torch.equal(k.gemm(a, b, b_mn=b_mn, epi=k.EPI_SWIGLU), k.gemm(a, b, b_mn=b_mn, epi=k.EPI_SWIGLU, max_ctas=148))
