@@ -329,6 +329,15 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
     tmem_relinquish();
   }
   if (!chain_wait()) return;
+  // K is on its way while the query tiles that can see it are found
+  if (warp == 0) {
+    one_lane([&] {
+      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
+      mbar_expect_tx(k_full, TILE_BYTES);
+      for (int c = 0; c < BWD_D / 64; ++c)
+        tma_load_3d(smem + OFF_K + c * (BWD_T * 128), &tmK, k_full, c * 64, b * p.Sk + kv0, hkv);
+    });
+  }
   list_visible_tiles<BWD_T>(p, SEG, b, kb, n_tiles, flags, list, n_list);
   tc_fence_before();
   __syncthreads();
@@ -340,13 +349,9 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
 
   if (warp == 0) {
     // ------------------------------------------------------------------ producer
-    if (n_steps > 0) {
-      if (lane == 0) {
-        tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
-        mbar_expect_tx(k_full, TILE_BYTES);
-        for (int c = 0; c < BWD_D / 64; ++c)
-          tma_load_3d(smem + OFF_K + c * (BWD_T * 128), &tmK, k_full, c * 64, b * p.Sk + kv0, hkv);
-      }
+    if (n_steps == 0) {
+      mbar_wait_warp(k_full, 0, p.status, kTimeoutTmaFull, 22);   // (nothing reads it, but it has to have landed)
+    } else {
       const bool aux_rows = p.q_pos != nullptr || p.q_seg != nullptr;
       int step = 0;
       bool ok = true;
@@ -696,16 +701,27 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   chain_launch();
   if (!chain_wait()) return;
 
-  if (threadIdx.x < BWD_T) {
-    const int r = q0 + threadIdx.x;
-    if (r < p.Sq) {
-      const int qp = p.q_pos ? p.q_pos[(long long)b * p.Sq + r] : r + pos_off;
+  // Q is on its way while the key blocks that it can see are found
+  if (warp == 0) {
+    one_lane([&] {
+      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
+      mbar_expect_tx(q_full, TILE_BYTES);
+#pragma unroll
+      for (int c = 0; c < BWD_D / 64; ++c)
+        tma_load_3d(smem + OFF_Q + c * (BWD_T * 128), &tmQ, q_full, c * 64, b * p.Sq + q0, hq);
+    });
+  }
+  int qpos_min = q0 + pos_off, qpos_max = min(q0 + BWD_T, p.Sq) - 1 + pos_off;
+  if (p.q_pos) {
+    if (threadIdx.x < BWD_T && q0 + (int)threadIdx.x < p.Sq) {
+      const int qp = p.q_pos[(long long)b * p.Sq + q0 + threadIdx.x];
       atomicMin(&tile_minmax[0], qp);
       atomicMax(&tile_minmax[1], qp);
     }
+    __syncthreads();
+    qpos_min = tile_minmax[0];
+    qpos_max = tile_minmax[1];
   }
-  __syncthreads();
-  const int qpos_min = tile_minmax[0], qpos_max = tile_minmax[1];
   const int nblk_total = (p.Sk + BWD_T - 1) / BWD_T;
   int blk_hi = p.causal ? min(nblk_total, qpos_max / BWD_T + 1) : nblk_total;
   int blk_lo = (p.window > 0 && qpos_min >= p.window) ? (qpos_min - p.window + 1) / BWD_T : 0;
@@ -728,12 +744,9 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (nblk > 0 && elect_one()) {
-      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
-      mbar_expect_tx(q_full, TILE_BYTES);
-#pragma unroll
-      for (int c = 0; c < BWD_D / 64; ++c)
-        tma_load_3d(smem + OFF_Q + c * (BWD_T * 128), &tmQ, q_full, c * 64, b * p.Sq + q0, hq);
+    if (nblk == 0) {
+      mbar_wait_warp(q_full, 0, p.status, kTimeoutTmaFull, 32);   // (nothing reads it, but it has to have landed)
+    } else if (elect_one()) {
       for (int j = 0; j < nblk; ++j) {
         const int sk = j % DQ_KSTAGES, sv = j % DQ_VSTAGES;
         const int row = b * p.Sk + (blk_lo + j) * BWD_T;
@@ -1387,16 +1400,17 @@ attn_bwd_dq192_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_cons
   chain_launch();
   if (!chain_wait()) return;
 
-  if (threadIdx.x < BWD_T) {
-    const int r = q0 + threadIdx.x;
-    if (r < p.Sq) {
-      const int qp = p.q_pos ? p.q_pos[(long long)b * p.Sq + r] : r + pos_off;
+  int qpos_min = q0 + pos_off, qpos_max = min(q0 + BWD_T, p.Sq) - 1 + pos_off;
+  if (p.q_pos) {
+    if (threadIdx.x < BWD_T && q0 + (int)threadIdx.x < p.Sq) {
+      const int qp = p.q_pos[(long long)b * p.Sq + q0 + threadIdx.x];
       atomicMin(&tile_minmax[0], qp);
       atomicMax(&tile_minmax[1], qp);
     }
+    __syncthreads();
+    qpos_min = tile_minmax[0];
+    qpos_max = tile_minmax[1];
   }
-  __syncthreads();
-  const int qpos_min = tile_minmax[0], qpos_max = tile_minmax[1];
   const int nblk_total = (p.Sk + BWD_T - 1) / BWD_T;
   int blk_hi = p.causal ? min(nblk_total, qpos_max / BWD_T + 1) : nblk_total;
   int blk_lo = (p.window > 0 && qpos_min >= p.window) ? (qpos_min - p.window + 1) / BWD_T : 0;

@@ -309,17 +309,28 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
   if (p.cp_world <= 1) chain_launch();   // (with an exchange, this kernel waits for other GPUs)
   if (!chain_wait()) return;
 
+  // The tile's rows are on their way while the key blocks they can see are found.
+  if (warp == 0) {
+    one_lane([&] {
+      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
+      mbar_expect_tx(q_full, L::Q_BYTES);
+#pragma unroll
+      for (int c = 0; c < DQK / 64; ++c)
+        tma_load_3d(smem + c * (FWD_BM * 128), &tmQ, q_full, c * 64, b * p.Sq + q0, hq);
+    });
+  }
   // Range of positions covered by this tile's query rows.
-  if (threadIdx.x < FWD_BM) {
-    const int r = q0 + threadIdx.x;
-    if (r < p.Sq) {
-      const int qp = p.q_pos ? p.q_pos[(long long)b * p.Sq + r] : r + pos_off;
+  int qpos_min = q0 + pos_off, qpos_max = min(q0 + FWD_BM, p.Sq) - 1 + pos_off;
+  if (p.q_pos) {
+    if (threadIdx.x < FWD_BM && q0 + (int)threadIdx.x < p.Sq) {
+      const int qp = p.q_pos[(long long)b * p.Sq + q0 + threadIdx.x];
       atomicMin(&tile_minmax[0], qp);
       atomicMax(&tile_minmax[1], qp);
     }
+    __syncthreads();
+    qpos_min = tile_minmax[0];
+    qpos_max = tile_minmax[1];
   }
-  __syncthreads();
-  const int qpos_min = tile_minmax[0], qpos_max = tile_minmax[1];
   const int nblk_total = (p.Sk + FWD_BN - 1) / FWD_BN;
   int blk_hi = p.causal ? min(nblk_total, qpos_max / FWD_BN + 1) : nblk_total;
   int blk_lo = (p.window > 0 && qpos_min >= p.window) ? (qpos_min - p.window + 1) / FWD_BN : 0;
@@ -350,12 +361,9 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
 
   if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer
-    if (nblk > 0 && elect_one()) {
-      tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV);
-      mbar_expect_tx(q_full, L::Q_BYTES);
-#pragma unroll
-      for (int c = 0; c < DQK / 64; ++c)
-        tma_load_3d(sQ + c * (FWD_BM * 128), &tmQ, q_full, c * 64, b * p.Sq + q0, hq);
+    if (nblk == 0) {
+      mbar_wait_warp(q_full, 0, p.status, kTimeoutTmaFull, 13);   // (nothing reads it, but it has to have landed)
+    } else if (elect_one()) {
       for (int j = 0; j < nblk; ++j) {
         const int s = j & 1;
         const uint32_t ph = (j >> 1) & 1;
