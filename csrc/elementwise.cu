@@ -69,11 +69,13 @@ rmsnorm_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, c
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const uint4* xr = x + (size_t)row * nvec;
     float vals[VPT][8];
+    uint4 wu[VPT];              // (asked for with the row, not behind its sum)
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
       int i = threadIdx.x + j * NORM_THREADS;
       if (i < nvec) {
+        wu[j] = w[i];
         unpack8(xr[i], vals[j]);
         if (res) {
           float r[8];
@@ -94,7 +96,7 @@ rmsnorm_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, c
       int i = threadIdx.x + j * NORM_THREADS;
       if (i < nvec) {
         float wv[8], o[8];
-        unpack8(w[i], wv);
+        unpack8(wu[j], wv);
 #pragma unroll
         for (int e = 0; e < 8; ++e) o[e] = wv[e] * rbf(vals[j][e] * rstd);
         y[(size_t)row * nvec + i] = pack8(o);

@@ -350,6 +350,10 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       const int row = t0 + t, col = n0 + c;
       if (row >= p.T || col >= N) continue;
       const int n = min(4, N - col);
+      // (the residual is asked for ahead of the neighbours' sums)
+      const __nv_bfloat16* res = p.epi == TPB_EPI_BF16_RES ? p.aux + (long long)row * p.ldaux + col : nullptr;
+      uint2 old = make_uint2(0, 0);
+      if (res && n >= 4) old = *reinterpret_cast<const uint2*>(res);
       float4 a = F32 ? sum_pairs(smem_u32(part + t * SK_TN + c), NT * SK_TN * 4, p.splits)
                      : sum_partials(smem_u32(part + t * SK_TN + c), p.splits);
       a.x *= alpha; a.y *= alpha; a.z *= alpha; a.w *= alpha;
@@ -373,16 +377,14 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
         }
         continue;
       }
-      if (p.epi == TPB_EPI_BF16_RES) {
-        const __nv_bfloat16* r = p.aux + (long long)row * p.ldaux + col;
+      if (res) {
         if (n >= 4) {
-          const uint2 o = *reinterpret_cast<const uint2*>(r);
-          const float2 r0 = unpack_bf16(o.x), r1 = unpack_bf16(o.y);
+          const float2 r0 = unpack_bf16(old.x), r1 = unpack_bf16(old.y);
           a.x += r0.x; a.y += r0.y; a.z += r1.x; a.w += r1.y;
         } else {
-          a.x += __bfloat162float(r[0]);
-          if (n > 1) a.y += __bfloat162float(r[1]);
-          if (n > 2) a.z += __bfloat162float(r[2]);
+          a.x += __bfloat162float(res[0]);
+          if (n > 1) a.y += __bfloat162float(res[1]);
+          if (n > 2) a.z += __bfloat162float(res[2]);
         }
       }
       store4(reinterpret_cast<__nv_bfloat16*>(second ? p.C2 : p.C) + (long long)row * (second ? p.ldC2 : p.ldc) + col, a, n);

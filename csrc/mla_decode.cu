@@ -54,20 +54,26 @@ mla_prep_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__
   const int b = blockIdx.x;
   const float* cs = cosT + (size_t)pos * (MLA_R / 2);
   const float* sn = sinT + (size_t)pos * (MLA_R / 2);
+  const __nv_bfloat16* row = ckv + (size_t)b * (C + MLA_R);
+  // the latent and its weight are asked for first: their sum is the longest way through this kernel
+  constexpr int PER = MLA_MAX_C / MLA_THREADS;
+  float v[PER], nw[PER], ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int i = threadIdx.x + k * MLA_THREADS;
+    v[k] = i < C ? __bfloat162float(row[i]) : 0.f;
+    nw[k] = i < C ? __bfloat162float(norm_w[i]) : 0.f;
+  }
   for (int i = threadIdx.x; i < H * (MLA_R / 2); i += MLA_THREADS) {
     const int h = i / (MLA_R / 2), j = i % (MLA_R / 2);
     __nv_bfloat16* x = q + ((size_t)b * H + h) * (dn + MLA_R) + dn;
     mla_rotate(x, x, j, interleaved, cs[j], sn[j]);
   }
-  const __nv_bfloat16* row = ckv + (size_t)b * (C + MLA_R);
   if (threadIdx.x < MLA_R / 2)
     mla_rotate(row + C, pe_cache + b * pe_bs + (size_t)pos * MLA_R, threadIdx.x, interleaved, cs[threadIdx.x],
                sn[threadIdx.x]);
-  float ss = 0.f;
-  for (int i = threadIdx.x; i < C; i += MLA_THREADS) {
-    const float v = __bfloat162float(row[i]);
-    ss += v * v;
-  }
+#pragma unroll
+  for (int k = 0; k < PER; ++k) ss += v[k] * v[k];
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
@@ -77,9 +83,11 @@ mla_prep_kernel(__nv_bfloat16* __restrict__ q, const __nv_bfloat16* __restrict__
   for (int w = 0; w < 8; ++w) ss += red[w];
   const float rstd = rsqrtf(ss / (float)C + eps);
   // the same two roundings as the norm kernel of the other paths
-  for (int i = threadIdx.x; i < C; i += MLA_THREADS)
-    kv_cache[b * kv_bs + (size_t)pos * C + i] =
-        __float2bfloat16(__bfloat162float(norm_w[i]) * mla_rbf(__bfloat162float(row[i]) * rstd));
+#pragma unroll
+  for (int k = 0; k < PER; ++k) {
+    const int i = threadIdx.x + k * MLA_THREADS;
+    if (i < C) kv_cache[b * kv_bs + (size_t)pos * C + i] = __float2bfloat16(nw[k] * mla_rbf(v[k] * rstd));
+  }
 }
 
 // Grid (H, C / 64, ceil(B / 8)).  A thread holds 8 columns of every 32nd d: its 16-byte loads of the weight
@@ -374,6 +382,33 @@ mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ par
   const int h = blockIdx.x, b = blockIdx.y;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const float* ml = part_ml + ((size_t)b * H + h) * ranges * 2;
+  const int rank = share > 1 ? (int)cluster_ctarank() : 0;
+  const int cols = C / share, pairs = cols / 2;      // this CTA's columns, two to a thread
+  const int groups = MLA_THREADS / pairs;            // threads with the same columns take every groups-th range
+  const int pr = threadIdx.x % pairs, grp = threadIdx.x / pairs;
+  // Everything that comes from memory is asked for at once: the weight rows of this warp, the first partial sums and, below,
+  // the ranges' maxima.  (One after the other, each waiting for the one before, a decode step of three layers took 294 us;
+  // this way, with the norms' weights and the residuals asked for early too, 281.)
+  const uint4* wv = reinterpret_cast<const uint4*>(w + ((size_t)h * (dn + dv) + dn) * C);
+  const int cv = C / 8;
+  const int j0 = blockIdx.z * rows, j1 = min(dv, j0 + rows);
+  constexpr int WK = MLA_MAX_C / 8 / 32, AHEAD = 12;
+  uint4 wr[WK][4];
+  auto load_rows = [&](int j) {
+#pragma unroll
+    for (int k = 0; k < WK; ++k)
+#pragma unroll
+      for (int r = 0; r < 4; ++r)
+        wr[k][r] = (lane + 32 * k < cv && j + r < j1) ? wv[(size_t)(j + r) * cv + lane + 32 * k] : make_uint4(0, 0, 0, 0);
+  };
+  load_rows(j0 + 4 * warp);
+  const float* po = part_o + ((size_t)b * H + h) * ranges * C + rank * cols + 2 * pr;
+  float2 ahead[AHEAD];
+#pragma unroll
+  for (int i = 0; i < AHEAD; ++i) {
+    const int r = grp + i * groups;
+    if (grp < groups && r < ranges) ahead[i] = *reinterpret_cast<const float2*>(po + (size_t)r * C);
+  }
   if (warp == 0) {
     float m = -INFINITY;
     for (int r = lane; r < ranges; r += 32) m = fmaxf(m, ml[2 * r]);
@@ -391,16 +426,19 @@ mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ par
     for (int r = lane; r < ranges; r += 32) merge_w[r] *= inv;
   }
   __syncthreads();
-  const int rank = share > 1 ? (int)cluster_ctarank() : 0;
-  const int cols = C / share, pairs = cols / 2;      // this CTA's columns, two to a thread
-  const int groups = MLA_THREADS / pairs;            // threads with the same columns take every groups-th range
-  const int pr = threadIdx.x % pairs, grp = threadIdx.x / pairs;
   {
     float x = 0.f, y = 0.f;
     if (grp < groups) {
-      const float* po = part_o + ((size_t)b * H + h) * ranges * C + rank * cols + 2 * pr;
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) {
+        const int r = grp + i * groups;
+        if (r < ranges) {
+          x += merge_w[r] * ahead[i].x;
+          y += merge_w[r] * ahead[i].y;
+        }
+      }
 #pragma unroll 8
-      for (int r = grp; r < ranges; r += groups) {
+      for (int r = grp + AHEAD * groups; r < ranges; r += groups) {
         const float2 v = *reinterpret_cast<const float2*>(po + (size_t)r * C);
         x += merge_w[r] * v.x;
         y += merge_w[r] * v.y;
@@ -427,17 +465,13 @@ mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ par
     __syncthreads();
   }
   // a warp takes four rows at a time: their loads are in flight together
-  const uint4* wv = reinterpret_cast<const uint4*>(w + ((size_t)h * (dn + dv) + dn) * C);
-  const int cv = C / 8;
-  const int j0 = blockIdx.z * rows, j1 = min(dv, j0 + rows);
   for (int j = j0 + 4 * warp; j < j1; j += 4 * (MLA_THREADS / 32)) {
+    if (j != j0 + 4 * warp) load_rows(j);
     float s[4] = {};
 #pragma unroll
-    for (int k = 0; k < MLA_MAX_C / 8 / 32; ++k) {
+    for (int k = 0; k < WK; ++k) {
       const int c = lane + 32 * k;
-      uint4 v[4];
-#pragma unroll
-      for (int r = 0; r < 4; ++r) v[r] = (c < cv && j + r < j1) ? wv[(size_t)(j + r) * cv + c] : make_uint4(0, 0, 0, 0);
+      const uint4* v = wr[k];
       if (c < cv) {
         const float4 x0 = *reinterpret_cast<const float4*>(olat + c * 8), x1 = *reinterpret_cast<const float4*>(olat + c * 8 + 4);
 #pragma unroll
