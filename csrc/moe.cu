@@ -36,8 +36,9 @@ __device__ __forceinline__ float warp_sum_f(float v) {
 //   mode 1: s = sigmoid(logits); selection score = s + bias, restricted to the topk_group
 //           groups with the largest (sum of top-2 selection scores); weights = s at the
 //           selected experts, normalised (if norm_topk) and multiplied by `scale`.
+// (The bias may be bf16, as a model keeps it: a conversion was a launch of its own, and one that breaks the chain of launches.)
 template <typename T>
-__global__ void router_topk_kernel(const T* __restrict__ logits, const float* __restrict__ bias,
+__global__ void router_topk_kernel(const T* __restrict__ logits, const void* __restrict__ bias, int bias_bf16,
                                    float* __restrict__ w_out, int* __restrict__ idx_out,
                                    float* __restrict__ scores_out, int tokens, int E, int K, int mode, int n_group,
                                    int topk_group, int norm_topk, float scale) {
@@ -78,7 +79,11 @@ __global__ void router_topk_kernel(const T* __restrict__ logits, const float* __
         const int e = j * 32 + lane;
         const bool ok = j < per_lane && e < E;
         s[j] = ok ? 1.f / (1.f + __expf(-s[j])) : 0.f;
-        sel[j] = ok ? s[j] + (bias ? bias[e] : 0.f) : -INFINITY;
+        sel[j] = -INFINITY;
+        if (ok)
+          sel[j] = s[j] + (!bias ? 0.f
+                           : bias_bf16 ? __bfloat162float(reinterpret_cast<const __nv_bfloat16*>(bias)[e])
+                                       : reinterpret_cast<const float*>(bias)[e]);
       }
       if (n_group > 1) {
         const int gs = E / n_group;
@@ -726,19 +731,20 @@ extern "C" int tpb_linear_f32_bwd(const float* dy, const void* x, const void* w,
 #define STREAM(s) reinterpret_cast<cudaStream_t>(s)
 static inline int rc_of(cudaError_t e) { return e == cudaSuccess ? 0 : 1000 + (int)e; }
 
-extern "C" int tpb_router_topk(const void* logits, int logits_is_bf16, const float* bias, float* w_out, int* idx_out,
+extern "C" int tpb_router_topk(const void* logits, int bf16, const void* bias, float* w_out, int* idx_out,
                                float* scores_out, int tokens, int E, int K, int mode, int n_group, int topk_group,
                                int norm_topk, float scale, void* stream) {
   if (E > 32 * ROUTER_MAX_PER_LANE || K > 32 || K > E || E <= 0) return -2;
   if (mode == 1 && n_group > 1 && (E % n_group || n_group > 32 || topk_group > n_group)) return -2;
   if (tokens <= 0) return 0;
   const int grid = grid_for_items((long long)tokens * 32, 256);
-  if (logits_is_bf16)
+  const int bias_bf16 = (bf16 >> 1) & 1;
+  if (bf16 & 1)
     chain(router_topk_kernel<__nv_bfloat16>, grid, 256, 0, STREAM(stream),
-          (const __nv_bfloat16*)logits, bias, w_out, idx_out, scores_out, tokens, E, K, mode, n_group, topk_group,
+          (const __nv_bfloat16*)logits, bias, bias_bf16, w_out, idx_out, scores_out, tokens, E, K, mode, n_group, topk_group,
         norm_topk, scale);
   else
-    chain(router_topk_kernel<float>, grid, 256, 0, STREAM(stream), (const float*)logits, bias, w_out, idx_out, scores_out,
+    chain(router_topk_kernel<float>, grid, 256, 0, STREAM(stream), (const float*)logits, bias, bias_bf16, w_out, idx_out, scores_out,
                                                                 tokens, E, K, mode, n_group, topk_group, norm_topk,
                                                                 scale);
   return rc_of(cudaGetLastError());

@@ -959,9 +959,9 @@ py::object router_topk(py::handle lg_, py::handle bias_, int64_t k, int64_t mode
                        bool norm_topk, double scale) {
   Tensor lg, bias, w, idx, scores;
   if (at::GradMode::is_enabled() || !unobserved() || !unpack(lg_, lg) || !unpack(bias_, bias)) return py::none();
-  if (bias.defined() && plain_rows(bias)) bias = bias.to(at::kFloat);
+  const bool bias16 = bias.defined() && plain_rows(bias);
   if (!(plain_rows(lg, at::kFloat) || plain_rows(lg)) || lg.dim() != 2 || lg.size(1) > 256 || k < 1 || k > lg.size(1) ||
-      !small(lg.size(0)) || (bias.defined() && (!plain_rows(bias, at::kFloat) || bias.numel() != lg.size(1))))
+      !small(lg.size(0)) || (bias.defined() && (!(bias16 || plain_rows(bias, at::kFloat)) || bias.numel() != lg.size(1))))
     return py::none();
   {
     py::gil_scoped_release nogil;
@@ -969,7 +969,7 @@ py::object router_topk(py::handle lg_, py::handle bias_, int64_t k, int64_t mode
     w = empty_like_type(lg, {t, k}, at::kFloat);
     idx = empty_like_type(lg, {t, k}, at::kInt);
     scores = empty_like_type(lg, {t, e}, at::kFloat);
-    check(tpb_router_topk(cptr(lg), lg.scalar_type() == at::kBFloat16, static_cast<const float*>(cptr(bias)),
+    check(tpb_router_topk(cptr(lg), (lg.scalar_type() == at::kBFloat16 ? 1 : 0) + (bias16 ? 2 : 0), cptr(bias),
                           static_cast<float*>(mptr(w)), static_cast<int*>(mptr(idx)), static_cast<float*>(mptr(scores)), (int)t,
                           (int)e, (int)k, (int)mode, (int)n_group, (int)topk_group, norm_topk, (float)scale, stream()),
           "router_topk");

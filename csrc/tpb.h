@@ -155,7 +155,8 @@ int tpb_embedding_fwd_peer(void* const* shards, int world, long long shard_elems
 
 // Router: one warp per token.  mode 0 softmax-top-k(-renormalise); mode 1 sigmoid + bias with
 // group-limited selection.  w_out [T,K] fp32, idx_out [T,K] int32, scores_out [T,E] fp32 (optional).
-int tpb_router_topk(const void* logits, int logits_is_bf16, const float* bias, float* w_out, int* idx_out,
+// (bf16: bit 0, the logits are bf16 and not fp32; bit 1, the bias is.)
+int tpb_router_topk(const void* logits, int bf16, const void* bias, float* w_out, int* idx_out,
                     float* scores_out, int tokens, int E, int K, int mode, int n_group, int topk_group, int norm_topk,
                     float scale, void* stream);
 // out[r,:] = src_row[r] >= 0 ? row_scale[r] * x[src_row[r],:] : 0

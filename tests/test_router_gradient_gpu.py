@@ -106,3 +106,17 @@ def test_router_batched_gradients(cuda_lib, mode, norm):
     for i in range(3):
       (one,) = torch.autograd.grad(outs, lg, [g[i] for g in grads], retain_graph=True)
       assert torch.allclose(got[i], one, rtol=1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("E,K,groups", [(64, 6, 1), (256, 8, 8), (33, 3, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_router_takes_a_bf16_bias(cuda_lib, E, K, groups, dtype):
+  """As a model keeps it: the same choices and weights as with its fp32 copy, native and from Python."""
+  torch.manual_seed(E)
+  lg, bias = torch.randn(77, E, device="cuda").to(dtype), (0.3 * torch.randn(E, device="cuda")).bfloat16()
+  args = (K, 1, groups, max(1, groups // 2), True, 2.5)
+  want = moe._router_forward(lg, bias.float(), *args)
+  with torch.no_grad():
+    native = ops._native().router_topk(lg, bias, *args)
+  for got in (moe._router_forward(lg, bias, *args), native):
+    assert all(torch.equal(a, b) for a, b in zip(got, want))

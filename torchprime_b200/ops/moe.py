@@ -51,8 +51,11 @@ def _router_forward(lg, bias, k, mode, n_group, topk_group, norm_topk, scale):
   w = torch.empty(t, k, dtype=torch.float32, device=lg.device)
   idx = torch.empty(t, k, dtype=torch.int32, device=lg.device)
   scores = torch.empty(t, e, dtype=torch.float32, device=lg.device)
-  b = bias.float().contiguous() if bias is not None else None
-  check(lib().tpb_router_topk(ptr(lg), int(lg.dtype == torch.bfloat16), ptr(b), ptr(w), ptr(idx), ptr(scores), t, e,
+  b = None
+  if bias is not None:
+    b = (bias if bias.dtype == torch.bfloat16 else bias.float()).contiguous()
+  bf16 = int(lg.dtype == torch.bfloat16) + 2 * int(b is not None and b.dtype == torch.bfloat16)
+  check(lib().tpb_router_topk(ptr(lg), bf16, ptr(b), ptr(w), ptr(idx), ptr(scores), t, e,
                               k, mode, n_group, topk_group, int(norm_topk), float(scale), stream_ptr()),
         "router_topk")
   return w, idx, scores
