@@ -1070,10 +1070,9 @@ extern "C" int tpb_attn_fwd_softcap(const void* q, const void* k, const void* v,
   if (dv != 128 || (dqk != 128 && dqk != 192) || Hq % Hkv) return -2;
   if ((ldq % 8) || (ldk % 8) || (ldv % 8) || (ldo % 8)) return -2;
   if (B <= 0 || Sq <= 0 || Sk <= 0) return 0;
-  // TPB_ATTN_FWD_V2=1 selects the two-tile, 128-key-step kernel.  It is correct and 3-4 % ahead of the
-  // 64-key kernel at B=1, S=8192, 32/8 heads (0.565-0.571 against 0.590 ms on one box), no more: with
-  // its softmax threads doing nothing it still takes 0.513 ms, the time of its MMA stream and of the
-  // handshakes of the single issuing thread.  Earlier forms: one thread per row with 168 registers
+  // TPB_ATTN_FWD_V2=1 selects the two-tile, 128-key-step kernel.  It is correct and behind the 64-key kernel (B=1, S=8192, 32/8
+  // heads 502 us against 455; S=4096 152 against 132): its softmax threads are what the tensor core waits for, 570 of 1770 clocks a
+  // tile and step.  Earlier forms: one thread per row with 168 registers
   // spilled the 128 scores (0.66 ms); one softmax warpgroup serving both tiles (six warps, 210
   // registers) was slower still (1.04 ms), a single warp per scheduler cannot hide the TMEM and
   // MUFU latencies.

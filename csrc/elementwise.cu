@@ -822,6 +822,8 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 constexpr int NS_FWD_MIN_ROWS = 2048, NS_BWD_MIN_ROWS = 1024;
 static bool launch_rmsnorm_fwd_rows(const void* x, const void* w, void* y, float* rstd, int rows, int dim, float eps,
                                     cudaStream_t stream) {
+  static const bool disabled = []() { const char* v = getenv("TPB_RMSNORM_FWD_BULK"); return v && v[0] == '0'; }();
+  if (disabled) return false;
   const int nvec = dim / 8, row_bytes = dim * 2;
   if (!aligned16(x) || !aligned16(y) || !aligned16(w) || rows < NS_FWD_MIN_ROWS) return false;
   const int most = nvec <= 512 ? 16 : nvec <= 640 ? 12 : 8;
@@ -882,7 +884,8 @@ static bool launch_rmsnorm_bwd_rows(const void* dy, const void* x, const void* w
 
 // Rows that tpb_rmsnorm_bwd_dw needs behind the first one of its fp32 buffer.
 extern "C" int tpb_rmsnorm_bwd_parts(int rows, int dim) {
-  return dim % 8 || dim > 8 * NORM_THREADS * NORM_VPT || rows < NS_BWD_MIN_ROWS ? 0 : sm_count();
+  static const bool disabled = []() { const char* v = getenv("TPB_RMSNORM_BWD_BULK"); return v && v[0] == '0'; }();
+  return disabled || dim % 8 || dim > 8 * NORM_THREADS * NORM_VPT || rows < NS_BWD_MIN_ROWS ? 0 : sm_count();
 }
 
 extern "C" int tpb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres,
