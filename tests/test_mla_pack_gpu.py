@@ -25,6 +25,14 @@ def test_mla_pack(cuda_lib, b, s, heads, dn, dr, dv):
   assert bool(((drot.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1e-6 * heads * 4).all())
 
 
+# Heads that leave a group of four or a round of thirty-two partly filled, more vectors to a row than a warp has lanes, and
+# more tokens than one pass of the grid takes.
+@pytest.mark.parametrize("b,s,heads,dn,dr,dv", [(2, 9, 5, 264, 512, 8), (1, 17, 33, 8, 24, 272), (1, 3, 70, 16, 256, 16),
+                                                (1, 20001, 2, 8, 16, 8), (1, 524300, 1, 8, 8, 8)])
+def test_mla_pack_edges(cuda_lib, b, s, heads, dn, dr, dv):
+  test_mla_pack(cuda_lib, b, s, heads, dn, dr, dv)
+
+
 def test_latent_split(cuda_lib):
   x = torch.randn(2, 9, 48, device="cuda", dtype=torch.bfloat16, requires_grad=True)
   a, b = ops.latent_split(x, 32)
