@@ -869,6 +869,32 @@ py::object mla_pack(py::handle kv_, py::handle rot_, int64_t heads, int64_t dn, 
   return py::make_tuple(y[0], y[1]);
 }
 
+// The same written to where the caller keeps keys and values (batches any distance apart); false: nothing was written.
+bool mla_pack_into(py::handle kv_, py::handle rot_, int64_t heads, int64_t dn, int64_t dv, py::handle k_, py::handle v_) {
+  Tensor kv, rot, k, v;
+  if (!unobserved() || !unpack(kv_, kv) || !unpack(rot_, rot) || !unpack(k_, k) || !unpack(v_, v) || !plain_rows(kv) ||
+      !plain_rows(rot) || !plain(k) || !plain(v) || rot.dim() != 3 || kv.dim() != 3 || k.dim() != 4 || v.dim() != 4)
+    return false;
+  const int64_t b = rot.size(0), s = rot.size(1), dr = rot.size(2), dk = dn + dr;
+  const auto dense = [&](const Tensor& t, int64_t d) {
+    return t.sizes() == at::IntArrayRef({b, s, heads, d}) && t.stride(3) == 1 && t.stride(2) == d && t.stride(1) == heads * d &&
+           t.stride(0) % 8 == 0 && (b == 1 || t.stride(0) >= s * heads * d) && aligned(t) && t.device() == kv.device();
+  };
+  if (kv.size(0) != b || kv.size(1) != s || kv.size(2) != heads * (dn + dv) || dn % 8 || dv % 8 || dr % 8 || dr > 512 ||
+      b > 65535 || !aligned(kv) || !aligned(rot) || !dense(k, dk) || !dense(v, dv) ||
+      (at::GradMode::is_enabled() && (recording(kv) || recording(rot) || recording(k) || recording(v))))
+    return false;
+  {
+    py::gil_scoped_release nogil;
+    check(tpb_mla_pack_rows(cptr(kv), cptr(rot), dr, mptr(k), k.stride(0), mptr(v), v.stride(0), (int)b, s, (int)heads, (int)dn,
+                            (int)dr, (int)dv, stream()),
+          "mla_pack_into");
+    for (const Tensor& t : {k, v})
+      if (!t.is_inference()) t.unsafeGetTensorImpl()->bump_version();
+  }
+  return true;
+}
+
 // ------------------------------------------------------------------------------------------- without gradients only
 py::object embedding(py::handle ids_, py::handle table_) {
   Tensor ids, table, y;
@@ -1038,6 +1064,7 @@ PYBIND11_MODULE(_tpb_torch, m) {
   m.def("latent_split", &latent_split);
   m.def("latent_split_rope", &latent_split_rope);
   m.def("mla_pack", &mla_pack);
+  m.def("mla_pack_into", &mla_pack_into);
   m.def("embedding", &embedding);
   m.def("absorb_supported", &absorb_supported);
   m.def("absorb_step", &absorb_step);

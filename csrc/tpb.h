@@ -257,6 +257,8 @@ int tpb_grouped_gemm_skinny_bf16(const void* x, const void* w, const void* w2, v
 // ---- latent attention: k = [kv[:dn] | rot], v = kv[dn:] per head, and the gradients (mla_pack.cu)
 int tpb_mla_pack(const void* kv, const void* rot, long long rot_ld, void* k, void* v, long long tokens, int H, int dn,
                  int dr, int dv, void* stream);
+int tpb_mla_pack_rows(const void* kv, const void* rot, long long rot_ld, void* k, long long k_batch, void* v, long long v_batch,
+                      int batch, long long tokens, int H, int dn, int dr, int dv, void* stream);
 int tpb_mla_unpack(const void* dk, const void* dv_, void* dkv, void* drot, long long tokens, int H, int dn, int dr, int dv,
                    void* stream);
 

@@ -33,6 +33,20 @@ def test_mla_pack_edges(cuda_lib, b, s, heads, dn, dr, dv):
   test_mla_pack(cuda_lib, b, s, heads, dn, dr, dv)
 
 
+@pytest.mark.parametrize("b,s,at", [(1, 1, 0), (1, 130, 3), (3, 37, 5), (2, 8, 0)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_mla_pack_into_a_cache(cuda_lib, b, s, at, dtype):
+  heads, dn, dr, dv, room = 5, 24, 16, 40, 160
+  kv = torch.randn(b, s, heads * (dn + dv), device="cuda", dtype=torch.bfloat16)
+  rot = torch.randn(b, s, dr, device="cuda", dtype=torch.bfloat16)
+  kc = torch.full((b + 1, room, heads, dn + dr), 7.0, device="cuda", dtype=dtype)
+  vc = torch.full((b + 1, room, heads, dv), 7.0, device="cuda", dtype=dtype)
+  want_k, want_v = kc.clone(), vc.clone()
+  want_k[:b, at:at + s], want_v[:b, at:at + s] = ops.mla_pack(kv, rot, heads, dn, dv)
+  ops.mla_pack_into(kv, rot, heads, dn, dv, kc[:b, at:at + s], vc[:b, at:at + s])
+  assert torch.equal(kc, want_k) and torch.equal(vc, want_v)
+
+
 def test_latent_split(cuda_lib):
   x = torch.randn(2, 9, 48, device="cuda", dtype=torch.bfloat16, requires_grad=True)
   a, b = ops.latent_split(x, 32)

@@ -91,10 +91,15 @@ class DeepseekInferenceEngine:
       return scores.masked_fill(causal[None, :, None, :], float("-inf"))
 
     if self.attn_impl == "naive":
-      k, v = ops.mla_pack(ops.linear(latent, attn.kv_b_proj.weight), k_rot, h, dn, dv)
-      self.k_cache[li][:b, start:end] = k
-      self.v_cache[li][:b, start:end] = v
-      if start == 0 and x.is_cuda and s >= 128:
+      kv, k, v = ops.linear(latent, attn.kv_b_proj.weight), self.k_cache[li][:b, start:end], self.v_cache[li][:b, start:end]
+      prefill = start == 0 and x.is_cuda and s >= 128
+      if prefill and (b > 1 or self.dtype != x.dtype):     # the attention kernel takes rows of a batch back to back
+        k, v = ops.mla_pack(kv, k_rot, h, dn, dv)
+        self.k_cache[li][:b, start:end] = k
+        self.v_cache[li][:b, start:end] = v
+      else:
+        ops.mla_pack_into(kv, k_rot, h, dn, dv, k, v)
+      if prefill:
         o = ops.attention(q4, k, v, causal=True, scale=attn.scaling)
       else:
         kc, vc = self.k_cache[li][:b, :end], self.v_cache[li][:b, :end]

@@ -912,6 +912,14 @@ def mla_pack(kv, rot, heads, dn, dv):
   return k, kv[..., dn:].contiguous()
 
 
+def mla_pack_into(kv, rot, heads, dn, dv, k, v):
+  """:func:`mla_pack` of calls without a gradient, written to ``k`` [B,S,heads,dn+dr] and ``v`` [B,S,heads,dv], slices of a
+  cache: a pass over them less than a copy there, and two launches."""
+  if (nat := _native()) is None or not nat.mla_pack_into(kv, rot, heads, dn, dv, k, v):
+    for dst, src in zip((k, v), mla_pack(kv, rot, heads, dn, dv)):
+      dst.copy_(src)
+
+
 # --------------------------------------------------------------------------- lm head + CE
 class _LinearCrossEntropyFn(torch.autograd.Function):
   """Chunked lm_head + softmax cross entropy.  The forward pass also produces the
