@@ -331,6 +331,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   if (!chain_wait()) return;
   // K is on its way while the query tiles that can see it are found
   if (warp == 0) {
+    __syncwarp();   // thread 0's barriers, for whichever lane issues the copy (the others see them behind the list)
     one_lane([&] {
       tma_prefetch_desc(&tmQ); tma_prefetch_desc(&tmK); tma_prefetch_desc(&tmV); tma_prefetch_desc(&tmdO);
       mbar_expect_tx(k_full, TILE_BYTES);
