@@ -22,15 +22,16 @@
 //      Tensor stream per step j:  S(j+1), dQ(j), dP(j+1).
 //
 // Both kernels: warp 0 TMA producer, warp 1 MMA issuer, warps 2-9 compute.  Warps w and w+4
-// share a TMEM lane quarter and split the 128 score columns of a step; each writes its bf16
-// result over the first half of its OWN 64 input columns, so the two never touch each other's
+// share a TMEM lane quarter and take every other 32 of the 128 score columns of a step; each writes its bf16
+// result over the first half of its OWN 32 input columns, so the two never touch each other's
 // columns and the A operand of the following MMA is addressed per 16-column k-step.  That result is handed over in two
-// halves, so that its product starts while the second one is being made.
+// halves, columns 0..63 first, so that its product starts while the second one is being made and sums in their order.
 //
-// Bound by the products themselves and the cap on power: 2560 clocks of the dK/dV kernel's 128 x 128 step for 2048 of
-// MMAs and 1730 for 1536 in the dQ kernel, at 1.4 GHz.  What the dK/dV kernel waits for is its first phase (1240 clocks
-// between S^T and P^T).  One row of 8192 tokens, 32/8 heads, delta kernel included: 1410 us (1520 before the halves, the exchange of
-// Q's and dO's places and the list of visible tiles); of 4096 388 (417); two rows of 1999 tokens in segments 187 (220).
+// Bound by the products themselves and the cap on power: a 128 x 128 step's MMAs are 2048 clocks in the dK/dV kernel and 1536 in
+// the dQ kernel, at 1.4 GHz under the cap.  What the dK/dV kernel waits for is its first phase (1250 clocks
+// between S^T and P^T).  us through autograd, before the issuing warps stayed together, the halves, the exchange of Q's and dO's
+// places and the list of visible tiles / now: one row of 8192 tokens, 32/8 heads, 1710 to 1800 / 1430 to 1510, of 4096 505 / 473; two
+// rows of 1999 tokens 296 / 284, in segments 204 / 165 to 190.
 
 #include "common.cuh"
 #include "tpb.h"
@@ -207,19 +208,13 @@ __device__ __forceinline__ uint32_t pack_pair(f32x2 v) {
   f2_unpack(v, a, b);
   return pack_bf16(a, b);
 }
-// 2^-u as packed bf16, pair `c` of a row: every fourth pair on the FMA pipe.  A step's 128 x 128 exponentials take the MUFU 1024
-// clocks, half of what the step's MMAs take the tensor core, and stand in the chain between them.  (8192 tokens, 32/8 heads, us:
-// all on the MUFU 1451, every eighth 1421, every fourth 1410, three of eight 1420: the cap on power counts instructions too.)
-__device__ __forceinline__ uint32_t exp2_pair(int c, f32x2 u) {
+// 2^v as packed bf16.  A step's 128 x 128 exponentials take the MUFU 1024 clocks, half of what the step's MMAs take the tensor core,
+// and stand in the chain between them.  (A fourth of them as a polynomial on the FMA pipe gives 3 % of the backward of 8192 tokens,
+// but has 2^-126 where this has 0, makes infinity of a NaN and is ten times as far off.)
+__device__ __forceinline__ uint32_t exp2_pair(f32x2 v) {
   float a, b;
-  if ((c & 3) == 3) {
-    exp2_neg_pair(u, a, b);
-  } else {
-    f2_unpack(u, a, b);
-    a = ex2_approx(-a);
-    b = ex2_approx(-b);
-  }
-  return pack_bf16(a, b);
+  f2_unpack(v, a, b);
+  return pack_bf16(ex2_approx(a), ex2_approx(b));
 }
 
 // Operand tiles are [128 rows][128 d] in two 64-wide d blocks.  Descriptor low words (the high
@@ -231,8 +226,10 @@ __device__ __forceinline__ uint32_t mnmajor_lo(uint32_t tile) { return smem_desc
 __device__ __forceinline__ constexpr uint32_t kmajor_k(int k) { return (uint32_t)(((k >> 2) * (BWD_T * 128) + (k & 3) * 32) >> 4); }
 __device__ __forceinline__ constexpr uint32_t mnmajor_k(int k) { return (uint32_t)((k * 2048) >> 4); }
 // TMEM column (relative to the tile) where the bf16 A operand of k-step k lives: compute half
-// k >> 2 packed its 64 results into the first 32 columns of its own 64-column range.
+// k >> 2 packed its 64 results into the first 32 columns of its own 64-column range; or, a_col32, the one of every other
+// 32 columns its 32 results into the first 16 of them.
 __device__ __forceinline__ uint32_t a_col(int k) { return (uint32_t)((k >> 2) * 64 + (k & 3) * 8); }
+__device__ __forceinline__ uint32_t a_col32(int k) { return (uint32_t)((k >> 1) * 32 + (k & 1) * 8); }
 
 // The query tiles of QT rows that key block kb of batch row b can see, in order, kMasked set where scores need a mask; from
 // the positions (and segments) of each one's rows.  All threads of the block call; the caller synchronises behind it.
@@ -454,20 +451,20 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // Waits on the compute warps stay where the data is needed: hooking them into the previous
         // group would hold back that group's commit, which the compute warps are waiting for.
         // dV += P^T dO, first the k-steps whose P^T is there when the exponentials are half done
-        auto dv = [&](int k) { mma_ts_w(tmem_base + T_DV, tS + a_col(k), mDO + mnmajor_k(k), kDescHi, id_acc, (i | k) != 0); };
+        auto dv = [&](int k) { mma_ts_w(tmem_base + T_DV, tS + a_col32(k), mDO + mnmajor_k(k), kDescHi, id_acc, (i | k) != 0); };
         if (!wait_p(i, 0)) break;
         tc_fence_after();
-        one_lane([&] { dv(0); dv(1); dv(4); dv(5); });
+        one_lane([&] { dv(0); dv(1); dv(2); dv(3); });
         if (!wait_p(i, 1)) break;
         tc_fence_after();
-        ok = group([&](int k) { if (k == 2 || k == 3 || k >= 6) dv(k); },
+        ok = group([&](int k) { if (k >= 4) dv(k); },
                    [&] { return more ? wait_q(i + 1) : true; }, [&] { tc_commit(&do_empty[i & 1]); });
         if (!ok) break;
         if (more && !issue_s(i + 1, none)) break;
         if (!wait_ds(i)) break;
         tc_fence_after();
         // dK += dS^T Q
-        ok = group([&](int k) { mma_ts_w(tmem_base + T_DK, tDP + a_col(k), mQ + mnmajor_k(k), kDescHi, id_acc, (i | k) != 0); },
+        ok = group([&](int k) { mma_ts_w(tmem_base + T_DK, tDP + a_col32(k), mQ + mnmajor_k(k), kDescHi, id_acc, (i | k) != 0); },
                    [&] { return more ? wait_do(i + 1) : true; }, [&] { tc_commit(&q_empty[i & 1]); });
         if (!ok) break;
         if (more && !issue_dp(i + 1, none)) break;
@@ -477,15 +474,15 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
   } else {
     // ------------------------------------------------------------------ compute warps
     // Warp w may touch TMEM lanes 32*(w%4)..+31, so warps w and w+4 share a lane quarter (the
-    // same 32 key rows) and split the 128 query columns of a step between them.
+    // same 32 key rows) and split the 128 query columns of a step between them: half * 32 + (0..31) and 64 further on.
     const int qd = warp & 3;
-    const int half = (warp - 2) >> 2;             // which 64 of the 128 query columns
+    const int half = (warp - 2) >> 2;
     const int r_local = qd * 32 + lane;           // key row == TMEM lane
     const int kp = kv0 + r_local;                 // key position (keys are in natural order)
     const bool key_ok = kp < p.Sk;
     const int kseg = (p.kv_seg && key_ok) ? p.kv_seg[(long long)b * p.Sk + kp] : 0;
     const uint32_t tb = tmem_base + ((uint32_t)(qd * 32) << 16);
-    const uint32_t tS = tb + T_S + half * 64, tDP = tb + T_DP + half * 64;
+    const uint32_t tS = tb + T_S + half * 32, tDP = tb + T_DP + half * 32;
     const int win = p.window > 0 ? p.window : 0x7fffffff;   // keep needs qp - kp < win
     const int cmax = p.causal ? kp : -0x7fffffff;           // and qp >= cmax
     bool ok = true;
@@ -501,14 +498,14 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         // ---- phase 1: P^T = exp2(S^T * c - lse), kept packed for phase 2 and written over S^T
         if (!mbar_wait(s_full, step & 1, p.status, kTimeoutAccFull, 27)) { ok = false; break; }
         tc_fence_after();
-        uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;   // this half's 64 queries that may see the key
+        uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;   // of this half's queries those that may see the key
         if (need_mask) {
           if (p.q_pos) {
-            const int4* qp4 = reinterpret_cast<const int4*>(auxi + 2 * BWD_T + half * 64);
+            const int4* qp4 = reinterpret_cast<const int4*>(auxi + 2 * BWD_T + half * 32);
             keep0 = keep1 = 0;
 #pragma unroll 1
             for (int c4 = 0; c4 < 8; ++c4) {
-              const int4 a = qp4[c4], c = qp4[c4 + 8];
+              const int4 a = qp4[c4], c = qp4[c4 + 16];
               const int qa[4] = {a.x, a.y, a.z, a.w}, qc[4] = {c.x, c.y, c.z, c.w};
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
@@ -517,14 +514,14 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               }
             }
           } else {
-            const int at = t * BWD_T + pos_off + half * 64;   // position of the first one
+            const int at = t * BWD_T + pos_off + half * 32;   // position of the first one
             const int hi = kp - at + min(win, 0x40000000) - 1, lo = p.causal ? kp - at - 1 : -1;   // (kp - at < 2^30)
             keep0 = bits_upto(hi) & ~bits_upto(lo);
-            keep1 = bits_upto(hi - 32) & ~bits_upto(lo - 32);
+            keep1 = bits_upto(hi - 64) & ~bits_upto(lo - 64);
           }
           if (p.q_seg || p.kv_seg) {
-            const int* qs = auxi + 3 * BWD_T + half * 64;
-            same_segment_bits(p.q_seg ? qs[lane] : 0, p.q_seg ? qs[32 + lane] : 0, kseg, keep0, keep1);
+            const int* qs = auxi + 3 * BWD_T + half * 32;
+            same_segment_bits(p.q_seg ? qs[lane] : 0, p.q_seg ? qs[64 + lane] : 0, kseg, keep0, keep1);
           }
           if (!key_ok) keep0 = keep1 = 0;
         }
@@ -532,20 +529,19 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         uint32_t pk_f[SOFTCAP ? 32 : 1];   // 1 - tanh^2 of the capped scores (the derivative of the cap)
         uint32_t sreg[64];
         tmem_ld32(tS, sreg);
-        tmem_ld32(tS + 32, sreg + 32);
+        tmem_ld32(tS + 64, sreg + 32);
         tmem_wait_ld();
 #pragma unroll
         for (int ch = 0; ch < 2; ++ch) {
           const uint32_t* s = sreg + ch * 32;
-          const float4* lse4 = reinterpret_cast<const float4*>(aux + half * 64 + ch * 32);
+          const float4* lse4 = reinterpret_cast<const float4*>(aux + half * 32 + ch * 64);
           if (!need_mask && !SOFTCAP) {
-            const f32x2 nc2 = f2_pack(-p.scale_log2, -p.scale_log2);
+            const f32x2 c2 = f2_pack(p.scale_log2, p.scale_log2);
 #pragma unroll
             for (int c4 = 0; c4 < 8; ++c4) {
               const float4 L = lse4[c4];
-              pk_p[ch * 16 + 2 * c4] = exp2_pair(2 * c4, f2_fma(f2_pack_bits(s[4 * c4], s[4 * c4 + 1]), nc2, f2_pack(L.x, L.y)));
-              pk_p[ch * 16 + 2 * c4 + 1] =
-                  exp2_pair(2 * c4 + 1, f2_fma(f2_pack_bits(s[4 * c4 + 2], s[4 * c4 + 3]), nc2, f2_pack(L.z, L.w)));
+              pk_p[ch * 16 + 2 * c4] = exp2_pair(f2_fma(f2_pack_bits(s[4 * c4], s[4 * c4 + 1]), c2, f2_pack(-L.x, -L.y)));
+              pk_p[ch * 16 + 2 * c4 + 1] = exp2_pair(f2_fma(f2_pack_bits(s[4 * c4 + 2], s[4 * c4 + 3]), c2, f2_pack(-L.z, -L.w)));
             }
           } else if (!need_mask) {
 #pragma unroll
@@ -591,7 +587,7 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
               pk_p[ch * 16 + 2 * c4 + 1] = pack_bf16(pv[2], pv[3]);
             }
           }
-          tmem_st16(tS + ch * 16, pk_p + ch * 16);
+          tmem_st16(tS + ch * 64, pk_p + ch * 16);
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();
@@ -607,18 +603,19 @@ attn_bwd_dkv_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_consta
         {
           uint32_t dreg[64], pk_ds[32];
           tmem_ld32(tDP, dreg);
-          tmem_ld32(tDP + 32, dreg + 32);
+          tmem_ld32(tDP + 64, dreg + 32);
           tmem_wait_ld();
-          const float4* dlt4 = reinterpret_cast<const float4*>(aux + BWD_T + half * 64);
+          const float4* dlt4 = reinterpret_cast<const float4*>(aux + BWD_T + half * 32);
 #pragma unroll
           for (int c4 = 0; c4 < 16; ++c4) {
-            const float4 Dl = dlt4[c4];
+            const float4 Dl = dlt4[c4 + (c4 >> 3) * 8];
             pk_ds[2 * c4] = mul_bf16x2(pk_p[2 * c4], pack_pair(f2_sub(f2_pack_bits(dreg[4 * c4], dreg[4 * c4 + 1]), f2_pack(Dl.x, Dl.y))));
             pk_ds[2 * c4 + 1] =
                 mul_bf16x2(pk_p[2 * c4 + 1], pack_pair(f2_sub(f2_pack_bits(dreg[4 * c4 + 2], dreg[4 * c4 + 3]), f2_pack(Dl.z, Dl.w))));
           }
-          // all 64 inputs of this warp are in registers, so its first 32 columns can be overwritten
-          tmem_st32(tDP, pk_ds);
+          // all 64 inputs of this warp are in registers, so the first halves of its columns can be overwritten
+          tmem_st16(tDP, pk_ds);
+          tmem_st16(tDP + 64, pk_ds + 16);
         }
         tmem_wait_st();
         tc_fence_before();
@@ -810,14 +807,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
         const bool more = j + 1 < nblk;
         if (more && !issue_s(j + 1, none)) break;
         const uint32_t mK = mnmajor_lo(aK0 + (j % DQ_KSTAGES) * TILE_BYTES);
-        // dQ += dS K   (K tile [128 keys][128 d]: N = d contiguous), in the order in which dS gets there
-        auto dq = [&](int k) { mma_ts_w(tmem_base + T_DQ, tDP + a_col(k), mK + mnmajor_k(k), kDescHi, id_dq, (j | k) != 0); };
+        // dQ += dS K   (K tile [128 keys][128 d]: N = d contiguous)
+        auto dq = [&](int k) { mma_ts_w(tmem_base + T_DQ, tDP + a_col32(k), mK + mnmajor_k(k), kDescHi, id_dq, (j | k) != 0); };
         if (!wait_ds(j, 0)) break;   // not hooked into S(j+1): that would hold back its commit
         tc_fence_after();
-        one_lane([&] { dq(0); dq(1); dq(4); dq(5); });
+        one_lane([&] { dq(0); dq(1); dq(2); dq(3); });
         if (!wait_ds(j, 1)) break;
         tc_fence_after();
-        ok = group([&](int k) { if (k == 2 || k == 3 || k >= 6) dq(k); },
+        ok = group([&](int k) { if (k >= 4) dq(k); },
                    [&] { return more ? wait_v(j + 1) : true; }, [&] { tc_commit(&k_empty[j % DQ_KSTAGES]); });
         if (!ok) break;
         if (more && !issue_dp(j + 1, [&] { return j + 2 < nblk ? wait_k(j + 2) : true; })) break;
@@ -827,7 +824,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
   } else {
     // ------------------------------------------------------------------ compute warps
     const int qd = warp & 3;
-    const int half = (warp - 2) >> 2;             // which 64 of the 128 key columns
+    const int half = (warp - 2) >> 2;             // which key columns: half * 32 + (0..31) and 64 further on
     const int r_local = qd * 32 + lane;           // query row == TMEM lane
     const int row = q0 + r_local;
     const bool row_ok = row < p.Sq;
@@ -838,7 +835,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
     const float lse2 = p.lse2[li];
     const float delta = p.delta[li];
     const uint32_t tb = tmem_base + ((uint32_t)(qd * 32) << 16);
-    const uint32_t tDP = tb + T_DP + half * 64;
+    const uint32_t tDP = tb + T_DP + half * 32;
     const int* ks = p.kv_seg ? p.kv_seg + (long long)b * p.Sk : nullptr;
     const int kmin = p.window > 0 && qpos >= p.window ? qpos - p.window : -1;   // keep needs kmin < kp <= kmax
     const int kmax = p.causal ? min(max(qpos, -1), p.Sk - 1) : p.Sk - 1;
@@ -853,14 +850,14 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       }
       const bool need_mask = (p.causal && kv0 + BWD_T - 1 > qpos_min) || (kv0 + BWD_T > p.Sk) ||
                              (p.window > 0 && qpos_max - kv0 >= p.window) || seg_mask;
-      const uint32_t tS = tb + T_S + (j & 1) * BWD_T + half * 64;
-      uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;   // this half's 64 keys that the row may see
+      const uint32_t tS = tb + T_S + (j & 1) * BWD_T + half * 32;
+      uint32_t keep0 = 0xffffffffu, keep1 = 0xffffffffu;   // of this half's keys those that the row may see
       if (need_mask) {
-        const int k0 = kv0 + half * 64, hi = kmax - k0, lo = kmin - k0;
+        const int k0 = kv0 + half * 32, hi = kmax - k0, lo = kmin - k0;
         keep0 = bits_upto(hi) & ~bits_upto(lo);
-        keep1 = bits_upto(hi - 32) & ~bits_upto(lo - 32);
+        keep1 = bits_upto(hi - 64) & ~bits_upto(lo - 64);
         if (ks && (!SEG || seg_mask))
-          same_segment_bits(__ldg(ks + min(k0 + lane, p.Sk - 1)), __ldg(ks + min(k0 + 32 + lane, p.Sk - 1)), qseg, keep0, keep1);
+          same_segment_bits(__ldg(ks + min(k0 + lane, p.Sk - 1)), __ldg(ks + min(k0 + 64 + lane, p.Sk - 1)), qseg, keep0, keep1);
       }
       // ---- phase 1: P = exp2(S * c - lse), packed bf16 in registers
       if (!mbar_wait(&s_full[j & 1], (j >> 1) & 1, p.status, kTimeoutAccFull, 36)) { ok = false; break; }
@@ -868,16 +865,16 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       uint32_t pk_p[32];
       uint32_t sreg[64];
       tmem_ld32(tS, sreg);
-      tmem_ld32(tS + 32, sreg + 32);
+      tmem_ld32(tS + 64, sreg + 32);
       tmem_wait_ld();
 #pragma unroll
       for (int ch = 0; ch < 2; ++ch) {
         const uint32_t* s = sreg + ch * 32;
         if (!need_mask && !SOFTCAP) {
-          const f32x2 nc2 = f2_pack(-p.scale_log2, -p.scale_log2), l2 = f2_pack(lse2, lse2);
+          const f32x2 c2 = f2_pack(p.scale_log2, p.scale_log2), nl2 = f2_pack(-lse2, -lse2);
 #pragma unroll
           for (int c = 0; c < 16; ++c)
-            pk_p[ch * 16 + c] = exp2_pair(c, f2_fma(f2_pack_bits(s[2 * c], s[2 * c + 1]), nc2, l2));
+            pk_p[ch * 16 + c] = exp2_pair(f2_fma(f2_pack_bits(s[2 * c], s[2 * c + 1]), c2, nl2));
         } else if (!need_mask) {
 #pragma unroll
           for (int c = 0; c < 32; c += 2) {
@@ -916,7 +913,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
       {
         uint32_t dreg[64], pk[16];
         tmem_ld32(tDP, dreg);
-        tmem_ld32(tDP + 32, dreg + 32);
+        tmem_ld32(tDP + 64, dreg + 32);
         tmem_wait_ld();
         const f32x2 d2 = f2_pack(delta, delta);
 #pragma unroll
@@ -924,7 +921,7 @@ attn_bwd_dq_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constan
 #pragma unroll
           for (int c = 0; c < 16; ++c)
             pk[c] = mul_bf16x2(pk_p[ch * 16 + c], pack_pair(f2_sub(f2_pack_bits(dreg[32 * ch + 2 * c], dreg[32 * ch + 2 * c + 1]), d2)));
-          tmem_st16(tDP + ch * 16, pk);
+          tmem_st16(tDP + ch * 64, pk);
           tmem_wait_st();
           tc_fence_before();
           __syncwarp();

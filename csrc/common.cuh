@@ -585,38 +585,14 @@ __device__ __forceinline__ float ex2_approx(float x) {
   return y;
 }
 
-// 2^-u for a pair u >= 0 on the FMA pipe, beside the exponentials that the MUFU evaluates at a quarter of that rate:
-// -u = n + f with n the nearest integer (the 1.5 * 2^23 trick), a polynomial for 2^f on [-0.5, 0.5] fitted for the least
-// largest relative error (2.7e-6, where the bf16 that the result is rounded to has 3.9e-3) and an integer add of n to the
-// exponent.  u is cut at 126 (2^-126, not 0); of a NaN comes a value that bf16 has no finite number for.
-__device__ __forceinline__ void exp2_neg_pair(f32x2 u, float& r0, float& r1) {
-  float u0, u1;
-  f2_unpack(u, u0, u1);
-  asm("min.NaN.f32 %0, %0, 0f42FC0000;" : "+f"(u0));
-  asm("min.NaN.f32 %0, %0, 0f42FC0000;" : "+f"(u1));
-  u = f2_pack(u0, u1);
-  const f32x2 magic = f2_pack(12582912.f, 12582912.f);
-  const f32x2 fl = f2_sub(magic, u);
-  const f32x2 g = f2_add(f2_sub(fl, magic), u);          // -f
-  f32x2 pl = f2_fma(f2_pack(0.00957010034f, 0.00957010034f), g, f2_pack(-0.0559178591f, -0.0559178591f));
-  pl = f2_fma(pl, g, f2_pack(0.240247443f, 0.240247443f));
-  pl = f2_fma(pl, g, f2_pack(-0.693121791f, -0.693121791f));
-  pl = f2_fma(pl, g, f2_pack(0.999999285f, 0.999999285f));
-  float p0, p1, n0, n1;
-  f2_unpack(pl, p0, p1);
-  f2_unpack(fl, n0, n1);
-  r0 = __int_as_float(__float_as_int(p0) + (__float_as_int(n0) << 23));
-  r1 = __int_as_float(__float_as_int(p1) + (__float_as_int(n1) << 23));
-}
-
 // ----------------------------------------------------------------------------
 // Attention masks as bits: a thread that holds 64 scores of one row (or column) keeps the ones whose bit is set.
 // ----------------------------------------------------------------------------
 // Bits 0..n (none for n < 0, all for n >= 31).
 __device__ __forceinline__ uint32_t bits_upto(int n) { return n < 0 ? 0u : 0xffffffffu >> (31 - min(n, 31)); }
 
-// Clears the bits whose segment is not this lane's `seg`; id0 / id1: the ids behind bits lane and 32 + lane (the whole
-// warp calls).  The warp turns the 64 ids into one mask per segment among its lanes, usually one or two.  (An id load and
+// Clears the bits whose segment is not this lane's `seg`; id0 / id1: the ids behind bit `lane` of keep0 and of
+// keep1 (the whole warp calls).  The warp turns the 64 ids into one mask per segment among its lanes, usually one or two.  (An id load and
 // a compare per score: forward of two rows of 1999 tokens in seven segments, 32/8 heads, 184 us, this way 58.)
 __device__ __forceinline__ void same_segment_bits(int id0, int id1, int seg, uint32_t& keep0, uint32_t& keep1) {
   uint32_t left = 0xffffffffu;

@@ -212,3 +212,43 @@ def test_forward_of_rows_without_keys(cuda_lib, dqk):
   got = A.attention(q, k, v, causal=False, q_segment_ids=ids, kv_segment_ids=torch.zeros_like(ids))
   want = ref.attention(q.float(), k.float(), v.float(), causal=False, q_segment_ids=ids, kv_segment_ids=torch.zeros_like(ids))
   assert bool((got[:, ids[0] != 0] == 0).all()) and _rel(got[:, ids[0] == 0], want[:, ids[0] == 0]) < 2e-2
+
+
+def test_backward_is_the_same_with_and_without_a_mask(cuda_lib):
+  """Segment ids that are all one (256 keys: no table of ranges, so every tile is masked) change no bit of any gradient."""
+  from torchprime_b200.ops import attention_sm100 as A
+  q, k, v = _qkv(2, 256, 4, 2, 128, fused=False, seed=11)
+  q = (3 * q).to(torch.bfloat16)
+  do = torch.randn(2, 256, 4, 128, device="cuda", dtype=torch.bfloat16)
+  ids = torch.zeros(2, 256, device="cuda", dtype=torch.int32)
+  o, lse = A.attn_fwd(q, k, v, causal=False)
+  plain = A.attn_bwd(do, q, k, v, o, lse, causal=False)
+  masked = A.attn_bwd(do, q, k, v, o, lse, causal=False, q_seg=ids, kv_seg=ids)
+  assert all(torch.equal(a, b) for a, b in zip(plain, masked))
+
+
+def test_backward_nan_is_nan_everywhere_it_reaches(cuda_lib):
+  """Not an infinity, which a check for NaN lets through."""
+  from torchprime_b200.ops import attention_sm100 as A
+  q, k, v = _qkv(1, 640, 2, 1, 128, fused=False, seed=3)
+  q[0, 600, 0, 7] = float("nan")
+  do = torch.randn(1, 640, 2, 128, device="cuda", dtype=torch.bfloat16)
+  o, lse = A.attn_fwd(q, k, v, causal=True)
+  dq, dk, dv = A.attn_bwd(do, q, k, v, o, lse, causal=True)
+  assert torch.isnan(dv[0, :601]).all() and torch.isnan(dk[0, :601]).all() and torch.isnan(dq[0, 600, 0]).all()
+
+
+def test_backward_rows_behind_the_last_add_nothing(cuda_lib):
+  """A last tile of two queries holds the next sequence's gradients in its other rows; their probability is 0, whatever
+  stands there (2^-126 of 1e37 would be seen)."""
+  from torchprime_b200.ops import attention_sm100 as A
+  q, _, _ = _qkv(2, 130, 2, 1, 128, fused=False, seed=5)
+  _, k, v = _qkv(2, 128, 2, 1, 128, fused=False, seed=6)
+  v = (1e-3 * v).to(torch.bfloat16)
+  do = torch.randn(2, 130, 2, 128, device="cuda").to(torch.bfloat16)
+  do[1] = 1e37
+  o, lse = A.attn_fwd(q, k, v, causal=False)
+  both = A.attn_bwd(do, q, k, v, o, lse, causal=False)
+  o, lse = A.attn_fwd(q[:1], k[:1], v[:1], causal=False)
+  one = A.attn_bwd(do[:1], q[:1], k[:1], v[:1], o, lse, causal=False)
+  assert all(torch.equal(a[:1], b) for a, b in zip(both, one))
