@@ -344,8 +344,10 @@ __device__ __forceinline__ uint32_t cluster_ctarank() {
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
-// The same where nothing written in front of it has to be seen behind it: the CTAs of a cluster have all got here, so none of
-// them reads another's shared memory any more.  (The release above waits until a thread's results have reached memory.)
+// The same where nothing written in front of it has to be seen behind it: the CTAs of a cluster have all got here.  It says
+// nothing of what is still under way from one of them to another, whose shared memory may be the next block's by then.  So
+// every load of a neighbour's memory feeds a store or a sum that is made in front of this, and the owner of a barrier that
+// neighbours arrive on has waited for the last of them.  (The release above waits until a thread's results have reached memory.)
 __device__ __forceinline__ void cluster_leave() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
@@ -360,7 +362,7 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
 }
 // The same for a barrier that only says when: no write of this thread has to be seen behind it (tensor memory that has been
 // read, with tc_fence_before in front).  A release to the whole cluster waits until all of the thread's writes are out, 1500 to
-// 2200 clocks while the memory is busy.
+// 2200 clocks while the memory is busy.  The barrier's owner waits for every one of them before it leaves.
 __device__ __forceinline__ void mbar_arrive_remote(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }

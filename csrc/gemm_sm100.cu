@@ -524,6 +524,18 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
       }
+      if (PAIR && ok) {
+        // The other CTA of the pair signals these barriers, the other pair ring_free: the last signals, which no further
+        // tile waits for, have arrived before this CTA leaves and its shared memory is another's.
+        for (int s = 0; s < NST && ok; ++s) {
+          ok = mbar_wait(&empty[stage], phase ^ 1, p.status, kTimeoutStageFree, 1);
+          if (++stage == NST) {
+            stage = 0;
+            phase ^= 1;
+          }
+        }
+        if (KSPLIT && ok && cta < num_tiles) mbar_wait_cluster(ring_free, tiles_done & 1, p.status, kTimeoutStageFree, 9);
+      }
     }
   } else if (warp == 1) {
     // -------------------------------------------------------------- MMA issuer
@@ -542,7 +554,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
         const int acc = local & 1;
         const uint32_t acc_phase = (local >> 1) & 1;
         ++local;
-        if (!mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, p.status, kTimeoutAccFree, 2)) break;
+        if (!mbar_wait_warp(&acc_empty[acc], acc_phase ^ 1, p.status, kTimeoutAccFree, 2)) { ok = false; break; }
         tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * BN;
         // The MMA queue is shallow: whatever this thread does between two MMAs is tensor idle
@@ -593,6 +605,13 @@ gemm_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUt
           }
         }
         if (ok) one_lane([&] { if (PAIR) tc_commit_pair(&acc_full[acc], lead); else tc_commit(&acc_full[acc]); });
+      }
+      if (PAIR && ok) {   // the same for the last accumulator of each buffer, handed back by both CTAs
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+          const int used = (local + 1 - a) >> 1;
+          if (used > 0 && !mbar_wait_warp(&acc_empty[a], (used - 1) & 1, p.status, kTimeoutAccFree, 2)) break;
+        }
       }
     }
   } else {

@@ -18,3 +18,26 @@ def test_barriers_are_initialised_before_another_lane_uses_them(name):
       used = re.search(r"\bone_lane\(|\belect_one\(", body[at:])
       if used:
         assert BLOCK_SYNC.search(body[at:at + used.start()]), f"{kernel} uses its barriers before they are seen"
+
+
+def _without_loops(body, head):
+  """``body`` without the loops that begin with ``head``."""
+  while (start := body.find(head)) >= 0:
+    at, depth = body.index("{", body.index(")", start)), 0
+    while True:
+      depth += {"{": 1, "}": -1}.get(body[at], 0)
+      at += 1
+      if not depth:
+        break
+    body = body[:start] + body[at:]
+  return body
+
+
+@pytest.mark.parametrize("barrier", ["acc_empty", "empty", "ring_free"])
+def test_a_pair_waits_for_the_last_signals_of_its_neighbours(barrier):
+  """In the tile loop these barriers are waited for ahead of a reuse; the signals after the last one have a wait of their own,
+  so that none reaches shared memory whose CTA has left."""
+  body = _kernels(_source("gemm_sm100.cu"))["gemm_kernel"]
+  assert "cluster_leave()" in body
+  rest = _without_loops(body, "for (int t = cta;")
+  assert re.search(r"mbar_wait(?:_warp|_cluster)?\(&?%s\b" % barrier, rest), f"nobody waits for the last arrival on {barrier}"
