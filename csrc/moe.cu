@@ -696,14 +696,17 @@ logit_dw_kernel(const float* __restrict__ dy, const __nv_bfloat16* __restrict__ 
   cluster_sync_all();
   // this CTA's eight of the 64 rows, two columns to a thread
   const int n = rank * (RG_TILE / RG_SPLIT) + (int)threadIdx.x / (RG_TILE / 2), c = (int)threadIdx.x % (RG_TILE / 2) * 2;
-  float s0 = 0.f, s1 = 0.f;
+  if (n0 + n < N && c0 + c < K) {   // (around the loads too: one whose result is not stored could still be under way at the end)
+    float s0 = 0.f, s1 = 0.f;
 #pragma unroll
-  for (int r = 0; r < RG_SPLIT; ++r) {
-    float a, b;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(map_to_cta(smem_u32(&part[n][c]), r)) : "memory");
-    s0 += a; s1 += b;
+    for (int r = 0; r < RG_SPLIT; ++r) {
+      float a, b;
+      asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(a), "=f"(b) : "r"(map_to_cta(smem_u32(&part[n][c]), r)) : "memory");
+      s0 += a; s1 += b;
+    }
+    *reinterpret_cast<uint32_t*>(dw + (size_t)(n0 + n) * K + c0 + c) = pack_bf16(s0, s1);
   }
-  if (n0 + n < N && c0 + c < K) *reinterpret_cast<uint32_t*>(dw + (size_t)(n0 + n) * K + c0 + c) = pack_bf16(s0, s1);
+  __syncwarp();
   cluster_leave();           // nobody's shared memory goes away while a neighbour reads it
 }
 

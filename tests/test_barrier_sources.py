@@ -41,3 +41,10 @@ def test_a_pair_waits_for_the_last_signals_of_its_neighbours(barrier):
   assert "cluster_leave()" in body
   rest = _without_loops(body, "for (int t = cta;")
   assert re.search(r"mbar_wait(?:_warp|_cluster)?\(&?%s\b" % barrier, rest), f"nobody waits for the last arrival on {barrier}"
+
+
+def test_loads_of_a_neighbours_memory_feed_a_store():
+  """Threads without a result load nothing: nothing would wait for such a load before the neighbour leaves."""
+  body = _kernels(_source("moe.cu"))["logit_dw_kernel"]
+  tail = body[body.rindex("cluster_sync_all()"):]
+  assert 0 < tail.find("if (n0 + n < N && c0 + c < K) {") < tail.index("ld.shared::cluster")
