@@ -278,7 +278,7 @@ rmsnorm_bwd_rows_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ 
   if (!chain_begin()) return;
   extern __shared__ uint8_t nb_smem_raw[];
   uint8_t* smem = nb_smem_raw + ((128u - (smem_u32(nb_smem_raw) & 127u)) & 127u);
-  __shared__ float red[GROUPS][2][4];
+  __shared__ __align__(16) float red[GROUPS][2][4];
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int grp = warp / 4, tid = threadIdx.x % NB_GROUP;
   const uint32_t row_bytes = (uint32_t)nvec * 16u;

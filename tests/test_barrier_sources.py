@@ -48,3 +48,13 @@ def test_loads_of_a_neighbours_memory_feed_a_store():
   body = _kernels(_source("moe.cu"))["logit_dw_kernel"]
   tail = body[body.rindex("cluster_sync_all()"):]
   assert 0 < tail.find("if (n0 + n < N && c0 + c < K) {") < tail.index("ld.shared::cluster")
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_shared_arrays_read_as_vectors_are_aligned_for_them(name):
+  """A __shared__ array has its element's alignment unless it says more."""
+  for kernel, body in _kernels(_source(name)).items():
+    for decl in re.finditer(r"__shared__ ((?:__align__\(\d+\) )?)(float|int|__nv_bfloat16|unsigned|uint8_t) (\w+)\[", body):
+      if not decl.group(1):
+        as_vector = re.search(r"reinterpret_cast<(?:const )?(?:float|int|uint|double)[24]\*>\(&?%s\b" % decl.group(3), body)
+        assert as_vector is None, f"{kernel}: {decl.group(3)} is read as {as_vector.group()}"
