@@ -598,7 +598,7 @@ logit_dx_kernel(const float* __restrict__ dy, const __nv_bfloat16* __restrict__ 
   if (!chain_begin()) return;
   __shared__ __align__(16) float sdy[RG_ROWS][RG_STEP + 4];
   __shared__ __align__(16) __nv_bfloat16 sw[RG_STEP][RG_COLS];
-  const int t0 = blockIdx.y * RG_ROWS, c0 = blockIdx.x * RG_COLS;
+  const int t0 = blockIdx.x * RG_ROWS, c0 = blockIdx.y * RG_COLS;   // (only a grid's first dimension holds any number of rows)
   const int lane = threadIdx.x & 31, r0 = (threadIdx.x >> 5) * 8;
   float acc[8][4] = {};
   for (int n0 = 0; n0 < N; n0 += RG_STEP) {
@@ -718,12 +718,12 @@ using namespace tpb;
 extern "C" int tpb_linear_f32_bwd(const float* dy, const void* x, const void* w, void* dx, void* dw, int T, int N, int K,
                                   long long ldx, long long ldw, void* stream) {
   if (T <= 0 || N <= 0 || K <= 0) return -2;
-  if (K % 8 || ldx % 8 || ldw % 8 || (T + RG_ROWS - 1) / RG_ROWS > 65535 || (N + RG_TILE - 1) / RG_TILE > 65535) return -2;
+  if (K % 8 || ldx % 8 || ldw % 8 || (K + RG_COLS - 1) / RG_COLS > 65535 || (N + RG_TILE - 1) / RG_TILE > 65535) return -2;
   for (const void* p : {x, w, (const void*)dx, (const void*)dw})
     if (reinterpret_cast<uintptr_t>(p) % 16) return -2;
   cudaStream_t s = reinterpret_cast<cudaStream_t>(stream);
   if (dx)
-    chain(logit_dx_kernel, dim3((K + RG_COLS - 1) / RG_COLS, (T + RG_ROWS - 1) / RG_ROWS), RG_THREADS, 0, s, dy,
+    chain(logit_dx_kernel, dim3((T + RG_ROWS - 1) / RG_ROWS, (K + RG_COLS - 1) / RG_COLS), RG_THREADS, 0, s, dy,
           (const __nv_bfloat16*)w, (__nv_bfloat16*)dx, T, N, K, ldw);
   if (dw)
     chain_clusters(logit_dw_kernel, RG_SPLIT, dim3(RG_SPLIT * ((K + RG_TILE - 1) / RG_TILE), (N + RG_TILE - 1) / RG_TILE), RG_THREADS, 0,

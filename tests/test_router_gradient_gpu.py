@@ -120,3 +120,17 @@ def test_router_takes_a_bf16_bias(cuda_lib, E, K, groups, dtype):
     native = ops._native().router_topk(lg, bias, *args)
   for got in (moe._router_forward(lg, bias, *args), native):
     assert all(torch.equal(a, b) for a, b in zip(got, want))
+
+
+def test_linear_f32_gradients_of_very_many_rows(cuda_lib):
+  """One row more than a grid's second dimension has blocks of 64."""
+  t, n, kk = 64 * 65535 + 1, 48, 8
+  x = torch.randn(t, kk, device="cuda").bfloat16().requires_grad_(True)
+  w = torch.randn(n, kk, device="cuda").bfloat16().requires_grad_(True)
+  dy = torch.randn(1, n, device="cuda").expand(t, n)
+  dx, dw = torch.autograd.grad(ops.linear_f32(x, w), (x, w), dy)
+  one = (dy[:1].double() @ w.detach().double())
+  assert bool(((dx.double() - one).abs() <= 2 ** -8 * one.abs() + 1e-5).all())
+  want = dy[0].double()[:, None] * x.detach().double().sum(0)
+  size = dy[0].double().abs()[:, None] * x.detach().double().abs().sum(0)
+  assert bool(((dw.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6 * size).all())
