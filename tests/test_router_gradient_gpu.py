@@ -134,3 +134,26 @@ def test_linear_f32_gradients_of_very_many_rows(cuda_lib):
   want = dy[0].double()[:, None] * x.detach().double().sum(0)
   size = dy[0].double().abs()[:, None] * x.detach().double().abs().sum(0)
   assert bool(((dw.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6 * size).all())
+
+
+@pytest.mark.parametrize("give_back", ["columns first", "elsewhere", "unaligned", "wider"])
+def test_linear_f32_gradients_with_saved_tensor_hooks(cuda_lib, give_back):
+  """Hooks may give saved tensors back in another layout, alignment or type; torch's operators take them as they are."""
+  torch.manual_seed(1)
+  x = torch.randn(300, 64, device="cuda").bfloat16().requires_grad_(True)
+  w = torch.randn(16, 64, device="cuda").bfloat16().requires_grad_(True)
+  dy = torch.randn(300, 16, device="cuda")
+
+  def back(t):
+    if give_back == "columns first":
+      return t.t().contiguous().t()
+    if give_back == "unaligned":
+      return torch.cat([t.flatten()[:1], t.flatten()])[1:].view(t.shape)
+    return t.float() if give_back == "wider" else t.clone()
+
+  with torch.autograd.graph.saved_tensors_hooks(lambda t: t, back):
+    y = ops.linear_f32(x, w)
+    dx, dw = torch.autograd.grad(y, (x, w), dy)
+  for got, a, b in ((dx, dy.double(), w.detach().double()), (dw, dy.double().t(), x.detach().double())):
+    want, size = a @ b, a.abs() @ b.abs()
+    assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6 * size).all())

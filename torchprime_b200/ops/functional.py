@@ -344,9 +344,11 @@ class _LinearF32Fn(torch.autograd.Function):
   @staticmethod
   def backward(ctx, dy):
     x, w = ctx.saved_tensors
-    # a router's sizes; a gradient that is recorded itself, or several at once, takes torch's operators
+    # a router's sizes; a gradient that is recorded itself, or several at once, takes torch's operators, and so do tensors that
+    # saved-tensor hooks gave back in another layout or place
     if (x.shape[0] >= 256 and w.shape[0] <= 512 and dy.dtype == torch.float32 and not torch.is_grad_enabled()
-        and not batched(dy)):
+        and not batched(dy) and use_kernels(x, w) and _gemm_friendly(x, [w]) and x.data_ptr() % 16 == 0
+        and w.data_ptr() % 16 == 0):
       from . import kernels as k
       return k.linear_f32_bwd(dy.contiguous(), x, w, *ctx.needs_input_grad)
     dx = (dy @ w.float()).to(x.dtype) if ctx.needs_input_grad[0] else None
