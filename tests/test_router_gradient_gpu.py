@@ -157,3 +157,30 @@ def test_linear_f32_gradients_with_saved_tensor_hooks(cuda_lib, give_back):
   for got, a, b in ((dx, dy.double(), w.detach().double()), (dw, dy.double().t(), x.detach().double())):
     want, size = a @ b, a.abs() @ b.abs()
     assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6 * size).all())
+
+
+@pytest.mark.parametrize("T,N,K,dx_kernel,dw_kernel", [
+  (255, 64, 2048, False, False), (256, 64, 2048, True, True), (4096, 64, 2048, True, True), (4096, 8, 512, True, True),
+  (4097, 8, 512, False, False), (5000, 16, 1024, False, False), (8192, 24, 512, True, True), (8200, 32, 2048, False, False),
+  (9000, 40, 1024, True, False), (9000, 48, 2048, True, True), (256, 128, 4096, True, False), (260, 128, 4096, False, False),
+  (1500, 128, 2048, False, True), (4097, 160, 512, False, False), (700, 256, 1024, False, True), (700, 256, 2048, False, False),
+  (300, 512, 512, False, False)])
+def test_logit_gradients_by_rule(cuda_lib, monkeypatch, T, N, K, dx_kernel, dw_kernel):
+  """Each gradient comes from the kernel where that is the faster one, and is the same operators' bits as ever elsewhere."""
+  from torchprime_b200.ops import kernels as k
+  torch.manual_seed(T)
+  asked = [False, False]
+  kernel = k.linear_f32_bwd
+  monkeypatch.setattr(k, "linear_f32_bwd", lambda dy, x, w, a=True, b=True: (asked.__setitem__(slice(None), [a, b]), kernel(dy, x, w, a, b))[1])
+  x = torch.randn(T, K, device="cuda").bfloat16().requires_grad_(True)
+  w = torch.randn(N, K, device="cuda").bfloat16().requires_grad_(True)
+  dy = torch.randn(T, N, device="cuda")
+  dx, dw = torch.autograd.grad(ops.linear_f32(x, w), (x, w), dy)
+  assert asked == [dx_kernel, dw_kernel]
+  for got, by_kernel, a, b, lib in ((dx, dx_kernel, dy.double(), w.detach().double(), (dy @ w.float()).to(torch.bfloat16)),
+                                    (dw, dw_kernel, dy.double().t(), x.detach().double(), (dy.t() @ x.float()).to(torch.bfloat16))):
+    want, size = a @ b, a.abs() @ b.abs()
+    assert bool(((got.double() - want).abs() <= 2 ** -8 * want.abs() + 1e-6 * size).all())
+    assert by_kernel or torch.equal(got, lib)
+  (only,) = torch.autograd.grad(ops.linear_f32(x, w.detach()), x, dy)
+  assert torch.equal(only, dx)

@@ -334,6 +334,27 @@ def linear_pair(x, w1, w2):
   return linear(x, w1), linear(x, w2)
 
 
+def logit_kernels_pay(t, n, k):
+  """Whether the kernels for the input's and for the weight's gradient of fp32 logits (t rows, n logits, k columns) beat torch's
+  fp32 products and their conversions.  They save copies and launches; per multiply-add the library is up to 1.5 times as
+  fast, and they make 64 logits at least.  us, kernel / torch, input gradient and weight gradient:
+  64 x 2048: 256 rows 8 / 15, 7 / 17; 4096 34 / 45, 54 / 86; 65536 485 / 551, 782 / 787     64 x 512: 65536 126 / 153, 328 / 258
+  8 x 2048: 700 rows 13 / 17, 12 / 25; 4096 32 / 28, 52 / 84; 16384 121 / 78, 195 / 265     8 x 512: 8192 20 / 21, 43 / 39
+  32 x 2048: 4096 rows 33 / 35, 53 / 65; 8192 63 / 58, 100 / 117; 16384 122 / 108, 196 / 183
+  128 x 512: 1500 rows 17 / 19, 17 / 39     128 x 2048: 4096 rows 64 / 67, 91 / 102; 16384 242 / 222, 341 / 296
+  72 x 2048: 1500 rows 28 / 29, 37 / 42; 4096 63 / 50, 90 / 101; 8192 121 / 87, 174 / 168     72 x 7168: 700 rows 45 / 40, 53 / 47
+  256 x 512: 700 rows 24 / 20, 14 / 23; 4096 53 / 35, 54 / 78     256 x 2048: 700 rows 49 / 32, 35 / 33; 4096 123 / 110, 152 / 126
+  256 x 7168: 4096 rows 419 / 337, 463 / 397"""
+  if t < 256:
+    return False, False
+  dx = (n > 40 or t * k <= n << 18) if n <= 64 else n <= 128 and t * k <= 1 << 20
+  if n <= 64:
+    dw = t <= 4096 or (n > 16 and t <= 8192) or (n >= 40 and k >= 2048)
+  else:
+    dw = t <= 4096 and (k <= 2048 if n <= 192 else n <= 256 and k <= 1024)
+  return dx, dw
+
+
 class _LinearF32Fn(torch.autograd.Function):
   @staticmethod
   def forward(ctx, x, w):
@@ -346,13 +367,18 @@ class _LinearF32Fn(torch.autograd.Function):
     x, w = ctx.saved_tensors
     # a router's sizes; a gradient that is recorded itself, or several at once, takes torch's operators, and so do tensors that
     # saved-tensor hooks gave back in another layout or place
-    if (x.shape[0] >= 256 and w.shape[0] <= 512 and dy.dtype == torch.float32 and not torch.is_grad_enabled()
-        and not batched(dy) and use_kernels(x, w) and _gemm_friendly(x, [w]) and x.data_ptr() % 16 == 0
-        and w.data_ptr() % 16 == 0):
+    want_dx, want_dw = ctx.needs_input_grad
+    dx = dw = None
+    if (dy.dtype == torch.float32 and not torch.is_grad_enabled() and not batched(dy) and use_kernels(x, w)
+        and _gemm_friendly(x, [w]) and x.data_ptr() % 16 == 0 and w.data_ptr() % 16 == 0):
       from . import kernels as k
-      return k.linear_f32_bwd(dy.contiguous(), x, w, *ctx.needs_input_grad)
-    dx = (dy @ w.float()).to(x.dtype) if ctx.needs_input_grad[0] else None
-    dw = (dy.t() @ x.float()).to(w.dtype) if ctx.needs_input_grad[1] else None
+      pay_dx, pay_dw = logit_kernels_pay(x.shape[0], *w.shape)
+      if (want_dx and pay_dx) or (want_dw and pay_dw):
+        dx, dw = k.linear_f32_bwd(dy.contiguous(), x, w, want_dx and pay_dx, want_dw and pay_dw)
+    if want_dx and dx is None:
+      dx = (dy @ w.float()).to(x.dtype)
+    if want_dw and dw is None:
+      dw = (dy.t() @ x.float()).to(w.dtype)
     return dx, dw
 
 
