@@ -540,10 +540,13 @@ using namespace tpb;
 
 // y1 = x w1^T and y2 = x w2^T, x [T,K], all rows back to back, in one launch (a decode step's query and latent projections: six of
 // its microseconds are a second launch).  -2 where one of the two is not this kernel's by the rules above.
+extern "C" int tpb_linear_pair_pays(int T, int N1, int N2, int K) {
+  return T > 0 && N1 > 0 && N2 > 0 && K > 0 && K % 8 == 0 && N1 % 8 == 0 && N2 % 8 == 0 && skinny_wins(T, N1, K, false) &&
+         skinny_wins(T, N2, K, false);
+}
 extern "C" int tpb_linear_pair_bf16(const void* x, const void* w1, const void* w2, void* y1, void* y2, int T, int N1, int N2, int K,
                                     void* stream) {
-  if (T <= 0 || N1 <= 0 || N2 <= 0 || K <= 0) return -2;
-  if (K % 8 || N1 % 8 || N2 % 8 || !skinny_wins(T, N1, K, false) || !skinny_wins(T, N2, K, false)) return -2;
+  if (!tpb_linear_pair_pays(T, N1, N2, K)) return -2;
   for (const void* q : {x, w1, w2, (const void*)y1, (const void*)y2})
     if (reinterpret_cast<uintptr_t>(q) % 16) return -2;
   SkinnyParams p = {};

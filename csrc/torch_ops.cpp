@@ -265,8 +265,8 @@ py::object linear_pair(py::handle x_, py::handle w1_, py::handle w2_) {
     return py::none();
   const int64_t k = w1.k, rows = x.numel() / x.size(-1);
   if (x.size(-1) != k || w2.k != k || !small(rows) || !small(w1.rows) || !small(w2.rows) || x.get_device() != w1.t[0].get_device() ||
-      x.get_device() != w2.t[0].get_device())
-    return py::none();
+      x.get_device() != w2.t[0].get_device() || !tpb_linear_pair_pays((int)rows, (int)w1.rows, (int)w2.rows, (int)k))
+    return py::none();       // (ahead of the results' allocation: a prefill comes here once a layer)
   Tensor y1, y2;
   int rc;
   {

@@ -244,7 +244,8 @@ int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, const float* co
 int tpb_linear_f32_bwd(const float* dy, const void* x, const void* w, void* dx, void* dw, int T, int N, int K, long long ldx,
                        long long ldw, void* stream);
 
-// y1 = x w1^T and y2 = x w2^T in one launch; -2 where one of them is not the few-rows kernel's.
+// y1 = x w1^T and y2 = x w2^T in one launch; -2 where one of them is not the few-rows kernel's (which _pays says beforehand).
+int tpb_linear_pair_pays(int T, int N1, int N2, int K);
 int tpb_linear_pair_bf16(const void* x, const void* w1, const void* w2, void* y1, void* y2, int T, int N1, int N2, int K,
                          void* stream);
 

@@ -336,3 +336,14 @@ def test_two_products_refuse_what_one_launch_cannot_do(cuda_lib):
   w1.requires_grad_(True)
   y1, y2 = ops.linear_pair(x, w1, w2)
   assert y1.requires_grad and not y2.requires_grad
+
+
+@pytest.mark.parametrize("rows", [200, 900])
+def test_two_products_allocate_nothing_where_they_do_not_run(cuda_lib, rows):
+  from torchprime_b200.ops import functional as ops
+  x = torch.randn(rows, 1024, device="cuda", dtype=torch.bfloat16)
+  w1, w2 = (torch.randn(n, 1024, device="cuda", dtype=torch.bfloat16) for n in (3072, 576))
+  before = torch.cuda.memory_stats()["allocation.all.allocated"]
+  with torch.no_grad():
+    assert ops._native().linear_pair(x, w1, w2) is None
+  assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
