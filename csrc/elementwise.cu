@@ -882,7 +882,7 @@ static bool launch_rmsnorm_bwd_rows(const void* dy, const void* x, const void* w
   return true;
 }
 
-// Rows that tpb_rmsnorm_bwd_dw needs behind the first one of its fp32 buffer.
+// Rows of scratch that tpb_rmsnorm_bwd_dw takes.
 extern "C" int tpb_rmsnorm_bwd_parts(int rows, int dim) {
   static const bool disabled = []() { const char* v = getenv("TPB_RMSNORM_BWD_BULK"); return v && v[0] == '0'; }();
   return disabled || dim % 8 || dim > 8 * NORM_THREADS * NORM_VPT || rows < NS_BWD_MIN_ROWS ? 0 : sm_count();
@@ -1008,16 +1008,15 @@ extern "C" int tpb_scale_cast_bf16(const float* src, void* dst, long long n, con
   return rc(cudaGetLastError());
 }
 
-// tpb_rmsnorm_bwd with the weight gradient written instead of added to: dw_f32 is [1 + tpb_rmsnorm_bwd_parts(rows, dim)][dim],
-// its first row the result and the others scratch; with dw_bf16 also delivered in bf16.
+// tpb_rmsnorm_bwd with the weight gradient written to dw_f32 instead of added to; with dw_bf16 also delivered in bf16.
 extern "C" int tpb_rmsnorm_bwd_dw(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
-                                  float* dw_f32, void* dw_bf16, int rows, int dim, void* stream) {
-  const int parts = tpb_rmsnorm_bwd_parts(rows, dim);
-  if (parts > 0 && aligned16(dy) && aligned16(x) && aligned16(w) && aligned16(dx) && aligned16(dres) && aligned16(dw_f32) &&
-      reinterpret_cast<uintptr_t>(dw_bf16) % 8 == 0 &&
-      launch_rmsnorm_bwd_rows(dy, x, w, rstd, dres, dx, dw_f32 + dim, rows, dim, STREAM(stream))) {
-    chain(norm_dw_kernel, (dim / 4 + 15) / 16, 256, 0, STREAM(stream), (const float4*)(dw_f32 + dim), (float4*)dw_f32,
-          (uint2*)dw_bf16, parts, dim / 4);
+                                  float* dw_f32, void* dw_bf16, float* parts, int rows, int dim, void* stream) {
+  const int n = parts ? tpb_rmsnorm_bwd_parts(rows, dim) : 0;
+  if (n > 0 && aligned16(dy) && aligned16(x) && aligned16(w) && aligned16(dx) && aligned16(dres) && aligned16(dw_f32) &&
+      aligned16(parts) && reinterpret_cast<uintptr_t>(dw_bf16) % 8 == 0 &&
+      launch_rmsnorm_bwd_rows(dy, x, w, rstd, dres, dx, parts, rows, dim, STREAM(stream))) {
+    chain(norm_dw_kernel, (dim / 4 + 15) / 16, 256, 0, STREAM(stream), (const float4*)parts, (float4*)dw_f32, (uint2*)dw_bf16, n,
+          dim / 4);
     return rc(cudaGetLastError());
   }
   cudaError_t e = cudaMemsetAsync(dw_f32, 0, sizeof(float) * dim, STREAM(stream));

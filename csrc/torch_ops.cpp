@@ -427,15 +427,16 @@ variable_list norm_bwd(AutogradContext* ctx, const Tensor& dy_, const Tensor& dr
   TORCH_CHECK(plain(dy) && (!dres.defined() || plain(dres)), "rms_norm: gradient of an unexpected kind");
   const int64_t d = x.size(-1);
   const int rows = (int)(x.numel() / d);
-  Tensor dx = empty_as(x, x.sizes()), dwf = empty_like_type(w, {1 + tpb_rmsnorm_bwd_parts(rows, (int)d), d}, at::kFloat), dw;
+  Tensor dx = empty_as(x, x.sizes()), dwf = empty_like_type(w, {d}, at::kFloat), dw, parts;
+  if (const int n = tpb_rmsnorm_bwd_parts(rows, (int)d)) parts = empty_like_type(w, {n, d}, at::kFloat);
   const bool late = ctx->needs_input_grad(1) && any_main_grad(&w, 1);
   if (ctx->needs_input_grad(1) && !late) dw = empty_as(w, {d});
   check(tpb_rmsnorm_bwd_dw(cptr(dy), cptr(x), cptr(w), static_cast<const float*>(cptr(rstd)), cptr(dres), mptr(dx),
-                           static_cast<float*>(mptr(dwf)), mptr(dw), rows, (int)d, stream()),
+                           static_cast<float*>(mptr(dwf)), mptr(dw), static_cast<float*>(mptr(parts)), rows, (int)d, stream()),
         "rmsnorm_bwd");
   if (late) {
     py::gil_scoped_acquire gil;
-    py::reinterpret_borrow<py::object>(g_late_norm)(py::reinterpret_steal<py::object>(THPVariable_Wrap(w)), py::cast(dwf.select(0, 0)));
+    py::reinterpret_borrow<py::object>(g_late_norm)(py::reinterpret_steal<py::object>(THPVariable_Wrap(w)), py::cast(dwf));
   }
   return {dx, dw, Tensor()};
 }

@@ -48,3 +48,14 @@ def test_bad_values_stay_in_their_row(cuda_lib):
     assert torch.isfinite(t[good]).all()
     assert torch.isnan(t[7]).all() and not torch.isfinite(t[2099]).all()
   assert torch.isnan(dw).all()
+
+
+@pytest.mark.parametrize("rows", [100, 4000])
+def test_weight_gradient_holds_no_scratch(cuda_lib, rows):
+  """The gradient that is returned keeps its own dim values alive and no partial sums."""
+  from torchprime_b200.ops import kernels as k
+  x = torch.randn(rows, 1024, device="cuda").bfloat16()
+  w = torch.ones(1024, device="cuda").bfloat16()
+  _, rstd, _ = k.rmsnorm_fwd(x, w, 1e-5)
+  _, dw = k.rmsnorm_bwd(torch.randn_like(x), x, w, rstd)
+  assert dw.untyped_storage().nbytes() == 4 * 1024

@@ -115,10 +115,12 @@ def rmsnorm_bwd(dy, x, w, rstd, dres=None, dw_f32=None):
   dr2 = dres.reshape(-1, d) if dres is not None else None
   if dw_f32 is None:
     rows = x2.shape[0]
-    sums = torch.empty(1 + lib().tpb_rmsnorm_bwd_parts(rows, d), d, dtype=torch.float32, device=x.device)
-    check(lib().tpb_rmsnorm_bwd_dw(ptr(dy2), ptr(x2), ptr(w), ptr(rstd), ptr(dr2), ptr(dx), ptr(sums), None, rows, d,
+    dw = torch.empty(d, dtype=torch.float32, device=x.device)
+    n = lib().tpb_rmsnorm_bwd_parts(rows, d)
+    parts = torch.empty(n, d, dtype=torch.float32, device=x.device) if n else None
+    check(lib().tpb_rmsnorm_bwd_dw(ptr(dy2), ptr(x2), ptr(w), ptr(rstd), ptr(dr2), ptr(dx), ptr(dw), None, ptr(parts), rows, d,
                                    stream_ptr()), "rmsnorm_bwd")
-    return dx.view(x.shape), sums[0]
+    return dx.view(x.shape), dw
   check(lib().tpb_rmsnorm_bwd(ptr(dy2), ptr(x2), ptr(w), ptr(rstd), ptr(dr2), ptr(dx), ptr(dw_f32), x2.shape[0], d,
                               stream_ptr()), "rmsnorm_bwd")
   return dx.view(x.shape), dw_f32
