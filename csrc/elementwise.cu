@@ -402,10 +402,10 @@ rmsnorm_bwd_rows_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ 
   }
 }
 
-// dw[c] = sum over the n rows of parts, in fp32 and, with dw_bf16, rounded.  A block takes 64 columns: sixteen threads of four
+// dw[c] = (`add`: dw[c] +) sum over the n rows of parts, in fp32 and, with dw_bf16, rounded.  A block takes 64 columns: sixteen threads of four
 // columns each side by side, sixteen rows at a time.
 __global__ void __launch_bounds__(256)
-norm_dw_kernel(const float4* __restrict__ parts, float4* __restrict__ dw, uint2* __restrict__ dw_bf16, int n, int dim4) {
+norm_dw_kernel(const float4* __restrict__ parts, float4* __restrict__ dw, uint2* __restrict__ dw_bf16, int n, int dim4, int add) {
   if (!chain_begin()) return;
   __shared__ float4 sums[16][16];
   const int c = threadIdx.x & 15, r0 = threadIdx.x >> 4, col = blockIdx.x * 16 + c;
@@ -423,6 +423,10 @@ norm_dw_kernel(const float4* __restrict__ parts, float4* __restrict__ dw, uint2*
 #pragma unroll
   for (int r = 1; r < 16; ++r) {
     const float4 v = sums[r][c];
+    a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
+  }
+  if (add) {
+    const float4 v = dw[col];
     a.x += v.x; a.y += v.y; a.z += v.z; a.w += v.w;
   }
   dw[col] = a;
@@ -1008,18 +1012,19 @@ extern "C" int tpb_scale_cast_bf16(const float* src, void* dst, long long n, con
   return rc(cudaGetLastError());
 }
 
-// tpb_rmsnorm_bwd with the weight gradient written to dw_f32 instead of added to; with dw_bf16 also delivered in bf16.
+// tpb_rmsnorm_bwd with the weight gradient written to dw_f32 or, with `add`, added to what is there; with dw_bf16 the result is
+// also delivered in bf16.
 extern "C" int tpb_rmsnorm_bwd_dw(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
-                                  float* dw_f32, void* dw_bf16, float* parts, int rows, int dim, void* stream) {
+                                  float* dw_f32, void* dw_bf16, float* parts, int add, int rows, int dim, void* stream) {
   const int n = parts ? tpb_rmsnorm_bwd_parts(rows, dim) : 0;
   if (n > 0 && aligned16(dy) && aligned16(x) && aligned16(w) && aligned16(dx) && aligned16(dres) && aligned16(dw_f32) &&
       aligned16(parts) && reinterpret_cast<uintptr_t>(dw_bf16) % 8 == 0 &&
       launch_rmsnorm_bwd_rows(dy, x, w, rstd, dres, dx, parts, rows, dim, STREAM(stream))) {
     chain(norm_dw_kernel, (dim / 4 + 15) / 16, 256, 0, STREAM(stream), (const float4*)parts, (float4*)dw_f32, (uint2*)dw_bf16, n,
-          dim / 4);
+          dim / 4, add);
     return rc(cudaGetLastError());
   }
-  cudaError_t e = cudaMemsetAsync(dw_f32, 0, sizeof(float) * dim, STREAM(stream));
+  const cudaError_t e = add ? cudaSuccess : cudaMemsetAsync(dw_f32, 0, sizeof(float) * dim, STREAM(stream));
   if (e != cudaSuccess) return rc(e);
   const int r = tpb_rmsnorm_bwd(dy, x, w, rstd, dres, dx, dw_f32, rows, dim, stream);
   return r || !dw_bf16 ? r : tpb_cast_f32_to_bf16(dw_f32, dw_bf16, dim, 1.f, 0, stream);

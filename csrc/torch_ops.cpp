@@ -432,7 +432,7 @@ variable_list norm_bwd(AutogradContext* ctx, const Tensor& dy_, const Tensor& dr
   const bool late = ctx->needs_input_grad(1) && any_main_grad(&w, 1);
   if (ctx->needs_input_grad(1) && !late) dw = empty_as(w, {d});
   check(tpb_rmsnorm_bwd_dw(cptr(dy), cptr(x), cptr(w), static_cast<const float*>(cptr(rstd)), cptr(dres), mptr(dx),
-                           static_cast<float*>(mptr(dwf)), mptr(dw), static_cast<float*>(mptr(parts)), rows, (int)d, stream()),
+                           static_cast<float*>(mptr(dwf)), mptr(dw), static_cast<float*>(mptr(parts)), 0, rows, (int)d, stream()),
         "rmsnorm_bwd");
   if (late) {
     py::gil_scoped_acquire gil;

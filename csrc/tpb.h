@@ -55,11 +55,11 @@ int tpb_rmsnorm_fwd(const void* x, const void* res, const void* w, void* y, void
 // dx = d/dx of the above (+ dres if given).  dw_f32 [dim] is accumulated with atomics.
 int tpb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres,
                     void* dx, float* dw_f32, int rows, int dim, void* stream);
-// The same with the sums written to dw_f32 [dim] and, if given, dw_bf16; parts is scratch, [tpb_rmsnorm_bwd_parts(rows, dim)][dim]
-// (without it, and where that is 0, they are accumulated with atomics after a clearing).
+// The same with the sums written (`add`: added) to dw_f32 [dim] and, if given, dw_bf16; parts is scratch,
+// [tpb_rmsnorm_bwd_parts(rows, dim)][dim] (without it, and where that is 0, they are accumulated with atomics).
 int tpb_rmsnorm_bwd_parts(int rows, int dim);
 int tpb_rmsnorm_bwd_dw(const void* dy, const void* x, const void* w, const float* rstd, const void* dres, void* dx,
-                       float* dw_f32, void* dw_bf16, float* parts, int rows, int dim, void* stream);
+                       float* dw_f32, void* dw_bf16, float* parts, int add, int rows, int dim, void* stream);
 
 // In-place rotate-half RoPE on `heads` heads of width `dim` starting at column
 // `col0` of a [tokens, ld] bf16 matrix.  cos/sin: fp32 [max_pos, dim/2].

@@ -59,3 +59,22 @@ def test_weight_gradient_holds_no_scratch(cuda_lib, rows):
   _, rstd, _ = k.rmsnorm_fwd(x, w, 1e-5)
   _, dw = k.rmsnorm_bwd(torch.randn_like(x), x, w, rstd)
   assert dw.untyped_storage().nbytes() == 4 * 1024
+
+
+@pytest.mark.parametrize("rows", [300, 2100])
+def test_weight_gradient_is_added_to_what_is_there(cuda_lib, rows):
+  """From as many rows on as a call without a sum to add to does, this one takes the streamed kernel, so that its sum is that
+  one's bit for bit (fewer rows are added with atomics: fp32 sums in any order)."""
+  from torchprime_b200.ops import kernels as k
+  x, dy = (torch.randn(rows, 2048, device="cuda").bfloat16() for _ in range(2))
+  w = torch.ones(2048, device="cuda").bfloat16()
+  _, rstd, _ = k.rmsnorm_fwd(x, w, 1e-5)
+  dx, dw = k.rmsnorm_bwd(dy, x, w, rstd)
+  old = torch.randn(2048, device="cuda")
+  into = old.clone()
+  dx2, got = k.rmsnorm_bwd(dy, x, w, rstd, dw_f32=into)
+  assert got.data_ptr() == into.data_ptr() and torch.equal(dx, dx2)
+  if rows >= 1024:
+    assert torch.equal(into, old + dw)
+  else:
+    assert _rel(into, (old + dw).double()) < 1e-6

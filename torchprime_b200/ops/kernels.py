@@ -107,23 +107,19 @@ def rmsnorm_fwd(x, w, eps, res=None, want_h=False):
 
 
 def rmsnorm_bwd(dy, x, w, rstd, dres=None, dw_f32=None):
-  """dx (+ dres) and dw in fp32 [dim]; with ``dw_f32`` it is added (atomics) to what is there."""
+  """dx (+ dres) and dw in fp32 [dim]; with ``dw_f32`` it is added to what is there (few rows: with atomics)."""
   d = x.shape[-1]
   dy2, x2 = dy.reshape(-1, d), x.reshape(-1, d)
   assert dy2.is_contiguous() and x2.is_contiguous()
   dx = torch.empty_like(x2)
   dr2 = dres.reshape(-1, d) if dres is not None else None
-  if dw_f32 is None:
-    rows = x2.shape[0]
-    dw = torch.empty(d, dtype=torch.float32, device=x.device)
-    n = lib().tpb_rmsnorm_bwd_parts(rows, d)
-    parts = torch.empty(n, d, dtype=torch.float32, device=x.device) if n else None
-    check(lib().tpb_rmsnorm_bwd_dw(ptr(dy2), ptr(x2), ptr(w), ptr(rstd), ptr(dr2), ptr(dx), ptr(dw), None, ptr(parts), rows, d,
-                                   stream_ptr()), "rmsnorm_bwd")
-    return dx.view(x.shape), dw
-  check(lib().tpb_rmsnorm_bwd(ptr(dy2), ptr(x2), ptr(w), ptr(rstd), ptr(dr2), ptr(dx), ptr(dw_f32), x2.shape[0], d,
-                              stream_ptr()), "rmsnorm_bwd")
-  return dx.view(x.shape), dw_f32
+  rows = x2.shape[0]
+  n = lib().tpb_rmsnorm_bwd_parts(rows, d)
+  dw = torch.empty(d, dtype=torch.float32, device=x.device) if dw_f32 is None else dw_f32
+  parts = torch.empty(n, d, dtype=torch.float32, device=x.device) if n else None
+  check(lib().tpb_rmsnorm_bwd_dw(ptr(dy2), ptr(x2), ptr(w), ptr(rstd), ptr(dr2), ptr(dx), ptr(dw), None, ptr(parts),
+                                 int(dw_f32 is not None), rows, d, stream_ptr()), "rmsnorm_bwd")
+  return dx.view(x.shape), dw
 
 
 def rope_(x2d, col0, heads, dim, cos, sin, seq_len, pos=None, inverse=False, interleaved=False, head_stride=None):
