@@ -195,7 +195,7 @@ __device__ __forceinline__ void bulk_row_load(void* smem_dst, const void* src, u
 // Forward: a warp to a row, the row in its registers (VPL 16-byte vectors a lane), its next rows on their way.  The sum over
 // the row is five shuffles.  8192 x 4096: 26.0 us (5.2 TB/s), 27.3 with 256 threads to a row and three barriers; x 2048 16 and 27.
 template <int VPL>
-__global__ void __launch_bounds__(VPL <= 16 ? 512 : VPL <= 20 ? 384 : 256)
+__global__ void __launch_bounds__(512)
 rmsnorm_fwd_rows_kernel(const uint4* __restrict__ x, const uint4* __restrict__ w, uint4* __restrict__ y,
                         float* __restrict__ rstd_out, int rows, int nvec, float eps, int stages, int* status) {
   if (!chain_begin()) return;
@@ -262,6 +262,83 @@ rmsnorm_fwd_rows_kernel(const uint4* __restrict__ x, const uint4* __restrict__ w
   }
   for (; k < issued; ++k)   // a wait ran out: what was asked for still lands here (bounded again)
     mbar_wait_warp(&full[k % stages], (uint32_t)(k / stages) & 1u, status, kTimeoutTmaFull, 74);
+}
+
+// Forward of wide rows: 256 threads to a row, three CTAs per SM, each with two rows of shared memory.  (A warp's share of a row of
+// 8192 is 1 KB in its registers, and six warps are all that the rings leave room for.)  The weight stays in registers.  The next row
+// is asked for when this one has arrived: bound by memory, where more rows under way are slower (8192 x 8192, us: 44, asked
+// for a row earlier 45, two 50; 3000 x 8192 18, 18, 18.4).  A stage is handed back by the barrier that opens every iteration, which
+// also carries the give-up decision of a wait that ran out.
+template <int VPT>
+__global__ void __launch_bounds__(NORM_THREADS)
+rmsnorm_fwd_wide_kernel(const uint4* __restrict__ x, const uint4* __restrict__ w, uint4* __restrict__ y,
+                        float* __restrict__ rstd_out, int rows, int nvec, float eps, int* status) {
+  if (!chain_begin()) return;
+  extern __shared__ uint8_t nw_smem_raw[];
+  uint8_t* smem = nw_smem_raw + ((128u - (smem_u32(nw_smem_raw) & 127u)) & 127u);
+  uint64_t* full = reinterpret_cast<uint64_t*>(smem);   // [2]
+  uint4* stage = reinterpret_cast<uint4*>(smem + 128);
+  __shared__ float red[32];
+  const uint32_t row_bytes = (uint32_t)nvec * 16u;
+  const int mine = (rows - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x;   // grid <= rows
+  auto issue = [&](int k) {   // thread 0
+    mbar_expect_tx(&full[k & 1], row_bytes);
+    bulk_row_load(stage + (k & 1) * nvec, x + ((size_t)blockIdx.x + (size_t)k * gridDim.x) * nvec, row_bytes, &full[k & 1]);
+  };
+  int issued = 0;
+  if (threadIdx.x == 0) {
+    mbar_init(&full[0], 1);
+    mbar_init(&full[1], 1);
+    fence_barrier_init();
+    issue(issued++);
+  }
+  float wv[VPT][8];
+#pragma unroll
+  for (int j = 0; j < VPT; ++j) {
+    const int i = threadIdx.x + j * NORM_THREADS;
+    if (i < nvec) unpack8(w[i], wv[j]);
+  }
+  bool ok = true;
+  int k = 0, drain_from = -1;
+  for (; k < mine; ++k) {
+    ok = __syncthreads_and(ok);     // every thread is done with the stage the next request goes into (and sees the barriers)
+    if (!ok) break;
+    ok = mbar_wait(&full[k & 1], (uint32_t)(k >> 1) & 1u, status, kTimeoutTmaFull, 75);
+    if (!ok && drain_from < 0) drain_from = k;
+    if (threadIdx.x == 0 && ok && issued < mine) {
+      fence_proxy_async();
+      issue(issued++);
+    }
+    const uint4* sx = stage + (k & 1) * nvec;
+    const size_t row = (size_t)blockIdx.x + (size_t)k * gridDim.x;
+    float v[VPT][8];
+    float ss = 0.f;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      const int i = threadIdx.x + j * NORM_THREADS;
+      if (i < nvec) {
+        unpack8(sx[i], v[j]);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) ss += v[j][e] * v[j][e];
+      }
+    }
+    const float rstd = rsqrtf(block_sum(ss, red) / (float)(nvec * 8) + eps);
+    if (threadIdx.x == 0 && rstd_out) rstd_out[row] = rstd;
+#pragma unroll
+    for (int j = 0; j < VPT; ++j) {
+      const int i = threadIdx.x + j * NORM_THREADS;
+      if (i < nvec) {
+        float o[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) o[e] = wv[j][e] * rbf(v[j][e] * rstd);
+        y[row * nvec + i] = pack8(o);
+      }
+    }
+  }
+  if (drain_from < 0 && k < mine) drain_from = k;
+  if (drain_from >= 0 && threadIdx.x == 0)   // a wait ran out: what was asked for still lands here (bounded again)
+    for (int kk = drain_from; kk < issued; ++kk)
+      mbar_wait(&full[kk & 1], (uint32_t)(kk >> 1) & 1u, status, kTimeoutTmaFull, 76);
 }
 
 // Backward: 128 threads to a row, GROUPS of them in a CTA, each with a ring of rows (dy | x | dres) of its own.  A thread
@@ -819,18 +896,20 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 
 // Streamed forms: rows that can be bulk-copied (16-byte aligned bases; the pitch is a multiple of 16 bytes), no residual
 // added in the forward, and enough of them: fewer rows than warps of the streamed forward leave it with nothing to run ahead
-// of, and the CTAs of one row each start sooner.  us, CTAs per row / streamed, inputs from HBM:
-//   forward, 2048 wide: 2000 rows 9.4 / 11, 3000 14.4 / 13.4, 8192 27 / 16;   4096 wide: 900 11 / 13, 8192 31 (27 with the
-//   previous streamed form) / 26
+// of, and the CTAs of one row each start sooner.  us, CTAs per row / streamed, inputs larger than L2 in all:
+//   forward, a warp to a row: 2048 wide: 1900 rows 4.9 / 5.1, 2200 6.1 / 5.3, 8192 17.5 / 15.4;   3072: 2200 9.1 / 7.4, 8192 30 / 20
+//     4096: 2200 rows 9.6 / 10.8, 3200 12.6 / 13.0, 4000 15.3 / 15.7, 6000 24.5 / 20.7, 8192 34 / 26.9
+//   forward, 256 threads to a row / a warp to a row: 5120: 900 rows 6.9 / 6.1 / 7.1, 8192 44 / 32.5 / 35.5;   6144: 2200 13.0 / 11.2 / 16.4,
+//     8192 48 / 36 / 47;   8192: 1200 11.2 / 8.9 / 17, 3200 26.7 / 18.5 / 31.5, 8192 61 / 43.7 / 75.5
 //   backward with a residual, 4096 wide: 1000 rows 23 / 19, 4000 33 / 31, 8192 55 / 50;   5120 wide: 2000 29 / 22, 8192 93 / 60
-constexpr int NS_FWD_MIN_ROWS = 2048, NS_BWD_MIN_ROWS = 1024;
+constexpr int NS_BWD_MIN_ROWS = 1024;
 static bool launch_rmsnorm_fwd_rows(const void* x, const void* w, void* y, float* rstd, int rows, int dim, float eps,
                                     cudaStream_t stream) {
   static const bool disabled = []() { const char* v = getenv("TPB_RMSNORM_FWD_BULK"); return v && v[0] == '0'; }();
   if (disabled) return false;
   const int nvec = dim / 8, row_bytes = dim * 2;
-  if (!aligned16(x) || !aligned16(y) || !aligned16(w) || rows < NS_FWD_MIN_ROWS) return false;
-  const int most = nvec <= 512 ? 16 : nvec <= 640 ? 12 : 8;
+  if (nvec > 512 || !aligned16(x) || !aligned16(y) || !aligned16(w) || rows < (nvec <= 384 ? 2048 : 4000)) return false;
+  constexpr int most = 16;
   int stages = NS_SMEM / (most * row_bytes);
   stages = stages > NS_MAX_STAGES ? NS_MAX_STAGES : stages < 2 ? 2 : stages;
   int warps = NS_SMEM / (stages * row_bytes);
@@ -844,8 +923,22 @@ static bool launch_rmsnorm_fwd_rows(const void* x, const void* w, void* y, float
     chain(rmsnorm_fwd_rows_kernel<V>, sm_count(), 32 * warps, smem, stream, (const uint4*)x, (const uint4*)w, (uint4*)y, rstd, \
           rows, nvec, eps, stages, status_block());                                                                          \
   } while (0)
-  if (nvec <= 256) TPB_NORM_FWD(8); else if (nvec <= 512) TPB_NORM_FWD(16); else if (nvec <= 640) TPB_NORM_FWD(20); else TPB_NORM_FWD(32);
+  if (nvec <= 256) TPB_NORM_FWD(8); else TPB_NORM_FWD(16);
 #undef TPB_NORM_FWD
+  return true;
+}
+
+constexpr int NS_WIDE_CTAS = 3, NS_WIDE_SMEM = 66 * 1024;   // (as much as lets three on an SM and no fourth beside an idle one)
+static bool launch_rmsnorm_fwd_wide(const void* x, const void* w, void* y, float* rstd, int rows, int dim, float eps,
+                                    cudaStream_t stream) {
+  static const bool disabled = []() { const char* v = getenv("TPB_RMSNORM_FWD_BULK"); return v && v[0] == '0'; }();
+  const int nvec = dim / 8, grid = NS_WIDE_CTAS * sm_count();
+  if (disabled || nvec <= 512 || !aligned16(x) || !aligned16(y) || !aligned16(w) || rows < 2 * grid) return false;
+  static const cudaError_t set =
+      cudaFuncSetAttribute(rmsnorm_fwd_wide_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, NS_WIDE_SMEM);
+  if (set != cudaSuccess) return false;
+  chain(rmsnorm_fwd_wide_kernel<4>, grid, NORM_THREADS, NS_WIDE_SMEM, stream, (const uint4*)x, (const uint4*)w, (uint4*)y, rstd,
+        rows, nvec, eps, status_block());
   return true;
 }
 
@@ -853,7 +946,9 @@ extern "C" int tpb_rmsnorm_fwd(const void* x, const void* res, const void* w, vo
                                int rows, int dim, float eps, void* stream) {
   if (dim % 8 || dim > 8 * NORM_THREADS * NORM_VPT) return -2;
   if (rows <= 0) return 0;
-  if (!res && launch_rmsnorm_fwd_rows(x, w, y, rstd, rows, dim, eps, STREAM(stream))) return rc(cudaGetLastError());
+  if (!res && (launch_rmsnorm_fwd_rows(x, w, y, rstd, rows, dim, eps, STREAM(stream)) ||
+               launch_rmsnorm_fwd_wide(x, w, y, rstd, rows, dim, eps, STREAM(stream))))
+    return rc(cudaGetLastError());
   const int nvec = dim / 8;
   const int vpt = (nvec + NORM_THREADS - 1) / NORM_THREADS;
   const int per_sm = vpt <= 2 ? 8 : 4;

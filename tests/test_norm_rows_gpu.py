@@ -78,3 +78,20 @@ def test_weight_gradient_is_added_to_what_is_there(cuda_lib, rows):
     assert torch.equal(into, old + dw)
   else:
     assert _rel(into, (old + dw).double()) < 1e-6
+
+
+@pytest.mark.parametrize("rows,dim", [(887, 5120), (888, 5120), (889, 4104), (1333, 8192), (3999, 4096), (4000, 4096), (4001, 3080),
+                                      (2047, 3072), (2048, 3072), (5000, 6144)])
+def test_forward_of_wide_and_of_many_rows(cuda_lib, rows, dim):
+  """Both sides of every edge between the forms; the form of a CTA to a row, which a residual of zeros asks for, sums in another
+  order than the one of a warp to a row."""
+  from torchprime_b200.ops import kernels as k
+  torch.manual_seed(dim)
+  x = torch.randn(rows, dim, device="cuda").bfloat16()
+  w = (1 + 0.1 * torch.randn(dim, device="cuda")).bfloat16()
+  y, rstd, _ = k.rmsnorm_fwd(x, w, 1e-5)
+  y2, rstd2, _ = k.rmsnorm_fwd(x, w, 1e-5, res=torch.zeros_like(x), want_h=True)
+  r = torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5)
+  assert _rel(rstd, r[:, 0]) < 1e-6 and _rel(y, x.double() * r * w.double()) < 2 ** -8
+  if dim > 4096:
+    assert torch.equal(y, y2) and torch.equal(rstd, rstd2)
