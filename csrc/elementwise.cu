@@ -59,7 +59,10 @@ constexpr int NORM_VPT = 4;  // most 16-byte vectors kept in registers per threa
 // The kernels are instantiated for 1, 2 and 4 vectors per thread: a 4096-wide row needs two, and
 // the instantiation that holds exactly that many leaves registers for more resident CTAs, which
 // is what a latency-bound row-per-CTA kernel needs to fill the memory pipe.
-template <int VPT>
+// EARLY: the weight is asked for with the row and not behind its sum.  That is for few rows, where the chain of loads is all there is
+// (16 rows of 4096: 2.6 -> 2.4 us); its registers cost resident CTAs (8192 rows of 4096 with a residual 49 -> 60 us, 2048 wide 25 ->
+// 32.5), but for rows of more than 4096, which have fewer than that anyway (8192 rows of 8192 with a residual 113 both ways).
+template <int VPT, bool EARLY>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, const uint4* __restrict__ w,
                    uint4* __restrict__ y, uint4* __restrict__ h_out, float* __restrict__ rstd_out, int rows,
@@ -69,13 +72,13 @@ rmsnorm_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, c
   for (int row = blockIdx.x; row < rows; row += gridDim.x) {
     const uint4* xr = x + (size_t)row * nvec;
     float vals[VPT][8];
-    uint4 wu[VPT];              // (asked for with the row, not behind its sum)
+    uint4 wu[VPT];
     float ss = 0.f;
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
       int i = threadIdx.x + j * NORM_THREADS;
       if (i < nvec) {
-        wu[j] = w[i];
+        if (EARLY) wu[j] = w[i];
         unpack8(xr[i], vals[j]);
         if (res) {
           float r[8];
@@ -96,7 +99,7 @@ rmsnorm_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, c
       int i = threadIdx.x + j * NORM_THREADS;
       if (i < nvec) {
         float wv[8], o[8];
-        unpack8(wu[j], wv);
+        unpack8(EARLY ? wu[j] : w[i], wv);
 #pragma unroll
         for (int e = 0; e < 8; ++e) o[e] = wv[e] * rbf(vals[j][e] * rstd);
         y[(size_t)row * nvec + i] = pack8(o);
@@ -953,9 +956,12 @@ extern "C" int tpb_rmsnorm_fwd(const void* x, const void* res, const void* w, vo
   const int vpt = (nvec + NORM_THREADS - 1) / NORM_THREADS;
   const int per_sm = vpt <= 2 ? 8 : 4;
   const int grid = rows < sm_count() * per_sm ? rows : sm_count() * per_sm;
-#define TPB_LAUNCH_NORM_FWD(V) chain(rmsnorm_fwd_kernel<V>, grid, NORM_THREADS, 0, STREAM(stream), \
+  const bool early = rows <= 2 * sm_count();
+#define TPB_LAUNCH_NORM_FWD(V, EARLY) chain(rmsnorm_fwd_kernel<V, EARLY>, grid, NORM_THREADS, 0, STREAM(stream), \
       (const uint4*)x, (const uint4*)res, (const uint4*)w, (uint4*)y, (uint4*)h_out, rstd, rows, nvec, eps)
-  if (vpt <= 1) TPB_LAUNCH_NORM_FWD(1); else if (vpt == 2) TPB_LAUNCH_NORM_FWD(2); else TPB_LAUNCH_NORM_FWD(4);
+  if (vpt > 2) TPB_LAUNCH_NORM_FWD(4, true);
+  else if (vpt == 2) { if (early) TPB_LAUNCH_NORM_FWD(2, true); else TPB_LAUNCH_NORM_FWD(2, false); }
+  else if (early) TPB_LAUNCH_NORM_FWD(1, true); else TPB_LAUNCH_NORM_FWD(1, false);
 #undef TPB_LAUNCH_NORM_FWD
   return rc(cudaGetLastError());
 }

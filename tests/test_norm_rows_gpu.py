@@ -95,3 +95,16 @@ def test_forward_of_wide_and_of_many_rows(cuda_lib, rows, dim):
   assert _rel(rstd, r[:, 0]) < 1e-6 and _rel(y, x.double() * r * w.double()) < 2 ** -8
   if dim > 4096:
     assert torch.equal(y, y2) and torch.equal(rstd, rstd2)
+
+
+@pytest.mark.parametrize("dim", [8, 2048, 2056, 4096, 4104])
+def test_few_and_many_rows_of_a_cta_each_are_the_same(cuda_lib, dim):
+  """The form that asks for the weight with the row and the one that asks behind its sum differ in nothing else."""
+  from torchprime_b200.ops import kernels as k
+  sms = torch.cuda.get_device_properties(0).multi_processor_count
+  x, res = (torch.randn(2 * sms + 1, dim, device="cuda").bfloat16() for _ in range(2))
+  w = (1 + 0.1 * torch.randn(dim, device="cuda")).bfloat16()
+  for r in (None, res):
+    many = k.rmsnorm_fwd(x, w, 1e-5, res=r, want_h=True)
+    few = k.rmsnorm_fwd(x[:-1], w, 1e-5, res=None if r is None else r[:-1], want_h=True)
+    assert all(a is None or torch.equal(a[:-1], b) for a, b in zip(many, few))
