@@ -900,18 +900,20 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 // Streamed forms: rows that can be bulk-copied (16-byte aligned bases; the pitch is a multiple of 16 bytes), no residual
 // added in the forward, and enough of them: fewer rows than warps of the streamed forward leave it with nothing to run ahead
 // of, and the CTAs of one row each start sooner.  us, CTAs per row / streamed, inputs larger than L2 in all:
-//   forward, a warp to a row: 2048 wide: 1900 rows 4.9 / 5.1, 2200 6.1 / 5.3, 8192 17.5 / 15.4;   3072: 2200 9.1 / 7.4, 8192 30 / 20
-//     4096: 2200 rows 9.6 / 10.8, 3200 12.6 / 13.0, 4000 15.3 / 15.7, 6000 24.5 / 20.7, 8192 34 / 26.9
+//   forward, a warp to a row: 512 wide: 2600 rows 4.3 / 4.5, 4000 5.2 / 4.7, 32768 30.8 / 23.8;   1024: 2600 rows 4.5 / 5.3, 10000 12.4 /
+//     12.4, 32768 38 / 31;   2048: 2600 rows 5.9 / 7.6, 12000 20.4 / 20.1, 32768 52.5 / 47.5 (one vector to a thread of the CTA: quick);
+//     2304: 2300 rows 8.7 / 6.3, 8192 25 / 16;   3072: 2200 9.2 / 7.4, 8192 29 / 20;   4096: 3200 rows 11.6 / 12.9, 4500 17.1 / 16.8, 8192 34 / 27
 //   forward, 256 threads to a row / a warp to a row: 5120: 900 rows 6.9 / 6.1 / 7.1, 8192 44 / 32.5 / 35.5;   6144: 2200 13.0 / 11.2 / 16.4,
 //     8192 48 / 36 / 47;   8192: 1200 11.2 / 8.9 / 17, 3200 26.7 / 18.5 / 31.5, 8192 61 / 43.7 / 75.5
 //   backward with a residual, 4096 wide: 1000 rows 23 / 19, 4000 33 / 31, 8192 55 / 50;   5120 wide: 2000 29 / 22, 8192 93 / 60
 constexpr int NS_BWD_MIN_ROWS = 1024;
+static int norm_fwd_rows_from(int nvec) { return nvec <= 96 ? 3000 : nvec <= 256 ? 12000 : nvec <= 384 ? 2048 : 4500; }
 static bool launch_rmsnorm_fwd_rows(const void* x, const void* w, void* y, float* rstd, int rows, int dim, float eps,
                                     cudaStream_t stream) {
   static const bool disabled = []() { const char* v = getenv("TPB_RMSNORM_FWD_BULK"); return v && v[0] == '0'; }();
   if (disabled) return false;
   const int nvec = dim / 8, row_bytes = dim * 2;
-  if (nvec > 512 || !aligned16(x) || !aligned16(y) || !aligned16(w) || rows < (nvec <= 384 ? 2048 : 4000)) return false;
+  if (nvec > 512 || !aligned16(x) || !aligned16(y) || !aligned16(w) || rows < norm_fwd_rows_from(nvec)) return false;
   constexpr int most = 16;
   int stages = NS_SMEM / (most * row_bytes);
   stages = stages > NS_MAX_STAGES ? NS_MAX_STAGES : stages < 2 ? 2 : stages;

@@ -80,8 +80,9 @@ def test_weight_gradient_is_added_to_what_is_there(cuda_lib, rows):
     assert _rel(into, (old + dw).double()) < 1e-6
 
 
-@pytest.mark.parametrize("rows,dim", [(887, 5120), (888, 5120), (889, 4104), (1333, 8192), (3999, 4096), (4000, 4096), (4001, 3080),
-                                      (2047, 3072), (2048, 3072), (5000, 6144)])
+@pytest.mark.parametrize("rows,dim", [(887, 5120), (888, 5120), (889, 4104), (1333, 8192), (4499, 4096), (4500, 4096), (4501, 3080),
+                                      (2047, 3072), (2048, 3072), (2050, 2056), (5000, 6144), (2999, 768), (3000, 768), (3001, 8),
+                                      (11999, 2048), (12000, 2048), (12001, 776)])
 def test_forward_of_wide_and_of_many_rows(cuda_lib, rows, dim):
   """Both sides of every edge between the forms; the form of a CTA to a row, which a residual of zeros asks for, sums in another
   order than the one of a warp to a row."""
