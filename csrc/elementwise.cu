@@ -905,8 +905,9 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 //     2304: 2300 rows 8.7 / 6.3, 8192 25 / 16;   3072: 2200 9.2 / 7.4, 8192 29 / 20;   4096: 3200 rows 11.6 / 12.9, 4500 17.1 / 16.8, 8192 34 / 27
 //   forward, 256 threads to a row / a warp to a row: 5120: 900 rows 6.9 / 6.1 / 7.1, 8192 44 / 32.5 / 35.5;   6144: 2200 13.0 / 11.2 / 16.4,
 //     8192 48 / 36 / 47;   8192: 1200 11.2 / 8.9 / 17, 3200 26.7 / 18.5 / 31.5, 8192 61 / 43.7 / 75.5
-//   backward with a residual, 4096 wide: 1000 rows 23 / 19, 4000 33 / 31, 8192 55 / 50;   5120 wide: 2000 29 / 22, 8192 93 / 60
-constexpr int NS_BWD_MIN_ROWS = 1024;
+//   backward with a residual, 4096 wide: 1000 rows 23 / 19, 4000 33 / 31, 8192 55 / 50;   5120 wide: 2000 29 / 22, 8192 93 / 60;
+//     8192 wide: 600 rows 23.4 / 16.0, 1000 33.5 / 19.3
+static int norm_bwd_rows_from(int dim) { return dim > 4096 ? 576 : 1024; }
 static int norm_fwd_rows_from(int nvec) { return nvec <= 96 ? 3000 : nvec <= 256 ? 12000 : nvec <= 384 ? 2048 : 4500; }
 static bool launch_rmsnorm_fwd_rows(const void* x, const void* w, void* y, float* rstd, int rows, int dim, float eps,
                                     cudaStream_t stream) {
@@ -992,7 +993,7 @@ static bool launch_rmsnorm_bwd_rows(const void* dy, const void* x, const void* w
 // Rows of scratch that tpb_rmsnorm_bwd_dw takes.
 extern "C" int tpb_rmsnorm_bwd_parts(int rows, int dim) {
   static const bool disabled = []() { const char* v = getenv("TPB_RMSNORM_BWD_BULK"); return v && v[0] == '0'; }();
-  return disabled || dim % 8 || dim > 8 * NORM_THREADS * NORM_VPT || rows < NS_BWD_MIN_ROWS ? 0 : sm_count();
+  return disabled || dim % 8 || dim > 8 * NORM_THREADS * NORM_VPT || rows < norm_bwd_rows_from(dim) ? 0 : sm_count();
 }
 
 extern "C" int tpb_rmsnorm_bwd(const void* dy, const void* x, const void* w, const float* rstd, const void* dres,

@@ -109,3 +109,12 @@ def test_few_and_many_rows_of_a_cta_each_are_the_same(cuda_lib, dim):
     many = k.rmsnorm_fwd(x, w, 1e-5, res=r, want_h=True)
     few = k.rmsnorm_fwd(x[:-1], w, 1e-5, res=None if r is None else r[:-1], want_h=True)
     assert all(a is None or torch.equal(a[:-1], b) for a, b in zip(many, few))
+
+
+@pytest.mark.parametrize("rows,dim,streamed", [(575, 8192, False), (576, 8192, True), (600, 4104, True), (1023, 4096, False), (1024, 4096, True),
+                                               (700, 6144, True)])
+def test_backward_of_few_wide_rows(cuda_lib, rows, dim, streamed):
+  """The streamed form, whose partial sums take scratch, begins earlier for wide rows."""
+  from torchprime_b200.ops import kernels as k
+  assert (cuda_lib.tpb_rmsnorm_bwd_parts(rows, dim) > 0) == streamed
+  test_forward_and_backward(cuda_lib, rows, dim, True)
