@@ -53,6 +53,7 @@ struct AttnFwdParams {
   long long ldo;       // elements between consecutive tokens of O
   float* lse;          // [B, Hq, Sq]
   int* status;
+  int grp_heads;       // query heads (of all sequences) whose tiles are taken together: fwd_group_heads()
   // Context-parallel K/V exchange fused into the kernel (cp_world > 1): the first cp_copiers CTAs
   // push this rank's K/V rows into every rank's gathered buffers (plain 16-byte stores over NVLink,
   // natural key order, so the zig-zag permutation costs nothing) and raise one flag per 128 keys in
@@ -275,12 +276,14 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant__
     cp_pusher(p);
     return;
   }
-  // The heaviest (latest) tiles of all heads come first under a causal mask, so that what runs last is short.  (Head by head
+  // The heaviest (latest) tiles of a group of heads come first under a causal mask, so that what runs last is short.  (Head by head
   // the last head's longest tile began when the others ended, us: 8192 tokens, 32/8 heads 528, this way 480; 4096 160 and 135; two
   // rows of 1999 tokens in segments 78 and 64; 2048 tokens, 16 heads of 192, all of whose CTAs run at once, 55 and 43.)
   const int id = (int)blockIdx.x - (p.cp_world > 1 ? p.cp_copiers : 0);
-  const int qt = n_qtiles - 1 - id / (p.Hq * p.B);
-  const int hq = (id / p.B) % p.Hq, b = id % p.B;
+  const int grp = id / (n_qtiles * p.grp_heads), within = id - grp * n_qtiles * p.grp_heads;
+  const int heads = min(p.grp_heads, p.Hq * p.B - grp * p.grp_heads);
+  const int qt = n_qtiles - 1 - within / heads, head = grp * p.grp_heads + within % heads;
+  const int hq = head % p.Hq, b = head / p.Hq;
   const int hkv = hq / (p.Hq / p.Hkv);
   const int q0 = qt * FWD_BM;
   const int pos_off = p.Sk - p.Sq;
@@ -1039,6 +1042,17 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap tmQ, const __grid_constant_
   }
 }
 
+// Query heads (a multiple of a key head's) whose tiles are taken together, longest first: as many as have 32 MB of keys and values,
+// which then stay in L2 while the machine works through them.  All heads of all sequences together read them from
+// memory over and over once they are more than L2 holds.  us, head by head / groups of 32 MB / all together, in turn, 32 heads of 128 on
+// as many key heads: thirty-two rows of 1024 tokens, causal, 405 / 411 / 504, eight of 4096 1208 / 1180 / 1365, two of 16384 4555 / 4140 /
+// 4290; not causal sixteen of 2048 1190 / 1156 / 1404, two of 16384 8040 / 8640 / 9540 (12500 by themselves); eight rows of 1024, 128 heads of 192, causal,
+// 674 / 681 / 787; one row of 8192, 32/8 heads, causal, 510 / 486 / 489.
+static int fwd_group_heads(int B, int Sk, int Hq, int Hkv, int dqk) {
+  const long long fit = (32LL << 20) / ((long long)Sk * (dqk + FWD_DV) * 2), all = (long long)B * Hkv;
+  return (int)((fit < 1 ? 1 : fit < all ? fit : all) * (Hq / Hkv));
+}
+
 template <int DQK, bool SEG>
 cudaError_t launch_fwd(const CUtensorMap& tq, const CUtensorMap& tk, const CUtensorMap& tv, const AttnFwdParams& p,
                        cudaStream_t stream) {
@@ -1122,6 +1136,7 @@ extern "C" int tpb_attn_fwd_softcap(const void* q, const void* k, const void* v,
   }
   p.O = reinterpret_cast<__nv_bfloat16*>(o); p.ldo = ldo; p.lse = lse;
   p.status = status_block();
+  p.grp_heads = fwd_group_heads(B, Sk, Hq, Hkv, dqk);
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   cudaError_t e = p.kv_rng ? (dqk == 128 ? launch_fwd<128, true>(tq, tk, tv, p, stream) : launch_fwd<192, true>(tq, tk, tv, p, stream))
                            : (dqk == 128 ? launch_fwd<128, false>(tq, tk, tv, p, stream)
@@ -1204,6 +1219,7 @@ extern "C" int tpb_attn_fwd_cp(const void* q, const void* k_local, const void* v
     if (e != cudaSuccess) return 1000 + (int)e;
     configured = true;
   }
+  p.grp_heads = Hq * B;
   const int n_qtiles = (Sq + FWD_BM - 1) / FWD_BM;
   const int grid = p.cp_copiers + n_qtiles * Hq * B;
   attn_fwd_kernel<128, false><<<grid, FWD_THREADS, FwdSmem<128>::TOTAL, reinterpret_cast<cudaStream_t>(stream_)>>>(tq, tk, tv, p);

@@ -252,3 +252,19 @@ def test_backward_rows_behind_the_last_add_nothing(cuda_lib):
   o, lse = A.attn_fwd(q[:1], k[:1], v[:1], causal=False)
   one = A.attn_bwd(do[:1], q[:1], k[:1], v[:1], o, lse, causal=False)
   assert all(torch.equal(a[:1], b) for a, b in zip(both, one))
+
+
+@pytest.mark.parametrize("b,s,hq,hkv,d", [(3, 300, 6, 3, 128), (1, 40000, 4, 2, 128), (5, 9000, 2, 1, 128), (1, 30000, 3, 3, 192)])
+def test_forward_covers_every_tile_of_every_group_of_heads(cuda_lib, b, s, hq, hkv, d):
+  """Heads in one group, in groups of one key head and in groups of which the last is smaller: rows of every head, first and
+  last tile of each sequence among them, against fp32; the rest finite."""
+  from torchprime_b200.ops import attention_sm100 as A
+  q, k, v = _qkv(b, s, hq, hkv, d, fused=False, seed=s)
+  o, lse = A.attn_fwd(q, k, v, causal=True)
+  assert torch.isfinite(o).all() and torch.isfinite(lse).all()
+  for i in range(b):
+    for r in (0, 127, 128, s // 2, s - 129, s - 1):
+      for h in range(hq):
+        sc = (k[i, :r + 1, h * hkv // hq].float() @ q[i, r, h].float()) / d ** 0.5
+        want = sc.softmax(0) @ v[i, :r + 1, h * hkv // hq].float()
+        assert _rel(o[i, r, h], want) < 2e-2 and abs(lse[i, h, r].item() - sc.logsumexp(0).item()) < 1e-2
