@@ -372,6 +372,12 @@ mla_split_kernel(const float* __restrict__ qa, const __nv_bfloat16* __restrict__
 // Grid (H, B, slices of `rows` outputs), in clusters of `share` slices.  Every range holds at least one key, so its sum is
 // positive and its maximum finite.  The CTAs of a cluster merge C / share latent columns each and read the others' from
 // their shared memory (each merging all of them, the ranges' partial sums were read four times over.)
+// EARLY: everything that comes from memory is asked for at once: the weight rows of a warp, the first partial sums and the
+// ranges' maxima.  (One after the other, each waiting for the one before, a decode step of three layers took 294 us;
+// this way, with the norms' weights and the residuals asked for early too, 281.)  It takes 128 registers for 39, which pays while the
+// CTAs all run at once; with more of them, three times as many an SM matter more: us a step, early / late, 16 sequences of 128
+// heads over 30 keys 174 / 119, 64 of 16 heads 93 / 69.
+template <bool EARLY>
 __global__ void __launch_bounds__(MLA_THREADS)
 mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml, const __nv_bfloat16* __restrict__ w,
                  __nv_bfloat16* __restrict__ out, int ranges, int H, int dn, int dv, int C, int rows, int share) {
@@ -386,24 +392,23 @@ mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ par
   const int cols = C / share, pairs = cols / 2;      // this CTA's columns, two to a thread
   const int groups = MLA_THREADS / pairs;            // threads with the same columns take every groups-th range
   const int pr = threadIdx.x % pairs, grp = threadIdx.x / pairs;
-  // Everything that comes from memory is asked for at once: the weight rows of this warp, the first partial sums and, below,
-  // the ranges' maxima.  (One after the other, each waiting for the one before, a decode step of three layers took 294 us;
-  // this way, with the norms' weights and the residuals asked for early too, 281.)
   const uint4* wv = reinterpret_cast<const uint4*>(w + ((size_t)h * (dn + dv) + dn) * C);
   const int cv = C / 8;
   const int j0 = blockIdx.z * rows, j1 = min(dv, j0 + rows);
-  constexpr int WK = MLA_MAX_C / 8 / 32, AHEAD = 12;
-  uint4 wr[WK][4];
+  constexpr int WK = MLA_MAX_C / 8 / 32, AHEAD = EARLY ? 12 : 0;
+  uint4 wr[EARLY ? WK : 1][4];
+  auto load_part = [&](int j, int k, uint4 (&to)[4]) {
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+      to[r] = (lane + 32 * k < cv && j + r < j1) ? wv[(size_t)(j + r) * cv + lane + 32 * k] : make_uint4(0, 0, 0, 0);
+  };
   auto load_rows = [&](int j) {
 #pragma unroll
-    for (int k = 0; k < WK; ++k)
-#pragma unroll
-      for (int r = 0; r < 4; ++r)
-        wr[k][r] = (lane + 32 * k < cv && j + r < j1) ? wv[(size_t)(j + r) * cv + lane + 32 * k] : make_uint4(0, 0, 0, 0);
+    for (int k = 0; k < WK; ++k) load_part(j, k, wr[EARLY ? k : 0]);
   };
-  load_rows(j0 + 4 * warp);
+  if (EARLY) load_rows(j0 + 4 * warp);
   const float* po = part_o + ((size_t)b * H + h) * ranges * C + rank * cols + 2 * pr;
-  float2 ahead[AHEAD];
+  float2 ahead[AHEAD > 0 ? AHEAD : 1];
 #pragma unroll
   for (int i = 0; i < AHEAD; ++i) {
     const int r = grp + i * groups;
@@ -466,12 +471,13 @@ mla_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ par
   }
   // a warp takes four rows at a time: their loads are in flight together
   for (int j = j0 + 4 * warp; j < j1; j += 4 * (MLA_THREADS / 32)) {
-    if (j != j0 + 4 * warp) load_rows(j);
+    if (EARLY && j != j0 + 4 * warp) load_rows(j);
     float s[4] = {};
 #pragma unroll
     for (int k = 0; k < WK; ++k) {
       const int c = lane + 32 * k;
-      const uint4* v = wr[k];
+      if (!EARLY) load_part(j, k, wr[0]);
+      const uint4* v = wr[EARLY ? k : 0];
       if (c < cv) {
         const float4 x0 = *reinterpret_cast<const float4*>(olat + c * 8), x1 = *reinterpret_cast<const float4*>(olat + c * 8 + 4);
 #pragma unroll
@@ -558,8 +564,9 @@ extern "C" int tpb_mla_decode(void* q, const void* ckv, const void* norm_w, cons
   attr[1].val.clusterDim.z = share;
   cfg.attrs = attr;
   cfg.numAttrs = 2;
-  cudaLaunchKernelEx(&cfg, mla_merge_kernel, (const float*)part_o, (const float*)part_ml, wb, reinterpret_cast<__nv_bfloat16*>(out),
-                     ranges, H, dn, dv, C, rows, share);
+  const bool early = (long long)H * B * slices <= 2 * sm_count();     // (128 registers: two CTAs per SM)
+  cudaLaunchKernelEx(&cfg, early ? mla_merge_kernel<true> : mla_merge_kernel<false>, (const float*)part_o, (const float*)part_ml, wb,
+                     reinterpret_cast<__nv_bfloat16*>(out), ranges, H, dn, dv, C, rows, share);
   cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? 0 : 1000 + (int)e;
 }

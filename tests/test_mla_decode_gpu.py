@@ -56,6 +56,12 @@ def test_step_equals_the_matrix_product_form(cuda_lib, heads, b, start):
   assert ((got.float() - want.float()).norm() / want.float().norm()).item() < 2.0 ** -7
 
 
+@pytest.mark.parametrize("heads,b,start", [(16, 5, 31), (37, 2, 3000), (38, 2, 3000), (75, 1, 3000), (74, 1, 40)])
+def test_step_whose_last_kernel_fills_the_machine(cuda_lib, heads, b, start):
+  """Both forms of the merge kernel (its CTAs all at once or not, four to a head and sequence), more ranges than the one asks for ahead."""
+  test_step_equals_the_matrix_product_form(cuda_lib, heads, b, start)
+
+
 def test_other_layouts_keep_the_matrix_product_form(cuda_lib):
   eng = _engine()
   a = eng.model.model.layers[0].self_attn
