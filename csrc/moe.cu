@@ -409,7 +409,7 @@ moe_plan_kernel(const int* __restrict__ idx, int n, int K, int E, int M, int ali
   __shared__ int total_s[PLAN_MAX_E];
   __shared__ int scan[PLAN_MAX_E / 32];
   const int ctas = gridDim.x, rank = blockIdx.x;               // one cluster
-  const int tile = min(align, 128);
+  const int tile_log = 31 - __clz(min(align, 128));
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int gtid = rank * PLAN_THREADS + threadIdx.x, gthreads = ctas * PLAN_THREADS;
   for (int e = lane; e < E; e += 32) wcount[warp][e] = 0;
@@ -447,9 +447,10 @@ moe_plan_kernel(const int* __restrict__ idx, int n, int K, int E, int M, int ali
   } else {
     total = own;
   }
-  // padded segments: a scan over the experts, 32 to a warp
+  // padded segments: a scan over the experts, 32 to a warp (align and tile are powers of two)
+  int pad = 0, start = 0;
   if (threadIdx.x < PLAN_MAX_E) {
-    const int pad = threadIdx.x < E ? (total + align - 1) / align * align : 0;
+    pad = threadIdx.x < E ? (total + align - 1) & ~(align - 1) : 0;
     int sum = pad;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -457,32 +458,31 @@ moe_plan_kernel(const int* __restrict__ idx, int n, int K, int E, int M, int ali
       if (lane >= o) sum += v;
     }
     if (lane == 31) scan[warp] = sum;
-    off_pad[threadIdx.x + 1] = sum;
-    total_s[threadIdx.x] = total;
-    if (threadIdx.x < E && rank == 0) counts[threadIdx.x] = total;
+    start = sum - pad;
   }
   __syncthreads();
-  if (threadIdx.x < PLAN_MAX_E) {
-    int add = 0;
-    for (int w = 0; w < warp; ++w) add += scan[w];
-    off_pad[threadIdx.x + 1] += add;
-  }
-  if (threadIdx.x == 0) off_pad[0] = 0;
-  __syncthreads();
-  if (rank == 0 && threadIdx.x <= E) k_offsets[threadIdx.x] = off_pad[threadIdx.x];
   if (threadIdx.x < E) {
-    int run = off_pad[threadIdx.x] + before;
+    for (int w = 0; w < warp; ++w) start += scan[w];
+    const int end = start + pad;
+    off_pad[threadIdx.x] = start;
+    total_s[threadIdx.x] = total;
+    if (threadIdx.x == E - 1) off_pad[E] = end;
+    if (rank == 0) {
+      counts[threadIdx.x] = total;
+      k_offsets[threadIdx.x] = start;
+      if (threadIdx.x == E - 1) k_offsets[E] = end;
+      for (int t = start >> tile_log; t < end >> tile_log; ++t) tile_expert[t] = threadIdx.x;
+    }
+    int run = start + before;
 #pragma unroll 8
     for (int w = 0; w < 32; ++w) {
       const int c = wcount[w][threadIdx.x];
       wcount[w][threadIdx.x] = run;
       run += c;
     }
-    if (rank == 0)
-      for (int t = off_pad[threadIdx.x] / tile; t < off_pad[threadIdx.x + 1] / tile; ++t) tile_expert[t] = threadIdx.x;
   }
-  for (int t = off_pad[E] / tile + gtid; t < M / tile; t += gthreads) tile_expert[t] = -1;
   __syncthreads();
+  for (int t = (off_pad[E] >> tile_log) + gtid; t < M >> tile_log; t += gthreads) tile_expert[t] = -1;
   // padding rows: the end of every expert's segment (one warp per expert) and everything past the last
   // one (filled here and not by memsets of the whole arrays: three launches fewer)
   for (int e = gwarp; e < E; e += warps) {
