@@ -274,7 +274,7 @@ __global__ void moe_gather_kernel(const uint4* __restrict__ x, const int* __rest
 // out[t, :] = sum_k w[t,k] * rows[dest[t,k], :]   (dest < 0: dropped pair; w null: weight 1)
 // The rows of KA pairs of a thread are on their way together: eight where there are fewer threads than the machine holds (a decode
 // step's four tokens of six experts 9.3 -> 7.3 us with its launch, 300 tokens 11.3 -> 9.3), one where the others hide
-// the wait and registers count (4096 tokens, two experts 26.7 us; 31.8 with eight).
+// the wait and registers count (4096 tokens, two experts 26.7 us; 31.8 with eight), and for one pair (16 tokens of 5120 2.7 -> 2.2).
 template <int KA>
 __global__ void moe_combine_kernel(const uint4* __restrict__ rows, const int* __restrict__ dest,
                                    const float* __restrict__ w, uint4* __restrict__ out, long long tokens, int K,
@@ -286,21 +286,30 @@ __global__ void moe_combine_kernel(const uint4* __restrict__ rows, const int* __
     const long long t = i / nvec;
     const int c = (int)(i % nvec);
     float acc[8] = {};
-    for (int k0 = 0; k0 < K; k0 += KA) {
-      int r[KA];
-      uint4 v[KA];
+    auto add = [&](int k, const uint4& v) {
+      const float wk = w ? w[t * K + k] : 1.f;
+      const float2 a = unpack_bf16(v.x), b = unpack_bf16(v.y), cc = unpack_bf16(v.z), d = unpack_bf16(v.w);
+      acc[0] += wk * a.x; acc[1] += wk * a.y; acc[2] += wk * b.x; acc[3] += wk * b.y;
+      acc[4] += wk * cc.x; acc[5] += wk * cc.y; acc[6] += wk * d.x; acc[7] += wk * d.y;
+    };
+    if (KA == 1) {
+      for (int k = 0; k < K; ++k) {
+        const int r = dest[t * K + k];
+        if (r < 0) continue;
+        add(k, rows[(long long)r * nvec + c]);
+      }
+    } else {
+      for (int k0 = 0; k0 < K; k0 += KA) {
+        int r[KA];
+        uint4 v[KA];
 #pragma unroll
-      for (int k = 0; k < KA; ++k) r[k] = k0 + k < K ? dest[t * K + k0 + k] : -1;
+        for (int k = 0; k < KA; ++k) r[k] = k0 + k < K ? dest[t * K + k0 + k] : -1;
 #pragma unroll
-      for (int k = 0; k < KA; ++k)
-        if (r[k] >= 0) v[k] = rows[(long long)r[k] * nvec + c];
+        for (int k = 0; k < KA; ++k)
+          if (r[k] >= 0) v[k] = rows[(long long)r[k] * nvec + c];
 #pragma unroll
-      for (int k = 0; k < KA; ++k) {
-        if (r[k] < 0) continue;
-        const float wk = w ? w[t * K + k0 + k] : 1.f;
-        const float2 a = unpack_bf16(v[k].x), b = unpack_bf16(v[k].y), cc = unpack_bf16(v[k].z), d = unpack_bf16(v[k].w);
-        acc[0] += wk * a.x; acc[1] += wk * a.y; acc[2] += wk * b.x; acc[3] += wk * b.y;
-        acc[4] += wk * cc.x; acc[5] += wk * cc.y; acc[6] += wk * d.x; acc[7] += wk * d.y;
+        for (int k = 0; k < KA; ++k)
+          if (r[k] >= 0) add(k0 + k, v[k]);
       }
     }
     out[i] = make_uint4(pack_bf16(acc[0], acc[1]), pack_bf16(acc[2], acc[3]), pack_bf16(acc[4], acc[5]),
@@ -793,7 +802,7 @@ extern "C" int tpb_moe_combine(const void* rows, const int* dest, const float* w
   if (dim % 8) return -2;
   if (tokens <= 0) return 0;
   const long long items = tokens * (dim / 8);
-  if (items <= 512LL * sm_count())
+  if (K > 1 && items <= 512LL * sm_count())
     chain(moe_combine_kernel<8>, grid_for_items(items, 256), 256, 0, STREAM(stream), (const uint4*)rows, dest, w, (uint4*)out, tokens,
           K, dim / 8);
   else
