@@ -265,3 +265,13 @@ def test_moe_models_train_on_gpu_and_match_torch_backend(cuda_lib, model, extra,
   for (la, ga), (lb, gb) in zip(losses["auto"], losses["torch"]):
     assert abs(la - lb) < 0.05, losses
     assert abs(ga - gb) / max(gb, 1e-6) < 0.1, losses
+
+
+@pytest.mark.parametrize("E,K,T,align", [(64, 6, 1440, 128), (64, 6, 1451, 256), (64, 6, 2560, 256), (64, 6, 2570, 128), (64, 6, 4700, 128),
+                                         (64, 6, 4779, 256), (64, 6, 5640, 128), (128, 8, 3200, 128), (128, 8, 7168, 256), (256, 8, 4096, 128),
+                                         (256, 8, 14400, 256), (16, 1, 2048, 256), (16, 1, 8500, 128), (8, 2, 2500, 128), (8, 2, 4096, 256)])
+def test_segment_rows_by_experts(cuda_lib, E, K, T, align):
+  """The average load decides together with the number of experts: many of them keep to 128 rows where only even loads would gain."""
+  idx = torch.rand(T, E, device="cuda").topk(K, -1)[1].to(torch.int32)
+  plan = moe.build_dispatch_plan(idx, E)
+  assert plan.row_align == align

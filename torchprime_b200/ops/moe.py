@@ -143,14 +143,30 @@ class DispatchPlan:
                              # below 128 only grouped_mlp_few_rows can read the plan)
 
 
-def pair_tiles_pay(per: float) -> bool:
+def pair_tiles_pay(per: float, experts: int) -> bool:
   """Whether segments of 256 rows, which let the grouped GEMMs use 256 x 256 CTA-pair tiles, are worth their padding for
-  ``per`` rows per expert on average.  They are where the second half of the last segment is used by most experts, and from
-  two segments on.  Routed MLP, both passes but two weight gradients, 128 / 256 rows (us):
-  64 experts of 2048 x 1408: 112 rows 829 / 883, 144 970 / 915, 224 1080 / 1014, 256 1243 / 1267, 320 1389 / 1478, 448 1547 / 1408
-  16 experts of 5120 x 8192: 112 rows 2687 / 2815, 128 3144 / 2787, 224 3489 / 3244, 288 4498 / 4694, 384 5142 / 4708
-  8 experts of 4096 x 14336: 112 rows 1919 / 1876, 160 2319 / 2032, 288 2978 / 3298, 448 3904 / 3465, 768 6080 / 5610"""
-  return 128 <= per <= 240 or per >= 352
+  ``per`` rows per expert on average: a row costs 0.88 of what it does on 128-row tiles, so they are where the second half of the
+  last segment is used by most experts, and from some segments on.  How many rows each expert gets is only known on the
+  device; with many experts some are far from the average, and loads that differ take the first of the two away.  Time with 128-row
+  segments over that with 256-row ones of the routed MLP, both passes; even loads / loads that differ by half an average / by a whole one:
+      rows   8 experts, 4096 x 14336   16, 5120 x 8192       64, 2048 x 1408       128, 2048 x 768       256, 7168 x 2048
+      100    1.03 / 1.11 / 1.08        0.93 / 0.93 / 0.97    0.92 / 0.98 / 0.95    0.85 / 0.90 / 0.94    0.91 / 0.94 / 0.97
+      128    1.09 / 1.09 / 0.92        1.08 / 1.00 / 0.94    0.99 / 1.01 / 0.96    0.95 / 0.94 / 0.97    1.01 / 0.97 / 0.98
+      144    1.18 / 1.19 / 1.02        1.15 / 0.99 / 0.98    1.10 / 0.99 / 0.97    1.08 / 0.96 / 0.94    1.16 / 0.95 / 0.97
+      200    1.13 / 1.11 / 1.10        1.15 / 1.04 / 1.02    1.10 / 1.00 / 0.95    1.05 / 0.96 / 0.95    1.11 / 0.98 / 0.98
+      240    1.15 / 1.01 / 0.98        1.13 / 1.02 / 1.03    1.12 / 1.01 / 0.96    1.06 / 1.00 / 0.98    1.10 / 1.02 / 0.97
+      280    0.98 / 0.98 / 0.99        0.96 / 0.99 / 0.99    0.96 / 1.03 / 1.03    0.95 / 1.00 / 0.97    0.90 / 0.99 / 1.02
+      352    1.04 / 1.17 / 1.10        1.02 / 1.08 / 1.03    0.98 / 1.09 / 1.03    0.96 / 0.99 / 0.99    0.92 / 0.99 / 0.99
+      448    1.13 / 1.13 / 1.00        1.12 / 1.04 / 0.98    1.13 / 1.04 / 1.01    1.15 / 1.04 / 1.01    1.13 / 1.01 / 1.01
+      600    1.01 / 1.07 / 1.03        0.95 / 1.06 / 1.04    1.04 / 1.06 / 1.03    1.03 / 1.05 / 1.05    0.95 / 0.99 / 1.01
+      900    1.12 / 1.14 / 1.02        1.11 / 1.07 / 1.05    1.08 / 1.04 / 1.06    1.07 / 1.09 / 1.07    1.03 / 1.00 / 0.99
+  The buffers hold the worst case, 127 or 255 rows more than its pairs for every expert: half as much again at 136 rows on average,
+  another reason why many experts keep to 128 there."""
+  if 528 <= per <= 640:
+    return False
+  if experts <= 16:
+    return 128 <= per <= 240 or per >= 352
+  return (experts <= 64 and 136 <= per <= 240) or per >= 448
 
 
 def build_dispatch_plan(idx: torch.Tensor, num_experts: int, capacity: int | None = None,
@@ -165,7 +181,7 @@ def build_dispatch_plan(idx: torch.Tensor, num_experts: int, capacity: int | Non
   e = num_experts
   dev = idx.device
   if row_align is None:
-    row_align = 256 if capacity is None and pair_tiles_pay(t * k / e) else ROW_ALIGN
+    row_align = 256 if capacity is None and pair_tiles_pay(t * k / e, e) else ROW_ALIGN
   assert row_align in (128, 256)
   if use_kernel is None:
     use_kernel = capacity is None and idx.is_cuda and _kernels_ok() and e <= 256
