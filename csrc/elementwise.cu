@@ -108,6 +108,22 @@ rmsnorm_fwd_kernel(const uint4* __restrict__ x, const uint4* __restrict__ res, c
   }
 }
 
+// dx of a vector from o = g - xh * dot, with every rounding said: g = dy * w and xh = x * rstd are products rounded by themselves,
+// and the residual's gradient is added to the rounded value or (fused) inside the last multiplication.  Which of the two is what the
+// compiler once chose, kept so that a size's gradients stay the same bits: fused in rows above 2048 where a CTA takes a row, and
+// in streamed rows for all but the last of the 1, 2 or 4 vectors that a thread of 256 would have.
+__device__ __forceinline__ void norm_dx(float (&o)[8], float rs, const uint4* res, bool fused) {
+  if (res) {
+    float r[8];
+    unpack8(*res, r);
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] = fused ? fmaf(rs, o[e], r[e]) : __fadd_rn(__fmul_rn(rs, o[e]), r[e]);
+  } else {
+#pragma unroll
+    for (int e = 0; e < 8; ++e) o[e] = __fmul_rn(rs, o[e]);
+  }
+}
+
 template <int VPT>
 __global__ void __launch_bounds__(NORM_THREADS)
 rmsnorm_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x, const uint4* __restrict__ w,
@@ -138,10 +154,10 @@ rmsnorm_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x, co
         unpack8(x[(size_t)row * nvec + i], xv);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          xh[j][e] = xv[e] * rs;
-          dw_acc[j][e] += dyv[e] * xh[j][e];
-          g[j][e] = dyv[e] * wv[j][e];
-          dot += g[j][e] * xh[j][e];
+          xh[j][e] = __fmul_rn(xv[e], rs);
+          dw_acc[j][e] = fmaf(dyv[e], xh[j][e], dw_acc[j][e]);
+          g[j][e] = __fmul_rn(dyv[e], wv[j][e]);
+          dot = fmaf(g[j][e], xh[j][e], dot);
         }
       }
     }
@@ -152,13 +168,8 @@ rmsnorm_bwd_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ x, co
       if (i < nvec) {
         float o[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = rs * (g[j][e] - xh[j][e] * dot);
-        if (dres) {
-          float r[8];
-          unpack8(dres[(size_t)row * nvec + i], r);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) o[e] += r[e];
-        }
+        for (int e = 0; e < 8; ++e) o[e] = fmaf(-xh[j][e], dot, g[j][e]);
+        norm_dx(o, rs, dres ? dres + (size_t)row * nvec + i : nullptr, VPT > 1);
         dx[(size_t)row * nvec + i] = pack8(o);
       }
     }
@@ -195,8 +206,26 @@ __device__ __forceinline__ void bulk_row_load(void* smem_dst, const void* src, u
                : "memory");
 }
 
+// The sum of a row in the order of 256 threads: p[w] is what the lanes of their warp w hold, added up over the lanes as warp_sum does
+// and over the warps as block_sum does, in twelve shuffles (each halves the number of sums a lane has under way).
+__device__ __forceinline__ float sum_of_warps(const float (&p)[8]) {
+  const int lane = threadIdx.x & 31;
+  float q[4], r[2];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) q[i] = (lane & 16 ? p[i + 4] : p[i]) + __shfl_xor_sync(0xffffffffu, lane & 16 ? p[i] : p[i + 4], 16);
+#pragma unroll
+  for (int i = 0; i < 2; ++i) r[i] = (lane & 8 ? q[i + 2] : q[i]) + __shfl_xor_sync(0xffffffffu, lane & 8 ? q[i] : q[i + 2], 8);
+  float s = (lane & 4 ? r[1] : r[0]) + __shfl_xor_sync(0xffffffffu, lane & 4 ? r[0] : r[1], 4);
+  s += __shfl_xor_sync(0xffffffffu, s, 2);
+  s += __shfl_xor_sync(0xffffffffu, s, 1);         // the sum of warp lane / 4 (bits 4, 3, 2)
+  s += __shfl_xor_sync(0xffffffffu, s, 16);
+  s += __shfl_xor_sync(0xffffffffu, s, 8);
+  s += __shfl_xor_sync(0xffffffffu, s, 4);
+  return s;
+}
+
 // Forward: a warp to a row, the row in its registers (VPL 16-byte vectors a lane), its next rows on their way.  The sum over
-// the row is five shuffles.  8192 x 4096: 26.0 us (5.2 TB/s), 27.3 with 256 threads to a row and three barriers; x 2048 16 and 27.
+// the row is twelve shuffles, in the order of the other forms, so that all give the same bits.  8192 x 4096: 26.0 us (5.2 TB/s), 27.3 with 256 threads to a row and three barriers; x 2048 16 and 27.
 template <int VPL>
 __global__ void __launch_bounds__(512)
 rmsnorm_fwd_rows_kernel(const uint4* __restrict__ x, const uint4* __restrict__ w, uint4* __restrict__ y,
@@ -229,7 +258,7 @@ rmsnorm_fwd_rows_kernel(const uint4* __restrict__ x, const uint4* __restrict__ w
     if (!mbar_wait_warp(&full[k % stages], (uint32_t)(k / stages) & 1u, status, kTimeoutTmaFull, 73)) break;
     const uint4* sx = ring + (k % stages) * nvec;
     uint4 v[VPL];
-    float ss = 0.f;
+    float ss[8] = {};           // by warps of 256 threads: vector i is thread i % 256's
 #pragma unroll
     for (int j = 0; j < VPL; ++j) {
       const int i = lane + 32 * j;
@@ -238,7 +267,7 @@ rmsnorm_fwd_rows_kernel(const uint4* __restrict__ x, const uint4* __restrict__ w
         float f[8];
         unpack8(v[j], f);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) ss += f[e] * f[e];
+        for (int e = 0; e < 8; ++e) ss[j & 7] += f[e] * f[e];
       }
     }
     __syncwarp();
@@ -247,7 +276,7 @@ rmsnorm_fwd_rows_kernel(const uint4* __restrict__ x, const uint4* __restrict__ w
       issue(issued);
     }
     issued += issued < mine;
-    const float rstd = rsqrtf(warp_sum(ss) / (float)(nvec * 8) + eps);
+    const float rstd = rsqrtf(sum_of_warps(ss) / (float)(nvec * 8) + eps);
     const size_t row = (size_t)first + (size_t)k * step;
     if (lane == 0 && rstd_out) rstd_out[row] = rstd;
 #pragma unroll
@@ -358,7 +387,7 @@ rmsnorm_bwd_rows_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ 
   if (!chain_begin()) return;
   extern __shared__ uint8_t nb_smem_raw[];
   uint8_t* smem = nb_smem_raw + ((128u - (smem_u32(nb_smem_raw) & 127u)) & 127u);
-  __shared__ __align__(16) float red[GROUPS][2][4];
+  __shared__ __align__(16) float red[GROUPS][2][8];
   const int warp = warp_index(), lane = threadIdx.x & 31;
   const int grp = warp / 4, tid = threadIdx.x % NB_GROUP;
   const uint32_t row_bytes = (uint32_t)nvec * 16u;
@@ -401,7 +430,7 @@ rmsnorm_bwd_rows_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ 
     const size_t row = (size_t)first + (size_t)k * step;
     const float rs_next = k + 1 < mine ? rstd[row + step] : 0.f;
     uint4 dv[VPT], xv[VPT], rv[VPT];
-    float dot = 0.f;
+    float dots[2] = {};         // this thread's of 256, and thread + 128's
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
       const int i = tid + j * NB_GROUP;
@@ -415,14 +444,18 @@ rmsnorm_bwd_rows_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ 
         unpack8(sw[i], wv);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
-          const float xh = xf[e] * rs;
-          acc[j][e] += d[e] * xh;
-          dot += d[e] * wv[e] * xh;
+          const float xh = __fmul_rn(xf[e], rs);
+          acc[j][e] = fmaf(d[e], xh, acc[j][e]);
+          dots[j & 1] = fmaf(__fmul_rn(d[e], wv[e]), xh, dots[j & 1]);
         }
       }
     }
-    dot = warp_sum(dot);
-    if (lane == 0) red[grp][k & 1][warp & 3] = dot;
+    dots[0] = warp_sum(dots[0]);
+    dots[1] = warp_sum(dots[1]);
+    if (lane == 0) {
+      red[grp][k & 1][warp & 3] = dots[0];
+      red[grp][k & 1][4 + (warp & 3)] = dots[1];
+    }
     // the row's sum is complete, its stage has been read, and all of the group know whether one of them gave up waiting
     int all;
     asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.b32 p, %1, 0;\n\tbarrier.cta.red.and.pred q, %2, %3, p;\n\tselp.b32 %0, 1, 0, q;\n\t}"
@@ -435,8 +468,8 @@ rmsnorm_bwd_rows_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ 
       issue(issued);
     }
     issued += issued < mine;
-    const float4 r4 = *reinterpret_cast<const float4*>(red[grp][k & 1]);
-    dot = ((r4.x + r4.y) + (r4.z + r4.w)) * inv_d;
+    const float4 a4 = *reinterpret_cast<const float4*>(red[grp][k & 1]), b4 = *reinterpret_cast<const float4*>(red[grp][k & 1] + 4);
+    const float dot = (((a4.x + b4.x) + (a4.z + b4.z)) + ((a4.y + b4.y) + (a4.w + b4.w))) * inv_d;   // as block_sum adds eight warps
 #pragma unroll
     for (int j = 0; j < VPT; ++j) {
       const int i = tid + j * NB_GROUP;
@@ -446,13 +479,8 @@ rmsnorm_bwd_rows_kernel(const uint4* __restrict__ dy, const uint4* __restrict__ 
         unpack8(xv[j], xf);
         unpack8(sw[i], wv);
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] = rs * (d[e] * wv[e] - xf[e] * rs * dot);
-        if (dres) {
-          float r[8];
-          unpack8(rv[j], r);
-#pragma unroll
-          for (int e = 0; e < 8; ++e) o[e] += r[e];
-        }
+        for (int e = 0; e < 8; ++e) o[e] = fmaf(-__fmul_rn(xf[e], rs), dot, __fmul_rn(d[e], wv[e]));
+        norm_dx(o, rs, dres ? &rv[j] : nullptr, (j >> 1) < (VPT <= 2 ? 0 : VPT <= 4 ? 1 : 3));
         dx[row * nvec + i] = pack8(o);
       }
     }
@@ -907,7 +935,7 @@ static bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 
 //     8192 48 / 36 / 47;   8192: 1200 11.2 / 8.9 / 17, 3200 26.7 / 18.5 / 31.5, 8192 61 / 43.7 / 75.5
 //   backward with a residual, 4096 wide: 1000 rows 23 / 19, 4000 33 / 31, 8192 55 / 50;   5120 wide: 2000 29 / 22, 8192 93 / 60;
 //     8192 wide: 600 rows 23.4 / 16.0, 1000 33.5 / 19.3
-static int norm_bwd_rows_from(int dim) { return dim > 4096 ? 576 : 1024; }
+static int norm_bwd_rows_from(int dim) { return dim > 4096 ? 592 : 1024; }
 static int norm_fwd_rows_from(int nvec) { return nvec <= 96 ? 3000 : nvec <= 256 ? 12000 : nvec <= 384 ? 2048 : 4500; }
 static bool launch_rmsnorm_fwd_rows(const void* x, const void* w, void* y, float* rstd, int rows, int dim, float eps,
                                     cudaStream_t stream) {
