@@ -5,7 +5,7 @@
 // (about 80 GB/s), while HBM would feed all 148.  Here the roles are swapped and the contraction is split:
 //   * W is the A operand: 128 output features are the 128 lanes of the accumulator, and the tokens
 //     are the N dimension of the MMA (a multiple of 16 up to 128), so no MMA or shared-memory bandwidth goes into rows
-//     that do not exist beyond the next of those sizes;
+//     that do not exist beyond the next multiple of 16 (but for the last half chunk of the accumulator's read at 48, 80 or 112);
 //   * a cluster of S <= 8 CTAs shares one 128-feature tile, each CTA contracting over 1/S of K.
 //     The fp32 partial tiles meet in distributed shared memory, where every CTA adds the S partials of
 //     1/S of the tokens in rank order (no workspace, no atomics, the same result every run).

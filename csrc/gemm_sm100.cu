@@ -1289,7 +1289,7 @@ static int run_gemm(const GemmCall& g, cudaStream_t stream) {
   // CTA pairs: whatever the number of their tiles.  What an SM does is the same (128 x 256 results), but a pair's SM brings in and
   // reads half of B: 512 clocks a k-block, where the single kernel is bound by shared memory at 768.  us, single / pair, 64 tiles
   // or fewer of 256 x 256: K = 4096, 300 to 1024 rows 30 / 25; K = 2048, 900 x 3072 17.7 / 16.1, 2048 x 2048 17.7 / 16.1; K = 10944,
-  // 2048 x 2048 73.7 / 61.3; K = 512, 4096 columns 10.5 / 10.3 (profiles/pair_tiles_gemm_sweep.md).  Up to 128 rows half of a pair has
+  // 2048 x 2048 73.7 / 61.3; K = 512, 4096 columns 10.5 / 10.3.  Up to 128 rows half of a pair has
   // none.  With a gather or a scatter inside, where the tiles fill the machine.
   const int pair_mode = gemm_pair_mode();
   static const int max_pairs = resident_clusters(2);

@@ -347,3 +347,17 @@ def test_two_products_allocate_nothing_where_they_do_not_run(cuda_lib, rows):
   with torch.no_grad():
     assert ops._native().linear_pair(x, w1, w2) is None
   assert torch.cuda.memory_stats()["allocation.all.allocated"] == before
+
+
+@pytest.mark.parametrize("rows", [129, 200, 300, 469])
+@pytest.mark.parametrize("n1,n2,kk", [(3072, 576, 2048), (1536, 576, 5120), (1024, 264, 1032)])
+def test_two_products_of_more_rows_than_a_tile(cuda_lib, rows, n1, n2, kk):
+  """Several token tiles, the second product's behind the first one's in the grid."""
+  from torchprime_b200.ops import functional as ops
+  torch.manual_seed(rows)
+  x = torch.randn(rows, kk, device="cuda", dtype=torch.bfloat16)
+  w1, w2 = (torch.randn(n, kk, device="cuda", dtype=torch.bfloat16) for n in (n1, n2))
+  with torch.no_grad():
+    both = ops.linear_pair(x, w1, w2)
+  for y, w in zip(both, (w1, w2)):
+    _close(y, x.double() @ w.double().t(), float(kk))
