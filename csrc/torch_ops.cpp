@@ -427,16 +427,25 @@ variable_list norm_bwd(AutogradContext* ctx, const Tensor& dy_, const Tensor& dr
   TORCH_CHECK(plain(dy) && (!dres.defined() || plain(dres)), "rms_norm: gradient of an unexpected kind");
   const int64_t d = x.size(-1);
   const int rows = (int)(x.numel() / d);
-  Tensor dx = empty_as(x, x.sizes()), dwf = empty_like_type(w, {d}, at::kFloat), dw, parts;
-  if (const int n = tpb_rmsnorm_bwd_parts(rows, (int)d)) parts = empty_like_type(w, {n, d}, at::kFloat);
   const bool late = ctx->needs_input_grad(1) && any_main_grad(&w, 1);
-  if (ctx->needs_input_grad(1) && !late) dw = empty_as(w, {d});
+  // fp32 sums and scratch in one allocation, unless the sums are handed on and would keep the scratch alive
+  const int64_t n = tpb_rmsnorm_bwd_parts(rows, (int)d);
+  Tensor dx = empty_as(x, x.sizes()), sums, parts, dw;
+  if (late) {
+    sums = empty_like_type(w, {d}, at::kFloat);
+    if (n) parts = empty_like_type(w, {n, d}, at::kFloat);
+  } else {
+    sums = empty_like_type(w, {1 + n, d}, at::kFloat);
+    if (ctx->needs_input_grad(1)) dw = empty_as(w, {d});
+  }
+  float* const sums_p = static_cast<float*>(mptr(sums));
+  float* const parts_p = late ? static_cast<float*>(mptr(parts)) : n ? sums_p + d : nullptr;
   check(tpb_rmsnorm_bwd_dw(cptr(dy), cptr(x), cptr(w), static_cast<const float*>(cptr(rstd)), cptr(dres), mptr(dx),
-                           static_cast<float*>(mptr(dwf)), mptr(dw), static_cast<float*>(mptr(parts)), 0, rows, (int)d, stream()),
+                           sums_p, mptr(dw), parts_p, 0, rows, (int)d, stream()),
         "rmsnorm_bwd");
   if (late) {
     py::gil_scoped_acquire gil;
-    py::reinterpret_borrow<py::object>(g_late_norm)(py::reinterpret_steal<py::object>(THPVariable_Wrap(w)), py::cast(dwf));
+    py::reinterpret_borrow<py::object>(g_late_norm)(py::reinterpret_steal<py::object>(THPVariable_Wrap(w)), py::cast(sums));
   }
   return {dx, dw, Tensor()};
 }
