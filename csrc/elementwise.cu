@@ -225,7 +225,8 @@ __device__ __forceinline__ float sum_of_warps(const float (&p)[8]) {
 }
 
 // Forward: a warp to a row, the row in its registers (VPL 16-byte vectors a lane), its next rows on their way.  The sum over
-// the row is twelve shuffles, in the order of the other forms, so that all give the same bits.  8192 x 4096: 26.0 us (5.2 TB/s), 27.3 with 256 threads to a row and three barriers; x 2048 16 and 27.
+// the row is twelve shuffles, in the order of the other forms, so that all give the same bits.  8192 x 4096: 26.7 us (5.0 TB/s), 27.8
+// with 256 threads to a row and three barriers; x 3072 20 and 29.
 template <int VPL>
 __global__ void __launch_bounds__(512)
 rmsnorm_fwd_rows_kernel(const uint4* __restrict__ x, const uint4* __restrict__ w, uint4* __restrict__ y,
