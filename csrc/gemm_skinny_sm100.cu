@@ -390,6 +390,7 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constan
       store4(reinterpret_cast<__nv_bfloat16*>(second ? p.C2 : p.C) + (long long)row * (second ? p.ldC2 : p.ldc) + col, a, n);
     }
   }
+  __syncwarp();
   cluster_leave();           // nobody's shared memory goes away while a neighbour reads it
   if (warp == 1) {
     tc_fence_after();

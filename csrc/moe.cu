@@ -520,6 +520,7 @@ moe_plan_kernel(const int* __restrict__ idx, int n, int K, int E, int M, int ali
       src_pair[pos] = i;
     }
   }
+  __syncwarp();
   if (ctas > 1) cluster_leave();             // own_s is read by the others until here
 }
 

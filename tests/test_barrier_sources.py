@@ -58,3 +58,11 @@ def test_shared_arrays_read_as_vectors_are_aligned_for_them(name):
       if not decl.group(1):
         as_vector = re.search(r"reinterpret_cast<(?:const )?(?:float|int|uint|double)[24]\*>\(&?%s\b" % decl.group(3), body)
         assert as_vector is None, f"{kernel}: {decl.group(3)} is read as {as_vector.group()}"
+
+
+@pytest.mark.parametrize("name", FILES)
+def test_warps_part_from_a_cluster_together(name):
+  """The cluster barrier is the aligned one: all lanes of a warp arrive at once, also those that have left a loop early."""
+  for kernel, body in _kernels(_source(name)).items():
+    for m in re.finditer(r"(?:if \([^()]*\) )?cluster_leave\(\);", body):
+      assert re.search(r"__sync(?:threads|warp)\(\);\s*$", body[:m.start()]), f"{kernel} may part in pieces"
